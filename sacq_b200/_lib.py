@@ -11,6 +11,7 @@ import re
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libsacq_b200.so")
+NATIVE_PATH = os.path.join(HERE, "_native.so")
 HEADER_PATH = os.path.join(os.path.dirname(HERE), "include", "sacq_b200.h")
 
 SACQ_OK = 0
@@ -97,6 +98,7 @@ SIGNATURES = {
 }
 
 _lib = None
+_native = None
 
 
 def declared_symbols() -> list[str]:
@@ -124,6 +126,20 @@ def load() -> ctypes.CDLL:
         raise ImportError("libsacq_b200.so ABI version mismatch")
     _lib = lib
     return lib
+
+
+def native():
+    """The extension module with the host side of the layer calls (csrc/host/native_calls.cpp)."""
+    global _native
+    if _native is None:
+        load()
+        if not os.path.exists(NATIVE_PATH):
+            raise ImportError(f"{NATIVE_PATH} is missing. Build it with `python -m sacq_b200.build`.")
+        import torch  # noqa: F401  (its libraries have to be loaded first)
+        from . import _native as module
+        module.set_error_class(SacqError)
+        _native = module
+    return _native
 
 
 def last_error() -> str:

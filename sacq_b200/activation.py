@@ -17,6 +17,10 @@ from . import _lib
 
 def quantize_rows(x: torch.Tensor, mode: str = "fp8_e4m3fn", out: torch.Tensor | None = None,
                   scale_out: torch.Tensor | None = None):
+    if out is None and scale_out is None and (mode == "fp8_e4m3fn" or mode == "int8_symmetric"):
+        pair = _lib.native().quantize_rows(x, mode == "int8_symmetric")
+        if pair is not None:
+            return pair
     if x.ndim != 2 or x.dtype != torch.bfloat16:
         raise TypeError("quantize_rows expects a 2-D bfloat16 tensor")
     if mode not in ("fp8_e4m3fn", "int8_symmetric"):
@@ -49,6 +53,9 @@ def act_quantize_rows(kind: str, a: torch.Tensor, b: torch.Tensor | None = None)
     kinds = {"silu_mul": 0, "gelu": 1}
     if kind not in kinds:
         raise ValueError(f"unknown activation kind {kind!r}")
+    pair = _lib.native().act_quantize_rows(kinds[kind], a, b)
+    if pair is not None:
+        return pair
     if a.ndim != 2 or a.dtype != torch.bfloat16 or not a.is_cuda:
         raise TypeError("act_quantize_rows expects 2-D bfloat16 CUDA tensors")
     if kind == "silu_mul":
@@ -75,6 +82,9 @@ def modulate_quantize_rows(x: torch.Tensor, scale: torch.Tensor, shift: torch.Te
     """AdaLN modulation fused into the quantizer (``sacq_modulate_quant_fp8``): the bytes of
     ``quantize_rows(x * (1 + scale) + shift)`` for bf16 ``x [M, K]`` and bf16 vectors
     ``scale, shift [K]``, in one launch."""
+    pair = _lib.native().modulate_quantize_rows(x, scale, shift)
+    if pair is not None:
+        return pair
     if x.ndim != 2 or x.dtype != torch.bfloat16 or not x.is_cuda:
         raise TypeError("modulate_quantize_rows expects a 2-D bfloat16 CUDA tensor")
     k = x.shape[1]
@@ -103,6 +113,9 @@ def layernorm_quantize_rows(x: torch.Tensor, weight: torch.Tensor | None = None,
     ``(q, scale)`` or ``(q, scale, y)`` with the bf16 normalised tensor.  ``y`` agrees with
     ``torch.nn.functional.layer_norm`` to one bf16 ulp (different reduction order); ``q`` and
     ``scale`` are exactly ``quantize_rows(y)``."""
+    made = _lib.native().layernorm_quantize_rows(x, weight, bias, eps, mod_scale, mod_shift, return_normalized)
+    if made is not None:
+        return made
     if x.ndim != 2 or x.dtype != torch.bfloat16 or not x.is_cuda:
         raise TypeError("layernorm_quantize_rows expects a 2-D bfloat16 CUDA tensor")
     k = x.shape[1]

@@ -1,4 +1,5 @@
-"""Builds ``libsacq_b200.so`` in-tree with nvcc for sm_100a.
+"""Builds ``libsacq_b200.so`` in-tree with nvcc for sm_100a, and ``_native.so``, the host side of the
+layer calls as a CPython extension (g++ against the installed PyTorch), beside it.
 
     python -m sacq_b200.build [--force] [--verbose]
 
@@ -20,6 +21,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ_DIR = os.path.join(HERE, "build")
 LIB_PATH = os.path.join(HERE, "libsacq_b200.so")
+NATIVE_SRC = os.path.join(CSRC, "host", "native_calls.cpp")
+NATIVE_PATH = os.path.join(HERE, "_native.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -53,9 +56,33 @@ def up_to_date() -> bool:
     return all(os.path.getmtime(p) <= t for p in _deps())
 
 
+def build_native(force: bool = False) -> str:
+    """Compile the extension module if its source or the public header is newer.  Returns its path."""
+    deps = [NATIVE_SRC, os.path.abspath(__file__)] + glob.glob(os.path.join(HERE, "..", "include", "*.h"))
+    if not force and os.path.exists(NATIVE_PATH) and \
+            all(os.path.getmtime(p) <= os.path.getmtime(NATIVE_PATH) for p in deps):
+        return NATIVE_PATH
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+           f"-I{root}/include", f"-I{root}/include/torch/csrc/api/include", f"-I{cuda}/include",
+           f"-I{sysconfig.get_paths()['include']}", NATIVE_SRC, "-o", NATIVE_PATH,
+           f"-L{root}/lib", f"-L{HERE}", "-l:libsacq_b200.so", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda",
+           "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError("g++ failed for %s:\n%s\n%s" % (NATIVE_SRC, res.stdout, res.stderr))
+    return NATIVE_PATH
+
+
 def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) -> str:
-    """Compile and link the library if any source is newer than it.  Returns its path."""
+    """Compile and link the library (and the extension module) where a source is newer.  Returns the library's path."""
     if not force and up_to_date():
+        build_native()
         return LIB_PATH
     nvcc = _nvcc()
     os.makedirs(OBJ_DIR, exist_ok=True)
@@ -77,6 +104,7 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) 
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError("link failed:\n%s\n%s" % (res.stdout, res.stderr))
+    build_native(force)
     return LIB_PATH
 
 

@@ -42,39 +42,25 @@ def _stream_ptr(index: int | None = None) -> int:
 class _Workspace:
     """Scratch shared by the layers of a process, one set per (device, stream): split-K partial
     sums and the zero-initialised arrival counters of the small-M kernel, plus the FP8
-    activation staging buffers.  Calls on one stream are ordered and may share a set; calls on
-    different streams may overlap on the GPU, so each stream gets its own.  Grown on demand."""
+    activation staging buffers.  The buffers live in the extension module, which the native calls
+    take them from; this is the general route's view of the set of the current stream."""
 
-    _by_device: dict[tuple[int, int], "_Workspace"] = {}
-
-    def __init__(self, device: torch.device):
-        self.device = device
-        self.ws = None
-        self.q = None
-        self.scale = None
-        self.host_scratch = None
+    def __init__(self, index: int):
+        self.index = index
 
     @classmethod
     def get(cls, device: torch.device) -> "_Workspace":
-        idx = device.index if device.index is not None else torch.cuda.current_device()
-        key = (idx, _stream_ptr(idx))
-        w = cls._by_device.get(key)
-        if w is None:
-            w = cls(torch.device("cuda", idx))
-            cls._by_device[key] = w
-        return w
+        return cls(device.index if device.index is not None else torch.cuda.current_device())
+
+    @property
+    def ws(self) -> torch.Tensor:
+        return self.scratch(0)
 
     def scratch(self, nbytes: int) -> torch.Tensor:
-        if self.ws is None or self.ws.numel() < nbytes:
-            self.ws = torch.zeros(max(nbytes, 1 << 20), dtype=torch.uint8, device=self.device)
-        return self.ws
+        return _lib.native().workspace(self.index, nbytes)
 
-    def act(self, m: int, k: int):
-        if self.q is None or self.q.numel() < m * k:
-            self.q = torch.empty(max(m * k, 1 << 16), dtype=torch.uint8, device=self.device)
-        if self.scale is None or self.scale.numel() < m:
-            self.scale = torch.empty(max(m, 1024), dtype=torch.float32, device=self.device)
-        return self.q, self.scale
+    def host_scratch(self, nbytes: int) -> torch.Tensor:
+        return _lib.native().host_scratch(self.index, nbytes)
 
 
 class PrecomputedPackedVectorCodebookLinear(torch.nn.Module):
@@ -160,8 +146,6 @@ class PrecomputedPackedVectorCodebookLinear(torch.nn.Module):
         if self.codebook.ndim != 2 or self.codebook.shape[1] != self.vector_dim:
             raise ValueError(f"codebook shape {tuple(self.codebook.shape)} does not match vector_dim")
         self.runtime_kernel_eligible = True
-        self._ws_bytes = {}
-        self._host_bytes = {}
         self._dev = device_obj                        # plain attribute: a buffer lookup per call costs a microsecond
         self._handle = None
         self._create_handle()
@@ -188,6 +172,7 @@ class PrecomputedPackedVectorCodebookLinear(torch.nn.Module):
         handle = ctypes.c_void_p()
         _lib.check(self._lib.sacq_layer_create(ctypes.byref(desc), ctypes.byref(handle)))
         self._handle = handle
+        self._native = _lib.native().Layer(handle.value, dev.index, self.out_features, self.in_features)
 
     def __del__(self):
         # runs during interpreter shutdown too: touch nothing but plain attributes
@@ -250,6 +235,9 @@ class PrecomputedPackedVectorCodebookLinear(torch.nn.Module):
         'int8_symmetric')``) x per-output-row int8 weights (decoded per call), exact int32
         accumulation, ``bf16(fma(sa, float(acc) * sw, bias))``.  q int8 ``[M, K]``, scale fp32 ``[M]``,
         weight_row_scale = ``self.weight_row_scale('int8_symmetric')`` -> bf16 ``[M, N]``."""
+        y = self._native.linear_w8a8(q, scale, weight_row_scale, out, True)
+        if y is not None:
+            return y
         if q.dim() != 2 or q.shape[1] != self.in_features:
             raise ValueError("q must be [M, in_features]")
         if not q.is_cuda or q.device != self.codebook.device:
@@ -277,6 +265,9 @@ class PrecomputedPackedVectorCodebookLinear(torch.nn.Module):
         e4m3 weights (re-quantized from the codebook weights, decoded per call), fp32 accumulation,
         ``bf16(fma(sa, acc * sw, bias))`` -- ``torch._scaled_mm(aq, wq.t(), sa, sw, bias)``.  q e4m3 (or its
         bytes) ``[M, K]``, scale fp32 ``[M]``, weight_row_scale = ``self.weight_row_scale('fp8_e4m3fn')``."""
+        y = self._native.linear_w8a8(q, scale, weight_row_scale, out, False)
+        if y is not None:
+            return y
         if q.dim() != 2 or q.shape[1] != self.in_features:
             raise ValueError("q must be [M, in_features]")
         if not q.is_cuda or q.device != self.codebook.device:
@@ -313,6 +304,9 @@ class PrecomputedPackedVectorCodebookLinear(torch.nn.Module):
         """GEMM on already-quantized activations: q e4m3 ``[M, K]``, scale fp32 ``[M]`` -> bf16 ``[M, N]``.
         ``residual`` (bf16 ``[M, N]``) is added in the GEMM epilogue: the bytes of
         ``linear_a8(q, scale) + residual``."""
+        y = self._native.linear_a8(q, scale, out, residual, False)
+        if y is not None:
+            return y
         if q.dim() != 2 or q.shape[1] != self.in_features:
             raise ValueError("q must be [M, in_features]")
         if not q.is_cuda or q.device != self.codebook.device:
@@ -346,6 +340,9 @@ class PrecomputedPackedVectorCodebookLinear(torch.nn.Module):
     def linear_a8i(self, q: torch.Tensor, scale: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
         """GEMM on INT8 per-token activations (``quantize_rows(x, 'int8_symmetric')``): q int8
         ``[M, K]``, scale fp32 ``[M]`` -> bf16 ``[M, N]``, with the exact (not re-quantized) weights."""
+        y = self._native.linear_a8(q, scale, out, None, True)
+        if y is not None:
+            return y
         if q.dim() != 2 or q.shape[1] != self.in_features:
             raise ValueError("q must be [M, in_features]")
         if not q.is_cuda or q.device != self.codebook.device:
@@ -367,6 +364,9 @@ class PrecomputedPackedVectorCodebookLinear(torch.nn.Module):
 
     def forward_int8(self, x: torch.Tensor) -> torch.Tensor:
         """``forward`` with INT8 instead of FP8 per-token activations."""
+        y = self._native.forward_int8(x)
+        if y is not None:
+            return y
         from .activation import quantize_rows
         if x.shape[-1] != self.in_features:
             raise ValueError("Linear shape mismatch")
@@ -379,6 +379,9 @@ class PrecomputedPackedVectorCodebookLinear(torch.nn.Module):
 
     def forward_residual(self, x: torch.Tensor, residual: torch.Tensor) -> torch.Tensor:
         """``self(x) + residual`` with the addition done in the GEMM epilogue (bf16 operands)."""
+        y = self._native.forward_residual(x, residual)
+        if y is not None:
+            return y
         from .activation import quantize_rows
         if x.shape[-1] != self.in_features:
             raise ValueError("Linear shape mismatch")
@@ -392,39 +395,23 @@ class PrecomputedPackedVectorCodebookLinear(torch.nn.Module):
         return y if x.dtype == torch.bfloat16 else y.to(x.dtype)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        y = self._native.forward(x)
+        return y if y is not None else self._forward_general(x)
+
+    def _forward_general(self, x: torch.Tensor) -> torch.Tensor:
+        """What the native call does not take: other dtypes, strided or empty inputs, and the errors."""
         if x.shape[-1] != self.in_features:
             raise ValueError("Linear shape mismatch")
         dev = self._dev
         if not x.is_cuda or x.device != dev:
             raise ValueError("Matching CUDA operands required")
-        a = x if x.dim() == 2 else x.reshape(-1, self.in_features)
-        if a.dtype != torch.bfloat16:
-            a = a.to(torch.bfloat16)
-        if a.stride(-1) != 1:
-            a = a.contiguous()
+        a = x.reshape(-1, self.in_features).to(torch.bfloat16).contiguous()
         m = a.shape[0]
-        y = torch.empty((m, self.out_features), dtype=torch.bfloat16, device=dev)
         if m > 0 and self.out_features > 0:
-            ws = _Workspace.get(dev)
-            need = self._ws_bytes.get(m)
-            if need is None:
-                need = self._ws_bytes[m] = int(self._lib.sacq_workspace_bytes(self._handle, m))
-            buf = ws.scratch(need)
-            q, s = ws.act(m, self.in_features)
-            if torch.cuda.current_device() == dev.index:
-                rc = self._lib.sacq_linear_bf16(
-                    self._handle, a.data_ptr(), a.stride(0), m, q.data_ptr(), s.data_ptr(), y.data_ptr(),
-                    y.stride(0), buf.data_ptr(), buf.numel(), _stream_ptr(dev.index))
-            else:
-                with torch.cuda.device(dev):
-                    rc = self._lib.sacq_linear_bf16(
-                        self._handle, a.data_ptr(), a.stride(0), m, q.data_ptr(), s.data_ptr(), y.data_ptr(),
-                        y.stride(0), buf.data_ptr(), buf.numel(), _stream_ptr(dev.index))
-            if rc != 0:
-                _lib.check(rc)
-        if x.dim() != 2:
-            y = y.reshape(*x.shape[:-1], self.out_features)
-        return y if x.dtype == torch.bfloat16 else y.to(x.dtype)
+            y = self._native.forward(a)
+        else:
+            y = torch.empty((m, self.out_features), dtype=torch.bfloat16, device=dev)
+        return y.reshape(*x.shape[:-1], self.out_features).to(x.dtype)
 
     def forward_host(self, x_host: torch.Tensor, out_host: torch.Tensor | None = None) -> torch.Tensor:
         """Forward for host-resident activations: ``x_host`` is a CPU bf16 ``[M, K]`` tensor
@@ -438,20 +425,11 @@ class PrecomputedPackedVectorCodebookLinear(torch.nn.Module):
         m = x_host.shape[0]
         if out_host is None:
             out_host = torch.empty((m, self.out_features), dtype=torch.bfloat16, pin_memory=x_host.is_pinned())
-        dev = self._dev
-        need = self._host_bytes.get(m)
-        if need is None:
-            need = self._host_bytes[m] = int(self._lib.sacq_host_forward_scratch_bytes(self._handle, m))
-        ws = _Workspace.get(dev)
-        if ws.host_scratch is None or ws.host_scratch.numel() < need:
-            ws.host_scratch = torch.zeros(max(need, 1 << 22), dtype=torch.uint8, device=dev)
-        buf = ws.host_scratch
-        if m > 0 and self.out_features > 0:
-            # the library switches to the layer's device itself; the stream is that device's current one
-            rc = self._lib.sacq_linear_bf16_host(self._handle, x_host.data_ptr(), m, out_host.data_ptr(),
-                                                 buf.data_ptr(), buf.numel(), _stream_ptr(dev.index))
-            if rc != 0:
-                _lib.check(rc)
+        if m > 0 and self.out_features > 0 and self._native.forward_host(x_host, out_host) is None:
+            # an out_host of another shape of the same elements, or not a plain tensor: its memory is what counts
+            buf = _Workspace.get(self._dev).host_scratch(int(self._lib.sacq_host_forward_scratch_bytes(self._handle, m)))
+            _lib.check(self._lib.sacq_linear_bf16_host(self._handle, x_host.data_ptr(), m, out_host.data_ptr(),
+                                                       buf.data_ptr(), buf.numel(), _stream_ptr(self._dev.index)))
         return out_host
 
     # ------------------------------------------------------------------ extras
@@ -464,8 +442,7 @@ class PrecomputedPackedVectorCodebookLinear(torch.nn.Module):
                 "large_tmem2": 10, "large_tmem3": 11, "large_tmem_grouped": 12, "large_tmem_grouped1": 13,
                 "large_tmem_grouped2": 14, "large_tmem_grouped3": 15}.get(which, which)
         _lib.check(self._lib.sacq_layer_set_kernel(self._handle, int(code)))
-        self._ws_bytes.clear()
-        self._host_bytes.clear()
+        self._native.forget_sizes()
 
     def kernel_for(self, m: int) -> str:
         k = self._lib.sacq_layer_kernel_for(self._handle, m)
@@ -497,6 +474,9 @@ def forward_shared(layers, x: torch.Tensor):
     identical to ``layer(x)``."""
     from .activation import quantize_rows
     layers = list(layers)
+    ys = _lib.native().forward_shared(layers, x)
+    if ys is not None:
+        return ys
     k = layers[0].in_features
     if any(l.in_features != k for l in layers):
         raise ValueError("layers that share an input must have the same in_features")
@@ -516,8 +496,10 @@ def linear_a8_multi(layers, q: torch.Tensor, scale: torch.Tensor):
     """GEMMs of several layers on one set of quantized activations (``sacq_linear_a8_multi``):
     layers of one geometry run as a single launch at small M.  Returns one bf16 ``[M, N_l]``
     tensor per layer, byte-identical to ``layer.linear_a8(q, scale)``."""
-    import ctypes
     layers = list(layers)
+    ys = _lib.native().linear_a8_multi(layers, q, scale)
+    if ys is not None:
+        return ys
     first = layers[0]
     if q.dim() != 2 or any(l.in_features != q.shape[1] for l in layers):
         raise ValueError("q must be [M, in_features] of every layer")
