@@ -45,7 +45,7 @@ def _sources():
 
 
 def _deps():
-    return _sources() + glob.glob(os.path.join(CSRC, "*.cuh")) + \
+    return _sources() + glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "host", "*.h")) + \
         glob.glob(os.path.join(HERE, "..", "include", "*.h")) + [os.path.abspath(__file__)]
 
 
@@ -58,7 +58,7 @@ def up_to_date() -> bool:
 
 def build_native(force: bool = False) -> str:
     """Compile the extension module if its source or the public header is newer.  Returns its path."""
-    deps = [NATIVE_SRC, os.path.abspath(__file__)] + glob.glob(os.path.join(HERE, "..", "include", "*.h"))
+    deps = [NATIVE_SRC, os.path.join(CSRC, "host", "internal.h"), os.path.abspath(__file__)] + glob.glob(os.path.join(HERE, "..", "include", "*.h"))
     if not force and os.path.exists(NATIVE_PATH) and \
             all(os.path.getmtime(p) <= os.path.getmtime(NATIVE_PATH) for p in deps):
         return NATIVE_PATH

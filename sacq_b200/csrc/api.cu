@@ -7,6 +7,8 @@
 #include <new>
 
 #include "common.cuh"
+#include "host/internal.h"
+#include "split_k.cuh"
 
 static_assert(sizeof(sacq_layer_desc) == 88, "sacq_layer_desc layout is part of the ABI");
 
@@ -62,17 +64,28 @@ int64_t small_m_slab_rows(const sacq_layer* L) {
 }
 
 // Rows from which the grouped tensor-core kernel beats the index-unpacking warp-MMA kernel
-// (which walks the weights once per 16-token chunk).  Measured crossovers: 33 rows on layers
-// wide enough to give the tensor-core grid a CTA for most SMs (N = 6144), 48-64 rows at
-// N = 2048, about 96 rows below that.
+// (which walks the weights once per 16-token chunk).
 int64_t grouped_min_m(const sacq_layer* L) {
-  if (L->d.out_features >= 32 * (int64_t)L->num_sms) return 33;
-  return L->d.out_features >= 2048 ? 48 : 96;
+  if (L->d.out_features >= 32 * (int64_t)L->num_sms) return 17;
+  return 48;
 }
 constexpr int64_t kTmemMinM = 1024;
 constexpr int64_t kTmemMinMBigCodebook = 128;
-// INT8 activations have no FP8 warp-MMA path, so the tensor-core kernel takes over earlier.
-constexpr int64_t kGroupedMinMInt8 = 48;
+
+// From how many tokens a split-K kernel, which walks the weights once, beats a small-M kernel, which walks them
+// once per 16-token chunk: from the second chunk on wide or deep layers, from the third on all but the smallest.
+bool split_wins(const sacq_layer* L, int64_t M, int64_t smallest) {
+  const int64_t work = L->d.in_features * L->d.out_features;
+  return (M > 16 && (L->d.out_features >= 4096 || work >= (8 << 20))) || (M > 32 && work > smallest);
+}
+
+// Layers with grouped scales below grouped_min_m(): the index-unpacking choice of the small-M path hands over to
+// the fp16 split-K kernel (quantizer + GEMM, d = 4, 10-bit, group 64: 2048x2048 12.8 / 9.9 us at 33 tokens,
+// 6144x2048 25.2 / 14.1 at 17, 4096x1024 16.2 / 10.9 at 33; 1024x1024 and 2048x1024 stay).
+bool small_m_hands_over(const sacq_layer* L, int64_t M) {
+  return (L->force_kernel == 0 || L->force_kernel == 1 || L->force_kernel == 6) && L->num_groups > 1 &&
+         M <= large_m_grouped_slab() && M < grouped_min_m(L) && split_wins(L, M, 2 << 20) && large_m_grouped_supported(L);
+}
 
 int pick_kernel(const sacq_layer* L, int64_t M) {
   if (L->force_kernel == 7) return large_m_grouped_supported(L) ? 3 : SACQ_ERR_UNSUPPORTED;
@@ -85,26 +98,18 @@ int pick_kernel(const sacq_layer* L, int64_t M) {
   // the expanded weights in tensor memory wins on every layer shape (its 128-row tiles need that
   // many tokens to fill the device).  The threshold does not depend on the layer's width, so
   // the row shards of a split layer run the kernel the whole layer would, and reproduce it
-  // bit for bit.  Layers whose codebook does not fit shared memory have no other tensor-core
+  // bit for bit (so does the split-K kernel, which sums in an order that depends on K alone).  Layers whose codebook does not fit shared memory have no other tensor-core
   // kernel and switch earlier.
   if (large_m_tmem_supported(L) && (M >= kTmemMinM || (M >= kTmemMinMBigCodebook && !large_m_supported(L)))) return 4;
-  // Above 64 rows the tcgen05 kernel always wins.
-  // Between 17 and 64 rows the small-M kernel walks its row tiles once per 16-token chunk
-  // while one tensor-core M tile covers them all; that pays off once the layer has enough
-  // output rows to give the tensor-core grid a CTA for most SMs (measured: N = 6144 yes,
-  // N <= 2048 no).
+  // Below, quantizer + GEMM of the small-M and the split-K kernel at 17 tokens: 1024x4096 10.9 / 6.8 us,
+  // 6144x2048 15.4 / 11.5, 2048x6144 15.5 / 8.9; at 33: 1024x1024 7.3 / 5.7, 2048x2048 9.2 / 8.8, 4096x1024
+  // 9.5 / 9.2, 2048x1024 even.
   if (large_m_supported(L)) {
-    if (M > 64) return 2;
-    if (M > 16 && L->d.out_features >= 32 * (int64_t)L->num_sms) return 2;   // 2048x6144 at M = 32: 14.1 us against 11.3 us
-    // ... and from 49 rows on deep layers: four 16-token chunks of K = 6144 cost the warp-MMA
-    // kernel 28.8 us, the tensor-core kernel 24.5 us (measured at N = 2048).
-    if (M > 48 && L->d.in_features >= 4096) return 2;
-    // ... and on layers of 2048 or more rows (2048 x 2048 at M = 64: 9.8 us against 8.9 us)
-    if (M > 48 && L->d.out_features >= 2048) return 2;
+    if (split_wins(L, M, 0)) return 2;
   } else if (large_m_tmem_grouped_supported(L) && M >= large_m_tmem_grouped_min_m(L)) {
     return 5;                                          // grouped scales, odd index widths: weights in tensor memory
   } else if (M >= grouped_min_m(L) && large_m_grouped_supported(L)) {
-    return 3;                                          // ... expanded weight tiles in shared memory
+    return 3;                                          // ... K split over clusters
   }
   return small_m_supported(L) ? 1 : SACQ_ERR_UNSUPPORTED;
 }
@@ -207,6 +212,7 @@ SACQ_API int sacq_layer_destroy(sacq_layer_t* L) {
   if (L == nullptr) return SACQ_OK;
   DeviceGuard guard(L->d.device);
   large_m_release(L);
+  split_k_release(L);
   if (L->cb_f16) cudaFree(L->cb_f16);
   if (L->cb_hilo) cudaFree(L->cb_hilo);
   if (L->d_status) cudaFree(L->d_status);
@@ -248,7 +254,7 @@ SACQ_API int sacq_quant_act_fp8(const void* x_bf16, int64_t x_pitch, int64_t M, 
   if (scale_out == nullptr || ((x_bf16 == nullptr || q_out == nullptr) && K > 0))
     return set_error(SACQ_ERR_INVALID_ARGUMENT, "null argument");
   if (K == 0) return set_error(SACQ_ERR_INVALID_ARGUMENT, "K must be positive");
-  return launch_quant_act_fp8(x_bf16, x_pitch, M, K, q_out, scale_out, static_cast<cudaStream_t>(stream));
+  return launch_quant_act(x_bf16, x_pitch, M, K, false, false, q_out, scale_out, static_cast<cudaStream_t>(stream));
 }
 
 SACQ_API int sacq_act_quant_fp8(int kind, const void* a_bf16, int64_t a_pitch, const void* b_bf16, int64_t b_pitch,
@@ -317,17 +323,19 @@ SACQ_API int sacq_layer_kernel_for(const sacq_layer_t* L, int64_t M) {
 
 SACQ_API int64_t sacq_workspace_bytes(const sacq_layer_t* L, int64_t M) {
   if (L == nullptr || M < 0) return 0;
-  if (pick_kernel(L, M) == 3) return kCounterBytes + large_m_grouped_workspace_bytes(L, M);
-  if (pick_kernel(L, M) == 5) return kCounterBytes + large_m_tmem_grouped_workspace_bytes(L, M);
+  const int k = pick_kernel(L, M);
+  if (k == 3 || (k == 1 && small_m_hands_over(L, M))) return kCounterBytes + large_m_grouped_workspace_bytes(L, M);
+  if (k == 5) return kCounterBytes + large_m_tmem_grouped_workspace_bytes(L, M);
   const int64_t slab = small_m_slab_rows(L);
   return small_m_workspace_bytes(L, M < slab ? M : slab);
 }
 
 namespace {
 // Common body of sacq_linear_a8 and sacq_linear_a8_residual.
+// form: what q holds (fp16 only where the chosen kernel takes it, see sacq_forward_call).
 int linear_a8_impl(const sacq_layer_t* L, const void* q, const float* scale, int64_t M, const void* residual,
                    int64_t ldr, void* y_out, int64_t ldy, void* workspace, int64_t workspace_bytes, void* stream,
-                   const BcastDst* bc = nullptr) {
+                   const BcastDst* bc = nullptr, ActForm form = kActE4M3) {
   if (int rc = check_layer(L)) return rc;
   if (M < 0) return set_error(SACQ_ERR_INVALID_ARGUMENT, "M=%lld is negative", (long long)M);
   if (M == 0 || L->d.out_features == 0) return SACQ_OK;
@@ -341,8 +349,9 @@ int linear_a8_impl(const sacq_layer_t* L, const void* q, const float* scale, int
                      (long long)L->d.out_features);
   DeviceGuard guard(L->d.device);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int k = pick_kernel(L, M);
+  int k = pick_kernel(L, M);
   if (k < 0) return set_error(k, "no kernel can run this layer geometry");
+  if (k == 1 && small_m_hands_over(L, M)) k = 3;
   if (k == 2) return launch_large_m(L, q, scale, M, y_out, ldy, s, residual, ldr, bc);
   if (k == 4)
     return launch_large_m_tmem(L, q, scale, M, y_out, ldy, s, residual, ldr, bc,
@@ -353,10 +362,10 @@ int linear_a8_impl(const sacq_layer_t* L, const void* q, const float* scale, int
                        (long long)sacq_workspace_bytes(L, M), (long long)workspace_bytes);
     if (k == 5)
       return launch_large_m_tmem_grouped(L, q, scale, M, y_out, ldy, static_cast<uint8_t*>(workspace) + kCounterBytes,
-                                         workspace_bytes - kCounterBytes, s, residual, ldr, 0, bc,
+                                         workspace_bytes - kCounterBytes, s, residual, ldr, form, bc,
                                          L->force_kernel >= 13 ? L->force_kernel - 12 : 0);
     return launch_large_m_grouped(L, q, scale, M, y_out, ldy, static_cast<uint8_t*>(workspace) + kCounterBytes,
-                                  workspace_bytes - kCounterBytes, s, residual, ldr, 0, bc);
+                                  workspace_bytes - kCounterBytes, s, residual, ldr, form, bc);
   }
   const int64_t slab = small_m_slab_rows(L);
   for (int64_t m0 = 0; m0 < M; m0 += slab) {
@@ -377,10 +386,17 @@ int linear_a8_impl(const sacq_layer_t* L, const void* q, const float* scale, int
 }  // namespace
 
 namespace {
-// INT8 activations run on the kernels that widen the activation bytes to fp16 themselves:
-// the grouped tensor-core kernel (tcgen05 kind::f16) from kGroupedMinM rows, below that the
-// fp16 warp-MMA kernel where the layer's geometry allows it, else the CUDA-core kernel.
-int int8_small_selector(const sacq_layer* L) { return small_m_int8_selector(L); }
+// INT8 activations run on the kernels that take them widened to fp16: the tensor-core kernels of grouped scales,
+// which run on any layer, or at small M the fp16 warp-MMA kernel where the layer's geometry allows it (8-, 12-
+// and 16-bit indices) and it is the faster one (quantizer + GEMM: 2048x2048 8.1 / 12.0 us at 16 tokens and
+// 13.9 / 12.7 at 40, 1536x1536 8.9 / 10.6 at 40), else the CUDA-core kernel.
+enum Int8Route { kInt8Small, kInt8Grouped, kInt8TmemGrouped };
+Int8Route int8_route(const sacq_layer* L, int64_t M) {
+  if (large_m_tmem_grouped_supported(L) && M >= large_m_tmem_grouped_min_m(L)) return kInt8TmemGrouped;
+  if (!large_m_grouped_supported(L)) return kInt8Small;
+  const int64_t warp_mma_wins = small_m_int8_selector(L) == 5 ? (L->d.out_features < 2048 ? 48 : 16) : 0;
+  return M > warp_mma_wins ? kInt8Grouped : kInt8Small;
+}
 }  // namespace
 
 SACQ_API int sacq_quant_act_int8(const void* x_bf16, int64_t x_pitch, int64_t M, int64_t K, void* q_out, float* scale_out,
@@ -393,19 +409,50 @@ SACQ_API int sacq_quant_act_int8(const void* x_bf16, int64_t x_pitch, int64_t M,
   if (scale_out == nullptr || ((x_bf16 == nullptr || q_out == nullptr) && K > 0))
     return set_error(SACQ_ERR_INVALID_ARGUMENT, "null argument");
   if (K == 0) return set_error(SACQ_ERR_INVALID_ARGUMENT, "K must be positive");
-  return launch_quant_act_int8(x_bf16, x_pitch, M, K, q_out, scale_out, static_cast<cudaStream_t>(stream));
+  return launch_quant_act(x_bf16, x_pitch, M, K, true, false, q_out, scale_out, static_cast<cudaStream_t>(stream));
 }
 
 SACQ_API int64_t sacq_workspace_bytes_int8(const sacq_layer_t* L, int64_t M) {
   if (L == nullptr || M < 0) return 0;
-  if (large_m_tmem_grouped_supported(L) && M >= large_m_tmem_grouped_min_m(L))
-    return kCounterBytes + large_m_tmem_grouped_workspace_bytes(L, M);
-  if (M >= kGroupedMinMInt8 && large_m_grouped_supported(L)) return kCounterBytes + large_m_grouped_workspace_bytes(L, M);
+  const Int8Route r = int8_route(L, M);
+  if (r == kInt8TmemGrouped) return kCounterBytes + large_m_tmem_grouped_workspace_bytes(L, M);
+  if (r == kInt8Grouped) return kCounterBytes + large_m_grouped_workspace_bytes(L, M);
   sacq_layer view = *L;
-  view.force_kernel = int8_small_selector(L);
+  view.force_kernel = small_m_int8_selector(L);
   const int64_t slab = small_m_slab_rows(L);
   return small_m_workspace_bytes(&view, M < slab ? M : slab);
 }
+
+namespace {
+int linear_a8i_impl(const sacq_layer_t* L, const void* q, const float* scale, int64_t M, void* y_out, int64_t ldy,
+                    void* workspace, int64_t workspace_bytes, void* stream, ActForm form) {
+  DeviceGuard guard(L->d.device);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const Int8Route r = int8_route(L, M);
+  if (r != kInt8Small) {
+    if (workspace == nullptr || workspace_bytes < kCounterBytes)
+      return set_error(SACQ_ERR_WORKSPACE, "workspace of %lld bytes needed, %lld given",
+                       (long long)sacq_workspace_bytes_int8(L, M), (long long)workspace_bytes);
+    return (r == kInt8TmemGrouped)
+               ? launch_large_m_tmem_grouped(L, q, scale, M, y_out, ldy, static_cast<uint8_t*>(workspace) + kCounterBytes,
+                                             workspace_bytes - kCounterBytes, s, nullptr, 0, form)
+               : launch_large_m_grouped(L, q, scale, M, y_out, ldy, static_cast<uint8_t*>(workspace) + kCounterBytes,
+                                        workspace_bytes - kCounterBytes, s, nullptr, 0, form);
+  }
+  if (!small_m_supported(L)) return set_error(SACQ_ERR_UNSUPPORTED, "no kernel can run this layer geometry");
+  sacq_layer view = *L;
+  view.force_kernel = small_m_int8_selector(L);
+  const int64_t slab = small_m_slab_rows(L);
+  for (int64_t m0 = 0; m0 < M; m0 += slab) {
+    const int64_t rows = (M - m0) < slab ? (M - m0) : slab;
+    const int rc = launch_small_m(&view, static_cast<const uint8_t*>(q) + m0 * L->d.in_features, scale + m0, rows,
+                                  static_cast<uint16_t*>(y_out) + m0 * ldy, ldy, workspace, workspace_bytes, s, nullptr,
+                                  0, 1);
+    if (rc != SACQ_OK) return rc;
+  }
+  return SACQ_OK;
+}
+}  // namespace
 
 SACQ_API int sacq_linear_a8i(const sacq_layer_t* L, const void* q_int8, const float* scale, int64_t M, void* y_out,
                              int64_t ldy, void* workspace, int64_t workspace_bytes, void* stream) {
@@ -417,34 +464,7 @@ SACQ_API int sacq_linear_a8i(const sacq_layer_t* L, const void* q_int8, const fl
   if (ldy < L->d.out_features)
     return set_error(SACQ_ERR_INVALID_ARGUMENT, "ldy=%lld smaller than out_features=%lld", (long long)ldy,
                      (long long)L->d.out_features);
-  DeviceGuard guard(L->d.device);
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (large_m_tmem_grouped_supported(L) && M >= large_m_tmem_grouped_min_m(L)) {
-    if (workspace == nullptr || workspace_bytes < kCounterBytes)
-      return set_error(SACQ_ERR_WORKSPACE, "workspace of %lld bytes needed, %lld given",
-                       (long long)sacq_workspace_bytes_int8(L, M), (long long)workspace_bytes);
-    return launch_large_m_tmem_grouped(L, q_int8, scale, M, y_out, ldy, static_cast<uint8_t*>(workspace) + kCounterBytes,
-                                       workspace_bytes - kCounterBytes, s, nullptr, 0, 1);
-  }
-  if (M >= kGroupedMinMInt8 && large_m_grouped_supported(L)) {
-    if (workspace == nullptr || workspace_bytes < kCounterBytes)
-      return set_error(SACQ_ERR_WORKSPACE, "workspace of %lld bytes needed, %lld given",
-                       (long long)sacq_workspace_bytes_int8(L, M), (long long)workspace_bytes);
-    return launch_large_m_grouped(L, q_int8, scale, M, y_out, ldy, static_cast<uint8_t*>(workspace) + kCounterBytes,
-                                  workspace_bytes - kCounterBytes, s, nullptr, 0, 1);
-  }
-  if (!small_m_supported(L)) return set_error(SACQ_ERR_UNSUPPORTED, "no kernel can run this layer geometry");
-  sacq_layer view = *L;
-  view.force_kernel = int8_small_selector(L);
-  const int64_t slab = small_m_slab_rows(L);
-  for (int64_t m0 = 0; m0 < M; m0 += slab) {
-    const int64_t rows = (M - m0) < slab ? (M - m0) : slab;
-    const int rc = launch_small_m(&view, static_cast<const uint8_t*>(q_int8) + m0 * L->d.in_features, scale + m0, rows,
-                                  static_cast<uint16_t*>(y_out) + m0 * ldy, ldy, workspace, workspace_bytes, s, nullptr,
-                                  0, 1);
-    if (rc != SACQ_OK) return rc;
-  }
-  return SACQ_OK;
+  return linear_a8i_impl(L, q_int8, scale, M, y_out, ldy, workspace, workspace_bytes, stream, kActInt8);
 }
 
 SACQ_API int sacq_weight_row_scale_int8(const sacq_layer_t* L, float* sw_out, void* stream) {
@@ -468,6 +488,21 @@ SACQ_API int64_t sacq_workspace_bytes_w8a8(const sacq_layer_t* L, int64_t M) {
   return kCounterBytes + ((L->d.out_features * L->d.in_features + 255) & ~(int64_t)255);
 }
 
+namespace {
+// Up to a few hundred tokens the recipes run as one kernel whose expanders make the weight bytes on the way to the
+// tensor cores; above, making them once for all token tiles and a dense GEMM is faster (quantizer included,
+// 2048x6144 at d = 4: 33 / 34 us at 512 tokens, 44 / 36 at 1,000; 6144x2048 50 / 52 and 2048x2048 24 / 28 at 1,000).
+bool recipe_in_one(const sacq_layer* L, const void* q, const float* act_scale, const float* w_scale, int64_t M, void* y,
+                   int64_t ldy, SplitMode mode, cudaStream_t s, int* rc) {
+  SplitChoice c;
+  if (M > (L->d.out_features >= 4096 ? 512 : 1024) || reinterpret_cast<uintptr_t>(q) % 16 != 0 || reinterpret_cast<uintptr_t>(L->d.codebook) % 16 != 0 ||
+      (mode == kSplitInt8 && L->d.in_features * 127 * 127 > 2147483647LL) || !split_k_choose(L, M, mode, &c))
+    return false;
+  *rc = launch_split_k(&L, 1, q, act_scale, M, &y, &ldy, mode, c, s, nullptr, 0, nullptr, w_scale);
+  return true;
+}
+}  // namespace
+
 SACQ_API int sacq_linear_w8a8_int8(const sacq_layer_t* L, const void* q_int8, const float* act_scale, const float* w_scale,
                                    int64_t M, void* y_out, int64_t ldy, void* workspace, int64_t workspace_bytes,
                                    void* stream) {
@@ -490,8 +525,10 @@ SACQ_API int sacq_linear_w8a8_int8(const sacq_layer_t* L, const void* q_int8, co
   DeviceGuard guard(L->d.device);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   // per call, as the reference does: packed stream -> int8 weight rows, then the dense integer GEMM
+  int rc = SACQ_OK;
+  if (recipe_in_one(L, q_int8, act_scale, w_scale, M, y_out, ldy, kSplitInt8, s, &rc)) return rc;
   void* wq = static_cast<uint8_t*>(workspace) + kCounterBytes;
-  if (int rc = launch_decode_weight_int8(L, w_scale, wq, s)) return rc;
+  if ((rc = launch_decode_weight_int8(L, w_scale, wq, s)) != SACQ_OK) return rc;
   return launch_dense_i8(L, q_int8, act_scale, wq, w_scale, M, y_out, ldy, s);
 }
 
@@ -517,8 +554,10 @@ SACQ_API int sacq_linear_w8a8_fp8(const sacq_layer_t* L, const void* q_e4m3, con
   DeviceGuard guard(L->d.device);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   // per call, as the reference does: packed stream -> e4m3 weight rows, then the dense FP8 GEMM
+  int rc = SACQ_OK;
+  if (recipe_in_one(L, q_e4m3, act_scale, w_scale, M, y_out, ldy, kSplitFp8, s, &rc)) return rc;
   void* wq = static_cast<uint8_t*>(workspace) + kCounterBytes;
-  if (int rc = launch_decode_weight_fp8(L, w_scale, wq, s)) return rc;
+  if ((rc = launch_decode_weight_fp8(L, w_scale, wq, s)) != SACQ_OK) return rc;
   return launch_dense_i8(L, q_e4m3, act_scale, wq, w_scale, M, y_out, ldy, s, true);
 }
 
@@ -616,7 +655,8 @@ SACQ_API int sacq_linear_a8_multi(const sacq_layer_t* const* layers, int num_lay
   {
     // one launch when every layer would use the staged small-M kernel on a common geometry
     bool small = num_layers >= 2;
-    for (int l = 0; l < num_layers && small; ++l) small = pick_kernel(layers[l], M) == 1;
+    for (int l = 0; l < num_layers && small; ++l)
+      small = pick_kernel(layers[l], M) == 1 && !small_m_hands_over(layers[l], M);
     if (small) {
       DeviceGuard guard(layers[0]->d.device);
       const int rc = launch_small_m_multi(layers, num_layers, q, scale, M, y_outs, ldys,
@@ -632,6 +672,17 @@ SACQ_API int sacq_linear_a8_multi(const sacq_layer_t* const* layers, int num_lay
                                           static_cast<cudaStream_t>(stream));
       if (rc != SACQ_ERR_UNSUPPORTED) return rc;
     }
+    // ... or its fp16 form for grouped scales
+    bool grouped = num_layers >= 2 && workspace != nullptr && workspace_bytes > kCounterBytes;
+    for (int l = 0; l < num_layers && grouped; ++l)
+      grouped = pick_kernel(layers[l], M) == 3 || (pick_kernel(layers[l], M) == 1 && small_m_hands_over(layers[l], M));
+    if (grouped) {
+      DeviceGuard guard(layers[0]->d.device);
+      const int rc = launch_large_m_grouped_multi(layers, num_layers, q, scale, M, y_outs, ldys,
+                                                  static_cast<uint8_t*>(workspace) + kCounterBytes,
+                                                  workspace_bytes - kCounterBytes, static_cast<cudaStream_t>(stream));
+      if (rc != SACQ_ERR_UNSUPPORTED) return rc;
+    }
   }
   for (int l = 0; l < num_layers; ++l) {
     const int rc = sacq_linear_a8(layers[l], q, scale, M, y_outs[l], ldys[l], workspace, workspace_bytes, stream);
@@ -640,14 +691,52 @@ SACQ_API int sacq_linear_a8_multi(const sacq_layer_t* const* layers, int num_lay
   return SACQ_OK;
 }
 
+// Quantizer + GEMM of one call.  Where the GEMM takes fp16 activations, the quantizer writes them as fp16 into
+// the workspace itself: one launch less than quantizing to bytes and widening those (2 us of host time and as
+// much of the GPU's at small sizes), the same values.
+int sacq_forward_call(const sacq_layer_t* L, const void* x_bf16, int64_t x_pitch, int64_t M, int int8, const void* residual,
+                      int64_t ldr, void* q_scratch, float* scale_scratch, void* y_out, int64_t ldy, void* workspace,
+                      int64_t workspace_bytes, void* stream) {
+  if (int rc = check_layer(L)) return rc;
+  if (M == 0) return SACQ_OK;
+  const int64_t K = L->d.in_features;
+  int64_t slab = 0;                                   // tokens up to which the GEMM takes fp16 activations in one piece
+  int64_t need = 0;
+  if (M > 0 && L->d.out_features > 0) {
+    const Int8Route r = int8 ? int8_route(L, M) : kInt8Small;
+    const int k = int8 ? 0 : pick_kernel(L, M);
+    if (r == kInt8TmemGrouped || k == 5) {
+      slab = large_m_tmem_grouped_slab();
+      need = large_m_tmem_grouped_workspace_bytes(L, M);
+    } else if (r == kInt8Grouped || k == 3 || (k == 1 && small_m_hands_over(L, M))) {
+      slab = large_m_grouped_slab();
+      need = large_m_grouped_workspace_bytes(L, M);
+    }
+  }
+  const bool wide = M <= slab && K % 8 == 0 && x_bf16 != nullptr && reinterpret_cast<uintptr_t>(x_bf16) % 16 == 0 &&
+                    x_pitch % 8 == 0 && x_pitch >= K && workspace != nullptr && scale_scratch != nullptr && y_out != nullptr &&
+                    reinterpret_cast<uintptr_t>(workspace) % 256 == 0 && workspace_bytes >= kCounterBytes + need;
+  if (wide) {
+    DeviceGuard guard(L->d.device);
+    void* a16 = static_cast<uint8_t*>(workspace) + kCounterBytes;
+    if (int rc = launch_quant_act(x_bf16, x_pitch, M, K, int8 != 0, true, a16, scale_scratch, static_cast<cudaStream_t>(stream)))
+      return rc;
+    if (int8) return linear_a8i_impl(L, a16, scale_scratch, M, y_out, ldy, workspace, workspace_bytes, stream, kActHalf);
+    return linear_a8_impl(L, a16, scale_scratch, M, residual, ldr, y_out, ldy, workspace, workspace_bytes, stream, nullptr,
+                          kActHalf);
+  }
+  const int rc = int8 ? sacq_quant_act_int8(x_bf16, x_pitch, M, K, q_scratch, scale_scratch, stream)
+                      : sacq_quant_act_fp8(x_bf16, x_pitch, M, K, q_scratch, scale_scratch, stream);
+  if (rc != SACQ_OK) return rc;
+  if (int8) return sacq_linear_a8i(L, q_scratch, scale_scratch, M, y_out, ldy, workspace, workspace_bytes, stream);
+  return linear_a8_impl(L, q_scratch, scale_scratch, M, residual, ldr, y_out, ldy, workspace, workspace_bytes, stream);
+}
+
 SACQ_API int sacq_linear_bf16(const sacq_layer_t* L, const void* x_bf16, int64_t x_pitch, int64_t M, void* q_scratch,
                      float* scale_scratch, void* y_out, int64_t ldy, void* workspace, int64_t workspace_bytes,
                      void* stream) {
-  if (int rc = check_layer(L)) return rc;
-  if (M == 0) return SACQ_OK;
-  int rc = sacq_quant_act_fp8(x_bf16, x_pitch, M, L->d.in_features, q_scratch, scale_scratch, stream);
-  if (rc != SACQ_OK) return rc;
-  return sacq_linear_a8(L, q_scratch, scale_scratch, M, y_out, ldy, workspace, workspace_bytes, stream);
+  return sacq_forward_call(L, x_bf16, x_pitch, M, 0, nullptr, 0, q_scratch, scale_scratch, y_out, ldy, workspace,
+                           workspace_bytes, stream);
 }
 
 // Layout of the device scratch of sacq_linear_bf16_host: workspace first (its counter

@@ -19,6 +19,7 @@ constexpr int kNumSMsB200 = 148;
 // ----------------------------------------------------------------------------
 
 struct LargeMPlan;  // built lazily by the large-M kernel's host code
+struct SplitPlan;   // ... and by the split-K kernel's
 
 }  // namespace sacq
 
@@ -40,6 +41,7 @@ struct sacq_layer {
   int* d_status;             // device status word, 0 = ok
   int64_t resident_bytes;
   sacq::LargeMPlan* large_plan;
+  sacq::SplitPlan* split_plan;
 };
 
 namespace sacq {
@@ -65,8 +67,10 @@ int launch_dequant_bf16(const sacq_layer* L, void* w_out, cudaStream_t s);
 int launch_weight_row_scale(const sacq_layer* L, float* sw, cudaStream_t s, float limit = kE4M3Max);
 int launch_decode_weight_fp8(const sacq_layer* L, const float* sw, void* wq, cudaStream_t s);
 int launch_decode_weight_int8(const sacq_layer* L, const float* sw, void* wq, cudaStream_t s);
-int launch_quant_act_fp8(const void* x, int64_t pitch, int64_t M, int64_t K, void* q, float* scale, cudaStream_t s);
-int launch_quant_act_int8(const void* x, int64_t pitch, int64_t M, int64_t K, void* q, float* scale, cudaStream_t s);
+// Per-token quantizer, e4m3 or int8.  wide: the encoded values go out as fp16 [M, K] (the operand of the fp16
+// tensor-core kernels) instead of bytes.
+int launch_quant_act(const void* x, int64_t pitch, int64_t M, int64_t K, bool int8, bool wide, void* q, float* scale,
+                     cudaStream_t s);
 int launch_act_quant_fp8(int kind, const void* a, int64_t a_pitch, const void* b, int64_t b_pitch, const void* c,
                          int64_t M, int64_t K, void* q, float* scale, cudaStream_t s);
 int launch_layernorm_quant_fp8(const void* x, int64_t pitch, const void* gamma, const void* beta, float eps,
@@ -115,19 +119,28 @@ bool dense_i8_supported(const sacq_layer* L);
 int launch_dense_i8(const sacq_layer* L, const void* q, const float* act_scale, const void* wq, const float* w_scale,
                     int64_t M, void* y, int64_t ldy, cudaStream_t s, bool fp8 = false);
 
+// What the activations of a fp16 tensor-core kernel come as: bytes to be widened, or fp16 [M, K] already
+// (M at most one slab).
+enum ActForm { kActE4M3 = 0, kActInt8 = 1, kActHalf = 2 };
+
 bool large_m_grouped_supported(const sacq_layer* L);
 int64_t large_m_grouped_workspace_bytes(const sacq_layer* L, int64_t M);
 int launch_large_m_grouped(const sacq_layer* L, const void* q, const float* scale, int64_t M, void* y, int64_t ldy,
                            void* ws, int64_t ws_bytes, cudaStream_t s, const void* residual = nullptr,
-                           int64_t ldr = 0, int act_int8 = 0, const BcastDst* bc = nullptr);
+                           int64_t ldr = 0, ActForm form = kActE4M3, const BcastDst* bc = nullptr);
+int64_t large_m_grouped_slab(void);
+
+int launch_large_m_grouped_multi(const sacq_layer* const* layers, int n, const void* q, const float* scale, int64_t M,
+                                 void* const* ys, const int64_t* ldys, void* ws, int64_t ws_bytes, cudaStream_t s);
 
 // Grouped-scale tensor-core kernel with the weights in tensor memory (linear_large_m_tmem_grouped.cu).
 bool large_m_tmem_grouped_supported(const sacq_layer* L);
 int64_t large_m_tmem_grouped_workspace_bytes(const sacq_layer* L, int64_t M);
 int64_t large_m_tmem_grouped_min_m(const sacq_layer* L);
+int64_t large_m_tmem_grouped_slab(void);
 int launch_large_m_tmem_grouped(const sacq_layer* L, const void* q, const float* scale, int64_t M, void* y, int64_t ldy,
                                 void* ws, int64_t ws_bytes, cudaStream_t s, const void* residual = nullptr,
-                                int64_t ldr = 0, int act_int8 = 0, const BcastDst* bc = nullptr, int nt_force = 0);
+                                int64_t ldr = 0, ActForm form = kActE4M3, const BcastDst* bc = nullptr, int nt_force = 0);
 
 // ----------------------------------------------------------------------------
 // device side

@@ -26,7 +26,7 @@
 #include <unordered_map>
 #include <utility>
 
-#include "../../../include/sacq_b200.h"
+#include "internal.h"
 
 namespace {
 
@@ -210,10 +210,8 @@ PyObject* layer_forward_residual(LayerObject* L, PyObject* const* a, Py_ssize_t 
   at::Tensor& ws = scratch(w, need_bytes(L, r.m, kNeedA8), L->dev);
   act_buffers(w, r.m, L->k, L->dev);
   at::Tensor y = result_like(*x, r.m, L->n, L->dev);
-  int rc = sacq_quant_act_fp8(r.ptr, r.pitch, r.m, L->k, w.q.data_ptr(), (float*)w.scale.data_ptr(), at_.stream);
-  if (rc == 0)
-    rc = sacq_linear_a8_residual(L->handle, w.q.data_ptr(), (const float*)w.scale.data_ptr(), r.m, rr.ptr, rr.pitch,
-                                 y.data_ptr(), L->n, ws.data_ptr(), ws.numel(), at_.stream);
+  const int rc = sacq_forward_call(L->handle, r.ptr, r.pitch, r.m, 0, rr.ptr, rr.pitch, w.q.data_ptr(),
+                                   (float*)w.scale.data_ptr(), y.data_ptr(), L->n, ws.data_ptr(), ws.numel(), at_.stream);
   return rc == 0 ? THPVariable_Wrap(std::move(y)) : raise_status(rc);
   NATIVE_CATCH
 }
@@ -228,10 +226,8 @@ PyObject* layer_forward_int8(LayerObject* L, PyObject* x_obj) {
   at::Tensor& ws = scratch(w, need_bytes(L, r.m, kNeedInt8), L->dev);
   act_buffers(w, r.m, L->k, L->dev);
   at::Tensor y = result_like(*x, r.m, L->n, L->dev);
-  int rc = sacq_quant_act_int8(r.ptr, r.pitch, r.m, L->k, w.q.data_ptr(), (float*)w.scale.data_ptr(), at_.stream);
-  if (rc == 0)
-    rc = sacq_linear_a8i(L->handle, w.q.data_ptr(), (const float*)w.scale.data_ptr(), r.m, y.data_ptr(), L->n,
-                         ws.data_ptr(), ws.numel(), at_.stream);
+  const int rc = sacq_forward_call(L->handle, r.ptr, r.pitch, r.m, 1, nullptr, 0, w.q.data_ptr(), (float*)w.scale.data_ptr(),
+                                   y.data_ptr(), L->n, ws.data_ptr(), ws.numel(), at_.stream);
   return rc == 0 ? THPVariable_Wrap(std::move(y)) : raise_status(rc);
   NATIVE_CATCH
 }

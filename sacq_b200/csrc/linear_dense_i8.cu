@@ -16,9 +16,7 @@
 //   warp 0 (one lane) : TMA producer: per 128-byte K block two 128-token activation tiles and one
 //                       256-row weight tile, SWIZZLE_128B, no multicast; 3 stages of 64 KB;
 //   warp 1 (one lane) : tcgen05.mma kind::i8, M128 x N256 x K32, into TWO int32 accumulators (one
-//                       per token sub-tile, 2 x 256 = all 512 TMEM columns) that alternate
-//                       instruction by instruction: consecutive MMAs into one accumulator wait
-//                       for each other (about 100 ns per instruction against 65 ns of tensor work);
+//                       per token sub-tile, 2 x 256 = all 512 TMEM columns) that share every weight tile;
 //   warps 2..17       : epilogue: TMEM lane quarter x token sub-tile x column half each.
 // A last token tile of at most 128 tokens loads and multiplies one sub-tile only.
 // Every mbarrier wait is bounded (status word + CTA-wide abort flag), as in the other
@@ -59,11 +57,6 @@ struct DenseParams {
   int M, N, K;
 };
 
-// kind::i8 instruction descriptor: int32 accumulate, A = B = signed 8-bit, both K-major.
-__host__ __device__ constexpr uint32_t make_idesc_i8(int bn) {
-  return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
-}
-
 __device__ __forceinline__ void umma_i8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                         uint32_t accumulate) {
   asm volatile(
@@ -94,7 +87,7 @@ dense_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + kMiscOff);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + kMiscOff + 8);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = (int)warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int n0 = blockIdx.x * kDBN, m0 = blockIdx.y * (kDSub * kBM);
   const int num_kb = (p.K + kDBK - 1) / kDBK;
   const int subs = (p.M - m0 > kBM) ? 2 : 1;        // token sub-tiles of this CTA that hold tokens
@@ -114,47 +107,52 @@ dense_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
 
   if (warp == 0) {
-    if (lane == 0) {
-      for (int kb = 0; kb < num_kb; ++kb) {
-        const int st = kb % kDStages;
-        if (!mbar_wait(bar(EMPTY + st), ((kb / kDStages) & 1) ^ 1, abort_flag, p.status)) break;
+    int st = 0;
+    uint32_t free_parity = 1;
+    for (int kb = 0; kb < num_kb; ++kb) {
+      if (!mbar_wait_warp(bar(EMPTY + st), free_parity, abort_flag, p.status)) break;
+      const uint32_t dst = base + st * kStageBytes;
+      if (elect_one()) {
         mbar_arrive_expect_tx(bar(FULL + st), (uint32_t)(subs * kDTileA + kDTileB));
-        const uint32_t dst = base + st * kStageBytes;
-        for (int t = 0; t < subs; ++t) tma_load_2d(dst + t * kDTileA, &tmap_a, kb * kDBK, m0 + t * kBM, bar(FULL + st));
+        tma_load_2d(dst, &tmap_a, kb * kDBK, m0, bar(FULL + st));
+        if (subs == 2) tma_load_2d(dst + kDTileA, &tmap_a, kb * kDBK, m0 + kBM, bar(FULL + st));
         tma_load_2d(dst + kDSub * kDTileA, &tmap_b, kb * kDBK, n0, bar(FULL + st));
       }
+      if (++st == kDStages) { st = 0; free_parity ^= 1; }
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t kIdesc = FP8 ? make_idesc(kDBN) : make_idesc_i8(kDBN);
-      bool ok = true;
-      for (int kb = 0; kb < num_kb && ok; ++kb) {
-        const int st = kb % kDStages;
-        ok = mbar_wait(bar(FULL + st), (kb / kDStages) & 1, abort_flag, p.status);
-        if (!ok) break;
-        tc_fence_after();
-        const uint64_t a0_desc = make_smem_desc(base + st * kStageBytes);
-        const uint64_t a1_desc = make_smem_desc(base + st * kStageBytes + kDTileA);
-        const uint64_t b_desc = make_smem_desc(base + st * kStageBytes + kDSub * kDTileA);
+    constexpr uint32_t kIdesc = FP8 ? make_idesc(kDBN) : make_idesc_i8(kDBN);
+    bool ok = true;
+    int st = 0;
+    uint32_t full_parity = 0;
+    for (int kb = 0; kb < num_kb; ++kb) {
+      ok = mbar_wait_warp(bar(FULL + st), full_parity, abort_flag, p.status);
+      if (!ok) break;
+      tc_fence_after();
+      const uint64_t a0_desc = make_smem_desc(base + st * kStageBytes);
+      const uint64_t a1_desc = make_smem_desc(base + st * kStageBytes + kDTileA);
+      const uint64_t b_desc = make_smem_desc(base + st * kStageBytes + kDSub * kDTileA);
 #pragma unroll
-        for (int ks = 0; ks < kDBK / 32; ++ks) {
-          const uint64_t adv = (uint64_t)((ks * 32) >> 4);
-          if constexpr (FP8) {
-            umma_f8(tmem_base, a0_desc + adv, b_desc + adv, kIdesc, (kb | ks) != 0);
-            if (subs == 2) umma_f8(tmem_base + kDBN, a1_desc + adv, b_desc + adv, kIdesc, (kb | ks) != 0);
-          } else {
-            umma_i8(tmem_base, a0_desc + adv, b_desc + adv, kIdesc, (kb | ks) != 0);
-            if (subs == 2) umma_i8(tmem_base + kDBN, a1_desc + adv, b_desc + adv, kIdesc, (kb | ks) != 0);
-          }
+      for (int ks = 0; ks < kDBK / 32; ++ks) {
+        const uint64_t adv = (uint64_t)((ks * 32) >> 4);
+        const uint32_t acc = (kb | ks) != 0;
+        if (elect_one()) {
+          if constexpr (FP8) umma_f8(tmem_base, a0_desc + adv, b_desc + adv, kIdesc, acc);
+          else umma_i8(tmem_base, a0_desc + adv, b_desc + adv, kIdesc, acc);
         }
-        umma_commit(bar(EMPTY + st));
+        if (subs == 2 && elect_one()) {
+          if constexpr (FP8) umma_f8(tmem_base + kDBN, a1_desc + adv, b_desc + adv, kIdesc, acc);
+          else umma_i8(tmem_base + kDBN, a1_desc + adv, b_desc + adv, kIdesc, acc);
+        }
       }
-      if (ok) umma_commit(bar(ACC_FULL));
+      if (elect_one()) umma_commit(bar(EMPTY + st));
+      if (++st == kDStages) { st = 0; full_parity ^= 1; }
     }
+    if (ok && elect_one()) umma_commit(bar(ACC_FULL));
     __syncwarp();
   } else {
     const int et = threadIdx.x - 64;                  // 0..511

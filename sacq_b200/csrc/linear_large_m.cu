@@ -1,492 +1,24 @@
-// Large-M quantized linear on the 5th-generation tensor cores (sm_100a):
-//   y[m,n] = bf16( s[m] * (sum_k q[m,k] * cb[idx[n,k/d], k%d]) * scale[n] + bias[n] )
-//
-// One CTA computes a 128-token x 128-row output tile.
-//   * warp 0 (one lane)  : TMA producer.  cp.async.bulk.tensor loads the 128 x 128-byte
-//     e4m3 activation tile of every K block (SWIZZLE_128B) and, every second K block,
-//     the tile of packed index bytes for the CTA's 128 weight rows.  No multicast.
-//   * warps 2..9         : expanders.  They read the index bytes from shared memory,
-//     gather each codeword's FP8 high and low halves (16 bytes for d = 8) from the
-//     shared-memory codebook and write them into two K-major, 128B-swizzled B tiles --
-//     the canonical UMMA layout, produced by threads instead of by TMA -- then
-//     fence.proxy.async and arrive on the stage's mbarrier.
-//   * warp 1 (one lane)  : issues tcgen05.mma kind::f8f6f4; with one token sub-tile ONE per K step with the two B
-//     tiles as a single operand of N = 2*BN rows (M128 N256 K32 for BN = 128): A x B_hi
-//     lands in accumulator columns [0, BN), A x B_lo in [BN, 2*BN) of TMEM; tcgen05.commit
-//     releases the stage.
-//   * warps 2..9 again   : epilogue.  tcgen05.ld both accumulator halves, add them, apply
-//     fma(s[m], acc * scale[n], bias[n]) in the reference's order
-//     (int8_ordered_epilogue_20261028_r1.py:11-22) and store bf16.
-//
-// Why two FP8 MMAs per step: kind::f8f6f4 needs both operands in <= 8 bits, but a single
-// e4m3 rounding of the bf16 codewords misses the 1e-2 GEMM tolerance (2.7 % relative
-// error); hi = e4m3(c * 2^e), lo = e4m3(c * 2^e - hi) reproduces every bf16 codeword
-// whose magnitude is within 2^-10 of the largest exactly, at the cost of executing twice
-// the algorithmic flops.
-//
-// Stands in for the reference's decode-to-8-bit + 8-bit GEMM pair
-// (a8_joint_pair_r1.py:38-127,374 and perrow_a8_candidate_r3.py:56-69) and its
-// decode-in-mainloop GEMM (codebook_cutlass_kernel.cu:234-583).
-//
-// Every mbarrier wait is bounded: on expiry the waiting thread writes a code to the
-// layer's status word and raises a CTA-wide abort flag that all other waits poll, so the
-// CTA always reaches the common exit, frees its TMEM and returns.
+// Tensor-core path of per-channel layers from a few dozen tokens up to the batched sizes: argument checks
+// and launch of the split-K kernel (linear_split_k.cu), the tensor-map helpers every tensor-core kernel
+// uses, and a layer's index-tile map.
 #include <cuda.h>
-#include <math.h>
 
 #include <mutex>
 
 #include "common.cuh"
+#include "split_k.cuh"
 #include "umma.cuh"
 
 namespace sacq {
 
-namespace {
-
-using namespace umma;
-
-constexpr int kMaxBN = 128;       // weight rows per tile (accumulator columns): BN in {32, 64, 128}
-constexpr int kBK = 128;          // e4m3 elements (= bytes) per K block: one 128B swizzle row
-constexpr int kMaxStages = 3;     // 3 stages with one 128-row M sub-tile, 2 with two
-constexpr int kTileBytes = kBM * kBK;            // 16 KB: one operand tile
-
-template <int BITS>
-__device__ __forceinline__ uint32_t field8(const uint32_t (&w)[BITS / 4], int j) {
-  const int bit = j * BITS;
-  const int word = bit >> 5;
-  const int off = bit & 31;
-  if (off + BITS <= 32) return (w[word] >> off) & ((1u << BITS) - 1u);
-  return __funnelshift_r(w[word], w[word + 1 < BITS / 4 ? word + 1 : word], off) & ((1u << BITS) - 1u);
-}
-
-// NIDX consecutive BITS-wide fields starting at field `first` of a little-endian stream
-// that begins at the 4-byte aligned address `base`; `first` is a multiple of NIDX.
-template <int BITS, int NIDX>
-__device__ __forceinline__ void load_fields(const uint8_t* base, int first, uint32_t (&out)[NIDX]) {
-  constexpr int kBits = BITS * NIDX;
-  constexpr uint32_t kMask = (1u << BITS) - 1u;
-  const uint32_t* w32 = reinterpret_cast<const uint32_t*>(base);
-  if constexpr (kBits % 32 == 0) {
-    constexpr int NW = kBits / 32;
-    uint32_t w[NW];
-    const int w0 = first * BITS / 32;
-#pragma unroll
-    for (int j = 0; j < NW; ++j) w[j] = w32[w0 + j];
-#pragma unroll
-    for (int j = 0; j < NIDX; ++j) {
-      const int bit = j * BITS, word = bit >> 5, off = bit & 31;
-      out[j] = (off + BITS <= 32) ? ((w[word] >> off) & kMask)
-                                  : (__funnelshift_r(w[word], w[word + 1 < NW ? word + 1 : word], off) & kMask);
-    }
-  } else {
-    static_assert(kBits <= 48, "unaligned field windows must fit 64 bits after a 16-bit offset");
-    const int start = first * BITS;
-    const uint64_t v = (((uint64_t)w32[(start >> 5) + 1] << 32) | w32[start >> 5]) >> (start & 31);
-#pragma unroll
-    for (int j = 0; j < NIDX; ++j) out[j] = (uint32_t)(v >> (j * BITS)) & kMask;
-  }
-}
-
-struct LargeMParams {
-  const uint8_t* cb_hilo;       // [C][2][D] e4m3
-  const uint16_t* scales;       // bf16 [N]
-  const uint16_t* bias;         // bf16 [N] or null
-  const float* act_scale;       // [M]
-  uint16_t* y;                  // bf16 [M, ldy]
-  const uint16_t* residual;     // bf16 [M, ldr] added to the rounded output, or null
-  int64_t ldr;
-  int n_bc;                     // further copies of the output (peer GPUs' buffers), same pitch as y
-  uint16_t* ybc[kMaxBcast];
-  int* status;
-  int64_t ldy;
-  int M, N, K, C;
-  float out_mul;                // 2^-cb8_exp_shift
-};
-
-// Up to four layers of one geometry in one launch (blockIdx.z = layer).
-constexpr int kMaxLayersPerLaunch = 4;
-struct alignas(64) LargeMMulti {
-  CUtensorMap idx[kMaxLayersPerLaunch];     // packed-index tile maps, one per layer
-  LargeMParams layer[kMaxLayersPerLaunch];
-};
-
-// Shared-memory carve-up (offsets from a 1024-byte aligned base).
-struct SmemLayout {
-  uint32_t stage_off;      // stages x {MT x A 16 KB, B_hi, B_lo of BN x 128 bytes}
-  uint32_t stage_bytes;
-  uint32_t idx_off;        // 2 x [128 rows][sb_bytes]
-  uint32_t cb_off;         // [C][2][D]
-  uint32_t sw_off;         // float[128] scale[n] * out_mul
-  uint32_t bias_off;       // float[128]
-  uint32_t bar_off;        // mbarriers
-  uint32_t misc_off;       // tmem base, abort flag
-  uint32_t total;
-};
-
-// A pipeline stage holds kbs K blocks (1 or 2; 2 = exactly one index super-block): every
-// barrier round trip costs each role several hundred cycles, so narrow tiles, whose K blocks
-// are cheap, take two per stage.  Stages: 3 where they fit, else 2.
-__host__ __device__ constexpr int stages_for(int bn, int mt, int kbs) {
-  return kbs == 2 ? (bn == 32 ? 3 : 2) : (mt == 2 ? 2 : kMaxStages);
-}
-
-__host__ __device__ inline SmemLayout make_layout(int bn, int mt, int sb_bytes, int cb_bytes, int kbs = 1) {
-  SmemLayout L;
-  L.stage_off = 0;
-  L.stage_bytes = kbs * (mt * kTileBytes + 2 * bn * kBK);
-  L.idx_off = stages_for(bn, mt, kbs) * L.stage_bytes;
-  L.cb_off = L.idx_off + 2 * bn * sb_bytes;
-  L.cb_off = (L.cb_off + 127) & ~127u;
-  L.sw_off = L.cb_off + ((cb_bytes + 127) & ~127);
-  L.bias_off = L.sw_off + kMaxBN * 4;
-  L.bar_off = L.bias_off + kMaxBN * 4;
-  L.misc_off = L.bar_off + 16 * 8;
-  L.total = L.misc_off + 64;
-  return L;
-}
-
-// D in {4, 8}, BITS in {8, 12, 16}, BN in {32, 64, 128}.  grid = (ceil(N/BN), ceil(M/128)).
-// Smaller BN trades tensor-core efficiency for more CTAs when M is only a few tiles.  MT = 2
-// gives the CTA two 128-token sub-tiles (two TMEM accumulators) that share every expanded
-// B tile: the shared-memory gathers, not the MMAs, are what limits this kernel.
-// The high and the low B tile are issued as ONE MMA of N = 2*BN (they are adjacent in shared
-// memory, so they form one K-major operand): A x hi lands in accumulator columns [0, BN),
-// A x lo in [BN, 2*BN), and the epilogue adds them.  A small-N MMA is bound by its
-// shared-memory operand reads, so reading the A tile once instead of twice is what counts at
-// small and medium M.  Every tile shape does this, so the order in which an output element is
-// summed does not depend on the tile shape and the shards of a split layer reproduce the whole
-// layer bit for bit.
-template <int D, int BITS, int BN, int MT, int KBS>
-__global__ void __launch_bounds__(kThreads, 1)
-large_m_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ LargeMMulti mp) {
-  // blockIdx.z selects the layer: sibling projections that read the same activations run as
-  // one launch; grid.x covers the widest of them, CTAs beyond a narrower layer leave at once
-  const LargeMParams& p = mp.layer[blockIdx.z];
-  const CUtensorMap* tmap_idx_p = &mp.idx[blockIdx.z];
-  if ((int)blockIdx.x * BN >= p.N) return;
-  // the next kernel of the stream, if launched with programmatic serialization, may be scheduled
-  // from here on (its launch latency overlaps this grid); it waits for this grid before it touches memory
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  constexpr int IDX_PER_KB = kBK / D;                 // indices per row per K block
-  constexpr int KB_BYTES = IDX_PER_KB * BITS / 8;     // index bytes per row per K block
-  constexpr int SB_BYTES = 2 * KB_BYTES;              // ... per super block (two K blocks): multiple of 16
-  constexpr int CW_BYTES = 2 * D;                     // hi + lo bytes per codeword
-  constexpr int PARTS = kExpanderThreads / BN;        // expander threads per weight row
-  constexpr int CPT = 8 / PARTS;                      // 16-byte chunks each of them writes per K block
-  constexpr int IPC = 16 / D;                         // indices per chunk
-  constexpr int ACC_COLS = 2 * BN;                    // accumulator columns per token sub-tile (high | low)
-  constexpr uint32_t kIdesc = make_idesc(ACC_COLS);
-  constexpr int B_TILE = BN * kBK;
-  constexpr int kStages = stages_for(BN, MT, KBS);
-  constexpr int A_BYTES = MT * kTileBytes;            // A tiles of one K block
-  constexpr int B_OFF = KBS * A_BYTES;                // the stage's B tiles follow all of its A tiles
-
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t raw = smem_u32(smem_raw);
-  const uint32_t base = (raw + 1023u) & ~1023u;
-  uint8_t* sm = smem_raw + (base - raw);
-  const SmemLayout L = make_layout(BN, MT, SB_BYTES, p.C * CW_BYTES, KBS);
-
-  // barrier indices
-  constexpr int A_FULL = 0, B_FULL = kMaxStages, EMPTY = 2 * kMaxStages, IDX_FULL = 3 * kMaxStages,
-                IDX_EMPTY = 3 * kMaxStages + 2, ACC_FULL = 3 * kMaxStages + 4, CB_FULL = 3 * kMaxStages + 5;
-  const uint32_t bars = base + L.bar_off;
-  auto bar = [&](int i) { return bars + 8u * i; };
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + L.misc_off);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + L.misc_off + 8);
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n0 = blockIdx.x * BN;
-  const int m0 = blockIdx.y * (kBM * MT);
-  const int num_kb = p.K / kBK;
-  const uint32_t cb_bytes = (uint32_t)(p.C * CW_BYTES);
-  const bool cb_bulk = (cb_bytes & 15u) == 0;         // bulk copies move multiples of 16 bytes
-
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < kStages; ++i) {
-      mbar_init(bar(A_FULL + i), 1);
-      mbar_init(bar(B_FULL + i), kExpanderThreads / 32);
-      mbar_init(bar(EMPTY + i), 1);
-    }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(bar(IDX_FULL + i), 1);
-      mbar_init(bar(IDX_EMPTY + i), kExpanderThreads / 32);
-    }
-    mbar_init(bar(ACC_FULL), 1);
-    mbar_init(bar(CB_FULL), 1);
-    *abort_flag = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    prefetch_tensormap(&tmap_a);
-    prefetch_tensormap(tmap_idx_p);
-  }
-  if (warp == 1) tmem_alloc(smem_u32(tmem_slot), (uint32_t)(ACC_COLS * MT));
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-
-  if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      if (cb_bulk) {                                  // the codebook: one bulk copy, ahead of everything else
-        mbar_arrive_expect_tx(bar(CB_FULL), cb_bytes);
-        bulk_load(base + L.cb_off, p.cb_hilo, cb_bytes, bar(CB_FULL));
-      }
-      for (int it = 0; it < num_kb / KBS; ++it) {
-        const int kb0 = it * KBS;
-        if ((kb0 & 1) == 0) {
-          const int sb = kb0 >> 1, slot = sb & 1;
-          if (!mbar_wait(bar(IDX_EMPTY + slot), ((sb >> 1) & 1) ^ 1, abort_flag, p.status)) break;
-          mbar_arrive_expect_tx(bar(IDX_FULL + slot), BN * SB_BYTES);
-          tma_load_2d(base + L.idx_off + slot * BN * SB_BYTES, tmap_idx_p, sb * SB_BYTES, n0, bar(IDX_FULL + slot));
-        }
-        const int st = it % kStages;
-        if (!mbar_wait(bar(EMPTY + st), ((it / kStages) & 1) ^ 1, abort_flag, p.status)) break;
-        mbar_arrive_expect_tx(bar(A_FULL + st), KBS * A_BYTES);
-#pragma unroll
-        for (int kk = 0; kk < KBS; ++kk)
-#pragma unroll
-          for (int mt = 0; mt < MT; ++mt)
-            tma_load_2d(base + L.stage_off + st * L.stage_bytes + kk * A_BYTES + mt * kTileBytes, &tmap_a,
-                        (kb0 + kk) * kBK, m0 + mt * kBM, bar(A_FULL + st));
-      }
-    }
-    __syncwarp();
-  } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      bool ok = true;
-      for (int it = 0; it < num_kb / KBS && ok; ++it) {
-        const int st = it % kStages;
-        const uint32_t ph = (it / kStages) & 1;
-        ok = mbar_wait(bar(A_FULL + st), ph, abort_flag, p.status) &&
-             mbar_wait(bar(B_FULL + st), ph, abort_flag, p.status);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t s_addr = base + L.stage_off + st * L.stage_bytes;
-#pragma unroll
-        for (int kk = 0; kk < KBS; ++kk) {
-          const uint32_t a_addr = s_addr + kk * A_BYTES;
-          const uint64_t b_desc = make_smem_desc(s_addr + B_OFF + kk * 2 * B_TILE);            // high and low halves as one operand
-#pragma unroll
-          for (int ks = 0; ks < kBK / 32; ++ks) {
-            const uint64_t adv = (uint64_t)((ks * 32) >> 4);
-#pragma unroll
-            for (int mt = 0; mt < MT; ++mt) {
-              const uint64_t a_desc = make_smem_desc(a_addr + mt * kTileBytes);
-              umma_f8(tmem_base + (uint32_t)(mt * ACC_COLS), a_desc + adv, b_desc + adv, kIdesc, (it | kk | ks) != 0);
-            }
-          }
-        }
-        umma_commit(bar(EMPTY + st));
-      }
-      if (ok) umma_commit(bar(ACC_FULL));
-    }
-    __syncwarp();
-  } else {
-    // ------------------------------------------------------------------ expanders, then epilogue
-    const int et = threadIdx.x - 64;                 // 0..255
-    const int row = et % BN;
-    const int part = et / BN;                        // which CPT chunks of the row's 8 this thread writes
-    {
-      // codebook (hi/lo) and the per-column epilogue constants
-      if (!cb_bulk) {
-        const uint4* src = reinterpret_cast<const uint4*>(p.cb_hilo);
-        uint4* dst = reinterpret_cast<uint4*>(sm + L.cb_off);
-        const int n16 = (p.C * CW_BYTES) >> 4;
-        for (int i = et; i < n16; i += kExpanderThreads) cp_async_16(dst + i, src + i);
-      }
-      if (et < BN) {
-        const int n = min(n0 + et, p.N - 1);
-        reinterpret_cast<float*>(sm + L.sw_off)[et] = bf16_bits_to_float(__ldg(p.scales + n)) * p.out_mul;
-        reinterpret_cast<float*>(sm + L.bias_off)[et] = p.bias ? bf16_bits_to_float(__ldg(p.bias + n)) : 0.f;
-      }
-      cp_async_wait_all();
-      expander_barrier();
-    }
-    const uint8_t* cbs = sm + L.cb_off;
-    bool ok = true;
-    if (cb_bulk) ok = mbar_wait(bar(CB_FULL), 0, abort_flag, p.status);
-    for (int it = 0; it < num_kb / KBS && ok; ++it) {
-      const int kb0 = it * KBS;
-      const int sb = kb0 >> 1, slot = sb & 1;
-      const int st = it % kStages;
-      ok = mbar_wait(bar(IDX_FULL + slot), (sb >> 1) & 1, abort_flag, p.status) &&
-           mbar_wait(bar(EMPTY + st), ((it / kStages) & 1) ^ 1, abort_flag, p.status);
-      if (!ok) break;
-#pragma unroll
-      for (int kk = 0; kk < KBS; ++kk) {
-      const int kb = kb0 + kk;
-      // this thread's CPT * IPC indices of the row's K block
-      uint32_t idx[CPT * IPC];
-      load_fields<BITS, CPT * IPC>(sm + L.idx_off + slot * BN * SB_BYTES + row * SB_BYTES + (kb & 1) * KB_BYTES,
-                                   part * CPT * IPC, idx);
-      uint8_t* bhi = sm + L.stage_off + st * L.stage_bytes + B_OFF + kk * 2 * B_TILE + row * 128;
-      uint8_t* blo = bhi + B_TILE;
-      const int sw = row & 7;
-#pragma unroll
-      for (int c = 0; c < CPT; ++c) {
-        const int chunk = part * CPT + c;              // logical 16-byte chunk of the 128-byte row
-        uint4 hi4, lo4;
-        if constexpr (D == 8) {
-          const uint4 c0 = *reinterpret_cast<const uint4*>(cbs + (size_t)idx[c * IPC] * 16);
-          const uint4 c1 = *reinterpret_cast<const uint4*>(cbs + (size_t)idx[c * IPC + 1] * 16);
-          hi4 = make_uint4(c0.x, c0.y, c1.x, c1.y);
-          lo4 = make_uint4(c0.z, c0.w, c1.z, c1.w);
-        } else {
-          uint2 cw[4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) cw[j] = *reinterpret_cast<const uint2*>(cbs + (size_t)idx[c * IPC + j] * 8);
-          hi4 = make_uint4(cw[0].x, cw[1].x, cw[2].x, cw[3].x);
-          lo4 = make_uint4(cw[0].y, cw[1].y, cw[2].y, cw[3].y);
-        }
-        *reinterpret_cast<uint4*>(bhi + ((chunk ^ sw) * 16)) = hi4;
-        *reinterpret_cast<uint4*>(blo + ((chunk ^ sw) * 16)) = lo4;
-      }
-      }
-      fence_proxy_async();                            // generic-proxy writes -> visible to the tensor core
-      __syncwarp();
-      if (lane == 0) {                                // one arrival per warp keeps the barrier off the critical path
-        mbar_arrive(bar(B_FULL + st));
-        const int kb = kb0 + KBS - 1;                 // last K block of this stage
-        if ((kb & 1) == 1 || kb == num_kb - 1) mbar_arrive(bar(IDX_EMPTY + slot));
-      }
-    }
-
-    // ---- epilogue: this warp's TMEM lane quarter, half of the 128 columns
-    // the token scales of this warp's rows are fetched before the wait for the accumulator, so
-    // their global-memory latency is off the critical path
-    float sa_pre[MT];
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
-      const int m = m0 + mt * kBM + (warp & 3) * 32 + lane;
-      sa_pre[mt] = m < p.M ? __ldg(p.act_scale + m) : 0.f;
-    }
-    if (ok) ok = mbar_wait(bar(ACC_FULL), 0, abort_flag, p.status);
-    ok = expander_all(ok);                            // uniform over the expanders: tcgen05.ld and the staging barriers are collective
-    if (ok) {
-      tc_fence_after();
-      const int quarter = warp & 3;                   // TMEM lanes 32*quarter .. +31
-      const int col_half = (warp - 2) >> 2;           // two warps share a quarter: they split the 32-column groups
-      const float* swp = reinterpret_cast<const float*>(sm + L.sw_off);
-      const float* bp = reinterpret_cast<const float*>(sm + L.bias_off);
-      // The accumulator tile goes through shared memory (the pipeline stages are idle now) so
-      // that the global stores are whole row segments instead of 64 bytes per thread.
-      constexpr int SP = BN * 2 + 16;                 // staging row pitch: 16 bytes of skew against bank conflicts
-      uint8_t* stg = sm + L.stage_off;
-      if (p.n_bc == 0) {
-        // one GPU: every thread stores its own 64-byte row pieces (measured 2-10 % faster than staging)
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt) {
-          const int m = m0 + mt * kBM + quarter * 32 + lane;
-          const float sa = sa_pre[mt];
-#pragma unroll
-          for (int cc = col_half; cc < BN / 32; cc += 2) {
-            const int c0 = cc * 32;
-            uint32_t r[32];
-            tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(mt * ACC_COLS + c0), r);
-            {
-              uint32_t rl[32];
-              tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(mt * ACC_COLS + BN + c0), rl);
-#pragma unroll
-              for (int c = 0; c < 32; ++c) r[c] = __float_as_uint(__uint_as_float(r[c]) + __uint_as_float(rl[c]));
-            }
-            if (m < p.M) {
-              uint16_t* yrow = p.y + (int64_t)m * p.ldy + n0 + c0;
-              const uint16_t* rrow = p.residual ? p.residual + (int64_t)m * p.ldr + n0 + c0 : nullptr;
-              // bf16(v), or bf16(bf16(v) + residual): the two roundings of `linear(x) + residual`
-              auto fin = [&](float v, int c) -> uint32_t {
-                uint16_t o = float_to_bf16_bits(v);
-                if (rrow != nullptr)
-                  o = float_to_bf16_bits(__fadd_rn(bf16_bits_to_float(o), bf16_bits_to_float(__ldg(rrow + c))));
-                return (uint32_t)o;
-              };
-              const bool vec = (n0 + c0 + 32 <= p.N) && ((reinterpret_cast<uintptr_t>(yrow) & 15) == 0);
-              if (vec) {
-#pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                  uint32_t o[4];
-#pragma unroll
-                  for (int j = 0; j < 4; ++j) {
-                    const int c = v * 8 + 2 * j;
-                    const float y0 = fmaf(sa, __uint_as_float(r[c]) * swp[c0 + c], bp[c0 + c]);
-                    const float y1 = fmaf(sa, __uint_as_float(r[c + 1]) * swp[c0 + c + 1], bp[c0 + c + 1]);
-                    o[j] = fin(y0, c) | (fin(y1, c + 1) << 16);
-                  }
-                  *reinterpret_cast<uint4*>(yrow + v * 8) = make_uint4(o[0], o[1], o[2], o[3]);
-                }
-              } else {
-#pragma unroll
-                for (int c = 0; c < 32; ++c)
-                  if (n0 + c0 + c < p.N)
-                    yrow[c] = (uint16_t)fin(fmaf(sa, __uint_as_float(r[c]) * swp[c0 + c], bp[c0 + c]), c);
-              }
-            }
-          }
-        }
-      } else {
-        // further copies on peer GPUs: stage the tile, then store whole row segments everywhere
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt) {
-          const int m = m0 + mt * kBM + quarter * 32 + lane;
-          const float sa = sa_pre[mt];
-          uint8_t* srow = stg + (quarter * 32 + lane) * SP;
-#pragma unroll
-          for (int cc = col_half; cc < BN / 32; cc += 2) {
-            const int c0 = cc * 32;
-            uint32_t r[32];
-            tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(mt * ACC_COLS + c0), r);
-            {
-              uint32_t rl[32];
-              tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(mt * ACC_COLS + BN + c0), rl);
-#pragma unroll
-              for (int c = 0; c < 32; ++c) r[c] = __float_as_uint(__uint_as_float(r[c]) + __uint_as_float(rl[c]));
-            }
-            const uint16_t* rrow = (p.residual && m < p.M) ? p.residual + (int64_t)m * p.ldr + n0 + c0 : nullptr;
-            // bf16(v), or bf16(bf16(v) + residual): the two roundings of `linear(x) + residual`
-            auto fin = [&](float v, int c) -> uint32_t {
-              uint16_t o = float_to_bf16_bits(v);
-              if (rrow != nullptr && n0 + c0 + c < p.N)
-                o = float_to_bf16_bits(__fadd_rn(bf16_bits_to_float(o), bf16_bits_to_float(__ldg(rrow + c))));
-              return (uint32_t)o;
-            };
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-              uint32_t o[4];
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const int c = v * 8 + 2 * j;
-                const float y0 = fmaf(sa, __uint_as_float(r[c]) * swp[c0 + c], bp[c0 + c]);
-                const float y1 = fmaf(sa, __uint_as_float(r[c + 1]) * swp[c0 + c + 1], bp[c0 + c + 1]);
-                o[j] = fin(y0, c) | (fin(y1, c + 1) << 16);
-              }
-              *reinterpret_cast<uint4*>(srow + (c0 + v * 8) * 2) = make_uint4(o[0], o[1], o[2], o[3]);
-            }
-          }
-          expander_barrier();                             // the tile is staged
-          store_staged_tile<BN>(stg, SP, et, m0 + mt * kBM, p.M, n0, p.N, p.y, p.ldy, p.ybc, p.n_bc);
-          expander_barrier();                             // before the next sub-tile reuses the staging rows
-        }
-      }
-    }
-  }
-
-  // ---- common exit: every thread arrives here, also after an aborted wait
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 1) tmem_dealloc(tmem_base, (uint32_t)(ACC_COLS * MT));
-}
-
-
-}  // namespace
-
 struct LargeMPlan {
-  CUtensorMap tmap_idx[3];      // index-tile maps for BN = 32, 64, 128
-  bool have[3];
-  int sb_bytes;
+  CUtensorMap tmap_idx;         // index super-blocks (two 128-k blocks) x 128 weight rows
+  bool have;
 };
 
 namespace {
+
+constexpr int kBK = 128;          // e4m3 elements (= bytes) per K block: one 128B swizzle row
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -526,56 +58,35 @@ int encode_bytes_2d(CUtensorMap* map, const void* base, uint64_t row_bytes, uint
   return SACQ_OK;
 }
 
+int encode_bytes_3d(CUtensorMap* map, const void* base, uint64_t row_bytes, uint64_t rows, uint64_t dim2, uint64_t row_pitch,
+                    uint64_t dim2_pitch, uint32_t box_bytes, uint32_t box_rows, uint32_t box2) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (fn == nullptr) return set_error(SACQ_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+  const cuuint64_t dims[3] = {row_bytes, rows, dim2};
+  const cuuint64_t strides[2] = {row_pitch, dim2_pitch};
+  const cuuint32_t box[3] = {box_bytes, box_rows, box2};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return set_error(SACQ_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
+  return SACQ_OK;
+}
+
 namespace {
 
 int sb_bytes_for(const sacq_layer* L) { return 2 * (kBK / L->d.vector_dim) * L->d.index_bits / 8; }
 
-template <int D, int BITS, int BN, int MT, int KBS = 1>
-cudaError_t launch_bn(const CUtensorMap& ta, const LargeMMulti& mp, dim3 grid, cudaStream_t s) {
-  const size_t smem = make_layout(BN, MT, 2 * (kBK / D) * BITS / 8, mp.layer[0].C * 2 * D, KBS).total + 1024;
-  static bool configured[64] = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64 || !configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(large_m_kernel<D, BITS, BN, MT, KBS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         227 * 1024);
-    if (e != cudaSuccess) return e;
-    if (dev >= 0 && dev < 64) configured[dev] = true;
-  }
-  // (Programmatic dependent launch behind the quantizer was measured and is not used here: the
-  // early-resident 200 KB CTAs slowed the kernels around them more than the overlap gained.)
-  large_m_kernel<D, BITS, BN, MT, KBS><<<grid, kThreads, smem, s>>>(ta, mp);
-  return cudaGetLastError();
-}
-
-template <int D, int BITS>
-cudaError_t launch_one(const CUtensorMap& ta, const LargeMMulti& mp, int bn, int mt, dim3 grid, cudaStream_t s) {
-  // every tile shape issues the high and the low tile as one MMA: an output's summation order
-  // is then the same for all shapes (a layer's shards reproduce the whole layer bit for bit)
-  if (mt == 2) {
-    if (bn == 32) return launch_bn<D, BITS, 32, 2>(ta, mp, grid, s);
-    if (bn == 64) return launch_bn<D, BITS, 64, 2>(ta, mp, grid, s);
-    return launch_bn<D, BITS, 128, 2>(ta, mp, grid, s);
-  }
-  // narrow tiles with one token sub-tile: two K blocks per pipeline stage when that fits
-  const bool two = make_layout(bn, 1, 2 * (kBK / D) * BITS / 8, mp.layer[0].C * 2 * D, 2).total + 1024 <= 227 * 1024;
-  if (bn == 32) return two ? launch_bn<D, BITS, 32, 1, 2>(ta, mp, grid, s) : launch_bn<D, BITS, 32, 1>(ta, mp, grid, s);
-  if (bn == 64) return two ? launch_bn<D, BITS, 64, 1, 2>(ta, mp, grid, s) : launch_bn<D, BITS, 64, 1>(ta, mp, grid, s);
-  return launch_bn<D, BITS, 128, 1>(ta, mp, grid, s);
-}
+std::mutex g_plan_mutex;   // layers build their index tile map on first use, possibly from several host threads
 
 }  // namespace
 
 bool large_m_supported(const sacq_layer* L) {
   const sacq_layer_desc& d = L->d;
-  if (d.vector_dim != 8 && d.vector_dim != 4) return false;
   if (d.index_bits != 8 && d.index_bits != 12 && d.index_bits != 16) return false;
-  if (!L->rows_16b_aligned) return false;
   if (d.in_features % (2 * kBK) != 0) return false;
-  if (L->num_groups != 1 || has_shift(L)) return false;
-  const size_t cb_bytes = (size_t)L->cb_entries * d.vector_dim * 2;
-  if (make_layout(kMaxBN, 1, sb_bytes_for(L), (int)cb_bytes).total + 1024 > 227 * 1024) return false;
-  return true;
+  SplitChoice c;
+  return split_k_choose(L, 1, kSplitHiLo, &c);
 }
 
 void large_m_release(sacq_layer* L) {
@@ -583,156 +94,43 @@ void large_m_release(sacq_layer* L) {
   L->large_plan = nullptr;
 }
 
-namespace {
-
-// Tile shape: (token sub-tiles per CTA, weight rows per CTA) with the smallest
-// waves x time-per-CTA.  Fitted to measurements (us): a CTA takes about
-// 3.4 + K/2048 * (4.8 + 0.0755 * BN + 3.0 * (MT - 1)): fixed prologue/epilogue, pipeline
-// latency per K block (halved, 2.4, where a stage holds two K blocks: one sub-tile of 32 or
-// 64 rows), expansion per weight row, MMA issue per extra sub-tile.
-bool choose_tile(const sacq_layer* L, int64_t M, const int64_t* ns, int n_layers, int& bn, int& mt) {
-  const sacq_layer_desc& d = L->d;
-  const size_t cb_bytes = (size_t)L->cb_entries * d.vector_dim * 2;
-  bn = 0;
-  mt = 1;
-  double best = 1e30;
-  for (int cand_mt = 1; cand_mt <= (M > kBM ? 2 : 1); ++cand_mt) {
-    const int64_t m_tiles = (M + kBM * cand_mt - 1) / (kBM * cand_mt);
-    for (int cand = 128; cand >= 32; cand >>= 1) {
-      if (make_layout(cand, cand_mt, sb_bytes_for(L), (int)cb_bytes).total + 1024 > 227 * 1024) continue;
-      int64_t tiles = 0;
-      for (int l = 0; l < n_layers; ++l) tiles += ((ns[l] + cand - 1) / cand) * m_tiles;
-      const int64_t waves = (tiles + L->num_sms - 1) / L->num_sms;
-      const bool two_kb = cand_mt == 1 && cand <= 64 &&
-                          make_layout(cand, 1, sb_bytes_for(L), (int)cb_bytes, 2).total + 1024 <= 227 * 1024;
-      const double per_cta = 3.4 + (double)d.in_features / 2048.0 *
-                                       ((two_kb ? 2.4 : 4.8) + 0.0755 * cand + 3.0 * (cand_mt - 1));
-      const double cost = (double)waves * per_cta;
-      if (cost < best - 1e-9) { best = cost; bn = cand; mt = cand_mt; }
-    }
-  }
-  return bn != 0;
-}
-
-std::mutex g_plan_mutex;   // layers build their index tile maps on first use, possibly from several host threads
-
-int ensure_idx_map(sacq_layer* Lm, int bn, const CUtensorMap** out) {
+int large_m_index_map(const sacq_layer* Lc, const CUtensorMap** out) {
+  sacq_layer* L = const_cast<sacq_layer*>(Lc);
   std::lock_guard<std::mutex> lock(g_plan_mutex);
-  if (Lm->large_plan == nullptr) {
-    LargeMPlan* plan = new LargeMPlan();
-    plan->sb_bytes = sb_bytes_for(Lm);
-    plan->have[0] = plan->have[1] = plan->have[2] = false;
-    Lm->large_plan = plan;
-  }
-  const int bi = bn == 32 ? 0 : (bn == 64 ? 1 : 2);
-  if (!Lm->large_plan->have[bi]) {
-    const uint64_t row_bytes = (uint64_t)(Lm->row_bits / 8);
-    const int rc = encode_bytes_2d(&Lm->large_plan->tmap_idx[bi], Lm->d.packed, row_bytes, (uint64_t)Lm->d.out_features,
-                                   row_bytes, (uint32_t)Lm->large_plan->sb_bytes, (uint32_t)bn,
-                                   CU_TENSOR_MAP_SWIZZLE_NONE);
+  if (L->large_plan == nullptr) L->large_plan = new LargeMPlan();
+  if (!L->large_plan->have) {
+    const uint64_t row_bytes = (uint64_t)(L->row_bits / 8);
+    const int rc = encode_bytes_2d(&L->large_plan->tmap_idx, L->d.packed, row_bytes, (uint64_t)L->d.out_features, row_bytes,
+                                   (uint32_t)sb_bytes_for(L), 128u, CU_TENSOR_MAP_SWIZZLE_NONE);
     if (rc != SACQ_OK) return rc;
-    Lm->large_plan->have[bi] = true;
+    L->large_plan->have = true;
   }
-  *out = &Lm->large_plan->tmap_idx[bi];
+  *out = &L->large_plan->tmap_idx;
   return SACQ_OK;
-}
-
-// n layers (n = 1: the plain launch) on one set of quantized activations.
-int launch_layers(const sacq_layer* const* layers, int n, const void* q, const float* scale, int64_t M,
-                  void* const* ys, const int64_t* ldys, int bn, int mt, cudaStream_t s, const void* residual,
-                  int64_t ldr, const BcastDst* bc) {
-  const sacq_layer* L0 = layers[0];
-  const sacq_layer_desc& d0 = L0->d;
-  CUtensorMap ta;
-  {
-    const int rc = encode_bytes_2d(&ta, q, (uint64_t)d0.in_features, (uint64_t)M, (uint64_t)d0.in_features, kBK, kBM,
-                                   CU_TENSOR_MAP_SWIZZLE_128B);
-    if (rc != SACQ_OK) return rc;
-  }
-  LargeMMulti mp{};
-  int64_t widest = 0;
-  for (int l = 0; l < n; ++l) {
-    const sacq_layer* L = layers[l];
-    const CUtensorMap* ti = nullptr;
-    const int rc = ensure_idx_map(const_cast<sacq_layer*>(L), bn, &ti);
-    if (rc != SACQ_OK) return rc;
-    mp.idx[l] = *ti;
-    LargeMParams& p = mp.layer[l];
-    p.cb_hilo = L->cb_hilo;
-    p.scales = static_cast<const uint16_t*>(L->d.scales);
-    p.bias = static_cast<const uint16_t*>(L->d.bias);
-    p.act_scale = scale;
-    p.y = static_cast<uint16_t*>(ys[l]);
-    p.status = L->d_status;
-    p.ldy = ldys[l];
-    p.residual = static_cast<const uint16_t*>(residual);
-    p.ldr = ldr;
-    if (bc != nullptr) {
-      p.n_bc = bc->n;
-      for (int i = 0; i < bc->n; ++i) p.ybc[i] = static_cast<uint16_t*>(bc->ptr[i]);
-    }
-    p.M = (int)M; p.N = (int)L->d.out_features; p.K = (int)L->d.in_features; p.C = L->cb_entries;
-    p.out_mul = ldexpf(1.f, -L->cb8_exp_shift);
-    if (L->d.out_features > widest) widest = L->d.out_features;
-  }
-  const dim3 grid((unsigned)((widest + bn - 1) / bn), (unsigned)((M + kBM * mt - 1) / (kBM * mt)), (unsigned)n);
-  if (grid.y > 65535) return set_error(SACQ_ERR_UNSUPPORTED, "M=%lld exceeds the grid limit", (long long)M);
-  cudaError_t e;
-  const int D = d0.vector_dim, B = d0.index_bits;
-  if (D == 8 && B == 12) e = launch_one<8, 12>(ta, mp, bn, mt, grid, s);
-  else if (D == 8 && B == 8) e = launch_one<8, 8>(ta, mp, bn, mt, grid, s);
-  else if (D == 8 && B == 16) e = launch_one<8, 16>(ta, mp, bn, mt, grid, s);
-  else if (D == 4 && B == 12) e = launch_one<4, 12>(ta, mp, bn, mt, grid, s);
-  else if (D == 4 && B == 8) e = launch_one<4, 8>(ta, mp, bn, mt, grid, s);
-  else e = launch_one<4, 16>(ta, mp, bn, mt, grid, s);
-  count_launch();
-  if (e != cudaSuccess) return cuda_fail(e, "large-M launch");
-  return SACQ_OK;
-}
-
-}  // namespace
-
-int large_m_index_map(const sacq_layer* L, int rows, const CUtensorMap** out) {
-  return ensure_idx_map(const_cast<sacq_layer*>(L), rows, out);
 }
 
 int launch_large_m(const sacq_layer* L, const void* q, const float* scale, int64_t M, void* y, int64_t ldy,
                    cudaStream_t s, const void* residual, int64_t ldr, const BcastDst* bc) {
-  const sacq_layer_desc& d = L->d;
   if (!large_m_supported(L)) return set_error(SACQ_ERR_UNSUPPORTED, "large-M kernel cannot run this layer geometry");
-  if (M <= 0 || d.out_features == 0) return SACQ_OK;
-  if (M > (1 << 30)) return set_error(SACQ_ERR_UNSUPPORTED, "M=%lld too large", (long long)M);
-  if (reinterpret_cast<uintptr_t>(q) % 16 != 0)
-    return set_error(SACQ_ERR_ALIGNMENT, "large-M kernel: quantized activations must be 16-byte aligned");
-  int bn = 0, mt = 1;
-  const int64_t n_rows = d.out_features;
-  if (!choose_tile(L, M, &n_rows, 1, bn, mt))
-    return set_error(SACQ_ERR_UNSUPPORTED, "large-M kernel: no tile fits shared memory");
-  return launch_layers(&L, 1, q, scale, M, &y, &ldy, bn, mt, s, residual, ldr, bc);
+  if (M <= 0 || L->d.out_features == 0) return SACQ_OK;
+  SplitChoice c;
+  if (!split_k_choose(L, M, kSplitHiLo, &c)) return set_error(SACQ_ERR_UNSUPPORTED, "M=%lld too large", (long long)M);
+  return launch_split_k(&L, 1, q, scale, M, &y, &ldy, kSplitHiLo, c, s, residual, ldr, bc);
 }
 
 // Several layers of one geometry on the same quantized activations as ONE launch.  Returns
 // SACQ_ERR_UNSUPPORTED (nothing launched) when they cannot share one: the caller falls back
-// to one launch per layer.  An output's summation order does not depend on the tile shape, so
-// the results are byte-identical to separate launches.
+// to one launch per layer.  An output's summation order depends on K alone, so the results are
+// byte-identical to separate launches.
 int launch_large_m_multi(const sacq_layer* const* layers, int n, const void* q, const float* scale, int64_t M,
                          void* const* ys, const int64_t* ldys, cudaStream_t s) {
-  if (n < 2 || n > kMaxLayersPerLaunch || M <= 0 || M > (1 << 30)) return SACQ_ERR_UNSUPPORTED;
+  if (n < 2 || n > kSplitMaxLayers || M <= 0) return SACQ_ERR_UNSUPPORTED;
   if (reinterpret_cast<uintptr_t>(q) % 16 != 0) return SACQ_ERR_UNSUPPORTED;
-  const sacq_layer_desc& d0 = layers[0]->d;
-  int64_t ns[kMaxLayersPerLaunch];
-  for (int l = 0; l < n; ++l) {
-    const sacq_layer* L = layers[l];
-    const sacq_layer_desc& d = L->d;
-    if (!large_m_supported(L) || d.in_features != d0.in_features || d.vector_dim != d0.vector_dim ||
-        d.index_bits != d0.index_bits || d.codebook_size != d0.codebook_size || d.device != d0.device ||
-        d.out_features <= 0)
-      return SACQ_ERR_UNSUPPORTED;
-    ns[l] = d.out_features;
-  }
-  int bn = 0, mt = 1;
-  if (!choose_tile(layers[0], M, ns, n, bn, mt)) return SACQ_ERR_UNSUPPORTED;
-  return launch_layers(layers, n, q, scale, M, ys, ldys, bn, mt, s, nullptr, 0, nullptr);
+  for (int l = 0; l < n; ++l)
+    if (!large_m_supported(layers[l])) return SACQ_ERR_UNSUPPORTED;
+  SplitChoice c;
+  if (!split_k_choose_multi(layers, n, M, kSplitHiLo, &c)) return SACQ_ERR_UNSUPPORTED;
+  return launch_split_k(layers, n, q, scale, M, ys, ldys, kSplitHiLo, c, s);
 }
 
 }  // namespace sacq

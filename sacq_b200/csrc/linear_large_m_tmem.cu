@@ -147,15 +147,13 @@ large_m_tmem_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   constexpr int KB_BYTES = IDX_PER_KB * BITS / 8;     // index bytes per row per K block
   constexpr int SB_BYTES = 2 * KB_BYTES;              // ... per super block (two K blocks): multiple of 16
   constexpr int CW_BYTES = 2 * D;                     // hi + lo bytes per codeword
-  // A TMEM weight stage holds W_K k of the 128 rows.  Half-block stages (W_K = 64, four of them beside
-  // a 384-column accumulator instead of two whole blocks) were measured SLOWER (2048x6144 at M = 8192:
+  // A TMEM weight stage holds one K block of the 128 rows.  Half-block stages (four of them beside a
+  // 384-column accumulator instead of two whole blocks) were measured SLOWER (2048x6144 at M = 8192:
   // 217 against 183 us): the per-stage cost of the expanders (barrier waits, tcgen05.wait::st, fences)
   // does not shrink with the stage.
-  constexpr int W_K = 128;
-  constexpr int WPB = kBK / W_K;                      // weight stages per K block
-  constexpr int W_COLS = W_K / 2;                     // TMEM columns of a stage: W_K / 4 high + W_K / 4 low
-  constexpr int WQ = W_K / 16;                        // 32-bit words a thread writes per half (4 or 8)
-  constexpr int IPT = (W_K / D) / 4;                  // indices per expander thread per weight stage (a quarter row)
+  constexpr int W_COLS = kBK / 2;                     // TMEM columns of a stage: kBK / 4 high + kBK / 4 low
+  constexpr int WQ = kBK / 16;                        // 32-bit words a thread writes per half
+  constexpr int IPT = (kBK / D) / 4;                  // indices per expander thread per weight stage (a quarter row)
   constexpr int kWStages = NT == 3 ? 2 : kMaxWStages; // TMEM weight stages
   constexpr uint32_t kWCol0 = BT;                     // first weight-stage column
   constexpr uint32_t kTmemCols = 512;
@@ -177,7 +175,7 @@ large_m_tmem_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + L.misc_off);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + L.misc_off + 8);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = (int)warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int n0 = blockIdx.x * kRows;
   const int m0 = blockIdx.y * BT;
   const int num_kb = p.K / kBK;
@@ -210,80 +208,83 @@ large_m_tmem_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
   if (threadIdx.x == 0) SACQ_TR(0, 0);
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      if constexpr (CB_SMEM) {
+    if constexpr (CB_SMEM) {
+      if (elect_one()) {
         mbar_arrive_expect_tx(bar(CB_FULL), cb_bytes);
         bulk_load(base + L.cb_off, p.cb_hilo, cb_bytes, bar(CB_FULL));
       }
-      for (int kb = 0; kb < num_kb; ++kb) {
-        if ((kb & 1) == 0) {
-          const int sb = kb >> 1, slot = sb & 1;
-          if (!mbar_wait(bar(IDX_EMPTY + slot), ((sb >> 1) & 1) ^ 1, abort_flag, p.status)) break;
+    }
+    int st = 0;
+    uint32_t free_parity = 1;
+    for (int kb = 0; kb < num_kb; ++kb) {
+      if ((kb & 1) == 0) {
+        const int sb = kb >> 1, slot = sb & 1;
+        if (!mbar_wait_warp(bar(IDX_EMPTY + slot), ((sb >> 1) & 1) ^ 1, abort_flag, p.status)) break;
+        if (elect_one()) {
           mbar_arrive_expect_tx(bar(IDX_FULL + slot), kRows * SB_BYTES);
           tma_load_2d(base + L.idx_off + slot * L.idx_slot, &tmap_idx, sb * SB_BYTES, n0, bar(IDX_FULL + slot));
         }
-        const int st = kb % act_stages;
-        if (!mbar_wait(bar(ACT_EMPTY + st), ((kb / act_stages) & 1) ^ 1, abort_flag, p.status)) break;
+      }
+      if (!mbar_wait_warp(bar(ACT_EMPTY + st), free_parity, abort_flag, p.status)) break;
+      if (elect_one()) {
         if (SACQ_ABLATE(4) && kb >= act_stages) {      // no loads: the stage keeps its first tile
           mbar_arrive(bar(ACT_FULL + st));
-          continue;
-        }
-        mbar_arrive_expect_tx(bar(ACT_FULL + st), nt_valid * kTokTile);
+        } else {
+          mbar_arrive_expect_tx(bar(ACT_FULL + st), nt_valid * kTokTile);
 #pragma unroll
-        for (int t = 0; t < NT; ++t)
-          if (t < nt_valid)
-            tma_load_2d(base + L.act_off + st * L.act_stage + t * kTokTile, &tmap_a, kb * kBK, m0 + t * kBM,
-                        bar(ACT_FULL + st));
+          for (int t = 0; t < NT; ++t)
+            if (t < nt_valid)
+              tma_load_2d(base + L.act_off + st * L.act_stage + t * kTokTile, &tmap_a, kb * kBK, m0 + t * kBM,
+                          bar(ACT_FULL + st));
+        }
       }
+      if (++st == act_stages) { st = 0; free_parity ^= 1; }
     }
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      bool ok = true;
-      for (int wb = 0; wb < num_kb * WPB && ok; ++wb) {
-        const int kb = wb / WPB, sub = wb % WPB;       // K block and which part of it this weight stage holds
-        const int st = kb % act_stages, ws = wb % kWStages;
-        ok = (sub != 0 || mbar_wait(bar(ACT_FULL + st), (kb / act_stages) & 1, abort_flag, p.status)) &&
-             mbar_wait(bar(W_FULL + ws), (wb / kWStages) & 1, abort_flag, p.status);
-        if (!ok) break;
-        tc_fence_after();
-        SACQ_TR(1, wb + 8);
-        const uint32_t act_addr = base + L.act_off + st * L.act_stage;
-        const uint32_t w_col = kWCol0 + (uint32_t)(ws * W_COLS);
+    bool ok = true;
+    int st = 0, ws = 0;
+    uint32_t act_parity = 0, w_parity = 0;
+    for (int kb = 0; kb < num_kb; ++kb) {
+      ok = mbar_wait_warp(bar(ACT_FULL + st), act_parity, abort_flag, p.status) &&
+           mbar_wait_warp(bar(W_FULL + ws), w_parity, abort_flag, p.status);
+      if (!ok) break;
+      tc_fence_after();
+      if (lane == 0) SACQ_TR(1, kb + 8);
+      const uint32_t act_addr = base + L.act_off + st * L.act_stage;
+      const uint32_t w_col = tmem_base + kWCol0 + (uint32_t)(ws * W_COLS);
 #pragma unroll
-        for (int ksl = 0; ksl < W_K / 32; ++ksl) {
-          const int ks = sub * (W_K / 32) + ksl;       // 32-byte K step inside the 128-byte activation rows
-          const uint64_t adv = (uint64_t)((ks * 32) >> 4);
+      for (int ks = 0; ks < kBK / 32; ++ks) {
+        const uint64_t adv = (uint64_t)((ks * 32) >> 4);
 #pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            if (SACQ_ABLATE(8)) continue;
-            const uint32_t a_tmem = tmem_base + w_col + (uint32_t)(half * (W_COLS / 2) + ksl * 8);
-            const uint32_t acc = (wb | ksl | half) != 0;
-            // 384 tokens go as two N = 192 instructions into two accumulators, not as N = 256 + N = 128: an
-            // instruction costs about the same 60 ns for any N from 128 to 256 (microbenchmark: the pair
-            // takes 114 against 126 ns), and consecutive instructions into ONE accumulator wait for each
-            // other (137 ns each), so the two accumulators alternate
-            if (NT == 3 && nt_valid == 3) {
-              umma_f8_ts(tmem_base, a_tmem, make_smem_desc(act_addr) + adv, kIdesc192, acc);
+        for (int half = 0; half < 2; ++half) {
+          if (SACQ_ABLATE(8)) continue;
+          const uint32_t a_tmem = w_col + (uint32_t)(half * (W_COLS / 2) + ks * 8);
+          const uint32_t acc = (kb | ks | half) != 0;
+          if (NT == 3 && nt_valid == 3) {
+            // an instruction takes at most 256 tokens: 384 go as two N = 192
+            if (elect_one()) umma_f8_ts(tmem_base, a_tmem, make_smem_desc(act_addr) + adv, kIdesc192, acc);
+            if (elect_one())
               umma_f8_ts(tmem_base + 192u, a_tmem, make_smem_desc(act_addr + kTokTile * 3 / 2) + adv, kIdesc192, acc);
-            } else if (NT >= 2 && nt_valid >= 2) {
-              umma_f8_ts(tmem_base, a_tmem, make_smem_desc(act_addr) + adv, kIdesc256, acc);
-            } else {
-              umma_f8_ts(tmem_base, a_tmem, make_smem_desc(act_addr) + adv, kIdesc128, acc);
-            }
+          } else if (NT >= 2 && nt_valid >= 2) {
+            if (elect_one()) umma_f8_ts(tmem_base, a_tmem, make_smem_desc(act_addr) + adv, kIdesc256, acc);
+          } else {
+            if (elect_one()) umma_f8_ts(tmem_base, a_tmem, make_smem_desc(act_addr) + adv, kIdesc128, acc);
           }
         }
-        if (sub == WPB - 1) umma_commit(bar(ACT_EMPTY + st));
-        umma_commit(bar(W_EMPTY + ws));
       }
-      if (ok) umma_commit(bar(ACC_FULL));
+      if (elect_one()) umma_commit(bar(ACT_EMPTY + st));
+      if (elect_one()) umma_commit(bar(W_EMPTY + ws));
+      if (++st == act_stages) { st = 0; act_parity ^= 1; }
+      if (++ws == kWStages) { ws = 0; w_parity ^= 1; }
     }
+    if (ok && elect_one()) umma_commit(bar(ACC_FULL));
     __syncwarp();
   } else {
     // ------------------------------------------------------------------ expanders, then epilogue
@@ -306,18 +307,16 @@ large_m_tmem_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     }
     const uint8_t* cbs = CB_SMEM ? sm + L.cb_off : p.cb_hilo;
     bool ok = CB_SMEM ? mbar_wait(bar(CB_FULL), 0, abort_flag, p.status) : true;
-    for (int wb = 0; wb < num_kb * WPB && ok; ++wb) {
-      const int kb = wb / WPB, sub = wb % WPB;
+    for (int kb = 0; kb < num_kb && ok; ++kb) {
       const int sb = kb >> 1, slot = sb & 1;
-      const int ws = wb % kWStages;
-      ok = (sub != 0 || mbar_wait(bar(IDX_FULL + slot), (sb >> 1) & 1, abort_flag, p.status)) &&
-           mbar_wait(bar(W_EMPTY + ws), ((wb / kWStages) & 1) ^ 1, abort_flag, p.status);
+      const int ws = kb % kWStages;
+      ok = mbar_wait(bar(IDX_FULL + slot), (sb >> 1) & 1, abort_flag, p.status) &&
+           mbar_wait(bar(W_EMPTY + ws), ((kb / kWStages) & 1) ^ 1, abort_flag, p.status);
       if (!ok) break;
       tc_fence_after();                              // the MMAs that read this stage are complete
-      if (warp == 2 && lane == 0) SACQ_TR(2, wb + 8);
+      if (warp == 2 && lane == 0) SACQ_TR(2, kb + 8);
       uint32_t idx[IPT];
-      load_fields_w<BITS, IPT>(sm + L.idx_off + slot * L.idx_slot + row * SB_BYTES + (kb & 1) * KB_BYTES +
-                                   sub * (KB_BYTES / WPB),
+      load_fields_w<BITS, IPT>(sm + L.idx_off + slot * L.idx_slot + row * SB_BYTES + (kb & 1) * KB_BYTES,
                                kpart * IPT, idx);
       uint32_t hi[WQ], lo[WQ];
       if (SACQ_ABLATE(1)) {
@@ -351,10 +350,10 @@ large_m_tmem_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
-      if (warp == 2 && lane == 0) SACQ_TR(5, wb + 8);
+      if (warp == 2 && lane == 0) SACQ_TR(5, kb + 8);
       if (lane == 0) {
         mbar_arrive(bar(W_FULL + ws));
-        if (sub == WPB - 1 && ((kb & 1) == 1 || kb == num_kb - 1)) mbar_arrive(bar(IDX_EMPTY + slot));
+        if ((kb & 1) == 1 || kb == num_kb - 1) mbar_arrive(bar(IDX_EMPTY + slot));
       }
     }
 
@@ -494,7 +493,7 @@ int launch_large_m_tmem(const sacq_layer* L, const void* q, const float* scale, 
   }
   const CUtensorMap* ti = nullptr;
   {
-    const int rc = large_m_index_map(L, kRows, &ti);
+    const int rc = large_m_index_map(L, &ti);
     if (rc != SACQ_OK) return rc;
   }
   // the output leaves by tiled bulk stores when y (and every peer copy of a column split) allows it:

@@ -36,6 +36,7 @@
 #include "common.cuh"
 #include "tmem_weights.cuh"
 #include "umma.cuh"
+#include "widen.cuh"
 
 namespace sacq {
 
@@ -130,7 +131,7 @@ large_m_tmem_grouped_kernel(const __grid_constant__ CUtensorMap tmap_a, const __
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + L.misc_off);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + L.misc_off + 8);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = (int)warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int n0 = blockIdx.x * kRows;
   const int m0 = blockIdx.y * BT;
   const int num_kb = p.K / kBKh;
@@ -162,23 +163,26 @@ large_m_tmem_grouped_kernel(const __grid_constant__ CUtensorMap tmap_a, const __
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
   if (threadIdx.x == 0) SACQ_GTR(0, 1);
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      for (int kb = 0; kb < num_kb; ++kb) {
-        if (kb % KB_PER_SB == 0) {
-          const int sb = kb / KB_PER_SB, slot = sb & 1;
-          if (!mbar_wait(bar(IDX_EMPTY + slot), ((sb >> 1) & 1) ^ 1, abort_flag, p.status)) break;
+    int st = 0;
+    uint32_t free_parity = 1;
+    for (int kb = 0; kb < num_kb; ++kb) {
+      if (kb % KB_PER_SB == 0) {
+        const int sb = kb / KB_PER_SB, slot = sb & 1;
+        if (!mbar_wait_warp(bar(IDX_EMPTY + slot), ((sb >> 1) & 1) ^ 1, abort_flag, p.status)) break;
+        if (elect_one()) {
           mbar_arrive_expect_tx(bar(IDX_FULL + slot), (uint32_t)(kRows * sb_bytes));
           for (int sl = 0; sl < p.bits; ++sl)          // one 16-byte column slice of the 128 rows per copy
             tma_load_2d(base + L.idx_off + slot * L.idx_slot + sl * (kRows * 16), &tmap_idx, sb * sb_bytes + sl * 16, n0,
                         bar(IDX_FULL + slot));
         }
-        const int st = kb % act_stages;
-        if (!mbar_wait(bar(ACT_EMPTY + st), ((kb / act_stages) & 1) ^ 1, abort_flag, p.status)) break;
+      }
+      if (!mbar_wait_warp(bar(ACT_EMPTY + st), free_parity, abort_flag, p.status)) break;
+      if (elect_one()) {
         mbar_arrive_expect_tx(bar(ACT_FULL + st), nt_valid * kTokTile);
 #pragma unroll
         for (int t = 0; t < NT; ++t)
@@ -186,45 +190,47 @@ large_m_tmem_grouped_kernel(const __grid_constant__ CUtensorMap tmap_a, const __
             tma_load_2d(base + L.act_off + st * L.act_stage + t * kTokTile, &tmap_a, kb * 128, m0 + t * kBM,
                         bar(ACT_FULL + st));
       }
+      if (++st == act_stages) { st = 0; free_parity ^= 1; }
     }
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      bool ok = true;
-      for (int wi = 0; wi < num_kb / 2 && ok; ++wi) {         // weight stage by weight stage: two K blocks each
-        const int ws = wi % kGWStages;
-        ok = mbar_wait(bar(W_FULL + ws), (wi / kGWStages) & 1, abort_flag, p.status);
+    bool ok = true;
+    int st = 0, ws = 0;
+    uint32_t act_parity = 0, w_parity = 0;
+    for (int wi = 0; wi < num_kb / 2 && ok; ++wi) {           // weight stage by weight stage: two K blocks each
+      ok = mbar_wait_warp(bar(W_FULL + ws), w_parity, abort_flag, p.status);
 #pragma unroll
-        for (int sub = 0; sub < 2 && ok; ++sub) {
-          const int kb = 2 * wi + sub, st = kb % act_stages;
-          ok = mbar_wait(bar(ACT_FULL + st), (kb / act_stages) & 1, abort_flag, p.status);
-          if (!ok) break;
-          if (sub == 0) tc_fence_after();
-          SACQ_GTR(1, kb + 8);
-          const uint32_t act_addr = base + L.act_off + st * L.act_stage;
-          const uint32_t w_col = kWCol0 + (uint32_t)(ws * 64 + sub * 32);
+      for (int sub = 0; sub < 2; ++sub) {
+        ok = ok && mbar_wait_warp(bar(ACT_FULL + st), act_parity, abort_flag, p.status);
+        if (!ok) break;
+        tc_fence_after();
+        if (lane == 0) SACQ_GTR(1, 2 * wi + sub + 8);
+        const uint32_t act_addr = base + L.act_off + st * L.act_stage;
+        const uint32_t w_col = tmem_base + kWCol0 + (uint32_t)(ws * 64 + sub * 32);
 #pragma unroll
-          for (int ks = 0; ks < kBKh / 16; ++ks) {
-            const uint64_t adv = (uint64_t)((ks * 32) >> 4);              // 16 fp16 = 32 bytes per K step
-            const uint32_t a_tmem = tmem_base + w_col + (uint32_t)(ks * 8);
-            const uint32_t acc = (kb | ks) != 0;
-            if (NT == 3 && nt_valid == 3) {
-              // two N = 192 instructions into two accumulators (an instruction costs about 60 ns whatever its N)
-              umma_f16_ts(tmem_base, a_tmem, make_smem_desc(act_addr) + adv, kIdesc192, acc);
+        for (int ks = 0; ks < kBKh / 16; ++ks) {
+          const uint64_t adv = (uint64_t)((ks * 32) >> 4);              // 16 fp16 = 32 bytes per K step
+          const uint32_t a_tmem = w_col + (uint32_t)(ks * 8);
+          const uint32_t acc = (wi | sub | ks) != 0;
+          if (NT == 3 && nt_valid == 3) {
+            // an instruction takes at most 256 tokens: 384 go as two N = 192
+            if (elect_one()) umma_f16_ts(tmem_base, a_tmem, make_smem_desc(act_addr) + adv, kIdesc192, acc);
+            if (elect_one())
               umma_f16_ts(tmem_base + 192u, a_tmem, make_smem_desc(act_addr + kTokTile * 3 / 2) + adv, kIdesc192, acc);
-            } else if (NT >= 2 && nt_valid >= 2) {
-              umma_f16_ts(tmem_base, a_tmem, make_smem_desc(act_addr) + adv, kIdesc256, acc);
-            } else {
-              umma_f16_ts(tmem_base, a_tmem, make_smem_desc(act_addr) + adv, kIdesc128, acc);
-            }
+          } else if (NT >= 2 && nt_valid >= 2) {
+            if (elect_one()) umma_f16_ts(tmem_base, a_tmem, make_smem_desc(act_addr) + adv, kIdesc256, acc);
+          } else {
+            if (elect_one()) umma_f16_ts(tmem_base, a_tmem, make_smem_desc(act_addr) + adv, kIdesc128, acc);
           }
-          umma_commit(bar(ACT_EMPTY + st));
         }
-        if (ok) umma_commit(bar(W_EMPTY + ws));
+        if (elect_one()) umma_commit(bar(ACT_EMPTY + st));
+        if (++st == act_stages) { st = 0; act_parity ^= 1; }
       }
-      if (ok) umma_commit(bar(ACC_FULL));
+      if (ok && elect_one()) umma_commit(bar(W_EMPTY + ws));
+      if (++ws == kGWStages) { ws = 0; w_parity ^= 1; }
     }
+    if (ok && elect_one()) umma_commit(bar(ACC_FULL));
     __syncwarp();
   } else {
     // ------------------------------------------------------------------ expanders, then epilogue
@@ -352,35 +358,6 @@ large_m_tmem_grouped_kernel(const __grid_constant__ CUtensorMap tmap_a, const __
   if (warp == 1) tmem_dealloc(tmem_base, kTmemCols);
 }
 
-// e4m3 (or int8, I8) [M, K] -> fp16 [M, K] (exact); one CTA per token row.
-template <bool I8>
-__global__ void __launch_bounds__(256) widen_act_f16_kernel(const uint8_t* __restrict__ q, int64_t K,
-                                                            __half* __restrict__ a16) {
-  const int64_t m = blockIdx.x;
-  const uint2* src = reinterpret_cast<const uint2*>(q + m * K);
-  uint4* dst = reinterpret_cast<uint4*>(a16 + m * K);
-  for (int64_t i = threadIdx.x; i < (K >> 3); i += blockDim.x) {
-    const uint2 v = __ldg(src + i);
-    uint32_t w[4];
-    const uint32_t in[2] = {v.x, v.y};
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      if constexpr (I8) {
-        const __half2 a = __halves2half2(__int2half_rn((int)(int8_t)(in[j] & 0xff)), __int2half_rn((int)(int8_t)((in[j] >> 8) & 0xff)));
-        const __half2 b = __halves2half2(__int2half_rn((int)(int8_t)((in[j] >> 16) & 0xff)), __int2half_rn((int)(int8_t)(in[j] >> 24)));
-        w[2 * j] = *reinterpret_cast<const uint32_t*>(&a);
-        w[2 * j + 1] = *reinterpret_cast<const uint32_t*>(&b);
-      } else {
-        const __half2_raw a = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(in[j] & 0xffff), __NV_E4M3);
-        const __half2_raw b = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(in[j] >> 16), __NV_E4M3);
-        w[2 * j] = (uint32_t)a.x | ((uint32_t)a.y << 16);
-        w[2 * j + 1] = (uint32_t)b.x | ((uint32_t)b.y << 16);
-      }
-    }
-    dst[i] = make_uint4(w[0], w[1], w[2], w[3]);
-  }
-}
-
 constexpr int64_t kGSlabTokens = 3072;   // tokens widened per launch (8 tiles of 384): bounds the fp16 scratch
 
 int g_act_stages(const sacq_layer* L, int nt) {
@@ -416,6 +393,8 @@ cudaError_t glaunch_d(const CUtensorMap& ta, const CUtensorMap& ti, const CUtens
 
 }  // namespace
 
+int64_t large_m_tmem_grouped_slab(void) { return kGSlabTokens; }
+
 bool large_m_tmem_grouped_supported(const sacq_layer* L) {
   const sacq_layer_desc& d = L->d;
   if (d.vector_dim != 8 && d.vector_dim != 4) return false;
@@ -427,11 +406,12 @@ bool large_m_tmem_grouped_supported(const sacq_layer* L) {
   return g_act_stages(L, 1) >= 2;
 }
 
-// From how many tokens this kernel beats the shared-memory-tile kernel of linear_large_m_grouped.cu
-// (measured at d = 4, 10-bit, group 64: 2048x6144 27.6 against 33.1 us at M = 300 and 37 against 66 us
-// at M = 1024; 2048x2048 and 6144x2048 break even at M = 1024 and win 1.5-1.9x from M = 4096).
+// From how many tokens this kernel beats the split-K kernel (linear_large_m_grouped.cu), whose clusters stop
+// paying once whole token tiles fill the device (quantizer + GEMM at d = 4, 10-bit, group 64: 2048x6144
+// 28.5 / 25.8 us at 512 tokens, 24.3 / 18.9 the other way round at 300; 1024x4096 18.9 / 17.2 at 768; 2048x2048
+// 23.8 / 24.7 at 1,000 and 36.5 / 28.1 at 1,500; 6144x2048 47.5 / 54.4 and 71.7 / 62.2).
 int64_t large_m_tmem_grouped_min_m(const sacq_layer* L) {
-  return L->d.out_features >= 5120 ? 288 : 1024;
+  return L->d.out_features >= 5120 ? 448 : L->d.out_features >= 4096 ? 704 : 1024;
 }
 
 // Workspace behind the counter region: the fp16 activations of one token slab.
@@ -442,7 +422,7 @@ int64_t large_m_tmem_grouped_workspace_bytes(const sacq_layer* L, int64_t M) {
 
 int launch_large_m_tmem_grouped(const sacq_layer* L, const void* q, const float* scale, int64_t M, void* y, int64_t ldy,
                                 void* ws, int64_t ws_bytes, cudaStream_t s, const void* residual, int64_t ldr,
-                                int act_int8, const BcastDst* bc, int nt_force) {
+                                ActForm form, const BcastDst* bc, int nt_force) {
   const sacq_layer_desc& d = L->d;
   if (!large_m_tmem_grouped_supported(L))
     return set_error(SACQ_ERR_UNSUPPORTED, "grouped TMEM-weight kernel cannot run this layer geometry");
@@ -450,14 +430,14 @@ int launch_large_m_tmem_grouped(const sacq_layer* L, const void* q, const float*
   if (reinterpret_cast<uintptr_t>(q) % 8 != 0)
     return set_error(SACQ_ERR_ALIGNMENT, "quantized activations must be 8-byte aligned");
   const int64_t need = large_m_tmem_grouped_workspace_bytes(L, M);
-  if (ws == nullptr || ws_bytes < need)
+  if (form == kActHalf ? M > kGSlabTokens : ws == nullptr || ws_bytes < need)
     return set_error(SACQ_ERR_WORKSPACE, "workspace of %lld bytes needed behind the counter region, %lld given",
                      (long long)need, (long long)ws_bytes);
-  if (reinterpret_cast<uintptr_t>(ws) % 256 != 0)
+  if (form != kActHalf && reinterpret_cast<uintptr_t>(ws) % 256 != 0)
     return set_error(SACQ_ERR_ALIGNMENT, "workspace must be 256-byte aligned");
   const int64_t K = d.in_features, N = d.out_features;
   const int64_t slab = M < kGSlabTokens ? M : kGSlabTokens;
-  __half* a16 = static_cast<__half*>(ws);
+  const void* a16 = form == kActHalf ? q : ws;
 
   GTmemParams p{};
   p.cb_f16 = L->cb_f16;
@@ -476,12 +456,8 @@ int launch_large_m_tmem_grouped(const sacq_layer* L, const void* q, const float*
   const int64_t row_tiles = (N + kRows - 1) / kRows;
   for (int64_t m0 = 0; m0 < M; m0 += slab) {
     const int64_t rows = (M - m0) < slab ? (M - m0) : slab;
-    if (act_int8)
-      widen_act_f16_kernel<true><<<(unsigned)rows, 256, 0, s>>>(static_cast<const uint8_t*>(q) + m0 * K, K, a16);
-    else
-      widen_act_f16_kernel<false><<<(unsigned)rows, 256, 0, s>>>(static_cast<const uint8_t*>(q) + m0 * K, K, a16);
-    count_launch();
-    SACQ_CUDA_TRY(cudaGetLastError());
+    if (form != kActHalf)
+      if (int rc = launch_widen(static_cast<const uint8_t*>(q) + m0 * K, rows, K, form == kActInt8, ws, s)) return rc;
     // token sub-tiles per CTA: the largest tile that does not add a wave
     int nt = nt_force;
     if (nt < 1 || nt > 3) {

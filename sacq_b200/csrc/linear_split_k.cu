@@ -1,0 +1,862 @@
+// Quantized linear for a few dozen to a few hundred tokens (sm_100a): tensor-memory weights, the K
+// dimension split over a thread-block cluster.
+//   y[m,n] = bf16( s[m] * (sum_k q[m,k] * W[n,k]) + bias[n] )
+//
+// What bounds these sizes is neither bandwidth nor the tensor pipe but how often a weight is expanded
+// and how many SMs share the expansion: a codeword gather costs a fixed share of an SM's shared-memory
+// rate (3 gathers per clock), so every token tile that expands the layer again costs the whole layer
+// again, and a tile of 128 weight rows x all tokens leaves most SMs without work (2,048 rows are 16
+// tiles).  Here a CTA takes 128 weight rows x ALL tokens (up to 384) x one slice of K, so each weight is
+// expanded once on the whole device, and the S CTAs of a cluster that share an output tile add their
+// fp32 partial sums through distributed shared memory:
+//   * warp 0        TMA producer: the slice's packed indices ([slice][row][16 bytes]: conflict-free
+//                   reads whatever the index width), the codebook, then the activation tiles;
+//   * warp 1        MMA issuer: tcgen05.mma with the weights as the A operand in tensor memory, N = tokens;
+//   * warps 2..17   expanders: one weight row and a quarter of every 128-k stage each: index fields ->
+//                   codeword gathers -> tcgen05.st.  kSplitHiLo: the e4m3 high and low halves of the
+//                   codewords against e4m3 activations (kind::f8f6f4), one scale per row in the epilogue.
+//                   kSplitHalf: fp16(codeword x group scale) against activations widened to fp16
+//                   (kind::f16): grouped scales, and INT8 activations on any layer.  kSplitInt8 / kSplitFp8:
+//                   the 8-bit weight bytes of the two recipes, made here instead of in a pass of their own
+//                   over a 1-byte copy of the weights;
+//   * reduction     every CTA puts its fp32 partial sums into its own shared memory, [token][row]; after a
+//                   cluster barrier each owns a token range of the tile, reads that range from its S - 1
+//                   peers (16 bytes per lane), adds the slices pairwise and writes y.
+// A CTA may take several slices, each with accumulator columns of its own: the order in which an output is
+// summed stays the same when many tokens leave no use for a cluster.
+// Every mbarrier wait is bounded (status word + CTA-wide abort flag); an aborted CTA still reaches both
+// cluster barriers, so its peers do too.  No cluster multicast.
+#include <cuda.h>
+#include <math.h>
+#include <stdio.h>
+#include <stdlib.h>
+#include <string.h>
+
+#include <mutex>
+#include <type_traits>
+
+#include "common.cuh"
+#include "encode.cuh"
+#include "split_k.cuh"
+#include "tmem_weights.cuh"
+#include "umma.cuh"
+
+namespace sacq {
+
+namespace {
+
+using namespace umma;
+using namespace tmemw;
+
+constexpr int kStageK = 128;          // k per weight stage
+constexpr int kMaxAct = 6;            // activation tiles in flight (128 bytes of every token each)
+constexpr int kMaxW = 4;              // weight stages in tensor memory
+constexpr int kMaxTok = 384;          // tokens per CTA
+constexpr int kSliceBytes = kRows * 16;
+constexpr float kHalfPreScale = 4096.f;   // keeps fp16(codeword x scale) far from the subnormals
+
+struct SplitLayer {
+  const uint8_t* cb;            // kSplitHiLo: e4m3 [C][2][D]; kSplitHalf: fp16 [C][D]; recipes: bf16 [C][D]
+  const uint16_t* scales;       // bf16 [N, num_groups]
+  const uint16_t* bias;         // bf16 [N] or null
+  uint16_t* y;                  // bf16 [M, ldy]
+  int64_t ldy;
+  int* status;
+  int N;
+  float scale_mul;              // kSplitHalf: power of two applied to every scale before it is rounded to fp16
+  float out_mul;                // power of two that undoes the operands' scaling
+};
+
+struct alignas(64) SplitParams {
+  CUtensorMap idx[kSplitMaxLayers];     // [16 bytes][128 rows][max_slices] boxes over the packed rows
+  SplitLayer layer[kSplitMaxLayers];
+  const float* act_scale;       // [M]
+  const float* row_scale;       // recipes: [N], the weight bytes' scale
+  uint16_t shift;               // recipes: bf16 bits
+  const uint16_t* residual;     // bf16 [M, ldr] added to the rounded output, or null
+  int64_t ldr;
+  int n_bc;                     // further copies of the output (peer GPUs' buffers), same pitch as y
+  uint16_t* ybc[kMaxBcast];
+  int M, K, C, bits, num_groups, group_size;
+  int split;                    // CTAs per cluster
+  int parts;                    // consecutive slices of K per CTA, each with accumulator columns of its own
+  int tok;                      // tokens per CTA (multiple of 16; of 32 above 256)
+  int act_stages, max_slices, max_groups;
+};
+
+struct SplitLayout {
+  uint32_t idx_off, cb_off, sc_off, fixed_off, sa_off, sw_off, bias_off, bar_off, misc_off, total;
+};
+
+// tokens of the tile a rank reduces and writes
+__host__ __device__ constexpr int owned_tokens(int tok, int split) { return ((tok + split - 1) / split + 7) & ~7; }
+
+__host__ __device__ inline SplitLayout split_layout(int tok, int split, int act_stages, int slices, int groups, int cb_bytes) {
+  SplitLayout L;
+  L.idx_off = (uint32_t)(act_stages * tok * 128);
+  L.cb_off = L.idx_off + (uint32_t)(slices * kSliceBytes);
+  L.sc_off = L.cb_off + (uint32_t)((cb_bytes + 127) & ~127);
+  const uint32_t pipe = L.sc_off + (uint32_t)((groups > 0 ? kRows * (groups | 1) * 2 + 127 : 0) & ~127);
+  // the partial sums of the reduction take the place of everything the main loop is done with
+  const uint32_t recv = (uint32_t)(tok * kRows * 4);
+  L.fixed_off = pipe > recv ? pipe : recv;
+  L.sa_off = L.fixed_off;
+  L.sw_off = L.sa_off + (uint32_t)(tok * 4);
+  L.bias_off = L.sw_off + kRows * 4;
+  L.bar_off = L.bias_off + kRows * 4;
+  L.misc_off = L.bar_off + 32 * 8;
+  L.total = L.misc_off + 64;
+  return L;
+}
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t peer_address(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ uint4 load_peer(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+      ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// 16 accumulator columns of the warp's lane quarter.
+__device__ __forceinline__ void tmem_ld_16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+
+// a + b of two partial sums held as bits: fp32, or int32 (INT, exact).
+template <bool INT>
+__device__ __forceinline__ uint32_t add_bits(uint32_t a, uint32_t b) {
+  return INT ? a + b : __float_as_uint(__uint_as_float(a) + __uint_as_float(b));
+}
+template <bool INT>
+__device__ __forceinline__ uint4 add_bits4(const uint4& a, const uint4& b) {
+  return make_uint4(add_bits<INT>(a.x, b.x), add_bits<INT>(a.y, b.y), add_bits<INT>(a.z, b.z), add_bits<INT>(a.w, b.w));
+}
+// r += 16 accumulator columns.
+template <bool INT>
+__device__ __forceinline__ void add_columns(uint32_t (&r)[16], uint32_t taddr) {
+  uint32_t b[16];
+  tmem_ld_16(taddr, b);
+#pragma unroll
+  for (int j = 0; j < 16; ++j) r[j] = add_bits<INT>(r[j], b[j]);
+}
+
+// A window of up to 64 bits at bit `bit` of a row whose 16-byte slices lie kSliceBytes apart; `bit` is
+// warp-uniform, `need` bits of it are used (a slice is only read if one of them lies in it).
+__device__ __forceinline__ uint64_t slice_window(const uint8_t* row_slices, int bit, int need) {
+  const uint8_t* s0 = row_slices + (bit >> 7) * kSliceBytes;
+  const uint4 a = *reinterpret_cast<const uint4*>(s0);
+  uint4 b = a;
+  if ((bit & 127) + need > 128) b = *reinterpret_cast<const uint4*>(s0 + kSliceBytes);
+  uint32_t lo, mid, hi;
+  switch ((bit >> 5) & 3) {
+    case 0: lo = a.x; mid = a.y; hi = a.z; break;
+    case 1: lo = a.y; mid = a.z; hi = a.w; break;
+    case 2: lo = a.z; mid = a.w; hi = b.x; break;
+    default: lo = a.w; mid = b.x; hi = b.y; break;
+  }
+  const uint32_t sh = (uint32_t)(bit & 31);
+  return ((uint64_t)__funnelshift_r(mid, hi, sh) << 32) | __funnelshift_r(lo, mid, sh);
+}
+
+// Adds the slices of K pairwise, (0 + 1) + (2 + 3) and so on, whichever CTA does it, and writes y: tokens [0, count) of this CTA's share,
+// a warp per token, four consecutive outputs per lane.  `part` = this lane's partial sums of token 0 in the
+// CTA's own shared memory.  Everything that does not depend on the token is set up once: this loop is bound by
+// instruction issue (with the addresses and alignment tests inside it took 0.4 us per token and warp).
+template <int S, bool INT>
+__device__ __forceinline__ void reduce_tokens(const SplitParams& p, const SplitLayer& lay, int warp, int lane, int count,
+                                              int m_first, int n0, uint32_t part, const float* sa, float4 sw, float4 bs) {
+  const int n = n0 + lane * 4;
+  const int valid = min(4, lay.N - n);
+  if (valid <= 0) return;
+  uint32_t src[S];
+#pragma unroll
+  for (int s = 0; s < S; ++s) src[s] = S == 1 ? part : peer_address(part, (uint32_t)s);
+  uint16_t* y = lay.y + (int64_t)m_first * lay.ldy + n;
+  const int64_t ldy = lay.ldy;
+  const uint16_t* res = p.residual ? p.residual + (int64_t)m_first * p.ldr + n : nullptr;
+  const int64_t ldr = p.ldr;
+  const bool vec_y = valid == 4 && (reinterpret_cast<uintptr_t>(y) & 7) == 0 && (ldy & 3) == 0;
+  const bool vec_r = valid == 4 && (reinterpret_cast<uintptr_t>(res) & 7) == 0 && (ldr & 3) == 0;
+  const bool plain = vec_y && (res == nullptr || vec_r) && p.n_bc == 0;
+  const uint2 none = make_uint2(0u, 0u);
+  const bool has_bias = lay.bias != nullptr;
+#pragma unroll 2
+  for (int t = warp; t < count; t += kXWarps) {
+    uint4 v[S];
+#pragma unroll
+    for (int s = 0; s < S; ++s) v[s] = load_peer(src[s] + (uint32_t)(t * (kRows * 4)));
+#pragma unroll
+    for (int w = 1; w < S; w *= 2)
+#pragma unroll
+      for (int s = 0; s + w < S; s += 2 * w) v[s] = add_bits4<INT>(v[s], v[s + w]);
+    const float sc = sa[t];
+    auto fin = [&](uint32_t a, float w, float b) {
+      const float x = __fmul_rn(INT ? __int2float_rn((int)a) : __uint_as_float(a), w);
+      return has_bias ? fmaf(sc, x, b) : __fmul_rn(sc, x);
+    };
+    const float o0 = fin(v[0].x, sw.x, bs.x), o1 = fin(v[0].y, sw.y, bs.y), o2 = fin(v[0].z, sw.z, bs.z),
+                o3 = fin(v[0].w, sw.w, bs.w);
+    __nv_bfloat162 lo = __floats2bfloat162_rn(o0, o1), hi = __floats2bfloat162_rn(o2, o3);
+    // bf16(bf16(v) + residual): the two roundings of `linear(x) + residual`
+    auto add = [](__nv_bfloat162 o, uint32_t r) {
+      const uint32_t b = *reinterpret_cast<const uint32_t*>(&o);
+      return __floats2bfloat162_rn(__fadd_rn(__uint_as_float(b << 16), __uint_as_float(r << 16)),
+                                   __fadd_rn(__uint_as_float(b & 0xffff0000u), __uint_as_float(r & 0xffff0000u)));
+    };
+    if (plain) {
+      if (res != nullptr) {
+        const uint2 r = __ldg(reinterpret_cast<const uint2*>(res + t * ldr));
+        lo = add(lo, r.x);
+        hi = add(hi, r.y);
+      }
+      *reinterpret_cast<uint2*>(y + t * ldy) =
+          make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+      continue;
+    }
+    if (res != nullptr) {
+      uint2 r = none;
+      const uint16_t* rp = res + t * ldr;
+      r.x = __ldg(rp);
+      if (valid > 1) r.x |= (uint32_t)__ldg(rp + 1) << 16;
+      if (valid > 2) r.y = __ldg(rp + 2);
+      if (valid > 3) r.y |= (uint32_t)__ldg(rp + 3) << 16;
+      lo = add(lo, r.x);
+      hi = add(hi, r.y);
+    }
+    const uint32_t w0 = *reinterpret_cast<const uint32_t*>(&lo), w1 = *reinterpret_cast<const uint32_t*>(&hi);
+    for (int c = -1; c < p.n_bc; ++c) {
+      uint16_t* out = c < 0 ? y + t * ldy : p.ybc[c] + (int64_t)(m_first + t) * ldy + n;
+      if (valid == 4 && (reinterpret_cast<uintptr_t>(out) & 7) == 0) {
+        *reinterpret_cast<uint2*>(out) = make_uint2(w0, w1);
+      } else {
+        out[0] = (uint16_t)w0;
+        if (valid > 1) out[1] = (uint16_t)(w0 >> 16);
+        if (valid > 2) out[2] = (uint16_t)w1;
+        if (valid > 3) out[3] = (uint16_t)(w1 >> 16);
+      }
+    }
+  }
+}
+
+#ifdef SACQ_TRACE
+// Profiling builds only (-DSACQ_TRACE): CTA (0, 0, 0) records %globaltimer at a few points.
+__device__ long long g_split_trace[64];
+#define SACQ_SPT(slot) do { if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && (slot) < 64) { long long _t; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(_t)); g_split_trace[slot] = _t; } } while (0)
+#else
+#define SACQ_SPT(slot) do { } while (0)
+#endif
+
+// grid = (row tiles x split, token tiles, layers), clusters of `split` CTAs along x.
+template <int D, int MODE>
+__global__ void __launch_bounds__(kCtaThreads, 1)
+split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ SplitParams p) {
+  constexpr uint32_t kTmemCols = 512;
+  constexpr int CW_BYTES = 2 * D;
+  constexpr bool F16 = MODE == kSplitHalf, RECIPE = MODE >= kSplitInt8, INT = MODE == kSplitInt8;
+  constexpr int TILES = F16 ? 2 : 1;                  // activation tiles (128 bytes of every token) per weight stage
+  constexpr int W_COLS = RECIPE ? 32 : 64;            // TMEM columns of a weight stage
+  const int S = p.split;
+  const int n0 = ((int)blockIdx.x / S) * kRows;
+  const SplitLayer& lay = p.layer[blockIdx.z];
+  if (n0 >= lay.N) return;                            // a narrower sibling: uniform over the cluster
+  if (threadIdx.x == 0) SACQ_SPT(0);
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw = smem_u32(smem_raw);
+  const uint32_t base = (raw + 1023u) & ~1023u;
+  uint8_t* sm = smem_raw + (base - raw);
+  const uint32_t cb_bytes = (uint32_t)(p.C * CW_BYTES);
+  const SplitLayout L = split_layout(p.tok, S, p.act_stages, p.max_slices, F16 || RECIPE ? p.max_groups : 0, (int)cb_bytes);
+
+  constexpr int ACT_FULL = 0, ACT_EMPTY = kMaxAct, W_FULL = 2 * kMaxAct, W_EMPTY = W_FULL + kMaxW, IDX_FULL = W_EMPTY + kMaxW,
+                CB_FULL = IDX_FULL + 1, ACC_FULL = IDX_FULL + 2;
+  static_assert(ACC_FULL < 32, "barrier region");
+  const uint32_t bars = base + L.bar_off;
+  auto bar = [&](int i) { return bars + 8u * i; };
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + L.misc_off);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + L.misc_off + 8);
+
+  const int warp = (int)warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int rank = S > 1 ? (int)cluster_rank() : 0;
+  const int m0 = blockIdx.y * p.tok;
+  const int nkb = p.K / kStageK;
+  const int parts = p.parts, slices = S * parts;
+  // this CTA's weight stages, and the first one (counted from kb0) of its slice `v`
+  const int kb0 = rank * parts * nkb / slices, kbs = (rank + 1) * parts * nkb / slices - kb0;
+  auto part_begin = [&](int v) { return (rank * parts + v) * nkb / slices - kb0; };
+  const int tok = p.tok, acc_cols = tok * parts;
+  const bool halves = tok > 256;                      // an instruction (and a TMA box) takes at most 256 tokens
+  const int w_stages = min(kMaxW, ((int)kTmemCols - acc_cols) / W_COLS);
+  const int act_stages = p.act_stages;
+  const int bit_begin = (kb0 * kStageK / D) * p.bits;
+  const int slice0 = bit_begin >> 7;
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kMaxAct; ++i) {
+      mbar_init(bar(ACT_FULL + i), 1);
+      mbar_init(bar(ACT_EMPTY + i), 1);
+    }
+    for (int i = 0; i < kMaxW; ++i) {
+      mbar_init(bar(W_FULL + i), kXWarps);
+      mbar_init(bar(W_EMPTY + i), 1);
+    }
+    mbar_init(bar(IDX_FULL), 1);
+    mbar_init(bar(CB_FULL), 1);
+    mbar_init(bar(ACC_FULL), 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    fence_proxy_async();
+  }
+  if (warp == 0) {
+    __syncwarp();
+    // constant operands: their copies start before anything else
+    if (elect_one()) {
+      mbar_arrive_expect_tx(bar(IDX_FULL), (uint32_t)(p.max_slices * kSliceBytes));
+      tma_load_3d(base + L.idx_off, &p.idx[blockIdx.z], 0, n0, slice0, bar(IDX_FULL));
+      mbar_arrive_expect_tx(bar(CB_FULL), cb_bytes);
+      bulk_load(base + L.cb_off, lay.cb, cb_bytes, bar(CB_FULL));
+      prefetch_tensormap(&tmap_a);
+    }
+  }
+  if (warp == 1) tmem_alloc(smem_u32(tmem_slot), kTmemCols);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
+  if (threadIdx.x == 0) SACQ_SPT(1);
+
+  bool ok = true;
+  if (warp == 0) {
+    // ------------------------------------------------------------------ activation tiles, token scales
+    asm volatile("griddepcontrol.wait;" ::: "memory");   // q and the scales come from the kernel in front
+    if (lane == 0) SACQ_SPT(2);
+    float sa[kMaxTok / 32];                           // the token scales: fetched now, put down behind the last copy
+#pragma unroll
+    for (int i = 0; i < kMaxTok / 32; ++i) {
+      const int t = i * 32 + lane;
+      sa[i] = t < tok && m0 + t < p.M ? __ldg(p.act_scale + m0 + t) : 0.f;
+    }
+    int st = 0;
+    uint32_t free_parity = 1;
+    for (int i = 0; i < kbs * TILES; ++i) {
+      if (!mbar_wait_warp(bar(ACT_EMPTY + st), free_parity, abort_flag, lay.status)) break;
+      const uint32_t dst = base + (uint32_t)(st * tok * 128);
+      const int x = (kb0 * TILES + i) * 128;
+      if (elect_one()) {
+        mbar_arrive_expect_tx(bar(ACT_FULL + st), (uint32_t)(tok * 128));
+        tma_load_2d(dst, &tmap_a, x, m0, bar(ACT_FULL + st));
+        if (halves) tma_load_2d(dst + (uint32_t)(tok / 2 * 128), &tmap_a, x, m0 + tok / 2, bar(ACT_FULL + st));
+      }
+      if (++st == act_stages) { st = 0; free_parity ^= 1; }
+    }
+#pragma unroll
+    for (int i = 0; i < kMaxTok / 32; ++i)
+      if (i * 32 + lane < tok) reinterpret_cast<float*>(sm + L.sa_off)[i * 32 + lane] = sa[i];
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer
+    const uint32_t idesc = INT ? make_idesc_i8(halves ? tok / 2 : tok) : make_idesc(halves ? tok / 2 : tok);
+    int st = 0, ws = 0;
+    uint32_t act_parity = 0, w_parity = 0;
+    int part = -1, next_part = 0, begin = 0;          // slice of K, the stage at which the next one begins
+    for (int wi = 0; wi < kbs && ok; ++wi) {
+      if (wi == next_part) {
+        begin = wi;
+        next_part = ++part + 1 < parts ? part_begin(part + 1) : kbs;
+      }
+      ok = mbar_wait_warp(bar(W_FULL + ws), w_parity, abort_flag, lay.status);
+      const uint32_t w_col = tmem_base + (uint32_t)(acc_cols + ws * W_COLS);
+      const uint32_t d_col = tmem_base + (uint32_t)(part * tok);
+#pragma unroll
+      for (int sub = 0; sub < TILES; ++sub) {
+        ok = ok && mbar_wait_warp(bar(ACT_FULL + st), act_parity, abort_flag, lay.status);
+        if (!ok) break;
+        tc_fence_after();
+        if (lane == 0) SACQ_SPT(16 + wi * TILES + sub);
+        const uint32_t act = base + (uint32_t)(st * tok * 128);
+        const uint64_t b0 = make_smem_desc(act);
+        const uint64_t b1 = make_smem_desc(act + (uint32_t)(tok / 2 * 128));
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) {              // 32 bytes of every token per step
+#pragma unroll
+          for (int h = 0; h < (MODE == kSplitHiLo ? 2 : 1); ++h) {       // high and low halves of the codewords
+            const uint32_t a = w_col + (F16 ? (uint32_t)(sub * 32 + ks * 8) : (uint32_t)(h * 32 + ks * 8));
+            const uint32_t acc = (uint32_t)(((wi - begin) | sub | ks | h) != 0);
+            const uint64_t adv = (uint64_t)(ks * 2);
+            if (elect_one()) {
+              if constexpr (F16) umma_f16_ts(d_col, a, b0 + adv, idesc, acc);
+              else if constexpr (INT) umma_i8_ts(d_col, a, b0 + adv, idesc, acc);
+              else umma_f8_ts(d_col, a, b0 + adv, idesc, acc);
+            }
+            if (halves && elect_one()) {
+              if constexpr (F16) umma_f16_ts(d_col + (uint32_t)(tok / 2), a, b1 + adv, idesc, acc);
+              else if constexpr (INT) umma_i8_ts(d_col + (uint32_t)(tok / 2), a, b1 + adv, idesc, acc);
+              else umma_f8_ts(d_col + (uint32_t)(tok / 2), a, b1 + adv, idesc, acc);
+            }
+          }
+        }
+        if (elect_one()) umma_commit(bar(ACT_EMPTY + st));
+        if (++st == act_stages) { st = 0; act_parity ^= 1; }
+      }
+      if (ok && elect_one()) umma_commit(bar(W_EMPTY + ws));
+      if (++ws == w_stages) { ws = 0; w_parity ^= 1; }
+    }
+    if (ok && elect_one()) umma_commit(bar(ACC_FULL));
+    __syncwarp();
+  } else {
+    // ------------------------------------------------------------------ expanders
+    const int et = threadIdx.x - 64;
+    const int quarter = warp & 3;                     // TMEM lane quarter this warp may access
+    const int row = quarter * 32 + lane;
+    const int kpart = (warp - 2) >> 2;                // which quarter of a stage's 128 bytes (or of each 64-k tile)
+    const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
+    if (et < kRows) {
+      const int n = min(n0 + et, lay.N - 1);
+      reinterpret_cast<float*>(sm + L.sw_off)[et] =
+          RECIPE ? __ldg(p.row_scale + n) : F16 ? lay.out_mul : bf16_bits_to_float(__ldg(lay.scales + n)) * lay.out_mul;
+      reinterpret_cast<float*>(sm + L.bias_off)[et] = lay.bias ? bf16_bits_to_float(__ldg(lay.bias + n)) : 0.f;
+    }
+    constexpr bool GROUPS = F16 || RECIPE;             // scales enter the weight operand
+    const int g_first = GROUPS ? kb0 * kStageK / p.group_size : 0;
+    const int g_count = GROUPS ? ((kb0 + kbs) * kStageK - 1) / p.group_size - g_first + 1 : 0;
+    const int sc_pitch = g_count | 1;                 // odd: the 32 rows of a warp fall on different banks
+    uint16_t* sc = reinterpret_cast<uint16_t*>(sm + L.sc_off);
+    if constexpr (GROUPS) {
+      for (int i = et; i < kRows * g_count; i += kXThreads) {
+        const int r = i / g_count, g = i - r * g_count;
+        const int n = min(n0 + r, lay.N - 1);
+        sc[r * sc_pitch + g] = __ldg(lay.scales + (int64_t)n * p.num_groups + g_first + g);
+      }
+    }
+    xbarrier();
+    const uint8_t* cbs = sm + L.cb_off;
+    const uint8_t* rowidx = sm + L.idx_off + row * 16;
+    const uint32_t mask = (1u << p.bits) - 1u;
+    const int bits = p.bits;
+    ok = mbar_wait(bar(IDX_FULL), 0, abort_flag, lay.status) && mbar_wait(bar(CB_FULL), 0, abort_flag, lay.status);
+    if (et == 0) SACQ_SPT(3);
+    int grp = 0, grp_end = GROUPS ? (g_first + 1) * p.group_size - kb0 * kStageK : 0;    // k (in the slice) at which the scale changes
+    // One stage's 16 words of this thread.  The next stage's words are gathered before the wait for this
+    // stage's tcgen05.st: the gathers, which bound the loop, then never wait for a store's latency.
+    const RowWeights rw = row_weights(RECIPE ? __ldg(p.row_scale + min(n0 + row, lay.N - 1)) : 1.f);
+    const __nv_bfloat162 shift2 = __halves2bfloat162(__ushort_as_bfloat16(p.shift), __ushort_as_bfloat16(p.shift));
+    auto expand = [&](int wi, uint32_t (&w)[16]) {
+      if constexpr (RECIPE) {
+        // 32 weights of this thread's row, 16 at a time: bf16(bf16(c * s) + shift) divided by the row scale and
+        // encoded (the arithmetic of decode_rows_kernel in dequant.cu)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          constexpr int IPT = 16 / D;
+          const int k = wi * kStageK + kpart * 32 + h * 16;       // in the slice
+          const int g = p.num_groups == 1 ? 0 : (kb0 * kStageK + k) / p.group_size - g_first;
+          const __nv_bfloat16 s = __ushort_as_bfloat16(sc[row * sc_pitch + g]);
+          const uint64_t win = slice_window(rowidx, ((kb0 * kStageK + k) / D) * bits - slice0 * 128, IPT * bits);
+          uint32_t pair[8];
+#pragma unroll
+          for (int j = 0; j < IPT; ++j) {
+            const uint32_t i = (uint32_t)(win >> (j * bits)) & mask;
+            if constexpr (D == 8) {
+              const uint4 v = *reinterpret_cast<const uint4*>(cbs + i * 16);
+              pair[4 * j] = v.x; pair[4 * j + 1] = v.y; pair[4 * j + 2] = v.z; pair[4 * j + 3] = v.w;
+            } else {
+              const uint2 v = *reinterpret_cast<const uint2*>(cbs + i * 8);
+              pair[2 * j] = v.x; pair[2 * j + 1] = v.y;
+            }
+          }
+          encode_weights16<INT>(pair, __halves2bfloat162(s, s), shift2, rw, reinterpret_cast<uint32_t (&)[4]>(w[4 * h]));
+        }
+      } else if constexpr (F16) {
+        constexpr int IPT = 16 / D;                   // indices per thread and 64-k tile
+#pragma unroll
+        for (int sub = 0; sub < 2; ++sub) {
+          if (wi * kStageK + sub * 64 >= grp_end) { ++grp; grp_end += p.group_size; }
+          // scale x 2^e is a bf16 significand with a small exponent: exact in fp16
+          const __half2 s2 = __half2half2(__float2half_rn(bf16_bits_to_float(sc[row * sc_pitch + grp]) * lay.scale_mul));
+          const int bit = (((kb0 + wi) * kStageK + sub * 64 + kpart * 16) / D) * bits - slice0 * 128;
+          const uint64_t win = slice_window(rowidx, bit, IPT * bits);
+#pragma unroll
+          for (int j = 0; j < IPT; ++j) {
+            const uint32_t i = (uint32_t)(win >> (j * bits)) & mask;
+            uint32_t c[D / 2];
+            if constexpr (D == 8) {
+              const uint4 v = *reinterpret_cast<const uint4*>(cbs + i * 16);
+              c[0] = v.x; c[1] = v.y; c[2] = v.z; c[3] = v.w;
+            } else {
+              const uint2 v = *reinterpret_cast<const uint2*>(cbs + i * 8);
+              c[0] = v.x; c[1] = v.y;
+            }
+#pragma unroll
+            for (int e = 0; e < D / 2; ++e) {
+              const __half2 h = __hmul2(*reinterpret_cast<const __half2*>(&c[e]), s2);
+              w[sub * 8 + j * (D / 2) + e] = *reinterpret_cast<const uint32_t*>(&h);
+            }
+          }
+        }
+      } else {
+        const int bit = (((kb0 + wi) * kStageK + kpart * 32) / D) * bits - slice0 * 128;
+#pragma unroll
+        for (int v = 0; v < 8 / D; ++v) {             // four indices per window
+          const uint64_t win = slice_window(rowidx, bit + v * 4 * bits, 4 * bits);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const uint32_t i = (uint32_t)(win >> (j * bits)) & mask;
+            if constexpr (D == 8) {
+              const uint4 c = *reinterpret_cast<const uint4*>(cbs + i * 16);
+              w[2 * j] = c.x; w[2 * j + 1] = c.y;
+              w[8 + 2 * j] = c.z; w[8 + 2 * j + 1] = c.w;
+            } else {
+              const uint2 c = *reinterpret_cast<const uint2*>(cbs + i * 8);
+              w[4 * v + j] = c.x;
+              w[8 + 4 * v + j] = c.y;
+            }
+          }
+        }
+      }
+    };
+    int ws = 0;
+    uint32_t w_parity = 1;
+    uint32_t cur[16], nxt[16];
+    if (ok) expand(0, cur);
+    for (int wi = 0; wi < kbs && ok; ++wi) {
+      ok = mbar_wait(bar(W_EMPTY + ws), w_parity, abort_flag, lay.status);
+      if (!ok) break;
+      tc_fence_after();                               // the MMAs that read this stage are complete
+      // two quarters of the stage: high and low halves, or the two 64-k tiles
+      const uint32_t w_addr = lane_addr + (uint32_t)(acc_cols + ws * W_COLS + kpart * 8);
+      tmem_st_32x8(w_addr, reinterpret_cast<const uint32_t (&)[8]>(cur[0]));
+      if constexpr (!RECIPE) tmem_st_32x8(w_addr + 32u, reinterpret_cast<const uint32_t (&)[8]>(cur[8]));
+      if (wi + 1 < kbs) expand(wi + 1, nxt);
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(W_FULL + ws));
+      if (++ws == w_stages) { ws = 0; w_parity ^= 1; }
+#pragma unroll
+      for (int j = 0; j < (RECIPE ? 8 : 16); ++j) cur[j] = nxt[j];
+    }
+    if (et == 0) SACQ_SPT(4);
+    if (ok) ok = mbar_wait(bar(ACC_FULL), 0, abort_flag, lay.status);
+    if (et == 0) SACQ_SPT(5);
+    ok = __all_sync(0xffffffffu, ok);
+  }
+
+  // ---- reduction: the accumulators of the cluster's CTAs -> y.  Every thread takes part in the barriers.
+  if (warp >= 2 && ok) {
+    // [token][row] fp32, in the place of everything the main loop is done with (its last MMA has completed, so
+    // every stage has been written and read); a warp writes 128 consecutive bytes per token
+    const int quarter = warp & 3, row = quarter * 32 + lane, kpart = (warp - 2) >> 2;
+    tc_fence_after();
+    for (int c0 = kpart * 16; c0 < tok; c0 += 64) {
+      const uint32_t at = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0;
+      uint32_t r[16];
+      tmem_ld_16(at, r);
+      if (parts >= 2) add_columns<INT>(r, at + (uint32_t)tok);
+      if (parts == 4) {                               // (0 + 1) + (2 + 3), as the reduction over CTAs adds them
+        uint32_t r2[16];
+        tmem_ld_16(at + (uint32_t)(2 * tok), r2);
+        add_columns<INT>(r2, at + (uint32_t)(3 * tok));
+#pragma unroll
+        for (int j = 0; j < 16; ++j) r[j] = add_bits<INT>(r[j], r2[j]);
+      }
+      uint32_t* dst = reinterpret_cast<uint32_t*>(sm) + c0 * kRows + row;
+#pragma unroll
+      for (int j = 0; j < 16; ++j) dst[j * kRows] = r[j];
+    }
+    tc_fence_before();
+  }
+  if (threadIdx.x == 64) SACQ_SPT(6);
+  if (S > 1) cluster_sync();
+  else __syncthreads();
+  if (threadIdx.x == 64) SACQ_SPT(7);
+  if (warp >= 2 && ok) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int first = rank * owned_tokens(tok, S);    // the tokens this CTA writes
+    const int count = min(owned_tokens(tok, S), min(tok, p.M - m0) - first);
+    const float* sa = reinterpret_cast<const float*>(sm + L.sa_off) + first;
+    const float4 sw = reinterpret_cast<const float4*>(sm + L.sw_off)[lane];
+    const float4 bs = reinterpret_cast<const float4*>(sm + L.bias_off)[lane];
+    const uint32_t part = base + (uint32_t)(first * (kRows * 4) + lane * 16);
+    if (S == 1) reduce_tokens<1, INT>(p, lay, warp - 2, lane, count, m0 + first, n0, part, sa, sw, bs);
+    else if (S == 2) reduce_tokens<2, INT>(p, lay, warp - 2, lane, count, m0 + first, n0, part, sa, sw, bs);
+    else if (S == 8) reduce_tokens<8, INT>(p, lay, warp - 2, lane, count, m0 + first, n0, part, sa, sw, bs);
+    else reduce_tokens<4, INT>(p, lay, warp - 2, lane, count, m0 + first, n0, part, sa, sw, bs);
+  }
+
+  if (threadIdx.x == 64) SACQ_SPT(8);
+  // ---- common exit: a CTA's partial sums stay until its peers have read them
+  tc_fence_before();
+  if (S > 1) cluster_sync();
+  else __syncthreads();
+  if (threadIdx.x == 64) SACQ_SPT(9);
+  if (warp == 1) tmem_dealloc(tmem_base, kTmemCols);
+}
+
+}  // namespace
+
+#ifdef SACQ_TRACE
+extern "C" SACQ_API int sacq_debug_split_trace(long long* out) {
+  return cudaMemcpyFromSymbol(out, g_split_trace, sizeof(g_split_trace)) == cudaSuccess ? 0 : -1;
+}
+#endif
+
+struct SplitPlan {
+  static constexpr int kMaps = 8;
+  CUtensorMap idx[kMaps];       // one per slice count in use
+  int slices[kMaps];
+  int count;
+};
+
+namespace {
+
+std::mutex g_split_mutex;       // layers build their index maps on first use, possibly from several host threads
+
+// Boxes of [16 bytes][128 rows][slices] over the packed rows (dimensions: bytes of a 16-byte slice, rows, slices of
+// a row), so one copy brings a tile's index slices in the order the expanders read them.
+int slice_map(sacq_layer* L, int slices, CUtensorMap* out) {
+  std::lock_guard<std::mutex> lock(g_split_mutex);
+  if (L->split_plan == nullptr) L->split_plan = new SplitPlan();
+  SplitPlan* plan = L->split_plan;
+  for (int i = 0; i < plan->count; ++i)
+    if (plan->slices[i] == slices) {
+      *out = plan->idx[i];
+      return SACQ_OK;
+    }
+  const uint64_t row_bytes = (uint64_t)(L->row_bits / 8);
+  const int rc = encode_bytes_3d(out, L->d.packed, 16, (uint64_t)L->d.out_features, row_bytes / 16, row_bytes, 16, 16u,
+                                 (uint32_t)kRows, (uint32_t)slices);
+  if (rc != SACQ_OK) return rc;
+  const int at = plan->count < SplitPlan::kMaps ? plan->count++ : SplitPlan::kMaps - 1;
+  plan->idx[at] = *out;
+  plan->slices[at] = slices;
+  return SACQ_OK;
+}
+
+size_t split_smem(const SplitLayout& l) {
+  const size_t need = l.total + 1024;
+  return need < 116 * 1024 ? 116 * 1024 : need;       // two CTAs (each takes all 512 TMEM columns) never share an SM
+}
+
+// Clusters of `split` such CTAs that run at once (a cluster stays within one GPC).
+int active_clusters(int split, int num_sms) {
+  return split == 8 ? num_sms * 15 / 148 : split == 4 ? num_sms * 33 / 148 : num_sms / split;
+}
+
+template <int D, int MODE>
+cudaError_t launch_kernel(const CUtensorMap& ta, const SplitParams& p, dim3 grid, size_t smem, cudaStream_t s) {
+  static bool configured[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64 || !configured[dev]) {
+    const cudaError_t e = cudaFuncSetAttribute(split_k_kernel<D, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e != cudaSuccess) return e;
+    if (dev >= 0 && dev < 64) configured[dev] = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kCtaThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)p.split;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = p.split > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, split_k_kernel<D, MODE>, ta, p);
+}
+
+// Index slices and scale groups of the largest K slice.
+void slice_extent(const sacq_layer* L, int split, int* slices, int* groups) {
+  const int nkb = (int)(L->d.in_features / kStageK), d = L->d.vector_dim, bits = L->d.index_bits;
+  *slices = *groups = 0;
+  for (int r = 0; r < split; ++r) {
+    const int k0 = r * nkb / split * kStageK, k1 = (r + 1) * nkb / split * kStageK;
+    const int n = ((k1 / d * bits + 127) >> 7) - ((k0 / d * bits) >> 7);
+    const int g = (k1 - 1) / L->d.group_size - k0 / L->d.group_size + 1;
+    if (n > *slices) *slices = n;
+    if (g > *groups) *groups = g;
+  }
+}
+
+// How many slices K is cut into: a function of K alone, so the order in which an output is summed depends
+// neither on the number of tokens nor on the layer's width -- a batch gives each of its rows the bytes of a
+// smaller call, sibling layers share a launch, and the row shards of a split layer reproduce it.  About 1,024
+// of K per CTA: measured at 64 and 300 tokens, two slices are the best or within 10 % of it for K = 1,024 and
+// 2,048 on 1,024- to 6,144-row layers, four for K = 4,096 and 6,144 (larger clusters leave SMs idle: 33 clusters
+// of 4, 22 of 6, 15 of 8 run at once); eight above, where a slice's indices would no longer fit shared memory.
+int slices_for(int64_t K) { return K < 1024 ? 1 : K < 4096 ? 2 : K < 8192 ? 4 : 8; }
+
+// Completes a choice of tokens and slices; false if it does not fit shared memory.
+bool split_fits(const sacq_layer* L, SplitMode mode, SplitChoice* c) {
+  const int cb_bytes = L->cb_entries * L->d.vector_dim * 2, groups = mode == kSplitHiLo ? 0 : 1;
+  slice_extent(L, c->split, &c->max_slices, &c->max_groups);
+  const int tiles = ((int)(L->d.in_features / kStageK) + c->split - 1) / c->split * (mode == kSplitHalf ? 2 : 1);
+  for (c->act_stages = tiles < 2 ? 2 : tiles < kMaxAct ? tiles : kMaxAct; c->act_stages >= 2; --c->act_stages)
+    if (split_smem(split_layout(c->tok, c->split, c->act_stages, c->max_slices, groups * c->max_groups, cb_bytes)) <= 227 * 1024)
+      return true;
+  return false;
+}
+
+// Time of one CTA with `tok` tokens and `kbs` weight stages (us): prologue, the slower of expansion, MMAs and
+// activation tiles per stage, reduction.
+double split_cta_us(int vector_dim, SplitMode mode, int tok, int kbs, int split) {
+  double stage = mode >= kSplitInt8 ? 0.75 : vector_dim == 8 ? 0.48 : 0.6;
+  if (0.002 * tok > stage) stage = 0.002 * tok;
+  return 2.5 + kbs * stage + 0.015 * tok + (split > 1 ? 0.8 : 0.0);
+}
+
+}  // namespace
+
+bool split_k_choose(const sacq_layer* L, int64_t M, SplitMode mode, SplitChoice* out) {
+  const sacq_layer_desc& d = L->d;
+  if (d.vector_dim != 8 && d.vector_dim != 4) return false;
+  if (d.index_bits > 16 || !L->rows_16b_aligned || d.in_features % kStageK != 0) return false;
+  if (mode < kSplitInt8 && has_shift(L)) return false;
+  if (mode == kSplitHiLo ? L->num_groups != 1 : d.group_size % (mode == kSplitHalf ? 64 : 16) != 0) return false;
+  // the recipes read the codebook as it came, which is not padded to whole 16-byte units
+  if (mode >= kSplitInt8 && d.codebook_size * d.vector_dim % 8 != 0) return false;
+  const int cb_bytes = L->cb_entries * d.vector_dim * 2;
+  if (cb_bytes % 16 != 0 || M <= 0 || M > (1 << 20)) return false;
+  const int nkb = (int)(d.in_features / kStageK);
+  const int64_t row_tiles = (d.out_features + kRows - 1) / kRows;
+  const int slices = slices_for(d.in_features);
+  *out = SplitChoice();
+  const int least = (int)((M + kMaxTok - 1) / kMaxTok);
+  for (int split = 1; split <= slices; split *= 2) {
+    const int kbs = (nkb + split - 1) / split;
+    const int at_once = active_clusters(split, L->num_sms);
+    for (int tiles = least; tiles <= 3 * least + 1; ++tiles) {
+      int tok = (int)(((M + tiles - 1) / tiles + 15) & ~(int64_t)15);
+      if (tok > 256) tok = (tok + 31) & ~31;
+      if (slices / split > 4 || tok * (slices / split) > kMaxTok) continue;
+      SplitChoice c;
+      c.tok = tok;
+      c.tiles = (int)((M + tok - 1) / tok);
+      c.split = split;
+      c.parts = slices / split;
+      if (!split_fits(L, mode, &c)) continue;
+      const int64_t waves = (row_tiles * c.tiles + at_once - 1) / at_once;
+      // every CTA fetches the codebook through L2
+      const int64_t ctas = row_tiles * c.tiles * split, resident = waves * L->num_sms;
+      c.us = waves * split_cta_us(d.vector_dim, mode, tok, kbs, split) + 0.01 * (double)(ctas < resident ? ctas : resident);
+      if (c.us < out->us) *out = c;
+    }
+  }
+#ifdef SACQ_TUNE
+  if (const char* e = getenv("SACQ_SPLIT")) {
+    SplitChoice c;
+    if (sscanf(e, "%d,%d,%d", &c.tok, &c.split, &c.parts) == 3) {
+      c.tiles = (int)((M + c.tok - 1) / c.tok);
+      c.us = 0;
+      if (c.tok * c.parts > kMaxTok || c.split * c.parts > nkb || !split_fits(L, mode, &c)) return false;
+      *out = c;
+    }
+  }
+#endif
+  return out->tok != 0;
+}
+
+bool split_k_choose_multi(const sacq_layer* const* layers, int n, int64_t M, SplitMode mode, SplitChoice* out) {
+  const sacq_layer_desc& d0 = layers[0]->d;
+  int64_t rows = 0;
+  for (int l = 0; l < n; ++l) {
+    const sacq_layer_desc& d = layers[l]->d;
+    if (d.in_features != d0.in_features || d.vector_dim != d0.vector_dim || d.index_bits != d0.index_bits ||
+        d.codebook_size != d0.codebook_size || d.group_size != d0.group_size || d.device != d0.device || d.out_features <= 0)
+      return false;
+    rows += (d.out_features + kRows - 1) / kRows * kRows;
+  }
+  sacq_layer all = *layers[0];                        // token tiles for the rows of all layers together
+  all.d.out_features = rows;
+  return split_k_choose(&all, M, mode, out);
+}
+
+void split_k_release(sacq_layer* L) {
+  delete L->split_plan;
+  L->split_plan = nullptr;
+}
+
+int launch_split_k(const sacq_layer* const* layers, int n, const void* act, const float* scale, int64_t M, void* const* ys,
+                   const int64_t* ldys, SplitMode mode, const SplitChoice& c, cudaStream_t s, const void* residual,
+                   int64_t ldr, const BcastDst* bc, const float* row_scale) {
+  const sacq_layer_desc& d0 = layers[0]->d;
+  if (reinterpret_cast<uintptr_t>(act) % 16 != 0)
+    return set_error(SACQ_ERR_ALIGNMENT, "quantized activations must be 16-byte aligned");
+  SplitParams p;
+  memset(&p, 0, sizeof(p));
+  CUtensorMap ta;
+  const uint64_t act_row = (uint64_t)d0.in_features * (mode == kSplitHalf ? 2 : 1);
+  int rc = encode_bytes_2d(&ta, act, act_row, (uint64_t)M, act_row, 128u, (uint32_t)(c.tok <= 256 ? c.tok : c.tok / 2),
+                           CU_TENSOR_MAP_SWIZZLE_128B);
+  if (rc != SACQ_OK) return rc;
+  int64_t widest = 0;
+  for (int l = 0; l < n; ++l) {
+    const sacq_layer* L = layers[l];
+    rc = slice_map(const_cast<sacq_layer*>(L), c.max_slices, &p.idx[l]);
+    if (rc != SACQ_OK) return rc;
+    SplitLayer& q = p.layer[l];
+    q.cb = mode == kSplitHiLo ? L->cb_hilo
+           : mode == kSplitHalf ? reinterpret_cast<const uint8_t*>(L->cb_f16) : static_cast<const uint8_t*>(L->d.codebook);
+    q.scales = static_cast<const uint16_t*>(L->d.scales);
+    q.bias = static_cast<const uint16_t*>(L->d.bias);
+    q.y = static_cast<uint16_t*>(ys[l]);
+    q.ldy = ldys[l];
+    q.status = L->d_status;
+    q.N = (int)L->d.out_features;
+    q.scale_mul = ldexpf(kHalfPreScale, L->sc_exp_shift);
+    q.out_mul = mode == kSplitHalf ? ldexpf(1.f / kHalfPreScale, -(L->cb_exp_shift + L->sc_exp_shift)) : ldexpf(1.f, -L->cb8_exp_shift);
+    if (L->d.out_features > widest) widest = L->d.out_features;
+  }
+  p.act_scale = scale;
+  p.row_scale = row_scale;
+  p.shift = d0.shift_bf16;
+  p.residual = static_cast<const uint16_t*>(residual);
+  p.ldr = ldr;
+  if (bc != nullptr) {
+    p.n_bc = bc->n;
+    for (int i = 0; i < bc->n; ++i) p.ybc[i] = static_cast<uint16_t*>(bc->ptr[i]);
+  }
+  p.M = (int)M; p.K = (int)d0.in_features; p.C = mode >= kSplitInt8 ? d0.codebook_size : layers[0]->cb_entries;
+  p.bits = d0.index_bits; p.num_groups = (int)layers[0]->num_groups; p.group_size = d0.group_size;
+  p.split = c.split; p.parts = c.parts; p.tok = c.tok; p.act_stages = c.act_stages; p.max_slices = c.max_slices; p.max_groups = c.max_groups;
+  const dim3 grid((unsigned)((widest + kRows - 1) / kRows * c.split), (unsigned)c.tiles, (unsigned)n);
+  const size_t smem = split_smem(split_layout(c.tok, c.split, c.act_stages, c.max_slices, mode == kSplitHiLo ? 0 : c.max_groups,
+                                              layers[0]->cb_entries * d0.vector_dim * 2));
+  cudaError_t e;
+  const bool d8 = d0.vector_dim == 8;
+  switch (mode) {
+    case kSplitHiLo: e = d8 ? launch_kernel<8, kSplitHiLo>(ta, p, grid, smem, s) : launch_kernel<4, kSplitHiLo>(ta, p, grid, smem, s); break;
+    case kSplitHalf: e = d8 ? launch_kernel<8, kSplitHalf>(ta, p, grid, smem, s) : launch_kernel<4, kSplitHalf>(ta, p, grid, smem, s); break;
+    case kSplitInt8: e = d8 ? launch_kernel<8, kSplitInt8>(ta, p, grid, smem, s) : launch_kernel<4, kSplitInt8>(ta, p, grid, smem, s); break;
+    default: e = d8 ? launch_kernel<8, kSplitFp8>(ta, p, grid, smem, s) : launch_kernel<4, kSplitFp8>(ta, p, grid, smem, s); break;
+  }
+  count_launch();
+  if (e != cudaSuccess) return cuda_fail(e, "split-K launch");
+  return SACQ_OK;
+}
+
+}  // namespace sacq

@@ -1,0 +1,39 @@
+// Interface of the cluster split-K tensor-core kernel (linear_split_k.cu).
+#pragma once
+
+#include <stdint.h>
+
+#include "common.cuh"
+
+namespace sacq {
+
+constexpr int kSplitMaxLayers = 4;    // sibling layers of one launch
+
+// What the weight operand of a call is:
+enum SplitMode {
+  kSplitHiLo = 0,   // e4m3 high and low halves of the codewords, e4m3 activations; one scale per row
+  kSplitHalf = 1,   // fp16(codeword x scale), activations widened to fp16: grouped scales, INT8 activations
+  kSplitInt8 = 2,   // the INT8 recipe's weight bytes, int8 activations, int32 sums
+  kSplitFp8 = 3     // the FP8 recipe's weight bytes, e4m3 activations
+};
+
+// How one call is cut up: token tiles of `tok` tokens, clusters of `split` CTAs with `parts` slices of K each.
+struct SplitChoice {
+  int tok = 0, tiles = 0, split = 0, parts = 1, act_stages = 0, max_slices = 0, max_groups = 0;
+  double us = 1e30;             // modelled time
+};
+
+// The best cut for M tokens; false if the kernel cannot run the layer in that form.
+bool split_k_choose(const sacq_layer* L, int64_t M, SplitMode mode, SplitChoice* out);
+
+// The same for several layers in one launch; false if they are not of one geometry.
+bool split_k_choose_multi(const sacq_layer* const* layers, int n, int64_t M, SplitMode mode, SplitChoice* out);
+
+// n layers of one geometry (n = 1: the plain launch) on one set of activations: bytes [M, K], or for kSplitHalf
+// the activations already widened to fp16 [M, K].  row_scale: the recipes' per-row weight scales [N] (n = 1).
+int launch_split_k(const sacq_layer* const* layers, int n, const void* act, const float* scale, int64_t M, void* const* ys,
+                   const int64_t* ldys, SplitMode mode, const SplitChoice& c, cudaStream_t s, const void* residual = nullptr,
+                   int64_t ldr = 0, const BcastDst* bc = nullptr, const float* row_scale = nullptr);
+void split_k_release(sacq_layer* L);
+
+}  // namespace sacq

@@ -60,6 +60,24 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   }
 }
 
+// One lane of a converged warp.  Instructions whose operands live in uniform registers (tcgen05.mma, TMA
+// copies) are issued as `if (elect_one()) ...` from code that the whole warp runs with warp-uniform
+// operands: inside a branch that only one lane takes, the compiler moves every operand into uniform
+// registers one by one for each instruction, which made an MMA cost about 120 clocks whatever its size.
+// Issued this way one with N columns takes N / 2 clocks (A in tensor memory; measured from N = 16 on),
+// and instructions that follow each other into one accumulator do not wait for each other.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+  return r != 0;
+}
+// A value that is the same in all lanes, marked as such.
+__device__ __forceinline__ uint32_t warp_uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+// mbar_wait by a whole converged warp, with one answer for all lanes.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status));
+}
+
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
@@ -135,6 +153,11 @@ __host__ __device__ constexpr uint32_t make_idesc(int bn) {
   return (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
 }
 
+// kind::i8 instruction descriptor: int32 accumulate, A = B = signed 8-bit, both K-major, N, M.
+__host__ __device__ constexpr uint32_t make_idesc_i8(int bn) {
+  return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+}
+
 __device__ __forceinline__ void cp_async_16(void* smem_dst, const void* gmem_src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(gmem_src) : "memory");
 }
@@ -207,8 +230,12 @@ __device__ __forceinline__ void store_staged_tile(const uint8_t* stg, int pitch,
 int encode_bytes_2d(CUtensorMap* map, const void* base, uint64_t row_bytes, uint64_t rows, uint64_t pitch_bytes,
                     uint32_t box_bytes, uint32_t box_rows, CUtensorMapSwizzle swizzle);
 
+// 3-D byte tensor [dim2][rows][row_bytes] with a [box2][box_rows][box_bytes] box, not swizzled (linear_large_m.cu).
+int encode_bytes_3d(CUtensorMap* map, const void* base, uint64_t row_bytes, uint64_t rows, uint64_t dim2, uint64_t row_pitch,
+                    uint64_t dim2_pitch, uint32_t box_bytes, uint32_t box_rows, uint32_t box2);
+
 // Tile map over a layer's packed index rows: box = one index super-block (two 128-k blocks) x
-// `rows` weight rows (32, 64 or 128).  Built on first use and kept by the layer.
-int large_m_index_map(const sacq_layer* L, int rows, const CUtensorMap** out);
+// 128 weight rows.  Built on first use and kept by the layer.
+int large_m_index_map(const sacq_layer* L, const CUtensorMap** out);
 
 }  // namespace sacq
