@@ -11,6 +11,7 @@
 // coalesced word loads, codewords come from L1/L2 (the codebook is at most 1 MB),
 // and the output is written with one 16-byte (d=8) or 8-byte (d=4) store per thread.
 #include "common.cuh"
+#include "encode.cuh"
 
 #include <math.h>
 #include <string.h>
@@ -186,6 +187,71 @@ decode_weight_int8_kernel(const uint32_t* __restrict__ words, const uint16_t* __
   }
 }
 
+// The 8-bit weight rows of the two recipes for the layouts they run on: a warp per 1,024 weights of a row, 16
+// weights per lane and step (one 16-byte store), the codebook in shared memory where it fits (SMEM).
+//
+// What bounds it: the one-thread-per-vector kernels above spend a 16-byte L1 gather (a tag lookup per lane: d = 4
+// took 25 us for 12.6 M weights), an index-to-row division and an IEEE division per weight (d = 8: 15 us).  Here
+// the gathers go to shared memory, the row's divisor is set up once, and the quotients are bracketed
+// (RowDivisor).  The int8 bound: |z| is clamped to RN(127 s) first, beyond which every quotient rounds to +-127.
+constexpr int kSegSteps = 64;         // 16-weight steps of a row that a warp takes
+
+template <int D, bool I8, bool SMEM>
+__global__ void __launch_bounds__(512, 2)
+decode_rows_kernel(const uint32_t* __restrict__ words, const uint16_t* __restrict__ cb, const uint16_t* __restrict__ scales,
+                   const float* __restrict__ sw, uint8_t* __restrict__ wq, int64_t N, int K, int bits, int group_size,
+                   int num_groups, uint16_t shift, int cb_bytes) {
+  extern __shared__ __align__(16) uint8_t table[];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if constexpr (SMEM) {                               // the codebook is constant: fetched ahead of the kernel in front
+    for (int i = threadIdx.x; i < cb_bytes / 8; i += blockDim.x)
+      reinterpret_cast<uint2*>(table)[i] = __ldg(reinterpret_cast<const uint2*>(cb) + i);
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  __syncthreads();
+  const uint8_t* tb = SMEM ? table : reinterpret_cast<const uint8_t*>(cb);
+  constexpr int V = 16 / D;                           // vectors per step
+  const __nv_bfloat162 shift2 = __halves2bfloat162(__ushort_as_bfloat16(shift), __ushort_as_bfloat16(shift));
+  const int lane = threadIdx.x & 31;
+  const int warps = (int)gridDim.x * (int)(blockDim.x >> 5);
+  const int steps = K / 16, vpr = K / D, segs = (steps + kSegSteps - 1) / kSegSteps;
+  const uint32_t mask = (1u << bits) - 1u;
+  const int items = (int)N * segs;
+  for (int item = (int)blockIdx.x * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5); item < items; item += warps) {
+    const int64_t n = item / segs;
+    const int begin = (item - (int)n * segs) * kSegSteps, end = min(begin + kSegSteps, steps);
+    const RowWeights r = row_weights(__ldg(sw + n));
+    uint4* out = reinterpret_cast<uint4*>(wq + n * K);
+    uint16_t s = __ldg(scales + n * num_groups);
+#pragma unroll 2
+    for (int st = begin + lane; st < end; st += 32) {
+      const int64_t p = (n * vpr + (int64_t)st * V) * bits;
+      const uint32_t* w = words + (p >> 5);
+      const uint32_t off = (uint32_t)(p & 31);
+      const uint32_t w0 = __ldg(w), w1 = __ldg(w + 1);
+      uint64_t win = __funnelshift_r(w0, w1, off);
+      if constexpr (V == 4) win |= (uint64_t)__funnelshift_r(w1, off + 4u * bits > 64u ? __ldg(w + 2) : 0u, off) << 32;
+      if (num_groups > 1) s = __ldg(scales + n * num_groups + st * 16 / group_size);
+      uint32_t pair[8];                               // 16 codebook elements
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        const uint32_t i = (uint32_t)(win >> (v * bits)) & mask;
+        if constexpr (D == 8) {
+          const uint4 c = SMEM ? *reinterpret_cast<const uint4*>(tb + i * 16) : __ldg(reinterpret_cast<const uint4*>(tb) + i);
+          pair[4 * v] = c.x; pair[4 * v + 1] = c.y; pair[4 * v + 2] = c.z; pair[4 * v + 3] = c.w;
+        } else {
+          const uint2 c = SMEM ? *reinterpret_cast<const uint2*>(tb + i * 8) : __ldg(reinterpret_cast<const uint2*>(tb) + i);
+          pair[2 * v] = c.x; pair[2 * v + 1] = c.y;
+        }
+      }
+      uint32_t a[4];
+      const __nv_bfloat16 sb = __ushort_as_bfloat16(s);
+      encode_weights16<I8>(pair, __halves2bfloat162(sb, sb), shift2, r, a);
+      out[st] = make_uint4(a[0], a[1], a[2], a[3]);
+    }
+  }
+}
+
 // ---- derived tables -------------------------------------------------------
 
 __global__ void codebook_absmax_kernel(const uint16_t* __restrict__ cb, int64_t count, float* __restrict__ out) {
@@ -285,16 +351,68 @@ int launch_weight_row_scale(const sacq_layer* L, float* sw, cudaStream_t s, floa
   return SACQ_OK;
 }
 
+namespace {
+
+template <int D, bool I8, bool SMEM>
+cudaError_t launch_decode_rows_inst(const sacq_layer* L, const float* sw, uint8_t* wq, cudaStream_t s) {
+  const sacq_layer_desc& d = L->d;
+  const int cb_bytes = d.codebook_size * D * 2;
+  static bool configured[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (SMEM && (dev < 0 || dev >= 64 || !configured[dev])) {
+    const cudaError_t e = cudaFuncSetAttribute(decode_rows_kernel<D, I8, SMEM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024);
+    if (e != cudaSuccess) return e;
+    if (dev >= 0 && dev < 64) configured[dev] = true;
+  }
+  const int64_t items = d.out_features * ((d.in_features / 16 + kSegSteps - 1) / kSegSteps);
+  const int64_t ctas = (items + 15) / 16, most = 2 * (int64_t)L->num_sms;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(ctas < most ? ctas : most));
+  cfg.blockDim = dim3(512);
+  cfg.dynamicSmemBytes = SMEM ? (size_t)((cb_bytes + 15) & ~15) : 0;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, decode_rows_kernel<D, I8, SMEM>, static_cast<const uint32_t*>(d.packed),
+                            static_cast<const uint16_t*>(d.codebook), static_cast<const uint16_t*>(d.scales), sw, wq,
+                            d.out_features, (int)d.in_features, d.index_bits, d.group_size, (int)L->num_groups,
+                            d.shift_bf16, cb_bytes);
+}
+
+// The row kernel, or cudaErrorNotSupported for a layout it does not take.
+template <bool I8>
+cudaError_t launch_decode_rows(const sacq_layer* L, const float* sw, void* wq, cudaStream_t s) {
+  const sacq_layer_desc& d = L->d;
+  const int D = d.vector_dim;
+  if ((D != 8 && D != 4) || d.index_bits > 16 || d.in_features % 16 != 0 || (L->num_groups > 1 && d.group_size % 16 != 0) ||
+      !aligned(wq, 16) || !aligned(d.codebook, 16) || d.out_features * ((d.in_features / 16 + kSegSteps - 1) / kSegSteps) > 0x3fffffff)
+    return cudaErrorNotSupported;
+  uint8_t* out = static_cast<uint8_t*>(wq);
+  const bool smem = (int64_t)d.codebook_size * D * 2 <= 64 * 1024;
+  if (D == 8) return smem ? launch_decode_rows_inst<8, I8, true>(L, sw, out, s) : launch_decode_rows_inst<8, I8, false>(L, sw, out, s);
+  return smem ? launch_decode_rows_inst<4, I8, true>(L, sw, out, s) : launch_decode_rows_inst<4, I8, false>(L, sw, out, s);
+}
+
+}  // namespace
+
 int launch_decode_weight_int8(const sacq_layer* L, const float* sw, void* wq, cudaStream_t s) {
   const sacq_layer_desc& d = L->d;
   const int64_t total = d.out_features * L->vectors_per_row;
   if (total == 0) return SACQ_OK;
-  decode_weight_int8_kernel<<<grid_for(total, 256, L->num_sms), 256, 0, s>>>(
-      static_cast<const uint32_t*>(d.packed), static_cast<const uint16_t*>(d.codebook),
-      static_cast<const uint16_t*>(d.scales), sw, static_cast<int8_t*>(wq), total, (int)L->vectors_per_row,
-      d.vector_dim, d.index_bits, d.group_size, (int)L->num_groups, host_bf16_to_float(d.shift_bf16));
+  cudaError_t e = launch_decode_rows<true>(L, sw, wq, s);
+  if (e == cudaErrorNotSupported) {
+    decode_weight_int8_kernel<<<grid_for(total, 256, L->num_sms), 256, 0, s>>>(
+        static_cast<const uint32_t*>(d.packed), static_cast<const uint16_t*>(d.codebook),
+        static_cast<const uint16_t*>(d.scales), sw, static_cast<int8_t*>(wq), total, (int)L->vectors_per_row,
+        d.vector_dim, d.index_bits, d.group_size, (int)L->num_groups, host_bf16_to_float(d.shift_bf16));
+    e = cudaGetLastError();
+  }
   count_launch();
-  SACQ_CUDA_TRY(cudaGetLastError());
+  SACQ_CUDA_TRY(e);
   return SACQ_OK;
 }
 
@@ -302,12 +420,16 @@ int launch_decode_weight_fp8(const sacq_layer* L, const float* sw, void* wq, cud
   const sacq_layer_desc& d = L->d;
   const int64_t total = d.out_features * L->vectors_per_row;
   if (total == 0) return SACQ_OK;
-  decode_weight_fp8_kernel<<<grid_for(total, 256, L->num_sms), 256, 0, s>>>(
-      static_cast<const uint32_t*>(d.packed), static_cast<const uint16_t*>(d.codebook),
-      static_cast<const uint16_t*>(d.scales), sw, static_cast<uint8_t*>(wq), total, (int)L->vectors_per_row,
-      d.vector_dim, d.index_bits, d.group_size, (int)L->num_groups, host_bf16_to_float(d.shift_bf16));
+  cudaError_t e = launch_decode_rows<false>(L, sw, wq, s);
+  if (e == cudaErrorNotSupported) {
+    decode_weight_fp8_kernel<<<grid_for(total, 256, L->num_sms), 256, 0, s>>>(
+        static_cast<const uint32_t*>(d.packed), static_cast<const uint16_t*>(d.codebook),
+        static_cast<const uint16_t*>(d.scales), sw, static_cast<uint8_t*>(wq), total, (int)L->vectors_per_row,
+        d.vector_dim, d.index_bits, d.group_size, (int)L->num_groups, host_bf16_to_float(d.shift_bf16));
+    e = cudaGetLastError();
+  }
   count_launch();
-  SACQ_CUDA_TRY(cudaGetLastError());
+  SACQ_CUDA_TRY(e);
   return SACQ_OK;
 }
 
