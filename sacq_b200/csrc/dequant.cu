@@ -220,7 +220,7 @@ decode_rows_kernel(const uint32_t* __restrict__ words, const uint16_t* __restric
   for (int item = (int)blockIdx.x * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5); item < items; item += warps) {
     const int64_t n = item / segs;
     const int begin = (item - (int)n * segs) * kSegSteps, end = min(begin + kSegSteps, steps);
-    const RowWeights r = row_weights(__ldg(sw + n));
+    const RowWeights r = row_weights<I8>(__ldg(sw + n));
     uint4* out = reinterpret_cast<uint4*>(wq + n * K);
     uint16_t s = __ldg(scales + n * num_groups);
 #pragma unroll 2

@@ -113,14 +113,17 @@ __device__ __forceinline__ void encode_pairs(const uint32_t (&w)[P], const RowDi
 // like the fp32 operation followed by a conversion).
 struct RowWeights {
   RowDivisor d;
-  __nv_bfloat162 lim, neg_lim;  // int8: |w| is clamped to the largest bf16 below 127.5 times the row scale; that one
-                                // is above 126.5 times it (bf16 values are at most 1/128 apart), so it encodes to 127
+  // |w| is clamped to a bf16 value that encodes to the largest byte, so that a caller's own row scale cannot overflow
+  // the quotient.  int8: the largest one below 127.5 times the row scale; it is above 126.5 times it (bf16 values
+  // are at most 1/128 apart).  e4m3: about 1,000 times the row scale, which saturates.
+  __nv_bfloat162 lim, neg_lim;
 };
+template <bool I8>
 __device__ __forceinline__ RowWeights row_weights(float sw) {
   RowWeights w;
   w.d = row_divisor(sw);
   // a row scale that is not an ordinary number takes the division, which clamps by itself
-  const __nv_bfloat16 l = w.d.fast ? __float2bfloat16_rz(127.4999f * sw) : __ushort_as_bfloat16(0x7f80);
+  const __nv_bfloat16 l = w.d.fast ? __float2bfloat16_rz((I8 ? 127.4999f : 1000.f) * sw) : __ushort_as_bfloat16(0x7f80);
   w.lim = __halves2bfloat162(l, l);
   w.neg_lim = __hneg2(w.lim);
   return w;
@@ -136,6 +139,7 @@ __device__ __forceinline__ void encode_weights16(const uint32_t (&pair)[8], __nv
   for (int j = 0; j < 8; ++j) {
     __nv_bfloat162 v = __hadd2_rn(__hmul2_rn(*reinterpret_cast<const __nv_bfloat162*>(&pair[j]), s2), shift2);
     if constexpr (I8) v = __hmin2(__hmax2(v, r.neg_lim), r.lim);
+    else v = __hmin2_nan(__hmax2_nan(v, r.neg_lim), r.lim);      // a NaN stays one
     w[j] = *reinterpret_cast<const uint32_t*>(&v);
   }
   encode_pairs<I8, 8>(w, r.d, out);

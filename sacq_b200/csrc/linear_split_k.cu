@@ -459,7 +459,7 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     int grp = 0, grp_end = GROUPS ? (g_first + 1) * p.group_size - kb0 * kStageK : 0;    // k (in the slice) at which the scale changes
     // One stage's 16 words of this thread.  The next stage's words are gathered before the wait for this
     // stage's tcgen05.st: the gathers, which bound the loop, then never wait for a store's latency.
-    const RowWeights rw = row_weights(RECIPE ? __ldg(p.row_scale + min(n0 + row, lay.N - 1)) : 1.f);
+    const RowWeights rw = row_weights<INT>(RECIPE ? __ldg(p.row_scale + min(n0 + row, lay.N - 1)) : 1.f);
     const __nv_bfloat162 shift2 = __halves2bfloat162(__ushort_as_bfloat16(p.shift), __ushort_as_bfloat16(p.shift));
     auto expand = [&](int wi, uint32_t (&w)[16]) {
       if constexpr (RECIPE) {
