@@ -34,17 +34,6 @@ __device__ __forceinline__ void store8(void* row, int64_t ch, const uint2& o) {
   else reinterpret_cast<uint2*>(row)[ch] = o;
 }
 
-// Scale of a row from its largest |x|: a NaN maximum fails `> 0` like in the reference's torch.where, so the row
-// keeps scale 1 and its NaN elements stay NaN; an infinite maximum gives an infinite scale.  Neither takes the
-// bracket (the first because its elements are not bounded by the scale).
-template <bool I8>
-__device__ __forceinline__ RowDivisor scale_of(float mx) {
-  const bool ordinary = mx > 0.f;
-  RowDivisor d = row_divisor(ordinary ? __fdiv_rn(mx, I8 ? 127.0f : kE4M3Max) : 1.0f);
-  d.fast = d.fast && ordinary;
-  return d;
-}
-
 // Threads of a CTA that handles one row of K elements in 16-byte chunks: a chunk per thread while the rows
 // are few (their latency is all there is: 6,144 elements on 768 threads instead of three rounds of 256), 256
 // threads when the rows outnumber what the device holds at once.

@@ -69,12 +69,19 @@ int64_t grouped_min_m(const sacq_layer* L) {
   if (L->d.out_features >= 32 * (int64_t)L->num_sms) return 17;
   return 48;
 }
-constexpr int64_t kTmemMinM = 1024;
-constexpr int64_t kTmemMinMBigCodebook = 128;
+// From how many rows the tensor-core kernel that keeps the expanded weights in tensor memory wins (its 128-row tiles
+// need that many tokens to fill the device).  A codebook that is gathered from L2 makes an expansion twice as dear,
+// and the split-K kernel expands a wide layer again for every second 384-token tile.
+int64_t tmem_min_m(const sacq_layer* L) {
+  return !split_k_codebook_in_smem(L) && L->d.out_features >= 4096 ? 384 : 1024;
+}
 
 // From how many tokens a split-K kernel, which walks the weights once, beats a small-M kernel, which walks them
 // once per 16-token chunk: from the second chunk on wide or deep layers, from the third on all but the smallest.
+// A codebook in L2 leaves the small-M kernel 2 warps' gathers in flight per scheduler: on wide layers the split-K
+// kernel wins from one token on (2048x6144, 65,536 entries: 17.8 / 13.4 us at 16 tokens, 46 / 15.6 at 64).
 bool split_wins(const sacq_layer* L, int64_t M, int64_t smallest) {
+  if (!split_k_codebook_in_smem(L)) return M > 16 || L->d.out_features >= 4096;
   const int64_t work = L->d.in_features * L->d.out_features;
   return (M > 16 && (L->d.out_features >= 4096 || work >= (8 << 20))) || (M > 32 && work > smallest);
 }
@@ -94,13 +101,10 @@ int pick_kernel(const sacq_layer* L, int64_t M) {
   if (L->force_kernel == 1 || L->force_kernel >= 3)
     return small_m_supported(L) ? 1 : SACQ_ERR_UNSUPPORTED;
   if (L->force_kernel == 2) return large_m_supported(L) ? 2 : SACQ_ERR_UNSUPPORTED;
-  // A shape rule, not a backend switch.  From kTmemMinM rows the tensor-core kernel that keeps
-  // the expanded weights in tensor memory wins on every layer shape (its 128-row tiles need that
-  // many tokens to fill the device).  The threshold does not depend on the layer's width, so
-  // the row shards of a split layer run the kernel the whole layer would, and reproduce it
-  // bit for bit (so does the split-K kernel, which sums in an order that depends on K alone).  Layers whose codebook does not fit shared memory have no other tensor-core
-  // kernel and switch earlier.
-  if (large_m_tmem_supported(L) && (M >= kTmemMinM || (M >= kTmemMinMBigCodebook && !large_m_supported(L)))) return 4;
+  // A shape rule, not a backend switch.  The thresholds of the per-channel kernels do not depend on a layer's
+  // width as long as its codebook fits shared memory, so the row shards of a split layer run the kernel the whole
+  // layer would, and reproduce it bit for bit (the split-K kernel sums in an order that depends on K alone).
+  if (large_m_tmem_supported(L) && M >= tmem_min_m(L)) return 4;
   // Below, quantizer + GEMM of the small-M and the split-K kernel at 17 tokens: 1024x4096 10.9 / 6.8 us,
   // 6144x2048 15.4 / 11.5, 2048x6144 15.5 / 8.9; at 33: 1024x1024 7.3 / 5.7, 2048x2048 9.2 / 8.8, 4096x1024
   // 9.5 / 9.2, 2048x1024 even.
@@ -394,7 +398,8 @@ enum Int8Route { kInt8Small, kInt8Grouped, kInt8TmemGrouped };
 Int8Route int8_route(const sacq_layer* L, int64_t M) {
   if (large_m_tmem_grouped_supported(L) && M >= large_m_tmem_grouped_min_m(L)) return kInt8TmemGrouped;
   if (!large_m_grouped_supported(L)) return kInt8Small;
-  const int64_t warp_mma_wins = small_m_int8_selector(L) == 5 ? (L->d.out_features < 2048 ? 48 : 16) : 0;
+  const bool warp_mma = small_m_int8_selector(L) == 5 && (split_k_codebook_in_smem(L) || L->d.out_features < 4096);
+  const int64_t warp_mma_wins = !warp_mma ? 0 : L->d.out_features < 2048 && split_k_codebook_in_smem(L) ? 48 : 16;
   return M > warp_mma_wins ? kInt8Grouped : kInt8Small;
 }
 }  // namespace
@@ -495,7 +500,7 @@ namespace {
 bool recipe_in_one(const sacq_layer* L, const void* q, const float* act_scale, const float* w_scale, int64_t M, void* y,
                    int64_t ldy, SplitMode mode, cudaStream_t s, int* rc) {
   SplitChoice c;
-  if (M > (L->d.out_features >= 4096 ? 512 : 1024) || reinterpret_cast<uintptr_t>(q) % 16 != 0 || reinterpret_cast<uintptr_t>(L->d.codebook) % 16 != 0 ||
+  if (M > (L->d.out_features >= 4096 || !split_k_codebook_in_smem(L) ? 512 : 1024) || reinterpret_cast<uintptr_t>(q) % 16 != 0 || reinterpret_cast<uintptr_t>(L->d.codebook) % 16 != 0 ||
       (mode == kSplitInt8 && L->d.in_features * 127 * 127 > 2147483647LL) || !split_k_choose(L, M, mode, &c))
     return false;
   *rc = launch_split_k(&L, 1, q, act_scale, M, &y, &ldy, mode, c, s, nullptr, 0, nullptr, w_scale);
@@ -691,30 +696,49 @@ SACQ_API int sacq_linear_a8_multi(const sacq_layer_t* const* layers, int num_lay
   return SACQ_OK;
 }
 
-// Quantizer + GEMM of one call.  Where the GEMM takes fp16 activations, the quantizer writes them as fp16 into
-// the workspace itself: one launch less than quantizing to bytes and widening those (2 us of host time and as
-// much of the GPU's at small sizes), the same values.
-int sacq_forward_call(const sacq_layer_t* L, const void* x_bf16, int64_t x_pitch, int64_t M, int int8, const void* residual,
-                      int64_t ldr, void* q_scratch, float* scale_scratch, void* y_out, int64_t ldy, void* workspace,
-                      int64_t workspace_bytes, void* stream) {
+namespace {
+// Whether a forward on a staged warp-MMA kernel quantizes its activations in the GEMM's own CTAs.  It saves a launch
+// (eager calls are bound by the host at 7 us with it and at 5.4 without) and costs the GPU each CTA's own pass over the
+// tokens: a gain there too while that is one warp's work per token or less (2048x1024 at 8 tokens 4.9 us either way,
+// 2048x2048 5.6 against 5.9, at 16 tokens 6.3 against 6.1), a loss on layers that keep the GPU busy anyway (2048x6144
+// 8.9 against 8.4 at one token, 6144x2048 10.7 against 8.4 at 8).
+bool quantizes_in_gemm(const sacq_layer* L, int64_t M) {
+  return L->d.in_features * L->d.out_features <= (4 << 20) && M * L->d.in_features <= (32 << 10) &&
+         M <= small_m_staged_warps(L, M);
+}
+
+// Quantizer + GEMM of one call, in one launch where the GEMM can quantize for itself (own_quantizer = false allows it).
+// Where the GEMM takes fp16 activations, the quantizer writes them as fp16 into the workspace: one launch less than
+// quantizing to bytes and widening those (2 us of host time and as much of the GPU's at small sizes), the same values.
+int forward_impl(const sacq_layer_t* L, const void* x_bf16, int64_t x_pitch, int64_t M, int int8, const void* residual,
+                 int64_t ldr, void* q_scratch, float* scale_scratch, void* y_out, int64_t ldy, void* workspace,
+                 int64_t workspace_bytes, void* stream, bool own_quantizer) {
   if (int rc = check_layer(L)) return rc;
   if (M == 0) return SACQ_OK;
   const int64_t K = L->d.in_features;
   int64_t slab = 0;                                   // tokens up to which the GEMM takes fp16 activations in one piece
   int64_t need = 0;
-  if (M > 0 && L->d.out_features > 0) {
+  const bool rows_ok = M > 0 && L->d.out_features > 0 && K % 8 == 0 && x_bf16 != nullptr &&
+                       reinterpret_cast<uintptr_t>(x_bf16) % 16 == 0 && x_pitch % 8 == 0 && x_pitch >= K && y_out != nullptr &&
+                       ldy >= L->d.out_features;
+  if (rows_ok) {
     const Int8Route r = int8 ? int8_route(L, M) : kInt8Small;
     const int k = int8 ? 0 : pick_kernel(L, M);
+    const bool over = k == 1 && small_m_hands_over(L, M);
+    if (k == 1 && !over && !own_quantizer && quantizes_in_gemm(L, M)) {
+      DeviceGuard guard(L->d.device);
+      return launch_small_m(L, q_scratch, scale_scratch, M, y_out, ldy, workspace, workspace_bytes,
+                            static_cast<cudaStream_t>(stream), residual, ldr, 0, nullptr, x_bf16, x_pitch);
+    }
     if (r == kInt8TmemGrouped || k == 5) {
       slab = large_m_tmem_grouped_slab();
       need = large_m_tmem_grouped_workspace_bytes(L, M);
-    } else if (r == kInt8Grouped || k == 3 || (k == 1 && small_m_hands_over(L, M))) {
+    } else if (r == kInt8Grouped || k == 3 || over) {
       slab = large_m_grouped_slab();
       need = large_m_grouped_workspace_bytes(L, M);
     }
   }
-  const bool wide = M <= slab && K % 8 == 0 && x_bf16 != nullptr && reinterpret_cast<uintptr_t>(x_bf16) % 16 == 0 &&
-                    x_pitch % 8 == 0 && x_pitch >= K && workspace != nullptr && scale_scratch != nullptr && y_out != nullptr &&
+  const bool wide = rows_ok && M <= slab && workspace != nullptr && scale_scratch != nullptr &&
                     reinterpret_cast<uintptr_t>(workspace) % 256 == 0 && workspace_bytes >= kCounterBytes + need;
   if (wide) {
     DeviceGuard guard(L->d.device);
@@ -730,6 +754,21 @@ int sacq_forward_call(const sacq_layer_t* L, const void* x_bf16, int64_t x_pitch
   if (rc != SACQ_OK) return rc;
   if (int8) return sacq_linear_a8i(L, q_scratch, scale_scratch, M, y_out, ldy, workspace, workspace_bytes, stream);
   return linear_a8_impl(L, q_scratch, scale_scratch, M, residual, ldr, y_out, ldy, workspace, workspace_bytes, stream);
+}
+
+// Whether the kernel of a call with M tokens may store its result straight into pinned host memory: one whose stores
+// are whole segments of a token's row (the split-K kernel 256 bytes per warp, the staged warp-MMA kernels 16 to 96).
+bool stores_reach_host(const sacq_layer* L, int64_t M) {
+  const int k = pick_kernel(L, M);
+  return k == 2 || k == 3 || (k == 1 && (small_m_hands_over(L, M) || small_m_staged_warps(L, M) > 0));
+}
+}  // namespace
+
+int sacq_forward_call(const sacq_layer_t* L, const void* x_bf16, int64_t x_pitch, int64_t M, int int8, const void* residual,
+                      int64_t ldr, void* q_scratch, float* scale_scratch, void* y_out, int64_t ldy, void* workspace,
+                      int64_t workspace_bytes, void* stream) {
+  return forward_impl(L, x_bf16, x_pitch, M, int8, residual, ldr, q_scratch, scale_scratch, y_out, ldy, workspace,
+                      workspace_bytes, stream, false);
 }
 
 SACQ_API int sacq_linear_bf16(const sacq_layer_t* L, const void* x_bf16, int64_t x_pitch, int64_t M, void* q_scratch,
@@ -802,11 +841,16 @@ SACQ_API int sacq_linear_bf16_host(const sacq_layer_t* L, const void* x_host, in
     x_dev = x_alias;                                   // the quantizer reads the pinned buffer itself
   else
     SACQ_CUDA_TRY(cudaMemcpyAsync(base + h.x, x_host, (size_t)(M * K * 2), cudaMemcpyHostToDevice, s));
-  const int rc = sacq_linear_bf16(L, x_dev, K, M, base + h.q, reinterpret_cast<float*>(base + h.scale),
-                                  base + h.y, N, base + h.ws, h.scale, stream);
-  if (rc != SACQ_OK) return rc;
   void* y_alias = M * N * 2 <= kDirectHostIoBytes && reinterpret_cast<uintptr_t>(y_host) % 16 == 0
                       ? pinned_alias(y_host) : nullptr;
+  // rows of whole 128-byte lines: the GEMM stores them to the host itself (another kernel that copies them out costs
+  // the call 3 us; rows that share lines would cross the bus in pieces)
+  const bool stores_out = y_alias != nullptr && N % 64 == 0 && reinterpret_cast<uintptr_t>(y_host) % 128 == 0 &&
+                          stores_reach_host(L, M);
+  // the quantizer keeps its own launch: it reads the host's rows once, not once per CTA of the GEMM
+  const int rc = forward_impl(L, x_dev, K, M, 0, nullptr, 0, base + h.q, reinterpret_cast<float*>(base + h.scale),
+                              stores_out ? y_alias : base + h.y, N, base + h.ws, h.scale, stream, true);
+  if (rc != SACQ_OK || stores_out) return rc;
   if (y_alias != nullptr) return launch_copy_to_host(base + h.y, y_alias, M * N * 2, L->num_sms, s);
   SACQ_CUDA_TRY(cudaMemcpyAsync(y_host, base + h.y, (size_t)(M * N * 2), cudaMemcpyDeviceToHost, s));
   return SACQ_OK;

@@ -95,7 +95,10 @@ struct BcastDst {
 // `residual` (bf16 [M, ldr], may be null) is added to the rounded output in every GEMM epilogue.
 int launch_small_m(const sacq_layer* L, const void* q, const float* scale, int64_t M, void* y, int64_t ldy,
                    void* ws, int64_t ws_bytes, cudaStream_t s, const void* residual = nullptr, int64_t ldr = 0,
-                   int act_int8 = 0, const BcastDst* bc = nullptr);
+                   int act_int8 = 0, const BcastDst* bc = nullptr, const void* x = nullptr, int64_t x_pitch = 0);
+// Warps per CTA if M tokens run on a staged warp-MMA kernel, which can quantize its activations itself (`x`, bf16 rows
+// that are 16-byte aligned, instead of q and scale); else 0.
+int small_m_staged_warps(const sacq_layer* L, int64_t M);
 
 int launch_small_m_multi(const sacq_layer* const* layers, int n, const void* q, const float* scale, int64_t M,
                          void* const* ys, const int64_t* ldys, cudaStream_t s);

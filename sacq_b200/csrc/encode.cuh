@@ -41,7 +41,9 @@ __device__ __forceinline__ float pair_hi(uint32_t w) { return __uint_as_float(w 
 // 34(1), 1990: with r = RN(1/s) and q within one ulp of z / s the residual is exact and q' is RN(z / s)).  The first
 // correction brings q within an ulp, the second makes it exact for any s.  (Locating the quotient between z r(1 - e)
 // and z r(1 + e) and dividing only where the two encode differently is not faster: scales are quotients of 8-bit
-// significands by 127 and 448, so exact ties are common, and every warp met one.)
+// significands by 127 and 448, so exact ties are common, and every warp met one.)  Checked against the division over
+// the whole domain of the activation quantizers: every finite bf16 maximum, both formats, every bf16 value up to it
+// (2.1 G quotients each), no byte differs.
 struct RowDivisor {
   float s, r;
   bool fast;                    // s in 2^-80 .. 2^80: every residual that can matter is exact; else divide
@@ -58,6 +60,17 @@ __device__ __forceinline__ uint64_t quotient2(uint64_t z, uint64_t ns, uint64_t 
   uint64_t q = mul2(z, r);
   q = fma2(fma2(q, ns, z), r, q);
   return fma2(fma2(q, ns, z), r, q);
+}
+
+// Scale of a row from its largest |x|: a NaN maximum fails `> 0` like in the reference's torch.where, so the row
+// keeps scale 1 and its NaN elements stay NaN; an infinite maximum gives an infinite scale.  Both divide
+// (the elements of the first are not bounded by its scale).
+template <bool I8>
+__device__ __forceinline__ RowDivisor scale_of(float mx) {
+  const bool ordinary = mx > 0.f;
+  RowDivisor d = row_divisor(ordinary ? __fdiv_rn(mx, I8 ? 127.0f : kE4M3Max) : 1.0f);
+  d.fast = d.fast && ordinary;
+  return d;
 }
 
 // Two encoded values of one row -> two bytes, by IEEE division.  I8: round-half-to-even to int8 in [-127, 127]

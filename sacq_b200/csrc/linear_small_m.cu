@@ -573,6 +573,11 @@ bool small_m_supported(const sacq_layer* L) {
   return L->d.index_bits <= 24 && L->d.vector_dim <= 64;
 }
 
+int small_m_staged_warps(const sacq_layer* L, int64_t M) {
+  const Plan pl = make_plan(L, M);
+  return pl.staged && !has_shift(L) ? pl.warps : 0;
+}
+
 int64_t small_m_workspace_bytes(const sacq_layer* L, int64_t M) {
   if (M <= 0) return sacq_workspace_counter_bytes();
   const Plan pl = make_plan(L, M);
@@ -625,7 +630,7 @@ SmallMParams fill_params(const sacq_layer* L, const Plan& pl, const void* q, con
 
 int launch_small_m(const sacq_layer* L, const void* q, const float* scale, int64_t M, void* y, int64_t ldy,
                    void* ws, int64_t ws_bytes, cudaStream_t s, const void* residual, int64_t ldr, int act_int8,
-                   const BcastDst* bc) {
+                   const BcastDst* bc, const void* x, int64_t x_pitch) {
   const sacq_layer_desc& d = L->d;
   if (M == 0 || d.out_features == 0) return SACQ_OK;
   if (M > (1 << 20)) return set_error(SACQ_ERR_UNSUPPORTED, "small-M kernel: M=%lld too large", (long long)M);
@@ -651,6 +656,9 @@ int launch_small_m(const sacq_layer* L, const void* q, const float* scale, int64
   p.residual = static_cast<const uint16_t*>(residual);
   p.ldr = ldr;
   p.act_int8 = act_int8;
+  p.x = static_cast<const uint16_t*>(x);
+  p.x_pitch = x_pitch;
+  if (x != nullptr && !pl.staged) return set_error(SACQ_ERR_UNSUPPORTED, "only the staged warp-MMA variants quantize");
   if (bc != nullptr) {
     p.n_bc = bc->n;
     for (int i = 0; i < bc->n; ++i) p.ybc[i] = static_cast<uint16_t*>(bc->ptr[i]);

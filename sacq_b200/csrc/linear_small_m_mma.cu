@@ -298,7 +298,7 @@ __host__ __device__ inline StagedLayout staged_layout(int C, int D, int K, int64
   L.idx_off = (uint32_t)((C * D * 2 + 127) & ~127);
   L.act_off = L.idx_off + 2 * (uint32_t)((8 * r8 * (row_bytes + staged_idx_pad(row_bytes)) + 127) & ~127);
   L.red_off = L.act_off + (uint32_t)act_bufs * (uint32_t)((16 * (K + kActPad) + 127) & ~127);
-  L.sa_off = L.red_off + (uint32_t)(warps * r8 * 4 * 32 * 4);
+  L.sa_off = (L.red_off + (uint32_t)(warps * r8 * 4 * kRedPitch * 4) + 15) & ~15u;
   L.bar_off = L.sa_off + 512;             // 16 token scales + 48 row scales + 48 row biases
   L.total = L.bar_off + 64;
   return L;
@@ -421,7 +421,10 @@ __device__ __forceinline__ void staged_body(const SmallMParams& p, const int cta
   asm volatile("griddepcontrol.wait;" ::: "memory");                // activations come from that kernel
   SACQ_ST(2);
   SACQ_TL(t_dep);
-  if (threadIdx.x < 16 && first_rt < p.row_blocks) {
+  if (p.x != nullptr) {
+    quantize_tokens(p.x + (int64_t)m_base * p.x_pitch, p.x_pitch, p.K, toks_here, act_s, act_pitch, sa_s,
+                    reinterpret_cast<uint32_t*>(red));
+  } else if (threadIdx.x < 16 && first_rt < p.row_blocks) {
     issue_act(chunk, 0);
     sa_s[threadIdx.x] = threadIdx.x < toks_here ? __ldg(p.act_scale + m_base + threadIdx.x) : 0.f;
   }
@@ -456,7 +459,7 @@ __device__ __forceinline__ void staged_body(const SmallMParams& p, const int cta
     if (first) {
       ok = mbar_wait_bounded(bar_cb, 0, p.status) && ok;
       SACQ_ST(3);
-      ok = mbar_wait_bounded(bar_act0, 0, p.status) && ok;
+      if (p.x == nullptr) ok = mbar_wait_bounded(bar_act0, 0, p.status) && ok;
       SACQ_ST(4);
       SACQ_TL(t_ready);
       first = false;
@@ -607,22 +610,25 @@ __device__ __forceinline__ void staged_body(const SmallMParams& p, const int cta
     SACQ_ST(8 + 6 * it + 2);
 #pragma unroll
     for (int r = 0; r < R8; ++r) {
-      red[(warp * kFrag + r * 4 + 0) * 32 + lane] = fmaf(acc[r][0], p.out_mul, p.shift * xs_a);
-      red[(warp * kFrag + r * 4 + 1) * 32 + lane] = fmaf(acc[r][1], p.out_mul, p.shift * xs_a);
-      red[(warp * kFrag + r * 4 + 2) * 32 + lane] = fmaf(acc[r][2], p.out_mul, p.shift * xs_b);
-      red[(warp * kFrag + r * 4 + 3) * 32 + lane] = fmaf(acc[r][3], p.out_mul, p.shift * xs_b);
+      red[(warp * kFrag + r * 4 + 0) * kRedPitch + lane] = fmaf(acc[r][0], p.out_mul, p.shift * xs_a);
+      red[(warp * kFrag + r * 4 + 1) * kRedPitch + lane] = fmaf(acc[r][1], p.out_mul, p.shift * xs_a);
+      red[(warp * kFrag + r * 4 + 2) * kRedPitch + lane] = fmaf(acc[r][2], p.out_mul, p.shift * xs_b);
+      red[(warp * kFrag + r * 4 + 3) * kRedPitch + lane] = fmaf(acc[r][3], p.out_mul, p.shift * xs_b);
     }
     __syncthreads();
     SACQ_ST(8 + 6 * it + 3);
-    for (int e = threadIdx.x; e < kFrag * 32; e += blockDim.x) {
-      float v = 0.f;
-      for (int w = 0; w < nwarps; ++w) v += red[w * kFrag * 32 + e];
-      const int ln = e & 31, j = (e >> 5) & 3, r = e >> 7;
-      const int ml = (ln >> 2) + ((j & 2) ? 8 : 0);
-      const int n = n_base + r * 8 + 2 * (ln & 3) + (j & 1);
-      if (ml < toks_here && n < p.N) {
-        store_out(p, m_base + ml, n, fmaf(sa_s[ml], v, rowb_s[n - n_base]));
+    // two neighbouring outputs per thread, a token's 8 * R8 outputs by consecutive threads
+    for (int e = threadIdx.x; e < kFrag * 16; e += blockDim.x) {
+      const int tt = e & 3, r = (e >> 2) % R8, ml = (e >> 2) / R8;
+      const float* src = red + (r * 4 + (ml >= 8 ? 2 : 0)) * kRedPitch + (ml & 7) * 4 + tt;
+      float v0 = 0.f, v1 = 0.f;
+      for (int w = 0; w < nwarps; ++w) {
+        v0 += src[w * kFrag * kRedPitch];
+        v1 += src[w * kFrag * kRedPitch + kRedPitch];
       }
+      const int nl = r * 8 + 2 * tt, n = n_base + nl;
+      if (ml < toks_here && n < p.N)
+        store_out2(p, m_base + ml, n, fmaf(sa_s[ml], v0, rowb_s[nl]), fmaf(sa_s[ml], v1, rowb_s[nl + 1]), n + 1 < p.N);
     }
     SACQ_ST(8 + 6 * it + 4);
     __syncthreads();                                   // red and the row constants are reused next

@@ -90,7 +90,7 @@ __host__ __device__ inline UnpLayout unp_layout(int C, int D, int K, int64_t row
   L.act_pitch = (uint32_t)(K + kActPadU);
   L.sc_off = L.act_off + (uint32_t)((16 * L.act_pitch + 127) & ~127);
   L.red_off = L.sc_off + (uint32_t)((rows * num_groups * 4 + 127) & ~127);
-  L.sa_off = L.red_off + (uint32_t)(warps * r8 * 4 * 32 * 4);
+  L.sa_off = (L.red_off + (uint32_t)(warps * r8 * 4 * kRedPitch * 4) + 15) & ~15u;
   L.bar_off = L.sa_off + 256;                                          // 16 token scales + up to 48 row biases
   L.total = L.bar_off + 64;
   return L;
@@ -153,7 +153,10 @@ __global__ void __launch_bounds__(kMaxWarpsU * 32, 1) small_m_mma_unpacked_kerne
   // from here on (its launch latency overlaps this grid); it waits for this grid before it touches memory
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");                  // activations come from that kernel
-  if (threadIdx.x < 16 && first_rt < p.row_blocks) {
+  if (p.x != nullptr) {
+    quantize_tokens(p.x + (int64_t)m_base * p.x_pitch, p.x_pitch, p.K, toks_here, act_s, (int)L.act_pitch, sa_s,
+                    reinterpret_cast<uint32_t*>(red));
+  } else if (threadIdx.x < 16 && first_rt < p.row_blocks) {
     const int m = threadIdx.x;
     if (m < toks_here) bulk_g2s(act_s + m * L.act_pitch, p.q + (int64_t)(m_base + m) * p.K, (uint32_t)p.K, bar_act);
     if (m == 0) mbar_expect_u(bar_act, (uint32_t)(toks_here * p.K));
@@ -181,7 +184,7 @@ __global__ void __launch_bounds__(kMaxWarpsU * 32, 1) small_m_mma_unpacked_kerne
     }
     if (first) {
       ok = mbar_wait_u(bar_cb, 0, p.status) && ok;
-      ok = mbar_wait_u(bar_act, 0, p.status) && ok;
+      if (p.x == nullptr) ok = mbar_wait_u(bar_act, 0, p.status) && ok;
       first = false;
     }
     ok = mbar_wait_u(bar_pk0 + 8 * buf, pk_parity[buf], p.status) && ok;
@@ -286,20 +289,24 @@ __global__ void __launch_bounds__(kMaxWarpsU * 32, 1) small_m_mma_unpacked_kerne
     // ---- K reduction across the CTA's warps, then the epilogue
 #pragma unroll
     for (int r = 0; r < R8; ++r) {
-      red[(warp * kFrag + r * 4 + 0) * 32 + lane] = fmaf(acc[r][0], p.out_mul, p.shift * xs_a);
-      red[(warp * kFrag + r * 4 + 1) * 32 + lane] = fmaf(acc[r][1], p.out_mul, p.shift * xs_a);
-      red[(warp * kFrag + r * 4 + 2) * 32 + lane] = fmaf(acc[r][2], p.out_mul, p.shift * xs_b);
-      red[(warp * kFrag + r * 4 + 3) * 32 + lane] = fmaf(acc[r][3], p.out_mul, p.shift * xs_b);
+      red[(warp * kFrag + r * 4 + 0) * kRedPitch + lane] = fmaf(acc[r][0], p.out_mul, p.shift * xs_a);
+      red[(warp * kFrag + r * 4 + 1) * kRedPitch + lane] = fmaf(acc[r][1], p.out_mul, p.shift * xs_a);
+      red[(warp * kFrag + r * 4 + 2) * kRedPitch + lane] = fmaf(acc[r][2], p.out_mul, p.shift * xs_b);
+      red[(warp * kFrag + r * 4 + 3) * kRedPitch + lane] = fmaf(acc[r][3], p.out_mul, p.shift * xs_b);
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < kFrag * 32; e += blockDim.x) {
-      float v = 0.f;
-      for (int w = 0; w < nwarps; ++w) v += red[w * kFrag * 32 + e];   // fixed order: deterministic
-      const int ln = e & 31, j = (e >> 5) & 3, r = e >> 7;
-      const int ml = (ln >> 2) + ((j & 2) ? 8 : 0);
-      const int nl = r * 8 + 2 * (ln & 3) + (j & 1);
-      if (ml < toks_here && n_base + nl < p.N)
-        store_out(p, m_base + ml, n_base + nl, fmaf(sa_s[ml], v, rowb_s[nl]));
+    // two neighbouring outputs per thread, a token's 8 * R8 outputs by consecutive threads
+    for (int e = threadIdx.x; e < kFrag * 16; e += blockDim.x) {
+      const int tt = e & 3, r = (e >> 2) % R8, ml = (e >> 2) / R8;
+      const float* src = red + (r * 4 + (ml >= 8 ? 2 : 0)) * kRedPitch + (ml & 7) * 4 + tt;
+      float v0 = 0.f, v1 = 0.f;
+      for (int w = 0; w < nwarps; ++w) {                              // fixed order: deterministic
+        v0 += src[w * kFrag * kRedPitch];
+        v1 += src[w * kFrag * kRedPitch + kRedPitch];
+      }
+      const int nl = r * 8 + 2 * tt, n = n_base + nl;
+      if (ml < toks_here && n < p.N)
+        store_out2(p, m_base + ml, n, fmaf(sa_s[ml], v0, rowb_s[nl]), fmaf(sa_s[ml], v1, rowb_s[nl + 1]), n + 1 < p.N);
     }
     __syncthreads();                                                  // red, indices and row constants are reused
   }

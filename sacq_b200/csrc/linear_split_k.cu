@@ -269,7 +269,7 @@ __device__ long long g_split_trace[64];
 #endif
 
 // grid = (row tiles x split, token tiles, layers), clusters of `split` CTAs along x.
-template <int D, int MODE>
+template <int D, int MODE, bool CB_SMEM>
 __global__ void __launch_bounds__(kCtaThreads, 1)
 split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ SplitParams p) {
   constexpr uint32_t kTmemCols = 512;
@@ -288,7 +288,8 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* sm = smem_raw + (base - raw);
   const uint32_t cb_bytes = (uint32_t)(p.C * CW_BYTES);
-  const SplitLayout L = split_layout(p.tok, S, p.act_stages, p.max_slices, F16 || RECIPE ? p.max_groups : 0, (int)cb_bytes);
+  const SplitLayout L = split_layout(p.tok, S, p.act_stages, p.max_slices, F16 || RECIPE ? p.max_groups : 0,
+                                     CB_SMEM ? (int)cb_bytes : 0);
 
   constexpr int ACT_FULL = 0, ACT_EMPTY = kMaxAct, W_FULL = 2 * kMaxAct, W_EMPTY = W_FULL + kMaxW, IDX_FULL = W_EMPTY + kMaxW,
                 CB_FULL = IDX_FULL + 1, ACC_FULL = IDX_FULL + 2;
@@ -335,8 +336,10 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     if (elect_one()) {
       mbar_arrive_expect_tx(bar(IDX_FULL), (uint32_t)(p.max_slices * kSliceBytes));
       tma_load_3d(base + L.idx_off, &p.idx[blockIdx.z], 0, n0, slice0, bar(IDX_FULL));
-      mbar_arrive_expect_tx(bar(CB_FULL), cb_bytes);
-      bulk_load(base + L.cb_off, lay.cb, cb_bytes, bar(CB_FULL));
+      if constexpr (CB_SMEM) {
+        mbar_arrive_expect_tx(bar(CB_FULL), cb_bytes);
+        bulk_load(base + L.cb_off, lay.cb, cb_bytes, bar(CB_FULL));
+      }
       prefetch_tensormap(&tmap_a);
     }
   }
@@ -450,11 +453,18 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       }
     }
     xbarrier();
-    const uint8_t* cbs = sm + L.cb_off;
+    const uint8_t* cbs = CB_SMEM ? sm + L.cb_off : lay.cb;
+    auto codeword16 = [&](uint32_t i) {
+      return CB_SMEM ? *reinterpret_cast<const uint4*>(cbs + i * 16) : __ldg(reinterpret_cast<const uint4*>(cbs) + i);
+    };
+    auto codeword8 = [&](uint32_t i) {
+      return CB_SMEM ? *reinterpret_cast<const uint2*>(cbs + i * 8) : __ldg(reinterpret_cast<const uint2*>(cbs) + i);
+    };
     const uint8_t* rowidx = sm + L.idx_off + row * 16;
     const uint32_t mask = (1u << p.bits) - 1u;
     const int bits = p.bits;
-    ok = mbar_wait(bar(IDX_FULL), 0, abort_flag, lay.status) && mbar_wait(bar(CB_FULL), 0, abort_flag, lay.status);
+    ok = mbar_wait(bar(IDX_FULL), 0, abort_flag, lay.status) &&
+         (!CB_SMEM || mbar_wait(bar(CB_FULL), 0, abort_flag, lay.status));
     if (et == 0) SACQ_SPT(3);
     int grp = 0, grp_end = GROUPS ? (g_first + 1) * p.group_size - kb0 * kStageK : 0;    // k (in the slice) at which the scale changes
     // One stage's 16 words of this thread.  The next stage's words are gathered before the wait for this
@@ -477,10 +487,10 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
           for (int j = 0; j < IPT; ++j) {
             const uint32_t i = (uint32_t)(win >> (j * bits)) & mask;
             if constexpr (D == 8) {
-              const uint4 v = *reinterpret_cast<const uint4*>(cbs + i * 16);
+              const uint4 v = codeword16(i);
               pair[4 * j] = v.x; pair[4 * j + 1] = v.y; pair[4 * j + 2] = v.z; pair[4 * j + 3] = v.w;
             } else {
-              const uint2 v = *reinterpret_cast<const uint2*>(cbs + i * 8);
+              const uint2 v = codeword8(i);
               pair[2 * j] = v.x; pair[2 * j + 1] = v.y;
             }
           }
@@ -500,10 +510,10 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             const uint32_t i = (uint32_t)(win >> (j * bits)) & mask;
             uint32_t c[D / 2];
             if constexpr (D == 8) {
-              const uint4 v = *reinterpret_cast<const uint4*>(cbs + i * 16);
+              const uint4 v = codeword16(i);
               c[0] = v.x; c[1] = v.y; c[2] = v.z; c[3] = v.w;
             } else {
-              const uint2 v = *reinterpret_cast<const uint2*>(cbs + i * 8);
+              const uint2 v = codeword8(i);
               c[0] = v.x; c[1] = v.y;
             }
 #pragma unroll
@@ -522,11 +532,11 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
           for (int j = 0; j < 4; ++j) {
             const uint32_t i = (uint32_t)(win >> (j * bits)) & mask;
             if constexpr (D == 8) {
-              const uint4 c = *reinterpret_cast<const uint4*>(cbs + i * 16);
+              const uint4 c = codeword16(i);
               w[2 * j] = c.x; w[2 * j + 1] = c.y;
               w[8 + 2 * j] = c.z; w[8 + 2 * j + 1] = c.w;
             } else {
-              const uint2 c = *reinterpret_cast<const uint2*>(cbs + i * 8);
+              const uint2 c = codeword8(i);
               w[4 * v + j] = c.x;
               w[8 + 4 * v + j] = c.y;
             }
@@ -662,13 +672,13 @@ int active_clusters(int split, int num_sms) {
   return split == 8 ? num_sms * 15 / 148 : split == 4 ? num_sms * 33 / 148 : num_sms / split;
 }
 
-template <int D, int MODE>
+template <int D, int MODE, bool CB_SMEM>
 cudaError_t launch_kernel(const CUtensorMap& ta, const SplitParams& p, dim3 grid, size_t smem, cudaStream_t s) {
   static bool configured[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || !configured[dev]) {
-    const cudaError_t e = cudaFuncSetAttribute(split_k_kernel<D, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    const cudaError_t e = cudaFuncSetAttribute(split_k_kernel<D, MODE, CB_SMEM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
@@ -686,7 +696,24 @@ cudaError_t launch_kernel(const CUtensorMap& ta, const SplitParams& p, dim3 grid
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = p.split > 1 ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, split_k_kernel<D, MODE>, ta, p);
+  return cudaLaunchKernelEx(&cfg, split_k_kernel<D, MODE, CB_SMEM>, ta, p);
+}
+
+template <int D, bool CB_SMEM>
+cudaError_t launch_mode(SplitMode mode, const CUtensorMap& ta, const SplitParams& p, dim3 grid, size_t smem, cudaStream_t s) {
+  switch (mode) {
+    case kSplitHiLo: return launch_kernel<D, kSplitHiLo, CB_SMEM>(ta, p, grid, smem, s);
+    case kSplitHalf: return launch_kernel<D, kSplitHalf, CB_SMEM>(ta, p, grid, smem, s);
+    case kSplitInt8: return launch_kernel<D, kSplitInt8, CB_SMEM>(ta, p, grid, smem, s);
+    default: return launch_kernel<D, kSplitFp8, CB_SMEM>(ta, p, grid, smem, s);
+  }
+}
+
+// Shared memory of the codebook: tables above 64 KB (65,536 entries) are gathered from global memory, where they stay
+// in L2.
+int codebook_smem(const sacq_layer* L) {
+  const int64_t bytes = (int64_t)L->cb_entries * L->d.vector_dim * 2;
+  return bytes <= 64 * 1024 ? (int)bytes : 0;
 }
 
 // Index slices and scale groups of the largest K slice.
@@ -712,7 +739,7 @@ int slices_for(int64_t K) { return K < 1024 ? 1 : K < 4096 ? 2 : K < 8192 ? 4 : 
 
 // Completes a choice of tokens and slices; false if it does not fit shared memory.
 bool split_fits(const sacq_layer* L, SplitMode mode, SplitChoice* c) {
-  const int cb_bytes = L->cb_entries * L->d.vector_dim * 2, groups = mode == kSplitHiLo ? 0 : 1;
+  const int cb_bytes = codebook_smem(L), groups = mode == kSplitHiLo ? 0 : 1;
   slice_extent(L, c->split, &c->max_slices, &c->max_groups);
   const int tiles = ((int)(L->d.in_features / kStageK) + c->split - 1) / c->split * (mode == kSplitHalf ? 2 : 1);
   for (c->act_stages = tiles < 2 ? 2 : tiles < kMaxAct ? tiles : kMaxAct; c->act_stages >= 2; --c->act_stages)
@@ -723,8 +750,9 @@ bool split_fits(const sacq_layer* L, SplitMode mode, SplitChoice* c) {
 
 // Time of one CTA with `tok` tokens and `kbs` weight stages (us): prologue, the slower of expansion, MMAs and
 // activation tiles per stage, reduction.
-double split_cta_us(int vector_dim, SplitMode mode, int tok, int kbs, int split) {
+double split_cta_us(int vector_dim, SplitMode mode, bool cb_smem, int tok, int kbs, int split) {
   double stage = mode >= kSplitInt8 ? 0.75 : vector_dim == 8 ? 0.48 : 0.6;
+  if (!cb_smem) stage = 8.0 / vector_dim;             // gathers from L2
   if (0.002 * tok > stage) stage = 0.002 * tok;
   return 2.5 + kbs * stage + 0.015 * tok + (split > 1 ? 0.8 : 0.0);
 }
@@ -739,8 +767,7 @@ bool split_k_choose(const sacq_layer* L, int64_t M, SplitMode mode, SplitChoice*
   if (mode == kSplitHiLo ? L->num_groups != 1 : d.group_size % (mode == kSplitHalf ? 64 : 16) != 0) return false;
   // the recipes read the codebook as it came, which is not padded to whole 16-byte units
   if (mode >= kSplitInt8 && d.codebook_size * d.vector_dim % 8 != 0) return false;
-  const int cb_bytes = L->cb_entries * d.vector_dim * 2;
-  if (cb_bytes % 16 != 0 || M <= 0 || M > (1 << 20)) return false;
+  if ((int64_t)L->cb_entries * d.vector_dim * 2 % 16 != 0 || M <= 0 || M > (1 << 20)) return false;
   const int nkb = (int)(d.in_features / kStageK);
   const int64_t row_tiles = (d.out_features + kRows - 1) / kRows;
   const int slices = slices_for(d.in_features);
@@ -762,7 +789,7 @@ bool split_k_choose(const sacq_layer* L, int64_t M, SplitMode mode, SplitChoice*
       const int64_t waves = (row_tiles * c.tiles + at_once - 1) / at_once;
       // every CTA fetches the codebook through L2
       const int64_t ctas = row_tiles * c.tiles * split, resident = waves * L->num_sms;
-      c.us = waves * split_cta_us(d.vector_dim, mode, tok, kbs, split) + 0.01 * (double)(ctas < resident ? ctas : resident);
+      c.us = waves * split_cta_us(d.vector_dim, mode, codebook_smem(L) > 0, tok, kbs, split) + 0.01 * (double)(ctas < resident ? ctas : resident);
       if (c.us < out->us) *out = c;
     }
   }
@@ -779,6 +806,8 @@ bool split_k_choose(const sacq_layer* L, int64_t M, SplitMode mode, SplitChoice*
 #endif
   return out->tok != 0;
 }
+
+bool split_k_codebook_in_smem(const sacq_layer* L) { return codebook_smem(L) > 0; }
 
 bool split_k_choose_multi(const sacq_layer* const* layers, int n, int64_t M, SplitMode mode, SplitChoice* out) {
   const sacq_layer_desc& d0 = layers[0]->d;
@@ -845,15 +874,10 @@ int launch_split_k(const sacq_layer* const* layers, int n, const void* act, cons
   p.split = c.split; p.parts = c.parts; p.tok = c.tok; p.act_stages = c.act_stages; p.max_slices = c.max_slices; p.max_groups = c.max_groups;
   const dim3 grid((unsigned)((widest + kRows - 1) / kRows * c.split), (unsigned)c.tiles, (unsigned)n);
   const size_t smem = split_smem(split_layout(c.tok, c.split, c.act_stages, c.max_slices, mode == kSplitHiLo ? 0 : c.max_groups,
-                                              layers[0]->cb_entries * d0.vector_dim * 2));
-  cudaError_t e;
-  const bool d8 = d0.vector_dim == 8;
-  switch (mode) {
-    case kSplitHiLo: e = d8 ? launch_kernel<8, kSplitHiLo>(ta, p, grid, smem, s) : launch_kernel<4, kSplitHiLo>(ta, p, grid, smem, s); break;
-    case kSplitHalf: e = d8 ? launch_kernel<8, kSplitHalf>(ta, p, grid, smem, s) : launch_kernel<4, kSplitHalf>(ta, p, grid, smem, s); break;
-    case kSplitInt8: e = d8 ? launch_kernel<8, kSplitInt8>(ta, p, grid, smem, s) : launch_kernel<4, kSplitInt8>(ta, p, grid, smem, s); break;
-    default: e = d8 ? launch_kernel<8, kSplitFp8>(ta, p, grid, smem, s) : launch_kernel<4, kSplitFp8>(ta, p, grid, smem, s); break;
-  }
+                                              codebook_smem(layers[0])));
+  const bool cb = codebook_smem(layers[0]) > 0;
+  const cudaError_t e = d0.vector_dim == 8 ? (cb ? launch_mode<8, true>(mode, ta, p, grid, smem, s) : launch_mode<8, false>(mode, ta, p, grid, smem, s))
+                                           : (cb ? launch_mode<4, true>(mode, ta, p, grid, smem, s) : launch_mode<4, false>(mode, ta, p, grid, smem, s));
   count_launch();
   if (e != cudaSuccess) return cuda_fail(e, "split-K launch");
   return SACQ_OK;

@@ -7,6 +7,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "encode.cuh"
 
 namespace sacq {
 namespace smallm {
@@ -22,6 +23,8 @@ struct SmallMParams {
   const uint16_t* scales;      // bf16 [N, num_groups]
   const uint16_t* bias;        // bf16 [N] or null
   const uint8_t* q;            // e4m3 [M, K]
+  const uint16_t* x;           // staged kernels: bf16 [M, x_pitch] to be quantized here instead of reading q, or null
+  int64_t x_pitch;
   int* status;                 // layer status word (bounded waits report here)
   const float* act_scale;      // [M]
   uint16_t* y;                 // bf16 [M, ldy]
@@ -79,6 +82,80 @@ __device__ __forceinline__ void store_out(const SmallMParams& p, int64_t m, int6
     o = float_to_bf16_bits(__fadd_rn(bf16_bits_to_float(o), bf16_bits_to_float(__ldg(p.residual + m * p.ldr + n))));
   p.y[m * p.ldy + n] = o;
   for (int i = 0; i < p.n_bc; ++i) p.ybc[i][m * p.ldy + n] = o;
+}
+
+// Two neighbouring outputs (n, n + 1) of one token; `two`: the second one exists.
+__device__ __forceinline__ void store_out2(const SmallMParams& p, int64_t m, int64_t n, float v0, float v1, bool two) {
+  uint16_t* y = p.y + m * p.ldy + n;
+  if (two && p.residual == nullptr && p.n_bc == 0 && (reinterpret_cast<uintptr_t>(y) & 3) == 0) {
+    *reinterpret_cast<__nv_bfloat162*>(y) = __floats2bfloat162_rn(v0, v1);
+    return;
+  }
+  store_out(p, m, n, v0);
+  if (two) store_out(p, m, n + 1, v1);
+}
+
+// Words between the 32-lane fragment rows of the cross-warp reduction: one more than the lanes, so that lanes which
+// read the same column of different 8-row sub-blocks fall on different banks.
+constexpr int kRedPitch = 33;
+
+// The activation quantizer inside a staged kernel: tokens [0, toks) of x -> e4m3 rows in shared memory and their
+// scales, the bytes of quant_act_kernel.  Called by all threads of the CTA; `tmp` has a word per warp.  Every CTA
+// quantizes the (at most 16) tokens it multiplies, while its codebook and index copies are in flight: for a few tokens
+// that is quicker than a launch of its own, which costs the host 2 us and the GPU one more dependent kernel.
+__device__ __forceinline__ void quantize_tokens(const uint16_t* x, int64_t pitch, int K, int toks, uint8_t* act, int act_pitch,
+                                                float* scales, uint32_t* tmp) {
+  constexpr int kKeep = 4;                            // 16-byte chunks a lane holds between the two passes
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+  const int wpt = toks < nwarps ? nwarps / toks : 1;  // warps per token
+  const int step = 32 * wpt, chunks = K >> 3;
+  for (int t0 = 0; t0 < toks; t0 += nwarps / wpt) {   // more than one round only with one warp per token
+    const int tok = t0 + warp / wpt;
+    const bool live = warp / wpt < nwarps / wpt && tok < toks;
+    const uint4* row = reinterpret_cast<const uint4*>(x + (int64_t)(live ? tok : 0) * pitch);
+    const int c0 = (warp % wpt) * 32 + lane;
+    uint32_t mx = 0u;
+    auto take = [&](const uint4& v) {
+      mx = __vmaxu2(mx, v.x & 0x7fff7fffu);
+      mx = __vmaxu2(mx, v.y & 0x7fff7fffu);
+      mx = __vmaxu2(mx, v.z & 0x7fff7fffu);
+      mx = __vmaxu2(mx, v.w & 0x7fff7fffu);
+    };
+    uint4 keep[kKeep];
+#pragma unroll
+    for (int i = 0; i < kKeep; ++i)
+      keep[i] = live && c0 + i * step < chunks ? __ldg(row + c0 + i * step) : make_uint4(0, 0, 0, 0);
+    if (live) {
+#pragma unroll 4
+      for (int c = c0 + kKeep * step; c < chunks; c += step) take(__ldg(row + c));
+    }
+#pragma unroll
+    for (int i = 0; i < kKeep; ++i) take(keep[i]);
+    uint32_t m = warp_max_bits(max(mx << 16, mx & 0xffff0000u));
+    if (wpt > 1) {
+      if (lane == 0) tmp[warp] = m;
+      __syncthreads();
+      const int first = warp / wpt * wpt;
+      for (int w = 0; w < wpt; ++w)
+        if (first + w < nwarps) m = max(m, tmp[first + w]);
+    }
+    const RowDivisor d = scale_of<false>(__uint_as_float(m));
+    if (live) {
+      if (lane == 0 && warp % wpt == 0) scales[tok] = d.s;
+      uint2* out = reinterpret_cast<uint2*>(act + tok * act_pitch);
+      auto put = [&](int c, const uint4& v) {
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+        uint32_t o[2];
+        encode_pairs<false, 4>(w, d, o);
+        out[c] = make_uint2(o[0], o[1]);
+      };
+#pragma unroll
+      for (int i = 0; i < kKeep; ++i)
+        if (c0 + i * step < chunks) put(c0 + i * step, keep[i]);
+#pragma unroll 2
+      for (int c = c0 + kKeep * step; c < chunks; c += step) put(c, __ldg(row + c));
+    }
+  }
 }
 
 __device__ __forceinline__ __half2 as_h2(uint32_t v) { return *reinterpret_cast<__half2*>(&v); }

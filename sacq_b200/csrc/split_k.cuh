@@ -34,6 +34,8 @@ bool split_k_choose_multi(const sacq_layer* const* layers, int n, int64_t M, Spl
 int launch_split_k(const sacq_layer* const* layers, int n, const void* act, const float* scale, int64_t M, void* const* ys,
                    const int64_t* ldys, SplitMode mode, const SplitChoice& c, cudaStream_t s, const void* residual = nullptr,
                    int64_t ldr = 0, const BcastDst* bc = nullptr, const float* row_scale = nullptr);
+// Whether the layer's codebook fits the kernel's shared memory (else it is gathered from L2).
+bool split_k_codebook_in_smem(const sacq_layer* L);
 void split_k_release(sacq_layer* L);
 
 }  // namespace sacq
