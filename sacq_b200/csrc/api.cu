@@ -494,13 +494,16 @@ SACQ_API int64_t sacq_workspace_bytes_w8a8(const sacq_layer_t* L, int64_t M) {
 }
 
 namespace {
-// Up to a few hundred tokens the recipes run as one kernel whose expanders make the weight bytes on the way to the
-// tensor cores; above, making them once for all token tiles and a dense GEMM is faster (quantizer included,
-// 2048x6144 at d = 4: 33 / 34 us at 512 tokens, 44 / 36 at 1,000; 6144x2048 50 / 52 and 2048x2048 24 / 28 at 1,000).
+// Few tokens run as one kernel, whose expanders make the weight bytes on the way to the tensor cores; for more, making
+// them once for all tiles and a dense GEMM is faster, except where the layer's own row tiles fill the chip and one token
+// tile holds the call (quantizer included, 6144 -> 2048: 14.3 / 23.0 us at 16 tokens, 21.9 / 20.8 at 200; 2048 -> 6144:
+// 16.7 / 17.0 at 200, 17.6 / 19.7 at 300, 27.7 / 21.1 at 400; with a codebook of 65,536 entries 20.2 / 20.1 at 200).
 bool recipe_in_one(const sacq_layer* L, const void* q, const float* act_scale, const float* w_scale, int64_t M, void* y,
                    int64_t ldy, SplitMode mode, cudaStream_t s, int* rc) {
   SplitChoice c;
-  if (M > (L->d.out_features >= 4096 || !split_k_codebook_in_smem(L) ? 512 : 1024) || reinterpret_cast<uintptr_t>(q) % 16 != 0 || reinterpret_cast<uintptr_t>(L->d.codebook) % 16 != 0 ||
+  const bool wide = L->d.out_features >= 4096 && L->d.in_features >= 2048;
+  if (M > (!wide ? 32 : split_k_codebook_in_smem(L) ? 320 : 200) || reinterpret_cast<uintptr_t>(q) % 16 != 0 ||
+      reinterpret_cast<uintptr_t>(L->d.codebook) % 16 != 0 ||
       (mode == kSplitInt8 && L->d.in_features * 127 * 127 > 2147483647LL) || !split_k_choose(L, M, mode, &c))
     return false;
   *rc = launch_split_k(&L, 1, q, act_scale, M, &y, &ldy, mode, c, s, nullptr, 0, nullptr, w_scale);
