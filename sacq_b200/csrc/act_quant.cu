@@ -241,17 +241,39 @@ namespace {
 
 __device__ __forceinline__ float round_bf16(float v) { return bf16_bits_to_float(float_to_bf16_bits(v)); }
 
+// fp32 silu of a bf16 value.  The quotient of the approximate exponential and division rounds to the bf16 value of
+// a / (1 + expf(-a)) for every bf16 a (all 65,536 compared), but where the divisor is out of __fdividef's range.  The
+// plain form, an IEEE division per element, bounded the kernel
+// (8,192 rows of 6,144: 73.8 us, now 50.3; 300 rows: 6.4, now 5.0).
+__device__ __forceinline__ float silu(float a) {
+  return a < -87.0f ? a / (1.0f + expf(-a)) : __fdividef(a, 1.0f + __expf(-a));
+}
+
 // KIND 0: bf16(bf16(silu(a)) * b); KIND 1: bf16(gelu(a)), erf form;
 // KIND 2: bf16(bf16(a * bf16(1 + b)) + c), the AdaLN modulation a * (1 + scale) + shift.
 template <int KIND>
 __device__ __forceinline__ float act_value(float a, float b, float c) {
   if constexpr (KIND == 0) {
-    const float s = round_bf16(a / (1.0f + expf(-a)));
-    return round_bf16(s * b);
+    return round_bf16(round_bf16(silu(a)) * b);
   } else if constexpr (KIND == 1) {
     return round_bf16(a * 0.5f * (1.0f + erff(a * 0.70710678118654752440f)));
   } else {
     return round_bf16(round_bf16(a * round_bf16(1.0f + b)) + c);
+  }
+}
+
+// act_value of the two bf16 values in each word.
+template <int KIND>
+__device__ __forceinline__ uint32_t act_pair(uint32_t a, uint32_t b, uint32_t c) {
+  const float a0 = __uint_as_float(a << 16), a1 = __uint_as_float(a & 0xffff0000u);
+  if constexpr (KIND == 0) {
+    // the product of two bf16 values is exact in fp32, so one rounding to bf16 is the same from either form
+    const __nv_bfloat162 y = __hmul2(__floats2bfloat162_rn(silu(a0), silu(a1)), *reinterpret_cast<const __nv_bfloat162*>(&b));
+    return *reinterpret_cast<const uint32_t*>(&y);
+  } else {
+    const float y0 = act_value<KIND>(a0, __uint_as_float(b << 16), __uint_as_float(c << 16));
+    const float y1 = act_value<KIND>(a1, __uint_as_float(b & 0xffff0000u), __uint_as_float(c & 0xffff0000u));
+    return (__float_as_uint(y0) >> 16) | (__float_as_uint(y1) & 0xffff0000u);   // both are bf16 values
   }
 }
 
@@ -289,12 +311,7 @@ act_quant_fp8_kernel(const uint16_t* __restrict__ a, int64_t a_pitch, const uint
       uint32_t aw[4] = {y[h].x, y[h].y, y[h].z, y[h].w};
       const uint32_t bw[4] = {bb[h].x, bb[h].y, bb[h].z, bb[h].w}, cw[4] = {cc[h].x, cc[h].y, cc[h].z, cc[h].w};
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float y0 = act_value<KIND>(__uint_as_float(aw[j] << 16), __uint_as_float(bw[j] << 16), __uint_as_float(cw[j] << 16));
-        const float y1 = act_value<KIND>(__uint_as_float(aw[j] & 0xffff0000u), __uint_as_float(bw[j] & 0xffff0000u),
-                                         __uint_as_float(cw[j] & 0xffff0000u));
-        aw[j] = (__float_as_uint(y0) >> 16) | (__float_as_uint(y1) & 0xffff0000u);   // both are bf16 values
-      }
+      for (int j = 0; j < 4; ++j) aw[j] = act_pair<KIND>(aw[j], bw[j], cw[j]);
       y[h] = make_uint4(aw[0], aw[1], aw[2], aw[3]);
       if (tid + (int64_t)h * T < (K >> 3)) mx = chunk_max(mx, y[h]);
     }
