@@ -112,7 +112,6 @@ void large_m_release(sacq_layer* L);
 
 // Tensor-core kernel that keeps the expanded weights in tensor memory (linear_large_m_tmem.cu).
 bool large_m_tmem_supported(const sacq_layer* L);
-int large_m_tmem_pick_nt(const sacq_layer* L, int64_t M);
 int launch_large_m_tmem(const sacq_layer* L, const void* q, const float* scale, int64_t M, void* y, int64_t ldy,
                         cudaStream_t s, const void* residual = nullptr, int64_t ldr = 0, const BcastDst* bc = nullptr,
                         int nt_force = 0);

@@ -7,6 +7,7 @@
 
 #include "common.cuh"
 #include "split_k.cuh"
+#include "tmem_weights.cuh"
 #include "umma.cuh"
 
 namespace sacq {
@@ -106,6 +107,30 @@ int large_m_index_map(const sacq_layer* Lc, const CUtensorMap** out) {
     L->large_plan->have = true;
   }
   *out = &L->large_plan->tmap_idx;
+  return SACQ_OK;
+}
+
+int tile_output(const sacq_layer* L, int64_t M, void* y, int64_t ldy, const void* residual, int64_t ldr, const BcastDst* bc,
+                tmemw::TmemOut* out, CUtensorMap* ty, tmemw::BcastMaps* tb) {
+  const sacq_layer_desc& d = L->d;
+  out->y = static_cast<uint16_t*>(y);
+  out->ldy = ldy;
+  out->residual = static_cast<const uint16_t*>(residual);
+  out->ldr = ldr;
+  out->M = (int)M;
+  out->N = (int)d.out_features;
+  bool tma = residual == nullptr && reinterpret_cast<uintptr_t>(y) % 16 == 0 && (ldy * 2) % 16 == 0 && d.out_features >= 32;
+  for (int i = 0; bc != nullptr && i < bc->n; ++i) {
+    out->ybc[i] = static_cast<uint16_t*>(bc->ptr[i]);
+    tma = tma && reinterpret_cast<uintptr_t>(bc->ptr[i]) % 16 == 0;
+  }
+  out->n_bc = bc != nullptr ? bc->n : 0;
+  out->y_tma = tma ? 1 : 0;
+  for (int i = tma ? -1 : out->n_bc; i < out->n_bc; ++i) {
+    const int rc = encode_bytes_2d(i < 0 ? ty : &tb->m[i], i < 0 ? y : bc->ptr[i], (uint64_t)d.out_features * 2, (uint64_t)M,
+                                   (uint64_t)ldy * 2, 64, 32, CU_TENSOR_MAP_SWIZZLE_64B);
+    if (rc != SACQ_OK) return rc;
+  }
   return SACQ_OK;
 }
 

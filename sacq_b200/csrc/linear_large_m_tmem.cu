@@ -1,40 +1,41 @@
-// Large-M quantized linear with the expanded weights held in TENSOR MEMORY (sm_100a):
+// Batched quantized linear with the expanded weights held in TENSOR MEMORY (sm_100a), persistent:
 //   y[m,n] = bf16( s[m] * (sum_k q[m,k] * cb[idx[n,k/d], k%d]) * scale[n] + bias[n] )
 //
-// The kernel of linear_large_m.cu writes every expanded weight tile to shared memory, from
-// where the tensor core reads it back together with the activation tile; its profile shows
-// shared memory, not the tensor pipe, as the limit (codeword gathers + two tile stores per
-// gather + the MMA's own operand reads all go through the same 128 bytes per clock).  Here
-// the roles of the operands are swapped:
-//   * the WEIGHTS are the MMA's A operand (128 weight rows = the 128 TMEM lanes) and live in
-//     tensor memory: an expander thread owns one weight row, gathers its codewords' FP8 high
-//     and low halves from the shared-memory codebook into registers and writes them with
-//     tcgen05.st -- no shared-memory store, no swizzle arithmetic;
-//   * the ACTIVATIONS are the B operand (N = tokens), TMA-loaded K-major / SWIZZLE_128B
-//     tiles, read by the tensor core straight from shared memory;
-//   * D[weight row, token] accumulates in TMEM: 128 lanes x (128 * NT) fp32 columns.
-// Per 32-wide K step the issuer thread runs one MMA with the high and one with the low
-// codeword halves into the same accumulator, so the summation order of an output element is
-// the same for every tile shape (row shards of a layer reproduce it bit for bit).
+//   * the WEIGHTS are the MMA's A operand (128 weight rows = the 128 TMEM lanes) and live in tensor
+//     memory: an expander thread gathers its row's codewords (FP8 high and low halves) from the
+//     shared-memory codebook into registers and writes them with tcgen05.st;
+//   * the ACTIVATIONS are the B operand (N = tokens), TMA-loaded K-major / SWIZZLE_128B tiles, read by
+//     the tensor core straight from shared memory;
+//   * D[weight row, token] accumulates in TMEM: 128 lanes x `tok` fp32 columns.
+// Per 32-wide K step one MMA with the high and one with the low codeword halves go into the same
+// accumulator, so the summation order of an output element is the same for every tile shape (row shards
+// of a layer reproduce it bit for bit).
 //
-// Shared-memory traffic per 128-k block drops to: activation operand reads + one 16-byte
-// gather per codeword.  With NT = 3 (384 tokens per CTA: one N = 256 and one N = 128 MMA
-// per half and K step) that is below what the tensor pipe needs for the same block.
+// A tile is 128 weight rows x `tok` tokens, a multiple of 32 up to 256 (one MMA) or of 64 up to 384 (two of
+// tok / 2).  TMEM: columns [0, tok) accumulate, the rest are weight stages of 64 (32 of high, 32 of low halves).
+// One CTA per SM takes tile after tile: the start-up of a CTA (3 us to its first MMA) is paid once, activation
+// tiles, indices and the first weight stages of the next tile are there when the epilogue ends, and a last, narrower
+// tile per weight row takes the tokens that are left.
 //
-// TMEM columns: [0, 128*NT) accumulator, then the weight stages: 64 columns each (32 = 128
-// e4m3 bytes per lane of high halves, 32 of low halves); 2 stages with NT = 3, else 4.
+// Roles: warp 0 = TMA producer (activation tiles, packed index tiles; no multicast), warp 1 = MMA issuer
+// and TMEM owner, warps 2..17 = expanders and, behind the first weight stages of the next tile, the epilogue.
+// Every mbarrier wait is bounded (status word + CTA-wide abort flag).
 //
-// Roles: warp 0 = TMA producer (activation tiles, packed index tiles; no multicast),
-// warp 1 = MMA issuer and TMEM owner, warps 2..9 = expanders and afterwards the epilogue
-// (tcgen05.ld of the thread's weight row, fma(s[m], acc * scale[n], bias[n]), bf16 stores:
-// the 32 lanes of a warp hold 32 consecutive n of one token, i.e. one 64-byte segment).
-// Every mbarrier wait is bounded as in linear_large_m.cu.
+// What bounds it: at 384 tokens the tensor cores and what feeds them (per K block 1536 clocks of MMAs; in shared memory
+// 683 of gathers, 768 of operand reads, 384 of arriving tiles), at the clock the power limit leaves; at up to 256
+// the expanders, 0.5 us per K block.  They gather AFTER the wait for their weight stage: gathering ahead of it, warps
+// that had time took the shared-memory banks from those that were waited for (0.65 us per K block).  Pairs of CTAs
+// (cta_group::2, half of the operand reads each) were no faster at 384 tokens and slower below.  GEMM alone, 8,192
+// tokens: 2048 -> 6144 159 -> 144 us, 1024 -> 4096 69 -> 55; 1,024 tokens: 6144 -> 2048 36 -> 29, 2048 -> 2048 16 -> 13
+// (before: one tile per CTA).
 //
 // Stands in for the reference's decode-to-8-bit + 8-bit GEMM pair at batched sizes
 // (a8_joint_pair_r1.py:38-127,374; perrow_a8_candidate_r3.py:56-69) and for its
 // decode-in-mainloop GEMM (codebook_cutlass_kernel.cu:234-583).
 #include <cuda.h>
 #include <math.h>
+#include <stdio.h>
+#include <stdlib.h>
 
 #include "common.cuh"
 #include "umma.cuh"
@@ -48,41 +49,43 @@ using namespace umma;
 using namespace tmemw;
 
 constexpr int kBK = 128;             // e4m3 bytes per K block (one 128-byte swizzle row)
-constexpr int kMaxActStages = 4;
+constexpr int kMaxActStages = 6;
 constexpr int kMaxWStages = 4;
+constexpr int kMaxTok = 384;
+constexpr int kWCols = kBK / 2;      // TMEM columns of a weight stage: kBK / 4 high + kBK / 4 low
 struct TmemParams {
   const uint8_t* cb_hilo;       // [C][2][D] e4m3
   const uint16_t* scales;       // bf16 [N]
   const uint16_t* bias;         // bf16 [N] or null
   const float* act_scale;       // [M]
-  uint16_t* y;                  // bf16 [M, ldy]
-  const uint16_t* residual;     // bf16 [M, ldr] or null
-  int64_t ldr;
-  int64_t ldy;
-  int n_bc;                     // further copies of the output (peer GPUs' buffers), same pitch as y
-  uint16_t* ybc[kMaxBcast];
   int* status;
-  int M, N, K, C;
+  TmemOut out;
+  int K, C;
+  // The tiles of the call: `full` = `row_tiles` x the whole tiles of `tok` tokens, then `row_tiles` of `rem` tokens (0: none)
+  // at token `rem_m0`.  Worker w takes the full tiles w, w + workers, ...; a worker from `rem_first` on, every
+  // (workers - rem_first)-th of the others.
+  int tok, rem, rem_m0, rem_first, full, row_tiles, workers;
+  int box;                      // tokens of one activation copy
   int act_stages;               // shared-memory activation stages, 2..kMaxActStages
-  int y_tma;                    // the output goes out by tiled bulk stores (aligned y, no residual, no peer copies)
   float out_mul;                // 2^-cb8_exp_shift
 };
 
 struct TmemLayout {
-  uint32_t act_off, act_stage, idx_off, idx_slot, cb_off, sw_off, bias_off, sa_off, bar_off, misc_off, total;
+  uint32_t act_off, act_stage, stg_off, idx_off, idx_slot, cb_off, sw_off, bias_off, sa_off, bar_off, misc_off, total;
 };
 
-__host__ __device__ inline TmemLayout tmem_layout(int nt, int act_stages, int sb_bytes, int cb_bytes) {
+__host__ __device__ inline TmemLayout tmem_layout(int tok, int act_stages, int sb_bytes, int cb_bytes) {
   TmemLayout L;
   L.act_off = 0;
-  L.act_stage = (uint32_t)(nt * kTokTile);
-  L.idx_off = act_stages * L.act_stage;
+  L.act_stage = (uint32_t)(tok * kBK);
+  L.stg_off = (uint32_t)act_stages * L.act_stage;
+  L.idx_off = L.stg_off + kEpiStaging;
   L.idx_slot = (uint32_t)(kRows * sb_bytes);
   L.cb_off = (L.idx_off + 2 * L.idx_slot + 127) & ~127u;
   L.sw_off = L.cb_off + (uint32_t)((cb_bytes + 127) & ~127);
-  L.bias_off = L.sw_off + kRows * 4;
-  L.sa_off = L.bias_off + kRows * 4;
-  L.bar_off = L.sa_off + (uint32_t)(nt * kBM * 4);
+  L.bias_off = L.sw_off + 2 * kRows * 4;             // two of each: a tile's are set up while the last one's are read
+  L.sa_off = L.bias_off + 2 * kRows * 4;
+  L.bar_off = L.sa_off + 2 * kMaxTok * 4;
   L.misc_off = L.bar_off + 32 * 8;
   L.total = L.misc_off + 64;
   return L;
@@ -118,70 +121,61 @@ __device__ __forceinline__ void load_fields_w(const uint8_t* base, int first, ui
   }
 }
 
-#ifdef SACQ_TRACE
-// Profiling builds only (-DSACQ_TRACE): CTA (0, 0) records %globaltimer at a few points per role.
-__device__ long long g_tmem_trace[8][72];
-#define SACQ_TR(role, slot) do { if (blockIdx.x == 0 && blockIdx.y == 0 && (slot) < 72) { long long _t; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(_t)); g_tmem_trace[role][slot] = _t; } } while (0)
-// Ablation switches of profiling builds (results are wrong with any of them set): 1 = no codeword gathers,
-// 2 = no tcgen05.st of the weights, 4 = activation tiles loaded for the first round of stages only, 8 = no MMAs.
-__device__ int g_tmem_ablate = 0;
-#define SACQ_ABLATE(bit) (g_tmem_ablate & (bit))
-#else
-#define SACQ_TR(role, slot) do { } while (0)
-#define SACQ_ABLATE(bit) false
-#endif
-
-// D in {4, 8}; BITS in {8, 12, 16}; NT = 128-token sub-tiles per CTA (1, 2 or 3); CB_SMEM: the
-// high/low codebook is staged in shared memory, else (a table too large for it: 65,536 entries)
-// gathered from global memory, where it stays L2-resident.
-// grid = (ceil(N / 128), ceil(M / (128 * NT))).  The last token tile may hold fewer valid
-// sub-tiles: only those are loaded and multiplied.
-template <int D, int BITS, int NT, bool CB_SMEM>
+// D in {4, 8}; BITS in {8, 12, 16}; CB_SMEM: the high/low codebook is staged in shared memory, else (a
+// table too large for it: 65,536 entries) gathered from global memory, where it stays L2-resident.
+// grid = workers.
+template <int D, int BITS, bool CB_SMEM>
 __global__ void __launch_bounds__(kCtaThreads, 1)
 large_m_tmem_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_idx,
                     const __grid_constant__ CUtensorMap tmap_y, const __grid_constant__ BcastMaps tmap_bc,
                     const __grid_constant__ TmemParams p) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  constexpr int BT = kBM * NT;                        // tokens per CTA = accumulator columns
   constexpr int IDX_PER_KB = kBK / D;                 // indices per row per K block
   constexpr int KB_BYTES = IDX_PER_KB * BITS / 8;     // index bytes per row per K block
   constexpr int SB_BYTES = 2 * KB_BYTES;              // ... per super block (two K blocks): multiple of 16
   constexpr int CW_BYTES = 2 * D;                     // hi + lo bytes per codeword
-  // A TMEM weight stage holds one K block of the 128 rows.  Half-block stages (four of them beside a
-  // 384-column accumulator instead of two whole blocks) were measured SLOWER (2048x6144 at M = 8192:
-  // 217 against 183 us): the per-stage cost of the expanders (barrier waits, tcgen05.wait::st, fences)
-  // does not shrink with the stage.
-  constexpr int W_COLS = kBK / 2;                     // TMEM columns of a stage: kBK / 4 high + kBK / 4 low
   constexpr int WQ = kBK / 16;                        // 32-bit words a thread writes per half
   constexpr int IPT = (kBK / D) / 4;                  // indices per expander thread per weight stage (a quarter row)
-  constexpr int kWStages = NT == 3 ? 2 : kMaxWStages; // TMEM weight stages
-  constexpr uint32_t kWCol0 = BT;                     // first weight-stage column
   constexpr uint32_t kTmemCols = 512;
-  static_assert(BT + kWStages * W_COLS <= 512, "TMEM budget");
-  constexpr uint32_t kIdesc256 = make_idesc(256), kIdesc128 = make_idesc(128), kIdesc192 = make_idesc(192);
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* sm = smem_raw + (base - raw);
-  const TmemLayout L = tmem_layout(NT, p.act_stages, SB_BYTES, CB_SMEM ? p.C * CW_BYTES : 0);
+  const TmemLayout L = tmem_layout(p.tok, p.act_stages, SB_BYTES, CB_SMEM ? p.C * CW_BYTES : 0);
 
   // barrier indices
-  constexpr int ACT_FULL = 0, ACT_EMPTY = kMaxActStages, W_FULL = 2 * kMaxActStages,
-                W_EMPTY = 2 * kMaxActStages + kMaxWStages, IDX_FULL = 2 * kMaxActStages + 2 * kMaxWStages,
-                IDX_EMPTY = IDX_FULL + 2, ACC_FULL = IDX_FULL + 4, CB_FULL = IDX_FULL + 5;
+  constexpr int ACT_FULL = 0, ACT_EMPTY = kMaxActStages, W_FULL = 2 * kMaxActStages, W_EMPTY = W_FULL + kMaxWStages,
+                IDX_FULL = W_EMPTY + kMaxWStages, IDX_EMPTY = IDX_FULL + 2, ACC_FULL = IDX_FULL + 4, ACC_EMPTY = IDX_FULL + 5, CB_FULL = IDX_FULL + 6;
+  static_assert(CB_FULL < 32, "barrier region");
   const uint32_t bars = base + L.bar_off;
   auto bar = [&](int i) { return bars + 8u * i; };
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + L.misc_off);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + L.misc_off + 8);
 
   const int warp = (int)warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
-  const int n0 = blockIdx.x * kRows;
-  const int m0 = blockIdx.y * BT;
+  const int worker = (int)blockIdx.x;
   const int num_kb = p.K / kBK;
   const int act_stages = p.act_stages;
+  const int w_stages = min(kMaxWStages, ((int)kTmemCols - p.tok) / kWCols);
+  // this worker's tiles, whole ones first
+  const int n_full = p.full > worker ? (p.full - worker + p.workers - 1) / p.workers : 0;
+  const int rem_step = p.workers - p.rem_first, rem0 = worker - p.rem_first;
+  const int items = n_full + (p.rem > 0 && rem0 >= 0 && rem0 < p.row_tiles ? (p.row_tiles - rem0 + rem_step - 1) / rem_step : 0);
+  auto tile = [&](int t, int& n0, int& m0, int& tok) {
+    int r;
+    if (t < n_full) {
+      const int i = worker + t * p.workers;
+      r = i % p.row_tiles;
+      m0 = i / p.row_tiles * p.tok;
+      tok = p.tok;
+    } else {
+      r = rem0 + (t - n_full) * rem_step;
+      m0 = p.rem_m0;
+      tok = p.rem;
+    }
+    n0 = r * kRows;
+  };
   const uint32_t cb_bytes = (uint32_t)(p.C * CW_BYTES);
-  const int nt_valid = min(NT, (p.M - m0 + kBM - 1) / kBM);       // sub-tiles of this CTA that hold tokens
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < kMaxActStages; ++i) {
@@ -197,53 +191,58 @@ large_m_tmem_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       mbar_init(bar(IDX_EMPTY + i), kXWarps);
     }
     mbar_init(bar(ACC_FULL), 1);
+    mbar_init(bar(ACC_EMPTY), kXWarps);
     mbar_init(bar(CB_FULL), 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    prefetch_tensormap(&tmap_a);
-    prefetch_tensormap(&tmap_idx);
-    if (p.y_tma) prefetch_tensormap(&tmap_y);
+    fence_proxy_async();
+  }
+  if (warp == 0) {
+    __syncwarp();
+    if (elect_one()) {                                // constant operands: their copies start before anything else
+      if constexpr (CB_SMEM) {
+        mbar_arrive_expect_tx(bar(CB_FULL), cb_bytes);
+        bulk_load(base + L.cb_off, p.cb_hilo, cb_bytes, bar(CB_FULL));
+      }
+      prefetch_tensormap(&tmap_a);
+      if (p.out.y_tma) prefetch_tensormap(&tmap_y);
+    }
   }
   if (warp == 1) tmem_alloc(smem_u32(tmem_slot), kTmemCols);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = warp_uniform(*tmem_slot);
-  if (threadIdx.x == 0) SACQ_TR(0, 0);
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if constexpr (CB_SMEM) {
-      if (elect_one()) {
-        mbar_arrive_expect_tx(bar(CB_FULL), cb_bytes);
-        bulk_load(base + L.cb_off, p.cb_hilo, cb_bytes, bar(CB_FULL));
-      }
-    }
-    int st = 0;
+    int st = 0, sb = 0;                               // index super blocks: counted over all tiles
     uint32_t free_parity = 1;
-    for (int kb = 0; kb < num_kb; ++kb) {
-      if ((kb & 1) == 0) {
-        const int sb = kb >> 1, slot = sb & 1;
-        if (!mbar_wait_warp(bar(IDX_EMPTY + slot), ((sb >> 1) & 1) ^ 1, abort_flag, p.status)) break;
-        if (elect_one()) {
-          mbar_arrive_expect_tx(bar(IDX_FULL + slot), kRows * SB_BYTES);
-          tma_load_2d(base + L.idx_off + slot * L.idx_slot, &tmap_idx, sb * SB_BYTES, n0, bar(IDX_FULL + slot));
+    bool ok = true;
+    for (int t = 0; t < items && ok; ++t) {
+      int n0, m0, tok;
+      tile(t, n0, m0, tok);
+      for (int kb = 0; kb < num_kb && ok; ++kb) {
+        if ((kb & 1) == 0) {
+          const int slot = sb & 1;
+          ok = mbar_wait_warp(bar(IDX_EMPTY + slot), ((sb >> 1) & 1) ^ 1, abort_flag, p.status);
+          if (!ok) break;
+          if (elect_one()) {
+            mbar_arrive_expect_tx(bar(IDX_FULL + slot), kRows * SB_BYTES);
+            tma_load_2d(base + L.idx_off + slot * L.idx_slot, &tmap_idx, (kb >> 1) * SB_BYTES, n0, bar(IDX_FULL + slot));
+          }
+          ++sb;
+          if (t == 0 && kb == 0) asm volatile("griddepcontrol.wait;" ::: "memory");   // activations: from the kernel in front
         }
+        ok = mbar_wait_warp(bar(ACT_EMPTY + st), free_parity, abort_flag, p.status);
+        if (!ok) break;
+        const uint32_t dst = base + L.act_off + st * L.act_stage;
+        if (elect_one()) mbar_arrive_expect_tx(bar(ACT_FULL + st), (uint32_t)(tok * kBK));
+        for (int b = 0; b < tok; b += p.box)
+          if (elect_one()) tma_load_2d(dst + (uint32_t)(b * kBK), &tmap_a, kb * kBK, m0 + b, bar(ACT_FULL + st));
+        if (++st == act_stages) { st = 0; free_parity ^= 1; }
       }
-      if (!mbar_wait_warp(bar(ACT_EMPTY + st), free_parity, abort_flag, p.status)) break;
-      if (elect_one()) {
-        if (SACQ_ABLATE(4) && kb >= act_stages) {      // no loads: the stage keeps its first tile
-          mbar_arrive(bar(ACT_FULL + st));
-        } else {
-          mbar_arrive_expect_tx(bar(ACT_FULL + st), nt_valid * kTokTile);
-#pragma unroll
-          for (int t = 0; t < NT; ++t)
-            if (t < nt_valid)
-              tma_load_2d(base + L.act_off + st * L.act_stage + t * kTokTile, &tmap_a, kb * kBK, m0 + t * kBM,
-                          bar(ACT_FULL + st));
-        }
-      }
-      if (++st == act_stages) { st = 0; free_parity ^= 1; }
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -251,40 +250,39 @@ large_m_tmem_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     bool ok = true;
     int st = 0, ws = 0;
     uint32_t act_parity = 0, w_parity = 0;
-    for (int kb = 0; kb < num_kb; ++kb) {
-      ok = mbar_wait_warp(bar(ACT_FULL + st), act_parity, abort_flag, p.status) &&
-           mbar_wait_warp(bar(W_FULL + ws), w_parity, abort_flag, p.status);
-      if (!ok) break;
-      tc_fence_after();
-      if (lane == 0) SACQ_TR(1, kb + 8);
-      const uint32_t act_addr = base + L.act_off + st * L.act_stage;
-      const uint32_t w_col = tmem_base + kWCol0 + (uint32_t)(ws * W_COLS);
+    for (int t = 0; t < items && ok; ++t) {
+      int n0, m0, tok;
+      tile(t, n0, m0, tok);
+      const int mmas = tok > 256 ? 2 : 1;             // an instruction takes at most 256 tokens
+      const uint32_t part = (uint32_t)(tok / mmas), idesc = make_idesc(tok / mmas);
+      // the epilogue has read the last tile's accumulators
+      if (t > 0 && !mbar_wait_warp(bar(ACC_EMPTY), (uint32_t)(t - 1) & 1u, abort_flag, p.status)) break;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        ok = mbar_wait_warp(bar(ACT_FULL + st), act_parity, abort_flag, p.status) &&
+             mbar_wait_warp(bar(W_FULL + ws), w_parity, abort_flag, p.status);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t act_addr = base + L.act_off + st * L.act_stage;
+        const uint64_t b0 = make_smem_desc(act_addr), b1 = make_smem_desc(act_addr + part * kBK);
+        const uint32_t w_col = tmem_base + (uint32_t)(kTmemCols - (ws + 1) * kWCols);
 #pragma unroll
-      for (int ks = 0; ks < kBK / 32; ++ks) {
-        const uint64_t adv = (uint64_t)((ks * 32) >> 4);
+        for (int ks = 0; ks < kBK / 32; ++ks) {
+          const uint64_t adv = (uint64_t)((ks * 32) >> 4);
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          if (SACQ_ABLATE(8)) continue;
-          const uint32_t a_tmem = w_col + (uint32_t)(half * (W_COLS / 2) + ks * 8);
-          const uint32_t acc = (kb | ks | half) != 0;
-          if (NT == 3 && nt_valid == 3) {
-            // an instruction takes at most 256 tokens: 384 go as two N = 192
-            if (elect_one()) umma_f8_ts(tmem_base, a_tmem, make_smem_desc(act_addr) + adv, kIdesc192, acc);
-            if (elect_one())
-              umma_f8_ts(tmem_base + 192u, a_tmem, make_smem_desc(act_addr + kTokTile * 3 / 2) + adv, kIdesc192, acc);
-          } else if (NT >= 2 && nt_valid >= 2) {
-            if (elect_one()) umma_f8_ts(tmem_base, a_tmem, make_smem_desc(act_addr) + adv, kIdesc256, acc);
-          } else {
-            if (elect_one()) umma_f8_ts(tmem_base, a_tmem, make_smem_desc(act_addr) + adv, kIdesc128, acc);
+          for (int lo = 0; lo < 2; ++lo) {
+            const uint32_t a_tmem = w_col + (uint32_t)(lo * (kWCols / 2) + ks * 8);
+            const uint32_t acc = (kb | ks | lo) != 0;
+            if (elect_one()) umma_f8_ts(tmem_base, a_tmem, b0 + adv, idesc, acc);
+            if (mmas == 2 && elect_one()) umma_f8_ts(tmem_base + part, a_tmem, b1 + adv, idesc, acc);
           }
         }
+        if (elect_one()) umma_commit(bar(ACT_EMPTY + st));
+        if (elect_one()) umma_commit(bar(W_EMPTY + ws));
+        if (++st == act_stages) { st = 0; act_parity ^= 1; }
+        if (++ws == w_stages) { ws = 0; w_parity ^= 1; }
       }
-      if (elect_one()) umma_commit(bar(ACT_EMPTY + st));
-      if (elect_one()) umma_commit(bar(W_EMPTY + ws));
-      if (++st == act_stages) { st = 0; act_parity ^= 1; }
-      if (++ws == kWStages) { ws = 0; w_parity ^= 1; }
+      if (ok && elect_one()) umma_commit(bar(ACC_FULL));
     }
-    if (ok && elect_one()) umma_commit(bar(ACC_FULL));
     __syncwarp();
   } else {
     // ------------------------------------------------------------------ expanders, then epilogue
@@ -293,36 +291,16 @@ large_m_tmem_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     const int row = quarter * 32 + lane;             // weight row of the tile = TMEM lane
     const int kpart = (warp - 2) >> 2;               // which 32 bytes of the 128-byte K block (0..3)
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
-    {
-      if (et < kRows) {
-        const int n = min(n0 + et, p.N - 1);
-        reinterpret_cast<float*>(sm + L.sw_off)[et] = bf16_bits_to_float(__ldg(p.scales + n)) * p.out_mul;
-        reinterpret_cast<float*>(sm + L.bias_off)[et] = p.bias ? bf16_bits_to_float(__ldg(p.bias + n)) : 0.f;
-      }
-      for (int i = et; i < BT; i += kXThreads) {
-        const int m = m0 + i;
-        reinterpret_cast<float*>(sm + L.sa_off)[i] = m < p.M ? __ldg(p.act_scale + m) : 0.f;
-      }
-      xbarrier();
-    }
     const uint8_t* cbs = CB_SMEM ? sm + L.cb_off : p.cb_hilo;
-    bool ok = CB_SMEM ? mbar_wait(bar(CB_FULL), 0, abort_flag, p.status) : true;
-    for (int kb = 0; kb < num_kb && ok; ++kb) {
-      const int sb = kb >> 1, slot = sb & 1;
-      const int ws = kb % kWStages;
-      ok = mbar_wait(bar(IDX_FULL + slot), (sb >> 1) & 1, abort_flag, p.status) &&
-           mbar_wait(bar(W_EMPTY + ws), ((kb / kWStages) & 1) ^ 1, abort_flag, p.status);
-      if (!ok) break;
-      tc_fence_after();                              // the MMAs that read this stage are complete
-      if (warp == 2 && lane == 0) SACQ_TR(2, kb + 8);
+    bool ok = CB_SMEM ? mbar_wait_warp(bar(CB_FULL), 0, abort_flag, p.status) : true;
+    // the codewords of the thread's quarter of the g-th K block, counted over all tiles: WQ words of high halves, WQ of low
+    auto gather = [&](int g, uint32_t (&hi)[WQ], uint32_t (&lo)[WQ]) {
+      const int sb = g >> 1, slot = sb & 1;           // K is a multiple of two blocks
+      if (!mbar_wait_warp(bar(IDX_FULL + slot), (sb >> 1) & 1, abort_flag, p.status)) return false;
       uint32_t idx[IPT];
-      load_fields_w<BITS, IPT>(sm + L.idx_off + slot * L.idx_slot + row * SB_BYTES + (kb & 1) * KB_BYTES,
+      load_fields_w<BITS, IPT>(sm + L.idx_off + slot * L.idx_slot + row * SB_BYTES + (g & 1) * KB_BYTES,
                                kpart * IPT, idx);
-      uint32_t hi[WQ], lo[WQ];
-      if (SACQ_ABLATE(1)) {
-#pragma unroll
-        for (int j = 0; j < WQ; ++j) { hi[j] = idx[j % IPT]; lo[j] = idx[j % IPT] >> 3; }
-      } else if constexpr (D == 8) {
+      if constexpr (D == 8) {
 #pragma unroll
         for (int j = 0; j < IPT; ++j) {
           const uint4 c = CB_SMEM ? *reinterpret_cast<const uint4*>(cbs + (size_t)idx[j] * 16)
@@ -339,45 +317,65 @@ large_m_tmem_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           lo[j] = c.y;
         }
       }
-      // the thread's quarter of the stage's k: WQ columns of the high half, WQ of the low half
-      const uint32_t w_addr = lane_addr + kWCol0 + (uint32_t)(ws * W_COLS + kpart * WQ);
-      if (!SACQ_ABLATE(2)) {
+      return true;
+    };
+    int ws = 0;
+    uint32_t w_parity = 1;
+    const int blocks = items * num_kb;
+    // A tile's epilogue runs behind the first weight stages of the next tile, all but one of which are free before the
+    // tile's last MMA ends: the tensor cores find them ready when the accumulators have been read.
+    const int ahead = min(w_stages - 1, num_kb);
+    int epi = 0, due = num_kb + ahead;                // the next epilogue, and behind how many blocks
+    uint32_t hi[WQ], lo[WQ];
+    for (int g = 0; g < blocks + ahead && ok; ++g) {
+      if (g < blocks) {
+        ok = mbar_wait_warp(bar(W_EMPTY + ws), w_parity, abort_flag, p.status);
+        if (!ok) break;
+        tc_fence_after();                              // the MMAs that read this stage are complete
+        ok = gather(g, hi, lo);
+        if (!ok) break;
+        // the thread's quarter of the stage's k: WQ columns of the high half, WQ of the low half
+        const uint32_t w_addr = lane_addr + (uint32_t)(kTmemCols - (ws + 1) * kWCols + kpart * WQ);
         tmem_st_32xn(w_addr, hi);
-        tmem_st_32xn(w_addr + (uint32_t)(W_COLS / 2), lo);
-      } else if (hi[0] + lo[WQ - 1] == 0x12345678u) {
-        p.status[0] = 99;                              // never true in practice: keeps the gathers alive
+        tmem_st_32xn(w_addr + (uint32_t)(kWCols / 2), lo);
+        if ((g & 1) == 1 && lane == 0) mbar_arrive(bar(IDX_EMPTY + ((g >> 1) & 1)));
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(W_FULL + ws));
+        if (++ws == w_stages) { ws = 0; w_parity ^= 1; }
       }
-      tmem_wait_st();
-      tc_fence_before();
-      __syncwarp();
-      if (warp == 2 && lane == 0) SACQ_TR(5, kb + 8);
-      if (lane == 0) {
-        mbar_arrive(bar(W_FULL + ws));
-        if ((kb & 1) == 1 || kb == num_kb - 1) mbar_arrive(bar(IDX_EMPTY + slot));
+      if (g + 1 != due) continue;
+      // ---- epilogue
+      int n0, m0, tok;
+      tile(epi, n0, m0, tok);
+      float* sw = reinterpret_cast<float*>(sm + L.sw_off) + (epi & 1) * kRows;
+      float* bias = reinterpret_cast<float*>(sm + L.bias_off) + (epi & 1) * kRows;
+      float* sa = reinterpret_cast<float*>(sm + L.sa_off) + (epi & 1) * kMaxTok;
+      if (et < kRows) {
+        const int n = min(n0 + et, p.out.N - 1);
+        sw[et] = bf16_bits_to_float(__ldg(p.scales + n)) * p.out_mul;
+        bias[et] = p.bias ? bf16_bits_to_float(__ldg(p.bias + n)) : 0.f;
       }
-    }
-
-    // ---- epilogue
-    if (ok) ok = mbar_wait(bar(ACC_FULL), 0, abort_flag, p.status);
-    if (warp == 2 && lane == 0) SACQ_TR(0, 3);
-    ok = xall(ok);                                    // tcgen05.ld and the staging barriers are collective
-    if (ok) {
+      asm volatile("griddepcontrol.wait;" ::: "memory");   // the token scales; the kernel in front has long gone
+      if (et < tok) sa[et] = m0 + et < p.out.M ? __ldg(p.act_scale + m0 + et) : 0.f;
+      ok = mbar_wait_warp(bar(ACC_FULL), (uint32_t)epi & 1u, abort_flag, p.status);
+      ok = xall(ok);                                  // also: the scales are in place
+      if (!ok) break;
       tc_fence_after();
-      TmemOut o;
-      o.y = p.y; o.ldy = p.ldy; o.residual = p.residual; o.ldr = p.ldr; o.n_bc = p.n_bc;
-      for (int i = 0; i < p.n_bc; ++i) o.ybc[i] = p.ybc[i];
-      o.M = p.M; o.N = p.N; o.y_tma = p.y_tma;
-      const float sw = reinterpret_cast<const float*>(sm + L.sw_off)[row];
-      const float bs = reinterpret_cast<const float*>(sm + L.bias_off)[row];
-      tmem_epilogue<NT>(o, &tmap_y, tmap_bc.m, lane_addr, row, kpart, et, reinterpret_cast<const float*>(sm + L.sa_off), sw, bs,
-                        sm + L.act_off, (act_stages * L.act_stage >= 2u * kStageTile) ? 2 : 1, m0, n0);
+      tile_epilogue(p.out, &tmap_y, tmap_bc.m, lane_addr, quarter, kpart, tok, sa, sw, bias, sm + L.stg_off, m0, n0,
+                        bar(ACC_EMPTY));
+      ++epi;
+      due += num_kb;
     }
+    // shared memory stays valid until every store has read it; the writes themselves (local and peer)
+    // are in the memory system then, like plain stores, and the grid's end orders them
+    tma_store_wait_read<0>();
   }
 
   // ---- common exit: every thread arrives here, also after an aborted wait
   tc_fence_before();
   __syncthreads();
-  if (threadIdx.x == 0) SACQ_TR(0, 4);
   if (warp == 1) tmem_dealloc(tmem_base, kTmemCols);
 }
 
@@ -393,52 +391,106 @@ size_t smem_request(const TmemLayout& lay) {
 // Codebooks up to 64 KB (high + low halves) are staged in shared memory, larger ones gathered from global memory.
 bool cb_in_smem(const sacq_layer* L) { return (size_t)L->cb_entries * L->d.vector_dim * 2 <= 64 * 1024; }
 
-int pick_act_stages(const sacq_layer* L, int nt) {
+// Activation stages: as many as fit.  Gathers from global memory need the rest of the SM's memory as L1 (a line for every
+// miss in flight): with 227 KB taken, 2048 -> 6144 with 65,536 codewords took 46 us at 1,024 tokens, with 164 KB 29.
+int pick_act_stages(const sacq_layer* L, int tok) {
   const int cb_bytes = cb_in_smem(L) ? L->cb_entries * L->d.vector_dim * 2 : 0;
-  for (int st = (nt == 3 ? 3 : kMaxActStages); st >= 2; --st)
-    if (tmem_layout(nt, st, sb_bytes_of(L), cb_bytes).total + 1024 <= 227 * 1024) return st;
-  return 0;
+  const uint32_t most = (cb_in_smem(L) ? 227 : 164) * 1024;
+  for (int st = kMaxActStages; st >= 2; --st)
+    if (tmem_layout(tok, st, sb_bytes_of(L), cb_bytes).total + 1024 <= most) return st;
+  return tmem_layout(tok, 2, sb_bytes_of(L), cb_bytes).total + 1024 <= 227 * 1024 ? 2 : 0;
 }
 
-template <int D, int BITS, int NT, bool CB_SMEM>
-cudaError_t launch_nt(const CUtensorMap& ta, const CUtensorMap& ti, const CUtensorMap& ty, const BcastMaps& tb,
+template <int D, int BITS, bool CB_SMEM>
+cudaError_t launch_cb(const CUtensorMap& ta, const CUtensorMap& ti, const CUtensorMap& ty, const BcastMaps& tb,
                       const TmemParams& p, dim3 grid, size_t smem, cudaStream_t s) {
   static bool configured[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || !configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(large_m_tmem_kernel<D, BITS, NT, CB_SMEM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(large_m_tmem_kernel<D, BITS, CB_SMEM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          227 * 1024);
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
-  large_m_tmem_kernel<D, BITS, NT, CB_SMEM><<<grid, kCtaThreads, smem, s>>>(ta, ti, ty, tb, p);
-  return cudaGetLastError();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kCtaThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, large_m_tmem_kernel<D, BITS, CB_SMEM>, ta, ti, ty, tb, p);
 }
 
 template <int D, int BITS>
 cudaError_t launch_db(const CUtensorMap& ta, const CUtensorMap& ti, const CUtensorMap& ty, const BcastMaps& tb,
-                      const TmemParams& p, int nt, bool cb_smem, dim3 grid, size_t smem, cudaStream_t s) {
-  if (!cb_smem) {
-    if (nt == 3) return launch_nt<D, BITS, 3, false>(ta, ti, ty, tb, p, grid, smem, s);
-    if (nt == 2) return launch_nt<D, BITS, 2, false>(ta, ti, ty, tb, p, grid, smem, s);
-    return launch_nt<D, BITS, 1, false>(ta, ti, ty, tb, p, grid, smem, s);
+                      const TmemParams& p, bool cb_smem, dim3 grid, size_t smem, cudaStream_t s) {
+  return cb_smem ? launch_cb<D, BITS, true>(ta, ti, ty, tb, p, grid, smem, s)
+                 : launch_cb<D, BITS, false>(ta, ti, ty, tb, p, grid, smem, s);
+}
+
+// A tile's width for `t` tokens: a multiple of 32, of 64 above 256 (two instructions).
+int width_of(int64_t t) {
+  const int64_t step = t > 256 ? 64 : 32;
+  return (int)((t + step - 1) / step * step);
+}
+
+// Time of a tile (us), fitted to 2048 -> 6144, 2048 -> 2048, 6144 -> 2048 and 1024 -> 4096 at 1,024 - 8,192 tokens.
+double tile_us(const sacq_layer* L, int tok) {
+  const double least = cb_in_smem(L) ? (L->d.vector_dim == 8 ? 0.52 : 0.65) : 11.5 / L->d.vector_dim;
+  const double block = 0.0026 * tok > least ? 0.0026 * tok : least;
+  return 2.3 + 0.0026 * tok + (double)L->d.in_features / kBK * block;
+}
+
+// The tiles of M tokens in tiles of `tok` and one of what is left, and the modelled time of the busiest worker.  The
+// remainders go to the workers that have a whole tile less than the others, or, where that makes too many for them, to all.
+double plan_tiles(const sacq_layer* L, int64_t M, int tok, TmemParams* p) {
+  p->row_tiles = (int)((L->d.out_features + kRows - 1) / kRows);
+  p->tok = tok;
+  p->full = (int)(M / tok) * p->row_tiles;
+  p->rem = width_of(M % tok);
+  p->rem_m0 = (int)(M / tok * tok);
+  const int at_once = L->num_sms, tiles = p->full + (p->rem > 0 ? p->row_tiles : 0);
+  p->workers = tiles < at_once ? tiles : at_once;
+  int rounds = p->full / p->workers, extra = p->full % p->workers;
+  double whole = (rounds + (extra > 0 ? 1 : 0)) * tile_us(L, tok);
+  p->rem_first = 0;
+  if (p->rem == 0) return whole;
+  auto rems = [&](int on) { return (p->row_tiles + on - 1) / on * tile_us(L, p->rem); };
+  const double few = rounds * tile_us(L, tok) + rems(p->workers - extra);
+  if (rounds == 0 && p->full > 0 && few >= whole + rems(extra)) {     // as many workers as whole tiles
+    p->workers = p->full;
+    return whole + rems(p->workers);
   }
-  if (nt == 3) return launch_nt<D, BITS, 3, true>(ta, ti, ty, tb, p, grid, smem, s);
-  if (nt == 2) return launch_nt<D, BITS, 2, true>(ta, ti, ty, tb, p, grid, smem, s);
-  return launch_nt<D, BITS, 1, true>(ta, ti, ty, tb, p, grid, smem, s);
+  const double all = whole + rems(p->workers);
+  if (rounds > 0 && few >= all) return all;
+  p->rem_first = extra;
+  return few > whole ? few : whole;
+}
+
+// Width of the whole tiles: the one with the shortest modelled time.  8,192 tokens of a 6,144-row layer, for instance, are
+// 1,008 tiles of 384 and 48 of 128 on 148 SMs: 7 rounds, where a grid of equal tiles takes 8.
+int pick_tok(const sacq_layer* L, int64_t M) {
+  if (M > (1 << 24)) return kMaxTok;
+  int best = kMaxTok;
+  double best_us = 1e30;
+  for (int t = kMaxTok; t >= 32; t -= t > 256 ? 64 : 32) {
+    if (M > t && t < 128) continue;
+    TmemParams p;
+    const double us = plan_tiles(L, M, t, &p);
+    if (us < best_us - 1e-9) {
+      best_us = us;
+      best = t;
+    }
+  }
+  return best;
 }
 
 }  // namespace
-
-#ifdef SACQ_TRACE
-extern "C" SACQ_API int sacq_debug_tmem_trace(long long* out) {
-  return cudaMemcpyFromSymbol(out, g_tmem_trace, sizeof(long long) * 8 * 72) == cudaSuccess ? 0 : -1;
-}
-extern "C" SACQ_API int sacq_debug_tmem_ablate(int flags) {
-  return cudaMemcpyToSymbol(g_tmem_ablate, &flags, sizeof(int)) == cudaSuccess ? 0 : -1;
-}
-#endif
 
 bool large_m_tmem_supported(const sacq_layer* L) {
   const sacq_layer_desc& d = L->d;
@@ -448,28 +500,7 @@ bool large_m_tmem_supported(const sacq_layer* L) {
   if (d.in_features % (2 * kBK) != 0) return false;
   if (L->num_groups != 1 || has_shift(L)) return false;
   if (((size_t)L->cb_entries * d.vector_dim * 2) % 16 != 0) return false;
-  return pick_act_stages(L, 1) >= 2;
-}
-
-// Token sub-tiles per CTA (1..3) for M tokens: the largest tile that does not add a wave, or 0
-// when the kernel cannot run the layer.
-int large_m_tmem_pick_nt(const sacq_layer* L, int64_t M) {
-  if (!large_m_tmem_supported(L)) return 0;
-  const int64_t row_tiles = (L->d.out_features + kRows - 1) / kRows;
-  int best = 0;
-  double best_cost = 1e30;
-  for (int nt = 3; nt >= 1; --nt) {
-    if (pick_act_stages(L, nt) < 2) continue;
-    const int64_t tiles = row_tiles * ((M + kBM * nt - 1) / (kBM * nt));
-    const int64_t waves = (tiles + L->num_sms - 1) / L->num_sms;
-    // whole waves x time of one CTA, fitted to measurements of 2048x6144, 2048x2048 and 6144x2048 at
-    // 1,024 - 8,192 tokens (us; k = K / 2048): 4.5 + 10 k, 5.6 + 13.5 k and 5.4 + 17.2 k for 1, 2, 3 sub-tiles
-    const double k = (double)L->d.in_features / 2048.0;
-    const double per_cta = nt == 3 ? 5.4 + 17.2 * k : nt == 2 ? 5.6 + 13.5 * k : 4.5 + 10.0 * k;
-    const double cost = (double)waves * per_cta;
-    if (cost < best_cost - 1e-9) { best_cost = cost; best = nt; }
-  }
-  return best;
+  return pick_act_stages(L, kMaxTok) >= 2;
 }
 
 int launch_large_m_tmem(const sacq_layer* L, const void* q, const float* scale, int64_t M, void* y, int64_t ldy,
@@ -480,14 +511,27 @@ int launch_large_m_tmem(const sacq_layer* L, const void* q, const float* scale, 
   if (M > (1 << 30)) return set_error(SACQ_ERR_UNSUPPORTED, "M=%lld too large", (long long)M);
   if (reinterpret_cast<uintptr_t>(q) % 16 != 0)
     return set_error(SACQ_ERR_ALIGNMENT, "quantized activations must be 16-byte aligned");
-  int nt = nt_force > 0 ? nt_force : large_m_tmem_pick_nt(L, M);
-  if (nt < 1 || nt > 3) return set_error(SACQ_ERR_UNSUPPORTED, "TMEM-weight kernel: no tile shape fits");
+  int tok = nt_force > 0 ? kBM * nt_force : pick_tok(L, M);
+#ifdef SACQ_TUNE
+  if (const char* e = getenv("SACQ_TOK")) tok = atoi(e);
+#endif
   const bool cb_smem = cb_in_smem(L);
-  const int act_stages = pick_act_stages(L, nt);
-  if (act_stages < 2) return set_error(SACQ_ERR_UNSUPPORTED, "TMEM-weight kernel: shared memory too small for %d sub-tiles", nt);
+  const int act_stages = pick_act_stages(L, tok);
+  if (M / tok + 1 > 0x7fffffff / ((d.out_features + kRows) / kRows))
+    return set_error(SACQ_ERR_UNSUPPORTED, "M=%lld: too many tiles", (long long)M);
+  TmemParams p{};
+  plan_tiles(L, M, tok, &p);
+  // one copy size for both kinds of tile
+  auto part_of = [](int t) { return t / (t > 256 ? 2 : 1); };
+  p.box = part_of(p.full > 0 ? p.tok : p.rem);
+  for (int a = part_of(p.rem); p.full > 0 && a > 0;) {
+    const int r = p.box % a;
+    p.box = a;
+    a = r;
+  }
   CUtensorMap ta;
   {
-    const int rc = encode_bytes_2d(&ta, q, (uint64_t)d.in_features, (uint64_t)M, (uint64_t)d.in_features, kBK, kBM,
+    const int rc = encode_bytes_2d(&ta, q, (uint64_t)d.in_features, (uint64_t)M, (uint64_t)d.in_features, kBK, p.box,
                                    CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc != SACQ_OK) return rc;
   }
@@ -496,59 +540,29 @@ int launch_large_m_tmem(const sacq_layer* L, const void* q, const float* scale, 
     const int rc = large_m_index_map(L, &ti);
     if (rc != SACQ_OK) return rc;
   }
-  // the output leaves by tiled bulk stores when y (and every peer copy of a column split) allows it:
-  // 16-byte aligned base and row pitch
-  bool y_tma = residual == nullptr && reinterpret_cast<uintptr_t>(y) % 16 == 0 && (ldy * 2) % 16 == 0 &&
-               d.out_features >= kRows;
-  for (int i = 0; bc != nullptr && i < bc->n; ++i) y_tma = y_tma && reinterpret_cast<uintptr_t>(bc->ptr[i]) % 16 == 0;
   CUtensorMap ty = ta;                                // a valid map is passed either way
-  static const BcastMaps kNoMaps = {};
-  BcastMaps tb_local;
-  const BcastMaps* tb = &kNoMaps;
-  if (y_tma) {
-    int rc = encode_bytes_2d(&ty, y, (uint64_t)d.out_features * 2, (uint64_t)M, (uint64_t)ldy * 2, kRows * 2, kBM,
-                             CU_TENSOR_MAP_SWIZZLE_NONE);
-    if (rc != SACQ_OK) return rc;
-    if (bc != nullptr && bc->n > 0) {
-      tb_local = kNoMaps;
-      for (int i = 0; i < bc->n; ++i) {
-        rc = encode_bytes_2d(&tb_local.m[i], bc->ptr[i], (uint64_t)d.out_features * 2, (uint64_t)M, (uint64_t)ldy * 2,
-                             kRows * 2, kBM, CU_TENSOR_MAP_SWIZZLE_NONE);
-        if (rc != SACQ_OK) return rc;
-      }
-      tb = &tb_local;
-    }
-  }
-  TmemParams p{};
-  p.y_tma = y_tma ? 1 : 0;
+  BcastMaps tb = {};
+  int rc = tile_output(L, M, y, ldy, residual, ldr, bc, &p.out, &ty, &tb);
+  if (rc != SACQ_OK) return rc;
   p.cb_hilo = L->cb_hilo;
   p.scales = static_cast<const uint16_t*>(d.scales);
   p.bias = static_cast<const uint16_t*>(d.bias);
   p.act_scale = scale;
-  p.y = static_cast<uint16_t*>(y);
-  p.residual = static_cast<const uint16_t*>(residual);
-  p.ldr = ldr;
-  p.ldy = ldy;
-  if (bc != nullptr) {
-    p.n_bc = bc->n;
-    for (int i = 0; i < bc->n; ++i) p.ybc[i] = static_cast<uint16_t*>(bc->ptr[i]);
-  }
   p.status = L->d_status;
-  p.M = (int)M; p.N = (int)d.out_features; p.K = (int)d.in_features; p.C = L->cb_entries;
+  p.K = (int)d.in_features; p.C = L->cb_entries;
   p.act_stages = act_stages;
   p.out_mul = ldexpf(1.f, -L->cb8_exp_shift);
-  const TmemLayout lay = tmem_layout(nt, act_stages, sb_bytes_of(L), cb_smem ? L->cb_entries * d.vector_dim * 2 : 0);
+  const TmemLayout lay = tmem_layout(tok, act_stages, sb_bytes_of(L), cb_smem ? L->cb_entries * d.vector_dim * 2 : 0);
   const size_t smem = smem_request(lay);
-  const dim3 grid((unsigned)((d.out_features + kRows - 1) / kRows), (unsigned)((M + kBM * nt - 1) / (kBM * nt)), 1);
-  if (grid.y > 65535) return set_error(SACQ_ERR_UNSUPPORTED, "M=%lld exceeds the grid limit", (long long)M);
+  const dim3 grid((unsigned)p.workers);
   cudaError_t e;
   const int D = d.vector_dim, B = d.index_bits;
-  if (D == 8 && B == 12) e = launch_db<8, 12>(ta, *ti, ty, *tb, p, nt, cb_smem, grid, smem, s);
-  else if (D == 8 && B == 8) e = launch_db<8, 8>(ta, *ti, ty, *tb, p, nt, cb_smem, grid, smem, s);
-  else if (D == 8 && B == 16) e = launch_db<8, 16>(ta, *ti, ty, *tb, p, nt, cb_smem, grid, smem, s);
-  else if (D == 4 && B == 12) e = launch_db<4, 12>(ta, *ti, ty, *tb, p, nt, cb_smem, grid, smem, s);
-  else if (D == 4 && B == 8) e = launch_db<4, 8>(ta, *ti, ty, *tb, p, nt, cb_smem, grid, smem, s);
-  else e = launch_db<4, 16>(ta, *ti, ty, *tb, p, nt, cb_smem, grid, smem, s);
+  if (D == 8 && B == 12) e = launch_db<8, 12>(ta, *ti, ty, tb, p, cb_smem, grid, smem, s);
+  else if (D == 8 && B == 8) e = launch_db<8, 8>(ta, *ti, ty, tb, p, cb_smem, grid, smem, s);
+  else if (D == 8 && B == 16) e = launch_db<8, 16>(ta, *ti, ty, tb, p, cb_smem, grid, smem, s);
+  else if (D == 4 && B == 12) e = launch_db<4, 12>(ta, *ti, ty, tb, p, cb_smem, grid, smem, s);
+  else if (D == 4 && B == 8) e = launch_db<4, 8>(ta, *ti, ty, tb, p, cb_smem, grid, smem, s);
+  else e = launch_db<4, 16>(ta, *ti, ty, tb, p, cb_smem, grid, smem, s);
   count_launch();
   if (e != cudaSuccess) return cuda_fail(e, "TMEM-weight large-M launch");
   return SACQ_OK;

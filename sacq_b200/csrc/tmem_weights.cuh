@@ -7,6 +7,7 @@
 #include <cuda.h>
 
 #include "common.cuh"
+#include "encode.cuh"
 #include "umma.cuh"
 
 namespace sacq {
@@ -218,5 +219,152 @@ __device__ __forceinline__ void tmem_epilogue(const TmemOut& o, const CUtensorMa
   if (o.y_tma && et == 0) tma_store_wait_read<0>();
 }
 
+// 16 lanes x 32 consecutive fp32 columns, as four 16 x 8 fragments: registers 4 j + 0, 1 = lane (thread / 4), columns
+// 8 j + 2 (thread % 4) + 0, 1; registers 4 j + 2, 3 = lane (thread / 4) + 8.
+__device__ __forceinline__ void tmem_ld_16x32(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+// Four 8 x 8 tiles of 16-bit elements, each stored transposed; thread l gives the row address l % 8 of tile l / 8.
+__device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared::cta.b16 [%0], {%1, %2, %3, %4};"
+               ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d)
+               : "memory");
+}
+
+constexpr int kWarpTile = 32 * 64;                    // a warp's staged output: 32 tokens x 32 weight rows, bf16
+constexpr int kEpiStaging = kXWarps * kWarpTile;     // one per expander warp
+
+// Epilogue of one tile, run by the expander warps after the accumulator is complete:
+//   y[m0 + token, n0 + row] = bf16(fma(sa[token], acc[row][token] * sw[row], bias[row]))
+// The accumulator holds y transposed (lane = weight row, column = token).  A warp takes its lane quarter of every
+// fourth 32 tokens: fragments whose register pairs are two tokens of one row, packed to bf16 and stored transposed
+// into a [32 tokens][32 rows] tile (stmatrix; 64-byte rows, 16-byte units swizzled as SWIZZLE_64B does), which
+// leaves by one tiled bulk store, clipped at the edges of y.  No barrier between warps.  With a residual or an
+// unaligned y the warp stores the tile itself, four lanes per token.  128 rows x 384 tokens take 2.4 us; with 2-byte
+// stores into a tile of the whole CTA and two barriers per 128 tokens they took 3.3.
+// `acc_empty` takes one arrival per warp as soon as it has read its accumulators.
+__device__ __forceinline__ void tile_epilogue(const TmemOut& o, const CUtensorMap* tmap_y, const CUtensorMap* tmap_bc,
+                                              uint32_t lane_addr, int quarter, int kpart, int tok, const float* sa,
+                                              const float* sw, const float* bias, uint8_t* stage_base, int m0, int n0, uint32_t acc_empty) {
+  const int lane = threadIdx.x & 31;
+  const int nw = n0 + quarter * 32;                   // first weight row of the warp
+  uint8_t* tile = stage_base + (quarter + 4 * kpart) * kWarpTile;
+  const int last = nw < o.N ? min(tok, o.M - m0) - 1 : -1;             // the last token to store, counted from m0
+  // the warp's accumulators have been read (or are not wanted): the next tile may overwrite them
+  auto release = [&] {
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(acc_empty);
+  };
+  if (kpart * 32 > last) {
+    release();
+    return;
+  }
+  uint64_t sw2[4], bs2[4];                            // of the thread's rows lane / 4 + 8 i
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = quarter * 32 + (lane >> 2) + 8 * i;
+    sw2[i] = f32x2(sw[r], sw[r]);
+    bs2[i] = f32x2(bias[r], bias[r]);
+  }
+#pragma unroll 1
+  for (int c = kpart; c * 32 <= last; c += 4) {
+    const int m = m0 + c * 32;
+    uint32_t a[16], b[16];
+    tmem_ld_16x32(lane_addr + (uint32_t)(c * 32), a);
+    tmem_ld_16x32(lane_addr + (16u << 16) + (uint32_t)(c * 32), b);
+    uint64_t s2[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 v = *reinterpret_cast<const float2*>(sa + c * 32 + 8 * j + 2 * (lane & 3));
+      s2[j] = f32x2(v.x, v.y);
+    }
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    if ((c + 4) * 32 > last) release();
+    tma_store_wait_read<0>();                         // the store before this one has read the tile
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      uint32_t w[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t* r = i < 2 ? a : b;
+        const int at = 4 * j + 2 * (i & 1);
+        float lo, hi;
+        halves_of(fma2(s2[j], mul2(f32x2(__uint_as_float(r[at]), __uint_as_float(r[at + 1])), sw2[i]), bs2[i]), lo, hi);
+        const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+        w[i] = *reinterpret_cast<const uint32_t*>(&v);
+      }
+      const int t = 8 * j + (lane & 7);               // token whose 16 bytes of rows 8 (lane / 8) .. + 7 the thread addresses
+      stmatrix_x4_trans(smem_u32(tile) + (uint32_t)(t * 64 + (((lane >> 3) ^ ((t >> 1) & 3)) * 16)), w[0], w[1], w[2], w[3]);
+    }
+    if (o.y_tma) {
+      fence_proxy_async();                            // generic-proxy writes -> visible to the bulk store
+      __syncwarp();
+      if (lane == 0) {
+        // one bulk-store group: the local copy and, in a column split, every peer's copy
+        tma_store_2d_issue(tmap_y, nw * 2, m, smem_u32(tile));
+        for (int i = 0; i < o.n_bc; ++i) tma_store_2d_issue(tmap_bc + i, nw * 2, m, smem_u32(tile));
+        tma_store_commit();
+      }
+    } else {
+      __syncwarp();
+#pragma unroll 1
+      for (int i = 0; i < 4; ++i) {
+        const int t = i * 8 + (lane >> 2), ch = lane & 3;
+        const int n = nw + ch * 8;
+        if (m + t >= o.M || n >= o.N) continue;
+        uint4 v = *reinterpret_cast<const uint4*>(tile + t * 64 + ((ch ^ ((t >> 1) & 3)) * 16));
+        const int64_t off = (int64_t)(m + t) * o.ldy + n;
+        const bool full = n + 8 <= o.N;
+        if (o.residual != nullptr) {
+          // bf16(bf16(v) + residual): the two roundings of `linear(x) + residual`
+          const uint16_t* rp = o.residual + (int64_t)(m + t) * o.ldr + n;
+          uint32_t w[4] = {v.x, v.y, v.z, v.w}, r[4] = {0u, 0u, 0u, 0u};
+          if (full && (reinterpret_cast<uintptr_t>(rp) & 15) == 0) {
+            const uint4 q = __ldg(reinterpret_cast<const uint4*>(rp));
+            r[0] = q.x; r[1] = q.y; r[2] = q.z; r[3] = q.w;
+          } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              if (n + e < o.N) r[e >> 1] |= (uint32_t)__ldg(rp + e) << (16 * (e & 1));
+          }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const __nv_bfloat162 x = __floats2bfloat162_rn(
+                __fadd_rn(__uint_as_float(w[e] << 16), __uint_as_float(r[e] << 16)),
+                __fadd_rn(__uint_as_float(w[e] & 0xffff0000u), __uint_as_float(r[e] & 0xffff0000u)));
+            w[e] = *reinterpret_cast<const uint32_t*>(&x);
+          }
+          v = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+        for (int i2 = -1; i2 < o.n_bc; ++i2) {
+          uint16_t* out = (i2 < 0 ? o.y : o.ybc[i2]) + off;
+          if (full && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
+            *reinterpret_cast<uint4*>(out) = v;
+          } else {
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              if (n + e < o.N) out[e] = (uint16_t)(w[e >> 1] >> (16 * (e & 1)));
+          }
+        }
+      }
+    }
+    __syncwarp();                                     // the tile may be written again
+  }
+}
+
 }  // namespace tmemw
+
+// Where a kernel's result goes, and the tensor maps of tile_epilogue's bulk stores (boxes of 32 tokens x 32 rows) over y and
+// over the peers' copies of it: they need a 16-byte aligned base and row pitch, and no residual.
+int tile_output(const sacq_layer* L, int64_t M, void* y, int64_t ldy, const void* residual, int64_t ldr, const BcastDst* bc,
+                tmemw::TmemOut* out, CUtensorMap* ty, tmemw::BcastMaps* tb);
+
 }  // namespace sacq
