@@ -34,8 +34,6 @@
 // decode-in-mainloop GEMM (codebook_cutlass_kernel.cu:234-583).
 #include <cuda.h>
 #include <math.h>
-#include <stdio.h>
-#include <stdlib.h>
 
 #include "common.cuh"
 #include "umma.cuh"
@@ -512,9 +510,6 @@ int launch_large_m_tmem(const sacq_layer* L, const void* q, const float* scale, 
   if (reinterpret_cast<uintptr_t>(q) % 16 != 0)
     return set_error(SACQ_ERR_ALIGNMENT, "quantized activations must be 16-byte aligned");
   int tok = nt_force > 0 ? kBM * nt_force : pick_tok(L, M);
-#ifdef SACQ_TUNE
-  if (const char* e = getenv("SACQ_TOK")) tok = atoi(e);
-#endif
   const bool cb_smem = cb_in_smem(L);
   const int act_stages = pick_act_stages(L, tok);
   if (M / tok + 1 > 0x7fffffff / ((d.out_features + kRows) / kRows))

@@ -737,15 +737,20 @@ void slice_extent(const sacq_layer* L, int split, int* slices, int* groups) {
 // of 4, 22 of 6, 15 of 8 run at once); eight above, where a slice's indices would no longer fit shared memory.
 int slices_for(int64_t K) { return K < 1024 ? 1 : K < 4096 ? 2 : K < 8192 ? 4 : 8; }
 
-// Completes a choice of tokens and slices; false if it does not fit shared memory.
+// Completes a choice of tokens and slices; false if it does not fit shared memory.  Gathers from global memory need the
+// rest of the SM's memory as L1, a line for every miss in flight: beyond 164 KB only what is needed at all (65,536
+// codewords: 2048 -> 6144 at 300 tokens 26.4 us with 227 KB taken, 20.6 now; 6144 -> 2048 at 400 38.8 / 27.4).
 bool split_fits(const sacq_layer* L, SplitMode mode, SplitChoice* c) {
   const int cb_bytes = codebook_smem(L), groups = mode == kSplitHiLo ? 0 : 1;
   slice_extent(L, c->split, &c->max_slices, &c->max_groups);
   const int tiles = ((int)(L->d.in_features / kStageK) + c->split - 1) / c->split * (mode == kSplitHalf ? 2 : 1);
-  for (c->act_stages = tiles < 2 ? 2 : tiles < kMaxAct ? tiles : kMaxAct; c->act_stages >= 2; --c->act_stages)
-    if (split_smem(split_layout(c->tok, c->split, c->act_stages, c->max_slices, groups * c->max_groups, cb_bytes)) <= 227 * 1024)
-      return true;
-  return false;
+  const size_t most = (cb_bytes > 0 ? 227 : 164) * 1024;
+  auto bytes = [&](int stages) {
+    return split_smem(split_layout(c->tok, c->split, stages, c->max_slices, groups * c->max_groups, cb_bytes));
+  };
+  for (c->act_stages = tiles < 2 ? 2 : tiles < kMaxAct ? tiles : kMaxAct; c->act_stages > 2; --c->act_stages)
+    if (bytes(c->act_stages) <= most) return true;
+  return bytes(2) <= 227 * 1024;
 }
 
 // Time of one CTA with `tok` tokens and `kbs` weight stages (us): prologue, the slower of expansion, MMAs and
@@ -793,17 +798,6 @@ bool split_k_choose(const sacq_layer* L, int64_t M, SplitMode mode, SplitChoice*
       if (c.us < out->us) *out = c;
     }
   }
-#ifdef SACQ_TUNE
-  if (const char* e = getenv("SACQ_SPLIT")) {
-    SplitChoice c;
-    if (sscanf(e, "%d,%d,%d", &c.tok, &c.split, &c.parts) == 3) {
-      c.tiles = (int)((M + c.tok - 1) / c.tok);
-      c.us = 0;
-      if (c.tok * c.parts > kMaxTok || c.split * c.parts > nkb || !split_fits(L, mode, &c)) return false;
-      *out = c;
-    }
-  }
-#endif
   return out->tok != 0;
 }
 
