@@ -1,0 +1,188 @@
+"""The tensor-core kernels, quantizers and weight encoders at the sizes where a tile, a slice of K, a remainder or a
+rule of the dispatch ends.  Oracle: the layer's own reconstruction (bit-exact against the CPU oracle elsewhere) in
+float64 or exact integer arithmetic, and torch's IEEE division for everything that is bytes."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+# A weight is the sum of two e4m3 halves (relative error 2^-8 at most) or an fp16 product (2^-11), the output is rounded
+# to bf16 (2^-9): relative to the result's norm no more than their sum.
+TOL = 2.0 ** -8 + 2.0 ** -9
+
+
+def _layer(N, K, d=8, C=4096, G=None, bias=True, seed=0):
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from sacq_b200 import PrecomputedPackedVectorCodebookLinear
+    from sacq_b200.synthetic import make_payload
+    p = make_payload(N, K, vector_dim=d, codebook_size=C, group_size=G, seed=N + K + C + seed, device="cuda", iters=1, fit=False)
+    b = (torch.randn(N, generator=torch.Generator().manual_seed(1)) * 0.05).to(torch.bfloat16) if bias else None
+    return PrecomputedPackedVectorCodebookLinear(p, b, "cuda")
+
+
+def _x(M, K, seed=3):
+    from sacq_b200.synthetic import make_activations
+    return make_activations(M, K, seed=seed).cuda()
+
+
+def _err(mod, y, q, s):
+    ref = (q.double() @ mod.dequantize_weight().double().t()) * s.reshape(-1, 1).double()
+    if mod.bias is not None:
+        ref = ref + mod.bias.double()
+    return float((y.double() - ref).norm() / ref.norm())
+
+
+@pytest.mark.parametrize("kernel,N,K,d,C,G", [
+    ("large", 100, 256, 8, 4096, None), ("large", 1000, 1024, 4, 4096, None), ("large", 128, 4096, 8, 256, None),
+    ("large", 257, 8192, 8, 4096, None), ("large", 520, 2048, 8, 65536, None),
+    ("large_grouped", 100, 512, 4, 81, 64), ("large_grouped", 333, 1024, 4, 2048, 64), ("large_grouped", 129, 4096, 8, 256, 128),
+    ("large_grouped", 64, 8192, 4, 64, 64)])
+def test_split_k_tile_and_slice_edges(kernel, N, K, d, C, G):
+    """One to eight slices of K; token tiles around 16, 256, 272 and 384 tokens.  A row's bytes do not depend on how many
+    rows there are, a residual adds like a separate addition, a wider output keeps its other columns."""
+    from sacq_b200 import quantize_rows
+    mod = _layer(N, K, d, C, G)
+    mod.set_kernel(kernel)
+    q, s = quantize_rows(_x(800, K))
+    whole = mod.linear_a8(q, s)
+    assert _err(mod, whole, q, s) <= TOL
+    for M in (1, 15, 17, 64, 255, 257, 272, 273, 384, 385):
+        y = mod.linear_a8(q[:M], s[:M])
+        assert torch.equal(y, whole[:M]), M
+        res = _x(M, N, seed=5)
+        assert torch.equal(mod.linear_a8(q[:M], s[:M], residual=res), y + res), M
+        out = torch.full((M, N + 3), 7.0, dtype=torch.bfloat16, device="cuda")
+        mod.linear_a8(q[:M], s[:M], out=out[:, :N])
+        assert torch.equal(out[:, :N], y) and float(out[:, N:].float().min()) == 7.0, M
+    assert mod.device_status() == 0
+
+
+@pytest.mark.parametrize("first,N,K,d,C,G", [
+    (8, 128, 256, 8, 4096, None), (8, 333, 768, 4, 256, None), (8, 6144, 256, 8, 4096, None), (8, 200, 2048, 8, 65536, None),
+    (12, 128, 512, 4, 81, 64), (12, 1000, 768, 4, 1024, 64), (12, 6144, 256, 8, 256, 128)])
+def test_batched_tiles_and_remainders(first, N, K, d, C, G):
+    """The kernels that keep the weights in tensor memory: the width of the tiles, the narrower last one, the number of
+    tiles per CTA and the way the output leaves change no byte."""
+    from sacq_b200 import quantize_rows
+    mod = _layer(N, K, d, C, G)
+    q, s = quantize_rows(_x(3300, K))
+    mod.set_kernel(first)
+    whole = mod.linear_a8(q, s)
+    assert _err(mod, whole, q, s) <= TOL
+    for M in (1, 31, 33, 127, 256, 257, 300, 385, 1000, 2049):
+        for which in range(first, first + 4):
+            mod.set_kernel(which)
+            assert torch.equal(mod.linear_a8(q[:M], s[:M]), whole[:M]), (M, which)
+        mod.set_kernel(first)
+        res = _x(M, N, seed=5)
+        assert torch.equal(mod.linear_a8(q[:M], s[:M], residual=res), whole[:M] + res), M
+        out = torch.full((M, N + 5), 7.0, dtype=torch.bfloat16, device="cuda")
+        mod.linear_a8(q[:M], s[:M], out=out[:, :N])
+        assert torch.equal(out[:, :N], whole[:M]) and float(out[:, N:].float().min()) == 7.0, M
+    assert mod.device_status() == 0
+
+
+@pytest.mark.parametrize("N,K,Ms", [(2000, 2048, (33, 300, 1000, 4100)), (1536, 6144, (33, 200, 1100, 2100)),
+                                    (6144, 1040, (321, 700, 5000)), (129, 256, (33, 129, 257))])
+def test_recipe_tiles(N, K, Ms):
+    """Every tile of the dense 8-bit GEMM, ragged token and row ends.  INT8 sums are exact, so the bytes are those of the
+    recipe's arithmetic on them; FP8 sums are fp32 in the tensor cores' order."""
+    from sacq_b200 import quantize_rows
+    mod = _layer(N, K, 8, 256, bias=False)
+    for mode in ("int8_symmetric", "fp8_e4m3fn"):
+        sw = mod.weight_row_scale(mode)
+        for M in Ms:
+            q, s = quantize_rows(_x(M, K), mode)
+            if mode == "int8_symmetric":
+                acc = q.double() @ mod.decode_weight_int8(sw).double().t()
+                want = ((acc.float() * sw.reshape(1, -1)) * s.reshape(-1, 1)).to(torch.bfloat16)
+                assert torch.equal(mod.linear_w8a8_int8(q, s, sw), want), M
+            else:
+                acc = q.double() @ mod.decode_weight_fp8(sw).double().t()
+                want = acc * sw.reshape(1, -1).double() * s.reshape(-1, 1).double()
+                y = mod.linear_w8a8_fp8(q, s, sw)
+                # fp32 sums of K products, each rounded at most once per addition, then one rounding to bf16
+                assert float((y.double() - want).norm() / want.norm()) <= 2.0 ** -9 + K * 2.0 ** -24, M
+    assert mod.device_status() == 0
+
+
+def _encode(z, s, mode):
+    v = z.float() / s                                   # a tensor divisor: IEEE division
+    if mode == "int8_symmetric":
+        return v.clamp(-127, 127).round().to(torch.int8)
+    return v.clamp(-448, 448).to(torch.float8_e4m3fn).view(torch.uint8)
+
+
+@pytest.mark.parametrize("K,d,C,G", [(16, 8, 16, None), (1008, 4, 128, None), (1040, 8, 256, None), (3088, 4, 2048, None),
+                                     (2048, 4, 1024, 64), (1040, 8, 65536, None)])
+def test_weight_bytes_equal_division(K, d, C, G):
+    """The 8-bit weight rows around a warp's 1,024 weights, for the layer's own row scales and for odd ones."""
+    mod = _layer(37, K, d, C, G)
+    w = mod.dequantize_weight()
+    for mode, decode in (("int8_symmetric", mod.decode_weight_int8), ("fp8_e4m3fn", mod.decode_weight_fp8)):
+        own = mod.weight_row_scale(mode).reshape(-1)
+        odd = own * torch.logspace(-3, 3, 37, device="cuda") * 1.000123
+        for sw in (own, odd):
+            got = decode(sw.reshape(mod.weight_row_scale(mode).shape).contiguous())
+            got = got if mode == "int8_symmetric" else got.view(torch.uint8)
+            assert torch.equal(got, _encode(w, sw.reshape(-1, 1), mode)), mode
+
+
+@pytest.mark.parametrize("M,K", [(1, 8), (3, 100), (5, 2048), (300, 2056), (2, 6144), (297, 6144), (4, 8200), (1, 40000)])
+def test_quantizer_bytes_equal_division(M, K):
+    """One to four chunks per thread, a warp or a CTA per row, rows longer than the registers hold."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from sacq_b200 import quantize_rows
+    x = _x(M, K)
+    x[0, : min(K, 6)] = torch.tensor([0.0, -0.0, 1e-39, -1e-39, 3.3e-38, 2.0 ** -126][: min(K, 6)], dtype=torch.bfloat16)
+    x[M - 1] *= 1e-20
+    for mode, top in (("int8_symmetric", 127.0), ("fp8_e4m3fn", 448.0)):
+        q, s = quantize_rows(x, mode)
+        want = x.float().abs().amax(1, keepdim=True) / torch.full((M, 1), top, device="cuda")
+        assert torch.equal(s.reshape(-1, 1), want)
+        got = q if mode == "int8_symmetric" else q.view(torch.uint8)
+        assert torch.equal(got, _encode(x, want, mode)), mode
+
+
+def test_silu_of_every_bf16_value():
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from sacq_b200 import act_quantize_rows, quantize_rows
+    a = torch.arange(65536, dtype=torch.int32).to(torch.int16).view(torch.bfloat16).cuda().reshape(-1, 64)
+    a = torch.where(torch.isfinite(a), a, torch.zeros_like(a))
+    for b in (torch.ones_like(a), torch.full_like(a, -0.37)):
+        q, s = act_quantize_rows("silu_mul", a, b)
+        q2, s2 = quantize_rows(torch.nn.functional.silu(a) * b)
+        assert torch.equal(s, s2) and torch.equal(q.view(torch.uint8), q2.view(torch.uint8))
+
+
+@pytest.mark.parametrize("N,K,d,C,G", [(2048, 2048, 8, 4096, None), (1000, 1024, 4, 1024, 64), (4096, 1024, 8, 65536, None)])
+def test_quantizer_inside_the_call_changes_no_byte(N, K, d, C, G):
+    """A call that quantizes on its way (few tokens: inside the GEMM) and the quantizer followed by the GEMM."""
+    from sacq_b200 import linear_a8_multi, quantize_rows
+    mod, other = _layer(N, K, d, C, G), _layer(N // 2, K, d, C, G, bias=False, seed=1)
+    for M in (1, 2, 7, 8, 9, 16, 17, 33, 64, 65, 300):
+        x = _x(M, K)
+        q, s = quantize_rows(x)
+        y = mod.linear_a8(q, s)
+        assert torch.equal(mod(x), y), M
+        assert _err(mod, y, q, s) <= TOL, M
+        qi, si = quantize_rows(x, "int8_symmetric")
+        assert torch.equal(mod.forward_int8(x), mod.linear_a8i(qi, si)), M
+        both = linear_a8_multi([mod, other], q, s)
+        assert torch.equal(both[0], y) and torch.equal(both[1], other.linear_a8(q, s)), M
+    assert mod.device_status() == 0 and other.device_status() == 0
+
+
+@pytest.mark.parametrize("N", [1024, 1000])
+def test_host_result_stored_by_the_gemm(N):
+    """Pinned results: stored by the GEMM where the rows are whole cache lines, copied otherwise."""
+    mod = _layer(N, 1024)
+    for M in (1, 16, 17, 64, 200):
+        x = _x(M, 1024)
+        out = torch.full((M, N), 5.0, dtype=torch.bfloat16).pin_memory()
+        mod.forward_host(x.cpu().pin_memory(), out)
+        torch.cuda.synchronize()
+        assert torch.equal(out, mod(x).cpu()), M
