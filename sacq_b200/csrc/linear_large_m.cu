@@ -110,6 +110,67 @@ int large_m_index_map(const sacq_layer* Lc, const CUtensorMap** out) {
   return SACQ_OK;
 }
 
+namespace {
+
+// A tile's width for `t` tokens: a multiple of 32, of 64 above 256 (two instructions).
+int width_of(int64_t t) {
+  const int64_t step = t > 256 ? 64 : 32;
+  return (int)((t + step - 1) / step * step);
+}
+
+// The tiles of M tokens in tiles of `tok` and one of what is left, and the modelled time of the busiest worker.  The
+// remainders go to the workers that have a whole tile less than the others, or, where that makes too many for them, to all.
+double plan_of(const sacq_layer* L, int64_t M, TileTime tile_us, int tok, tmemw::TilePlan* p) {
+  p->row_tiles = (int)((L->d.out_features + tmemw::kRows - 1) / tmemw::kRows);
+  p->tok = tok;
+  p->full = (int)(M / tok) * p->row_tiles;
+  p->rem = width_of(M % tok);
+  p->rem_m0 = (int)(M / tok * tok);
+  p->rem_first = 0;
+  const int tiles = p->full + (p->rem > 0 ? p->row_tiles : 0);
+  p->workers = tiles < L->num_sms ? tiles : L->num_sms;
+  const int rounds = p->full / p->workers, extra = p->full % p->workers;
+  const double whole = (rounds + (extra > 0 ? 1 : 0)) * tile_us(L, tok);
+  if (p->rem == 0) return whole;
+  auto rems = [&](int on) { return (p->row_tiles + on - 1) / on * tile_us(L, p->rem); };
+  const double few = rounds * tile_us(L, tok) + rems(p->workers - extra);
+  if (rounds == 0 && p->full > 0 && few >= whole + rems(extra)) {     // as many workers as whole tiles
+    p->workers = p->full;
+    return whole + rems(p->workers);
+  }
+  const double all = whole + rems(p->workers);
+  if (rounds > 0 && few >= all) return all;
+  p->rem_first = extra;
+  return few > whole ? few : whole;
+}
+
+}  // namespace
+
+// 8,192 tokens of a 6,144-row layer, for instance, are 1,008 tiles of 384 and 48 of 128 on 148 SMs: 7 rounds, where a grid
+// of equal tiles takes 8.
+bool plan_tiles(const sacq_layer* L, int64_t M, TileTime tile_us, int tok_force, tmemw::TilePlan* p) {
+  if (M / 32 + 1 > 0x7fffffff / ((L->d.out_features + tmemw::kRows) / tmemw::kRows)) return false;
+  double best_us = 1e30;
+  for (int t = tmemw::kMaxTok; t >= 32; t -= t > 256 ? 64 : 32) {
+    if (tok_force > 0 && t != tok_force) continue;
+    tmemw::TilePlan c;
+    const double us = plan_of(L, M, tile_us, t, &c);
+    if (us < best_us - 1e-9) {
+      best_us = us;
+      *p = c;
+    }
+  }
+  // one activation copy size for both kinds of tile
+  auto part_of = [](int t) { return t / (t > 256 ? 2 : 1); };
+  p->box = part_of(p->full > 0 ? p->tok : p->rem);
+  for (int a = part_of(p->rem); p->full > 0 && a > 0;) {
+    const int r = p->box % a;
+    p->box = a;
+    a = r;
+  }
+  return true;
+}
+
 int tile_output(const sacq_layer* L, int64_t M, void* y, int64_t ldy, const void* residual, int64_t ldr, const BcastDst* bc,
                 tmemw::TmemOut* out, CUtensorMap* ty, tmemw::BcastMaps* tb) {
   const sacq_layer_desc& d = L->d;

@@ -49,7 +49,6 @@ using namespace tmemw;
 constexpr int kBK = 128;             // e4m3 bytes per K block (one 128-byte swizzle row)
 constexpr int kMaxActStages = 6;
 constexpr int kMaxWStages = 4;
-constexpr int kMaxTok = 384;
 constexpr int kWCols = kBK / 2;      // TMEM columns of a weight stage: kBK / 4 high + kBK / 4 low
 struct TmemParams {
   const uint8_t* cb_hilo;       // [C][2][D] e4m3
@@ -59,11 +58,7 @@ struct TmemParams {
   int* status;
   TmemOut out;
   int K, C;
-  // The tiles of the call: `full` = `row_tiles` x the whole tiles of `tok` tokens, then `row_tiles` of `rem` tokens (0: none)
-  // at token `rem_m0`.  Worker w takes the full tiles w, w + workers, ...; a worker from `rem_first` on, every
-  // (workers - rem_first)-th of the others.
-  int tok, rem, rem_m0, rem_first, full, row_tiles, workers;
-  int box;                      // tokens of one activation copy
+  TilePlan plan;
   int act_stages;               // shared-memory activation stages, 2..kMaxActStages
   float out_mul;                // 2^-cb8_exp_shift
 };
@@ -77,7 +72,7 @@ __host__ __device__ inline TmemLayout tmem_layout(int tok, int act_stages, int s
   L.act_off = 0;
   L.act_stage = (uint32_t)(tok * kBK);
   L.stg_off = (uint32_t)act_stages * L.act_stage;
-  L.idx_off = L.stg_off + kEpiStaging;
+  L.idx_off = L.stg_off + epi_staging(tok);
   L.idx_slot = (uint32_t)(kRows * sb_bytes);
   L.cb_off = (L.idx_off + 2 * L.idx_slot + 127) & ~127u;
   L.sw_off = L.cb_off + (uint32_t)((cb_bytes + 127) & ~127);
@@ -139,7 +134,7 @@ large_m_tmem_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* sm = smem_raw + (base - raw);
-  const TmemLayout L = tmem_layout(p.tok, p.act_stages, SB_BYTES, CB_SMEM ? p.C * CW_BYTES : 0);
+  const TmemLayout L = tmem_layout(p.plan.tok, p.act_stages, SB_BYTES, CB_SMEM ? p.C * CW_BYTES : 0);
 
   // barrier indices
   constexpr int ACT_FULL = 0, ACT_EMPTY = kMaxActStages, W_FULL = 2 * kMaxActStages, W_EMPTY = W_FULL + kMaxWStages,
@@ -154,25 +149,10 @@ large_m_tmem_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   const int worker = (int)blockIdx.x;
   const int num_kb = p.K / kBK;
   const int act_stages = p.act_stages;
-  const int w_stages = min(kMaxWStages, ((int)kTmemCols - p.tok) / kWCols);
-  // this worker's tiles, whole ones first
-  const int n_full = p.full > worker ? (p.full - worker + p.workers - 1) / p.workers : 0;
-  const int rem_step = p.workers - p.rem_first, rem0 = worker - p.rem_first;
-  const int items = n_full + (p.rem > 0 && rem0 >= 0 && rem0 < p.row_tiles ? (p.row_tiles - rem0 + rem_step - 1) / rem_step : 0);
-  auto tile = [&](int t, int& n0, int& m0, int& tok) {
-    int r;
-    if (t < n_full) {
-      const int i = worker + t * p.workers;
-      r = i % p.row_tiles;
-      m0 = i / p.row_tiles * p.tok;
-      tok = p.tok;
-    } else {
-      r = rem0 + (t - n_full) * rem_step;
-      m0 = p.rem_m0;
-      tok = p.rem;
-    }
-    n0 = r * kRows;
-  };
+  const int w_stages = min(kMaxWStages, ((int)kTmemCols - p.plan.tok) / kWCols);
+  const TileWalk walk(p.plan, worker);
+  const int items = walk.items;
+  auto tile = [&](int t, int& n0, int& m0, int& tok) { walk.tile(p.plan, worker, t, n0, m0, tok); };
   const uint32_t cb_bytes = (uint32_t)(p.C * CW_BYTES);
 
   if (threadIdx.x == 0) {
@@ -237,7 +217,7 @@ large_m_tmem_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         if (!ok) break;
         const uint32_t dst = base + L.act_off + st * L.act_stage;
         if (elect_one()) mbar_arrive_expect_tx(bar(ACT_FULL + st), (uint32_t)(tok * kBK));
-        for (int b = 0; b < tok; b += p.box)
+        for (int b = 0; b < tok; b += p.plan.box)
           if (elect_one()) tma_load_2d(dst + (uint32_t)(b * kBK), &tmap_a, kb * kBK, m0 + b, bar(ACT_FULL + st));
         if (++st == act_stages) { st = 0; free_parity ^= 1; }
       }
@@ -431,61 +411,11 @@ cudaError_t launch_db(const CUtensorMap& ta, const CUtensorMap& ti, const CUtens
                  : launch_cb<D, BITS, false>(ta, ti, ty, tb, p, grid, smem, s);
 }
 
-// A tile's width for `t` tokens: a multiple of 32, of 64 above 256 (two instructions).
-int width_of(int64_t t) {
-  const int64_t step = t > 256 ? 64 : 32;
-  return (int)((t + step - 1) / step * step);
-}
-
 // Time of a tile (us), fitted to 2048 -> 6144, 2048 -> 2048, 6144 -> 2048 and 1024 -> 4096 at 1,024 - 8,192 tokens.
 double tile_us(const sacq_layer* L, int tok) {
   const double least = cb_in_smem(L) ? (L->d.vector_dim == 8 ? 0.52 : 0.65) : 11.5 / L->d.vector_dim;
   const double block = 0.0026 * tok > least ? 0.0026 * tok : least;
   return 2.3 + 0.0026 * tok + (double)L->d.in_features / kBK * block;
-}
-
-// The tiles of M tokens in tiles of `tok` and one of what is left, and the modelled time of the busiest worker.  The
-// remainders go to the workers that have a whole tile less than the others, or, where that makes too many for them, to all.
-double plan_tiles(const sacq_layer* L, int64_t M, int tok, TmemParams* p) {
-  p->row_tiles = (int)((L->d.out_features + kRows - 1) / kRows);
-  p->tok = tok;
-  p->full = (int)(M / tok) * p->row_tiles;
-  p->rem = width_of(M % tok);
-  p->rem_m0 = (int)(M / tok * tok);
-  const int at_once = L->num_sms, tiles = p->full + (p->rem > 0 ? p->row_tiles : 0);
-  p->workers = tiles < at_once ? tiles : at_once;
-  int rounds = p->full / p->workers, extra = p->full % p->workers;
-  double whole = (rounds + (extra > 0 ? 1 : 0)) * tile_us(L, tok);
-  p->rem_first = 0;
-  if (p->rem == 0) return whole;
-  auto rems = [&](int on) { return (p->row_tiles + on - 1) / on * tile_us(L, p->rem); };
-  const double few = rounds * tile_us(L, tok) + rems(p->workers - extra);
-  if (rounds == 0 && p->full > 0 && few >= whole + rems(extra)) {     // as many workers as whole tiles
-    p->workers = p->full;
-    return whole + rems(p->workers);
-  }
-  const double all = whole + rems(p->workers);
-  if (rounds > 0 && few >= all) return all;
-  p->rem_first = extra;
-  return few > whole ? few : whole;
-}
-
-// Width of the whole tiles: the one with the shortest modelled time.  8,192 tokens of a 6,144-row layer, for instance, are
-// 1,008 tiles of 384 and 48 of 128 on 148 SMs: 7 rounds, where a grid of equal tiles takes 8.
-int pick_tok(const sacq_layer* L, int64_t M) {
-  if (M > (1 << 24)) return kMaxTok;
-  int best = kMaxTok;
-  double best_us = 1e30;
-  for (int t = kMaxTok; t >= 32; t -= t > 256 ? 64 : 32) {
-    if (M > t && t < 128) continue;
-    TmemParams p;
-    const double us = plan_tiles(L, M, t, &p);
-    if (us < best_us - 1e-9) {
-      best_us = us;
-      best = t;
-    }
-  }
-  return best;
 }
 
 }  // namespace
@@ -509,24 +439,15 @@ int launch_large_m_tmem(const sacq_layer* L, const void* q, const float* scale, 
   if (M > (1 << 30)) return set_error(SACQ_ERR_UNSUPPORTED, "M=%lld too large", (long long)M);
   if (reinterpret_cast<uintptr_t>(q) % 16 != 0)
     return set_error(SACQ_ERR_ALIGNMENT, "quantized activations must be 16-byte aligned");
-  int tok = nt_force > 0 ? kBM * nt_force : pick_tok(L, M);
+  TmemParams p{};
+  if (!plan_tiles(L, M, tile_us, kBM * nt_force, &p.plan))
+    return set_error(SACQ_ERR_UNSUPPORTED, "M=%lld: too many tiles", (long long)M);
+  const int tok = p.plan.tok;
   const bool cb_smem = cb_in_smem(L);
   const int act_stages = pick_act_stages(L, tok);
-  if (M / tok + 1 > 0x7fffffff / ((d.out_features + kRows) / kRows))
-    return set_error(SACQ_ERR_UNSUPPORTED, "M=%lld: too many tiles", (long long)M);
-  TmemParams p{};
-  plan_tiles(L, M, tok, &p);
-  // one copy size for both kinds of tile
-  auto part_of = [](int t) { return t / (t > 256 ? 2 : 1); };
-  p.box = part_of(p.full > 0 ? p.tok : p.rem);
-  for (int a = part_of(p.rem); p.full > 0 && a > 0;) {
-    const int r = p.box % a;
-    p.box = a;
-    a = r;
-  }
   CUtensorMap ta;
   {
-    const int rc = encode_bytes_2d(&ta, q, (uint64_t)d.in_features, (uint64_t)M, (uint64_t)d.in_features, kBK, p.box,
+    const int rc = encode_bytes_2d(&ta, q, (uint64_t)d.in_features, (uint64_t)M, (uint64_t)d.in_features, kBK, p.plan.box,
                                    CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc != SACQ_OK) return rc;
   }
@@ -549,7 +470,7 @@ int launch_large_m_tmem(const sacq_layer* L, const void* q, const float* scale, 
   p.out_mul = ldexpf(1.f, -L->cb8_exp_shift);
   const TmemLayout lay = tmem_layout(tok, act_stages, sb_bytes_of(L), cb_smem ? L->cb_entries * d.vector_dim * 2 : 0);
   const size_t smem = smem_request(lay);
-  const dim3 grid((unsigned)p.workers);
+  const dim3 grid((unsigned)p.plan.workers);
   cudaError_t e;
   const int D = d.vector_dim, B = d.index_bits;
   if (D == 8 && B == 12) e = launch_db<8, 12>(ta, *ti, ty, tb, p, cb_smem, grid, smem, s);

@@ -51,7 +51,6 @@ using namespace tmemw;
 constexpr int kStageK = 128;          // k per weight stage
 constexpr int kMaxAct = 6;            // activation tiles in flight (128 bytes of every token each)
 constexpr int kMaxW = 4;              // weight stages in tensor memory
-constexpr int kMaxTok = 384;          // tokens per CTA
 constexpr int kSliceBytes = kRows * 16;
 constexpr float kHalfPreScale = 4096.f;   // keeps fp16(codeword x scale) far from the subnormals
 

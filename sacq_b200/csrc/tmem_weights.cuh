@@ -118,106 +118,42 @@ struct BcastMaps {
   CUtensorMap m[kMaxBcast];
 };
 
-// Epilogue of one CTA, run by all expander threads after the accumulator is complete:
-//   y[m0 + token, n0 + row] = bf16(fma(sa[token], acc[row][token] * sw, bs))
-// `lane_addr` = TMEM address of the warp's lane quarter (accumulator column 0), `row` = the
-// thread's weight row (TMEM lane), `kpart` = which 32 tokens of every 128-token sub-tile the
-// warp converts, `sap` = the NT*128 token scales in shared memory, `stage_base` = n_stage idle
-// buffers of kStageTile bytes.
-template <int NT>
-__device__ __forceinline__ void tmem_epilogue(const TmemOut& o, const CUtensorMap* tmap_y, const CUtensorMap* tmap_bc,
-                                              uint32_t lane_addr, int row,
-                                              int kpart, int et, const float* sap, float sw, float bs,
-                                              uint8_t* stage_base, int n_stage, int m0, int n0) {
-  // The accumulator holds y transposed (lane = weight row, column = token).  Each 128-token
-  // sub-tile goes through shared memory (the activation stages are idle now): a thread
-  // writes its row's values of 32 tokens as 2-byte elements of a dense [token][row] bf16
-  // tile; the tile then leaves by ONE tiled bulk store (clipped at the edges of y), which
-  // overlaps the staging of the next sub-tile in the other buffer.  With a residual, peer
-  // copies or an unaligned y the expander threads store the token rows themselves.
-  const int c0 = kpart * 32;                      // this warp's 32 tokens of every sub-tile
-#pragma unroll 1
-  for (int t = 0; t < NT; ++t) {
-    if (m0 + t * kBM >= o.M) break;               // uniform over the CTA
-    uint8_t* stg = stage_base + (t % n_stage) * kStageTile;
-    {
-      uint32_t r[32];
-      tmem_ld_32x32(lane_addr + (uint32_t)(t * kBM + c0), r);
-      uint8_t* dst = stg + c0 * (kRows * 2) + row * 2;
-      const float4* sa4 = reinterpret_cast<const float4*>(sap + t * kBM + c0);
-#pragma unroll
-      for (int c4 = 0; c4 < 8; ++c4) {
-        const float4 sa = sa4[c4];                // four token scales per (broadcast) load
-        const int c = c4 * 4;
-        // two conversions per instruction; the halves go to two token rows of the staging tile
-        const __nv_bfloat162 p01 = __floats2bfloat162_rn(fmaf(sa.x, __uint_as_float(r[c]) * sw, bs),
-                                                         fmaf(sa.y, __uint_as_float(r[c + 1]) * sw, bs));
-        const __nv_bfloat162 p23 = __floats2bfloat162_rn(fmaf(sa.z, __uint_as_float(r[c + 2]) * sw, bs),
-                                                         fmaf(sa.w, __uint_as_float(r[c + 3]) * sw, bs));
-        const uint32_t w01 = *reinterpret_cast<const uint32_t*>(&p01), w23 = *reinterpret_cast<const uint32_t*>(&p23);
-        *reinterpret_cast<uint16_t*>(dst + (c + 0) * (kRows * 2)) = (uint16_t)w01;
-        *reinterpret_cast<uint16_t*>(dst + (c + 1) * (kRows * 2)) = (uint16_t)(w01 >> 16);
-        *reinterpret_cast<uint16_t*>(dst + (c + 2) * (kRows * 2)) = (uint16_t)w23;
-        *reinterpret_cast<uint16_t*>(dst + (c + 3) * (kRows * 2)) = (uint16_t)(w23 >> 16);
-      }
-    }
-    const int m_first = m0 + t * kBM;
-    if (o.y_tma) {
-      fence_proxy_async();                        // generic-proxy writes -> visible to the bulk store
-      xbarrier();                                 // the sub-tile is staged
-      if (et == 0) {
-        // one bulk-store group per sub-tile: the local copy and, in a column split, every peer's copy
-        tma_store_2d_issue(tmap_y, n0 * 2, m_first, smem_u32(stg));
-        for (int c = 0; c < o.n_bc; ++c) tma_store_2d_issue(tmap_bc + c, n0 * 2, m_first, smem_u32(stg));
-        tma_store_commit();
-        // the other buffer's store (the previous sub-tile) must have read its tile before that
-        // buffer is written again; with a single buffer, this store itself
-        if (n_stage == 2) tma_store_wait_read<1>(); else tma_store_wait_read<0>();
-      }
-      xbarrier();
-    } else {
-      xbarrier();                                 // the sub-tile is staged
-#pragma unroll 2
-      for (int i = et; i < kBM * (kRows / 8); i += kXThreads) {
-        const int tok = i >> 4, ch = i & 15;
-        const int m = m_first + tok, n = n0 + ch * 8;
-        if (m >= o.M || n >= o.N) continue;
-        uint4 v = *reinterpret_cast<const uint4*>(stg + tok * (kRows * 2) + ch * 16);
-        const int64_t off = (int64_t)m * o.ldy + n;
-        const bool full = n + 8 <= o.N;
-        if (o.residual != nullptr) {
-          // bf16(bf16(v) + residual): the two roundings of `linear(x) + residual`
-          const uint16_t* rp = o.residual + (int64_t)m * o.ldr + n;
-          uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            if (n + e < o.N) {
-              const uint32_t a = (w[e >> 1] >> (16 * (e & 1))) & 0xffffu;
-              const uint32_t o = float_to_bf16_bits(__fadd_rn(bf16_bits_to_float(a), bf16_bits_to_float(__ldg(rp + e))));
-              w[e >> 1] = (w[e >> 1] & ~(0xffffu << (16 * (e & 1)))) | (o << (16 * (e & 1)));
-            }
-          }
-          v = make_uint4(w[0], w[1], w[2], w[3]);
-        }
-        for (int c = -1; c < o.n_bc; ++c) {
-          uint16_t* out = (c < 0 ? o.y : o.ybc[c]) + off;
-          if (full && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
-            *reinterpret_cast<uint4*>(out) = v;
-          } else {
-            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int e = 0; e < 8; ++e)
-              if (n + e < o.N) out[e] = (uint16_t)(w[e >> 1] >> (16 * (e & 1)));
-          }
-        }
-      }
-      if (n_stage == 1) xbarrier();               // before the next sub-tile reuses the staging rows
-    }
+// ---- persistent tiles ------------------------------------------------------------------------------------
+
+constexpr int kMaxTok = 384;         // tokens of a tile = accumulator columns
+
+// The tiles of a call: `full` = `row_tiles` x the whole tiles of `tok` tokens, then `row_tiles` of `rem` tokens (0: none)
+// at token `rem_m0`.  Worker w takes the full tiles w, w + workers, ...; a worker from `rem_first` on, every
+// (workers - rem_first)-th of the others.
+struct TilePlan {
+  int tok, rem, rem_m0, rem_first, full, row_tiles, workers;
+  int box;                      // tokens of one activation copy
+};
+
+// One worker's walk through them, whole tiles first.
+struct TileWalk {
+  int n_full, items, rem0, rem_step;
+  __device__ __forceinline__ TileWalk(const TilePlan& p, int worker) {
+    n_full = p.full > worker ? (p.full - worker + p.workers - 1) / p.workers : 0;
+    rem_step = p.workers - p.rem_first;
+    rem0 = worker - p.rem_first;
+    items = n_full + (p.rem > 0 && rem0 >= 0 && rem0 < p.row_tiles ? (p.row_tiles - rem0 + rem_step - 1) / rem_step : 0);
   }
-  // shared memory stays valid until every store has read it; the writes themselves (local and peer)
-  // are in the memory system then, like plain stores, and the grid's end orders them
-  if (o.y_tma && et == 0) tma_store_wait_read<0>();
-}
+  __device__ __forceinline__ void tile(const TilePlan& p, int worker, int t, int& n0, int& m0, int& tok) const {
+    int r;
+    if (t < n_full) {
+      const int i = worker + t * p.workers;
+      r = i % p.row_tiles;
+      m0 = i / p.row_tiles * p.tok;
+      tok = p.tok;
+    } else {
+      r = rem0 + (t - n_full) * rem_step;
+      m0 = p.rem_m0;
+      tok = p.rem;
+    }
+    n0 = r * kRows;
+  }
+};
 
 // 16 lanes x 32 consecutive fp32 columns, as four 16 x 8 fragments: registers 4 j + 0, 1 = lane (thread / 4), columns
 // 8 j + 2 (thread % 4) + 0, 1; registers 4 j + 2, 3 = lane (thread / 4) + 8.
@@ -237,7 +173,8 @@ __device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t a, uin
 }
 
 constexpr int kWarpTile = 32 * 64;                    // a warp's staged output: 32 tokens x 32 weight rows, bf16
-constexpr int kEpiStaging = kXWarps * kWarpTile;     // one per expander warp
+// One per expander warp that has tokens to store.
+__host__ __device__ constexpr uint32_t epi_staging(int tok) { return (uint32_t)((tok >= 128 ? 4 : (tok + 31) / 32) * 4 * kWarpTile); }
 
 // Epilogue of one tile, run by the expander warps after the accumulator is complete:
 //   y[m0 + token, n0 + row] = bf16(fma(sa[token], acc[row][token] * sw[row], bias[row]))
@@ -361,6 +298,11 @@ __device__ __forceinline__ void tile_epilogue(const TmemOut& o, const CUtensorMa
 }
 
 }  // namespace tmemw
+
+// Modelled time (us) of a tile of `tok` tokens; the plan with the shortest modelled time of the busiest worker (with
+// `tok_force` > 0, of that width).  false: too many tiles.
+typedef double (*TileTime)(const sacq_layer* L, int tok);
+bool plan_tiles(const sacq_layer* L, int64_t M, TileTime tile_us, int tok_force, tmemw::TilePlan* p);
 
 // Where a kernel's result goes, and the tensor maps of tile_epilogue's bulk stores (boxes of 32 tokens x 32 rows) over y and
 // over the peers' copies of it: they need a 16-byte aligned base and row pitch, and no residual.
