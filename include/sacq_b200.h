@@ -155,7 +155,7 @@ SACQ_API int sacq_peer_buffer_destroy(int device, void* dev_ptr);
  *   s = max|x| / 127 per row (1 for an all-zero row), q = int8(round_half_even(clamp(x / s, -127, 127))).
  * sacq_linear_a8i is sacq_linear_a8 for such activations: the same exact weights (no 8-bit
  * rounding of the weights, unlike the reference's INT8 GEMM), int8 widened to fp16 in front of
- * fp16 tensor-core MMAs (tcgen05 kind::f16 from 48 rows, warp MMAs below).  Its workspace is
+ * fp16 tensor-core MMAs (tcgen05 kind::f16 where the codebook and the token count favour it, warp MMAs below).  Its workspace is
  * sacq_workspace_bytes_int8(layer, M) bytes, 256-byte aligned, zero-filled once. */
 SACQ_API int sacq_quant_act_int8(const void* x_bf16, int64_t x_pitch, int64_t M, int64_t K, void* q_out,
                                  float* scale_out, void* stream);
@@ -299,18 +299,15 @@ SACQ_API int sacq_linear_a8_static_scratch(const sacq_layer_t* layer, const void
 SACQ_API int64_t sacq_static_scratch_bytes(void);
 
 /* Forces a GEMM kernel (for tests and benchmarks): 0 = automatic, 1 = small-M kernel
- * (its own choice of variant), 2 = tensor-core kernel with expanded weight tiles in shared
- * memory, 3 = small-M CUDA-core variant, 4 = small-M warp-MMA variant, 5 = warp-MMA variant
+ * (its own choice of variant), 2 = tensor-core kernel that splits K over clusters, 3 = small-M CUDA-core variant, 4 = small-M warp-MMA variant, 5 = warp-MMA variant
  * without shared-memory staging, 6 = warp-MMA variant that unpacks the indices in shared memory
- * (any index width, any group size that is a multiple of 32), 7 = tensor-core kernel for grouped
- * scales, 8 = tensor-core kernel with the expanded weights in tensor memory (9, 10, 11: the same
- * with 1, 2, 3 token sub-tiles of 128 per CTA), 12 = that design for grouped scales (13, 14, 15:
- * 1, 2, 3 sub-tiles).
+ * (any index width, any group size that is a multiple of 32), 7 = the split-K tensor-core
+ * kernel for grouped scales, 8 = tensor-core kernel for batches, persistent CTAs (9, 10, 11: with
+ * tiles of 128, 256, 384 tokens), 12 = that design for grouped scales (13, 14, 15: likewise).
  * Returns SACQ_ERR_UNSUPPORTED from the next forward if the forced kernel cannot run the layer. */
 SACQ_API int sacq_layer_set_kernel(sacq_layer_t* layer, int which);
-/* Which kernel a forward with M rows would use (1 = small-M, 2 = tensor-core kernel with
- * shared-memory weight tiles, 3 = tensor-core kernel for grouped scales, 4 = tensor-core kernel
- * with tensor-memory weights), or a negative error. */
+/* Which kernel a forward with M rows would use (1 = small-M, 2 = split-K tensor-core kernel,
+ * 3 = the same for grouped scales, 4 = tensor-core kernel for batches, 5 = the same for grouped scales), or a negative error. */
 SACQ_API int sacq_layer_kernel_for(const sacq_layer_t* layer, int64_t M);
 
 /* Reads the layer's device-side status word (synchronises the device): 0, or a

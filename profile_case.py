@@ -160,15 +160,6 @@ def print_trace(layer, a):
             print(f"  tile {it}: index rows landed {t[b]-t0}, CTA in step {t[b+1]-t0}, gathers+MMAs done {t[b+2]-t0}, "
                   f"partials exchanged {t[b+3]-t0}, reduced+stored {t[b+4]-t0}, tile closed {t[b+5]-t0}")
             it += 1
-    elif kern == "large_tmem" and hasattr(lib, "sacq_debug_tmem_trace"):
-        buf = (ctypes.c_longlong * (8 * 72))()
-        lib.sacq_debug_tmem_trace(buf)
-        t = [list(buf)[i * 72:(i + 1) * 72] for i in range(8)]
-        t0, nk = t[0][0], a.K // 128
-        print(f"TMEM-weight kernel, CTA (0,0) (ns from the end of the prologue): accumulator complete {t[0][3]-t0}, exit {t[0][4]-t0}")
-        print("  expander: weight stage free   ", [v - t0 for v in t[2][8:8 + nk]])
-        print("  expander: weight stage written", [v - t0 for v in t[5][8:8 + nk]])
-        print("  issuer: operands ready        ", [v - t0 for v in t[1][8:8 + nk]])
     else:
         print("no trace: the library was not built with -DSACQ_TRACE, or this kernel records none")
 

@@ -28,8 +28,6 @@
 // cluster barriers, so its peers do too.  No cluster multicast.
 #include <cuda.h>
 #include <math.h>
-#include <stdio.h>
-#include <stdlib.h>
 #include <string.h>
 
 #include <mutex>

@@ -16,11 +16,9 @@ namespace tmemw {
 using namespace umma;
 
 constexpr int kRows = 128;           // weight rows per CTA = TMEM lanes
-constexpr int kTokTile = kBM * 128;  // 16 KB: 128 tokens x one 128-byte K block
 constexpr int kXWarps = 16;                  // expander warps: four per TMEM lane quarter
 constexpr int kXThreads = kXWarps * 32;
 constexpr int kCtaThreads = 64 + kXThreads;  // + TMA producer warp + MMA issuer warp
-constexpr int kStageTile = kBM * kRows * 2;  // 32 KB: one staged [128 tokens][128 rows] bf16 output sub-tile
 
 __device__ __forceinline__ void xbarrier() { asm volatile("bar.sync 1, %0;" ::"n"(kXThreads) : "memory"); }
 // AND of a predicate over the expander threads (named barrier 1).

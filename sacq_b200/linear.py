@@ -436,7 +436,7 @@ class PrecomputedPackedVectorCodebookLinear(torch.nn.Module):
     def set_kernel(self, which: str | int) -> None:
         """Force a GEMM kernel: 'auto' (0), 'small' (1), 'large' (2), 'small_simt' (3), 'small_mma' (4),
         'small_mma_direct' (5), 'small_mma_unpacked' (6), 'large_grouped' (7), 'large_tmem' (8; 9-11 also
-        fix its token sub-tiles per CTA to 1-3), 'large_tmem_grouped' (12; 13-15 likewise)."""
+        fix its tiles to 128, 256 or 384 tokens), 'large_tmem_grouped' (12; 13-15 likewise)."""
         code = {"auto": 0, "small": 1, "large": 2, "small_simt": 3, "small_mma": 4, "small_mma_direct": 5,
                 "small_mma_unpacked": 6, "large_grouped": 7, "large_tmem": 8, "large_tmem1": 9,
                 "large_tmem2": 10, "large_tmem3": 11, "large_tmem_grouped": 12, "large_tmem_grouped1": 13,
