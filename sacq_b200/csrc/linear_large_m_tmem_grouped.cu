@@ -425,7 +425,9 @@ cudaError_t glaunch(const CUtensorMap& ta, const CUtensorMap& ti, const CUtensor
 // Time of a tile (us), fitted to d = 4, 10-bit, group 64 at 1,024 - 8,192 tokens.
 double g_tile_us(const sacq_layer* L, int tok) {
   if (g_act_stages(L, tok) < 2) return 1e9;
-  const double least = 0.75, rate = (tok <= 256 ? 0.0039 : 0.0035) * tok, block = rate > least ? rate : least;
+  // two activation stages (64 KB of codebook) leave the tensor cores waiting for tiles
+  const double least = 0.75, rate = (tok <= 256 ? 0.0039 : g_act_stages(L, tok) > 2 ? 0.0035 : 0.0042) * tok;
+  const double block = rate > least ? rate : least;
   return 3.0 + 0.0026 * tok + (double)L->d.in_features / 128 * block;
 }
 
@@ -445,11 +447,11 @@ bool large_m_tmem_grouped_supported(const sacq_layer* L) {
 }
 
 // From how many tokens this kernel beats the split-K kernel (linear_large_m_grouped.cu), whose clusters stop
-// paying once whole token tiles fill the device (quantizer + GEMM at d = 4, 10-bit, group 64: 2048x6144
-// 28.5 / 25.8 us at 512 tokens, 24.3 / 18.9 the other way round at 300; 1024x4096 18.9 / 17.2 at 768; 2048x2048
-// 23.8 / 24.7 at 1,000 and 36.5 / 28.1 at 1,500; 6144x2048 47.5 / 54.4 and 71.7 / 62.2).
+// paying once whole token tiles fill the device, and which walks more than 1,024 tokens in slabs (quantizer + GEMM at
+// d = 4, 10-bit, group 64, split-K / this: 2048x6144 32.4 / 23.8 us at 600 tokens; 1024x4096 13.1 / 12.8 at 600, 23.8 /
+// 15.3 at 1,024; 2048x2048 19.7 / 20.9 at 1,024, 33.5 / 23.0 at 1,500; 6144x2048 45.0 / 45.3 and 69.5 / 56.2).
 int64_t large_m_tmem_grouped_min_m(const sacq_layer* L) {
-  return L->d.out_features >= 5120 ? 448 : L->d.out_features >= 4096 ? 704 : 1024;
+  return L->d.out_features >= 5120 ? 448 : L->d.out_features >= 4096 ? 600 : 1025;
 }
 
 // Workspace behind the counter region: the fp16 activations of one token slab.
