@@ -20,6 +20,8 @@
 //   8 SUBS more warps : epilogue: TMEM lane quarter x token sub-tile x column half each, through shared memory
 //                       so that four lanes store a token's 64 bytes (16-byte pieces of 32 rows at a time left half of
 //                       every sector: 5.7 us of a 256 x 256 tile, now 2.5).
+// Rows that begin or end anywhere go out an element per lane, 64 contiguous bytes a store (2048 -> 6137, INT8, 1,500 tokens:
+// 112 us with a row per lane, 31 now).
 // A last token tile of at most 128 tokens loads and multiplies one sub-tile only.
 // What bounds it: the 256 x 256 tile the tensor cores (0.48 us per K block, 1024 of 1090 clocks), the small ones the
 // operands through L2 (about 19 TB/s over the chip).  1,024 tokens, 6144 -> 2048, FP8, weight bytes included: 45 us
@@ -205,27 +207,28 @@ dense_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
           return (uint32_t)float_to_bf16_bits(v);
         };
         uint16_t* y = p.y + n0 + c0;
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          uint32_t o[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) o[j] = fin(v * 8 + 2 * j) | (fin(v * 8 + 2 * j + 1) << 16);
+          *reinterpret_cast<uint4*>(stage + lane * kStagePitch + v * 16) = make_uint4(o[0], o[1], o[2], o[3]);
+        }
+        __syncwarp();
         if (n0 + c0 + 32 <= p.N && (reinterpret_cast<uintptr_t>(y) & 15) == 0 && (p.ldy & 7) == 0) {
-#pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            uint32_t o[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) o[j] = fin(v * 8 + 2 * j) | (fin(v * 8 + 2 * j + 1) << 16);
-            *reinterpret_cast<uint4*>(stage + lane * kStagePitch + v * 16) = make_uint4(o[0], o[1], o[2], o[3]);
-          }
-          __syncwarp();
 #pragma unroll
           for (int i = 0; i < 4; ++i) {               // four lanes per token: whole 32-byte sectors
             const int row = i * 8 + (lane >> 2);
             const uint4 o = *reinterpret_cast<const uint4*>(stage + row * kStagePitch + (lane & 3) * 16);
             if (mw + row < p.M) *reinterpret_cast<uint4*>(y + (mw + row) * p.ldy + (lane & 3) * 8) = o;
           }
-          __syncwarp();
-        } else if (m < p.M) {
-#pragma unroll
-          for (int c = 0; c < 32; ++c)
-            if (n0 + c0 + c < p.N) y[m * p.ldy + c] = (uint16_t)fin(c);
+        } else if (n0 + c0 + lane < p.N) {            // rows that begin or end anywhere: an element per lane
+          const int rows = (int)(p.M - mw < 32 ? p.M - mw : 32);
+#pragma unroll 8
+          for (int row = 0; row < rows; ++row)
+            y[(mw + row) * p.ldy + lane] = *reinterpret_cast<const uint16_t*>(stage + row * kStagePitch + lane * 2);
         }
+        __syncwarp();
       }
     }
   }
