@@ -80,18 +80,10 @@ int64_t tmem_min_m(const sacq_layer* L) {
 // once per 16-token chunk: from the second chunk on wide or deep layers, from the third on all but the smallest.
 // A codebook in L2 leaves the small-M kernel 2 warps' gathers in flight per scheduler: on wide layers the split-K
 // kernel wins from one token on (2048x6144, 65,536 entries: 17.8 / 13.4 us at 16 tokens, 46 / 15.6 at 64).
-bool split_wins(const sacq_layer* L, int64_t M, int64_t smallest) {
+bool split_wins(const sacq_layer* L, int64_t M) {
   if (!split_k_codebook_in_smem(L)) return M > 16 || L->d.out_features >= 4096;
   const int64_t work = L->d.in_features * L->d.out_features;
-  return (M > 16 && (L->d.out_features >= 4096 || work >= (8 << 20))) || (M > 32 && work > smallest);
-}
-
-// Layers with grouped scales below grouped_min_m(): the index-unpacking choice of the small-M path hands over to
-// the fp16 split-K kernel (quantizer + GEMM, d = 4, 10-bit, group 64: 2048x2048 12.8 / 9.9 us at 33 tokens,
-// 6144x2048 25.2 / 14.1 at 17, 4096x1024 16.2 / 10.9 at 33; 1024x1024 and 2048x1024 stay).
-bool small_m_hands_over(const sacq_layer* L, int64_t M) {
-  return (L->force_kernel == 0 || L->force_kernel == 1 || L->force_kernel == 6) && L->num_groups > 1 &&
-         M <= large_m_grouped_slab() && M < grouped_min_m(L) && split_wins(L, M, 2 << 20) && large_m_grouped_supported(L);
+  return (M > 16 && (L->d.out_features >= 4096 || work >= (8 << 20))) || M > 32;
 }
 
 int pick_kernel(const sacq_layer* L, int64_t M) {
@@ -109,7 +101,7 @@ int pick_kernel(const sacq_layer* L, int64_t M) {
   // 6144x2048 15.4 / 11.5, 2048x6144 15.5 / 8.9; at 33: 1024x1024 7.3 / 5.7, 2048x2048 9.2 / 8.8, 4096x1024
   // 9.5 / 9.2, 2048x1024 even.
   if (large_m_supported(L)) {
-    if (split_wins(L, M, 0)) return 2;
+    if (split_wins(L, M)) return 2;
   } else if (large_m_tmem_grouped_supported(L) && M >= large_m_tmem_grouped_min_m(L)) {
     return 5;                                          // grouped scales, odd index widths: weights in tensor memory
   } else if (M >= grouped_min_m(L) && large_m_grouped_supported(L)) {
@@ -328,7 +320,7 @@ SACQ_API int sacq_layer_kernel_for(const sacq_layer_t* L, int64_t M) {
 SACQ_API int64_t sacq_workspace_bytes(const sacq_layer_t* L, int64_t M) {
   if (L == nullptr || M < 0) return 0;
   const int k = pick_kernel(L, M);
-  if (k == 3 || (k == 1 && small_m_hands_over(L, M))) return kCounterBytes + large_m_grouped_workspace_bytes(L, M);
+  if (k == 3) return kCounterBytes + large_m_grouped_workspace_bytes(L, M);
   if (k == 5) return kCounterBytes + large_m_tmem_grouped_workspace_bytes(L, M);
   const int64_t slab = small_m_slab_rows(L);
   return small_m_workspace_bytes(L, M < slab ? M : slab);
@@ -353,9 +345,8 @@ int linear_a8_impl(const sacq_layer_t* L, const void* q, const float* scale, int
                      (long long)L->d.out_features);
   DeviceGuard guard(L->d.device);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  int k = pick_kernel(L, M);
+  const int k = pick_kernel(L, M);
   if (k < 0) return set_error(k, "no kernel can run this layer geometry");
-  if (k == 1 && small_m_hands_over(L, M)) k = 3;
   if (k == 2) return launch_large_m(L, q, scale, M, y_out, ldy, s, residual, ldr, bc);
   if (k == 4)
     return launch_large_m_tmem(L, q, scale, M, y_out, ldy, s, residual, ldr, bc,
@@ -663,8 +654,7 @@ SACQ_API int sacq_linear_a8_multi(const sacq_layer_t* const* layers, int num_lay
   {
     // one launch when every layer would use the staged small-M kernel on a common geometry
     bool small = num_layers >= 2;
-    for (int l = 0; l < num_layers && small; ++l)
-      small = pick_kernel(layers[l], M) == 1 && !small_m_hands_over(layers[l], M);
+    for (int l = 0; l < num_layers && small; ++l) small = pick_kernel(layers[l], M) == 1;
     if (small) {
       DeviceGuard guard(layers[0]->d.device);
       const int rc = launch_small_m_multi(layers, num_layers, q, scale, M, y_outs, ldys,
@@ -682,8 +672,7 @@ SACQ_API int sacq_linear_a8_multi(const sacq_layer_t* const* layers, int num_lay
     }
     // ... or its fp16 form for grouped scales
     bool grouped = num_layers >= 2 && workspace != nullptr && workspace_bytes > kCounterBytes;
-    for (int l = 0; l < num_layers && grouped; ++l)
-      grouped = pick_kernel(layers[l], M) == 3 || (pick_kernel(layers[l], M) == 1 && small_m_hands_over(layers[l], M));
+    for (int l = 0; l < num_layers && grouped; ++l) grouped = pick_kernel(layers[l], M) == 3;
     if (grouped) {
       DeviceGuard guard(layers[0]->d.device);
       const int rc = launch_large_m_grouped_multi(layers, num_layers, q, scale, M, y_outs, ldys,
@@ -727,8 +716,7 @@ int forward_impl(const sacq_layer_t* L, const void* x_bf16, int64_t x_pitch, int
   if (rows_ok) {
     const Int8Route r = int8 ? int8_route(L, M) : kInt8Small;
     const int k = int8 ? 0 : pick_kernel(L, M);
-    const bool over = k == 1 && small_m_hands_over(L, M);
-    if (k == 1 && !over && !own_quantizer && quantizes_in_gemm(L, M)) {
+    if (k == 1 && !own_quantizer && quantizes_in_gemm(L, M)) {
       DeviceGuard guard(L->d.device);
       return launch_small_m(L, q_scratch, scale_scratch, M, y_out, ldy, workspace, workspace_bytes,
                             static_cast<cudaStream_t>(stream), residual, ldr, 0, nullptr, x_bf16, x_pitch);
@@ -736,7 +724,7 @@ int forward_impl(const sacq_layer_t* L, const void* x_bf16, int64_t x_pitch, int
     if (r == kInt8TmemGrouped || k == 5) {
       slab = large_m_tmem_grouped_slab();
       need = large_m_tmem_grouped_workspace_bytes(L, M);
-    } else if (r == kInt8Grouped || k == 3 || over) {
+    } else if (r == kInt8Grouped || k == 3) {
       slab = large_m_grouped_slab();
       need = large_m_grouped_workspace_bytes(L, M);
     }
@@ -763,7 +751,7 @@ int forward_impl(const sacq_layer_t* L, const void* x_bf16, int64_t x_pitch, int
 // are whole segments of a token's row (the split-K kernel 256 bytes per warp, the staged warp-MMA kernels 16 to 96).
 bool stores_reach_host(const sacq_layer* L, int64_t M) {
   const int k = pick_kernel(L, M);
-  return k == 2 || k == 3 || (k == 1 && (small_m_hands_over(L, M) || small_m_staged_warps(L, M) > 0));
+  return k == 2 || k == 3 || (k == 1 && small_m_staged_warps(L, M) > 0);
 }
 }  // namespace
 
