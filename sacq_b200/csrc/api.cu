@@ -63,8 +63,9 @@ int64_t small_m_slab_rows(const sacq_layer* L) {
   return chunks * 16;
 }
 
-// Rows from which the grouped tensor-core kernel beats the index-unpacking warp-MMA kernel
-// (which walks the weights once per 16-token chunk).
+// Rows from which the grouped split-K kernel takes over from the index-unpacking warp-MMA kernel, which walks the
+// weights once per 16-token chunk (quantizer + GEMM, d = 4, 10-bit, group 64, the two kernels with exact weights:
+// 2048x6144 22.8 / 11.7 us at 32 rows; 1024x1024 7.5 / 6.8 and 6144x1536 35 / 13.8 at 48).
 int64_t grouped_min_m(const sacq_layer* L) {
   if (L->d.out_features >= 32 * (int64_t)L->num_sms) return 17;
   return 48;
@@ -188,13 +189,14 @@ SACQ_API int sacq_layer_create(const sacq_layer_desc* desc, sacq_layer_t** out_l
   const int64_t count = (int64_t)L->cb_entries * d.vector_dim;
   cudaError_t e = cudaMalloc(&L->cb_f16, (size_t)count * sizeof(__half));
   if (e == cudaSuccess) e = cudaMalloc(&L->cb_hilo, (size_t)count * 2);
+  if (e == cudaSuccess) e = cudaMalloc(&L->row_mul, (size_t)(d.out_features > 0 ? d.out_features : 1) * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc(&L->d_status, sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(L->d_status, 0, sizeof(int));
   if (e != cudaSuccess) {
     sacq_layer_destroy(L);
     return cuda_fail(e, "allocating derived codebook tables");
   }
-  L->resident_bytes = count * 4 + (int64_t)sizeof(int);
+  L->resident_bytes = count * 4 + d.out_features * (int64_t)sizeof(float) + (int64_t)sizeof(int);
   const int rc = launch_build_tables(L, nullptr);
   if (rc != SACQ_OK) {
     sacq_layer_destroy(L);
@@ -211,6 +213,7 @@ SACQ_API int sacq_layer_destroy(sacq_layer_t* L) {
   split_k_release(L);
   if (L->cb_f16) cudaFree(L->cb_f16);
   if (L->cb_hilo) cudaFree(L->cb_hilo);
+  if (L->row_mul) cudaFree(L->row_mul);
   if (L->d_status) cudaFree(L->d_status);
   delete L;
   return SACQ_OK;
@@ -360,7 +363,7 @@ int linear_a8_impl(const sacq_layer_t* L, const void* q, const float* scale, int
                                          workspace_bytes - kCounterBytes, s, residual, ldr, form, bc,
                                          L->force_kernel >= 13 ? L->force_kernel - 12 : 0);
     return launch_large_m_grouped(L, q, scale, M, y_out, ldy, static_cast<uint8_t*>(workspace) + kCounterBytes,
-                                  workspace_bytes - kCounterBytes, s, residual, ldr, form, bc);
+                                  workspace_bytes - kCounterBytes, s, residual, ldr, form, large_m_grouped_exact(L, M, false), bc);
   }
   const int64_t slab = small_m_slab_rows(L);
   for (int64_t m0 = 0; m0 < M; m0 += slab) {
@@ -433,7 +436,7 @@ int linear_a8i_impl(const sacq_layer_t* L, const void* q, const float* scale, in
                ? launch_large_m_tmem_grouped(L, q, scale, M, y_out, ldy, static_cast<uint8_t*>(workspace) + kCounterBytes,
                                              workspace_bytes - kCounterBytes, s, nullptr, 0, form)
                : launch_large_m_grouped(L, q, scale, M, y_out, ldy, static_cast<uint8_t*>(workspace) + kCounterBytes,
-                                        workspace_bytes - kCounterBytes, s, nullptr, 0, form);
+                                        workspace_bytes - kCounterBytes, s, nullptr, 0, form, large_m_grouped_exact(L, M, true));
   }
   if (!small_m_supported(L)) return set_error(SACQ_ERR_UNSUPPORTED, "no kernel can run this layer geometry");
   sacq_layer view = *L;

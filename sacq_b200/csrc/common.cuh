@@ -38,6 +38,7 @@ struct sacq_layer {
   int cb_exp_shift;          // power-of-two normalisation folded back in the epilogue
   int cb8_exp_shift;
   int sc_exp_shift;          // max |scale| * 2^sc_exp_shift lies in [0.5, 1) (grouped tensor-core kernel)
+  float* row_mul;            // [N] power of two: 1 / what brings the row's largest scale into [2^11, 2^12)
   int* d_status;             // device status word, 0 = ok
   int64_t resident_bytes;
   sacq::LargeMPlan* large_plan;
@@ -127,9 +128,11 @@ enum ActForm { kActE4M3 = 0, kActInt8 = 1, kActHalf = 2 };
 
 bool large_m_grouped_supported(const sacq_layer* L);
 int64_t large_m_grouped_workspace_bytes(const sacq_layer* L, int64_t M);
+// exact: the weights as two fp16 numbers, not rounded (large_m_grouped_exact: whether a call needs that).
+bool large_m_grouped_exact(const sacq_layer* L, int64_t M, bool int8);
 int launch_large_m_grouped(const sacq_layer* L, const void* q, const float* scale, int64_t M, void* y, int64_t ldy,
-                           void* ws, int64_t ws_bytes, cudaStream_t s, const void* residual = nullptr,
-                           int64_t ldr = 0, ActForm form = kActE4M3, const BcastDst* bc = nullptr);
+                           void* ws, int64_t ws_bytes, cudaStream_t s, const void* residual, int64_t ldr, ActForm form,
+                           bool exact, const BcastDst* bc = nullptr);
 int64_t large_m_grouped_slab(void);
 
 int launch_large_m_grouped_multi(const sacq_layer* const* layers, int n, const void* q, const float* scale, int64_t M,

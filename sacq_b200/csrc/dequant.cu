@@ -275,6 +275,24 @@ __global__ void index_max_kernel(const uint32_t* __restrict__ words, int64_t cou
   if ((threadIdx.x & 31) == 0) atomicMax(out, m);
 }
 
+// row_mul[n] = 2^-e with 2^e the power of two that brings the row's largest finite |scale| into [2^11, 2^12) (as far as
+// 2^e and 2^-e are normal numbers).
+__global__ void __launch_bounds__(256) row_mul_kernel(const uint16_t* __restrict__ scales, int64_t N, int num_groups,
+                                                      float* __restrict__ row_mul) {
+  const int64_t n = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (n >= N) return;
+  const int lane = threadIdx.x & 31;
+  uint32_t m = 0;
+  for (int g = lane; g < num_groups; g += 32) {
+    const uint32_t a = __ldg(scales + n * num_groups + g) & 0x7fffu;
+    if (a < 0x7f80u) m = max(m, a);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+  const int e = max(-126, min(126, 138 - (int)(m >> 7)));   // the scale is below 2^(exponent - 126)
+  if (lane == 0) row_mul[n] = __uint_as_float((uint32_t)(127 - e) << 23);
+}
+
 // cb_f16[i] = fp16(c * 2^e16); cb_hilo[c][0][j] = e4m3(c * 2^e8), cb_hilo[c][1][j] = e4m3(c*2^e8 - hi)
 __global__ void build_tables_kernel(const uint16_t* __restrict__ cb, int64_t C, int d, float mul16, float mul8,
                                     __half* __restrict__ cb_f16, uint8_t* __restrict__ cb_hilo) {
@@ -503,6 +521,12 @@ int launch_build_tables(sacq_layer* L, cudaStream_t s) {
       ldexpf(1.f, L->cb8_exp_shift), L->cb_f16, L->cb_hilo);
   count_launch();
   SACQ_CUDA_TRY(cudaGetLastError());
+  if (d.out_features > 0) {
+    row_mul_kernel<<<(unsigned)((d.out_features + 7) / 8), 256, 0, s>>>(static_cast<const uint16_t*>(d.scales), d.out_features,
+                                                                        (int)L->num_groups, L->row_mul);
+    count_launch();
+    SACQ_CUDA_TRY(cudaGetLastError());
+  }
   SACQ_CUDA_TRY(cudaStreamSynchronize(s));
   return SACQ_OK;
 }

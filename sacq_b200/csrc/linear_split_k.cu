@@ -16,7 +16,9 @@
 //                   codeword gathers -> tcgen05.st.  kSplitHiLo: the e4m3 high and low halves of the
 //                   codewords against e4m3 activations (kind::f8f6f4), one scale per row in the epilogue.
 //                   kSplitHalf: fp16(codeword x group scale) against activations widened to fp16
-//                   (kind::f16): grouped scales, and INT8 activations on any layer.  kSplitInt8 / kSplitFp8:
+//                   (kind::f16): grouped scales, and INT8 activations on any layer.  kSplitHalf2: that product
+//                   as two fp16 operands, h = fp16(c s) and fma(c, s, -h), which together are exact; for the
+//                   token counts and layers whose other kernel multiplies exact weights.  kSplitInt8 / kSplitFp8:
 //                   the 8-bit weight bytes of the two recipes, made here instead of in a pass of their own
 //                   over a 1-byte copy of the weights;
 //   * reduction     every CTA puts its fp32 partial sums into its own shared memory, [token][row]; after a
@@ -50,17 +52,19 @@ constexpr int kStageK = 128;          // k per weight stage
 constexpr int kMaxAct = 6;            // activation tiles in flight (128 bytes of every token each)
 constexpr int kMaxW = 4;              // weight stages in tensor memory
 constexpr int kSliceBytes = kRows * 16;
+__host__ __device__ constexpr int w_cols(int mode) { return mode == kSplitHalf2 ? 128 : mode >= kSplitInt8 ? 32 : 64; }
 constexpr float kHalfPreScale = 4096.f;   // keeps fp16(codeword x scale) far from the subnormals
 
 struct SplitLayer {
-  const uint8_t* cb;            // kSplitHiLo: e4m3 [C][2][D]; kSplitHalf: fp16 [C][D]; recipes: bf16 [C][D]
+  const uint8_t* cb;            // kSplitHiLo: e4m3 [C][2][D]; kSplitHalf, kSplitHalf2: fp16 [C][D]; recipes: bf16 [C][D]
   const uint16_t* scales;       // bf16 [N, num_groups]
   const uint16_t* bias;         // bf16 [N] or null
   uint16_t* y;                  // bf16 [M, ldy]
   int64_t ldy;
   int* status;
   int N;
-  float scale_mul;              // kSplitHalf: power of two applied to every scale before it is rounded to fp16
+  float scale_mul;              // kSplitHalf: power of two that brings the scales into the middle of fp16's range
+  const float* row_mul;         // kSplitHalf2: [N], the row's power of two (sacq_layer)
   float out_mul;                // power of two that undoes the operands' scaling
 };
 
@@ -271,9 +275,9 @@ __global__ void __launch_bounds__(kCtaThreads, 1)
 split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ SplitParams p) {
   constexpr uint32_t kTmemCols = 512;
   constexpr int CW_BYTES = 2 * D;
-  constexpr bool F16 = MODE == kSplitHalf, RECIPE = MODE >= kSplitInt8, INT = MODE == kSplitInt8;
+  constexpr bool PAIR = MODE == kSplitHalf2, F16 = MODE == kSplitHalf || PAIR, RECIPE = MODE >= kSplitInt8, INT = MODE == kSplitInt8;
   constexpr int TILES = F16 ? 2 : 1;                  // activation tiles (128 bytes of every token) per weight stage
-  constexpr int W_COLS = RECIPE ? 32 : 64;            // TMEM columns of a weight stage
+  constexpr int W_COLS = w_cols(MODE);                // TMEM columns of a weight stage
   const int S = p.split;
   const int n0 = ((int)blockIdx.x / S) * kRows;
   const SplitLayer& lay = p.layer[blockIdx.z];
@@ -400,8 +404,8 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) {              // 32 bytes of every token per step
 #pragma unroll
-          for (int h = 0; h < (MODE == kSplitHiLo ? 2 : 1); ++h) {       // high and low halves of the codewords
-            const uint32_t a = w_col + (F16 ? (uint32_t)(sub * 32 + ks * 8) : (uint32_t)(h * 32 + ks * 8));
+          for (int h = 0; h < (MODE == kSplitHiLo || PAIR ? 2 : 1); ++h) {       // high and low halves of the weights
+            const uint32_t a = w_col + (F16 ? (uint32_t)(h * 64 + sub * 32 + ks * 8) : (uint32_t)(h * 32 + ks * 8));
             const uint32_t acc = (uint32_t)(((wi - begin) | sub | ks | h) != 0);
             const uint64_t adv = (uint64_t)(ks * 2);
             if (elect_one()) {
@@ -468,7 +472,10 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     // stage's tcgen05.st: the gathers, which bound the loop, then never wait for a store's latency.
     const RowWeights rw = row_weights<INT>(RECIPE ? __ldg(p.row_scale + min(n0 + row, lay.N - 1)) : 1.f);
     const __nv_bfloat162 shift2 = __halves2bfloat162(__ushort_as_bfloat16(p.shift), __ushort_as_bfloat16(p.shift));
-    auto expand = [&](int wi, uint32_t (&w)[16]) {
+    // kSplitHalf2: the codewords as they are, and the two 64-k tiles' scales; the products are made at the store.
+    const float row_mul = PAIR ? __ldg(lay.row_mul + min(n0 + row, lay.N - 1)) : 1.f;
+    const float scale_mul = PAIR ? 1.f / row_mul : lay.scale_mul;       // a power of two
+    auto expand = [&](int wi, uint32_t (&w)[16], __half2 (&sc2)[2]) {
       if constexpr (RECIPE) {
         // 32 weights of this thread's row, 16 at a time: bf16(bf16(c * s) + shift) divided by the row scale and
         // encoded (the arithmetic of decode_rows_kernel in dequant.cu)
@@ -499,7 +506,8 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         for (int sub = 0; sub < 2; ++sub) {
           if (wi * kStageK + sub * 64 >= grp_end) { ++grp; grp_end += p.group_size; }
           // scale x 2^e is a bf16 significand with a small exponent: exact in fp16
-          const __half2 s2 = __half2half2(__float2half_rn(bf16_bits_to_float(sc[row * sc_pitch + grp]) * lay.scale_mul));
+          const __half2 s2 = __half2half2(__float2half_rn(bf16_bits_to_float(sc[row * sc_pitch + grp]) * scale_mul));
+          sc2[sub] = s2;
           const int bit = (((kb0 + wi) * kStageK + sub * 64 + kpart * 16) / D) * bits - slice0 * 128;
           const uint64_t win = slice_window(rowidx, bit, IPT * bits);
 #pragma unroll
@@ -516,7 +524,7 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 #pragma unroll
             for (int e = 0; e < D / 2; ++e) {
               const __half2 h = __hmul2(*reinterpret_cast<const __half2*>(&c[e]), s2);
-              w[sub * 8 + j * (D / 2) + e] = *reinterpret_cast<const uint32_t*>(&h);
+              w[sub * 8 + j * (D / 2) + e] = PAIR ? c[e] : *reinterpret_cast<const uint32_t*>(&h);
             }
           }
         }
@@ -544,16 +552,33 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     int ws = 0;
     uint32_t w_parity = 1;
     uint32_t cur[16], nxt[16];
-    if (ok) expand(0, cur);
+    __half2 cur_s[2], nxt_s[2];
+    if (ok) expand(0, cur, cur_s);
     for (int wi = 0; wi < kbs && ok; ++wi) {
       ok = mbar_wait(bar(W_EMPTY + ws), w_parity, abort_flag, lay.status);
       if (!ok) break;
       tc_fence_after();                               // the MMAs that read this stage are complete
       // two quarters of the stage: high and low halves, or the two 64-k tiles
       const uint32_t w_addr = lane_addr + (uint32_t)(acc_cols + ws * W_COLS + kpart * 8);
-      tmem_st_32x8(w_addr, reinterpret_cast<const uint32_t (&)[8]>(cur[0]));
-      if constexpr (!RECIPE) tmem_st_32x8(w_addr + 32u, reinterpret_cast<const uint32_t (&)[8]>(cur[8]));
-      if (wi + 1 < kbs) expand(wi + 1, nxt);
+      if constexpr (PAIR) {
+#pragma unroll
+        for (int sub = 0; sub < 2; ++sub) {
+          uint32_t hi[8], lo[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const __half2 c = *reinterpret_cast<const __half2*>(&cur[sub * 8 + j]);
+            const __half2 h = __hmul2_rn(c, cur_s[sub]), l = __hfma2(c, cur_s[sub], __hneg2(h));
+            hi[j] = *reinterpret_cast<const uint32_t*>(&h);
+            lo[j] = *reinterpret_cast<const uint32_t*>(&l);
+          }
+          tmem_st_32x8(w_addr + (uint32_t)(sub * 32), hi);
+          tmem_st_32x8(w_addr + (uint32_t)(64 + sub * 32), lo);
+        }
+      } else {
+        tmem_st_32x8(w_addr, reinterpret_cast<const uint32_t (&)[8]>(cur[0]));
+        if constexpr (!RECIPE) tmem_st_32x8(w_addr + 32u, reinterpret_cast<const uint32_t (&)[8]>(cur[8]));
+      }
+      if (wi + 1 < kbs) expand(wi + 1, nxt, nxt_s);
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
@@ -561,6 +586,10 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       if (++ws == w_stages) { ws = 0; w_parity ^= 1; }
 #pragma unroll
       for (int j = 0; j < (RECIPE ? 8 : 16); ++j) cur[j] = nxt[j];
+      if constexpr (PAIR) {
+        cur_s[0] = nxt_s[0];
+        cur_s[1] = nxt_s[1];
+      }
     }
     if (et == 0) SACQ_SPT(4);
     if (ok) ok = mbar_wait(bar(ACC_FULL), 0, abort_flag, lay.status);
@@ -573,6 +602,7 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     // [token][row] fp32, in the place of everything the main loop is done with (its last MMA has completed, so
     // every stage has been written and read); a warp writes 128 consecutive bytes per token
     const int quarter = warp & 3, row = quarter * 32 + lane, kpart = (warp - 2) >> 2;
+    const float row_mul = PAIR ? __ldg(lay.row_mul + min(n0 + row, lay.N - 1)) : 1.f;
     tc_fence_after();
     for (int c0 = kpart * 16; c0 < tok; c0 += 64) {
       const uint32_t at = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0;
@@ -588,7 +618,7 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       }
       uint32_t* dst = reinterpret_cast<uint32_t*>(sm) + c0 * kRows + row;
 #pragma unroll
-      for (int j = 0; j < 16; ++j) dst[j * kRows] = r[j];
+      for (int j = 0; j < 16; ++j) dst[j * kRows] = PAIR ? __float_as_uint(__uint_as_float(r[j]) * row_mul) : r[j];
     }
     tc_fence_before();
   }
@@ -659,6 +689,8 @@ int slice_map(sacq_layer* L, int slices, CUtensorMap* out) {
   return SACQ_OK;
 }
 
+bool is_f16(SplitMode mode) { return mode == kSplitHalf || mode == kSplitHalf2; }
+
 size_t split_smem(const SplitLayout& l) {
   const size_t need = l.total + 1024;
   return need < 116 * 1024 ? 116 * 1024 : need;       // two CTAs (each takes all 512 TMEM columns) never share an SM
@@ -701,6 +733,7 @@ cudaError_t launch_mode(SplitMode mode, const CUtensorMap& ta, const SplitParams
   switch (mode) {
     case kSplitHiLo: return launch_kernel<D, kSplitHiLo, CB_SMEM>(ta, p, grid, smem, s);
     case kSplitHalf: return launch_kernel<D, kSplitHalf, CB_SMEM>(ta, p, grid, smem, s);
+    case kSplitHalf2: return launch_kernel<D, kSplitHalf2, CB_SMEM>(ta, p, grid, smem, s);
     case kSplitInt8: return launch_kernel<D, kSplitInt8, CB_SMEM>(ta, p, grid, smem, s);
     default: return launch_kernel<D, kSplitFp8, CB_SMEM>(ta, p, grid, smem, s);
   }
@@ -740,7 +773,7 @@ int slices_for(int64_t K) { return K < 1024 ? 1 : K < 4096 ? 2 : K < 8192 ? 4 : 
 bool split_fits(const sacq_layer* L, SplitMode mode, SplitChoice* c) {
   const int cb_bytes = codebook_smem(L), groups = mode == kSplitHiLo ? 0 : 1;
   slice_extent(L, c->split, &c->max_slices, &c->max_groups);
-  const int tiles = ((int)(L->d.in_features / kStageK) + c->split - 1) / c->split * (mode == kSplitHalf ? 2 : 1);
+  const int tiles = ((int)(L->d.in_features / kStageK) + c->split - 1) / c->split * (is_f16(mode) ? 2 : 1);
   const size_t most = (cb_bytes > 0 ? 227 : 164) * 1024;
   auto bytes = [&](int stages) {
     return split_smem(split_layout(c->tok, c->split, stages, c->max_slices, groups * c->max_groups, cb_bytes));
@@ -755,7 +788,8 @@ bool split_fits(const sacq_layer* L, SplitMode mode, SplitChoice* c) {
 double split_cta_us(int vector_dim, SplitMode mode, bool cb_smem, int tok, int kbs, int split) {
   double stage = mode >= kSplitInt8 ? 0.75 : vector_dim == 8 ? 0.48 : 0.6;
   if (!cb_smem) stage = 8.0 / vector_dim;             // gathers from L2
-  if (0.002 * tok > stage) stage = 0.002 * tok;
+  const double mma = (mode == kSplitHalf2 ? 0.0042 : 0.002) * tok;
+  if (mma > stage) stage = mma;
   return 2.5 + kbs * stage + 0.015 * tok + (split > 1 ? 0.8 : 0.0);
 }
 
@@ -766,13 +800,14 @@ bool split_k_choose(const sacq_layer* L, int64_t M, SplitMode mode, SplitChoice*
   if (d.vector_dim != 8 && d.vector_dim != 4) return false;
   if (d.index_bits > 16 || !L->rows_16b_aligned || d.in_features % kStageK != 0) return false;
   if (mode < kSplitInt8 && has_shift(L)) return false;
-  if (mode == kSplitHiLo ? L->num_groups != 1 : d.group_size % (mode == kSplitHalf ? 64 : 16) != 0) return false;
+  if (mode == kSplitHiLo ? L->num_groups != 1 : d.group_size % (is_f16(mode) ? 64 : 16) != 0) return false;
   // the recipes read the codebook as it came, which is not padded to whole 16-byte units
   if (mode >= kSplitInt8 && d.codebook_size * d.vector_dim % 8 != 0) return false;
   if ((int64_t)L->cb_entries * d.vector_dim * 2 % 16 != 0 || M <= 0 || M > (1 << 20)) return false;
   const int nkb = (int)(d.in_features / kStageK);
   const int64_t row_tiles = (d.out_features + kRows - 1) / kRows;
   const int slices = slices_for(d.in_features);
+  const int most = mode == kSplitHalf2 ? 512 - 2 * w_cols(mode) : kMaxTok;       // accumulator columns beside two weight stages
   *out = SplitChoice();
   const int least = (int)((M + kMaxTok - 1) / kMaxTok);
   for (int split = 1; split <= slices; split *= 2) {
@@ -781,7 +816,7 @@ bool split_k_choose(const sacq_layer* L, int64_t M, SplitMode mode, SplitChoice*
     for (int tiles = least; tiles <= 3 * least + 1; ++tiles) {
       int tok = (int)(((M + tiles - 1) / tiles + 15) & ~(int64_t)15);
       if (tok > 256) tok = (tok + 31) & ~31;
-      if (slices / split > 4 || tok * (slices / split) > kMaxTok) continue;
+      if (slices / split > 4 || tok * (slices / split) > most) continue;
       SplitChoice c;
       c.tok = tok;
       c.tiles = (int)((M + tok - 1) / tok);
@@ -829,7 +864,7 @@ int launch_split_k(const sacq_layer* const* layers, int n, const void* act, cons
   SplitParams p;
   memset(&p, 0, sizeof(p));
   CUtensorMap ta;
-  const uint64_t act_row = (uint64_t)d0.in_features * (mode == kSplitHalf ? 2 : 1);
+  const uint64_t act_row = (uint64_t)d0.in_features * (is_f16(mode) ? 2 : 1);
   int rc = encode_bytes_2d(&ta, act, act_row, (uint64_t)M, act_row, 128u, (uint32_t)(c.tok <= 256 ? c.tok : c.tok / 2),
                            CU_TENSOR_MAP_SWIZZLE_128B);
   if (rc != SACQ_OK) return rc;
@@ -840,7 +875,7 @@ int launch_split_k(const sacq_layer* const* layers, int n, const void* act, cons
     if (rc != SACQ_OK) return rc;
     SplitLayer& q = p.layer[l];
     q.cb = mode == kSplitHiLo ? L->cb_hilo
-           : mode == kSplitHalf ? reinterpret_cast<const uint8_t*>(L->cb_f16) : static_cast<const uint8_t*>(L->d.codebook);
+           : is_f16(mode) ? reinterpret_cast<const uint8_t*>(L->cb_f16) : static_cast<const uint8_t*>(L->d.codebook);
     q.scales = static_cast<const uint16_t*>(L->d.scales);
     q.bias = static_cast<const uint16_t*>(L->d.bias);
     q.y = static_cast<uint16_t*>(ys[l]);
@@ -848,7 +883,10 @@ int launch_split_k(const sacq_layer* const* layers, int n, const void* act, cons
     q.status = L->d_status;
     q.N = (int)L->d.out_features;
     q.scale_mul = ldexpf(kHalfPreScale, L->sc_exp_shift);
-    q.out_mul = mode == kSplitHalf ? ldexpf(1.f / kHalfPreScale, -(L->cb_exp_shift + L->sc_exp_shift)) : ldexpf(1.f, -L->cb8_exp_shift);
+    q.row_mul = L->row_mul;
+    q.out_mul = mode == kSplitHalf    ? ldexpf(1.f / kHalfPreScale, -(L->cb_exp_shift + L->sc_exp_shift))
+                : mode == kSplitHalf2 ? ldexpf(1.f, -L->cb_exp_shift)
+                                      : ldexpf(1.f, -L->cb8_exp_shift);
     if (L->d.out_features > widest) widest = L->d.out_features;
   }
   p.act_scale = scale;

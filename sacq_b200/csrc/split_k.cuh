@@ -13,8 +13,9 @@ constexpr int kSplitMaxLayers = 4;    // sibling layers of one launch
 enum SplitMode {
   kSplitHiLo = 0,   // e4m3 high and low halves of the codewords, e4m3 activations; one scale per row
   kSplitHalf = 1,   // fp16(codeword x scale), activations widened to fp16: grouped scales, INT8 activations
-  kSplitInt8 = 2,   // the INT8 recipe's weight bytes, int8 activations, int32 sums
-  kSplitFp8 = 3     // the FP8 recipe's weight bytes, e4m3 activations
+  kSplitHalf2 = 2,  // the same product as two fp16 numbers, exactly: its 16 significant bits are 11 and 5
+  kSplitInt8 = 3,   // the INT8 recipe's weight bytes, int8 activations, int32 sums
+  kSplitFp8 = 4     // the FP8 recipe's weight bytes, e4m3 activations
 };
 
 // How one call is cut up: token tiles of `tok` tokens, clusters of `split` CTAs with `parts` slices of K each.
@@ -30,7 +31,7 @@ bool split_k_choose(const sacq_layer* L, int64_t M, SplitMode mode, SplitChoice*
 bool split_k_choose_multi(const sacq_layer* const* layers, int n, int64_t M, SplitMode mode, SplitChoice* out);
 
 // n layers of one geometry (n = 1: the plain launch) on one set of activations: bytes [M, K], or for kSplitHalf
-// the activations already widened to fp16 [M, K].  row_scale: the recipes' per-row weight scales [N] (n = 1).
+// and kSplitHalf2 the activations already widened to fp16 [M, K].  row_scale: the recipes' per-row weight scales [N] (n = 1).
 int launch_split_k(const sacq_layer* const* layers, int n, const void* act, const float* scale, int64_t M, void* const* ys,
                    const int64_t* ldys, SplitMode mode, const SplitChoice& c, cudaStream_t s, const void* residual = nullptr,
                    int64_t ldr = 0, const BcastDst* bc = nullptr, const float* row_scale = nullptr);

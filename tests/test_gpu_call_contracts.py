@@ -37,3 +37,45 @@ def test_a_forced_kernel_is_the_one_that_runs(N, K, M):
     mod.set_kernel("auto")
     assert mod.kernel_for(M) == "small" and torch.equal(mod.linear_a8(q, s), outs["small"])
     assert torch.equal(mod(_x(M, K)), outs["small"])
+
+
+def _exact(mod, q, s):
+    """Float64 sums of codeword x scale (not rounded to bf16 as the reconstruction is), rounded once to bf16."""
+    bits, n, k, g = mod.index_bits, mod.out_features, mod.in_features, mod.group_size
+    planes = (mod.packed_indices[: mod._packed_bytes].unsqueeze(1) >> torch.arange(8, device="cuda", dtype=torch.uint8)) & 1
+    fields = planes.reshape(-1)[: n * k // mod.vector_dim * bits].reshape(-1, bits).long()
+    w = mod.codebook.double()[(fields << torch.arange(bits, device="cuda")).sum(1)].reshape(n, k // g, g) * mod.scales.double().unsqueeze(-1)
+    y = q.double() @ w.reshape(n, k).t() * s.reshape(-1, 1).double()
+    return (y if mod.bias is None else y + mod.bias.double()).to(torch.bfloat16)
+
+
+@pytest.mark.parametrize("N,K,d,C,G", [
+    (6144, 1024, 4, 1024, 64), (1000, 1024, 4, 81, 64), (129, 8192, 4, 64, 64), (300, 1536, 8, 4096, 128),   # grouped scales
+    (1024, 2048, 8, 4096, None), (264, 1024, 4, 700, None), (520, 2048, 8, 65536, None)])                     # one per row
+def test_few_tokens_multiply_exact_weights(N, K, d, C, G):
+    """Whatever kernel takes a call of fewer than 96 tokens on grouped scales (48 on layers of 2,048 outputs, 33 on the widest),
+    or of fewer than 48 on INT8 activations (any number, where the codebook does not fit shared memory), its weights are
+    codeword x scale with all 16 significant bits.
+    An fp32 sum of up to 16 x 512 products is within about 2^-19 of the result, so about one output in 2^10 lies close
+    enough to the middle between two bf16 values to be rounded the other way; weights of 11 bits put every tenth there."""
+    from sacq_b200 import quantize_rows
+    mod = _layer(N, K, d, C, G, bias=True)
+    # rows and groups of very different scale: a row's own largest scale is what its operands are brought to
+    mod.scales *= torch.logspace(-9, 3, N, base=2.0, device="cuda").to(torch.bfloat16).unsqueeze(1)
+    if G is not None:
+        mod.scales[:, ::3] *= 2.0 ** -5
+    from sacq_b200 import PrecomputedPackedVectorCodebookLinear
+    mod = PrecomputedPackedVectorCodebookLinear(
+        {"codebook": mod.codebook, "scales": mod.scales, "in_features": K, "out_features": N, "group_size": G or K, "vector_dim": d,
+         "packed_indices": mod.packed_indices[: mod._packed_bytes], "index_bits": mod.index_bits, "index_shape": mod.index_shape},
+        mod.bias, "cuda")
+    x = _x(300, K)
+    for mode, call, sizes in (("fp8_e4m3fn", mod.linear_a8, (1, 17, 32) + ((33, 47, 48, 64, 95) if N < 2048 else ()) if G is not None else (1, 33)),
+                              ("int8_symmetric", mod.linear_a8i, (1, 4, 16, 17, 33, 47) + ((48, 95, 300) if C > 4096 else ()))):
+        q, s = quantize_rows(x, mode)
+        for M in sizes:
+            y, want = call(q[:M].contiguous(), s[:M].contiguous()), _exact(mod, q[:M], s[:M])
+            assert float((y != want).float().mean()) <= 2.0 ** -8, (mode, M)
+            # one step of bf16 is up to 2^-7 of the value: 2^-8 of the outputs off by one are 2^-11 of the norm
+            assert float((y.double() - want.double()).norm() / want.double().norm()) <= 2.0 ** -11, (mode, M)
+    assert mod.device_status() == 0
