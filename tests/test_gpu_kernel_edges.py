@@ -1,7 +1,6 @@
 """The tensor-core kernels, quantizers and weight encoders at the sizes where a tile, a slice of K, a remainder or a
 rule of the dispatch ends.  Oracle: the layer's own reconstruction (bit-exact against the CPU oracle elsewhere) in
-float64 or exact integer arithmetic, and torch's IEEE division for everything that is bytes.  (Collected last: an earlier
-test compares rows of an uninitialised buffer, whose bytes are what the tests before it left in the allocator.)"""
+float64 or exact integer arithmetic, and torch's IEEE division for everything that is bytes."""
 import pytest
 import torch
 
