@@ -87,6 +87,14 @@ bool split_wins(const sacq_layer* L, int64_t M) {
   return (M > 16 && (L->d.out_features >= 4096 || work >= (8 << 20))) || M > 32;
 }
 
+// Whether the persistent kernel takes a call that shared memory leaves the split-K kernel narrow tiles for: if it is
+// modelled to be faster.
+bool large_m_cedes(const sacq_layer* L, int64_t M) {
+  SplitChoice c;
+  return !split_k_tiles_fit(L, M, kSplitHiLo) && large_m_tmem_supported(L) &&
+         (!split_k_choose(L, M, kSplitHiLo, &c) || large_m_tmem_us(L, M) < c.us);
+}
+
 int pick_kernel(const sacq_layer* L, int64_t M) {
   if (L->force_kernel == 7) return large_m_grouped_supported(L) ? 3 : SACQ_ERR_UNSUPPORTED;
   if (L->force_kernel >= 12) return large_m_tmem_grouped_supported(L) ? 5 : SACQ_ERR_UNSUPPORTED;
@@ -102,11 +110,14 @@ int pick_kernel(const sacq_layer* L, int64_t M) {
   // 6144x2048 15.4 / 11.5, 2048x6144 15.5 / 8.9; at 33: 1024x1024 7.3 / 5.7, 2048x2048 9.2 / 8.8, 4096x1024
   // 9.5 / 9.2, 2048x1024 even.
   if (large_m_supported(L)) {
-    if (split_wins(L, M)) return 2;
+    if (split_wins(L, M)) return large_m_cedes(L, M) ? 4 : 2;
+  } else if (large_m_tmem_supported(L)) {              // a layer too deep for the split-K kernel
+    if (M >= (L->d.out_features >= 32 * (int64_t)L->num_sms ? 17 : 49)) return 4;
   } else if (large_m_tmem_grouped_supported(L) && M >= large_m_tmem_grouped_min_m(L)) {
     return 5;                                          // grouped scales, odd index widths: weights in tensor memory
-  } else if (M >= grouped_min_m(L) && large_m_grouped_supported(L)) {
-    return 3;                                          // ... K split over clusters
+  } else if (M >= grouped_min_m(L)) {
+    if (large_m_grouped_cedes(L, M, false)) return 5;
+    if (large_m_grouped_supported(L)) return 3;        // ... K split over clusters
   }
   return small_m_supported(L) ? 1 : SACQ_ERR_UNSUPPORTED;
 }
@@ -186,6 +197,7 @@ SACQ_API int sacq_layer_create(const sacq_layer_desc* desc, sacq_layer_t** out_l
   }
   L->num_sms = prop.multiProcessorCount;
   L->cb_entries = (d.codebook_size + 1) & ~1;
+  split_k_init(L);
   const int64_t count = (int64_t)L->cb_entries * d.vector_dim;
   cudaError_t e = cudaMalloc(&L->cb_f16, (size_t)count * sizeof(__half));
   if (e == cudaSuccess) e = cudaMalloc(&L->cb_hilo, (size_t)count * 2);
@@ -391,6 +403,7 @@ namespace {
 enum Int8Route { kInt8Small, kInt8Grouped, kInt8TmemGrouped };
 Int8Route int8_route(const sacq_layer* L, int64_t M) {
   if (large_m_tmem_grouped_supported(L) && M >= large_m_tmem_grouped_min_m(L)) return kInt8TmemGrouped;
+  if (large_m_grouped_cedes(L, M, true)) return kInt8TmemGrouped;
   if (!large_m_grouped_supported(L)) return kInt8Small;
   const bool warp_mma = small_m_int8_selector(L) == 5 && (split_k_codebook_in_smem(L) || L->d.out_features < 4096);
   const int64_t warp_mma_wins = !warp_mma ? 0 : L->d.out_features < 2048 && split_k_codebook_in_smem(L) ? 48 : 16;
@@ -498,7 +511,8 @@ bool recipe_in_one(const sacq_layer* L, const void* q, const float* act_scale, c
   const bool wide = L->d.out_features >= 4096 && L->d.in_features >= 2048;
   if (M > (!wide ? 32 : split_k_codebook_in_smem(L) ? 320 : 200) || reinterpret_cast<uintptr_t>(q) % 16 != 0 ||
       reinterpret_cast<uintptr_t>(L->d.codebook) % 16 != 0 ||
-      (mode == kSplitInt8 && L->d.in_features * 127 * 127 > 2147483647LL) || !split_k_choose(L, M, mode, &c))
+      (mode == kSplitInt8 && L->d.in_features * 127 * 127 > 2147483647LL) || !split_k_tiles_fit(L, M, mode) ||
+      !split_k_choose(L, M, mode, &c))
     return false;
   *rc = launch_split_k(&L, 1, q, act_scale, M, &y, &ldy, mode, c, s, nullptr, 0, nullptr, w_scale);
   return true;

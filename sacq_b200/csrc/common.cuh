@@ -40,6 +40,7 @@ struct sacq_layer {
   int sc_exp_shift;          // max |scale| * 2^sc_exp_shift lies in [0.5, 1) (grouped tensor-core kernel)
   float* row_mul;            // [N] power of two: 1 / what brings the row's largest scale into [2^11, 2^12)
   int* d_status;             // device status word, 0 = ok
+  int split_tok[5];          // per form of the split-K kernel (SplitMode): its widest token tile, 0 if it cannot run the layer
   int64_t resident_bytes;
   sacq::LargeMPlan* large_plan;
   sacq::SplitPlan* split_plan;
@@ -113,6 +114,7 @@ void large_m_release(sacq_layer* L);
 
 // Tensor-core kernel that keeps the expanded weights in tensor memory (linear_large_m_tmem.cu).
 bool large_m_tmem_supported(const sacq_layer* L);
+double large_m_tmem_us(const sacq_layer* L, int64_t M);          // modelled time
 int launch_large_m_tmem(const sacq_layer* L, const void* q, const float* scale, int64_t M, void* y, int64_t ldy,
                         cudaStream_t s, const void* residual = nullptr, int64_t ldr = 0, const BcastDst* bc = nullptr,
                         int nt_force = 0);
@@ -130,6 +132,7 @@ bool large_m_grouped_supported(const sacq_layer* L);
 int64_t large_m_grouped_workspace_bytes(const sacq_layer* L, int64_t M);
 // exact: the weights as two fp16 numbers, not rounded (large_m_grouped_exact: whether a call needs that).
 bool large_m_grouped_exact(const sacq_layer* L, int64_t M, bool int8);
+bool large_m_grouped_cedes(const sacq_layer* L, int64_t M, bool int8);
 int launch_large_m_grouped(const sacq_layer* L, const void* q, const float* scale, int64_t M, void* y, int64_t ldy,
                            void* ws, int64_t ws_bytes, cudaStream_t s, const void* residual, int64_t ldr, ActForm form,
                            bool exact, const BcastDst* bc = nullptr);
@@ -142,6 +145,7 @@ int launch_large_m_grouped_multi(const sacq_layer* const* layers, int n, const v
 bool large_m_tmem_grouped_supported(const sacq_layer* L);
 int64_t large_m_tmem_grouped_workspace_bytes(const sacq_layer* L, int64_t M);
 int64_t large_m_tmem_grouped_min_m(const sacq_layer* L);
+double large_m_tmem_grouped_us(const sacq_layer* L, int64_t M);
 int64_t large_m_tmem_grouped_slab(void);
 int launch_large_m_tmem_grouped(const sacq_layer* L, const void* q, const float* scale, int64_t M, void* y, int64_t ldy,
                                 void* ws, int64_t ws_bytes, cudaStream_t s, const void* residual = nullptr,

@@ -85,9 +85,7 @@ std::mutex g_plan_mutex;   // layers build their index tile map on first use, po
 bool large_m_supported(const sacq_layer* L) {
   const sacq_layer_desc& d = L->d;
   if (d.index_bits != 8 && d.index_bits != 12 && d.index_bits != 16) return false;
-  if (d.in_features % (2 * kBK) != 0) return false;
-  SplitChoice c;
-  return split_k_choose(L, 1, kSplitHiLo, &c);
+  return d.in_features % (2 * kBK) == 0 && L->split_tok[kSplitHiLo] > 0;
 }
 
 void large_m_release(sacq_layer* L) {
@@ -148,18 +146,19 @@ double plan_of(const sacq_layer* L, int64_t M, TileTime tile_us, int tok, tmemw:
 
 // 8,192 tokens of a 6,144-row layer, for instance, are 1,008 tiles of 384 and 48 of 128 on 148 SMs: 7 rounds, where a grid
 // of equal tiles takes 8.
-bool plan_tiles(const sacq_layer* L, int64_t M, TileTime tile_us, int tok_force, tmemw::TilePlan* p) {
+bool plan_tiles(const sacq_layer* L, int64_t M, TileTime tile_us, int tok_force, tmemw::TilePlan* p, double* us) {
   if (M / 32 + 1 > 0x7fffffff / ((L->d.out_features + tmemw::kRows) / tmemw::kRows)) return false;
   double best_us = 1e30;
   for (int t = tmemw::kMaxTok; t >= 32; t -= t > 256 ? 64 : 32) {
     if (tok_force > 0 && t != tok_force) continue;
     tmemw::TilePlan c;
-    const double us = plan_of(L, M, tile_us, t, &c);
-    if (us < best_us - 1e-9) {
-      best_us = us;
+    const double t_us = plan_of(L, M, tile_us, t, &c);
+    if (t_us < best_us - 1e-9) {
+      best_us = t_us;
       *p = c;
     }
   }
+  if (us != nullptr) *us = best_us;
   // one activation copy size for both kinds of tile
   auto part_of = [](int t) { return t / (t > 256 ? 2 : 1); };
   p->box = part_of(p->full > 0 ? p->tok : p->rem);
@@ -199,9 +198,20 @@ int launch_large_m(const sacq_layer* L, const void* q, const float* scale, int64
                    cudaStream_t s, const void* residual, int64_t ldr, const BcastDst* bc) {
   if (!large_m_supported(L)) return set_error(SACQ_ERR_UNSUPPORTED, "large-M kernel cannot run this layer geometry");
   if (M <= 0 || L->d.out_features == 0) return SACQ_OK;
-  SplitChoice c;
-  if (!split_k_choose(L, M, kSplitHiLo, &c)) return set_error(SACQ_ERR_UNSUPPORTED, "M=%lld too large", (long long)M);
-  return launch_split_k(&L, 1, q, scale, M, &y, &ldy, kSplitHiLo, c, s, residual, ldr, bc);
+  if (M > (1 << 30)) return set_error(SACQ_ERR_UNSUPPORTED, "M=%lld too large", (long long)M);
+  for (int64_t m0 = 0; m0 < M; m0 += kSplitMaxM) {
+    const int64_t rows = M - m0 < kSplitMaxM ? M - m0 : kSplitMaxM;
+    SplitChoice c;
+    if (!split_k_choose(L, rows, kSplitHiLo, &c)) return set_error(SACQ_ERR_UNSUPPORTED, "split-K kernel: no tile fits");
+    BcastDst slab{};
+    for (int i = 0; bc != nullptr && i < bc->n; ++i) slab.ptr[slab.n++] = static_cast<uint16_t*>(bc->ptr[i]) + m0 * ldy;
+    void* y_slab = static_cast<uint16_t*>(y) + m0 * ldy;
+    const int rc = launch_split_k(&L, 1, static_cast<const uint8_t*>(q) + m0 * L->d.in_features, scale + m0, rows, &y_slab,
+                                  &ldy, kSplitHiLo, c, s, residual ? static_cast<const uint16_t*>(residual) + m0 * ldr : nullptr,
+                                  ldr, bc ? &slab : nullptr);
+    if (rc != SACQ_OK) return rc;
+  }
+  return SACQ_OK;
 }
 
 // Several layers of one geometry on the same quantized activations as ONE launch.  Returns

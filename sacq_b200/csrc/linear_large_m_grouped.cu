@@ -41,9 +41,18 @@ bool large_m_grouped_exact(const sacq_layer* L, int64_t M, bool int8) {
   return M < (L->d.out_features >= 32 * (int64_t)L->num_sms ? 33 : L->d.out_features >= 2048 ? 48 : 96);
 }
 
-bool large_m_grouped_supported(const sacq_layer* L) {
+bool large_m_grouped_supported(const sacq_layer* L) { return L->d.index_bits >= 1 && L->split_tok[kSplitHalf] > 0; }
+
+// Whether the persistent kernel for grouped scales takes a call that shared memory leaves this one narrow tiles for, or none:
+// from where the weights need not be exact, if it is modelled to be faster by a margin (its model was fitted to shallower
+// layers: K = 28,672, 4,096 rows, d = 4, 11-bit, group 64 at 1,000 tokens: modelled 0.5 ms, measured 0.82).
+bool large_m_grouped_cedes(const sacq_layer* L, int64_t M, bool int8) {
+  const bool exact = large_m_grouped_exact(L, M, int8);
+  if (exact || split_k_tiles_fit(L, M, form_of(exact)) || !large_m_tmem_grouped_supported(L)) return false;
+  if (!large_m_grouped_supported(L)) return true;
+  const int64_t rows = M < kSlabTokens ? M : kSlabTokens;
   SplitChoice c;
-  return L->d.index_bits >= 1 && split_k_choose(L, 1, kSplitHalf, &c);
+  return !split_k_choose(L, rows, form_of(exact), &c) || 1.6 * large_m_tmem_grouped_us(L, M) < c.us * (double)M / (double)rows;
 }
 
 // Workspace behind the counter region: the fp16 activations of one token slab.

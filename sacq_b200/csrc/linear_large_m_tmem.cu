@@ -431,6 +431,12 @@ bool large_m_tmem_supported(const sacq_layer* L) {
   return pick_act_stages(L, kMaxTok) >= 2;
 }
 
+double large_m_tmem_us(const sacq_layer* L, int64_t M) {
+  TilePlan p;
+  double us;
+  return plan_tiles(L, M, tile_us, 0, &p, &us) ? us : 1e30;
+}
+
 int launch_large_m_tmem(const sacq_layer* L, const void* q, const float* scale, int64_t M, void* y, int64_t ldy,
                         cudaStream_t s, const void* residual, int64_t ldr, const BcastDst* bc, int nt_force) {
   const sacq_layer_desc& d = L->d;

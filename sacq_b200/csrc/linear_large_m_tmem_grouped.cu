@@ -454,6 +454,12 @@ int64_t large_m_tmem_grouped_min_m(const sacq_layer* L) {
   return L->d.out_features >= 5120 ? 448 : L->d.out_features >= 4096 ? 600 : 1025;
 }
 
+double large_m_tmem_grouped_us(const sacq_layer* L, int64_t M) {
+  TilePlan p;
+  double us;
+  return plan_tiles(L, M, g_tile_us, 0, &p, &us) ? us : 1e30;
+}
+
 // Workspace behind the counter region: the fp16 activations of one token slab.
 int64_t large_m_tmem_grouped_workspace_bytes(const sacq_layer* L, int64_t M) {
   const int64_t rows = M < kGSlabTokens ? M : kGSlabTokens;

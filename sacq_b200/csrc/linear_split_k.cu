@@ -793,9 +793,8 @@ double split_cta_us(int vector_dim, SplitMode mode, bool cb_smem, int tok, int k
   return 2.5 + kbs * stage + 0.015 * tok + (split > 1 ? 0.8 : 0.0);
 }
 
-}  // namespace
-
-bool split_k_choose(const sacq_layer* L, int64_t M, SplitMode mode, SplitChoice* out) {
+// What the kernel's index arithmetic needs of a layer.
+bool takes_layer(const sacq_layer* L, SplitMode mode) {
   const sacq_layer_desc& d = L->d;
   if (d.vector_dim != 8 && d.vector_dim != 4) return false;
   if (d.index_bits > 16 || !L->rows_16b_aligned || d.in_features % kStageK != 0) return false;
@@ -803,34 +802,75 @@ bool split_k_choose(const sacq_layer* L, int64_t M, SplitMode mode, SplitChoice*
   if (mode == kSplitHiLo ? L->num_groups != 1 : d.group_size % (is_f16(mode) ? 64 : 16) != 0) return false;
   // the recipes read the codebook as it came, which is not padded to whole 16-byte units
   if (mode >= kSplitInt8 && d.codebook_size * d.vector_dim % 8 != 0) return false;
-  if ((int64_t)L->cb_entries * d.vector_dim * 2 % 16 != 0 || M <= 0 || M > (1 << 20)) return false;
-  const int nkb = (int)(d.in_features / kStageK);
-  const int64_t row_tiles = (d.out_features + kRows - 1) / kRows;
-  const int slices = slices_for(d.in_features);
-  const int most = mode == kSplitHalf2 ? 512 - 2 * w_cols(mode) : kMaxTok;       // accumulator columns beside two weight stages
+  return (int64_t)L->cb_entries * d.vector_dim * 2 % 16 == 0;
+}
+
+// Accumulator columns beside two weight stages.
+int most_columns(SplitMode mode) { return mode == kSplitHalf2 ? 512 - 2 * w_cols(mode) : kMaxTok; }
+
+// Tokens of one of `tiles` equal tiles, in whole instructions: a multiple of 16, two of them above 256.
+int tile_width(int64_t M, int64_t tiles) {
+  const int64_t tok = ((M + tiles - 1) / tiles + 15) & ~(int64_t)15;
+  return (int)(tok > 256 ? (tok + 31) & ~(int64_t)31 : tok);
+}
+int least_tiles(int64_t M) { return (int)((M + kMaxTok - 1) / kMaxTok); }
+int most_tiles(int64_t M) { return 3 * least_tiles(M) + 1; }       // that the model is asked about
+
+SplitChoice cut_of(int64_t M, int tok, int split, int parts) {
+  SplitChoice c;
+  c.tok = tok;
+  c.tiles = (int)((M + tok - 1) / tok);
+  c.split = split;
+  c.parts = parts;
+  return c;
+}
+
+// Fills in what follows from a cut, its modelled time included; false if it does not fit.
+bool complete(const sacq_layer* L, SplitMode mode, SplitChoice* c) {
+  if (!split_fits(L, mode, c)) return false;
+  const int64_t row_tiles = (L->d.out_features + kRows - 1) / kRows;
+  const int kbs = ((int)(L->d.in_features / kStageK) + c->split - 1) / c->split;
+  const int at_once = active_clusters(c->split, L->num_sms);
+  const int64_t waves = (row_tiles * c->tiles + at_once - 1) / at_once;
+  // every CTA fetches the codebook through L2
+  const int64_t ctas = row_tiles * c->tiles * c->split, resident = waves * L->num_sms;
+  c->us = waves * split_cta_us(L->d.vector_dim, mode, codebook_smem(L) > 0, c->tok, kbs, c->split) +
+          0.01 * (double)(ctas < resident ? ctas : resident);
+  return true;
+}
+
+}  // namespace
+
+void split_k_init(sacq_layer* L) {
+  for (int mode = kSplitHiLo; mode <= kSplitFp8; ++mode) {
+    const SplitMode m = (SplitMode)mode;
+    int tok = takes_layer(L, m) ? most_columns(m) : 0;
+    for (; tok > 0; tok -= tok > 256 ? 32 : 16) {
+      SplitChoice c = cut_of(tok, tok, slices_for(L->d.in_features), 1);
+      if (split_fits(L, m, &c)) break;
+    }
+    L->split_tok[mode] = tok > 0 ? tok : 0;
+  }
+}
+
+bool split_k_tiles_fit(const sacq_layer* L, int64_t M, SplitMode mode) {
+  return L->split_tok[mode] == most_columns(mode) || M <= L->split_tok[mode];
+}
+
+bool split_k_choose(const sacq_layer* L, int64_t M, SplitMode mode, SplitChoice* out) {
   *out = SplitChoice();
-  const int least = (int)((M + kMaxTok - 1) / kMaxTok);
+  if (L->split_tok[mode] == 0 || M <= 0 || M > kSplitMaxM) return false;
+  const int slices = slices_for(L->d.in_features);
   for (int split = 1; split <= slices; split *= 2) {
-    const int kbs = (nkb + split - 1) / split;
-    const int at_once = active_clusters(split, L->num_sms);
-    for (int tiles = least; tiles <= 3 * least + 1; ++tiles) {
-      int tok = (int)(((M + tiles - 1) / tiles + 15) & ~(int64_t)15);
-      if (tok > 256) tok = (tok + 31) & ~31;
-      if (slices / split > 4 || tok * (slices / split) > most) continue;
-      SplitChoice c;
-      c.tok = tok;
-      c.tiles = (int)((M + tok - 1) / tok);
-      c.split = split;
-      c.parts = slices / split;
-      if (!split_fits(L, mode, &c)) continue;
-      const int64_t waves = (row_tiles * c.tiles + at_once - 1) / at_once;
-      // every CTA fetches the codebook through L2
-      const int64_t ctas = row_tiles * c.tiles * split, resident = waves * L->num_sms;
-      c.us = waves * split_cta_us(d.vector_dim, mode, codebook_smem(L) > 0, tok, kbs, split) + 0.01 * (double)(ctas < resident ? ctas : resident);
-      if (c.us < out->us) *out = c;
+    const int parts = slices / split;
+    for (int tiles = least_tiles(M); parts <= 4 && tiles <= most_tiles(M); ++tiles) {
+      SplitChoice c = cut_of(M, tile_width(M, tiles), split, parts);
+      if (c.tok * parts <= most_columns(mode) && complete(L, mode, &c) && c.us < out->us) *out = c;
     }
   }
-  return out->tok != 0;
+  if (out->tok != 0) return true;
+  *out = cut_of(M, L->split_tok[mode], slices, 1);    // narrower tiles than that: as wide as they fit
+  return complete(L, mode, out);
 }
 
 bool split_k_codebook_in_smem(const sacq_layer* L) { return codebook_smem(L) > 0; }

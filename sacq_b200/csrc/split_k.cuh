@@ -24,7 +24,14 @@ struct SplitChoice {
   double us = 1e30;             // modelled time
 };
 
-// The best cut for M tokens; false if the kernel cannot run the layer in that form.
+// Fills sacq_layer::split_tok, once, when the layer is made.
+void split_k_init(sacq_layer* L);
+// Whether shared memory leaves the call the tiles that the model wants.  A CTA holds the packed indices of its whole slice
+// of K, so deep layers have room for narrow tiles only, each of which expands the weights again.
+bool split_k_tiles_fit(const sacq_layer* L, int64_t M, SplitMode mode);
+
+// The best cut for M tokens (at most kSplitMaxM); false if the kernel cannot run the layer in that form.
+constexpr int64_t kSplitMaxM = 1 << 19;
 bool split_k_choose(const sacq_layer* L, int64_t M, SplitMode mode, SplitChoice* out);
 
 // The same for several layers in one launch; false if they are not of one geometry.

@@ -310,7 +310,7 @@ __device__ __forceinline__ void tile_epilogue(const TmemOut& o, const CUtensorMa
 // Modelled time (us) of a tile of `tok` tokens; the plan with the shortest modelled time of the busiest worker (with
 // `tok_force` > 0, of that width).  false: too many tiles.
 typedef double (*TileTime)(const sacq_layer* L, int tok);
-bool plan_tiles(const sacq_layer* L, int64_t M, TileTime tile_us, int tok_force, tmemw::TilePlan* p);
+bool plan_tiles(const sacq_layer* L, int64_t M, TileTime tile_us, int tok_force, tmemw::TilePlan* p, double* us = nullptr);
 
 // Where a kernel's result goes, and the tensor maps of tile_epilogue's bulk stores (boxes of 32 tokens x 32 rows) over y and
 // over the peers' copies of it: they need a 16-byte aligned base and row pitch, and no residual.

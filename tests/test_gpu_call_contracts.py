@@ -79,3 +79,40 @@ def test_few_tokens_multiply_exact_weights(N, K, d, C, G):
             # one step of bf16 is up to 2^-7 of the value: 2^-8 of the outputs off by one are 2^-11 of the norm
             assert float((y.double() - want.double()).norm() / want.double().norm()) <= 2.0 ** -11, (mode, M)
     assert mod.device_status() == 0
+
+
+@pytest.mark.parametrize("K,d,C,G", [(28672, 4, 4096, None), (30720, 4, 4096, None), (32768, 4, 4096, None),
+                                     (28672, 4, 2048, 64), (32768, 4, 2048, 64), (16384, 8, 65536, None)])
+def test_deep_layers_run_at_every_token_count(K, d, C, G):
+    """Layers whose slice of K leaves little or no shared memory for activation tiles: every token count runs, on e4m3 and
+    INT8 activations and on the two recipes, and a forced kernel that can run 16 tokens can run 1,000."""
+    from sacq_b200 import quantize_rows
+    mod = _layer(64, K, d, C, G)
+    w = mod.dequantize_weight().double()
+    tol = 2.0 ** -8 + 2.0 ** -9                          # e4m3 halves or bf16 reconstruction, bf16 output
+    x = _x(1100, K)
+    for mode, call in (("fp8_e4m3fn", mod.linear_a8), ("int8_symmetric", mod.linear_a8i)):
+        q, s = quantize_rows(x, mode)
+        ref = q.double() @ w.t() * s.double()
+        for M in (16, 17, 33, 65, 129, 200, 257, 700, 1000, 1023, 1100):
+            y = call(q[:M].contiguous(), s[:M].contiguous()).double()
+            assert float((y - ref[:M]).norm() / ref[:M].norm()) <= tol, (mode, M)
+    q, s = quantize_rows(x)
+    ref = q.double() @ w.t() * s.double()
+    for which in ("large", "large_grouped", "large_tmem", "large_tmem_grouped"):
+        mod.set_kernel(which)
+        try:
+            mod.linear_a8(q[:16], s[:16])
+        except Exception as e:
+            assert getattr(e, "code", 0) == -2, which
+            continue
+        for M in (385, 700, 1000):
+            y = mod.linear_a8(q[:M], s[:M])
+            assert float((y.double() - ref[:M]).norm() / ref[:M].norm()) <= tol, (which, M)
+            assert torch.equal(y[:16], mod.linear_a8(q[:16], s[:16])), (which, M)
+    mod.set_kernel("auto")
+    sw = mod.weight_row_scale("int8_symmetric")
+    qi, si = quantize_rows(x[:20].contiguous(), "int8_symmetric")
+    acc = qi.double() @ mod.decode_weight_int8(sw).double().t()
+    assert torch.equal(mod.linear_w8a8_int8(qi, si, sw), ((acc.float() * sw.reshape(1, -1)) * si).to(torch.bfloat16))
+    assert mod.device_status() == 0
