@@ -72,7 +72,7 @@ struct alignas(64) SplitParams {
   CUtensorMap idx[kSplitMaxLayers];     // [16 bytes][128 rows][max_slices] boxes over the packed rows
   SplitLayer layer[kSplitMaxLayers];
   const float* act_scale;       // [M]
-  const float* row_scale;       // recipes: [N], the weight bytes' scale
+  const float* row_scale;       // recipes: [N], the weight bytes' scale (the caller's buffer, not a layer constant)
   uint16_t shift;               // recipes: bf16 bits
   const uint16_t* residual;     // bf16 [M, ldr] added to the rounded output, or null
   int64_t ldr;
@@ -437,8 +437,8 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
     if (et < kRows) {
       const int n = min(n0 + et, lay.N - 1);
-      reinterpret_cast<float*>(sm + L.sw_off)[et] =
-          RECIPE ? __ldg(p.row_scale + n) : F16 ? lay.out_mul : bf16_bits_to_float(__ldg(lay.scales + n)) * lay.out_mul;
+      if constexpr (!RECIPE)
+        reinterpret_cast<float*>(sm + L.sw_off)[et] = F16 ? lay.out_mul : bf16_bits_to_float(__ldg(lay.scales + n)) * lay.out_mul;
       reinterpret_cast<float*>(sm + L.bias_off)[et] = lay.bias ? bf16_bits_to_float(__ldg(lay.bias + n)) : 0.f;
     }
     constexpr bool GROUPS = F16 || RECIPE;             // scales enter the weight operand
@@ -470,6 +470,11 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     int grp = 0, grp_end = GROUPS ? (g_first + 1) * p.group_size - kb0 * kStageK : 0;    // k (in the slice) at which the scale changes
     // One stage's 16 words of this thread.  The next stage's words are gathered before the wait for this
     // stage's tcgen05.st: the gathers, which bound the loop, then never wait for a store's latency.
+    // A recipe's row scales are the caller's and may come from the kernel in front; what has been read so far is the layer's.
+    if constexpr (RECIPE) {
+      asm volatile("griddepcontrol.wait;" ::: "memory");
+      if (et < kRows) reinterpret_cast<float*>(sm + L.sw_off)[et] = __ldg(p.row_scale + min(n0 + et, lay.N - 1));   // for the reduction
+    }
     const RowWeights rw = row_weights<INT>(RECIPE ? __ldg(p.row_scale + min(n0 + row, lay.N - 1)) : 1.f);
     const __nv_bfloat162 shift2 = __halves2bfloat162(__ushort_as_bfloat16(p.shift), __ushort_as_bfloat16(p.shift));
     // kSplitHalf2: the codewords as they are, and the two 64-k tiles' scales; the products are made at the store.

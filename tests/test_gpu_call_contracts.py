@@ -116,3 +116,23 @@ def test_deep_layers_run_at_every_token_count(K, d, C, G):
     acc = qi.double() @ mod.decode_weight_int8(sw).double().t()
     assert torch.equal(mod.linear_w8a8_int8(qi, si, sw), ((acc.float() * sw.reshape(1, -1)) * si).to(torch.bfloat16))
     assert mod.device_status() == 0
+
+
+@pytest.mark.parametrize("mode", ["int8_symmetric", "fp8_e4m3fn"])
+def test_recipe_reads_row_scales_of_the_kernel_in_front(mode):
+    """The recipe's row scales may be written by the launch directly before the call, on the same stream: here the
+    quantizer, which lets the kernel behind it start early, on the layer's own weights."""
+    from sacq_b200 import quantize_rows
+    mod = _layer(6144, 2048)
+    call = mod.linear_w8a8_int8 if mode == "int8_symmetric" else mod.linear_w8a8_fp8
+    w = mod.dequantize_weight()
+    want_sw = mod.weight_row_scale(mode).clone()
+    for M in (1, 16, 200, 1024):                        # inside the GEMM, and as rows of their own
+        q, s = quantize_rows(_x(M, 2048), mode)
+        want = call(q, s, want_sw)
+        wq = torch.empty(6144, 2048, dtype=torch.uint8, device="cuda")
+        for _ in range(10):
+            sw = torch.full((6144, 1), 1e30, device="cuda")
+            quantize_rows(w, mode, out=wq, scale_out=sw)
+            assert torch.equal(call(q, s, sw), want), M
+            assert torch.equal(sw, want_sw)
