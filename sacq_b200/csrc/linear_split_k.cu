@@ -464,8 +464,9 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     const uint8_t* rowidx = sm + L.idx_off + row * 16;
     const uint32_t mask = (1u << p.bits) - 1u;
     const int bits = p.bits;
-    ok = mbar_wait(bar(IDX_FULL), 0, abort_flag, lay.status) &&
-         (!CB_SMEM || mbar_wait(bar(CB_FULL), 0, abort_flag, lay.status));
+    // One answer per warp: what follows (tcgen05.st, its wait, __syncwarp) is the whole warp's.
+    ok = mbar_wait_warp(bar(IDX_FULL), 0, abort_flag, lay.status) &&
+         (!CB_SMEM || mbar_wait_warp(bar(CB_FULL), 0, abort_flag, lay.status));
     if (et == 0) SACQ_SPT(3);
     int grp = 0, grp_end = GROUPS ? (g_first + 1) * p.group_size - kb0 * kStageK : 0;    // k (in the slice) at which the scale changes
     // One stage's 16 words of this thread.  The next stage's words are gathered before the wait for this
@@ -560,7 +561,7 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     __half2 cur_s[2], nxt_s[2];
     if (ok) expand(0, cur, cur_s);
     for (int wi = 0; wi < kbs && ok; ++wi) {
-      ok = mbar_wait(bar(W_EMPTY + ws), w_parity, abort_flag, lay.status);
+      ok = mbar_wait_warp(bar(W_EMPTY + ws), w_parity, abort_flag, lay.status);
       if (!ok) break;
       tc_fence_after();                               // the MMAs that read this stage are complete
       // two quarters of the stage: high and low halves, or the two 64-k tiles
@@ -597,9 +598,8 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       }
     }
     if (et == 0) SACQ_SPT(4);
-    if (ok) ok = mbar_wait(bar(ACC_FULL), 0, abort_flag, lay.status);
+    if (ok) ok = mbar_wait_warp(bar(ACC_FULL), 0, abort_flag, lay.status);
     if (et == 0) SACQ_SPT(5);
-    ok = __all_sync(0xffffffffu, ok);
   }
 
   // ---- reduction: the accumulators of the cluster's CTAs -> y.  Every thread takes part in the barriers.
