@@ -199,16 +199,22 @@ SACQ_API int sacq_layer_create(const sacq_layer_desc* desc, sacq_layer_t** out_l
   L->cb_entries = (d.codebook_size + 1) & ~1;
   split_k_init(L);
   const int64_t count = (int64_t)L->cb_entries * d.vector_dim;
-  cudaError_t e = cudaMalloc(&L->cb_f16, (size_t)count * sizeof(__half));
-  if (e == cudaSuccess) e = cudaMalloc(&L->cb_hilo, (size_t)count * 2);
-  if (e == cudaSuccess) e = cudaMalloc(&L->row_mul, (size_t)(d.out_features > 0 ? d.out_features : 1) * sizeof(float));
-  if (e == cudaSuccess) e = cudaMalloc(&L->d_status, sizeof(int));
-  if (e == cudaSuccess) e = cudaMemset(L->d_status, 0, sizeof(int));
+  // one allocation for all that is derived from the layer (each of its own costs a layer's making milliseconds)
+  auto up = [](int64_t v) { return (v + 255) & ~(int64_t)255; };
+  const int64_t hilo_at = up(count * 2), mul_at = hilo_at + up(count * 2), status_at = mul_at + up(d.out_features * 4);
+  cudaError_t e = cudaMalloc(&L->derived, (size_t)(status_at + 256));
+  if (e == cudaSuccess) {
+    L->cb_f16 = reinterpret_cast<__half*>(L->derived);
+    L->cb_hilo = L->derived + hilo_at;
+    L->row_mul = reinterpret_cast<float*>(L->derived + mul_at);
+    L->d_status = reinterpret_cast<int*>(L->derived + status_at);
+    e = cudaMemset(L->d_status, 0, sizeof(int));
+  }
   if (e != cudaSuccess) {
     sacq_layer_destroy(L);
     return cuda_fail(e, "allocating derived codebook tables");
   }
-  L->resident_bytes = count * 4 + d.out_features * (int64_t)sizeof(float) + (int64_t)sizeof(int);
+  L->resident_bytes = status_at + 256;
   const int rc = launch_build_tables(L, nullptr);
   if (rc != SACQ_OK) {
     sacq_layer_destroy(L);
@@ -223,10 +229,7 @@ SACQ_API int sacq_layer_destroy(sacq_layer_t* L) {
   DeviceGuard guard(L->d.device);
   large_m_release(L);
   split_k_release(L);
-  if (L->cb_f16) cudaFree(L->cb_f16);
-  if (L->cb_hilo) cudaFree(L->cb_hilo);
-  if (L->row_mul) cudaFree(L->row_mul);
-  if (L->d_status) cudaFree(L->d_status);
+  if (L->derived) cudaFree(L->derived);
   delete L;
   return SACQ_OK;
 }

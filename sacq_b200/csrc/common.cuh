@@ -33,6 +33,7 @@ struct sacq_layer {
   int force_kernel;          // 0 auto, 1 small-M, 2 large-M, 3..6 small-M variants, 7 grouped tensor-core
   int cb_entries;            // codebook entries rounded up to even: the derived tables are whole 16-byte units
   // derived device tables (owned)
+  uint8_t* derived;          // the layer's own allocation; the next three and d_status lie in it
   __half* cb_f16;            // [cb_entries, d] (zero padded) codebook * 2^cb_exp_shift as fp16 (small-M kernel)
   uint8_t* cb_hilo;          // [cb_entries][2][d] (zero padded) e4m3 high/low split of codebook * 2^cb8_exp_shift (large-M kernel)
   int cb_exp_shift;          // power-of-two normalisation folded back in the epilogue
