@@ -374,6 +374,9 @@ large_m_tmem_grouped_kernel(const __grid_constant__ CUtensorMap tmap_a, const __
                     bar(ACC_EMPTY));
       if (alias) {
         tma_store_wait_read<0>();                     // the stores have read the staged tiles
+        // ... and so have the warp's own loads and stores (residual, unaligned y), which the activation copy that
+        // overwrites the stage, an asynchronous one, has to come after
+        fence_proxy_async();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(EPI_DONE));
       }

@@ -136,3 +136,23 @@ def test_recipe_reads_row_scales_of_the_kernel_in_front(mode):
             quantize_rows(w, mode, out=wq, scale_out=sw)
             assert torch.equal(call(q, s, sw), want), M
             assert torch.equal(sw, want_sw)
+
+
+@pytest.mark.parametrize("N,K,C,G", [(6144, 256, 1024, 64), (6137, 512, 81, 64)])
+def test_staged_output_and_the_next_tiles_activations(N, K, C, G):
+    """The persistent kernel for grouped scales stages a wide tile's output where the next tile's activations go.  With a
+    residual or an unaligned output its warps read the stage back themselves: many short tiles per CTA, every row compared
+    with the same rows of a call that has one tile each."""
+    from sacq_b200 import quantize_rows
+    mod = _layer(N, K, 4, C, G)
+    mod.set_kernel("large_tmem_grouped")
+    M = 3000
+    q, s = quantize_rows(_x(M, K))
+    parts = torch.cat([mod.linear_a8(q[i:i + 128], s[i:i + 128]) for i in range(0, M, 128)])
+    res = _x(M, N, seed=5)
+    wide = torch.full((M, N + 3), 7.0, dtype=torch.bfloat16, device="cuda")
+    for _ in range(5):
+        assert torch.equal(mod.linear_a8(q, s, residual=res), parts + res)
+        mod.linear_a8(q, s, out=wide[:, :N])
+        assert torch.equal(wide[:, :N], parts)
+    assert mod.device_status() == 0
