@@ -278,13 +278,15 @@ __device__ __forceinline__ uint32_t act_pair(uint32_t a, uint32_t b, uint32_t c)
 }
 
 // CH > 0: every row of a, b, c and q is 16-byte (q: 8-byte) aligned, K % 8 == 0 and a thread holds CH chunks of 8
-// results in registers between the passes.  CH = 0: any row, kept in shared memory.
-template <int KIND, int CH>
+// results in registers between the passes; of a row longer than that (TAIL) it keeps the rest in shared memory.
+// CH = 0: any row, kept in shared memory, an element at a time (rows of 14,336 took 54 us that way for 512 tokens of
+// SiLU, 29 here; of 100,000, 950 and 250).
+template <int KIND, int CH, bool TAIL>
 __global__ void __launch_bounds__(1024)
 act_quant_fp8_kernel(const uint16_t* __restrict__ a, int64_t a_pitch, const uint16_t* __restrict__ b, int64_t b_pitch,
                      const uint16_t* __restrict__ c, int64_t K, uint8_t* __restrict__ q,
                      float* __restrict__ scale_out) {
-  extern __shared__ __align__(16) uint16_t yrow[];    // CH = 0: the row's bf16 values between the passes
+  extern __shared__ __align__(16) uint16_t yrow[];    // CH = 0, TAIL: the row's (the tail's) bf16 values between the passes
   __shared__ uint32_t red[32];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");   // launched behind the producer of a / b with programmatic serialization
@@ -295,25 +297,38 @@ act_quant_fp8_kernel(const uint16_t* __restrict__ a, int64_t a_pitch, const uint
   uint8_t* qrow = q + m * K;
   uint32_t mx = 0u;                                  // bit pattern of the running maximum (absmax_bits)
   if constexpr (CH > 0) {
+    const int64_t chunks = K >> 3, kept = (int64_t)CH * T;
+    auto load = [&](int64_t ch, uint4& v, uint4& w, uint4& u) {
+      v = __ldg(reinterpret_cast<const uint4*>(arow) + ch);
+      if constexpr (KIND != 1) w = __ldg(reinterpret_cast<const uint4*>(brow) + ch);
+      if constexpr (KIND == 2) u = __ldg(reinterpret_cast<const uint4*>(c) + ch);
+    };
+    auto act = [&](const uint4& v, const uint4& w, const uint4& u) {
+      return make_uint4(act_pair<KIND>(v.x, w.x, u.x), act_pair<KIND>(v.y, w.y, u.y), act_pair<KIND>(v.z, w.z, u.z),
+                        act_pair<KIND>(v.w, w.w, u.w));
+    };
     uint4 y[CH], bb[CH], cc[CH];
 #pragma unroll
     for (int h = 0; h < CH; ++h) {                   // all loads first
       const int64_t ch = tid + (int64_t)h * T;
       y[h] = bb[h] = cc[h] = make_uint4(0, 0, 0, 0);
-      if (ch < (K >> 3)) {
-        y[h] = __ldg(reinterpret_cast<const uint4*>(arow) + ch);
-        if constexpr (KIND != 1) bb[h] = __ldg(reinterpret_cast<const uint4*>(brow) + ch);
-        if constexpr (KIND == 2) cc[h] = __ldg(reinterpret_cast<const uint4*>(c) + ch);
-      }
+      if (ch < chunks) load(ch, y[h], bb[h], cc[h]);
     }
 #pragma unroll
     for (int h = 0; h < CH; ++h) {
-      uint32_t aw[4] = {y[h].x, y[h].y, y[h].z, y[h].w};
-      const uint32_t bw[4] = {bb[h].x, bb[h].y, bb[h].z, bb[h].w}, cw[4] = {cc[h].x, cc[h].y, cc[h].z, cc[h].w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) aw[j] = act_pair<KIND>(aw[j], bw[j], cw[j]);
-      y[h] = make_uint4(aw[0], aw[1], aw[2], aw[3]);
-      if (tid + (int64_t)h * T < (K >> 3)) mx = chunk_max(mx, y[h]);
+      y[h] = act(y[h], bb[h], cc[h]);
+      if (tid + (int64_t)h * T < chunks) mx = chunk_max(mx, y[h]);
+    }
+    if constexpr (TAIL) {
+      uint4* tail = reinterpret_cast<uint4*>(yrow);
+#pragma unroll 4
+      for (int64_t ch = kept + tid; ch < chunks; ch += T) {
+        uint4 v, w = make_uint4(0, 0, 0, 0), u = w;
+        load(ch, v, w, u);
+        v = act(v, w, u);
+        tail[ch - kept] = v;                         // read again by this thread only
+        mx = chunk_max(mx, v);
+      }
     }
     mx = pair_max_bits(mx);
     const RowDivisor d = scale_of<false>(__uint_as_float(block_max_bits(mx, red)));
@@ -321,7 +336,12 @@ act_quant_fp8_kernel(const uint16_t* __restrict__ a, int64_t a_pitch, const uint
 #pragma unroll
     for (int h = 0; h < CH; ++h) {
       const int64_t ch = tid + (int64_t)h * T;
-      if (ch < (K >> 3)) reinterpret_cast<uint2*>(qrow)[ch] = encode8<false>(y[h], d);
+      if (ch < chunks) reinterpret_cast<uint2*>(qrow)[ch] = encode8<false>(y[h], d);
+    }
+    if constexpr (TAIL) {
+#pragma unroll 2
+      for (int64_t ch = kept + tid; ch < chunks; ch += T)
+        reinterpret_cast<uint2*>(qrow)[ch] = encode8<false>(reinterpret_cast<const uint4*>(yrow)[ch - kept], d);
     }
   } else {
     for (int64_t k = tid; k < K; k += T) {
@@ -348,15 +368,16 @@ act_quant_fp8_kernel(const uint16_t* __restrict__ a, int64_t a_pitch, const uint
   }
 }
 
-// The instance for a row of `chunks` 16-byte chunks on `threads` threads: 1..4 chunks in registers, else (0) any row.
+// The instance for rows of that many chunks a thread: 1..4 in registers, -1: four and a tail, else (0) any row.
 template <int KIND>
 const void* act_quant_instance(int64_t per_thread) {
   switch (per_thread) {
-    case 1: return (const void*)act_quant_fp8_kernel<KIND, 1>;
-    case 2: return (const void*)act_quant_fp8_kernel<KIND, 2>;
-    case 3: return (const void*)act_quant_fp8_kernel<KIND, 3>;
-    case 4: return (const void*)act_quant_fp8_kernel<KIND, 4>;
-    default: return (const void*)act_quant_fp8_kernel<KIND, 0>;
+    case 1: return (const void*)act_quant_fp8_kernel<KIND, 1, false>;
+    case 2: return (const void*)act_quant_fp8_kernel<KIND, 2, false>;
+    case 3: return (const void*)act_quant_fp8_kernel<KIND, 3, false>;
+    case 4: return (const void*)act_quant_fp8_kernel<KIND, 4, false>;
+    case -1: return (const void*)act_quant_fp8_kernel<KIND, 4, true>;
+    default: return (const void*)act_quant_fp8_kernel<KIND, 0, false>;
   }
 }
 
@@ -372,18 +393,20 @@ int launch_act_quant_fp8(int kind, const void* a, int64_t a_pitch, const void* b
                    (kind != 2 || reinterpret_cast<uintptr_t>(c) % 16 == 0);
   const unsigned threads = row_threads(M, K, kFewRows);
   int64_t per_thread = vec ? (K / 8 + threads - 1) / threads : 0;
-  if (per_thread > 4) per_thread = 0;
-  const size_t smem = per_thread == 0 ? (size_t)K * sizeof(uint16_t) : 0;
-  if (smem > 200 * 1024) return set_error(SACQ_ERR_UNSUPPORTED, "K=%lld: a row does not fit shared memory", (long long)K);
+  if (per_thread > 4) per_thread = -1;
+  const size_t smem = per_thread > 0 ? 0 : (size_t)(K - (per_thread < 0 ? 32 * (int64_t)threads : 0)) * sizeof(uint16_t);
+  if ((size_t)K * sizeof(uint16_t) > 200 * 1024 && per_thread <= 0)
+    return set_error(SACQ_ERR_UNSUPPORTED, "K=%lld: a row does not fit shared memory", (long long)K);
   const void* fn = kind == 0 ? act_quant_instance<0>(per_thread) : kind == 1 ? act_quant_instance<1>(per_thread)
                                                                              : act_quant_instance<2>(per_thread);
-  static bool configured[3][64] = {};
+  static bool configured[3][2][64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
-  if (smem > 48 * 1024 && (dev < 0 || dev >= 64 || !configured[kind][dev])) {
+  const int tail = per_thread < 0;
+  if (smem > 48 * 1024 && (dev < 0 || dev >= 64 || !configured[kind][tail][dev])) {
     const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute");
-    if (dev >= 0 && dev < 64) configured[kind][dev] = true;
+    if (dev >= 0 && dev < 64) configured[kind][tail][dev] = true;
   }
   const uint16_t* ap = static_cast<const uint16_t*>(a);
   const uint16_t* bp = kind == 1 ? nullptr : static_cast<const uint16_t*>(b);

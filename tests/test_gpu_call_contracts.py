@@ -156,3 +156,18 @@ def test_staged_output_and_the_next_tiles_activations(N, K, C, G):
         mod.linear_a8(q, s, out=wide[:, :N])
         assert torch.equal(wide[:, :N], parts)
     assert mod.device_status() == 0
+
+
+@pytest.mark.parametrize("M,K", [(1, 32776), (3, 102400), (297, 8200), (300, 14336), (512, 40960), (298, 8196), (2, 40001)])
+def test_activations_of_wide_rows(M, K):
+    """Rows of more chunks than the registers hold, aligned and not: the bytes of the separate tensor operations."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    import torch.nn.functional as F
+    from sacq_b200 import act_quantize_rows, modulate_quantize_rows, quantize_rows
+    a, b = _x(M, K), _x(M, K, seed=4)
+    a[M - 1] *= 1e-3
+    for got, y in ((act_quantize_rows("silu_mul", a, b), F.silu(a) * b), (act_quantize_rows("gelu", a), F.gelu(a)),
+                   (modulate_quantize_rows(a, b[0], b[M - 1]), a * (1 + b[0]) + b[M - 1])):
+        want = quantize_rows(y)
+        assert torch.equal(got[0].view(torch.uint8), want[0].view(torch.uint8)) and torch.equal(got[1], want[1])
