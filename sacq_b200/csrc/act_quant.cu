@@ -279,8 +279,7 @@ __device__ __forceinline__ uint32_t act_pair(uint32_t a, uint32_t b, uint32_t c)
 
 // CH > 0: every row of a, b, c and q is 16-byte (q: 8-byte) aligned, K % 8 == 0 and a thread holds CH chunks of 8
 // results in registers between the passes; of a row longer than that (TAIL) it keeps the rest in shared memory.
-// CH = 0: any row, kept in shared memory, an element at a time (rows of 14,336 took 54 us that way for 512 tokens of
-// SiLU, 29 here; of 100,000, 950 and 250).
+// CH = 0: any row, kept in shared memory, an element at a time (512 rows of 14,336, SiLU: 26.8 us that way, 11.5 here).
 template <int KIND, int CH, bool TAIL>
 __global__ void __launch_bounds__(1024)
 act_quant_fp8_kernel(const uint16_t* __restrict__ a, int64_t a_pitch, const uint16_t* __restrict__ b, int64_t b_pitch,
@@ -344,6 +343,7 @@ act_quant_fp8_kernel(const uint16_t* __restrict__ a, int64_t a_pitch, const uint
         reinterpret_cast<uint2*>(qrow)[ch] = encode8<false>(reinterpret_cast<const uint4*>(yrow)[ch - kept], d);
     }
   } else {
+#pragma unroll 4
     for (int64_t k = tid; k < K; k += T) {
       const float av = bf16_bits_to_float(__ldg(arow + k));
       const float bv = KIND == 1 ? 0.f : bf16_bits_to_float(__ldg(brow + k));
@@ -473,14 +473,15 @@ __device__ __forceinline__ float norm_value(float x, float mean, float rstd, boo
 
 // CH > 0: x, the vectors, y_out and q are 16-byte (q: 8-byte) aligned, K % 8 == 0 and a thread holds CH chunks of 8
 // elements in registers through all passes (in shared memory and one element at a time this kernel took 4.2 us for
-// 300 rows of 2,048).  CH = 0: any row, kept in shared memory.
-template <bool MOD, int CH>
+// 300 rows of 2,048); of a row longer than that (TAIL) it keeps the rest in shared memory, as bf16.  CH = 0: any row,
+// kept in shared memory.
+template <bool MOD, int CH, bool TAIL>
 __global__ void __launch_bounds__(1024)
 layernorm_quant_fp8_kernel(const uint16_t* __restrict__ x, int64_t pitch, const uint16_t* __restrict__ gamma,
                            const uint16_t* __restrict__ beta, float eps, const uint16_t* __restrict__ mod_scale,
                            const uint16_t* __restrict__ mod_shift, int64_t K, uint16_t* __restrict__ y_out,
                            int64_t y_pitch, uint8_t* __restrict__ q, float* __restrict__ scale_out) {
-  extern __shared__ __align__(16) float xrow[];       // CH = 0: the row in fp32, later its bf16 result in place
+  extern __shared__ __align__(16) float xrow[];       // CH = 0: the row in fp32, later its bf16 result in place; TAIL: chunks
   __shared__ float red_sum[32], red_sq[32];
   __shared__ uint32_t red_max[32];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -497,33 +498,47 @@ layernorm_quant_fp8_kernel(const uint16_t* __restrict__ x, int64_t pitch, const 
       const int64_t ch = tid + (int64_t)h * T;
       v[h] = ch < chunks ? __ldg(reinterpret_cast<const uint4*>(row) + ch) : make_uint4(0, 0, 0, 0);
     }
+    const int64_t kept = (int64_t)CH * T;
+    uint4* tail = reinterpret_cast<uint4*>(xrow);     // chunk ch at ch - kept, read by the thread that wrote it only
     auto word = [](const uint4& u, int j) { return j == 0 ? u.x : j == 1 ? u.y : j == 2 ? u.z : u.w; };
     auto lo = [](uint32_t w) { return __uint_as_float(w << 16); };
     auto hi = [](uint32_t w) { return __uint_as_float(w & 0xffff0000u); };
     float sum = 0.f;
+    auto add = [&](const uint4& u) {
 #pragma unroll
-    for (int h = 0; h < CH; ++h)
+      for (int j = 0; j < 4; ++j) sum += lo(word(u, j)) + hi(word(u, j));
+    };
 #pragma unroll
-      for (int j = 0; j < 4; ++j) sum += lo(word(v[h], j)) + hi(word(v[h], j));
+    for (int h = 0; h < CH; ++h) add(v[h]);
+    if constexpr (TAIL) {
+#pragma unroll 4
+      for (int64_t ch = kept + tid; ch < chunks; ch += T) {
+        const uint4 u = __ldg(reinterpret_cast<const uint4*>(row) + ch);
+        tail[ch - kept] = u;
+        add(u);
+      }
+    }
     const float mean = block_sum(sum, red_sum) / (float)K;
     float sq = 0.f;
+    auto add_sq = [&](const uint4& u) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float d0 = lo(word(u, j)) - mean, d1 = hi(word(u, j)) - mean;
+        sq += d0 * d0;
+        sq += d1 * d1;
+      }
+    };
 #pragma unroll
     for (int h = 0; h < CH; ++h)
-      if (tid + (int64_t)h * T < chunks) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float d0 = lo(word(v[h], j)) - mean, d1 = hi(word(v[h], j)) - mean;
-          sq += d0 * d0;
-          sq += d1 * d1;
-        }
-      }
+      if (tid + (int64_t)h * T < chunks) add_sq(v[h]);
+    if constexpr (TAIL) {
+#pragma unroll 4
+      for (int64_t ch = kept + tid; ch < chunks; ch += T) add_sq(tail[ch - kept]);
+    }
     const float var = block_sum(sq, red_sq) / (float)K;
     const float rstd = 1.0f / sqrtf(var + eps);
     const bool aw = gamma != nullptr, ab = beta != nullptr;
-#pragma unroll
-    for (int h = 0; h < CH; ++h) {
-      const int64_t ch = tid + (int64_t)h * T;
-      if (ch >= chunks) continue;
+    auto normalize = [&](const uint4& u, int64_t ch) {
       uint4 g = make_uint4(0, 0, 0, 0), b = g, ms = g, mt = g;
       if (aw) g = __ldg(reinterpret_cast<const uint4*>(gamma) + ch);
       if (ab) b = __ldg(reinterpret_cast<const uint4*>(beta) + ch);
@@ -534,15 +549,25 @@ layernorm_quant_fp8_kernel(const uint16_t* __restrict__ x, int64_t pitch, const 
       uint32_t o[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const float y0 = norm_value<MOD>(lo(word(v[h], j)), mean, rstd, aw, lo(word(g, j)), ab, lo(word(b, j)), lo(word(ms, j)),
+        const float y0 = norm_value<MOD>(lo(word(u, j)), mean, rstd, aw, lo(word(g, j)), ab, lo(word(b, j)), lo(word(ms, j)),
                                          lo(word(mt, j)));
-        const float y1 = norm_value<MOD>(hi(word(v[h], j)), mean, rstd, aw, hi(word(g, j)), ab, hi(word(b, j)), hi(word(ms, j)),
+        const float y1 = norm_value<MOD>(hi(word(u, j)), mean, rstd, aw, hi(word(g, j)), ab, hi(word(b, j)), hi(word(ms, j)),
                                          hi(word(mt, j)));
         o[j] = (__float_as_uint(y0) >> 16) | (__float_as_uint(y1) & 0xffff0000u);    // both are bf16 values
       }
-      v[h] = make_uint4(o[0], o[1], o[2], o[3]);
-      mx = chunk_max(mx, v[h]);
-      if (y_out != nullptr) reinterpret_cast<uint4*>(y_out + m * y_pitch)[ch] = v[h];
+      const uint4 y = make_uint4(o[0], o[1], o[2], o[3]);
+      mx = chunk_max(mx, y);
+      if (y_out != nullptr) reinterpret_cast<uint4*>(y_out + m * y_pitch)[ch] = y;
+      return y;
+    };
+#pragma unroll
+    for (int h = 0; h < CH; ++h) {
+      const int64_t ch = tid + (int64_t)h * T;
+      if (ch < chunks) v[h] = normalize(v[h], ch);
+    }
+    if constexpr (TAIL) {
+#pragma unroll 2
+      for (int64_t ch = kept + tid; ch < chunks; ch += T) tail[ch - kept] = normalize(tail[ch - kept], ch);
     }
     mx = pair_max_bits(mx);
     const RowDivisor d = scale_of<false>(__uint_as_float(block_max_bits(mx, red_max)));
@@ -552,9 +577,14 @@ layernorm_quant_fp8_kernel(const uint16_t* __restrict__ x, int64_t pitch, const 
       const int64_t ch = tid + (int64_t)h * T;
       if (ch < chunks) reinterpret_cast<uint2*>(qrow)[ch] = encode8<false>(v[h], d);
     }
+    if constexpr (TAIL) {
+#pragma unroll 2
+      for (int64_t ch = kept + tid; ch < chunks; ch += T) reinterpret_cast<uint2*>(qrow)[ch] = encode8<false>(tail[ch - kept], d);
+    }
   } else {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     float sum = 0.f;
+#pragma unroll 4
     for (int64_t k = tid; k < K; k += T) {
       const float v = bf16_bits_to_float(__ldg(row + k));
       xrow[k] = v;
@@ -562,12 +592,14 @@ layernorm_quant_fp8_kernel(const uint16_t* __restrict__ x, int64_t pitch, const 
     }
     const float mean = block_sum(sum, red_sum) / (float)K;
     float sq = 0.f;
+#pragma unroll 4
     for (int64_t k = tid; k < K; k += T) {
       const float dlt = xrow[k] - mean;
       sq += dlt * dlt;
     }
     const float var = block_sum(sq, red_sq) / (float)K;
     const float rstd = 1.0f / sqrtf(var + eps);
+#pragma unroll 4
     for (int64_t k = tid; k < K; k += T) {
       const float y = norm_value<MOD>(xrow[k], mean, rstd, gamma != nullptr, gamma ? bf16_bits_to_float(__ldg(gamma + k)) : 0.f,
                                       beta != nullptr, beta ? bf16_bits_to_float(__ldg(beta + k)) : 0.f,
@@ -579,6 +611,7 @@ layernorm_quant_fp8_kernel(const uint16_t* __restrict__ x, int64_t pitch, const 
     }
     const float s = scale_of<false>(__uint_as_float(block_max_bits(mx, red_max))).s;
     if (tid == 0) scale_out[m] = s;
+#pragma unroll 4
     for (int64_t k = tid; k < K; k += T)
       qrow[k] = (uint8_t)(float2_to_e4m3x2(sat448(__fdiv_rn(xrow[k], s)), 0.f) & 0xff);
   }
@@ -588,13 +621,14 @@ layernorm_quant_fp8_kernel(const uint16_t* __restrict__ x, int64_t pitch, const 
 
 namespace {
 template <bool MOD>
-const void* layernorm_instance(int64_t per_thread) {
+const void* layernorm_instance(int64_t per_thread) {  // as act_quant_instance
   switch (per_thread) {
-    case 1: return (const void*)layernorm_quant_fp8_kernel<MOD, 1>;
-    case 2: return (const void*)layernorm_quant_fp8_kernel<MOD, 2>;
-    case 3: return (const void*)layernorm_quant_fp8_kernel<MOD, 3>;
-    case 4: return (const void*)layernorm_quant_fp8_kernel<MOD, 4>;
-    default: return (const void*)layernorm_quant_fp8_kernel<MOD, 0>;
+    case 1: return (const void*)layernorm_quant_fp8_kernel<MOD, 1, false>;
+    case 2: return (const void*)layernorm_quant_fp8_kernel<MOD, 2, false>;
+    case 3: return (const void*)layernorm_quant_fp8_kernel<MOD, 3, false>;
+    case 4: return (const void*)layernorm_quant_fp8_kernel<MOD, 4, false>;
+    case -1: return (const void*)layernorm_quant_fp8_kernel<MOD, 4, true>;
+    default: return (const void*)layernorm_quant_fp8_kernel<MOD, 0, false>;
   }
 }
 }  // namespace
@@ -609,18 +643,20 @@ int launch_layernorm_quant_fp8(const void* x, int64_t pitch, const void* gamma, 
   const bool vec = K % 8 == 0 && pitch % 8 == 0 && al(x, 16) && al(gamma, 16) && al(beta, 16) && al(mod_scale, 16) &&
                    al(mod_shift, 16) && al(q, 8) && (y_out == nullptr || (al(y_out, 16) && y_pitch % 8 == 0));
   const unsigned threads = row_threads(M, K, kFewRows);
-  const int64_t per_thread = vec ? (K / 8 + threads - 1) / threads : 0;
-  const bool regs = per_thread >= 1 && per_thread <= 4;
-  const size_t smem = regs ? 0 : (size_t)K * sizeof(float);
-  if (smem > 200 * 1024) return set_error(SACQ_ERR_UNSUPPORTED, "K=%lld: a row does not fit shared memory", (long long)K);
-  const void* fn = mod ? layernorm_instance<true>(regs ? per_thread : 0) : layernorm_instance<false>(regs ? per_thread : 0);
-  static bool configured[2][64] = {};
+  int64_t per_thread = vec ? (K / 8 + threads - 1) / threads : 0;
+  if (per_thread > 4) per_thread = -1;
+  const size_t smem = per_thread > 0 ? 0 : per_thread < 0 ? (size_t)(K - 32 * (int64_t)threads) * sizeof(uint16_t) : (size_t)K * sizeof(float);
+  if ((size_t)K * sizeof(float) > 200 * 1024 && per_thread <= 0)
+    return set_error(SACQ_ERR_UNSUPPORTED, "K=%lld: a row does not fit shared memory", (long long)K);
+  const void* fn = mod ? layernorm_instance<true>(per_thread) : layernorm_instance<false>(per_thread);
+  static bool configured[2][2][64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
-  if (smem > 48 * 1024 && (dev < 0 || dev >= 64 || !configured[mod][dev])) {
+  const int tail = per_thread < 0;
+  if (smem > 48 * 1024 && (dev < 0 || dev >= 64 || !configured[mod][tail][dev])) {
     const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute");
-    if (dev >= 0 && dev < 64) configured[mod][dev] = true;
+    if (dev >= 0 && dev < 64) configured[mod][tail][dev] = true;
   }
   const uint16_t* xp = static_cast<const uint16_t*>(x);
   const uint16_t* gp = static_cast<const uint16_t*>(gamma);

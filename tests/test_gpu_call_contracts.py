@@ -171,3 +171,22 @@ def test_activations_of_wide_rows(M, K):
                    (modulate_quantize_rows(a, b[0], b[M - 1]), a * (1 + b[0]) + b[M - 1])):
         want = quantize_rows(y)
         assert torch.equal(got[0].view(torch.uint8), want[0].view(torch.uint8)) and torch.equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("M,K", [(1, 32776), (3, 51200), (297, 8200), (300, 14336), (298, 8196), (2, 40001)])
+def test_layernorm_of_wide_rows(M, K):
+    """The same row lengths through the fused LayerNorm: its y within two bf16 steps of torch's in fp32 (another order of
+    the sums, and the step of the modulation), its bytes those of its own y."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    import torch.nn.functional as F
+    from sacq_b200 import layernorm_quantize_rows, quantize_rows
+    x, v = _x(M, K), _x(4, K, seed=4)
+    for mod in (False, True):
+        q, s, y = layernorm_quantize_rows(x, v[0], v[1], 1e-5, *((v[2], v[3]) if mod else ()), return_normalized=True)
+        want = F.layer_norm(x.float(), (K,), v[0].float(), v[1].float(), 1e-5).to(torch.bfloat16)
+        if mod:
+            want = want * (1 + v[2]) + v[3]
+        assert float((y.float() - want.float()).norm() / want.float().norm()) <= 2.0 ** -8
+        want = quantize_rows(y)
+        assert torch.equal(q.view(torch.uint8), want[0].view(torch.uint8)) and torch.equal(s, want[1])
