@@ -19,6 +19,7 @@
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <map>
@@ -116,12 +117,14 @@ struct Target {
   }
 };
 
+// A C++ exception leaves as the Python exception that PyTorch makes of it (an allocation that fails as
+// torch.OutOfMemoryError, which callers catch to free memory and try again).
 #define NATIVE_TRY try {
-#define NATIVE_CATCH                                   \
-  }                                                    \
-  catch (const std::exception& e) {                    \
-    if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, e.what()); \
-    return nullptr;                                    \
+#define NATIVE_CATCH                                                                            \
+  }                                                                                             \
+  catch (...) {                                                                                 \
+    if (!PyErr_Occurred()) torch::translate_exception_to_python(std::current_exception());      \
+    return nullptr;                                                                             \
   }
 
 // Activations of a forward: any [..., K] bf16 tensor whose rows can be addressed with one pitch.

@@ -190,3 +190,14 @@ def test_layernorm_of_wide_rows(M, K):
         assert float((y.float() - want.float()).norm() / want.float().norm()) <= 2.0 ** -8
         want = quantize_rows(y)
         assert torch.equal(q.view(torch.uint8), want[0].view(torch.uint8)) and torch.equal(s, want[1])
+
+
+def test_an_allocation_that_fails_raises_out_of_memory():
+    """Callers catch torch.OutOfMemoryError, free memory and try again: a RuntimeError of another kind would pass them by.
+    The output of 2^23 rows of 2^14 (256 GB) is more than the device has; its input is 1 GB."""
+    mod = _layer(1 << 14, 64, 8, 16)
+    x = torch.zeros(1 << 23, 64, dtype=torch.bfloat16, device="cuda")
+    with pytest.raises(torch.OutOfMemoryError):
+        mod(x)
+    y = mod(x[:16])                                     # and the layer goes on working
+    assert tuple(y.shape) == (16, 1 << 14) and mod.device_status() == 0
