@@ -455,10 +455,12 @@ PyObject* py_layernorm_quantize_rows(PyObject*, PyObject* const* a, Py_ssize_t n
     PyErr_Clear();
     Py_RETURN_NONE;
   }
+  const int want_y = PyObject_IsTrue(a[6]);            // any truth value, as the general route takes it
+  if (want_y < 0) return nullptr;
   Target at_(dev);
   Encoded e(m, k, false, dev);
   at::Tensor y;
-  if (a[6] == Py_True) y = new_tensor({m, k}, at::kBFloat16, dev);
+  if (want_y) y = new_tensor({m, k}, at::kBFloat16, dev);
   const int rc = sacq_layernorm_quant_fp8(x->data_ptr(), x->stride(0), v[0], v[1], (float)eps, v[2], v[3], m, k,
                                           y.defined() ? y.data_ptr() : nullptr, k, e.q.data_ptr(), (float*)e.s.data_ptr(),
                                           at_.stream);

@@ -201,3 +201,12 @@ def test_an_allocation_that_fails_raises_out_of_memory():
         mod(x)
     y = mod(x[:16])                                     # and the layer goes on working
     assert tuple(y.shape) == (16, 1 << 14) and mod.device_status() == 0
+
+
+@pytest.mark.parametrize("flag,wanted", [(True, True), (1, True), ("yes", True), (False, False), (0, False), (None, False)])
+def test_return_normalized_takes_any_truth_value(flag, wanted):
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from sacq_b200 import layernorm_quantize_rows
+    out = layernorm_quantize_rows(_x(5, 64), return_normalized=flag)
+    assert len(out) == (3 if wanted else 2)
