@@ -94,9 +94,12 @@ const at::Tensor* tensor_of(PyObject* o) { return THPVariable_Check(o) ? &THPVar
 
 bool on_device(const at::Tensor& t, int dev) { return t.is_cuda() && t.get_device() == dev; }
 
+// A 2-D tensor whose rows are contiguous (the inner stride of rows of one element means nothing).
+bool whole_rows(const at::Tensor& t) { return t.dim() == 2 && (t.stride(1) == 1 || t.size(1) == 1); }
+
 // bf16 [m, k] rows with unit inner stride
 bool bf16_rows(const at::Tensor& t, int dev) {
-  return t.scalar_type() == at::kBFloat16 && on_device(t, dev) && t.dim() == 2 && t.stride(1) == 1;
+  return t.scalar_type() == at::kBFloat16 && on_device(t, dev) && whole_rows(t);
 }
 
 bool f32_vector(const at::Tensor& t, int64_t n, int dev) {
@@ -137,7 +140,7 @@ bool rows_of(const at::Tensor& x, int64_t k, int dev, Rows& r) {
   const int64_t nd = x.dim();
   if (nd < 1 || x.scalar_type() != at::kBFloat16 || !on_device(x, dev) || x.size(nd - 1) != k) return false;
   if (nd == 2) {
-    if (x.stride(1) != 1) return false;
+    if (!whole_rows(x)) return false;
     r = {x.data_ptr(), x.size(0), x.stride(0)};
   } else {
     if (!x.is_contiguous()) return false;

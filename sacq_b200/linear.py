@@ -399,13 +399,16 @@ class PrecomputedPackedVectorCodebookLinear(torch.nn.Module):
         return y if y is not None else self._forward_general(x)
 
     def _forward_general(self, x: torch.Tensor) -> torch.Tensor:
-        """What the native call does not take: other dtypes, strided or empty inputs, and the errors."""
+        """What the native call does not take: other dtypes, other strides, empty inputs, and the errors.  A view whose rows
+        have one pitch (a slice of the last dimension, a chunk of a fused projection) is read where it lies."""
         if x.shape[-1] != self.in_features:
             raise ValueError("Linear shape mismatch")
         dev = self._dev
         if not x.is_cuda or x.device != dev:
             raise ValueError("Matching CUDA operands required")
-        a = x.reshape(-1, self.in_features).to(torch.bfloat16).contiguous()
+        a = x.reshape(-1, self.in_features).to(torch.bfloat16)
+        if a.stride(-1) != 1:
+            a = a.contiguous()
         m = a.shape[0]
         if m > 0 and self.out_features > 0:
             y = self._native.forward(a)

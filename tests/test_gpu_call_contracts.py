@@ -210,3 +210,20 @@ def test_return_normalized_takes_any_truth_value(flag, wanted):
     from sacq_b200 import layernorm_quantize_rows
     out = layernorm_quantize_rows(_x(5, 64), return_normalized=flag)
     assert len(out) == (3 if wanted else 2)
+
+
+def test_strided_inputs_are_read_where_they_lie():
+    """A slice of a wider tensor, in two and in three dimensions, allocates its output and nothing else; other layouts are
+    made contiguous first.  All give the bytes of the contiguous input."""
+    mod = _layer(256, 512)
+    wide = _x(6 * 40, 1024).reshape(6, 40, 1024)
+    cases = [wide[..., :512], wide[..., 512:], wide[:, 7, :512], wide[0, :, 512:], wide[:3, :, :512].transpose(0, 1),
+             _x(512, 40).t(), _x(512, 6).t().unsqueeze(0), wide[..., :512].float()]
+    for i, x in enumerate(cases):
+        want = mod(x.contiguous())
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_stats()["allocation.all.allocated"]
+        y = mod(x)
+        made = torch.cuda.memory_stats()["allocation.all.allocated"] - before
+        assert torch.equal(y, want) and y.dtype == x.dtype and tuple(y.shape) == (*x.shape[:-1], 256), i
+        assert i >= 4 or made == 1, (i, made)
