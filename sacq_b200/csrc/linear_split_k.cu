@@ -52,6 +52,8 @@ constexpr int kStageK = 128;          // k per weight stage
 constexpr int kMaxAct = 6;            // activation tiles in flight (128 bytes of every token each)
 constexpr int kMaxW = 4;              // weight stages in tensor memory
 constexpr int kSliceBytes = kRows * 16;
+// fp16 forms: K may end in the middle of a stage; its second 64-k tile is then zeros on both sides.
+__host__ __device__ constexpr int stages_of(int64_t K) { return (int)((K + kStageK - 1) / kStageK); }
 __host__ __device__ constexpr int w_cols(int mode) { return mode == kSplitHalf2 ? 128 : mode >= kSplitInt8 ? 32 : 64; }
 constexpr float kHalfPreScale = 4096.f;   // keeps fp16(codeword x scale) far from the subnormals
 
@@ -303,7 +305,7 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   const int warp = (int)warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int rank = S > 1 ? (int)cluster_rank() : 0;
   const int m0 = blockIdx.y * p.tok;
-  const int nkb = p.K / kStageK;
+  const int nkb = stages_of(p.K);
   const int parts = p.parts, slices = S * parts;
   // this CTA's weight stages, and the first one (counted from kb0) of its slice `v`
   const int kb0 = rank * parts * nkb / slices, kbs = (rank + 1) * parts * nkb / slices - kb0;
@@ -443,7 +445,7 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     }
     constexpr bool GROUPS = F16 || RECIPE;             // scales enter the weight operand
     const int g_first = GROUPS ? kb0 * kStageK / p.group_size : 0;
-    const int g_count = GROUPS ? ((kb0 + kbs) * kStageK - 1) / p.group_size - g_first + 1 : 0;
+    const int g_count = GROUPS ? (min((kb0 + kbs) * kStageK, p.K) - 1) / p.group_size - g_first + 1 : 0;
     const int sc_pitch = g_count | 1;                 // odd: the 32 rows of a warp fall on different banks
     uint16_t* sc = reinterpret_cast<uint16_t*>(sm + L.sc_off);
     if constexpr (GROUPS) {
@@ -510,6 +512,12 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         constexpr int IPT = 16 / D;                   // indices per thread and 64-k tile
 #pragma unroll
         for (int sub = 0; sub < 2; ++sub) {
+          if ((kb0 + wi) * kStageK + sub * 64 >= p.K) {
+            sc2[sub] = __half2half2(__ushort_as_half(0));
+#pragma unroll
+            for (int j = 0; j < 8; ++j) w[sub * 8 + j] = 0u;
+            continue;
+          }
           if (wi * kStageK + sub * 64 >= grp_end) { ++grp; grp_end += p.group_size; }
           // scale x 2^e is a bf16 significand with a small exponent: exact in fp16
           const __half2 s2 = __half2half2(__float2half_rn(bf16_bits_to_float(sc[row * sc_pitch + grp]) * scale_mul));
@@ -753,10 +761,11 @@ int codebook_smem(const sacq_layer* L) {
 
 // Index slices and scale groups of the largest K slice.
 void slice_extent(const sacq_layer* L, int split, int* slices, int* groups) {
-  const int nkb = (int)(L->d.in_features / kStageK), d = L->d.vector_dim, bits = L->d.index_bits;
+  const int nkb = stages_of(L->d.in_features), d = L->d.vector_dim, bits = L->d.index_bits;
   *slices = *groups = 0;
   for (int r = 0; r < split; ++r) {
-    const int k0 = r * nkb / split * kStageK, k1 = (r + 1) * nkb / split * kStageK;
+    const int k0 = r * nkb / split * kStageK;
+    const int k1 = r + 1 < split ? (r + 1) * nkb / split * kStageK : (int)L->d.in_features;
     const int n = ((k1 / d * bits + 127) >> 7) - ((k0 / d * bits) >> 7);
     const int g = (k1 - 1) / L->d.group_size - k0 / L->d.group_size + 1;
     if (n > *slices) *slices = n;
@@ -778,7 +787,7 @@ int slices_for(int64_t K) { return K < 1024 ? 1 : K < 4096 ? 2 : K < 8192 ? 4 : 
 bool split_fits(const sacq_layer* L, SplitMode mode, SplitChoice* c) {
   const int cb_bytes = codebook_smem(L), groups = mode == kSplitHiLo ? 0 : 1;
   slice_extent(L, c->split, &c->max_slices, &c->max_groups);
-  const int tiles = ((int)(L->d.in_features / kStageK) + c->split - 1) / c->split * (is_f16(mode) ? 2 : 1);
+  const int tiles = (stages_of(L->d.in_features) + c->split - 1) / c->split * (is_f16(mode) ? 2 : 1);
   const size_t most = (cb_bytes > 0 ? 227 : 164) * 1024;
   auto bytes = [&](int stages) {
     return split_smem(split_layout(c->tok, c->split, stages, c->max_slices, groups * c->max_groups, cb_bytes));
@@ -802,7 +811,7 @@ double split_cta_us(int vector_dim, SplitMode mode, bool cb_smem, int tok, int k
 bool takes_layer(const sacq_layer* L, SplitMode mode) {
   const sacq_layer_desc& d = L->d;
   if (d.vector_dim != 8 && d.vector_dim != 4) return false;
-  if (d.index_bits > 16 || !L->rows_16b_aligned || d.in_features % kStageK != 0) return false;
+  if (d.index_bits > 16 || !L->rows_16b_aligned || d.in_features % (is_f16(mode) ? 64 : kStageK) != 0) return false;
   if (mode < kSplitInt8 && has_shift(L)) return false;
   if (mode == kSplitHiLo ? L->num_groups != 1 : d.group_size % (is_f16(mode) ? 64 : 16) != 0) return false;
   // the recipes read the codebook as it came, which is not padded to whole 16-byte units
@@ -834,7 +843,7 @@ SplitChoice cut_of(int64_t M, int tok, int split, int parts) {
 bool complete(const sacq_layer* L, SplitMode mode, SplitChoice* c) {
   if (!split_fits(L, mode, c)) return false;
   const int64_t row_tiles = (L->d.out_features + kRows - 1) / kRows;
-  const int kbs = ((int)(L->d.in_features / kStageK) + c->split - 1) / c->split;
+  const int kbs = (stages_of(L->d.in_features) + c->split - 1) / c->split;
   const int at_once = active_clusters(c->split, L->num_sms);
   const int64_t waves = (row_tiles * c->tiles + at_once - 1) / at_once;
   // every CTA fetches the codebook through L2

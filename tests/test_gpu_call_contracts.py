@@ -227,3 +227,24 @@ def test_strided_inputs_are_read_where_they_lie():
         made = torch.cuda.memory_stats()["allocation.all.allocated"] - before
         assert torch.equal(y, want) and y.dtype == x.dtype and tuple(y.shape) == (*x.shape[:-1], 256), i
         assert i >= 4 or made == 1, (i, made)
+
+
+@pytest.mark.parametrize("N,K,d,C,G", [(300, 960, 4, 256, 64), (129, 576, 4, 256, 64), (1000, 1088, 8, 65536, 64),
+                                       (2048, 4160, 4, 256, 64), (64, 64, 4, 256, 64)])
+def test_grouped_layers_that_end_inside_a_stage(N, K, d, C, G):
+    """K a multiple of 64 but not of 128: the tensor-core kernel takes the layer, to the last group, at every slice count."""
+    from sacq_b200 import quantize_rows
+    mod = _layer(N, K, d, C, G, bias=True)
+    w, tol = mod.dequantize_weight().double(), 2.0 ** -8 + 2.0 ** -9
+    x = _x(1100, K)
+    for mode, call in (("fp8_e4m3fn", mod.linear_a8), ("int8_symmetric", mod.linear_a8i)):
+        q, s = quantize_rows(x, mode)
+        ref = q.double() @ w.t() * s.double() + mod.bias.double()
+        for M in (1, 17, 47, 48, 96, 300, 1024, 1100):
+            y = call(q[:M].contiguous(), s[:M].contiguous()).double()
+            assert float((y - ref[:M]).norm() / ref[:M].norm()) <= tol, (mode, M)
+    assert mod.kernel_for(300) == "large_grouped"
+    q, s = quantize_rows(x)
+    mod.set_kernel("large_grouped")
+    whole = mod.linear_a8(q, s)
+    assert torch.equal(mod.linear_a8(q[:20], s[:20]), whole[:20]) and mod.device_status() == 0
