@@ -67,6 +67,8 @@ int64_t small_m_slab_rows(const sacq_layer* L) {
 // weights once per 16-token chunk (quantizer + GEMM, d = 4, 10-bit, group 64, the two kernels with exact weights:
 // 2048x6144 22.8 / 11.7 us at 32 rows; 1024x1024 7.5 / 6.8 and 6144x1536 35 / 13.8 at 48).
 int64_t grouped_min_m(const sacq_layer* L) {
+  // ... or from the CUDA-core kernel, at any number (2048x2048, 65,536 entries, group 128: 127 / 11 us at 17 rows)
+  if (!L->small_m_warp_mma) return 1;
   if (L->d.out_features >= 32 * (int64_t)L->num_sms) return 17;
   return 48;
 }
@@ -198,6 +200,7 @@ SACQ_API int sacq_layer_create(const sacq_layer_desc* desc, sacq_layer_t** out_l
   L->num_sms = prop.multiProcessorCount;
   L->cb_entries = (d.codebook_size + 1) & ~1;
   split_k_init(L);
+  L->small_m_warp_mma = small_m_staged_warps(L, 1) > 0;
   const int64_t count = (int64_t)L->cb_entries * d.vector_dim;
   // one allocation for all that is derived from the layer (each of its own costs a layer's making milliseconds)
   auto up = [](int64_t v) { return (v + 255) & ~(int64_t)255; };

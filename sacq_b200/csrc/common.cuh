@@ -41,6 +41,7 @@ struct sacq_layer {
   int sc_exp_shift;          // max |scale| * 2^sc_exp_shift lies in [0.5, 1) (grouped tensor-core kernel)
   float* row_mul;            // [N] power of two: 1 / what brings the row's largest scale into [2^11, 2^12)
   int* d_status;             // device status word, 0 = ok
+  bool small_m_warp_mma;     // whether the small-M path has a staged warp-MMA kernel for the layer
   int split_tok[5];          // per form of the split-K kernel (SplitMode): its widest token tile, 0 if it cannot run the layer
   int64_t resident_bytes;
   sacq::LargeMPlan* large_plan;

@@ -248,3 +248,19 @@ def test_grouped_layers_that_end_inside_a_stage(N, K, d, C, G):
     mod.set_kernel("large_grouped")
     whole = mod.linear_a8(q, s)
     assert torch.equal(mod.linear_a8(q[:20], s[:20]), whole[:20]) and mod.device_status() == 0
+
+
+@pytest.mark.parametrize("N,K,d,C,G", [(300, 1024, 8, 65536, 128), (64, 32768, 4, 2048, 64)])
+def test_grouped_layers_without_a_warp_mma_kernel(N, K, d, C, G):
+    """A codebook or a row of indices that the index-unpacking kernel has no room for: the split-K kernel takes the layer
+    from one token on, with exact weights."""
+    from sacq_b200 import quantize_rows
+    mod = _layer(N, K, d, C, G, bias=True)
+    for M in (1, 5, 16, 40):
+        q, s = quantize_rows(_x(M, K))
+        y, want = mod.linear_a8(q, s), _exact(mod, q, s)
+        assert mod.kernel_for(M) == "large_grouped"
+        # sums of up to 32,768 products: four times the bound of the shorter ones
+        assert float((y.double() - want.double()).norm() / want.double().norm()) <= 2.0 ** -10, M
+        assert torch.equal(mod(_x(M, K)), y)
+    assert mod.device_status() == 0
