@@ -712,14 +712,20 @@ SACQ_API int sacq_linear_a8_multi(const sacq_layer_t* const* layers, int num_lay
 }
 
 namespace {
-// Whether a forward on a staged warp-MMA kernel quantizes its activations in the GEMM's own CTAs.  It saves a launch
-// (eager calls are bound by the host at 7 us with it and at 5.4 without) and costs the GPU each CTA's own pass over the
-// tokens: a gain there too while that is one warp's work per token or less (2048x1024 at 8 tokens 4.9 us either way,
-// 2048x2048 5.6 against 5.9, at 16 tokens 6.3 against 6.1), a loss on layers that keep the GPU busy anyway (2048x6144
-// 8.9 against 8.4 at one token, 6144x2048 10.7 against 8.4 at 8).
-bool quantizes_in_gemm(const sacq_layer* L, int64_t M) {
-  return L->d.in_features * L->d.out_features <= (4 << 20) && M * L->d.in_features <= (32 << 10) &&
-         M <= small_m_staged_warps(L, M);
+// Whether a forward on a staged warp-MMA kernel quantizes its activations in the GEMM's own CTAs.  It saves a launch, which
+// costs the host 2 us of the 7 that an eager call of these sizes takes, and costs the GPU 0.3 to 1.3 us: each CTA's own
+// pass over the tokens (2048x2048, d = 4, 16 tokens 6.5 us against 5.4; 2048x1024 at one 4.5 / 4.2).  A captured call
+// pays for the GPU's time only and keeps the quantizer as a launch of its own; the bytes are the same.  On layers that
+// keep the GPU busy anyway it is a loss in eager calls too (2048x6144 8.9 against 8.4 at one token, 6144x2048 10.7 / 8.4 at 8).
+bool quantizes_in_gemm(const sacq_layer* L, int64_t M, cudaStream_t s) {
+  if (L->d.in_features * L->d.out_features > (4 << 20) || M * L->d.in_features > (32 << 10) || M > small_m_staged_warps(L, M))
+    return false;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &status) != cudaSuccess) {   // the default stream beside another thread's capture
+    cudaGetLastError();
+    return false;
+  }
+  return status == cudaStreamCaptureStatusNone;
 }
 
 // Quantizer + GEMM of one call, in one launch where the GEMM can quantize for itself (own_quantizer = false allows it).
@@ -739,7 +745,7 @@ int forward_impl(const sacq_layer_t* L, const void* x_bf16, int64_t x_pitch, int
   if (rows_ok) {
     const Int8Route r = int8 ? int8_route(L, M) : kInt8Small;
     const int k = int8 ? 0 : pick_kernel(L, M);
-    if (k == 1 && !own_quantizer && quantizes_in_gemm(L, M)) {
+    if (k == 1 && !own_quantizer && quantizes_in_gemm(L, M, static_cast<cudaStream_t>(stream))) {
       DeviceGuard guard(L->d.device);
       return launch_small_m(L, q_scratch, scale_scratch, M, y_out, ldy, workspace, workspace_bytes,
                             static_cast<cudaStream_t>(stream), residual, ldr, 0, nullptr, x_bf16, x_pitch);

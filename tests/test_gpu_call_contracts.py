@@ -264,3 +264,27 @@ def test_grouped_layers_without_a_warp_mma_kernel(N, K, d, C, G):
         assert float((y.double() - want.double()).norm() / want.double().norm()) <= 2.0 ** -10, M
         assert torch.equal(mod(_x(M, K)), y)
     assert mod.device_status() == 0
+
+
+@pytest.mark.parametrize("N,K,d,C,G", [(2048, 2048, 4, 4096, None), (1024, 1024, 4, 256, 64)])
+def test_a_captured_call_gives_the_eager_bytes(N, K, d, C, G):
+    """An eager call of few tokens quantizes inside the GEMM, a captured one in a launch of its own."""
+    mod = _layer(N, K, d, C, G, bias=True)
+    for M in (1, 8, 16, 17):
+        x = _x(M, K)
+        want = mod(x)
+        before = mod._lib.sacq_launch_count()
+        mod(x)
+        eager = mod._lib.sacq_launch_count() - before
+        torch.cuda.synchronize()
+        stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        with torch.cuda.stream(stream):
+            mod(x)                                      # the stream's workspace
+        torch.cuda.synchronize()
+        before = mod._lib.sacq_launch_count()
+        with torch.cuda.graph(graph, stream=stream):
+            y = mod(x)
+        assert mod._lib.sacq_launch_count() - before >= max(eager, 2), M
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y, want), M
