@@ -72,20 +72,25 @@ int64_t grouped_min_m(const sacq_layer* L) {
   if (L->d.out_features >= 32 * (int64_t)L->num_sms) return 17;
   return 48;
 }
-// From how many rows the tensor-core kernel that keeps the expanded weights in tensor memory wins (its 128-row tiles
-// need that many tokens to fill the device).  A codebook that is gathered from L2 makes an expansion twice as dear,
-// and the split-K kernel expands a wide layer again for every second 384-token tile.
+// From how many tokens the persistent kernel with the weights in tensor memory takes over; its 128-row tiles need that many
+// to fill the device.  The split-K kernel expands a wide layer again for every second 384-token tile, from about 700 tokens
+// on in a second wave (1024x4096 at 1,000 tokens 23.5 / 12.6 us, 2048x6144 39 / 24).  It keeps them up to 960 all the same:
+// the two sum in different orders, and up to there the tokens of a request get the same bytes alone and in a batch of
+// three (the price: 2048x6144 at 700 tokens 30.6 / 19.4).  A codebook that is gathered from L2 makes an expansion twice as
+// dear (2048x6144 at 400 30.4 / 28.7).  Narrower layers lose nothing (2048x2048 at 1,000 17.6 / 16.3, 6144x1536 30 / 37).
 int64_t tmem_min_m(const sacq_layer* L) {
-  return !split_k_codebook_in_smem(L) && L->d.out_features >= 4096 ? 384 : 1024;
+  if (L->d.out_features < 4096) return 1024;
+  return split_k_codebook_in_smem(L) ? 960 : 384;
 }
 
 // From how many tokens a split-K kernel, which walks the weights once, beats a small-M kernel, which walks them
 // once per 16-token chunk: from the second chunk on wide or deep layers, from the third on all but the smallest.
 // A codebook in L2 leaves the small-M kernel 2 warps' gathers in flight per scheduler: on wide layers the split-K
-// kernel wins from one token on (2048x6144, 65,536 entries: 17.8 / 13.4 us at 16 tokens, 46 / 15.6 at 64).
+// kernel wins from one token on (2048x6144, 65,536 entries: 17.8 / 13.4 us at 16 tokens, 46 / 15.6 at 64), on the
+// smallest from the third chunk on (2048x1024 at 32 tokens 8.3 / 9.3).
 bool split_wins(const sacq_layer* L, int64_t M) {
-  if (!split_k_codebook_in_smem(L)) return M > 16 || L->d.out_features >= 4096;
   const int64_t work = L->d.in_features * L->d.out_features;
+  if (!split_k_codebook_in_smem(L)) return M > (work <= (2 << 20) ? 32 : 16) || L->d.out_features >= 4096;
   return (M > 16 && (L->d.out_features >= 4096 || work >= (8 << 20))) || M > 32;
 }
 
@@ -104,9 +109,9 @@ int pick_kernel(const sacq_layer* L, int64_t M) {
   if (L->force_kernel == 1 || L->force_kernel >= 3)
     return small_m_supported(L) ? 1 : SACQ_ERR_UNSUPPORTED;
   if (L->force_kernel == 2) return large_m_supported(L) ? 2 : SACQ_ERR_UNSUPPORTED;
-  // A shape rule, not a backend switch.  The thresholds of the per-channel kernels do not depend on a layer's
-  // width as long as its codebook fits shared memory, so the row shards of a split layer run the kernel the whole
-  // layer would, and reproduce it bit for bit (the split-K kernel sums in an order that depends on K alone).
+  // A shape rule, not a backend switch.  The split-K kernel sums in an order that depends on K alone, so the row shards of
+  // a split per-channel layer reproduce the whole layer bit for bit where both run it, or both the persistent kernel:
+  // where a threshold depends on the width (17 to 32 tokens, 960 to 1,023, a codebook in L2) they may differ in the last bit.
   if (large_m_tmem_supported(L) && M >= tmem_min_m(L)) return 4;
   // Below, quantizer + GEMM of the small-M and the split-K kernel at 17 tokens: 1024x4096 10.9 / 6.8 us,
   // 6144x2048 15.4 / 11.5, 2048x6144 15.5 / 8.9; at 33: 1024x1024 7.3 / 5.7, 2048x2048 9.2 / 8.8, 4096x1024
