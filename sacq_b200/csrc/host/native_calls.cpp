@@ -9,8 +9,9 @@
 // Every function handles the plain case -- bf16 CUDA tensors of the layer's device with unit inner
 // stride, shapes that match -- and returns None otherwise without having launched anything; the
 // caller (linear.py, activation.py) then takes the general route, which converts what can be
-// converted and raises the errors.  Nothing here releases the GIL: the calls only enqueue work, and
-// holding it keeps the two launches of a forward together when two threads share a stream.
+// converted and raises the errors.  The calls only enqueue work and keep the GIL, which keeps the two
+// launches of a forward together when two threads share a stream.  forward_host releases it: a copy from
+// or to pageable memory waits for the stream, and a lock per scratch set keeps its launches together.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -23,6 +24,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <map>
+#include <mutex>
 #include <optional>
 #include <unordered_map>
 #include <utility>
@@ -40,6 +42,7 @@ struct Workspace {
   at::Tensor ws;            // zero-initialised: arrival counters lead, then kernel scratch
   at::Tensor q, scale;      // quantized activations of a forward
   at::Tensor host_scratch;  // everything a host-buffer forward needs on the device
+  std::mutex host_lock;     // ... and whose turn it is to use it; taken without the GIL only
 };
 
 std::map<std::pair<int, cudaStream_t>, Workspace>& pool() {
@@ -305,9 +308,19 @@ PyObject* layer_forward_host(LayerObject* L, PyObject* const* a, Py_ssize_t n) {
     Target at_(L->dev);
     w.host_scratch = zeroed(need > (1 << 22) ? need : (1 << 22), L->dev);
   }
-  // the library switches to the layer's device itself
-  const int rc = sacq_linear_bf16_host(L->handle, x->data_ptr(), m, y->data_ptr(), w.host_scratch.data_ptr(),
-                                       w.host_scratch.numel(), stream);
+  // the call's own references: another thread may let go of its tensors, or grow the scratch, meanwhile
+  const at::Tensor xt = *x, yt = *y, scratch_t = w.host_scratch;
+  const void* xp = xt.data_ptr();
+  void *yp = yt.data_ptr(), *sp = scratch_t.data_ptr();
+  const int64_t bytes = scratch_t.numel();
+  int rc;
+  Py_BEGIN_ALLOW_THREADS
+  {
+    std::lock_guard<std::mutex> turn(w.host_lock);
+    // the library switches to the layer's device itself
+    rc = sacq_linear_bf16_host(L->handle, xp, m, yp, sp, bytes, stream);
+  }
+  Py_END_ALLOW_THREADS
   if (rc != 0) return raise_status(rc);
   Py_INCREF(a[1]);
   return a[1];

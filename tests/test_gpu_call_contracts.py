@@ -288,3 +288,45 @@ def test_a_captured_call_gives_the_eager_bytes(N, K, d, C, G):
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(y, want), M
+
+
+def test_host_forward_leaves_other_threads_running():
+    """A result in pageable memory is copied by a call that waits for the stream: other Python threads run meanwhile.  And
+    threads that share a stream each get their own result."""
+    import threading
+    import time
+    mod = _layer(256, 512)
+    xs = [_x(40, 512, seed=i).cpu() for i in range(4)]
+    want = [mod(x.cuda()).cpu() for x in xs]
+    ticks, stop = [0], threading.Event()
+
+    def count():
+        while not stop.is_set():
+            time.sleep(0.001)
+            ticks[0] += 1
+    t = threading.Thread(target=count)
+    t.start()
+    torch.cuda.synchronize()
+    torch.cuda._sleep(400_000_000)                      # about 0.2 s of a busy stream
+    before = ticks[0]
+    y = mod.forward_host(xs[0])
+    during = ticks[0] - before
+    stop.set()
+    t.join()
+    torch.cuda.synchronize()
+    assert torch.equal(y, want[0]) and during >= 20, during
+
+    bad = []
+
+    def work(i):
+        for _ in range(50):
+            got = mod.forward_host(xs[i])
+            torch.cuda.current_stream().synchronize()
+            if not torch.equal(got, want[i]):
+                bad.append(i)
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
