@@ -258,7 +258,7 @@ SACQ_API int sacq_linear_a8_multi(const sacq_layer_t* const* layers, int num_lay
 
 /* Convenience: sacq_quant_act_fp8 + sacq_linear_a8 for a bf16 input (the module's
  * forward(x), SHIM:456-541).  `q_scratch` (M*K bytes) and `scale_scratch` (M floats)
- * are caller-provided device buffers. */
+ * are caller-provided device buffers, which hold the quantized activations afterwards. */
 SACQ_API int sacq_linear_bf16(const sacq_layer_t* layer, const void* x_bf16, int64_t x_pitch, int64_t M, void* q_scratch,
                      float* scale_scratch, void* y_out, int64_t ldy, void* workspace, int64_t workspace_bytes,
                      void* stream);

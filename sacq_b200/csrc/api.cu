@@ -799,8 +799,12 @@ int sacq_forward_call(const sacq_layer_t* L, const void* x_bf16, int64_t x_pitch
 SACQ_API int sacq_linear_bf16(const sacq_layer_t* L, const void* x_bf16, int64_t x_pitch, int64_t M, void* q_scratch,
                      float* scale_scratch, void* y_out, int64_t ldy, void* workspace, int64_t workspace_bytes,
                      void* stream) {
-  return sacq_forward_call(L, x_bf16, x_pitch, M, 0, nullptr, 0, q_scratch, scale_scratch, y_out, ldy, workspace,
-                           workspace_bytes, stream);
+  if (int rc = check_layer(L)) return rc;
+  if (M == 0) return SACQ_OK;
+  // the two calls it stands for: its caller finds the quantized activations in its scratch
+  const int rc = sacq_quant_act_fp8(x_bf16, x_pitch, M, L->d.in_features, q_scratch, scale_scratch, stream);
+  return rc != SACQ_OK ? rc
+                       : linear_a8_impl(L, q_scratch, scale_scratch, M, nullptr, 0, y_out, ldy, workspace, workspace_bytes, stream);
 }
 
 // Layout of the device scratch of sacq_linear_bf16_host: workspace first (its counter

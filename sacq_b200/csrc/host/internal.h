@@ -8,8 +8,9 @@
 extern "C" {
 #endif
 
-/* Quantizer + GEMM: sacq_linear_bf16 with an optional residual (bf16 [M, ldr], e4m3 activations only) or with
- * INT8 activations.  Scratch and workspace as for the separate calls. */
+/* Quantizer + GEMM with the bytes of the separate calls, optionally with a residual (bf16 [M, ldr], e4m3 activations
+ * only) or with INT8 activations.  Scratch and workspace as for those; what they hold afterwards is undefined (few
+ * tokens are quantized inside the GEMM, fp16 GEMMs take their activations as fp16). */
 SACQ_API int sacq_forward_call(const sacq_layer_t* layer, const void* x_bf16, int64_t x_pitch, int64_t M, int int8,
                                const void* residual, int64_t ldr, void* q_scratch, float* scale_scratch, void* y_out,
                                int64_t ldy, void* workspace, int64_t workspace_bytes, void* stream);

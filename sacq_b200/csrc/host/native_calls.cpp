@@ -201,8 +201,8 @@ PyObject* layer_forward(LayerObject* L, PyObject* x_obj) {
   at::Tensor& ws = scratch(w, need_bytes(L, r.m, kNeedA8), L->dev);
   act_buffers(w, r.m, L->k, L->dev);
   at::Tensor y = result_like(*x, r.m, L->n, L->dev);
-  const int rc = sacq_linear_bf16(L->handle, r.ptr, r.pitch, r.m, w.q.data_ptr(), (float*)w.scale.data_ptr(), y.data_ptr(),
-                                  L->n, ws.data_ptr(), ws.numel(), at_.stream);
+  const int rc = sacq_forward_call(L->handle, r.ptr, r.pitch, r.m, 0, nullptr, 0, w.q.data_ptr(), (float*)w.scale.data_ptr(),
+                                   y.data_ptr(), L->n, ws.data_ptr(), ws.numel(), at_.stream);
   return rc == 0 ? THPVariable_Wrap(std::move(y)) : raise_status(rc);
   NATIVE_CATCH
 }

@@ -330,3 +330,18 @@ def test_host_forward_leaves_other_threads_running():
     for t in threads:
         t.join()
     assert not bad
+
+
+@pytest.mark.parametrize("N,K,d,C,G,M", [(256, 1024, 8, 4096, None, 4), (256, 1024, 4, 256, 64, 300), (256, 1024, 8, 4096, None, 300)])
+def test_linear_bf16_leaves_the_quantized_activations(N, K, d, C, G, M):
+    """The C entry point is the quantizer and the GEMM in turn: its scratch holds what the first wrote."""
+    from sacq_b200 import _lib, quantize_rows
+    mod = _layer(N, K, d, C, G)
+    x = _x(M, K)
+    q, s = quantize_rows(x)
+    qs, ss = torch.full((M, K), 0x55, dtype=torch.uint8, device="cuda"), torch.full((M,), -1.0, device="cuda")
+    y, lib = torch.empty(M, N, dtype=torch.bfloat16, device="cuda"), mod._lib
+    ws = torch.zeros(int(lib.sacq_workspace_bytes(mod._handle, M)), dtype=torch.uint8, device="cuda")
+    _lib.check(lib.sacq_linear_bf16(mod._handle, x.data_ptr(), K, M, qs.data_ptr(), ss.data_ptr(), y.data_ptr(), N,
+                                    ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream))
+    assert torch.equal(y, mod(x)) and torch.equal(qs, q.view(torch.uint8)) and torch.equal(ss, s.reshape(-1))
