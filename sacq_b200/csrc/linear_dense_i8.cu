@@ -283,6 +283,7 @@ void dense_choose(const sacq_layer* L, int64_t M, int* subs, int* bn) {
   const int64_t kb = (L->d.in_features + kDBK - 1) / kDBK;
   double best = 1e30;
   for (const auto& t : tiles) {
+    if ((M + t.subs * kBM - 1) / (t.subs * kBM) > 65535 && t.subs == 1) continue;   // token tiles are the grid's second dimension
     const int64_t ctas = ((M + t.subs * kBM - 1) / (t.subs * kBM)) * ((L->d.out_features + t.bn - 1) / t.bn);
     const double sm = (double)((ctas + L->num_sms - 1) / L->num_sms) * (kb * t.block_us + t.tile_us);
     const double l2 = (double)ctas * kb * (t.subs * kBM + t.bn) * kDBK / 19e6 + 1.2;

@@ -345,3 +345,14 @@ def test_linear_bf16_leaves_the_quantized_activations(N, K, d, C, G, M):
     _lib.check(lib.sacq_linear_bf16(mod._handle, x.data_ptr(), K, M, qs.data_ptr(), ss.data_ptr(), y.data_ptr(), N,
                                     ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream))
     assert torch.equal(y, mod(x)) and torch.equal(qs, q.view(torch.uint8)) and torch.equal(ss, s.reshape(-1))
+
+
+def test_recipe_takes_more_tokens_than_the_small_tiles_can():
+    """8.4 to 16.7 million tokens: more tiles of 128 than a grid has, but not of 256."""
+    from sacq_b200 import quantize_rows
+    mod = _layer(64, 16, 8, 16)
+    M = 65535 * 128 + 77
+    sw = mod.weight_row_scale("int8_symmetric")
+    q, s = quantize_rows(_x(1 << 12, 16).repeat(M // (1 << 12) + 1, 1)[:M], "int8_symmetric")
+    y = mod.linear_w8a8_int8(q, s, sw)
+    assert torch.equal(y[-500:], mod.linear_w8a8_int8(q[-500:].contiguous(), s[-500:].contiguous(), sw))
