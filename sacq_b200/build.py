@@ -23,6 +23,7 @@ OBJ_DIR = os.path.join(HERE, "build")
 LIB_PATH = os.path.join(HERE, "libsacq_b200.so")
 NATIVE_SRC = os.path.join(CSRC, "host", "native_calls.cpp")
 NATIVE_PATH = os.path.join(HERE, "_native.so")
+NATIVE_KEY_PATH = os.path.join(OBJ_DIR, "native.key")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -56,11 +57,27 @@ def up_to_date() -> bool:
     return all(os.path.getmtime(p) <= t for p in _deps())
 
 
-def build_native(force: bool = False) -> str:
-    """Compile the extension module if its source or the public header is newer.  Returns its path."""
+def native_key() -> str:
+    """What a build of the extension module is bound to, besides its sources: one Python and one PyTorch."""
+    import torch
+    return f"{sys.version}\n{torch.__version__} {torch.version.git_version} {torch.compiled_with_cxx11_abi()}\n"
+
+
+def native_up_to_date() -> bool:
     deps = [NATIVE_SRC, os.path.join(CSRC, "host", "internal.h"), os.path.abspath(__file__)] + glob.glob(os.path.join(HERE, "..", "include", "*.h"))
-    if not force and os.path.exists(NATIVE_PATH) and \
-            all(os.path.getmtime(p) <= os.path.getmtime(NATIVE_PATH) for p in deps):
+    if not os.path.exists(NATIVE_PATH) or any(os.path.getmtime(p) > os.path.getmtime(NATIVE_PATH) for p in deps):
+        return False
+    try:
+        with open(NATIVE_KEY_PATH) as f:
+            return f.read() == native_key()
+    except OSError:
+        return False
+
+
+def build_native(force: bool = False) -> str:
+    """Compile the extension module if its source or the public header is newer, or if it was built for another Python or
+    PyTorch.  Returns its path."""
+    if not force and native_up_to_date():
         return NATIVE_PATH
     import sysconfig
 
@@ -76,6 +93,9 @@ def build_native(force: bool = False) -> str:
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError("g++ failed for %s:\n%s\n%s" % (NATIVE_SRC, res.stdout, res.stderr))
+    os.makedirs(OBJ_DIR, exist_ok=True)
+    with open(NATIVE_KEY_PATH, "w") as f:
+        f.write(native_key())
     return NATIVE_PATH
 
 

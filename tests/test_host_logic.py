@@ -184,3 +184,18 @@ def test_index_range_check():
         check_index_range(torch.tensor([0, 251], dtype=torch.int32), 251)
     with pytest.raises(IndexError):
         check_index_range(torch.tensor([-1, 2], dtype=torch.int32), 251)
+
+
+def test_native_module_is_rebuilt_for_another_python_or_torch(tmp_path, monkeypatch):
+    """The extension module is bound to one Python and one PyTorch, which its name does not carry."""
+    from sacq_b200 import build
+    so, key = tmp_path / "_native.so", tmp_path / "native.key"
+    monkeypatch.setattr(build, "NATIVE_PATH", str(so))
+    monkeypatch.setattr(build, "NATIVE_KEY_PATH", str(key))
+    assert not build.native_up_to_date()
+    so.write_bytes(b"")
+    assert not build.native_up_to_date()                # built before there were keys, or by hand
+    key.write_text(build.native_key())
+    assert build.native_up_to_date()
+    monkeypatch.setattr(torch, "__version__", "1.0.0")
+    assert not build.native_up_to_date()
