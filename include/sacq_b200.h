@@ -123,8 +123,9 @@ SACQ_API int64_t sacq_workspace_counter_bytes(void);
  *   y[m,n] = bf16( s[m] * sum_k q[m,k] * W[n,k]  + bias[n] )
  * q: e4m3 bytes [M, K]; scale: float [M]; y_out: bf16 [M, ldy] (ldy >= N elements).
  * Chooses the kernel from M and the layer geometry alone: warp-MMA kernels that gather
- * codewords straight into mma.sync fragments up to a few dozen rows, TMA + tcgen05 kernels
- * above that (expanded weight tiles in shared memory, or in tensor memory from 1024 rows);
+ * codewords straight into mma.sync fragments up to a few dozen rows, above that tcgen05 kernels
+ * that expand the weights into tensor memory (K split over clusters, persistent CTAs from about
+ * 1,000 rows);
  * a layer with a non-zero shift runs on the kernel that rebuilds the reference's two-rounding
  * reconstruction per weight. */
 SACQ_API int sacq_linear_a8(const sacq_layer_t* layer, const void* q, const float* scale, int64_t M, void* y_out,
@@ -153,10 +154,13 @@ SACQ_API int sacq_peer_buffer_destroy(int device, void* dev_ptr);
 /* INT8 per-token activations, the format of the reference's deployed recipe
  * (quantize_rows(x, 'int8_symmetric'), perrow_a8_candidate_r3.py:17-25):
  *   s = max|x| / 127 per row (1 for an all-zero row), q = int8(round_half_even(clamp(x / s, -127, 127))).
- * sacq_linear_a8i is sacq_linear_a8 for such activations: the same exact weights (no 8-bit
- * rounding of the weights, unlike the reference's INT8 GEMM), int8 widened to fp16 in front of
- * fp16 tensor-core MMAs (tcgen05 kind::f16 where the codebook and the token count favour it, warp MMAs below).  Its workspace is
- * sacq_workspace_bytes_int8(layer, M) bytes, 256-byte aligned, zero-filled once. */
+ * sacq_linear_a8i is sacq_linear_a8 for such activations: no 8-bit rounding of the weights, unlike
+ * the reference's INT8 GEMM; int8 widened to fp16 in front of fp16 MMAs.  The weights are exact up to
+ * 47 tokens, and at any number where the codebook does not fit shared memory; beyond they are
+ * codeword x scale with fp16's 11 significant bits, finer than the bf16 reconstruction.  (So are those
+ * of grouped scales in sacq_linear_a8, from 33, 48 or 96 tokens on layers of 4,736, 2,048 or fewer
+ * outputs.)  Its workspace is sacq_workspace_bytes_int8(layer, M) bytes, 256-byte aligned,
+ * zero-filled once. */
 SACQ_API int sacq_quant_act_int8(const void* x_bf16, int64_t x_pitch, int64_t M, int64_t K, void* q_out,
                                  float* scale_out, void* stream);
 SACQ_API int64_t sacq_workspace_bytes_int8(const sacq_layer_t* layer, int64_t M);
@@ -269,8 +273,8 @@ SACQ_API int sacq_linear_bf16(const sacq_layer_t* layer, const void* x_bf16, int
  * asynchronous) to the device, runs sacq_linear_bf16 and copies y (bf16 [M, N]) back, all
  * on `stream`, without synchronising.  When a host buffer is pinned (page-locked and mapped,
  * 16-byte aligned) and its transfer is at most 1 MiB, no copy engine is involved: the
- * quantizer kernel reads x from host memory directly and a copy kernel stores y to host
- * memory; the bytes crossing the bus are the same.  `dev_scratch` is caller-owned device memory of
+ * quantizer kernel reads x from host memory directly and the GEMM (rows of whole 128-byte lines)
+ * or a copy kernel stores y to host memory; the bytes crossing the bus are the same.  `dev_scratch` is caller-owned device memory of
  * sacq_host_forward_scratch_bytes(layer, M) bytes, 256-byte aligned, zero-filled once
  * before its first use; it may be reused by later calls on the same stream. */
 SACQ_API int sacq_linear_bf16_host(const sacq_layer_t* layer, const void* x_host, int64_t M, void* y_host,
@@ -299,8 +303,8 @@ SACQ_API int sacq_linear_a8_static_scratch(const sacq_layer_t* layer, const void
 SACQ_API int64_t sacq_static_scratch_bytes(void);
 
 /* Forces a GEMM kernel (for tests and benchmarks): 0 = automatic, 1 = small-M kernel
- * (its own choice of variant), 2 = tensor-core kernel that splits K over clusters, 3 = small-M CUDA-core variant, 4 = small-M warp-MMA variant, 5 = warp-MMA variant
- * without shared-memory staging, 6 = warp-MMA variant that unpacks the indices in shared memory
+ * (its own choice of variant), 2 = tensor-core kernel that splits K over clusters, 3 = small-M
+ * CUDA-core variant, 4 = small-M warp-MMA variant, 5 = warp-MMA variant without shared-memory staging, 6 = warp-MMA variant that unpacks the indices in shared memory
  * (any index width, any group size that is a multiple of 32), 7 = the split-K tensor-core
  * kernel for grouped scales, 8 = tensor-core kernel for batches, persistent CTAs (9, 10, 11: with
  * tiles of 128, 256, 384 tokens), 12 = that design for grouped scales (13, 14, 15: likewise).

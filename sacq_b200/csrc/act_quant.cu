@@ -124,13 +124,11 @@ quant_act_kernel(const uint16_t* __restrict__ x, int64_t pitch, int64_t K, uint8
   SACQ_TL(t_exit);
 }
 
-// The same quantizer for many rows: one WARP per row, eight rows per CTA, no block-wide barrier.  With
-// one CTA per row (above) a row's two phases are separated by two __syncthreads and 8,192 rows of
-// K = 2048 take 24 us against 8 us of HBM traffic; here a lane keeps its 16-byte chunks of the row
-// in registers across the warp reduction: 8 chunks of 8 elements per lane, i.e. rows of up to 2,048
-// elements.  Longer rows stay on the kernel above: keeping 24 chunks per lane costs 240 registers
-// and measured 77 us for 8,192 rows of 6,144 (re-reading the tail instead: 59 us) against 44 us
-// there.  Same arithmetic, same bytes.  Rows are 16-byte aligned, K % 8 == 0.
+// The same quantizer for many rows: one WARP per row, eight rows per CTA, no block-wide barrier.  A lane keeps its
+// 16-byte chunks of the row in registers across the warp reduction: 8 chunks of 8 elements, i.e. rows of up to 2,048
+// elements (8,192 rows of 2,048: 9.4 us, 7.7 of HBM time).  Longer rows stay on the kernel above: 24 chunks per lane
+// cost 240 registers, and reading the tail again was slower than a CTA per row too.  Same arithmetic, same bytes.  Rows
+// are 16-byte aligned, K % 8 == 0.
 constexpr int kRowsPerCta = 8;
 constexpr int kKeepChunks = 8;
 

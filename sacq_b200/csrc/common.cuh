@@ -12,7 +12,6 @@
 namespace sacq {
 
 constexpr float kE4M3Max = 448.0f;
-constexpr int kNumSMsB200 = 148;
 
 // ----------------------------------------------------------------------------
 // host side: the layer handle and error plumbing

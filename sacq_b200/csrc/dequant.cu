@@ -192,8 +192,9 @@ decode_weight_int8_kernel(const uint32_t* __restrict__ words, const uint16_t* __
 //
 // What bounds it: the one-thread-per-vector kernels above spend a 16-byte L1 gather (a tag lookup per lane: d = 4
 // took 25 us for 12.6 M weights), an index-to-row division and an IEEE division per weight (d = 8: 15 us).  Here
-// the gathers go to shared memory, the row's divisor is set up once, and the quotients are bracketed
-// (RowDivisor).  The int8 bound: |z| is clamped to RN(127 s) first, beyond which every quotient rounds to +-127.
+// the gathers go to shared memory, the row's divisor is set up once, and a quotient is two residual corrections of
+// z times its reciprocal (RowDivisor).  Weights are clamped first, to a bf16 value that encodes to the largest byte
+// (RowWeights), so that a caller's own row scale cannot overflow the quotient.
 constexpr int kSegSteps = 64;         // 16-weight steps of a row that a warp takes
 
 template <int D, bool I8, bool SMEM>

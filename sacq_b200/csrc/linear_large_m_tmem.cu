@@ -314,8 +314,8 @@ large_m_tmem_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         if (!ok) break;
         // the thread's quarter of the stage's k: WQ columns of the high half, WQ of the low half
         const uint32_t w_addr = lane_addr + (uint32_t)(kTmemCols - (ws + 1) * kWCols + kpart * WQ);
-        tmem_st_32xn(w_addr, hi);
-        tmem_st_32xn(w_addr + (uint32_t)(kWCols / 2), lo);
+        tmem_st_32x8(w_addr, hi);
+        tmem_st_32x8(w_addr + (uint32_t)(kWCols / 2), lo);
         if ((g & 1) == 1 && lane == 0) mbar_arrive(bar(IDX_EMPTY + ((g >> 1) & 1)));
         tmem_wait_st();
         tc_fence_before();

@@ -263,14 +263,6 @@ __device__ __forceinline__ void reduce_tokens(const SplitParams& p, const SplitL
   }
 }
 
-#ifdef SACQ_TRACE
-// Profiling builds only (-DSACQ_TRACE): CTA (0, 0, 0) records %globaltimer at a few points.
-__device__ long long g_split_trace[64];
-#define SACQ_SPT(slot) do { if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && (slot) < 64) { long long _t; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(_t)); g_split_trace[slot] = _t; } } while (0)
-#else
-#define SACQ_SPT(slot) do { } while (0)
-#endif
-
 // grid = (row tiles x split, token tiles, layers), clusters of `split` CTAs along x.
 template <int D, int MODE, bool CB_SMEM>
 __global__ void __launch_bounds__(kCtaThreads, 1)
@@ -284,7 +276,6 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   const int n0 = ((int)blockIdx.x / S) * kRows;
   const SplitLayer& lay = p.layer[blockIdx.z];
   if (n0 >= lay.N) return;                            // a narrower sibling: uniform over the cluster
-  if (threadIdx.x == 0) SACQ_SPT(0);
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -351,13 +342,11 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = warp_uniform(*tmem_slot);
-  if (threadIdx.x == 0) SACQ_SPT(1);
 
   bool ok = true;
   if (warp == 0) {
     // ------------------------------------------------------------------ activation tiles, token scales
     asm volatile("griddepcontrol.wait;" ::: "memory");   // q and the scales come from the kernel in front
-    if (lane == 0) SACQ_SPT(2);
     float sa[kMaxTok / 32];                           // the token scales: fetched now, put down behind the last copy
 #pragma unroll
     for (int i = 0; i < kMaxTok / 32; ++i) {
@@ -399,7 +388,6 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         ok = ok && mbar_wait_warp(bar(ACT_FULL + st), act_parity, abort_flag, lay.status);
         if (!ok) break;
         tc_fence_after();
-        if (lane == 0) SACQ_SPT(16 + wi * TILES + sub);
         const uint32_t act = base + (uint32_t)(st * tok * 128);
         const uint64_t b0 = make_smem_desc(act);
         const uint64_t b1 = make_smem_desc(act + (uint32_t)(tok / 2 * 128));
@@ -469,7 +457,6 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     // One answer per warp: what follows (tcgen05.st, its wait, __syncwarp) is the whole warp's.
     ok = mbar_wait_warp(bar(IDX_FULL), 0, abort_flag, lay.status) &&
          (!CB_SMEM || mbar_wait_warp(bar(CB_FULL), 0, abort_flag, lay.status));
-    if (et == 0) SACQ_SPT(3);
     int grp = 0, grp_end = GROUPS ? (g_first + 1) * p.group_size - kb0 * kStageK : 0;    // k (in the slice) at which the scale changes
     // One stage's 16 words of this thread.  The next stage's words are gathered before the wait for this
     // stage's tcgen05.st: the gathers, which bound the loop, then never wait for a store's latency.
@@ -605,9 +592,7 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         cur_s[1] = nxt_s[1];
       }
     }
-    if (et == 0) SACQ_SPT(4);
     if (ok) ok = mbar_wait_warp(bar(ACC_FULL), 0, abort_flag, lay.status);
-    if (et == 0) SACQ_SPT(5);
   }
 
   // ---- reduction: the accumulators of the cluster's CTAs -> y.  Every thread takes part in the barriers.
@@ -635,10 +620,8 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     }
     tc_fence_before();
   }
-  if (threadIdx.x == 64) SACQ_SPT(6);
   if (S > 1) cluster_sync();
   else __syncthreads();
-  if (threadIdx.x == 64) SACQ_SPT(7);
   if (warp >= 2 && ok) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int first = rank * owned_tokens(tok, S);    // the tokens this CTA writes
@@ -653,22 +636,14 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     else reduce_tokens<4, INT>(p, lay, warp - 2, lane, count, m0 + first, n0, part, sa, sw, bs);
   }
 
-  if (threadIdx.x == 64) SACQ_SPT(8);
   // ---- common exit: a CTA's partial sums stay until its peers have read them
   tc_fence_before();
   if (S > 1) cluster_sync();
   else __syncthreads();
-  if (threadIdx.x == 64) SACQ_SPT(9);
   if (warp == 1) tmem_dealloc(tmem_base, kTmemCols);
 }
 
 }  // namespace
-
-#ifdef SACQ_TRACE
-extern "C" SACQ_API int sacq_debug_split_trace(long long* out) {
-  return cudaMemcpyFromSymbol(out, g_split_trace, sizeof(g_split_trace)) == cudaSuccess ? 0 : -1;
-}
-#endif
 
 struct SplitPlan {
   static constexpr int kMaps = 8;

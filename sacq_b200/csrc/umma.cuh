@@ -60,10 +60,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 
 // One lane of a converged warp.  Instructions whose operands live in uniform registers (tcgen05.mma, TMA
 // copies) are issued as `if (elect_one()) ...` from code that the whole warp runs with warp-uniform
-// operands: inside a branch that only one lane takes, the compiler moves every operand into uniform
-// registers one by one for each instruction, which made an MMA cost about 120 clocks whatever its size.
-// Issued this way one with N columns takes N / 2 clocks (A in tensor memory; measured from N = 16 on),
-// and instructions that follow each other into one accumulator do not wait for each other.
+// operands.  Measured: an MMA issued inside a branch that only one lane takes cost about 120 clocks
+// whatever its size; issued this way one with N columns takes N / 2 clocks (A in tensor memory, from
+// N = 16 on), and instructions that follow each other into one accumulator do not wait for each other.
 __device__ __forceinline__ bool elect_one() {
   uint32_t r;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
