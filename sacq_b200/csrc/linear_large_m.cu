@@ -59,21 +59,6 @@ int encode_bytes_2d(CUtensorMap* map, const void* base, uint64_t row_bytes, uint
   return SACQ_OK;
 }
 
-int encode_bytes_3d(CUtensorMap* map, const void* base, uint64_t row_bytes, uint64_t rows, uint64_t dim2, uint64_t row_pitch,
-                    uint64_t dim2_pitch, uint32_t box_bytes, uint32_t box_rows, uint32_t box2) {
-  EncodeTiledFn fn = encode_tiled_fn();
-  if (fn == nullptr) return set_error(SACQ_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
-  const cuuint64_t dims[3] = {row_bytes, rows, dim2};
-  const cuuint64_t strides[2] = {row_pitch, dim2_pitch};
-  const cuuint32_t box[3] = {box_bytes, box_rows, box2};
-  const cuuint32_t estr[3] = {1, 1, 1};
-  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return set_error(SACQ_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
-  return SACQ_OK;
-}
-
 namespace {
 
 int sb_bytes_for(const sacq_layer* L) { return 2 * (kBK / L->d.vector_dim) * L->d.index_bits / 8; }

@@ -49,9 +49,10 @@ using namespace umma;
 using namespace tmemw;
 
 constexpr int kStageK = 128;          // k per weight stage
-constexpr int kMaxAct = 6;            // activation tiles in flight (128 bytes of every token each)
-constexpr int kMaxW = 4;              // weight stages in tensor memory
-constexpr int kSliceBytes = kRows * 16;
+constexpr int kMaxAct = 12;           // activation tiles in flight (128 bytes of every token each)
+constexpr int kMaxW = 7;              // weight stages in tensor memory
+constexpr int kBoxSlices = 4;         // 16-byte index slices per box (64 bytes of every row)
+constexpr int kBoxBytes = kRows * kBoxSlices * 16;
 // fp16 forms: K may end in the middle of a stage; its second 64-k tile is then zeros on both sides.
 __host__ __device__ constexpr int stages_of(int64_t K) { return (int)((K + kStageK - 1) / kStageK); }
 __host__ __device__ constexpr int w_cols(int mode) { return mode == kSplitHalf2 ? 128 : mode >= kSplitInt8 ? 32 : 64; }
@@ -70,44 +71,55 @@ struct SplitLayer {
   float out_mul;                // power of two that undoes the operands' scaling
 };
 
+// What a CTA's start depends on comes first: kernel parameters are read through a cache that is cold in every launch, a miss
+// per line.
 struct alignas(64) SplitParams {
-  CUtensorMap idx[kSplitMaxLayers];     // [16 bytes][128 rows][max_slices] boxes over the packed rows
-  SplitLayer layer[kSplitMaxLayers];
-  const float* act_scale;       // [M]
-  const float* row_scale;       // recipes: [N], the weight bytes' scale (the caller's buffer, not a layer constant)
+  int split;                    // CTAs per cluster
+  int parts;                    // consecutive slices of K per CTA, each with accumulator columns of its own
+  int tok;                      // tokens per CTA (multiple of 16; of 32 above 256)
+  int M, K, C, bits, num_groups, group_size;
+  int act_stages, max_slices, max_groups;
+  int own_recv;                 // the partial sums of the cluster have shared memory of their own
   uint16_t shift;               // recipes: bf16 bits
+  const float* act_scale;       // [M]
+  SplitLayer layer[kSplitMaxLayers];
+  CUtensorMap idx[kSplitMaxLayers];     // [64 bytes][128 rows] boxes over the packed rows, SWIZZLE_64B
+  const float* row_scale;       // recipes: [N], the weight bytes' scale (the caller's buffer, not a layer constant)
   const uint16_t* residual;     // bf16 [M, ldr] added to the rounded output, or null
   int64_t ldr;
   int n_bc;                     // further copies of the output (peer GPUs' buffers), same pitch as y
   uint16_t* ybc[kMaxBcast];
-  int M, K, C, bits, num_groups, group_size;
-  int split;                    // CTAs per cluster
-  int parts;                    // consecutive slices of K per CTA, each with accumulator columns of its own
-  int tok;                      // tokens per CTA (multiple of 16; of 32 above 256)
-  int act_stages, max_slices, max_groups;
 };
 
+// mbarriers of a CTA
+constexpr int ACT_FULL = 0, ACT_EMPTY = kMaxAct, W_FULL = 2 * kMaxAct, W_EMPTY = W_FULL + kMaxW, IDX_FULL = W_EMPTY + kMaxW,
+              CB_FULL = IDX_FULL + 2, ACC_FULL = CB_FULL + 1, RECV = ACC_FULL + 1, kBarriers = RECV + 1;
+
 struct SplitLayout {
-  uint32_t idx_off, cb_off, sc_off, fixed_off, sa_off, sw_off, bias_off, bar_off, misc_off, total;
+  uint32_t idx_off, cb_off, sc_off, recv_off, fixed_off, sa_off, sw_off, bias_off, bar_off, misc_off, total;
 };
 
 // tokens of the tile a rank reduces and writes
 __host__ __device__ constexpr int owned_tokens(int tok, int split) { return ((tok + split - 1) / split + 7) & ~7; }
 
-__host__ __device__ inline SplitLayout split_layout(int tok, int split, int act_stages, int slices, int groups, int cb_bytes) {
+__host__ __device__ constexpr int index_boxes(int slices) { return (slices + kBoxSlices - 1) / kBoxSlices; }
+
+__host__ __device__ inline SplitLayout split_layout(int tok, int split, int act_stages, int slices, int groups, int cb_bytes,
+                                                    bool own_recv) {
   SplitLayout L;
-  L.idx_off = (uint32_t)(act_stages * tok * 128);
-  L.cb_off = L.idx_off + (uint32_t)(slices * kSliceBytes);
+  L.idx_off = (uint32_t)((act_stages * tok * 128 + 1023) & ~1023);
+  L.cb_off = L.idx_off + (uint32_t)(index_boxes(slices) * kBoxBytes);
   L.sc_off = L.cb_off + (uint32_t)((cb_bytes + 127) & ~127);
   const uint32_t pipe = L.sc_off + (uint32_t)((groups > 0 ? kRows * (groups | 1) * 2 + 127 : 0) & ~127);
-  // the partial sums of the reduction take the place of everything the main loop is done with
-  const uint32_t recv = (uint32_t)(tok * kRows * 4);
-  L.fixed_off = pipe > recv ? pipe : recv;
+  // the partial sums: [source CTA][owned token][row] of a cluster, or of a CTA alone [token][row]
+  const uint32_t recv = (uint32_t)((split > 1 ? split * owned_tokens(tok, split) : tok) * kRows * 4);
+  L.recv_off = own_recv ? pipe : 0u;
+  L.fixed_off = own_recv ? pipe + recv : pipe > recv ? pipe : recv;
   L.sa_off = L.fixed_off;
   L.sw_off = L.sa_off + (uint32_t)(tok * 4);
   L.bias_off = L.sw_off + kRows * 4;
   L.bar_off = L.bias_off + kRows * 4;
-  L.misc_off = L.bar_off + 32 * 8;
+  L.misc_off = L.bar_off + kBarriers * 8;
   L.total = L.misc_off + 64;
   return L;
 }
@@ -122,19 +134,39 @@ __device__ __forceinline__ uint32_t peer_address(uint32_t addr, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
   return r;
 }
+__device__ __forceinline__ void store_peer(uint32_t addr, uint32_t v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+// Arrival at another CTA's mbarrier, behind this thread's stores into that CTA's shared memory (and those ordered before).
+__device__ __forceinline__ void mbar_arrive_peer(uint32_t addr) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+// Acquires, at cluster scope, what the arrivals of a completed phase released.
+__device__ __forceinline__ void mbar_acquire_cluster(uint32_t bar, uint32_t parity) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%0], %1;\n\t}"
+      ::"r"(bar), "r"(parity)
+      : "memory");
+}
+__device__ __forceinline__ uint4 load_shared(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+  return v;
+}
 __device__ __forceinline__ uint4 load_peer(uint32_t addr) {
   uint4 v;
   asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
   return v;
 }
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-      ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar)
-      : "memory");
-}
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// Both barriers, by a whole converged warp: one vote where both phases are complete already.
+__device__ __forceinline__ bool mbar_wait_two(uint32_t b0, uint32_t p0, uint32_t b1, uint32_t p1, volatile int* abort_flag, int* status) {
+  const bool r0 = mbar_try_wait(b0, p0), r1 = mbar_try_wait(b1, p1);
+  if (__all_sync(0xffffffffu, r0 && r1)) return true;
+  return mbar_wait_warp(b0, p0, abort_flag, status) && mbar_wait_warp(b1, p1, abort_flag, status);
 }
 // 16 accumulator columns of the warp's lane quarter.
 __device__ __forceinline__ void tmem_ld_16(uint32_t taddr, uint32_t (&r)[16]) {
@@ -165,13 +197,17 @@ __device__ __forceinline__ void add_columns(uint32_t (&r)[16], uint32_t taddr) {
   for (int j = 0; j < 16; ++j) r[j] = add_bits<INT>(r[j], b[j]);
 }
 
-// A window of up to 64 bits at bit `bit` of a row whose 16-byte slices lie kSliceBytes apart; `bit` is
-// warp-uniform, `need` bits of it are used (a slice is only read if one of them lies in it).
-__device__ __forceinline__ uint64_t slice_window(const uint8_t* row_slices, int bit, int need) {
-  const uint8_t* s0 = row_slices + (bit >> 7) * kSliceBytes;
-  const uint4 a = *reinterpret_cast<const uint4*>(s0);
+// The 16-byte slice `s` (warp-uniform) of a row in the index boxes: 64 bytes of every row per box, laid out by SWIZZLE_64B,
+// so the slices of eight consecutive rows lie on different banks.  at: the row's first byte; swizzle: its ((row / 2) & 3) * 16.
+__device__ __forceinline__ uint4 index_slice(const uint8_t* at, uint32_t swizzle, int s) {
+  return *reinterpret_cast<const uint4*>(at + (s >> 2) * kBoxBytes + ((uint32_t)((s & 3) << 4) ^ swizzle));
+}
+// A window of up to 64 bits at bit `bit` of a row; `bit` is warp-uniform, `need` bits of it are used (a slice is only
+// read if one of them lies in it).
+__device__ __forceinline__ uint64_t slice_window(const uint8_t* at, uint32_t swizzle, int bit, int need) {
+  const uint4 a = index_slice(at, swizzle, bit >> 7);
   uint4 b = a;
-  if ((bit & 127) + need > 128) b = *reinterpret_cast<const uint4*>(s0 + kSliceBytes);
+  if ((bit & 127) + need > 128) b = index_slice(at, swizzle, (bit >> 7) + 1);
   uint32_t lo, mid, hi;
   switch ((bit >> 5) & 3) {
     case 0: lo = a.x; mid = a.y; hi = a.z; break;
@@ -184,18 +220,19 @@ __device__ __forceinline__ uint64_t slice_window(const uint8_t* row_slices, int 
 }
 
 // Adds the slices of K pairwise, (0 + 1) + (2 + 3) and so on, whichever CTA does it, and writes y: tokens [0, count) of this CTA's share,
-// a warp per token, four consecutive outputs per lane.  `part` = this lane's partial sums of token 0 in the
-// CTA's own shared memory.  Everything that does not depend on the token is set up once: this loop is bound by
+// a warp per token, four consecutive outputs per lane.  `part` = this lane's partial sums of token 0 in the CTA's own
+// shared memory; those of the other CTAs are `stride` bytes apart, or (PEER) at the same place in theirs.  Everything that does not depend on the token is set up once: this loop is bound by
 // instruction issue (with the addresses and alignment tests inside it took 0.4 us per token and warp).
-template <int S, bool INT>
+template <int S, bool INT, bool PEER>
 __device__ __forceinline__ void reduce_tokens(const SplitParams& p, const SplitLayer& lay, int warp, int lane, int count,
-                                              int m_first, int n0, uint32_t part, const float* sa, float4 sw, float4 bs) {
+                                              int m_first, int n0, uint32_t part, uint32_t stride, const float* sa, float4 sw,
+                                              float4 bs) {
   const int n = n0 + lane * 4;
   const int valid = min(4, lay.N - n);
   if (valid <= 0) return;
   uint32_t src[S];
 #pragma unroll
-  for (int s = 0; s < S; ++s) src[s] = S == 1 ? part : peer_address(part, (uint32_t)s);
+  for (int s = 0; s < S; ++s) src[s] = PEER ? peer_address(part, (uint32_t)s) : part + (uint32_t)s * stride;
   uint16_t* y = lay.y + (int64_t)m_first * lay.ldy + n;
   const int64_t ldy = lay.ldy;
   const uint16_t* res = p.residual ? p.residual + (int64_t)m_first * p.ldr + n : nullptr;
@@ -209,7 +246,7 @@ __device__ __forceinline__ void reduce_tokens(const SplitParams& p, const SplitL
   for (int t = warp; t < count; t += kXWarps) {
     uint4 v[S];
 #pragma unroll
-    for (int s = 0; s < S; ++s) v[s] = load_peer(src[s] + (uint32_t)(t * (kRows * 4)));
+    for (int s = 0; s < S; ++s) v[s] = PEER ? load_peer(src[s] + (uint32_t)(t * (kRows * 4))) : load_shared(src[s] + (uint32_t)(t * (kRows * 4)));
 #pragma unroll
     for (int w = 1; w < S; w *= 2)
 #pragma unroll
@@ -283,11 +320,8 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   uint8_t* sm = smem_raw + (base - raw);
   const uint32_t cb_bytes = (uint32_t)(p.C * CW_BYTES);
   const SplitLayout L = split_layout(p.tok, S, p.act_stages, p.max_slices, F16 || RECIPE ? p.max_groups : 0,
-                                     CB_SMEM ? (int)cb_bytes : 0);
+                                     CB_SMEM ? (int)cb_bytes : 0, p.own_recv != 0);
 
-  constexpr int ACT_FULL = 0, ACT_EMPTY = kMaxAct, W_FULL = 2 * kMaxAct, W_EMPTY = W_FULL + kMaxW, IDX_FULL = W_EMPTY + kMaxW,
-                CB_FULL = IDX_FULL + 1, ACC_FULL = IDX_FULL + 2;
-  static_assert(ACC_FULL < 32, "barrier region");
   const uint32_t bars = base + L.bar_off;
   auto bar = [&](int i) { return bars + 8u * i; };
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + L.misc_off);
@@ -308,44 +342,49 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   const int bit_begin = (kb0 * kStageK / D) * p.bits;
   const int slice0 = bit_begin >> 7;
 
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < kMaxAct; ++i) {
-      mbar_init(bar(ACT_FULL + i), 1);
-      mbar_init(bar(ACT_EMPTY + i), 1);
-    }
-    for (int i = 0; i < kMaxW; ++i) {
-      mbar_init(bar(W_FULL + i), kXWarps);
-      mbar_init(bar(W_EMPTY + i), 1);
-    }
-    mbar_init(bar(IDX_FULL), 1);
-    mbar_init(bar(CB_FULL), 1);
-    mbar_init(bar(ACC_FULL), 1);
-    *abort_flag = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    fence_proxy_async();
-  }
+  const int boxes = index_boxes(p.max_slices), first_boxes = min(boxes, 2);
+  auto load_indices = [&](int from, int to, uint32_t full) {
+    mbar_arrive_expect_tx(full, (uint32_t)((to - from) * kBoxBytes));
+    for (int i = from; i < to; ++i)
+      tma_load_2d(base + L.idx_off + (uint32_t)(i * kBoxBytes), &p.idx[blockIdx.z], (slice0 + i * kBoxSlices) * 16, n0, full);
+  };
   if (warp == 0) {
-    __syncwarp();
-    // constant operands: their copies start before anything else
+    // constant operands: their copies start before anything else, those that the first stage needs first
     if (elect_one()) {
-      mbar_arrive_expect_tx(bar(IDX_FULL), (uint32_t)(p.max_slices * kSliceBytes));
-      tma_load_3d(base + L.idx_off, &p.idx[blockIdx.z], 0, n0, slice0, bar(IDX_FULL));
+      for (int i = 0; i < 3; ++i) mbar_init(bar(IDX_FULL + i), 1);
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      fence_proxy_async();
+      load_indices(0, first_boxes, bar(IDX_FULL));
       if constexpr (CB_SMEM) {
         mbar_arrive_expect_tx(bar(CB_FULL), cb_bytes);
         bulk_load(base + L.cb_off, lay.cb, cb_bytes, bar(CB_FULL));
       }
-      prefetch_tensormap(&tmap_a);
     }
+  } else if (warp == 2) {
+    for (int i = lane; i < kBarriers; i += 32)
+      if (i < IDX_FULL || i > CB_FULL) mbar_init(bar(i), i >= W_FULL && i < W_EMPTY ? kXWarps : i == RECV ? kXWarps * S + 1 : 1);
+    if (lane == 0) *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    fence_proxy_async();
   }
+  static_assert(CB_FULL == IDX_FULL + 2, "warp 0 makes these three");
   if (warp == 1) tmem_alloc(smem_u32(tmem_slot), kTmemCols);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = warp_uniform(*tmem_slot);
+  // Where the partial sums have a place of their own, peers may write theirs there from now on.
+  if (S > 1 && p.own_recv) cluster_arrive_relaxed();   // the mbarriers are released by their fence
 
   bool ok = true;
   if (warp == 0) {
     // ------------------------------------------------------------------ activation tiles, token scales
+    if (elect_one()) {
+      if (boxes > first_boxes) load_indices(first_boxes, boxes, bar(IDX_FULL + 1));
+      prefetch_tensormap(&tmap_a);
+    }
+    __syncwarp();
+    if (S > 1 && p.own_recv) cluster_wait();
     asm volatile("griddepcontrol.wait;" ::: "memory");   // q and the scales come from the kernel in front
     float sa[kMaxTok / 32];                           // the token scales: fetched now, put down behind the last copy
 #pragma unroll
@@ -356,7 +395,7 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     int st = 0;
     uint32_t free_parity = 1;
     for (int i = 0; i < kbs * TILES; ++i) {
-      if (!mbar_wait_warp(bar(ACT_EMPTY + st), free_parity, abort_flag, lay.status)) break;
+      if (i >= act_stages && !mbar_wait_warp(bar(ACT_EMPTY + st), free_parity, abort_flag, lay.status)) break;
       const uint32_t dst = base + (uint32_t)(st * tok * 128);
       const int x = (kb0 * TILES + i) * 128;
       if (elect_one()) {
@@ -369,34 +408,43 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 #pragma unroll
     for (int i = 0; i < kMaxTok / 32; ++i)
       if (i * 32 + lane < tok) reinterpret_cast<float*>(sm + L.sa_off)[i * 32 + lane] = sa[i];
+    // every copy has landed before a peer writes there or the CTA ends
+    mbar_wait_warp(bar(IDX_FULL), 0, abort_flag, lay.status);
+    if (boxes > first_boxes) mbar_wait_warp(bar(IDX_FULL + 1), 0, abort_flag, lay.status);
+    if (CB_SMEM) mbar_wait_warp(bar(CB_FULL), 0, abort_flag, lay.status);
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar(RECV));            // the token scales are in place (S > 1 and nothing sent: no one waits)
+    __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     const uint32_t idesc = INT ? make_idesc_i8(halves ? tok / 2 : tok) : make_idesc(halves ? tok / 2 : tok);
     int st = 0, ws = 0;
     uint32_t act_parity = 0, w_parity = 0;
     int part = -1, next_part = 0, begin = 0;          // slice of K, the stage at which the next one begins
+    if (S > 1 && p.own_recv) cluster_wait();
     for (int wi = 0; wi < kbs && ok; ++wi) {
       if (wi == next_part) {
         begin = wi;
         next_part = ++part + 1 < parts ? part_begin(part + 1) : kbs;
       }
-      ok = mbar_wait_warp(bar(W_FULL + ws), w_parity, abort_flag, lay.status);
       const uint32_t w_col = tmem_base + (uint32_t)(acc_cols + ws * W_COLS);
       const uint32_t d_col = tmem_base + (uint32_t)(part * tok);
 #pragma unroll
       for (int sub = 0; sub < TILES; ++sub) {
-        ok = ok && mbar_wait_warp(bar(ACT_FULL + st), act_parity, abort_flag, lay.status);
+        ok = sub == 0 ? mbar_wait_two(bar(W_FULL + ws), w_parity, bar(ACT_FULL + st), act_parity, abort_flag, lay.status)
+                      : mbar_wait_warp(bar(ACT_FULL + st), act_parity, abort_flag, lay.status);
         if (!ok) break;
         tc_fence_after();
         const uint32_t act = base + (uint32_t)(st * tok * 128);
         const uint64_t b0 = make_smem_desc(act);
         const uint64_t b1 = make_smem_desc(act + (uint32_t)(tok / 2 * 128));
+        const uint32_t fresh = (uint32_t)(((wi - begin) | sub) != 0);
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) {              // 32 bytes of every token per step
 #pragma unroll
           for (int h = 0; h < (MODE == kSplitHiLo || PAIR ? 2 : 1); ++h) {       // high and low halves of the weights
             const uint32_t a = w_col + (F16 ? (uint32_t)(h * 64 + sub * 32 + ks * 8) : (uint32_t)(h * 32 + ks * 8));
-            const uint32_t acc = (uint32_t)(((wi - begin) | sub | ks | h) != 0);
+            const uint32_t acc = ks == 0 && h == 0 ? fresh : 1u;
             const uint64_t adv = (uint64_t)(ks * 2);
             if (elect_one()) {
               if constexpr (F16) umma_f16_ts(d_col, a, b0 + adv, idesc, acc);
@@ -410,10 +458,11 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             }
           }
         }
-        if (elect_one()) umma_commit(bar(ACT_EMPTY + st));
+        // a stage that is not filled again needs no word that it is free
+        if (wi * TILES + sub + act_stages < kbs * TILES && elect_one()) umma_commit(bar(ACT_EMPTY + st));
+        if (sub == TILES - 1 && wi + w_stages < kbs && elect_one()) umma_commit(bar(W_EMPTY + ws));
         if (++st == act_stages) { st = 0; act_parity ^= 1; }
       }
-      if (ok && elect_one()) umma_commit(bar(W_EMPTY + ws));
       if (++ws == w_stages) { ws = 0; w_parity ^= 1; }
     }
     if (ok && elect_one()) umma_commit(bar(ACC_FULL));
@@ -451,12 +500,15 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     auto codeword8 = [&](uint32_t i) {
       return CB_SMEM ? *reinterpret_cast<const uint2*>(cbs + i * 8) : __ldg(reinterpret_cast<const uint2*>(cbs) + i);
     };
-    const uint8_t* rowidx = sm + L.idx_off + row * 16;
+    const uint8_t* rowidx = sm + L.idx_off + row * (kBoxSlices * 16);
+    const uint32_t swz = (uint32_t)((row >> 1) & 3) << 4;
     const uint32_t mask = (1u << p.bits) - 1u;
     const int bits = p.bits;
     // One answer per warp: what follows (tcgen05.st, its wait, __syncwarp) is the whole warp's.
     ok = mbar_wait_warp(bar(IDX_FULL), 0, abort_flag, lay.status) &&
          (!CB_SMEM || mbar_wait_warp(bar(CB_FULL), 0, abort_flag, lay.status));
+    // the first stage whose indices reach beyond the first boxes
+    const int late = boxes == first_boxes ? kbs : ((slice0 + first_boxes * kBoxSlices) * 128 - bit_begin) / (kStageK / D * bits);
     int grp = 0, grp_end = GROUPS ? (g_first + 1) * p.group_size - kb0 * kStageK : 0;    // k (in the slice) at which the scale changes
     // One stage's 16 words of this thread.  The next stage's words are gathered before the wait for this
     // stage's tcgen05.st: the gathers, which bound the loop, then never wait for a store's latency.
@@ -471,6 +523,8 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     const float row_mul = PAIR ? __ldg(lay.row_mul + min(n0 + row, lay.N - 1)) : 1.f;
     const float scale_mul = PAIR ? 1.f / row_mul : lay.scale_mul;       // a power of two
     auto expand = [&](int wi, uint32_t (&w)[16], __half2 (&sc2)[2]) {
+      if (wi == late) ok = ok && mbar_wait_warp(bar(IDX_FULL + 1), 0, abort_flag, lay.status);
+      if (!ok) return;
       if constexpr (RECIPE) {
         // 32 weights of this thread's row, 16 at a time: bf16(bf16(c * s) + shift) divided by the row scale and
         // encoded (the arithmetic of decode_rows_kernel in dequant.cu)
@@ -480,7 +534,7 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
           const int k = wi * kStageK + kpart * 32 + h * 16;       // in the slice
           const int g = p.num_groups == 1 ? 0 : (kb0 * kStageK + k) / p.group_size - g_first;
           const __nv_bfloat16 s = __ushort_as_bfloat16(sc[row * sc_pitch + g]);
-          const uint64_t win = slice_window(rowidx, ((kb0 * kStageK + k) / D) * bits - slice0 * 128, IPT * bits);
+          const uint64_t win = slice_window(rowidx, swz, ((kb0 * kStageK + k) / D) * bits - slice0 * 128, IPT * bits);
           uint32_t pair[8];
 #pragma unroll
           for (int j = 0; j < IPT; ++j) {
@@ -510,7 +564,7 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
           const __half2 s2 = __half2half2(__float2half_rn(bf16_bits_to_float(sc[row * sc_pitch + grp]) * scale_mul));
           sc2[sub] = s2;
           const int bit = (((kb0 + wi) * kStageK + sub * 64 + kpart * 16) / D) * bits - slice0 * 128;
-          const uint64_t win = slice_window(rowidx, bit, IPT * bits);
+          const uint64_t win = slice_window(rowidx, swz, bit, IPT * bits);
 #pragma unroll
           for (int j = 0; j < IPT; ++j) {
             const uint32_t i = (uint32_t)(win >> (j * bits)) & mask;
@@ -533,7 +587,7 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         const int bit = (((kb0 + wi) * kStageK + kpart * 32) / D) * bits - slice0 * 128;
 #pragma unroll
         for (int v = 0; v < 8 / D; ++v) {             // four indices per window
-          const uint64_t win = slice_window(rowidx, bit + v * 4 * bits, 4 * bits);
+          const uint64_t win = slice_window(rowidx, swz, bit + v * 4 * bits, 4 * bits);
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const uint32_t i = (uint32_t)(win >> (j * bits)) & mask;
@@ -554,11 +608,15 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     uint32_t w_parity = 1;
     uint32_t cur[16], nxt[16];
     __half2 cur_s[2], nxt_s[2];
-    if (ok) expand(0, cur, cur_s);
+    expand(0, cur, cur_s);
+    __syncwarp();
+    if (S > 1 && p.own_recv) cluster_wait();
     for (int wi = 0; wi < kbs && ok; ++wi) {
-      ok = mbar_wait_warp(bar(W_EMPTY + ws), w_parity, abort_flag, lay.status);
-      if (!ok) break;
-      tc_fence_after();                               // the MMAs that read this stage are complete
+      if (wi >= w_stages) {
+        ok = mbar_wait_warp(bar(W_EMPTY + ws), w_parity, abort_flag, lay.status);
+        if (!ok) break;
+        tc_fence_after();                             // the MMAs that read this stage are complete
+      }
       // two quarters of the stage: high and low halves, or the two 64-k tiles
       const uint32_t w_addr = lane_addr + (uint32_t)(acc_cols + ws * W_COLS + kpart * 8);
       if constexpr (PAIR) {
@@ -595,14 +653,17 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     if (ok) ok = mbar_wait_warp(bar(ACC_FULL), 0, abort_flag, lay.status);
   }
 
-  // ---- reduction: the accumulators of the cluster's CTAs -> y.  Every thread takes part in the barriers.
+  // ---- reduction: the accumulators of the cluster's CTAs -> y.  Every thread takes part in the cluster barrier.
+  const int own = owned_tokens(tok, S);
+  const bool send = S > 1 && p.own_recv, fetch = S > 1 && !send;   // fetch: a CTA keeps its partial sums, its peers read them
   if (warp >= 2 && ok) {
-    // [token][row] fp32, in the place of everything the main loop is done with (its last MMA has completed, so
-    // every stage has been written and read); a warp writes 128 consecutive bytes per token
+    // [token][row] fp32 into the shared memory of the CTA that owns the token, or the own; a warp writes 128 consecutive
+    // bytes per token.  (The main loop's last MMA has completed, so every stage has been written and read.)
     const int quarter = warp & 3, row = quarter * 32 + lane, kpart = (warp - 2) >> 2;
     const float row_mul = PAIR ? __ldg(lay.row_mul + min(n0 + row, lay.N - 1)) : 1.f;
+    const int tokens = min(tok, p.M - m0);
     tc_fence_after();
-    for (int c0 = kpart * 16; c0 < tok; c0 += 64) {
+    for (int c0 = kpart * 16; c0 < tokens; c0 += 64) {
       const uint32_t at = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0;
       uint32_t r[16];
       tmem_ld_16(at, r);
@@ -614,66 +675,94 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 #pragma unroll
         for (int j = 0; j < 16; ++j) r[j] = add_bits<INT>(r[j], r2[j]);
       }
-      uint32_t* dst = reinterpret_cast<uint32_t*>(sm) + c0 * kRows + row;
 #pragma unroll
-      for (int j = 0; j < 16; ++j) dst[j * kRows] = PAIR ? __float_as_uint(__uint_as_float(r[j]) * row_mul) : r[j];
+      for (int h = 0; h < 2; ++h) {                   // eight tokens have one owner
+        const int t = c0 + h * 8, owner = send ? t / own : rank;
+        const uint32_t dst = base + L.recv_off + (uint32_t)(((send ? rank * own + t - owner * own : t) * kRows + row) * 4);
+        if (owner == rank) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const uint32_t v = PAIR ? __float_as_uint(__uint_as_float(r[h * 8 + j]) * row_mul) : r[h * 8 + j];
+            asm volatile("st.shared.u32 [%0], %1;" ::"r"(dst + (uint32_t)(j * kRows * 4)), "r"(v) : "memory");
+          }
+        } else {
+          const uint32_t peer = peer_address(dst, (uint32_t)owner);
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            store_peer(peer + (uint32_t)(j * kRows * 4), PAIR ? __float_as_uint(__uint_as_float(r[h * 8 + j]) * row_mul) : r[h * 8 + j]);
+        }
+      }
     }
     tc_fence_before();
+    __syncwarp();
+    if (!fetch && lane < S) mbar_arrive_peer(peer_address(bar(RECV), (uint32_t)lane));
   }
-  if (S > 1) cluster_sync();
-  else __syncthreads();
+  __syncwarp();
+  if (fetch) {
+    cluster_arrive();
+    cluster_wait();
+  }
   if (warp >= 2 && ok) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int first = rank * owned_tokens(tok, S);    // the tokens this CTA writes
-    const int count = min(owned_tokens(tok, S), min(tok, p.M - m0) - first);
-    const float* sa = reinterpret_cast<const float*>(sm + L.sa_off) + first;
-    const float4 sw = reinterpret_cast<const float4*>(sm + L.sw_off)[lane];
-    const float4 bs = reinterpret_cast<const float4*>(sm + L.bias_off)[lane];
-    const uint32_t part = base + (uint32_t)(first * (kRows * 4) + lane * 16);
-    if (S == 1) reduce_tokens<1, INT>(p, lay, warp - 2, lane, count, m0 + first, n0, part, sa, sw, bs);
-    else if (S == 2) reduce_tokens<2, INT>(p, lay, warp - 2, lane, count, m0 + first, n0, part, sa, sw, bs);
-    else if (S == 8) reduce_tokens<8, INT>(p, lay, warp - 2, lane, count, m0 + first, n0, part, sa, sw, bs);
-    else reduce_tokens<4, INT>(p, lay, warp - 2, lane, count, m0 + first, n0, part, sa, sw, bs);
+    if (!fetch) ok = mbar_wait_warp(bar(RECV), 0, abort_flag, lay.status);
+    if (ok) {
+      if (!fetch) mbar_acquire_cluster(bar(RECV), 0);
+      asm volatile("griddepcontrol.wait;" ::: "memory");
+      const int first = rank * own;                   // the tokens this CTA writes
+      const int count = min(own, min(tok, p.M - m0) - first);
+      const float* sa = reinterpret_cast<const float*>(sm + L.sa_off) + first;
+      const float4 sw = reinterpret_cast<const float4*>(sm + L.sw_off)[lane];
+      const float4 bs = reinterpret_cast<const float4*>(sm + L.bias_off)[lane];
+      const uint32_t stride = (uint32_t)(own * kRows * 4);
+      const uint32_t part = base + L.recv_off + (uint32_t)(lane * 16) + (send ? 0u : (uint32_t)rank * stride);
+      auto reduce = [&](auto slices) {
+        constexpr int kS = decltype(slices)::value;
+        if (kS > 1 && fetch) reduce_tokens<kS, INT, true>(p, lay, warp - 2, lane, count, m0 + first, n0, part, 0u, sa, sw, bs);
+        else reduce_tokens<kS, INT, false>(p, lay, warp - 2, lane, count, m0 + first, n0, part, stride, sa, sw, bs);
+      };
+      if (S == 1) reduce(std::integral_constant<int, 1>{});
+      else if (S == 2) reduce(std::integral_constant<int, 2>{});
+      else if (S == 8) reduce(std::integral_constant<int, 8>{});
+      else reduce(std::integral_constant<int, 4>{});
+    }
   }
 
-  // ---- common exit: a CTA's partial sums stay until its peers have read them
+  // ---- common exit.  What peers send here has arrived (RECV), but a CTA that gave up may still be written to, and a CTA
+  // whose partial sums are fetched may still be read: it stays until its peers have arrived here too (or have left).
   tc_fence_before();
-  if (S > 1) cluster_sync();
-  else __syncthreads();
+  __syncwarp();
+  if (!fetch) __syncthreads();
+  if (fetch || (S > 1 && *abort_flag)) {
+    cluster_arrive();
+    cluster_wait();
+  }
   if (warp == 1) tmem_dealloc(tmem_base, kTmemCols);
 }
 
 }  // namespace
 
 struct SplitPlan {
-  static constexpr int kMaps = 8;
-  CUtensorMap idx[kMaps];       // one per slice count in use
-  int slices[kMaps];
-  int count;
+  CUtensorMap idx;              // boxes of [64 bytes][128 rows] over the packed rows
+  bool have;
 };
 
 namespace {
 
 std::mutex g_split_mutex;       // layers build their index maps on first use, possibly from several host threads
 
-// Boxes of [16 bytes][128 rows][slices] over the packed rows (dimensions: bytes of a 16-byte slice, rows, slices of
-// a row), so one copy brings a tile's index slices in the order the expanders read them.
-int slice_map(sacq_layer* L, int slices, CUtensorMap* out) {
+// Boxes of 64 bytes of 128 rows over the packed rows.  (Boxes of 16 bytes, in the order the expanders read them, cost the
+// copy engine a clock per 16 bytes: 24 slices of a row took 1.3 us longer to arrive.)
+int index_map(sacq_layer* L, CUtensorMap* out) {
   std::lock_guard<std::mutex> lock(g_split_mutex);
   if (L->split_plan == nullptr) L->split_plan = new SplitPlan();
   SplitPlan* plan = L->split_plan;
-  for (int i = 0; i < plan->count; ++i)
-    if (plan->slices[i] == slices) {
-      *out = plan->idx[i];
-      return SACQ_OK;
-    }
-  const uint64_t row_bytes = (uint64_t)(L->row_bits / 8);
-  const int rc = encode_bytes_3d(out, L->d.packed, 16, (uint64_t)L->d.out_features, row_bytes / 16, row_bytes, 16, 16u,
-                                 (uint32_t)kRows, (uint32_t)slices);
-  if (rc != SACQ_OK) return rc;
-  const int at = plan->count < SplitPlan::kMaps ? plan->count++ : SplitPlan::kMaps - 1;
-  plan->idx[at] = *out;
-  plan->slices[at] = slices;
+  if (!plan->have) {
+    const uint64_t row_bytes = (uint64_t)(L->row_bits / 8);
+    const int rc = encode_bytes_2d(&plan->idx, L->d.packed, row_bytes, (uint64_t)L->d.out_features, row_bytes,
+                                   (uint32_t)(kBoxSlices * 16), (uint32_t)kRows, CU_TENSOR_MAP_SWIZZLE_64B);
+    if (rc != SACQ_OK) return rc;
+    plan->have = true;
+  }
+  *out = plan->idx;
   return SACQ_OK;
 }
 
@@ -763,11 +852,18 @@ bool split_fits(const sacq_layer* L, SplitMode mode, SplitChoice* c) {
   const int cb_bytes = codebook_smem(L), groups = mode == kSplitHiLo ? 0 : 1;
   slice_extent(L, c->split, &c->max_slices, &c->max_groups);
   const int tiles = (stages_of(L->d.in_features) + c->split - 1) / c->split * (is_f16(mode) ? 2 : 1);
-  const size_t most = (cb_bytes > 0 ? 227 : 164) * 1024;
+  const size_t most = (cb_bytes > 0 ? 224 : 164) * 1024;
   auto bytes = [&](int stages) {
-    return split_smem(split_layout(c->tok, c->split, stages, c->max_slices, groups * c->max_groups, cb_bytes));
+    return split_smem(split_layout(c->tok, c->split, stages, c->max_slices, groups * c->max_groups, cb_bytes, c->own_recv));
   };
-  for (c->act_stages = tiles < 2 ? 2 : tiles < kMaxAct ? tiles : kMaxAct; c->act_stages > 2; --c->act_stages)
+  const int all = tiles < 2 ? 2 : tiles < kMaxAct ? tiles : kMaxAct;
+  if (c->split > 1 && c->tok <= (c->split == 2 ? 96 : 64)) {
+    c->own_recv = true;
+    for (c->act_stages = all; c->act_stages >= (all < 4 ? all : 4); --c->act_stages)
+      if (bytes(c->act_stages) <= most) return true;
+  }
+  c->own_recv = false;
+  for (c->act_stages = all; c->act_stages > 2; --c->act_stages)
     if (bytes(c->act_stages) <= most) return true;
   return bytes(2) <= 227 * 1024;
 }
@@ -900,7 +996,7 @@ int launch_split_k(const sacq_layer* const* layers, int n, const void* act, cons
   int64_t widest = 0;
   for (int l = 0; l < n; ++l) {
     const sacq_layer* L = layers[l];
-    rc = slice_map(const_cast<sacq_layer*>(L), c.max_slices, &p.idx[l]);
+    rc = index_map(const_cast<sacq_layer*>(L), &p.idx[l]);
     if (rc != SACQ_OK) return rc;
     SplitLayer& q = p.layer[l];
     q.cb = mode == kSplitHiLo ? L->cb_hilo
@@ -930,9 +1026,10 @@ int launch_split_k(const sacq_layer* const* layers, int n, const void* act, cons
   p.M = (int)M; p.K = (int)d0.in_features; p.C = mode >= kSplitInt8 ? d0.codebook_size : layers[0]->cb_entries;
   p.bits = d0.index_bits; p.num_groups = (int)layers[0]->num_groups; p.group_size = d0.group_size;
   p.split = c.split; p.parts = c.parts; p.tok = c.tok; p.act_stages = c.act_stages; p.max_slices = c.max_slices; p.max_groups = c.max_groups;
+  p.own_recv = c.own_recv ? 1 : 0;
   const dim3 grid((unsigned)((widest + kRows - 1) / kRows * c.split), (unsigned)c.tiles, (unsigned)n);
   const size_t smem = split_smem(split_layout(c.tok, c.split, c.act_stages, c.max_slices, mode == kSplitHiLo ? 0 : c.max_groups,
-                                              codebook_smem(layers[0])));
+                                              codebook_smem(layers[0]), c.own_recv));
   const bool cb = codebook_smem(layers[0]) > 0;
   const cudaError_t e = d0.vector_dim == 8 ? (cb ? launch_mode<8, true>(mode, ta, p, grid, smem, s) : launch_mode<8, false>(mode, ta, p, grid, smem, s))
                                            : (cb ? launch_mode<4, true>(mode, ta, p, grid, smem, s) : launch_mode<4, false>(mode, ta, p, grid, smem, s));

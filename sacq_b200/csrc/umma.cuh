@@ -161,10 +161,6 @@ __host__ __device__ constexpr uint32_t make_idesc_i8(int bn) {
 int encode_bytes_2d(CUtensorMap* map, const void* base, uint64_t row_bytes, uint64_t rows, uint64_t pitch_bytes,
                     uint32_t box_bytes, uint32_t box_rows, CUtensorMapSwizzle swizzle);
 
-// 3-D byte tensor [dim2][rows][row_bytes] with a [box2][box_rows][box_bytes] box, not swizzled (linear_large_m.cu).
-int encode_bytes_3d(CUtensorMap* map, const void* base, uint64_t row_bytes, uint64_t rows, uint64_t dim2, uint64_t row_pitch,
-                    uint64_t dim2_pitch, uint32_t box_bytes, uint32_t box_rows, uint32_t box2);
-
 // Tile map over a layer's packed index rows: box = one index super-block (two 128-k blocks) x
 // 128 weight rows.  Built on first use and kept by the layer.
 int large_m_index_map(const sacq_layer* L, const CUtensorMap** out);
