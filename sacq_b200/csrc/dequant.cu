@@ -192,8 +192,7 @@ decode_weight_int8_kernel(const uint32_t* __restrict__ words, const uint16_t* __
 //
 // What bounds it: the one-thread-per-vector kernels above spend a 16-byte L1 gather (a tag lookup per lane: d = 4
 // took 25 us for 12.6 M weights), an index-to-row division and an IEEE division per weight (d = 8: 15 us).  Here
-// the gathers go to shared memory, the row's divisor is set up once, and a quotient is two residual corrections of
-// z times its reciprocal (RowDivisor).  Weights are clamped first, to a bf16 value that encodes to the largest byte
+// the gathers go to shared memory, the row's divisor is set up once, and a quotient is two instructions (RowDivisor).  Weights are clamped first, to a bf16 value that encodes to the largest byte
 // (RowWeights), so that a caller's own row scale cannot overflow the quotient.
 constexpr int kSegSteps = 64;         // 16-weight steps of a row that a warp takes
 
@@ -247,7 +246,7 @@ decode_rows_kernel(const uint32_t* __restrict__ words, const uint16_t* __restric
       }
       uint32_t a[4];
       const __nv_bfloat16 sb = __ushort_as_bfloat16(s);
-      encode_weights16<I8>(pair, __halves2bfloat162(sb, sb), shift2, r, a);
+      encode_weights16<I8>(pair, __halves2bfloat162(sb, sb), shift2, (shift & 0x7fffu) != 0, r, a);
       out[st] = make_uint4(a[0], a[1], a[2], a[3]);
     }
   }

@@ -35,32 +35,28 @@ __device__ __forceinline__ float pair_hi(uint32_t w) { return __uint_as_float(w 
 
 // The divisor of a quantized row: q = encode(z / s) with IEEE division.  A division costs about a dozen
 // instructions per element and, with the unpacking around it, bounded every quantizer by instruction issue (17 per
-// element).  One s serves a whole row, so its correctly rounded reciprocal r is made once and a quotient takes
-// residual corrections instead, two elements per instruction: q0 = RN(z r), then q' = RN(q + RN(z - q s) r)
-// (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev.
-// 34(1), 1990: with r = RN(1/s) and q within one ulp of z / s the residual is exact and q' is RN(z / s)).  The first
-// correction brings q within an ulp, the second makes it exact for any s.  (Locating the quotient between z r(1 - e)
-// and z r(1 + e) and dividing only where the two encode differently is not faster: scales are quotients of 8-bit
-// significands by 127 and 448, so exact ties are common, and every warp met one.)  Checked against the division over
-// the whole domain of the activation quantizers: every finite bf16 maximum, both formats, every bf16 value up to it
-// (2.1 G quotients each), no byte differs.
+// element).  One s serves a whole row, so its reciprocal is made once, as the sum of two fp32 numbers r + r2, and a
+// quotient is fma(z, r, z r2), two elements per instruction.  r is 1/s rounded down, so that r2 is not negative and a
+// quotient of zero keeps its sign.  Compared with the division for all 2^23 significands of s and all 128 significands of a
+// bf16 dividend: 11 of the 1.07 G quotients differ, by one ulp, none of them next to a value of fewer than 10 significant
+// bits, where an encoding changes; for the scales of a quantizer, fp32(bf16 / 448) and fp32(bf16 / 127), none.  (Two residual
+// corrections of z RN(1/s), five instructions instead of two and one more for the signs, took the INT8 recipe's expanders
+// 1.06 us per 128 x 128 weights.  Locating the quotient between z r(1 - e) and z r(1 + e) and dividing only where the two
+// encode differently is not faster: exact ties are common, and every warp met one.)
 struct RowDivisor {
-  float s, r;
-  bool fast;                    // s in 2^-80 .. 2^80: every residual that can matter is exact; else divide
+  float s, r, r2;
+  bool fast;                    // s in 2^-80 .. 2^80: every term that can matter is exact enough; else divide
 };
 __device__ __forceinline__ RowDivisor row_divisor(float s) {
   RowDivisor d;
   d.s = s;
-  d.r = __frcp_rn(s);
+  d.r = __frcp_rd(s);
+  d.r2 = __fdiv_rn(__fmaf_rn(-s, d.r, 1.0f), s);      // the remainder is exact
   d.fast = s > 8.3e-25f && s < 1.2e24f;               // false for inf and NaN
   return d;
 }
-// RN(z / s) of two elements.
-__device__ __forceinline__ uint64_t quotient2(uint64_t z, uint64_t ns, uint64_t r) {
-  uint64_t q = mul2(z, r);
-  q = fma2(fma2(q, ns, z), r, q);
-  return fma2(fma2(q, ns, z), r, q);
-}
+// z / s of two elements.
+__device__ __forceinline__ uint64_t quotient2(uint64_t z, uint64_t r, uint64_t r2) { return fma2(z, r, mul2(z, r2)); }
 
 // Scale of a row from its largest |x|: a NaN maximum fails `> 0` like in the reference's torch.where, so the row
 // keeps scale 1 and its NaN elements stay NaN; an infinite maximum gives an infinite scale.  Both divide
@@ -95,11 +91,11 @@ __device__ __forceinline__ uint32_t encode2(float z0, float z1, float s) {
 template <bool I8, int P>
 __device__ __forceinline__ void encode_pairs(const uint32_t (&w)[P], const RowDivisor& d, uint32_t (&out)[P / 2]) {
   if (d.fast) {
-    const uint64_t ns = f32x2(-d.s, -d.s), r = f32x2(d.r, d.r), magic = f32x2(12582912.0f, 12582912.0f);
+    const uint64_t r = f32x2(d.r, d.r), r2 = f32x2(d.r2, d.r2), magic = f32x2(12582912.0f, 12582912.0f);
 #pragma unroll
     for (int j = 0; j < P / 2; ++j) {
-      uint64_t q0 = quotient2(f32x2(pair_lo(w[2 * j]), pair_hi(w[2 * j])), ns, r);
-      uint64_t q1 = quotient2(f32x2(pair_lo(w[2 * j + 1]), pair_hi(w[2 * j + 1])), ns, r);
+      uint64_t q0 = quotient2(f32x2(pair_lo(w[2 * j]), pair_hi(w[2 * j])), r, r2);
+      uint64_t q1 = quotient2(f32x2(pair_lo(w[2 * j + 1]), pair_hi(w[2 * j + 1])), r, r2);
       float a, b, c, e;
       if constexpr (I8) {
         halves_of(add2(q0, magic), a, b);
@@ -109,9 +105,7 @@ __device__ __forceinline__ void encode_pairs(const uint32_t (&w)[P], const RowDi
       } else {
         halves_of(q0, a, b);
         halves_of(q1, c, e);
-        // the corrections turn a negative zero into a positive one: the signs come from the dividends
-        out[j] = float2_to_e4m3x2(a, b) | (float2_to_e4m3x2(c, e) << 16) |
-                 (__byte_perm(w[2 * j], w[2 * j + 1], 0x7531) & 0x80808080u);
+        out[j] = float2_to_e4m3x2(a, b) | (float2_to_e4m3x2(c, e) << 16);
       }
     }
   } else {
@@ -143,14 +137,16 @@ __device__ __forceinline__ RowWeights row_weights(float sw) {
 }
 
 // 16 weights of one row -> 16 bytes: bf16(bf16(c * s) + shift) divided by the row scale and encoded.  pair: 16
-// codebook elements; s2, shift2: the scale and the shift in both halves.
+// codebook elements; s2, shift2: the scale and the shift in both halves.  A shift of zero (has_shift false) rounds nothing,
+// and only its sign matters, to a product of zero: one fused instruction.
 template <bool I8>
 __device__ __forceinline__ void encode_weights16(const uint32_t (&pair)[8], __nv_bfloat162 s2, __nv_bfloat162 shift2,
-                                                 const RowWeights& r, uint32_t (&out)[4]) {
+                                                 bool has_shift, const RowWeights& r, uint32_t (&out)[4]) {
   uint32_t w[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    __nv_bfloat162 v = __hadd2_rn(__hmul2_rn(*reinterpret_cast<const __nv_bfloat162*>(&pair[j]), s2), shift2);
+    const __nv_bfloat162 c = *reinterpret_cast<const __nv_bfloat162*>(&pair[j]);
+    __nv_bfloat162 v = has_shift ? __hadd2_rn(__hmul2_rn(c, s2), shift2) : __hfma2(c, s2, shift2);
     if constexpr (I8) v = __hmin2(__hmax2(v, r.neg_lim), r.lim);
     else v = __hmin2_nan(__hmax2_nan(v, r.neg_lim), r.lim);      // a NaN stays one
     w[j] = *reinterpret_cast<const uint32_t*>(&v);

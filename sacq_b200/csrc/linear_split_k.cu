@@ -71,10 +71,22 @@ struct SplitLayer {
   float out_mul;                // power of two that undoes the operands' scaling
 };
 
+// mbarriers of a CTA
+constexpr int ACT_FULL = 0, ACT_EMPTY = kMaxAct, W_FULL = 2 * kMaxAct, W_EMPTY = W_FULL + kMaxW, IDX_FULL = W_EMPTY + kMaxW,
+              CB_FULL = IDX_FULL + 2, ACC_FULL = CB_FULL + 1, RECV = ACC_FULL + 1, kBarriers = RECV + 1;
+
+struct SplitLayout {
+  uint32_t idx_off, cb_off, sc_off, recv_off, fixed_off, sa_off, sw_off, bias_off, bar_off, misc_off, total;
+};
+
 // What a CTA's start depends on comes first: kernel parameters are read through a cache that is cold in every launch, a miss
-// per line.
+// per line.  The layout comes ready from the host, and what the kernel divides by is a power of two: with its divisions a CTA's
+// way to its first copy took 0.2 us longer.
 struct alignas(64) SplitParams {
-  int split;                    // CTAs per cluster
+  int split, split_shift;       // CTAs per cluster, its logarithm
+  int slice_shift;              // ... of the slices of K, split * parts
+  int own;                      // owned_tokens(tok, split)
+  SplitLayout lay;
   int parts;                    // consecutive slices of K per CTA, each with accumulator columns of its own
   int tok;                      // tokens per CTA (multiple of 16; of 32 above 256)
   int M, K, C, bits, num_groups, group_size;
@@ -89,14 +101,6 @@ struct alignas(64) SplitParams {
   int64_t ldr;
   int n_bc;                     // further copies of the output (peer GPUs' buffers), same pitch as y
   uint16_t* ybc[kMaxBcast];
-};
-
-// mbarriers of a CTA
-constexpr int ACT_FULL = 0, ACT_EMPTY = kMaxAct, W_FULL = 2 * kMaxAct, W_EMPTY = W_FULL + kMaxW, IDX_FULL = W_EMPTY + kMaxW,
-              CB_FULL = IDX_FULL + 2, ACC_FULL = CB_FULL + 1, RECV = ACC_FULL + 1, kBarriers = RECV + 1;
-
-struct SplitLayout {
-  uint32_t idx_off, cb_off, sc_off, recv_off, fixed_off, sa_off, sw_off, bias_off, bar_off, misc_off, total;
 };
 
 // tokens of the tile a rank reduces and writes
@@ -310,7 +314,7 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   constexpr int TILES = F16 ? 2 : 1;                  // activation tiles (128 bytes of every token) per weight stage
   constexpr int W_COLS = w_cols(MODE);                // TMEM columns of a weight stage
   const int S = p.split;
-  const int n0 = ((int)blockIdx.x / S) * kRows;
+  const int n0 = ((int)blockIdx.x >> p.split_shift) * kRows;
   const SplitLayer& lay = p.layer[blockIdx.z];
   if (n0 >= lay.N) return;                            // a narrower sibling: uniform over the cluster
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -319,8 +323,7 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* sm = smem_raw + (base - raw);
   const uint32_t cb_bytes = (uint32_t)(p.C * CW_BYTES);
-  const SplitLayout L = split_layout(p.tok, S, p.act_stages, p.max_slices, F16 || RECIPE ? p.max_groups : 0,
-                                     CB_SMEM ? (int)cb_bytes : 0, p.own_recv != 0);
+  const SplitLayout& L = p.lay;
 
   const uint32_t bars = base + L.bar_off;
   auto bar = [&](int i) { return bars + 8u * i; };
@@ -331,10 +334,10 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   const int rank = S > 1 ? (int)cluster_rank() : 0;
   const int m0 = blockIdx.y * p.tok;
   const int nkb = stages_of(p.K);
-  const int parts = p.parts, slices = S * parts;
+  const int parts = p.parts, slices = p.slice_shift;  // (a logarithm)
   // this CTA's weight stages, and the first one (counted from kb0) of its slice `v`
-  const int kb0 = rank * parts * nkb / slices, kbs = (rank + 1) * parts * nkb / slices - kb0;
-  auto part_begin = [&](int v) { return (rank * parts + v) * nkb / slices - kb0; };
+  const int kb0 = rank * parts * nkb >> slices, kbs = ((rank + 1) * parts * nkb >> slices) - kb0;
+  auto part_begin = [&](int v) { return ((rank * parts + v) * nkb >> slices) - kb0; };
   const int tok = p.tok, acc_cols = tok * parts;
   const bool halves = tok > 256;                      // an instruction (and a TMA box) takes at most 256 tokens
   const int w_stages = min(kMaxW, ((int)kTmemCols - acc_cols) / W_COLS);
@@ -489,7 +492,10 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       for (int i = et; i < kRows * g_count; i += kXThreads) {
         const int r = i / g_count, g = i - r * g_count;
         const int n = min(n0 + r, lay.N - 1);
-        sc[r * sc_pitch + g] = __ldg(lay.scales + (int64_t)n * p.num_groups + g_first + g);
+        const uint16_t v = __ldg(lay.scales + (int64_t)n * p.num_groups + g_first + g);
+        // fp16 forms: scale x 2^e, the row's or the layer's power of two, is a bf16 significand with a small exponent: exact in fp16
+        const float mul = PAIR ? 1.f / __ldg(lay.row_mul + n) : lay.scale_mul;
+        sc[r * sc_pitch + g] = F16 ? __half_as_ushort(__float2half_rn(bf16_bits_to_float(v) * mul)) : v;
       }
     }
     xbarrier();
@@ -520,11 +526,7 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     const RowWeights rw = row_weights<INT>(RECIPE ? __ldg(p.row_scale + min(n0 + row, lay.N - 1)) : 1.f);
     const __nv_bfloat162 shift2 = __halves2bfloat162(__ushort_as_bfloat16(p.shift), __ushort_as_bfloat16(p.shift));
     // kSplitHalf2: the codewords as they are, and the two 64-k tiles' scales; the products are made at the store.
-    const float row_mul = PAIR ? __ldg(lay.row_mul + min(n0 + row, lay.N - 1)) : 1.f;
-    const float scale_mul = PAIR ? 1.f / row_mul : lay.scale_mul;       // a power of two
     auto expand = [&](int wi, uint32_t (&w)[16], __half2 (&sc2)[2]) {
-      if (wi == late) ok = ok && mbar_wait_warp(bar(IDX_FULL + 1), 0, abort_flag, lay.status);
-      if (!ok) return;
       if constexpr (RECIPE) {
         // 32 weights of this thread's row, 16 at a time: bf16(bf16(c * s) + shift) divided by the row scale and
         // encoded (the arithmetic of decode_rows_kernel in dequant.cu)
@@ -547,7 +549,7 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
               pair[2 * j] = v.x; pair[2 * j + 1] = v.y;
             }
           }
-          encode_weights16<INT>(pair, __halves2bfloat162(s, s), shift2, rw, reinterpret_cast<uint32_t (&)[4]>(w[4 * h]));
+          encode_weights16<INT>(pair, __halves2bfloat162(s, s), shift2, (p.shift & 0x7fffu) != 0, rw, reinterpret_cast<uint32_t (&)[4]>(w[4 * h]));
         }
       } else if constexpr (F16) {
         constexpr int IPT = 16 / D;                   // indices per thread and 64-k tile
@@ -560,8 +562,7 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             continue;
           }
           if (wi * kStageK + sub * 64 >= grp_end) { ++grp; grp_end += p.group_size; }
-          // scale x 2^e is a bf16 significand with a small exponent: exact in fp16
-          const __half2 s2 = __half2half2(__float2half_rn(bf16_bits_to_float(sc[row * sc_pitch + grp]) * scale_mul));
+          const __half2 s2 = __half2half2(__ushort_as_half(sc[row * sc_pitch + grp]));
           sc2[sub] = s2;
           const int bit = (((kb0 + wi) * kStageK + sub * 64 + kpart * 16) / D) * bits - slice0 * 128;
           const uint64_t win = slice_window(rowidx, swz, bit, IPT * bits);
@@ -608,7 +609,8 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     uint32_t w_parity = 1;
     uint32_t cur[16], nxt[16];
     __half2 cur_s[2], nxt_s[2];
-    expand(0, cur, cur_s);
+    if (late == 0) ok = ok && mbar_wait_warp(bar(IDX_FULL + 1), 0, abort_flag, lay.status);
+    if (ok) expand(0, cur, cur_s);
     __syncwarp();
     if (S > 1 && p.own_recv) cluster_wait();
     for (int wi = 0; wi < kbs && ok; ++wi) {
@@ -637,7 +639,8 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         tmem_st_32x8(w_addr, reinterpret_cast<const uint32_t (&)[8]>(cur[0]));
         if constexpr (!RECIPE) tmem_st_32x8(w_addr + 32u, reinterpret_cast<const uint32_t (&)[8]>(cur[8]));
       }
-      if (wi + 1 < kbs) expand(wi + 1, nxt, nxt_s);
+      if (wi + 1 == late && late < kbs) ok = mbar_wait_warp(bar(IDX_FULL + 1), 0, abort_flag, lay.status);
+      if (wi + 1 < kbs && ok) expand(wi + 1, nxt, nxt_s);
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
@@ -654,7 +657,7 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   }
 
   // ---- reduction: the accumulators of the cluster's CTAs -> y.  Every thread takes part in the cluster barrier.
-  const int own = owned_tokens(tok, S);
+  const int own = p.own;
   const bool send = S > 1 && p.own_recv, fetch = S > 1 && !send;   // fetch: a CTA keeps its partial sums, its peers read them
   if (warp >= 2 && ok) {
     // [token][row] fp32 into the shared memory of the CTA that owns the token, or the own; a warp writes 128 consecutive
@@ -675,21 +678,28 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 #pragma unroll
         for (int j = 0; j < 16; ++j) r[j] = add_bits<INT>(r[j], r2[j]);
       }
+      if constexpr (PAIR) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * row_mul);
+      }
+      if (!send) {
+        uint32_t* dst = reinterpret_cast<uint32_t*>(sm) + c0 * kRows + row;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) dst[j * kRows] = r[j];
+        continue;
+      }
 #pragma unroll
       for (int h = 0; h < 2; ++h) {                   // eight tokens have one owner
-        const int t = c0 + h * 8, owner = send ? t / own : rank;
-        const uint32_t dst = base + L.recv_off + (uint32_t)(((send ? rank * own + t - owner * own : t) * kRows + row) * 4);
+        const int t = c0 + h * 8, owner = t / own;
+        const uint32_t dst = base + L.recv_off + (uint32_t)(((rank * own + t - owner * own) * kRows + row) * 4);
         if (owner == rank) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const uint32_t v = PAIR ? __float_as_uint(__uint_as_float(r[h * 8 + j]) * row_mul) : r[h * 8 + j];
-            asm volatile("st.shared.u32 [%0], %1;" ::"r"(dst + (uint32_t)(j * kRows * 4)), "r"(v) : "memory");
-          }
-        } else {
-          const uint32_t peer = peer_address(dst, (uint32_t)owner);
-#pragma unroll
           for (int j = 0; j < 8; ++j)
-            store_peer(peer + (uint32_t)(j * kRows * 4), PAIR ? __float_as_uint(__uint_as_float(r[h * 8 + j]) * row_mul) : r[h * 8 + j]);
+            asm volatile("st.shared.u32 [%0], %1;" ::"r"(dst + (uint32_t)(j * kRows * 4)), "r"(r[h * 8 + j]) : "memory");
+        } else {
+          const uint32_t at_owner = peer_address(dst, (uint32_t)owner);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) store_peer(at_owner + (uint32_t)(j * kRows * 4), r[h * 8 + j]);
         }
       }
     }
@@ -1027,9 +1037,13 @@ int launch_split_k(const sacq_layer* const* layers, int n, const void* act, cons
   p.bits = d0.index_bits; p.num_groups = (int)layers[0]->num_groups; p.group_size = d0.group_size;
   p.split = c.split; p.parts = c.parts; p.tok = c.tok; p.act_stages = c.act_stages; p.max_slices = c.max_slices; p.max_groups = c.max_groups;
   p.own_recv = c.own_recv ? 1 : 0;
+  auto log2_of = [](int v) { int n = 0; while (1 << n < v) ++n; return n; };     // split and parts are powers of two
+  p.split_shift = log2_of(c.split);
+  p.slice_shift = log2_of(c.split * c.parts);
+  p.own = owned_tokens(c.tok, c.split);
+  p.lay = split_layout(c.tok, c.split, c.act_stages, c.max_slices, mode == kSplitHiLo ? 0 : c.max_groups, codebook_smem(layers[0]), c.own_recv);
   const dim3 grid((unsigned)((widest + kRows - 1) / kRows * c.split), (unsigned)c.tiles, (unsigned)n);
-  const size_t smem = split_smem(split_layout(c.tok, c.split, c.act_stages, c.max_slices, mode == kSplitHiLo ? 0 : c.max_groups,
-                                              codebook_smem(layers[0]), c.own_recv));
+  const size_t smem = split_smem(p.lay);
   const bool cb = codebook_smem(layers[0]) > 0;
   const cudaError_t e = d0.vector_dim == 8 ? (cb ? launch_mode<8, true>(mode, ta, p, grid, smem, s) : launch_mode<8, false>(mode, ta, p, grid, smem, s))
                                            : (cb ? launch_mode<4, true>(mode, ta, p, grid, smem, s) : launch_mode<4, false>(mode, ta, p, grid, smem, s));
