@@ -321,6 +321,30 @@ __device__ long long g_small_trace[96];
 #define SACQ_ST(slot) do { } while (0)
 #endif
 
+// The NF fields of a warp's share of a span: those of half `hf` (0 where the warp has the whole span), moved to bit 0.  One
+// code for both halves: with the half as a compile-time position every copy of the loop was there twice.
+template <int BITS, int NF>
+struct Fields {
+  static constexpr int kBits = BITS * NF, kWords = (kBits + 31) / 32;
+  static constexpr bool kShifts = NF < 8 && kBits % 32 != 0;                   // 12 bits, halves: 48 bits from bit 0 or 48
+  uint32_t w[kWords];
+  __device__ __forceinline__ void load(const uint8_t* span_words, int hf) {
+    const int bit = hf * kBits;
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(span_words) + (bit >> 5);
+    uint32_t raw[kWords];
+#pragma unroll
+    for (int j = 0; j < kWords; ++j) raw[j] = src[j];
+#pragma unroll
+    for (int j = 0; j < kWords; ++j)
+      w[j] = kShifts ? __funnelshift_r(raw[j], j + 1 < kWords ? raw[j + 1] : 0u, bit & 31) : raw[j];
+  }
+  __device__ __forceinline__ uint32_t get(int j) const {
+    const int bit = j * BITS, word = bit >> 5, off = bit & 31;
+    if (off + BITS <= 32) return (w[word] >> off) & ((1u << BITS) - 1u);
+    return __funnelshift_r(w[word], w[word + 1 < kWords ? word + 1 : word], off) & ((1u << BITS) - 1u);
+  }
+};
+
 // HALVES = warps sharing one 32-index span (each takes 8/HALVES of its MMA steps): with
 // two, a CTA runs up to 16 lighter warps, which hides more of the gather -> MMA latency.
 // `cta` of `ncta` CTAs work on the layer described by p (a launch may cover several layers).
@@ -330,7 +354,6 @@ __device__ __forceinline__ void staged_body(const SmallMParams& p, const int cta
   constexpr int NQ = NS * D / 16;          // uint4 loads covering them per token row
   extern __shared__ __align__(128) uint8_t smem[];
   using CwVec = typename std::conditional<D == 8, uint4, uint2>::type;
-  constexpr int WPG = BITS / 4;
   constexpr int kFrag = R8 * 4;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nwarps = blockDim.x >> 5;
@@ -359,6 +382,9 @@ __device__ __forceinline__ void staged_body(const SmallMParams& p, const int cta
     mbar_init(bar_idx0, 1);
     mbar_init(bar_idx0 + 8, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    const uint32_t cb_bytes = (uint32_t)(p.C * D * 2);
+    mbar_expect_tx(bar_cb, cb_bytes);
+    bulk_copy_g2s(smem + L.cb_off, p.cb_hilo, cb_bytes, bar_cb);    // layer constants: may overlap the previous kernel
   }
   __syncthreads();
 
@@ -402,22 +428,44 @@ __device__ __forceinline__ void staged_body(const SmallMParams& p, const int cta
   // This CTA's share: one token chunk (fixed for the CTA's lifetime, so its activation
   // tile is copied once) and the row tiles rt_first, rt_first + rt_stride, ...  The host
   // makes gridDim.x a multiple of the chunk count.
-  const int chunk = cta % p.chunks;
-  const int first_rt = cta / p.chunks;
-  const int rt_stride = ncta / p.chunks;
+  const bool one_chunk = p.chunks == 1;              // no divisions on the way to the first copy
+  const int chunk = one_chunk ? 0 : cta % p.chunks;
+  const int first_rt = one_chunk ? cta : cta / p.chunks;
+  const int rt_stride = one_chunk ? ncta : ncta / p.chunks;
   const int m_base = chunk * 16;
   const int toks_here = min(16, p.M - m_base);
   uint8_t* act_s = act_base;
-  if (threadIdx.x == 0) {
-    const uint32_t cb_bytes = (uint32_t)(p.C * D * 2);
-    mbar_expect_tx(bar_cb, cb_bytes);
-    bulk_copy_g2s(smem + L.cb_off, p.cb_hilo, cb_bytes, bar_cb);    // layer constants: may overlap
-  }                                                                  // the previous kernel of the stream
-  if (threadIdx.x < 8 * R8 && first_rt < p.row_blocks) issue_idx(first_rt, 0);
+  if (threadIdx.x < 8 * R8 && first_rt < p.row_blocks) {
+    issue_idx(first_rt, 0);
+    const int n = min(first_rt * 8 * R8 + (int)threadIdx.x, p.N - 1);
+    rowsc_s[threadIdx.x] = bf16_bits_to_float(__ldg(p.scales + (int64_t)n * p.num_groups));
+    rowb_s[threadIdx.x] = p.bias ? bf16_bits_to_float(__ldg(p.bias + n)) : 0.f;
+  }
   // the next kernel of the stream (a quantizer or another GEMM launched with programmatic
   // serialization) may be scheduled from here on; it waits for this grid before it touches memory
   SACQ_ST(1);
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+
+  // Codewords do not depend on the activations: the first ones of the warp's first item are gathered before the wait for
+  // the kernel in front, into registers, as far as these go.
+  constexpr int kItemRegs = NS * D / 2;                                      // of one sub-block
+  constexpr int kPreRegs = R8 == 6 ? 16 : HALVES == 1 ? 64 : 32;             // of all
+  constexpr int PR = kPreRegs / kItemRegs < R8 ? kPreRegs / kItemRegs : R8;  // sub-blocks
+  CwVec pre[PR][NS];
+  bool ok = true;
+  if (first_rt < p.row_blocks) {
+    ok = mbar_wait_bounded(bar_cb, 0, p.status) && mbar_wait_bounded(bar_idx0, 0, p.status);
+    if (ok && warp < p.spans_per_row * HALVES) {
+      const int rows_here = min(8 * R8, p.N - first_rt * 8 * R8);
+#pragma unroll
+      for (int r = 0; r < PR; ++r) {
+        Fields<BITS, NS> f;
+        f.load(smem + L.idx_off + min(r * 8 + g, rows_here - 1) * idx_pitch + warp / HALVES * (4 * BITS) + t * BITS, warp % HALVES);
+#pragma unroll
+        for (int j = 0; j < NS; ++j) pre[r][j] = cbs[f.get(j)];
+      }
+    }
+  }
   asm volatile("griddepcontrol.wait;" ::: "memory");                // activations come from that kernel
   SACQ_ST(2);
   SACQ_TL(t_dep);
@@ -428,13 +476,7 @@ __device__ __forceinline__ void staged_body(const SmallMParams& p, const int cta
     issue_act(chunk, 0);
     sa_s[threadIdx.x] = threadIdx.x < toks_here ? __ldg(p.act_scale + m_base + threadIdx.x) : 0.f;
   }
-  if (threadIdx.x < 8 * R8 && first_rt < p.row_blocks) {
-    const int n = min(first_rt * 8 * R8 + (int)threadIdx.x, p.N - 1);
-    rowsc_s[threadIdx.x] = bf16_bits_to_float(__ldg(p.scales + (int64_t)n * p.num_groups));
-    rowb_s[threadIdx.x] = p.bias ? bf16_bits_to_float(__ldg(p.bias + n)) : 0.f;
-  }
 
-  bool ok = true;
   uint32_t idx_parity[2] = {0, 0};
   bool first = true;
   int it = 0;
@@ -471,24 +513,15 @@ __device__ __forceinline__ void staged_body(const SmallMParams& p, const int cta
     if (!ok) break;                                    // a bounded wait expired: status word is set
     SACQ_ST(8 + 6 * it + 1);
 
-    // per-row scales of the two output rows this lane holds in each sub-block
-    float s0[R8], s1[R8];
-    int sn0[R8], sn1[R8];
-#pragma unroll
-    for (int r = 0; r < R8; ++r) {
-      sn0[r] = min(n_base + r * 8 + 2 * t, p.N - 1);
-      sn1[r] = min(n_base + r * 8 + 2 * t + 1, p.N - 1);
-      s0[r] = rowsc_s[r * 8 + 2 * t];
-      s1[r] = rowsc_s[r * 8 + 2 * t + 1];
-    }
     float acc[R8][4];
 #pragma unroll
     for (int r = 0; r < R8; ++r)
 #pragma unroll
       for (int j = 0; j < 4; ++j) acc[r][j] = 0.f;
-    float xs_a = 0.f, xs_b = 0.f;
 
-    for (int item = warp; item < p.spans_per_row * HALVES; item += nwarps) {
+    // one item: a span, or half of one; PRE: it is the one whose first codewords have been gathered
+    auto mma_item = [&](const int item, auto PRE) {
+      constexpr int kPre = decltype(PRE)::value ? PR : 0;     // sub-blocks whose codewords are there
       const int sp = item / HALVES, hf = item % HALVES;
       // A fragments are the raw e4m3 bytes: vector (8t + first + s) of token rows g and g+8.
       // FP8 MMAs need no widening; slots {4t..4t+3} carry bytes 0-3 and slots {16+4t..}
@@ -514,106 +547,87 @@ __device__ __forceinline__ void staged_body(const SmallMParams& p, const int cta
 #pragma unroll
         for (int j = 0; j < AW; ++j) fb[j] = 0u;
       }
-      if (p.shift != 0.f) {
-        float ta = 0.f, tb = 0.f;
-#pragma unroll
-        for (int j = 0; j < AW; ++j) {
-          uint32_t lo, hi;
-          e4m3x4_to_h2(fa[j], lo, hi);
-          ta += __low2float(as_h2(lo)) + __high2float(as_h2(lo)) + __low2float(as_h2(hi)) + __high2float(as_h2(hi));
-          e4m3x4_to_h2(fb[j], lo, hi);
-          tb += __low2float(as_h2(lo)) + __high2float(as_h2(lo)) + __low2float(as_h2(hi)) + __high2float(as_h2(hi));
-        }
-        ta += __shfl_xor_sync(0xffffffffu, ta, 1);
-        ta += __shfl_xor_sync(0xffffffffu, ta, 2);
-        tb += __shfl_xor_sync(0xffffffffu, tb, 1);
-        tb += __shfl_xor_sync(0xffffffffu, tb, 2);
-        xs_a += ta;
-        xs_b += tb;
-      }
       // Sub-blocks are processed RG at a time: their step accumulators interleave (independent MMA
-      // chains), while the 48-row tile keeps only half of them live at once (register budget).
-      constexpr int RG = R8 == 6 ? 3 : R8;
+      // chains), while the 48-row tile keeps only a third of them live at once (register budget).
+      constexpr int RG = R8 == 6 ? 2 : R8;
 #pragma unroll
       for (int r0 = 0; r0 < R8; r0 += RG) {
-        uint32_t wcur[RG][WPG];
+        Fields<BITS, NS> f[RG];
 #pragma unroll
-        for (int r = 0; r < RG; ++r) {
-          const int rr = min((r0 + r) * 8 + g, rows_here - 1);
-          const uint32_t* src = reinterpret_cast<const uint32_t*>(idx_s + rr * idx_pitch + sp * (4 * BITS) + t * BITS);
-#pragma unroll
-          for (int j = 0; j < WPG; ++j) wcur[r][j] = src[j];
-        }
+        for (int r = 0; r < RG; ++r)
+          if (r0 + r >= kPre)
+            f[r].load(idx_s + min((r0 + r) * 8 + g, rows_here - 1) * idx_pitch + sp * (4 * BITS) + t * BITS, hf);
         // two accumulators per sub-block (even / odd steps) halve the dependent MMA chain
         float cs[RG][4], ct[RG][4];
 #pragma unroll
         for (int r = 0; r < RG; ++r)
 #pragma unroll
           for (int j = 0; j < 4; ++j) { cs[r][j] = 0.f; ct[r][j] = 0.f; }
-        // the half index selects compile-time field positions, so dispatch on it once
-        auto mma_steps = [&](auto HF) {
-          constexpr int kFirst = decltype(HF)::value * NS;
-          if constexpr (D == 8) {
-            // one codeword per step: 16 bytes = e4m3 high half | low half
+        auto codeword = [&](int r, int j) { return r0 + r < kPre ? pre[(r0 + r) % PR][j] : cbs[f[r].get(j)]; };
+        if constexpr (D == 8) {
+          // one codeword per step: 16 bytes = e4m3 high half | low half
 #pragma unroll
-            for (int s8 = 0; s8 < NS; ++s8) {
+          for (int s8 = 0; s8 < NS; ++s8) {
 #pragma unroll
-              for (int r = 0; r < RG; ++r) {
-                const uint4 c = cbs[field8<BITS>(wcur[r], kFirst + s8)];
-                float (&acc2)[4] = (s8 & 1) ? ct[r] : cs[r];
-                mma_m16n8k32_e4m3(acc2, fa[2 * s8], fb[2 * s8], fa[2 * s8 + 1], fb[2 * s8 + 1], c.x, c.y);
-                mma_m16n8k32_e4m3(acc2, fa[2 * s8], fb[2 * s8], fa[2 * s8 + 1], fb[2 * s8 + 1], c.z, c.w);
-              }
-            }
-          } else {
-            // two 4-byte codewords per step (8 bytes each = high | low)
-#pragma unroll
-            for (int s2 = 0; s2 < NS / 2; ++s2) {
-#pragma unroll
-              for (int r = 0; r < RG; ++r) {
-                const uint2 ca = cbs[field8<BITS>(wcur[r], kFirst + 2 * s2)];
-                const uint2 cb2 = cbs[field8<BITS>(wcur[r], kFirst + 2 * s2 + 1)];
-                float (&acc2)[4] = (s2 & 1) ? ct[r] : cs[r];
-                mma_m16n8k32_e4m3(acc2, fa[2 * s2], fb[2 * s2], fa[2 * s2 + 1], fb[2 * s2 + 1], ca.x, cb2.x);
-                mma_m16n8k32_e4m3(acc2, fa[2 * s2], fb[2 * s2], fa[2 * s2 + 1], fb[2 * s2 + 1], ca.y, cb2.y);
-              }
+            for (int r = 0; r < RG; ++r) {
+              const CwVec c = codeword(r, s8);
+              float (&acc2)[4] = (s8 & 1) ? ct[r] : cs[r];
+              mma_m16n8k32_e4m3(acc2, fa[2 * s8], fb[2 * s8], fa[2 * s8 + 1], fb[2 * s8 + 1], c.x, c.y);
+              mma_m16n8k32_e4m3(acc2, fa[2 * s8], fb[2 * s8], fa[2 * s8 + 1], fb[2 * s8 + 1], c.z, c.w);
             }
           }
-        };
-        if constexpr (HALVES == 1) {
-          mma_steps(std::integral_constant<int, 0>{});
         } else {
-          if (hf == 0) mma_steps(std::integral_constant<int, 0>{});
-          else mma_steps(std::integral_constant<int, 1>{});
+          // two 4-byte codewords per step (8 bytes each = high | low)
+#pragma unroll
+          for (int s2 = 0; s2 < NS / 2; ++s2) {
+#pragma unroll
+            for (int r = 0; r < RG; ++r) {
+              const CwVec ca = codeword(r, 2 * s2), cb2 = codeword(r, 2 * s2 + 1);
+              float (&acc2)[4] = (s2 & 1) ? ct[r] : cs[r];
+              mma_m16n8k32_e4m3(acc2, fa[2 * s2], fb[2 * s2], fa[2 * s2 + 1], fb[2 * s2 + 1], ca.x, cb2.x);
+              mma_m16n8k32_e4m3(acc2, fa[2 * s2], fb[2 * s2], fa[2 * s2 + 1], fb[2 * s2 + 1], ca.y, cb2.y);
+            }
+          }
         }
 #pragma unroll
         for (int r = 0; r < RG; ++r)
 #pragma unroll
           for (int j = 0; j < 4; ++j) cs[r][j] += ct[r][j];
-        if (p.num_groups > 1) {
-          const int grp = (sp * kSpanIdx * D) / p.group_size;
-#pragma unroll
-          for (int r = 0; r < RG; ++r) {
-            s0[r0 + r] = bf16_bits_to_float(__ldg(p.scales + (int64_t)sn0[r0 + r] * p.num_groups + grp));
-            s1[r0 + r] = bf16_bits_to_float(__ldg(p.scales + (int64_t)sn1[r0 + r] * p.num_groups + grp));
-          }
-        }
+        // the scales of the two output rows this lane holds
+        const int grp = p.num_groups > 1 ? (sp * kSpanIdx * D) / p.group_size : 0;
 #pragma unroll
         for (int r = 0; r < RG; ++r) {
-          acc[r0 + r][0] = fmaf(s0[r0 + r], cs[r][0], acc[r0 + r][0]);
-          acc[r0 + r][1] = fmaf(s1[r0 + r], cs[r][1], acc[r0 + r][1]);
-          acc[r0 + r][2] = fmaf(s0[r0 + r], cs[r][2], acc[r0 + r][2]);
-          acc[r0 + r][3] = fmaf(s1[r0 + r], cs[r][3], acc[r0 + r][3]);
+          const int nl = (r0 + r) * 8 + 2 * t;
+          float s0, s1;
+          if (p.num_groups > 1) {
+            s0 = bf16_bits_to_float(__ldg(p.scales + (int64_t)min(n_base + nl, p.N - 1) * p.num_groups + grp));
+            s1 = bf16_bits_to_float(__ldg(p.scales + (int64_t)min(n_base + nl + 1, p.N - 1) * p.num_groups + grp));
+          } else {
+            s0 = rowsc_s[nl];
+            s1 = rowsc_s[nl + 1];
+          }
+          acc[r0 + r][0] = fmaf(s0, cs[r][0], acc[r0 + r][0]);
+          acc[r0 + r][1] = fmaf(s1, cs[r][1], acc[r0 + r][1]);
+          acc[r0 + r][2] = fmaf(s0, cs[r][2], acc[r0 + r][2]);
+          acc[r0 + r][3] = fmaf(s1, cs[r][3], acc[r0 + r][3]);
         }
       }
+    };
+    const int items = p.spans_per_row * HALVES;
+    int item = warp;
+    if (it == 0) {
+      if (item < items) mma_item(item, std::true_type{});
+      item += nwarps;
     }
+#pragma unroll 1
+    for (; item < items; item += nwarps) mma_item(item, std::false_type{});
     SACQ_ST(8 + 6 * it + 2);
 #pragma unroll
     for (int r = 0; r < R8; ++r) {
-      red[(warp * kFrag + r * 4 + 0) * kRedPitch + lane] = fmaf(acc[r][0], p.out_mul, p.shift * xs_a);
-      red[(warp * kFrag + r * 4 + 1) * kRedPitch + lane] = fmaf(acc[r][1], p.out_mul, p.shift * xs_a);
-      red[(warp * kFrag + r * 4 + 2) * kRedPitch + lane] = fmaf(acc[r][2], p.out_mul, p.shift * xs_b);
-      red[(warp * kFrag + r * 4 + 3) * kRedPitch + lane] = fmaf(acc[r][3], p.out_mul, p.shift * xs_b);
+      red[(warp * kFrag + r * 4 + 0) * kRedPitch + lane] = fmaf(acc[r][0], p.out_mul, 0.f);
+      red[(warp * kFrag + r * 4 + 1) * kRedPitch + lane] = fmaf(acc[r][1], p.out_mul, 0.f);
+      red[(warp * kFrag + r * 4 + 2) * kRedPitch + lane] = fmaf(acc[r][2], p.out_mul, 0.f);
+      red[(warp * kFrag + r * 4 + 3) * kRedPitch + lane] = fmaf(acc[r][3], p.out_mul, 0.f);
     }
     __syncthreads();
     SACQ_ST(8 + 6 * it + 3);
