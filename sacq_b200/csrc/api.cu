@@ -85,12 +85,13 @@ int64_t tmem_min_m(const sacq_layer* L) {
 
 // From how many tokens a split-K kernel, which walks the weights once, beats a small-M kernel, which walks them
 // once per 16-token chunk: from the second chunk on wide or deep layers, from the third on all but the smallest.
-// A codebook in L2 leaves the small-M kernel 2 warps' gathers in flight per scheduler: on wide layers the split-K
-// kernel wins from one token on (2048x6144, 65,536 entries: 17.8 / 13.4 us at 16 tokens, 46 / 15.6 at 64), on the
-// smallest from the third chunk on (2048x1024 at 32 tokens 8.3 / 9.3).
+// A codebook in L2 leaves the small-M kernel 2 warps' gathers in flight per scheduler: the split-K kernel wins from one
+// token on (65,536 entries, 2048x6144: 17.4 / 11.3 us at 16 tokens; 6144x2048 13.4 / 11.1 at one, 13.7 / 11.5 at 16;
+// 2048x2048 7.2 / 7.0 and 7.6 / 7.1), on the smallest layers from the second chunk on (2048x1024 6.4 / 7.2 at 16 and
+// 7.6 / 7.2 at 32, 1024x1024 5.5 / 5.8 and 6.4 / 5.8).
 bool split_wins(const sacq_layer* L, int64_t M) {
   const int64_t work = L->d.in_features * L->d.out_features;
-  if (!split_k_codebook_in_smem(L)) return M > (work <= (2 << 20) ? 32 : 16) || L->d.out_features >= 4096;
+  if (!split_k_codebook_in_smem(L)) return M > 16 || work > (2 << 20) || L->d.out_features >= 4096;
   return (M > 16 && (L->d.out_features >= 4096 || work >= (8 << 20))) || M > 32;
 }
 
