@@ -369,27 +369,33 @@ bool plan_unpacked(const sacq_layer* L, Plan& pl) {
   const int64_t sub = (d.out_features + 7) / 8;
   const int steps = (int)(d.in_features / 32);
   const int warps = steps < 16 ? steps : 16;
-  int64_t stride = L->num_sms / pl.chunks;
-  if (stride < 1) stride = 1;
   double best_cost = -1.0;
-  int best = 0;
+  int best = 0, best_ch = 1;
   const int r8_choices[4] = {1, 2, 4, 6};                 // 48-row tiles: one tile per SM on 6144-row layers
-  for (int ci = 0; ci < 4; ++ci) {
-    const int r8 = r8_choices[ci];
-    if (r8 > SACQ_UNPACKED_MAX_R8) continue;
-    const size_t need = small_m_mma_unpacked_smem(L->cb_entries, d.vector_dim, (int)d.in_features, L->row_bits / 8,
-                                                  (int)L->num_groups, r8, warps);
-    if (need > kSmemBudget) continue;
-    const int64_t row_tiles = (sub + r8 - 1) / r8;
-    const int64_t waves = (row_tiles + stride - 1) / stride;
-    // measured (us, dim-4 vectors with 64-wide groups on 2048 x 6144: 13.9 with three 16-row rounds, 11.95
-    // with one 48-row tile): 2.5 of launch and codebook copy, then per pass over the tiles 1.0 of fixed cost plus
-    // 1.4 per 8-row sub-block and 2048 of K (dim-8 vectors gather half as often)
-    const double cost = 2.5 + (double)waves * (1.0 + (d.vector_dim == 4 ? 1.4 : 0.8) * r8 * (double)d.in_features / 2048.0);
-    if (best_cost < 0 || cost < best_cost - 1e-9) { best_cost = cost; best = r8; }
+  const int most_ch = pl.chunks < 3 ? pl.chunks : 3;      // chunks of 16 tokens per CTA: one, or as many as there are up to three
+  for (int ch = 1; ch <= most_ch; ch += most_ch > 1 ? most_ch - 1 : 1) {
+    const int groups = (pl.chunks + ch - 1) / ch;
+    for (int ci = 0; ci < (ch > 1 ? 2 : 4); ++ci) {       // several chunks: their sums leave room for 16 rows
+      const int r8 = r8_choices[ci];
+      if (r8 > SACQ_UNPACKED_MAX_R8) continue;
+      const size_t need = small_m_mma_unpacked_smem(L->cb_entries, d.vector_dim, (int)d.in_features, L->row_bits / 8,
+                                                    (int)L->num_groups, r8, warps, ch);
+      if (need > kSmemBudget) continue;
+      const int64_t row_tiles = (sub + r8 - 1) / r8;
+      const int64_t stride = L->num_sms / groups > 1 ? L->num_sms / groups : 1;
+      const int64_t waves = (row_tiles + stride - 1) / stride;
+      // measured (us, dim-4 vectors with 64-wide groups on 2048 x 6144: 13.9 with three 16-row rounds, 11.95
+      // with one 48-row tile): 2.5 of launch and codebook copy, then per pass over the tiles 1.0 of fixed cost plus
+      // 1.4 per 8-row sub-block and 2048 of K (dim-8 vectors gather half as often), 0.4 more per further chunk
+      const double cost = 2.5 + (double)waves * (1.0 + ((d.vector_dim == 4 ? 1.4 : 0.8) + 0.4 * (ch - 1)) * r8 * (double)d.in_features / 2048.0);
+      if (best_cost < 0 || cost < best_cost - 1e-9) { best_cost = cost; best = r8; best_ch = ch; }
+    }
   }
   if (best == 0) return false;
   pl.unpacked = true;
+  pl.ch = best_ch;
+  pl.chunks = (pl.chunks + best_ch - 1) / best_ch;
+  int64_t stride = L->num_sms / pl.chunks > 1 ? L->num_sms / pl.chunks : 1;
   pl.mma = true;
   pl.staged = true;
   pl.r8 = best;
@@ -403,7 +409,7 @@ bool plan_unpacked(const sacq_layer* L, Plan& pl) {
   if (pl.grid < 1) pl.grid = 1;
   pl.act_bufs = 1;
   pl.smem = small_m_mma_unpacked_smem(L->cb_entries, d.vector_dim, (int)d.in_features, L->row_bits / 8,
-                                      (int)L->num_groups, best, warps);
+                                      (int)L->num_groups, best, warps, best_ch);
   return true;
 }
 

@@ -211,6 +211,7 @@ struct Plan {
   int r8;                    // warp-MMA variant: 8-row sub-blocks per tile (1, 2, 4; staged kernel also 6)
   bool staged;               // warp-MMA variant with bulk-copied tiles in shared memory
   int act_bufs;              // ... and how many activation tile buffers fit (1 or 2)
+  int ch;                    // ... and of 16-token chunks per CTA there (`chunks`: groups of that many)
   bool unpacked;             // warp-MMA variant that unpacks indices to 16 bits in shared memory
   size_t smem;
 };
@@ -273,7 +274,7 @@ size_t small_m_mma_staged_smem(int C, int D, int K, int64_t row_bytes, int r8, i
 
 // linear_small_m_unpacked.cu
 cudaError_t launch_small_m_mma_unpacked(const Plan& pl, const SmallMParams& p, cudaStream_t s);
-size_t small_m_mma_unpacked_smem(int C, int D, int K, int64_t row_bytes, int num_groups, int r8, int warps);
+size_t small_m_mma_unpacked_smem(int C, int D, int K, int64_t row_bytes, int num_groups, int r8, int warps, int ch);
 
 }  // namespace smallm
 }  // namespace sacq
