@@ -186,3 +186,41 @@ def test_host_result_stored_by_the_gemm(N):
         mod.forward_host(x.cpu().pin_memory(), out)
         torch.cuda.synchronize()
         assert torch.equal(out, mod(x).cpu()), M
+
+
+@pytest.mark.parametrize("N,K,d,C,G", [(520, 1024, 4, 512, 32), (300, 1536, 8, 4096, 128), (129, 6144, 4, 64, 64), (2048, 2048, 4, 1024, 64)])
+def test_unpacked_kernel_token_chunks(N, K, d, C, G):
+    """One to six chunks of 16 tokens, up to three of them in a CTA: a token's bytes are those of a call of its own chunk,
+    with and without a residual, and columns beyond the layer stay untouched."""
+    from sacq_b200 import quantize_rows
+    mod = _layer(N, K, d, C, G)
+    mod.set_kernel("small_mma_unpacked")
+    q, s = quantize_rows(_x(96, K))
+    whole = torch.cat([mod.linear_a8(q[m:m + 16], s[m:m + 16]) for m in range(0, 96, 16)])
+    assert _err(mod, whole, q, s) <= TOL
+    for M in (1, 9, 16, 17, 25, 32, 33, 47, 48, 49, 81, 96):
+        y = mod.linear_a8(q[:M], s[:M])
+        assert torch.equal(y, whole[:M]), M
+        res = _x(M, N, seed=5)
+        assert torch.equal(mod.linear_a8(q[:M], s[:M], residual=res), y + res), M
+        out = torch.full((M, N + 3), 7.0, dtype=torch.bfloat16, device="cuda")
+        mod.linear_a8(q[:M], s[:M], out=out[:, :N])
+        assert torch.equal(out[:, :N], y) and float(out[:, N:].float().min()) == 7.0, M
+    assert mod.device_status() == 0
+
+
+@pytest.mark.parametrize("kernel,N,K,d,C,G", [
+    ("large", 300, 1024, 8, 4096, None), ("large", 129, 4096, 4, 256, None), ("large", 100, 8192, 8, 4096, None),
+    ("large_grouped", 300, 2048, 4, 1024, 64), ("large_grouped", 129, 6144, 4, 64, 64)])
+def test_split_k_partial_sums(kernel, N, K, d, C, G):
+    """Token counts around the widths up to which a cluster's partial sums are sent to their owner and beyond which they are
+    fetched, and around the owners' shares: no byte depends on the way."""
+    from sacq_b200 import quantize_rows
+    mod = _layer(N, K, d, C, G)
+    mod.set_kernel(kernel)
+    q, s = quantize_rows(_x(240, K))
+    whole = mod.linear_a8(q, s)
+    assert _err(mod, whole, q, s) <= TOL
+    for M in (1, 7, 8, 9, 16, 31, 33, 48, 63, 65, 80, 95, 96, 97, 111, 112, 113, 200):
+        assert torch.equal(mod.linear_a8(q[:M], s[:M]), whole[:M]), M
+    assert mod.device_status() == 0

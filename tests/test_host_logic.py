@@ -199,3 +199,25 @@ def test_native_module_is_rebuilt_for_another_python_or_torch(tmp_path, monkeypa
     assert build.native_up_to_date()
     monkeypatch.setattr(torch, "__version__", "1.0.0")
     assert not build.native_up_to_date()
+
+
+@pytest.mark.parametrize("limit,steps", [(448.0, 24), (127.0, 12)])
+def test_two_term_reciprocal_divides_like_ieee(limit, steps):
+    """The encoders' quotient fma(z, r, z r2), r = 1/s rounded down and r2 = (1 - s r) / s, is fp32(z / s) for every scale
+    of a quantizer, fp32(largest / limit), and every bf16 dividend down to where the encoding is zero.  (80-bit extended
+    precision holds z r + z r2 exactly: 32 bits, and 24 more at 2^-24 of them.)"""
+    if np.finfo(np.longdouble).nmant < 63:
+        pytest.skip("needs 80-bit long double")
+    wide = np.longdouble
+    significands = np.arange(128, 256)
+    z = np.concatenate([significands * 2.0 ** -k for k in range(steps)]).astype(np.float32)
+    for largest in significands:
+        s = np.float32(np.float32(largest) / np.float32(limit))
+        r = np.float32(wide(1) / wide(s))
+        if wide(r) * wide(s) > 1:
+            r = np.nextafter(r, np.float32(0))
+        r2 = np.float32((wide(1) - wide(s) * wide(r)) / wide(s))
+        assert r2 >= 0
+        zz = z[z <= largest]
+        got = (zz.astype(wide) * wide(r) + (zz * r2).astype(np.float32).astype(wide)).astype(np.float32)
+        assert np.array_equal(got.view(np.uint32), (zz / s).astype(np.float32).view(np.uint32)), largest
