@@ -64,8 +64,9 @@ int64_t small_m_slab_rows(const sacq_layer* L) {
 }
 
 // Rows from which the grouped split-K kernel takes over from the index-unpacking warp-MMA kernel, which walks the
-// weights once per 16-token chunk (quantizer + GEMM, d = 4, 10-bit, group 64, the two kernels with exact weights:
-// 2048x6144 22.8 / 11.7 us at 32 rows; 1024x1024 7.5 / 6.8 and 6144x1536 35 / 13.8 at 48).
+// weights once per 48 tokens and multiplies exact weights (quantizer + GEMM, d = 4, 10-bit, group 64: 2048x6144 19.0 / 10.1 us
+// at 32 rows; 2048x2048 9.2 / 7.8 and 6144x2048 20.5 / 12.8 at 47, there with weights of 11 bits, which up to 47 rows would be
+// less than before; the smallest are even, 1024x1024 5.4 / 6.0).
 int64_t grouped_min_m(const sacq_layer* L) {
   // ... or from the CUDA-core kernel, at any number (2048x2048, 65,536 entries, group 128: 127 / 11 us at 17 rows)
   if (!L->small_m_warp_mma) return 1;

@@ -9,8 +9,8 @@
 // tiles).  Here a CTA takes 128 weight rows x ALL tokens (up to 384) x one slice of K, so each weight is
 // expanded once on the whole device, and the S CTAs of a cluster that share an output tile add their
 // fp32 partial sums through distributed shared memory:
-//   * warp 0        TMA producer: the slice's packed indices ([slice][row][16 bytes]: conflict-free
-//                   reads whatever the index width), the codebook, then the activation tiles;
+//   * warp 0        TMA producer: the slice's packed indices (64 bytes of every row per box, swizzled:
+//                   conflict-free reads whatever the index width), the codebook, then the activation tiles;
 //   * warp 1        MMA issuer: tcgen05.mma with the weights as the A operand in tensor memory, N = tokens;
 //   * warps 2..17   expanders: one weight row and a quarter of every 128-k stage each: index fields ->
 //                   codeword gathers -> tcgen05.st.  kSplitHiLo: the e4m3 high and low halves of the
@@ -21,13 +21,18 @@
 //                   token counts and layers whose other kernel multiplies exact weights.  kSplitInt8 / kSplitFp8:
 //                   the 8-bit weight bytes of the two recipes, made here instead of in a pass of their own
 //                   over a 1-byte copy of the weights;
-//   * reduction     every CTA puts its fp32 partial sums into its own shared memory, [token][row]; after a
-//                   cluster barrier each owns a token range of the tile, reads that range from its S - 1
-//                   peers (16 bytes per lane), adds the slices pairwise and writes y.
+//   * reduction     each CTA of a cluster owns a token range of the tile.  Narrow tiles: the others send it their fp32
+//                   partial sums, [token][row], and arrive at its mbarrier; wide ones: a CTA puts them into its own
+//                   shared memory and its peers fetch theirs behind a cluster barrier.  The owner adds the slices
+//                   pairwise and writes y.  (Shared memory crosses a cluster at 20 bytes a clock and SM either way; sent, it
+//                   crosses once and without barriers, but holds up the storing warps: 64 tokens, 2048 -> 2048 with the
+//                   quantizer 9.1 us fetched, 8.4 sent; 128 tokens, 2048 -> 6144 10.9 / 11.7.)
 // A CTA may take several slices, each with accumulator columns of its own: the order in which an output is
 // summed stays the same when many tokens leave no use for a cluster.
-// Every mbarrier wait is bounded (status word + CTA-wide abort flag); an aborted CTA still reaches both
-// cluster barriers, so its peers do too.  No cluster multicast.
+// In a row of calls a CTA starts when one of the call before ends, its activations come 4 us later; what it can do until then
+// is done ahead: copies, and the weights of up to seven stages.
+// Every mbarrier wait is bounded (status word + CTA-wide abort flag); an aborted CTA still reaches every
+// cluster barrier, so its peers do too, and stays until they have left.  No cluster multicast.
 #include <cuda.h>
 #include <math.h>
 #include <string.h>
