@@ -171,9 +171,9 @@ __global__ void __launch_bounds__(kMaxWarpsU * 32, 1) small_m_mma_unpacked_kerne
       const int n = min(n_base + r, p.N - 1);
       sc_s[e] = bf16_bits_to_float(__ldg(p.scales + (int64_t)n * p.num_groups + gi));
     }
-    if (threadIdx.x < kRows) {
-      const int n = min(n_base + (int)threadIdx.x, p.N - 1);
-      rowb_s[threadIdx.x] = p.bias ? bf16_bits_to_float(__ldg(p.bias + n)) : 0.f;
+    for (int r = threadIdx.x; r < kRows; r += blockDim.x) {           // a CTA may have one warp only
+      const int n = min(n_base + r, p.N - 1);
+      rowb_s[r] = p.bias ? bf16_bits_to_float(__ldg(p.bias + n)) : 0.f;
     }
     ok = mbar_wait_u(bar_pk0 + 8 * buf, pk_parity[buf], p.status) && ok;
     pk_parity[buf] ^= 1;
@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(kMaxWarpsU * 32, 1) small_m_mma_unpacked_kerne
       if (m < toks_here) bulk_g2s(act_s + m * L.act_pitch, p.q + (int64_t)(m_base + m) * p.K, (uint32_t)p.K, bar_act);
       if (m == 0) mbar_expect_u(bar_act, (uint32_t)(toks_here * p.K));
     }
-    if (threadIdx.x < kTokens) sa_s[threadIdx.x] = (int)threadIdx.x < toks_here ? __ldg(p.act_scale + m_base + threadIdx.x) : 0.f;
+    for (int m = threadIdx.x; m < kTokens; m += blockDim.x) sa_s[m] = m < toks_here ? __ldg(p.act_scale + m_base + m) : 0.f;
     if (CH == 1) ok = mbar_wait_u(bar_act, 0, p.status) && ok;
   }
 

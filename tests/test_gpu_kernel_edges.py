@@ -209,6 +209,26 @@ def test_unpacked_kernel_token_chunks(N, K, d, C, G):
     assert mod.device_status() == 0
 
 
+@pytest.mark.parametrize("N,K,d,C,bits", [(1000, 32, 4, 8192, 16), (16411, 32, 4, 4096, 16), (520, 64, 4, 256, 8), (16411, 64, 8, 4096, 16)])
+def test_unpacked_kernel_fewest_warps(N, K, d, C, bits):
+    """Layers of one or two MMA steps run CTAs of one or two warps: fewer threads than a CTA has tokens or row biases."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from sacq_b200 import PrecomputedPackedVectorCodebookLinear, pack_indices, quantize_rows
+    from sacq_b200.synthetic import make_payload
+    p = make_payload(N, K, vector_dim=d, codebook_size=C, group_size=32, seed=N + K, iters=1, fit=False, packed=False)
+    idx = p.pop("indices")
+    p.update(packed_indices=pack_indices(idx, bits), index_bits=bits, index_shape=tuple(idx.shape))
+    bias = torch.randn(N, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16)
+    mod = PrecomputedPackedVectorCodebookLinear(p, bias, "cuda")
+    mod.set_kernel("small_mma_unpacked")
+    q, s = quantize_rows(_x(64, K))
+    for M in (1, 16, 31, 33, 48, 64):
+        y = mod.linear_a8(q[:M], s[:M])
+        assert _err(mod, y, q[:M], s[:M]) <= TOL, M
+    assert mod.device_status() == 0
+
+
 @pytest.mark.parametrize("kernel,N,K,d,C,G", [
     ("large", 300, 1024, 8, 4096, None), ("large", 129, 4096, 4, 256, None), ("large", 100, 8192, 8, 4096, None),
     ("large_grouped", 300, 2048, 4, 1024, 64), ("large_grouped", 129, 6144, 4, 64, 64)])
