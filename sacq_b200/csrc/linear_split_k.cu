@@ -416,7 +416,7 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 #pragma unroll
     for (int i = 0; i < kMaxTok / 32; ++i)
       if (i * 32 + lane < tok) reinterpret_cast<float*>(sm + L.sa_off)[i * 32 + lane] = sa[i];
-    // every copy has landed before a peer writes there or the CTA ends
+    // every copy has landed before the CTA ends (the expanders see to it that none lands on partial sums)
     mbar_wait_warp(bar(IDX_FULL), 0, abort_flag, lay.status);
     if (boxes > first_boxes) mbar_wait_warp(bar(IDX_FULL + 1), 0, abort_flag, lay.status);
     if (CB_SMEM) mbar_wait_warp(bar(CB_FULL), 0, abort_flag, lay.status);
@@ -658,6 +658,9 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         cur_s[1] = nxt_s[1];
       }
     }
+    // Every CTA loads as many boxes as the longest slice of K has.  One whose own slice ends in the first of them has not
+    // waited for the others yet, and partial sums that are fetched go where those land.
+    if (ok && late >= kbs && boxes > first_boxes) ok = mbar_wait_warp(bar(IDX_FULL + 1), 0, abort_flag, lay.status);
     if (ok) ok = mbar_wait_warp(bar(ACC_FULL), 0, abort_flag, lay.status);
   }
 

@@ -244,3 +244,19 @@ def test_split_k_partial_sums(kernel, N, K, d, C, G):
     for M in (1, 7, 8, 9, 16, 31, 33, 48, 63, 65, 80, 95, 96, 97, 111, 112, 113, 200):
         assert torch.equal(mod.linear_a8(q[:M], s[:M]), whole[:M]), M
     assert mod.device_status() == 0
+
+
+@pytest.mark.parametrize("N,K,d,C,G,Ms", [(6144, 1152, 8, 65536, None, (289, 305, 320)), (2048, 4224, 4, 16, 64, (768, 700)),
+                                          (6144, 1152, 8, 65536, 128, (300, 384))])
+def test_split_k_unequal_slices(N, K, d, C, G, Ms):
+    """Slices of K of four and five (eight and nine) stages, where the longer one has a box of indices more: the partial sums
+    of the others take the place that this box was copied to."""
+    from sacq_b200 import quantize_rows
+    mod = _layer(N, K, d, C, G)
+    for M in Ms:
+        q, s = quantize_rows(_x(M, K))
+        y = mod.linear_a8(q, s)
+        assert _err(mod, y, q, s) <= TOL, M
+        for _ in range(20):
+            assert torch.equal(mod.linear_a8(q, s), y), M
+    assert mod.device_status() == 0
