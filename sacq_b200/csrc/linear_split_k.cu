@@ -56,8 +56,8 @@ using namespace tmemw;
 constexpr int kStageK = 128;          // k per weight stage
 constexpr int kMaxAct = 12;           // activation tiles in flight (128 bytes of every token each)
 constexpr int kMaxW = 7;              // weight stages in tensor memory
-constexpr int kBoxSlices = 4;         // 16-byte index slices per box (64 bytes of every row)
-constexpr int kBoxBytes = kRows * kBoxSlices * 16;
+constexpr int kSliceBytes = kRows * 16;
+constexpr int kFirstSlices = 8;       // 16-byte index slices of every row that arrive ahead of the codebook
 // fp16 forms: K may end in the middle of a stage; its second 64-k tile is then zeros on both sides.
 __host__ __device__ constexpr int stages_of(int64_t K) { return (int)((K + kStageK - 1) / kStageK); }
 __host__ __device__ constexpr int w_cols(int mode) { return mode == kSplitHalf2 ? 128 : mode >= kSplitInt8 ? 32 : 64; }
@@ -95,12 +95,12 @@ struct alignas(64) SplitParams {
   int parts;                    // consecutive slices of K per CTA, each with accumulator columns of its own
   int tok;                      // tokens per CTA (multiple of 16; of 32 above 256)
   int M, K, C, bits, num_groups, group_size;
-  int act_stages, max_slices, max_groups;
+  int act_stages, max_slices;
   int own_recv;                 // the partial sums of the cluster have shared memory of their own
   uint16_t shift;               // recipes: bf16 bits
   const float* act_scale;       // [M]
   SplitLayer layer[kSplitMaxLayers];
-  CUtensorMap idx[kSplitMaxLayers];     // [64 bytes][128 rows] boxes over the packed rows, SWIZZLE_64B
+  CUtensorMap idx[kSplitMaxLayers];     // [64 or 16 bytes][128 rows] boxes over the packed rows
   const float* row_scale;       // recipes: [N], the weight bytes' scale (the caller's buffer, not a layer constant)
   const uint16_t* residual;     // bf16 [M, ldr] added to the rounded output, or null
   int64_t ldr;
@@ -111,13 +111,13 @@ struct alignas(64) SplitParams {
 // tokens of the tile a rank reduces and writes
 __host__ __device__ constexpr int owned_tokens(int tok, int split) { return ((tok + split - 1) / split + 7) & ~7; }
 
-__host__ __device__ constexpr int index_boxes(int slices) { return (slices + kBoxSlices - 1) / kBoxSlices; }
+__host__ __device__ constexpr int index_boxes(int slices, int box_shift) { return (slices + (1 << box_shift) - 1) >> box_shift; }
 
-__host__ __device__ inline SplitLayout split_layout(int tok, int split, int act_stages, int slices, int groups, int cb_bytes,
-                                                    bool own_recv) {
+__host__ __device__ inline SplitLayout split_layout(int tok, int split, int act_stages, int slices, int box_shift, int groups,
+                                                    int cb_bytes, bool own_recv) {
   SplitLayout L;
   L.idx_off = (uint32_t)((act_stages * tok * 128 + 1023) & ~1023);
-  L.cb_off = L.idx_off + (uint32_t)(index_boxes(slices) * kBoxBytes);
+  L.cb_off = L.idx_off + (uint32_t)(index_boxes(slices, box_shift) * (kSliceBytes << box_shift));
   L.sc_off = L.cb_off + (uint32_t)((cb_bytes + 127) & ~127);
   const uint32_t pipe = L.sc_off + (uint32_t)((groups > 0 ? kRows * (groups | 1) * 2 + 127 : 0) & ~127);
   // the partial sums: [source CTA][owned token][row] of a cluster, or of a CTA alone [token][row]
@@ -206,17 +206,27 @@ __device__ __forceinline__ void add_columns(uint32_t (&r)[16], uint32_t taddr) {
   for (int j = 0; j < 16; ++j) r[j] = add_bits<INT>(r[j], b[j]);
 }
 
-// The 16-byte slice `s` (warp-uniform) of a row in the index boxes: 64 bytes of every row per box, laid out by SWIZZLE_64B,
-// so the slices of eight consecutive rows lie on different banks.  at: the row's first byte; swizzle: its ((row / 2) & 3) * 16.
-__device__ __forceinline__ uint4 index_slice(const uint8_t* at, uint32_t swizzle, int s) {
-  return *reinterpret_cast<const uint4*>(at + (s >> 2) * kBoxBytes + ((uint32_t)((s & 3) << 4) ^ swizzle));
-}
+// The packed indices of a thread's row in the boxes, 1 << BOX_SHIFT slices of 16 bytes of every row each.  64 bytes: laid out
+// by SWIZZLE_64B, so the slices of eight consecutive rows lie on different banks; 16 bytes: they do as they come.
+template <int BOX_SHIFT>
+struct IndexRow {
+  const uint8_t* at;            // the row's first byte
+  uint32_t swizzle;
+  __device__ __forceinline__ IndexRow(const uint8_t* boxes, int row)
+      : at(boxes + ((row * 16) << BOX_SHIFT)), swizzle(BOX_SHIFT == 2 ? (uint32_t)((row >> 1) & 3) << 4 : 0u) {}
+  // The 16-byte slice `s` (warp-uniform).
+  __device__ __forceinline__ uint4 slice(int s) const {
+    constexpr int kInBox = (1 << BOX_SHIFT) - 1;
+    return *reinterpret_cast<const uint4*>(at + (s >> BOX_SHIFT) * (kSliceBytes << BOX_SHIFT) + ((uint32_t)((s & kInBox) << 4) ^ swizzle));
+  }
+};
 // A window of up to 64 bits at bit `bit` of a row; `bit` is warp-uniform, `need` bits of it are used (a slice is only
 // read if one of them lies in it).
-__device__ __forceinline__ uint64_t slice_window(const uint8_t* at, uint32_t swizzle, int bit, int need) {
-  const uint4 a = index_slice(at, swizzle, bit >> 7);
+template <int BOX_SHIFT>
+__device__ __forceinline__ uint64_t slice_window(const IndexRow<BOX_SHIFT>& row, int bit, int need) {
+  const uint4 a = row.slice(bit >> 7);
   uint4 b = a;
-  if ((bit & 127) + need > 128) b = index_slice(at, swizzle, (bit >> 7) + 1);
+  if ((bit & 127) + need > 128) b = row.slice((bit >> 7) + 1);
   uint32_t lo, mid, hi;
   switch ((bit >> 5) & 3) {
     case 0: lo = a.x; mid = a.y; hi = a.z; break;
@@ -310,7 +320,7 @@ __device__ __forceinline__ void reduce_tokens(const SplitParams& p, const SplitL
 }
 
 // grid = (row tiles x split, token tiles, layers), clusters of `split` CTAs along x.
-template <int D, int MODE, bool CB_SMEM>
+template <int D, int MODE, bool CB_SMEM, int BOX_SHIFT>
 __global__ void __launch_bounds__(kCtaThreads, 1)
 split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ SplitParams p) {
   constexpr uint32_t kTmemCols = 512;
@@ -323,7 +333,7 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   const SplitLayer& lay = p.layer[blockIdx.z];
   if (n0 >= lay.N) return;                            // a narrower sibling: uniform over the cluster
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  extern __shared__ uint8_t smem_raw[];
+  extern __shared__ __align__(128) uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* sm = smem_raw + (base - raw);
@@ -350,11 +360,12 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   const int bit_begin = (kb0 * kStageK / D) * p.bits;
   const int slice0 = bit_begin >> 7;
 
-  const int boxes = index_boxes(p.max_slices), first_boxes = min(boxes, 2);
+  constexpr int kBoxBytes = kSliceBytes << BOX_SHIFT;
+  const int boxes = index_boxes(p.max_slices, BOX_SHIFT), first_boxes = min(boxes, kFirstSlices >> BOX_SHIFT);
   auto load_indices = [&](int from, int to, uint32_t full) {
     mbar_arrive_expect_tx(full, (uint32_t)((to - from) * kBoxBytes));
     for (int i = from; i < to; ++i)
-      tma_load_2d(base + L.idx_off + (uint32_t)(i * kBoxBytes), &p.idx[blockIdx.z], (slice0 + i * kBoxSlices) * 16, n0, full);
+      tma_load_2d(base + L.idx_off + (uint32_t)(i * kBoxBytes), &p.idx[blockIdx.z], (slice0 + (i << BOX_SHIFT)) * 16, n0, full);
   };
   if (warp == 0) {
     // constant operands: their copies start before anything else, those that the first stage needs first
@@ -511,15 +522,14 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     auto codeword8 = [&](uint32_t i) {
       return CB_SMEM ? *reinterpret_cast<const uint2*>(cbs + i * 8) : __ldg(reinterpret_cast<const uint2*>(cbs) + i);
     };
-    const uint8_t* rowidx = sm + L.idx_off + row * (kBoxSlices * 16);
-    const uint32_t swz = (uint32_t)((row >> 1) & 3) << 4;
+    const IndexRow<BOX_SHIFT> rowidx(sm + L.idx_off, row);
     const uint32_t mask = (1u << p.bits) - 1u;
     const int bits = p.bits;
     // One answer per warp: what follows (tcgen05.st, its wait, __syncwarp) is the whole warp's.
     ok = mbar_wait_warp(bar(IDX_FULL), 0, abort_flag, lay.status) &&
          (!CB_SMEM || mbar_wait_warp(bar(CB_FULL), 0, abort_flag, lay.status));
     // the first stage whose indices reach beyond the first boxes
-    const int late = boxes == first_boxes ? kbs : ((slice0 + first_boxes * kBoxSlices) * 128 - bit_begin) / (kStageK / D * bits);
+    const int late = boxes == first_boxes ? kbs : ((slice0 + kFirstSlices) * 128 - bit_begin) / (kStageK / D * bits);
     int grp = 0, grp_end = GROUPS ? (g_first + 1) * p.group_size - kb0 * kStageK : 0;    // k (in the slice) at which the scale changes
     // One stage's 16 words of this thread.  The next stage's words are gathered before the wait for this
     // stage's tcgen05.st: the gathers, which bound the loop, then never wait for a store's latency.
@@ -541,7 +551,7 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
           const int k = wi * kStageK + kpart * 32 + h * 16;       // in the slice
           const int g = p.num_groups == 1 ? 0 : (kb0 * kStageK + k) / p.group_size - g_first;
           const __nv_bfloat16 s = __ushort_as_bfloat16(sc[row * sc_pitch + g]);
-          const uint64_t win = slice_window(rowidx, swz, ((kb0 * kStageK + k) / D) * bits - slice0 * 128, IPT * bits);
+          const uint64_t win = slice_window(rowidx, ((kb0 * kStageK + k) / D) * bits - slice0 * 128, IPT * bits);
           uint32_t pair[8];
 #pragma unroll
           for (int j = 0; j < IPT; ++j) {
@@ -570,7 +580,7 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
           const __half2 s2 = __half2half2(__ushort_as_half(sc[row * sc_pitch + grp]));
           sc2[sub] = s2;
           const int bit = (((kb0 + wi) * kStageK + sub * 64 + kpart * 16) / D) * bits - slice0 * 128;
-          const uint64_t win = slice_window(rowidx, swz, bit, IPT * bits);
+          const uint64_t win = slice_window(rowidx, bit, IPT * bits);
 #pragma unroll
           for (int j = 0; j < IPT; ++j) {
             const uint32_t i = (uint32_t)(win >> (j * bits)) & mask;
@@ -593,7 +603,7 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         const int bit = (((kb0 + wi) * kStageK + kpart * 32) / D) * bits - slice0 * 128;
 #pragma unroll
         for (int v = 0; v < 8 / D; ++v) {             // four indices per window
-          const uint64_t win = slice_window(rowidx, swz, bit + v * 4 * bits, 4 * bits);
+          const uint64_t win = slice_window(rowidx, bit + v * 4 * bits, 4 * bits);
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const uint32_t i = (uint32_t)(win >> (j * bits)) & mask;
@@ -759,8 +769,8 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 }  // namespace
 
 struct SplitPlan {
-  CUtensorMap idx;              // boxes of [64 bytes][128 rows] over the packed rows
-  bool have;
+  CUtensorMap idx[2];           // boxes of [16 bytes][128 rows] and of [64 bytes][128 rows] over the packed rows
+  bool have[2];
 };
 
 namespace {
@@ -768,26 +778,28 @@ namespace {
 std::mutex g_split_mutex;       // layers build their index maps on first use, possibly from several host threads
 
 // Boxes of 64 bytes of 128 rows over the packed rows.  (Boxes of 16 bytes, in the order the expanders read them, cost the
-// copy engine a clock per 16 bytes: 24 slices of a row took 1.3 us longer to arrive.)
-int index_map(sacq_layer* L, CUtensorMap* out) {
+// copy engine a clock per 16 bytes: 24 slices of a row took 1.3 us longer to arrive.  They are for layers so deep that what a
+// last box of 64 bytes holds beyond the slice of K, up to 6 KB, is the room of a wider token tile.)
+int index_map(sacq_layer* L, int box_shift, CUtensorMap* out) {
   std::lock_guard<std::mutex> lock(g_split_mutex);
   if (L->split_plan == nullptr) L->split_plan = new SplitPlan();
   SplitPlan* plan = L->split_plan;
-  if (!plan->have) {
+  const int wide = box_shift != 0;
+  if (!plan->have[wide]) {
     const uint64_t row_bytes = (uint64_t)(L->row_bits / 8);
-    const int rc = encode_bytes_2d(&plan->idx, L->d.packed, row_bytes, (uint64_t)L->d.out_features, row_bytes,
-                                   (uint32_t)(kBoxSlices * 16), (uint32_t)kRows, CU_TENSOR_MAP_SWIZZLE_64B);
+    const int rc = encode_bytes_2d(&plan->idx[wide], L->d.packed, row_bytes, (uint64_t)L->d.out_features, row_bytes, 16u << box_shift,
+                                   (uint32_t)kRows, wide ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE);
     if (rc != SACQ_OK) return rc;
-    plan->have = true;
+    plan->have[wide] = true;
   }
-  *out = plan->idx;
+  *out = plan->idx[wide];
   return SACQ_OK;
 }
 
 bool is_f16(SplitMode mode) { return mode == kSplitHalf || mode == kSplitHalf2; }
 
 size_t split_smem(const SplitLayout& l) {
-  const size_t need = l.total + 1024;
+  const size_t need = l.total + 1024 - 128;           // the kernel rounds its start, a multiple of 128, up to one of 1,024
   return need < 116 * 1024 ? 116 * 1024 : need;       // two CTAs (each takes all 512 TMEM columns) never share an SM
 }
 
@@ -796,13 +808,13 @@ int active_clusters(int split, int num_sms) {
   return split == 8 ? num_sms * 15 / 148 : split == 4 ? num_sms * 33 / 148 : num_sms / split;
 }
 
-template <int D, int MODE, bool CB_SMEM>
+template <int D, int MODE, bool CB_SMEM, int BOX_SHIFT>
 cudaError_t launch_kernel(const CUtensorMap& ta, const SplitParams& p, dim3 grid, size_t smem, cudaStream_t s) {
   static bool configured[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || !configured[dev]) {
-    const cudaError_t e = cudaFuncSetAttribute(split_k_kernel<D, MODE, CB_SMEM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    const cudaError_t e = cudaFuncSetAttribute(split_k_kernel<D, MODE, CB_SMEM, BOX_SHIFT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
@@ -820,17 +832,17 @@ cudaError_t launch_kernel(const CUtensorMap& ta, const SplitParams& p, dim3 grid
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = p.split > 1 ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, split_k_kernel<D, MODE, CB_SMEM>, ta, p);
+  return cudaLaunchKernelEx(&cfg, split_k_kernel<D, MODE, CB_SMEM, BOX_SHIFT>, ta, p);
 }
 
-template <int D, bool CB_SMEM>
+template <int D, bool CB_SMEM, int BOX_SHIFT>
 cudaError_t launch_mode(SplitMode mode, const CUtensorMap& ta, const SplitParams& p, dim3 grid, size_t smem, cudaStream_t s) {
   switch (mode) {
-    case kSplitHiLo: return launch_kernel<D, kSplitHiLo, CB_SMEM>(ta, p, grid, smem, s);
-    case kSplitHalf: return launch_kernel<D, kSplitHalf, CB_SMEM>(ta, p, grid, smem, s);
-    case kSplitHalf2: return launch_kernel<D, kSplitHalf2, CB_SMEM>(ta, p, grid, smem, s);
-    case kSplitInt8: return launch_kernel<D, kSplitInt8, CB_SMEM>(ta, p, grid, smem, s);
-    default: return launch_kernel<D, kSplitFp8, CB_SMEM>(ta, p, grid, smem, s);
+    case kSplitHiLo: return launch_kernel<D, kSplitHiLo, CB_SMEM, BOX_SHIFT>(ta, p, grid, smem, s);
+    case kSplitHalf: return launch_kernel<D, kSplitHalf, CB_SMEM, BOX_SHIFT>(ta, p, grid, smem, s);
+    case kSplitHalf2: return launch_kernel<D, kSplitHalf2, CB_SMEM, BOX_SHIFT>(ta, p, grid, smem, s);
+    case kSplitInt8: return launch_kernel<D, kSplitInt8, CB_SMEM, BOX_SHIFT>(ta, p, grid, smem, s);
+    default: return launch_kernel<D, kSplitFp8, CB_SMEM, BOX_SHIFT>(ta, p, grid, smem, s);
   }
 }
 
@@ -872,18 +884,22 @@ bool split_fits(const sacq_layer* L, SplitMode mode, SplitChoice* c) {
   const int tiles = (stages_of(L->d.in_features) + c->split - 1) / c->split * (is_f16(mode) ? 2 : 1);
   const size_t most = (cb_bytes > 0 ? 224 : 164) * 1024;
   auto bytes = [&](int stages) {
-    return split_smem(split_layout(c->tok, c->split, stages, c->max_slices, groups * c->max_groups, cb_bytes, c->own_recv));
+    return split_smem(split_layout(c->tok, c->split, stages, c->max_slices, c->box_shift, groups * c->max_groups, cb_bytes, c->own_recv));
   };
   const int all = tiles < 2 ? 2 : tiles < kMaxAct ? tiles : kMaxAct;
+  c->box_shift = 2;
   if (c->split > 1 && c->tok <= (c->split == 2 ? 96 : 64)) {
     c->own_recv = true;
     for (c->act_stages = all; c->act_stages >= (all < 4 ? all : 4); --c->act_stages)
       if (bytes(c->act_stages) <= most) return true;
   }
   c->own_recv = false;
-  for (c->act_stages = all; c->act_stages > 2; --c->act_stages)
-    if (bytes(c->act_stages) <= most) return true;
-  return bytes(2) <= 227 * 1024;
+  for (; c->box_shift >= 0; c->box_shift -= 2) {
+    for (c->act_stages = all; c->act_stages > 2; --c->act_stages)
+      if (bytes(c->act_stages) <= most) return true;
+    if (bytes(2) <= 227 * 1024) return true;
+  }
+  return false;
 }
 
 // Time of one CTA with `tok` tokens and `kbs` weight stages (us): prologue, the slower of expansion, MMAs and
@@ -1014,7 +1030,7 @@ int launch_split_k(const sacq_layer* const* layers, int n, const void* act, cons
   int64_t widest = 0;
   for (int l = 0; l < n; ++l) {
     const sacq_layer* L = layers[l];
-    rc = index_map(const_cast<sacq_layer*>(L), &p.idx[l]);
+    rc = index_map(const_cast<sacq_layer*>(L), c.box_shift, &p.idx[l]);
     if (rc != SACQ_OK) return rc;
     SplitLayer& q = p.layer[l];
     q.cb = mode == kSplitHiLo ? L->cb_hilo
@@ -1043,18 +1059,22 @@ int launch_split_k(const sacq_layer* const* layers, int n, const void* act, cons
   }
   p.M = (int)M; p.K = (int)d0.in_features; p.C = mode >= kSplitInt8 ? d0.codebook_size : layers[0]->cb_entries;
   p.bits = d0.index_bits; p.num_groups = (int)layers[0]->num_groups; p.group_size = d0.group_size;
-  p.split = c.split; p.parts = c.parts; p.tok = c.tok; p.act_stages = c.act_stages; p.max_slices = c.max_slices; p.max_groups = c.max_groups;
+  p.split = c.split; p.parts = c.parts; p.tok = c.tok; p.act_stages = c.act_stages; p.max_slices = c.max_slices;
   p.own_recv = c.own_recv ? 1 : 0;
   auto log2_of = [](int v) { int n = 0; while (1 << n < v) ++n; return n; };     // split and parts are powers of two
   p.split_shift = log2_of(c.split);
   p.slice_shift = log2_of(c.split * c.parts);
   p.own = owned_tokens(c.tok, c.split);
-  p.lay = split_layout(c.tok, c.split, c.act_stages, c.max_slices, mode == kSplitHiLo ? 0 : c.max_groups, codebook_smem(layers[0]), c.own_recv);
+  p.lay = split_layout(c.tok, c.split, c.act_stages, c.max_slices, c.box_shift, mode == kSplitHiLo ? 0 : c.max_groups, codebook_smem(layers[0]), c.own_recv);
   const dim3 grid((unsigned)((widest + kRows - 1) / kRows * c.split), (unsigned)c.tiles, (unsigned)n);
   const size_t smem = split_smem(p.lay);
   const bool cb = codebook_smem(layers[0]) > 0;
-  const cudaError_t e = d0.vector_dim == 8 ? (cb ? launch_mode<8, true>(mode, ta, p, grid, smem, s) : launch_mode<8, false>(mode, ta, p, grid, smem, s))
-                                           : (cb ? launch_mode<4, true>(mode, ta, p, grid, smem, s) : launch_mode<4, false>(mode, ta, p, grid, smem, s));
+  auto launch = [&](auto box_shift) {
+    constexpr int kB = decltype(box_shift)::value;
+    if (d0.vector_dim == 8) return cb ? launch_mode<8, true, kB>(mode, ta, p, grid, smem, s) : launch_mode<8, false, kB>(mode, ta, p, grid, smem, s);
+    return cb ? launch_mode<4, true, kB>(mode, ta, p, grid, smem, s) : launch_mode<4, false, kB>(mode, ta, p, grid, smem, s);
+  };
+  const cudaError_t e = c.box_shift == 2 ? launch(std::integral_constant<int, 2>{}) : launch(std::integral_constant<int, 0>{});
   count_launch();
   if (e != cudaSuccess) return cuda_fail(e, "split-K launch");
   return SACQ_OK;

@@ -21,6 +21,7 @@ enum SplitMode {
 // How one call is cut up: token tiles of `tok` tokens, clusters of `split` CTAs with `parts` slices of K each.
 struct SplitChoice {
   int tok = 0, tiles = 0, split = 0, parts = 1, act_stages = 0, max_slices = 0, max_groups = 0;
+  int box_shift = 2;            // logarithm of the 16-byte index slices per box
   bool own_recv = false;        // whether the partial sums of a cluster have shared memory of their own
   double us = 1e30;             // modelled time
 };

@@ -260,3 +260,21 @@ def test_split_k_unequal_slices(N, K, d, C, G, Ms):
         for _ in range(20):
             assert torch.equal(mod.linear_a8(q, s), y), M
     assert mod.device_status() == 0
+
+
+@pytest.mark.parametrize("kernel,N,K,d,C,G", [
+    ("large_grouped", 200, 29696, 4, 32768, None), ("large_grouped", 300, 28672, 4, 2048, 64), ("large", 300, 28672, 8, 4096, None),
+    ("large_grouped", 129, 14336, 4, 4096, 64)])
+def test_split_k_deep_layers(kernel, N, K, d, C, G):
+    """Layers whose packed indices leave room for a token tile only as they are, without the rest of a 64-byte box: they stay on
+    the kernel, with the same widths of tiles, and no byte depends on the width of the boxes."""
+    from sacq_b200 import quantize_rows
+    mod = _layer(N, K, d, C, G)
+    assert mod.kernel_for(100) == kernel
+    mod.set_kernel(kernel)
+    q, s = quantize_rows(_x(400, K))
+    whole = mod.linear_a8(q, s)
+    assert _err(mod, whole, q, s) <= TOL
+    for M in (1, 16, 17, 100, 128, 130, 144, 145, 256, 257, 280, 289, 352, 353, 384):
+        assert torch.equal(mod.linear_a8(q[:M], s[:M]), whole[:M]), M
+    assert mod.device_status() == 0
