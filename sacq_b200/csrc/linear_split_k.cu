@@ -528,7 +528,8 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     // One answer per warp: what follows (tcgen05.st, its wait, __syncwarp) is the whole warp's.
     ok = mbar_wait_warp(bar(IDX_FULL), 0, abort_flag, lay.status) &&
          (!CB_SMEM || mbar_wait_warp(bar(CB_FULL), 0, abort_flag, lay.status));
-    // the first stage whose indices reach beyond the first boxes
+    // The first stage whose indices reach beyond the first boxes.  It is not the very first one: the boxes hold 897 bits of the
+    // slice at least, a stage has 512 at most.
     const int late = boxes == first_boxes ? kbs : ((slice0 + kFirstSlices) * 128 - bit_begin) / (kStageK / D * bits);
     int grp = 0, grp_end = GROUPS ? (g_first + 1) * p.group_size - kb0 * kStageK : 0;    // k (in the slice) at which the scale changes
     // One stage's 16 words of this thread.  The next stage's words are gathered before the wait for this
@@ -624,7 +625,6 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     uint32_t w_parity = 1;
     uint32_t cur[16], nxt[16];
     __half2 cur_s[2], nxt_s[2];
-    if (late == 0) ok = ok && mbar_wait_warp(bar(IDX_FULL + 1), 0, abort_flag, lay.status);
     if (ok) expand(0, cur, cur_s);
     __syncwarp();
     if (S > 1 && p.own_recv) cluster_wait();
