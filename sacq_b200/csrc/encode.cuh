@@ -137,8 +137,9 @@ __device__ __forceinline__ RowWeights row_weights(float sw) {
 }
 
 // 16 weights of one row -> 16 bytes: bf16(bf16(c * s) + shift) divided by the row scale and encoded.  pair: 16
-// codebook elements; s2, shift2: the scale and the shift in both halves.  A shift of zero (has_shift false) rounds nothing,
-// and only its sign matters, to a product of zero: one fused instruction.
+// codebook elements; s2, shift2: the scale and the shift in both halves.  A shift of zero (has_shift false) changes a weight in
+// its sign only, where the product is a zero or underflows to one (-0 + 0 = 0).  An int8 has no such sign: one fused instruction.
+// e4m3 keeps it, and a fused sum would round a negative product that underflows to -0: two instructions.
 template <bool I8>
 __device__ __forceinline__ void encode_weights16(const uint32_t (&pair)[8], __nv_bfloat162 s2, __nv_bfloat162 shift2,
                                                  bool has_shift, const RowWeights& r, uint32_t (&out)[4]) {
@@ -146,7 +147,7 @@ __device__ __forceinline__ void encode_weights16(const uint32_t (&pair)[8], __nv
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const __nv_bfloat162 c = *reinterpret_cast<const __nv_bfloat162*>(&pair[j]);
-    __nv_bfloat162 v = has_shift ? __hadd2_rn(__hmul2_rn(c, s2), shift2) : __hfma2(c, s2, shift2);
+    __nv_bfloat162 v = !I8 || has_shift ? __hadd2_rn(__hmul2_rn(c, s2), shift2) : __hfma2(c, s2, shift2);
     if constexpr (I8) v = __hmin2(__hmax2(v, r.neg_lim), r.lim);
     else v = __hmin2_nan(__hmax2_nan(v, r.neg_lim), r.lim);      // a NaN stays one
     w[j] = *reinterpret_cast<const uint32_t*>(&v);

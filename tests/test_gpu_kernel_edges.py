@@ -129,6 +129,26 @@ def test_weight_bytes_equal_division(K, d, C, G):
             assert torch.equal(got, _encode(w, sw.reshape(-1, 1), mode)), mode
 
 
+@pytest.mark.parametrize("K,d,C", [(1024, 8, 4096), (2048, 4, 1024), (1024, 8, 65536)])
+def test_weight_bytes_of_underflowing_products(K, d, C):
+    """Group scales so small that products of codewords underflow bf16: a product that does is a zero, to which the shift of
+    +0 is added, so its byte is that of +0; one that is still a subnormal keeps its sign."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from sacq_b200 import PrecomputedPackedVectorCodebookLinear
+    from sacq_b200.synthetic import make_payload
+    p = make_payload(40, K, vector_dim=d, codebook_size=C, group_size=64, seed=9, iters=1, fit=False)
+    p["scales"][:, 0::3] = 2.0 ** -133                   # the smallest bf16
+    p["scales"][:, 1::3] = 2.0 ** -130
+    mod = PrecomputedPackedVectorCodebookLinear(p, None, "cuda")
+    w = mod.dequantize_weight()
+    for mode, decode in (("int8_symmetric", mod.decode_weight_int8), ("fp8_e4m3fn", mod.decode_weight_fp8)):
+        sw = mod.weight_row_scale(mode)
+        got = decode(sw)
+        got = got if mode == "int8_symmetric" else got.view(torch.uint8)
+        assert torch.equal(got, _encode(w, sw.reshape(-1, 1), mode)), mode
+
+
 @pytest.mark.parametrize("M,K", [(1, 8), (3, 100), (5, 2048), (300, 2056), (2, 6144), (297, 6144), (4, 8200), (1, 40000)])
 def test_quantizer_bytes_equal_division(M, K):
     """One to four chunks per thread, a warp or a CTA per row, rows longer than the registers hold."""
