@@ -368,7 +368,7 @@ bool plan_unpacked(const sacq_layer* L, Plan& pl) {
   const sacq_layer_desc& d = L->d;
   const int64_t sub = (d.out_features + 7) / 8;
   const int steps = (int)(d.in_features / 32);
-  const int warps = steps < 16 ? steps : 16;
+  const int warps = steps < kMinWarpsU ? kMinWarpsU : steps < kMaxWarpsU ? steps : kMaxWarpsU;
   double best_cost = -1.0;
   int best = 0, best_ch = 1;
   const int r8_choices[4] = {1, 2, 4, 6};                 // 48-row tiles: one tile per SM on 6144-row layers

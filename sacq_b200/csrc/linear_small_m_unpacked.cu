@@ -28,7 +28,6 @@ namespace smallm {
 namespace {
 
 constexpr int kActPadU = 32;                      // bytes of padding per staged activation row
-constexpr int kMaxWarpsU = 16;
 
 __device__ __forceinline__ uint32_t sm_addr_u(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint32_t bar) {
@@ -109,6 +108,7 @@ __global__ void __launch_bounds__(kMaxWarpsU * 32, 1) small_m_mma_unpacked_kerne
   constexpr int kFrag = R8 * 4;
   constexpr int kRows = 8 * R8;
   constexpr int kTokens = 16 * CH;
+  static_assert(kRows <= 32 * kMinWarpsU && kTokens <= 32 * kMinWarpsU, "row constants and token scales: a thread each");
   constexpr int GPS = D == 8 ? 1 : 2;                                 // gathers per step and 8-row sub-block
   constexpr int PS = R8 > 2 ? 1 : CH > 1 ? 2 : 4;                     // steps gathered ahead: what the registers hold
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -171,9 +171,9 @@ __global__ void __launch_bounds__(kMaxWarpsU * 32, 1) small_m_mma_unpacked_kerne
       const int n = min(n_base + r, p.N - 1);
       sc_s[e] = bf16_bits_to_float(__ldg(p.scales + (int64_t)n * p.num_groups + gi));
     }
-    for (int r = threadIdx.x; r < kRows; r += blockDim.x) {           // a CTA may have one warp only
-      const int n = min(n_base + r, p.N - 1);
-      rowb_s[r] = p.bias ? bf16_bits_to_float(__ldg(p.bias + n)) : 0.f;
+    if (threadIdx.x < kRows) {
+      const int n = min(n_base + (int)threadIdx.x, p.N - 1);
+      rowb_s[threadIdx.x] = p.bias ? bf16_bits_to_float(__ldg(p.bias + n)) : 0.f;
     }
     ok = mbar_wait_u(bar_pk0 + 8 * buf, pk_parity[buf], p.status) && ok;
     pk_parity[buf] ^= 1;
@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(kMaxWarpsU * 32, 1) small_m_mma_unpacked_kerne
       if (m < toks_here) bulk_g2s(act_s + m * L.act_pitch, p.q + (int64_t)(m_base + m) * p.K, (uint32_t)p.K, bar_act);
       if (m == 0) mbar_expect_u(bar_act, (uint32_t)(toks_here * p.K));
     }
-    for (int m = threadIdx.x; m < kTokens; m += blockDim.x) sa_s[m] = m < toks_here ? __ldg(p.act_scale + m_base + m) : 0.f;
+    if (threadIdx.x < kTokens) sa_s[threadIdx.x] = (int)threadIdx.x < toks_here ? __ldg(p.act_scale + m_base + threadIdx.x) : 0.f;
     if (CH == 1) ok = mbar_wait_u(bar_act, 0, p.status) && ok;
   }
 

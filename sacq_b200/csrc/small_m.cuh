@@ -274,6 +274,7 @@ size_t small_m_mma_staged_smem(int C, int D, int K, int64_t row_bytes, int r8, i
 
 // linear_small_m_unpacked.cu
 cudaError_t launch_small_m_mma_unpacked(const Plan& pl, const SmallMParams& p, cudaStream_t s);
+constexpr int kMinWarpsU = 2, kMaxWarpsU = 16;   // per CTA; a thread for every token and row of a tile (48 at most)
 size_t small_m_mma_unpacked_smem(int C, int D, int K, int64_t row_bytes, int num_groups, int r8, int warps, int ch);
 
 }  // namespace smallm
