@@ -101,6 +101,14 @@ __host__ __device__ inline UnpLayout unp_layout(int C, int D, int K, int64_t row
   return L;
 }
 
+// Eight bytes that the kernel in front may have written while this grid was resident: no ld.global.nc.  volatile keeps it
+// behind griddepcontrol.wait.
+__device__ __forceinline__ uint2 load_written(const uint8_t* at) {
+  uint2 v;
+  asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(at));
+  return v;
+}
+
 template <int D, int R8, int CH>
 __global__ void __launch_bounds__(kMaxWarpsU * 32, 1) small_m_mma_unpacked_kernel(const SmallMParams p) {
   extern __shared__ __align__(128) uint8_t smem[];
@@ -254,8 +262,8 @@ __global__ void __launch_bounds__(kMaxWarpsU * 32, 1) small_m_mma_unpacked_kerne
       if (mb < toks_here) xb = *reinterpret_cast<const uint2*>(act_s + (g + 8) * L.act_pitch + 8 * t + st * 32);
     } else {
       const uint8_t* q = p.q + (int64_t)(m_base + ma) * p.K + 8 * t + st * 32;
-      if (ma < toks_here) xa = __ldg(reinterpret_cast<const uint2*>(q));
-      if (mb < toks_here) xb = __ldg(reinterpret_cast<const uint2*>(q + 8 * (int64_t)p.K));
+      if (ma < toks_here) xa = load_written(q);
+      if (mb < toks_here) xb = load_written(q + 8 * (int64_t)p.K);
     }
   };
 
