@@ -103,7 +103,6 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) small_m_kernel(const SmallM
   bool row_ok = false;
   const uint32_t* wsrc = nullptr;
   uint32_t wg[WPG];
-  float xsum[MT];
 
   auto decode_item = [&](int64_t item) {
     sg = (int)(item % p.num_sg);
@@ -142,14 +141,6 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) small_m_kernel(const SmallM
       act4_to_h2(p.act_int8, o[m].x, h.x, h.y);
       if constexpr (D == 8) act4_to_h2(p.act_int8, o[m].y, h.z, h.w);
       xs[m * kSpanIdx + lane] = h;
-      if (p.shift != 0.f) {
-        float t = __low2float(as_h2(h.x)) + __high2float(as_h2(h.x)) + __low2float(as_h2(h.y)) +
-                  __high2float(as_h2(h.y));
-        if constexpr (D == 8)
-          t += __low2float(as_h2(h.z)) + __high2float(as_h2(h.z)) + __low2float(as_h2(h.w)) +
-               __high2float(as_h2(h.w));
-        xsum[m] += warp_sum(t);
-      }
     }
     __syncwarp();
   };
@@ -157,8 +148,6 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) small_m_kernel(const SmallM
   const int64_t total_warps = (int64_t)gridDim.x * nwarps;
   int64_t item = (int64_t)warp * gridDim.x + blockIdx.x;
   bool have = item < p.num_items;
-#pragma unroll
-  for (int m = 0; m < MT; ++m) xsum[m] = 0.f;
   if (have) {
     decode_item(item);
     load_span(sp_begin);                // overlaps the codebook copy
@@ -221,10 +210,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) small_m_kernel(const SmallM
 
     float val[MT];
 #pragma unroll
-    for (int m = 0; m < MT; ++m) {
-      val[m] = fmaf(acc[m], p.out_mul, p.shift * xsum[m]);
-      xsum[m] = 0.f;
-    }
+    for (int m = 0; m < MT; ++m) val[m] = fmaf(acc[m], p.out_mul, 0.f);
     finish_rows<MT>(p, chunk, rb, sg, val, n, row_ok);
 
     item += total_warps;
@@ -788,8 +774,6 @@ int launch_small_m_multi(const sacq_layer* const* layers, int n, const void* q, 
     g.N[l] = (int)L->d.out_features;
     g.row_blocks[l] = rb[l];
     g.out_mul[l] = ldexpf(1.f, -L->cb8_exp_shift);
-    const uint32_t sb = (uint32_t)L->d.shift_bf16 << 16;
-    memcpy(&g.shift[l], &sb, sizeof(float));
   }
   g.cta_begin[n] = cta;
   pl.grid = cta;

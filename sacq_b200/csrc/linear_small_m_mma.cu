@@ -120,7 +120,6 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) small_m_mma_kernel(const Sm
     for (int r = 0; r < R8; ++r)
 #pragma unroll
       for (int j = 0; j < 4; ++j) acc[r][j] = 0.f;
-    float xs_a = 0.f, xs_b = 0.f;
 
     int sp = warp;
     for (; sp < p.spans_per_row; sp += nwarps) {
@@ -141,22 +140,6 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) small_m_mma_kernel(const Sm
             act4_to_h2(p.act_int8, wb[s], fb[s][0], fb[s][1]);
           }
         }
-      }
-      if (p.shift != 0.f) {
-        float ta = 0.f, tb = 0.f;
-#pragma unroll
-        for (int s = 0; s < 8; ++s)
-#pragma unroll
-          for (int j = 0; j < AREG; ++j) {
-            ta += __low2float(as_h2(fa[s][j])) + __high2float(as_h2(fa[s][j]));
-            tb += __low2float(as_h2(fb[s][j])) + __high2float(as_h2(fb[s][j]));
-          }
-        ta += __shfl_xor_sync(0xffffffffu, ta, 1);
-        ta += __shfl_xor_sync(0xffffffffu, ta, 2);
-        tb += __shfl_xor_sync(0xffffffffu, tb, 1);
-        tb += __shfl_xor_sync(0xffffffffu, tb, 2);
-        xs_a += ta;
-        xs_b += tb;
       }
       uint32_t wcur[R8][WPG];
 #pragma unroll
@@ -206,10 +189,10 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) small_m_mma_kernel(const Sm
     // ---- K reduction across the CTA's warps, then the epilogue
 #pragma unroll
     for (int r = 0; r < R8; ++r) {
-      red[(warp * kFrag + r * 4 + 0) * 32 + lane] = fmaf(acc[r][0], p.out_mul, p.shift * xs_a);
-      red[(warp * kFrag + r * 4 + 1) * 32 + lane] = fmaf(acc[r][1], p.out_mul, p.shift * xs_a);
-      red[(warp * kFrag + r * 4 + 2) * 32 + lane] = fmaf(acc[r][2], p.out_mul, p.shift * xs_b);
-      red[(warp * kFrag + r * 4 + 3) * 32 + lane] = fmaf(acc[r][3], p.out_mul, p.shift * xs_b);
+      red[(warp * kFrag + r * 4 + 0) * 32 + lane] = fmaf(acc[r][0], p.out_mul, 0.f);
+      red[(warp * kFrag + r * 4 + 1) * 32 + lane] = fmaf(acc[r][1], p.out_mul, 0.f);
+      red[(warp * kFrag + r * 4 + 2) * 32 + lane] = fmaf(acc[r][2], p.out_mul, 0.f);
+      red[(warp * kFrag + r * 4 + 3) * 32 + lane] = fmaf(acc[r][3], p.out_mul, 0.f);
     }
     __syncthreads();
     for (int e = threadIdx.x; e < kFrag * 32; e += blockDim.x) {
@@ -682,7 +665,6 @@ __global__ void __launch_bounds__(kMaxWarps * 32 * HALVES, 1) small_m_mma_staged
   p.N = g.N[l];
   p.row_blocks = g.row_blocks[l];
   p.out_mul = g.out_mul[l];
-  p.shift = g.shift[l];
   staged_body<D, BITS, R8, HALVES>(p, (int)blockIdx.x - g.cta_begin[l], g.cta_begin[l + 1] - g.cta_begin[l]);
 }
 

@@ -9,8 +9,8 @@
 // tiles).  Here a CTA takes 128 weight rows x ALL tokens (up to 384) x one slice of K, so each weight is
 // expanded once on the whole device, and the S CTAs of a cluster that share an output tile add their
 // fp32 partial sums through distributed shared memory:
-//   * warp 0        TMA producer: the slice's packed indices (64 bytes of every row per box, swizzled:
-//                   conflict-free reads whatever the index width), the codebook, then the activation tiles;
+//   * warp 0        TMA producer: the slice's packed indices (64 bytes of every row per box, swizzled, or 16 on the deepest
+//                   layers: conflict-free reads whatever the index width), the codebook, then the activation tiles;
 //   * warp 1        MMA issuer: tcgen05.mma with the weights as the A operand in tensor memory, N = tokens;
 //   * warps 2..17   expanders: one weight row and a quarter of every 128-k stage each: index fields ->
 //                   codeword gathers -> tcgen05.st.  kSplitHiLo: the e4m3 high and low halves of the
@@ -238,10 +238,11 @@ __device__ __forceinline__ uint64_t slice_window(const IndexRow<BOX_SHIFT>& row,
   return ((uint64_t)__funnelshift_r(mid, hi, sh) << 32) | __funnelshift_r(lo, mid, sh);
 }
 
-// Adds the slices of K pairwise, (0 + 1) + (2 + 3) and so on, whichever CTA does it, and writes y: tokens [0, count) of this CTA's share,
-// a warp per token, four consecutive outputs per lane.  `part` = this lane's partial sums of token 0 in the CTA's own
-// shared memory; those of the other CTAs are `stride` bytes apart, or (PEER) at the same place in theirs.  Everything that does not depend on the token is set up once: this loop is bound by
-// instruction issue (with the addresses and alignment tests inside it took 0.4 us per token and warp).
+// Adds the slices of K pairwise, (0 + 1) + (2 + 3) and so on, whichever CTA does it, and writes y: tokens [0, count) of this
+// CTA's share, a warp per token, four consecutive outputs per lane.  `part` = this lane's partial sums of token 0 in the CTA's
+// own shared memory; those of the other CTAs are `stride` bytes apart, or (PEER) at the same place in theirs.  Everything that
+// does not depend on the token is set up once: this loop is bound by instruction issue (with the addresses and alignment tests
+// inside it took 0.4 us per token and warp).
 template <int S, bool INT, bool PEER>
 __device__ __forceinline__ void reduce_tokens(const SplitParams& p, const SplitLayer& lay, int warp, int lane, int count,
                                               int m_first, int n0, uint32_t part, uint32_t stride, const float* sa, float4 sw,
@@ -349,10 +350,10 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   const int rank = S > 1 ? (int)cluster_rank() : 0;
   const int m0 = blockIdx.y * p.tok;
   const int nkb = stages_of(p.K);
-  const int parts = p.parts, slices = p.slice_shift;  // (a logarithm)
+  const int parts = p.parts, slice_shift = p.slice_shift;
   // this CTA's weight stages, and the first one (counted from kb0) of its slice `v`
-  const int kb0 = rank * parts * nkb >> slices, kbs = ((rank + 1) * parts * nkb >> slices) - kb0;
-  auto part_begin = [&](int v) { return ((rank * parts + v) * nkb >> slices) - kb0; };
+  const int kb0 = rank * parts * nkb >> slice_shift, kbs = ((rank + 1) * parts * nkb >> slice_shift) - kb0;
+  auto part_begin = [&](int v) { return ((rank * parts + v) * nkb >> slice_shift) - kb0; };
   const int tok = p.tok, acc_cols = tok * parts;
   const bool halves = tok > 256;                      // an instruction (and a TMA box) takes at most 256 tokens
   const int w_stages = min(kMaxW, ((int)kTmemCols - acc_cols) / W_COLS);

@@ -44,11 +44,11 @@ struct SmallMParams {
   int spans_per_item;          // consecutive spans one item covers
   int num_sg;                  // span groups per row = ceil(spans_per_row / spans_per_item)
   int row_blocks;              // ceil(N / 32)
-  int chunks;                  // ceil(M / MT)
+  int chunks;                  // ceil(M / MT); index-unpacking kernel: groups of as many 16-token chunks as a CTA multiplies
   int act_bufs;                // staged warp-MMA kernel: activation tile buffers (1 or 2)
   int64_t num_items;
   float out_mul;               // 2^-cb_exp_shift (fast) or 1 (generic)
-  float shift;
+  float shift;                 // generic kernel (a layer with a shift runs on no other)
   int act_int8;                // activations are int8 (the deployed recipe) instead of e4m3
   int n_bc;                    // further copies of the output (peer GPUs' buffers), same pitch as y
   uint16_t* ybc[kMaxBcast];
@@ -71,7 +71,6 @@ struct MultiParams {
   int N[kMaxMulti];
   int row_blocks[kMaxMulti];
   float out_mul[kMaxMulti];
-  float shift[kMaxMulti];
 };
 
 // Output store shared by every small-M variant: y = bf16(v), or bf16(bf16(v) + residual) --
