@@ -149,6 +149,49 @@ def test_weight_bytes_of_underflowing_products(K, d, C):
         assert torch.equal(got, _encode(w, sw.reshape(-1, 1), mode)), mode
 
 
+# The significands (24 bits, of row scales in [1, 2)) for which the encoders' quotient of some bf16 weight is not the division's:
+# by one ulp, of a quotient that no encoding has a boundary next to (tests/test_host_logic.py finds them).
+ODD_ROW_SCALES = (0x3f9cdfab, 0x3fbc49ab, 0x3fd0ab43, 0x3fd2d00f, 0x3fdb4e6b, 0x3fe190f3, 0x3fe241ef, 0x3fe5ae9f, 0x3feb3ca3,
+                  0x3ff28673, 0x3ff92863)
+
+
+def test_weight_bytes_for_any_row_scale():
+    """A caller's row scales: the odd ones, small whole numbers (quotients that are exact ties), random significands, each at
+    magnitudes where a row's quotients reach from zero to saturation.  Weights: every significand of a bf16 number at 16
+    exponents, both signs.  The bytes are those of the division; so are those that the GEMMs make for themselves."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from sacq_b200 import PrecomputedPackedVectorCodebookLinear, pack_indices
+    g = torch.Generator().manual_seed(4)
+    values = (torch.arange(128, 256) / 128.0).reshape(1, -1) * 2.0 ** torch.arange(-9, 7).reshape(-1, 1)
+    values = values.reshape(-1) * torch.tensor([1.0, -1.0]).repeat(1024)
+    base = torch.cat([torch.tensor(ODD_ROW_SCALES, dtype=torch.int32).view(torch.float32), torch.arange(1, 16).float(),
+                      (0x3f800000 + torch.randint(0, 1 << 23, (230,), generator=g, dtype=torch.int32)).view(torch.float32)])
+    sw = torch.cat([base * 2.0 ** -8, base * 2.0 ** -3, base]).cuda()
+    N, K = sw.numel(), 2048
+    idx = torch.stack([torch.randperm(256, generator=g) for _ in range(N)]).reshape(N, 1, 256)
+    payload = dict(format="packed_vector_codebook_v1", codebook=values[torch.randperm(2048, generator=g)].reshape(256, 8).bfloat16(),
+                   scales=torch.ones(N, 1).bfloat16(), shift=torch.zeros((), dtype=torch.bfloat16), in_features=K, out_features=N,
+                   group_size=K, vector_dim=8, packed_indices=pack_indices(idx, 8), index_bits=8, index_shape=(N, 1, 256))
+    mod = PrecomputedPackedVectorCodebookLinear(payload, None, "cuda")
+    w = mod.dequantize_weight()
+    for mode, decode, linear in (("int8_symmetric", mod.decode_weight_int8, mod.linear_w8a8_int8),
+                                 ("fp8_e4m3fn", mod.decode_weight_fp8, mod.linear_w8a8_fp8)):
+        rows = sw.reshape(mod.weight_row_scale(mode).shape).contiguous()
+        want = _encode(w, sw.reshape(-1, 1), mode)
+        got = decode(rows)
+        assert torch.equal(got if mode == "int8_symmetric" else got.view(torch.uint8), want), mode
+        bytes_of = want.float() if mode == "int8_symmetric" else want.view(torch.float8_e4m3fn).float()
+        for M in (32, 300):                              # weight bytes made inside the GEMM, and by a kernel of their own
+            k = torch.randperm(K, generator=g)[:M].cuda()
+            q = torch.zeros(M, K, device="cuda")
+            q[torch.arange(M), k] = 1.0
+            q = q.to(torch.int8 if mode == "int8_symmetric" else torch.float8_e4m3fn)
+            y = linear(q, torch.ones(M, 1, device="cuda"), rows)
+            assert torch.equal(y, (bytes_of[:, k].t() * sw.reshape(1, -1)).to(torch.bfloat16)), (mode, M)
+    assert mod.device_status() == 0
+
+
 @pytest.mark.parametrize("M,K", [(1, 8), (3, 100), (5, 2048), (300, 2056), (2, 6144), (297, 6144), (4, 8200), (1, 40000)])
 def test_quantizer_bytes_equal_division(M, K):
     """One to four chunks per thread, a warp or a CTA per row, rows longer than the registers hold."""

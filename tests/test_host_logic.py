@@ -1,6 +1,8 @@
 """CPU tests of the host-side code: bit packing, payload handling, the shared library's
 exported symbols.  No compute call is made (there is no GPU here)."""
 import ctypes
+import signal
+import subprocess
 
 import numpy as np
 import pytest
@@ -203,9 +205,10 @@ def test_native_module_is_rebuilt_for_another_python_or_torch(tmp_path, monkeypa
 
 @pytest.mark.parametrize("limit,steps", [(448.0, 24), (127.0, 12)])
 def test_two_term_reciprocal_divides_like_ieee(limit, steps):
-    """The encoders' quotient fma(z, r, z r2), r = 1/s rounded down and r2 = (1 - s r) / s, is fp32(z / s) for every scale
-    of a quantizer, fp32(largest / limit), and every bf16 dividend down to where the encoding is zero.  (80-bit extended
-    precision holds z r + z r2 exactly: 32 bits, and 24 more at 2^-24 of them.)"""
+    """The arithmetic of the encoders' quotient, restated: fma(z, r, z r2), r = 1/s rounded down and r2 = (1 - s r) / s, is
+    fp32(z / s) for every scale of a quantizer, fp32(largest / limit), and every bf16 dividend down to where the encoding is
+    zero.  (80-bit extended precision holds z r + z r2 exactly: 32 bits, and 24 more at 2^-24 of them.)  The kernels' own bytes
+    are compared in test_gpu_kernel_edges.py."""
     if np.finfo(np.longdouble).nmant < 63:
         pytest.skip("needs 80-bit long double")
     wide = np.longdouble
@@ -221,3 +224,52 @@ def test_two_term_reciprocal_divides_like_ieee(limit, steps):
         zz = z[z <= largest]
         got = (zz.astype(wide) * wide(r) + (zz * r2).astype(np.float32).astype(wide)).astype(np.float32)
         assert np.array_equal(got.view(np.uint32), (zz / s).astype(np.float32).view(np.uint32)), largest
+
+
+_QUOTIENTS = r"""
+#include <math.h>
+#include <stdint.h>
+#include <stdio.h>
+#include <string.h>
+static float value(uint32_t b) { float v; memcpy(&v, &b, 4); return v; }
+static uint32_t bits(float v) { uint32_t b; memcpy(&b, &v, 4); return b; }
+int main(void) {
+  for (uint32_t m = 0; m < 1u << 23; ++m) {
+    const float s = value(0x3f800000u | m);
+    float r = (float)(1.0 / (double)s);                 /* rounded down below: 1/s lies within an ulp of it */
+    if ((double)r * (double)s > 1.0) r = value(bits(r) - 1);
+    const float r2 = fmaf(-s, r, 1.0f) / s;
+    int differ = 0;
+    for (uint32_t i = 0; i < 128; ++i) {
+      const float z = value(0x3f800000u | i << 16);
+      differ |= bits(fmaf(z, r, z * r2)) != bits(z / s);
+    }
+    for (uint32_t i = 0; differ && i < 128; ++i) {
+      const float z = value(0x3f800000u | i << 16), q = fmaf(z, r, z * r2);
+      if (bits(q) != bits(z / s)) printf("%x %x %x\n", bits(s), bits(q), bits(z / s));
+    }
+  }
+  return 0;
+}
+"""
+
+
+def test_quotient_of_every_significand(tmp_path):
+    """The arithmetic of the encoders' quotient (csrc/encode.cuh: r = 1/s rounded down, r2 = (1 - s r) / s, fma(z, r, z r2)) for
+    all 2^23 significands of a row scale and all 128 of a bf16 dividend: 11 differ from the division, by one ulp, and neither
+    number is one of at most 16 significant bits, as every boundary between two codes is (e4m3: five bits, int8: eight).  So no
+    byte differs.  The bytes of the kernels themselves for these 11 scales: tests/test_gpu_kernel_edges.py."""
+    src = tmp_path / "quotients.c"
+    src.write_text(_QUOTIENTS)
+    build = subprocess.run(["gcc", "-O3", "-mfma", "-ffp-contract=off", str(src), "-o", str(tmp_path / "quotients"), "-lm"], capture_output=True)
+    if build.returncode != 0:
+        pytest.skip("needs gcc for a CPU with fused multiply-add")
+    run = subprocess.run([str(tmp_path / "quotients")], capture_output=True, text=True)
+    if run.returncode == -signal.SIGILL:
+        pytest.skip("needs a CPU with fused multiply-add")
+    lines = run.stdout.split()
+    found = np.array([int(v, 16) for v in lines], dtype=np.int64).reshape(-1, 3)
+    from test_gpu_kernel_edges import ODD_ROW_SCALES
+    assert tuple(found[:, 0]) == ODD_ROW_SCALES
+    assert np.abs(found[:, 1] - found[:, 2]).max() == 1
+    assert np.all(found[:, 1:] & 0xff)
