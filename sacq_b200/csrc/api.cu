@@ -66,7 +66,8 @@ int64_t small_m_slab_rows(const sacq_layer* L) {
 // Rows from which the grouped split-K kernel takes over from the index-unpacking warp-MMA kernel, which walks the
 // weights once per 48 tokens and multiplies exact weights (quantizer + GEMM, d = 4, 10-bit, group 64: 2048x6144 19.0 / 10.1 us
 // at 32 rows; 2048x2048 9.2 / 7.8 and 6144x2048 20.5 / 12.8 at 47, there with weights of 11 bits, which up to 47 rows would be
-// less than before; the smallest are even, 1024x1024 5.4 / 6.0).
+// less than before; the smallest lose a tenth, 1024x1024 5.4 / 6.0).  Whether wide layers gain below 17 rows in calls with the
+// quantizer is not measured; the GEMM alone does (2048x6144 at 16 12.1 / 9.4).
 int64_t grouped_min_m(const sacq_layer* L) {
   // ... or from the CUDA-core kernel, at any number (2048x2048, 65,536 entries, group 128: 127 / 11 us at 17 rows)
   if (!L->small_m_warp_mma) return 1;

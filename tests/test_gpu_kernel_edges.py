@@ -332,7 +332,7 @@ def test_split_k_deep_layers(kernel, N, K, d, C, G):
     """Layers whose packed indices leave room for a token tile only as they are, without the rest of a 64-byte box: they stay on
     the kernel, with the same widths of tiles, and no byte depends on the width of the boxes."""
     from sacq_b200 import quantize_rows
-    mod = _layer(N, K, d, C, G)
+    mod = _layer(N, K, d, C, G, bias=False)
     assert mod.kernel_for(100) == kernel
     mod.set_kernel(kernel)
     q, s = quantize_rows(_x(400, K))
@@ -340,4 +340,10 @@ def test_split_k_deep_layers(kernel, N, K, d, C, G):
     assert _err(mod, whole, q, s) <= TOL
     for M in (1, 16, 17, 100, 128, 130, 144, 145, 256, 257, 280, 289, 352, 353, 384):
         assert torch.equal(mod.linear_a8(q[:M], s[:M]), whole[:M]), M
+    sw = mod.weight_row_scale("int8_symmetric")          # weight bytes made inside the GEMM: int32 sums are exact
+    qi, si = quantize_rows(_x(32, K), "int8_symmetric")
+    acc = qi.double() @ mod.decode_weight_int8(sw).double().t()
+    want = ((acc.float() * sw.reshape(1, -1)) * si.reshape(-1, 1)).to(torch.bfloat16)
+    for M in (1, 16, 32):
+        assert torch.equal(mod.linear_w8a8_int8(qi[:M], si[:M], sw), want[:M]), M
     assert mod.device_status() == 0
