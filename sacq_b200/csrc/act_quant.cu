@@ -131,6 +131,7 @@ quant_act_kernel(const uint16_t* __restrict__ x, int64_t pitch, int64_t K, uint8
 // are 16-byte aligned, K % 8 == 0.
 constexpr int kRowsPerCta = 8;
 constexpr int kKeepChunks = 8;
+constexpr int64_t kRowsKernelMaxK = 256 * kKeepChunks;   // rows the lanes hold entirely in registers
 
 template <bool I8, bool WIDE>
 __global__ void __launch_bounds__(kRowsPerCta * 32)
@@ -165,12 +166,89 @@ quant_act_rows_kernel(const uint16_t* __restrict__ x, int64_t pitch, int64_t M, 
     store8<I8, WIDE>(qrow, ch, encode8<I8>(__ldg(row + ch), d));
 }
 
+// The same quantizer in front of a split-K GEMM (linear_split_k.cu), made to share an SM with that kernel's CTAs.  In a row of
+// calls this grid waits for the GEMM before it while the GEMM behind it already fetches and expands weights, so whatever
+// keeps the three apart is paid on every call.  Two things did.  An SM whose memory is divided for a kernel of little
+// shared memory takes no CTA of the GEMM before it is idle again, hence the launch's carve-out.  And a GEMM CTA (18 warps of
+// 88 registers) leaves 2,304 registers of an SM quarter: a warp of up to 72, where the row kernels have two or six.  GEMM CTAs
+// entered only when the one before had left, 1 to 2 us late.  Quantizer + GEMM in a graph, without / with this kernel:
+// 2048 -> 2048 at 64 tokens 7.5 / 6.5 us, 128 9.2 / 7.6, 6144 -> 2048 at 64 11.0 / 9.6, 128 13.2 / 11.5, 2048 -> 6144 at 64
+// 9.2 / 8.2, 300 16.0 / 14.4, 2048 -> 2048, d = 4, at 100 10.9 / 8.0.
+// T threads per row, 128 / T rows per CTA; a row lies in registers between the passes, CH 16-byte chunks per thread.
+// Same arithmetic, same bytes.
+constexpr int kBesideThreads = 128;
+
+template <int T, int CH, bool I8, bool WIDE>
+__global__ void __launch_bounds__(kBesideThreads, 7)
+quant_act_beside_kernel(const uint16_t* __restrict__ x, int64_t pitch, int64_t M, int64_t K, uint8_t* __restrict__ q,
+                        float* __restrict__ scale_out) {
+  constexpr int W = T / 32;                          // warps per row
+  __shared__ uint32_t red[kBesideThreads / 32];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int tid = threadIdx.x % T;
+  const int64_t m = (int64_t)blockIdx.x * (kBesideThreads / T) + threadIdx.x / T;
+  const bool live = m < M;
+  const uint4* row = reinterpret_cast<const uint4*>(x + m * pitch);
+  uint8_t* qrow = q + m * K * (WIDE ? 2 : 1);
+  const int64_t chunks = live ? K >> 3 : 0;
+  uint4 keep[CH];
+#pragma unroll
+  for (int c = 0; c < CH; ++c) {
+    const int64_t ch = tid + c * T;
+    keep[c] = make_uint4(0, 0, 0, 0);
+    if (ch < chunks) keep[c] = __ldg(row + ch);
+  }
+  uint32_t mx = 0u;
+#pragma unroll
+  for (int c = 0; c < CH; ++c) mx = chunk_max(mx, keep[c]);
+  mx = warp_max_bits(pair_max_bits(mx));
+  if constexpr (W > 1) {
+    const int warp = threadIdx.x >> 5;
+    if ((threadIdx.x & 31) == 0) red[warp] = mx;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < W; ++w) mx = max(mx, red[warp / W * W + w]);
+  }
+  const RowDivisor d = scale_of<I8>(__uint_as_float(mx));
+  if (live && tid == 0) scale_out[m] = d.s;
+#pragma unroll
+  for (int c = 0; c < CH; ++c) {
+    const int64_t ch = tid + c * T;
+    if (ch < chunks) store8<I8, WIDE>(qrow, ch, encode8<I8>(keep[c], d));
+  }
+}
+
+// Threads per row of the kernel above; 0: one of the others.  A row per CTA while about two per SM hold the rows (370:
+// 6144 -> 2048 at 290 tokens 16.1 / 15.1 us, at 450 18.9 / 19.5), beyond that a warp per row, where its registers hold one
+// (2048 -> 2048 at 700: row CTAs 13.6, warps 12.2 us).
+inline int beside_threads(int64_t M, int64_t K) {
+  if (M <= 370 && K <= kBesideThreads * 8 * kKeepChunks) return kBesideThreads;
+  return K <= kRowsKernelMaxK ? 32 : 0;
+}
+
+template <int T, bool I8, bool WIDE>
+cudaError_t launch_beside(cudaLaunchConfig_t& cfg, const uint16_t* x, int64_t pitch, int64_t M, int64_t K, uint8_t* q, float* scale) {
+  constexpr int R = kBesideThreads / T;
+  cfg.gridDim = dim3((unsigned)((M + R - 1) / R));
+  cfg.blockDim = dim3(kBesideThreads);
+  const int64_t per_thread = (K / 8 + T - 1) / T;
+  if (per_thread <= 2) return cudaLaunchKernelEx(&cfg, quant_act_beside_kernel<T, 2, I8, WIDE>, x, pitch, M, K, q, scale);
+  if (per_thread <= 4) return cudaLaunchKernelEx(&cfg, quant_act_beside_kernel<T, 4, I8, WIDE>, x, pitch, M, K, q, scale);
+  return cudaLaunchKernelEx(&cfg, quant_act_beside_kernel<T, kKeepChunks, I8, WIDE>, x, pitch, M, K, q, scale);
+}
+
 constexpr int64_t kRowsKernelMinM = 256;   // from here on the per-row CTAs outnumber what the device holds at once
-constexpr int64_t kRowsKernelMaxK = 256 * kKeepChunks;   // rows the lanes hold entirely in registers
 
 template <bool I8, bool WIDE>
-cudaError_t launch_quant(cudaLaunchConfig_t& cfg, bool vec, const uint16_t* x, int64_t pitch, int64_t M, int64_t K,
+cudaError_t launch_quant(cudaLaunchConfig_t& cfg, bool vec, bool beside, const uint16_t* x, int64_t pitch, int64_t M, int64_t K,
                          uint8_t* q, float* scale) {
+  const int t = vec && beside ? beside_threads(M, K) : 0;
+  if (t > 0) {
+    cfg.numAttrs = 2;
+    return t == 32 ? launch_beside<32, I8, WIDE>(cfg, x, pitch, M, K, q, scale)
+                   : launch_beside<kBesideThreads, I8, WIDE>(cfg, x, pitch, M, K, q, scale);
+  }
   if (vec && M >= kRowsKernelMinM && K <= kRowsKernelMaxK) {
     cfg.gridDim = dim3((unsigned)((M + kRowsPerCta - 1) / kRowsPerCta));
     cfg.blockDim = dim3(kRowsPerCta * 32);
@@ -199,7 +277,7 @@ SACQ_TL_DEFINE_DUMP(sacq_debug_timeline_quant)
 #endif
 
 int launch_quant_act(const void* x, int64_t pitch, int64_t M, int64_t K, bool int8, bool wide, void* q, float* scale,
-                     cudaStream_t s) {
+                     cudaStream_t s, bool beside) {
   if (M == 0 || K == 0) return SACQ_OK;
   const bool vec = (K % 8 == 0) && (pitch % 8 == 0) && (reinterpret_cast<uintptr_t>(x) % 16 == 0) &&
                    (reinterpret_cast<uintptr_t>(q) % (wide ? 16 : 8) == 0);
@@ -209,17 +287,19 @@ int launch_quant_act(const void* x, int64_t pitch, int64_t M, int64_t K, bool in
   cfg.gridDim = dim3((unsigned)M);
   cfg.blockDim = dim3(kThreads);
   cfg.stream = s;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;      // used by quant_act_beside_kernel
+  attr[1].val.sharedMemCarveout = cudaSharedmemCarveoutMaxShared;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   const uint16_t* xp = static_cast<const uint16_t*>(x);
   uint8_t* qp = static_cast<uint8_t*>(q);
-  if (int8) SACQ_CUDA_TRY(wide ? (launch_quant<true, true>(cfg, vec, xp, pitch, M, K, qp, scale))
-                               : (launch_quant<true, false>(cfg, vec, xp, pitch, M, K, qp, scale)));
-  else SACQ_CUDA_TRY(wide ? (launch_quant<false, true>(cfg, vec, xp, pitch, M, K, qp, scale))
-                          : (launch_quant<false, false>(cfg, vec, xp, pitch, M, K, qp, scale)));
+  if (int8) SACQ_CUDA_TRY(wide ? (launch_quant<true, true>(cfg, vec, beside, xp, pitch, M, K, qp, scale))
+                               : (launch_quant<true, false>(cfg, vec, beside, xp, pitch, M, K, qp, scale)));
+  else SACQ_CUDA_TRY(wide ? (launch_quant<false, true>(cfg, vec, beside, xp, pitch, M, K, qp, scale))
+                          : (launch_quant<false, false>(cfg, vec, beside, xp, pitch, M, K, qp, scale)));
   count_launch();
   return SACQ_OK;
 }

@@ -745,6 +745,7 @@ int forward_impl(const sacq_layer_t* L, const void* x_bf16, int64_t x_pitch, int
   if (int rc = check_layer(L)) return rc;
   if (M == 0) return SACQ_OK;
   const int64_t K = L->d.in_features;
+  bool beside = false;                                // the quantizer runs beside the split-K kernel
   int64_t slab = 0;                                   // tokens up to which the GEMM takes fp16 activations in one piece
   int64_t need = 0;
   const bool rows_ok = M > 0 && L->d.out_features > 0 && K % 8 == 0 && x_bf16 != nullptr &&
@@ -758,6 +759,8 @@ int forward_impl(const sacq_layer_t* L, const void* x_bf16, int64_t x_pitch, int
       return launch_small_m(L, q_scratch, scale_scratch, M, y_out, ldy, workspace, workspace_bytes,
                             static_cast<cudaStream_t>(stream), residual, ldr, 0, nullptr, x_bf16, x_pitch);
     }
+    // a projection with a residual follows attention, not a GEMM: nothing to share an SM with (prefill block at 300 tokens 90.7 / 91.2 us)
+    beside = (r == kInt8Grouped || k == 2 || k == 3) && residual == nullptr && split_k_beside(L, M);
     if (r == kInt8TmemGrouped || k == 5) {
       slab = large_m_tmem_grouped_slab();
       need = large_m_tmem_grouped_workspace_bytes(L, M);
@@ -771,14 +774,16 @@ int forward_impl(const sacq_layer_t* L, const void* x_bf16, int64_t x_pitch, int
   if (wide) {
     DeviceGuard guard(L->d.device);
     void* a16 = static_cast<uint8_t*>(workspace) + kCounterBytes;
-    if (int rc = launch_quant_act(x_bf16, x_pitch, M, K, int8 != 0, true, a16, scale_scratch, static_cast<cudaStream_t>(stream)))
+    if (int rc = launch_quant_act(x_bf16, x_pitch, M, K, int8 != 0, true, a16, scale_scratch, static_cast<cudaStream_t>(stream), beside))
       return rc;
     if (int8) return linear_a8i_impl(L, a16, scale_scratch, M, y_out, ldy, workspace, workspace_bytes, stream, kActHalf);
     return linear_a8_impl(L, a16, scale_scratch, M, residual, ldr, y_out, ldy, workspace, workspace_bytes, stream, nullptr,
                           kActHalf);
   }
-  const int rc = int8 ? sacq_quant_act_int8(x_bf16, x_pitch, M, K, q_scratch, scale_scratch, stream)
-                      : sacq_quant_act_fp8(x_bf16, x_pitch, M, K, q_scratch, scale_scratch, stream);
+  const int rc = beside && q_scratch != nullptr && scale_scratch != nullptr
+                     ? launch_quant_act(x_bf16, x_pitch, M, K, int8 != 0, false, q_scratch, scale_scratch, static_cast<cudaStream_t>(stream), true)
+                 : int8 ? sacq_quant_act_int8(x_bf16, x_pitch, M, K, q_scratch, scale_scratch, stream)
+                        : sacq_quant_act_fp8(x_bf16, x_pitch, M, K, q_scratch, scale_scratch, stream);
   if (rc != SACQ_OK) return rc;
   if (int8) return sacq_linear_a8i(L, q_scratch, scale_scratch, M, y_out, ldy, workspace, workspace_bytes, stream);
   return linear_a8_impl(L, q_scratch, scale_scratch, M, residual, ldr, y_out, ldy, workspace, workspace_bytes, stream);

@@ -993,6 +993,10 @@ bool split_k_choose(const sacq_layer* L, int64_t M, SplitMode mode, SplitChoice*
   return complete(L, mode, out);
 }
 
+bool split_k_beside(const sacq_layer* L, int64_t M) {
+  return codebook_smem(L) > 0 && M <= (L->d.out_features < 4096 ? 1024 : 512);
+}
+
 bool split_k_codebook_in_smem(const sacq_layer* L) { return codebook_smem(L) > 0; }
 
 bool split_k_choose_multi(const sacq_layer* const* layers, int n, int64_t M, SplitMode mode, SplitChoice* out) {

@@ -46,6 +46,11 @@ int launch_split_k(const sacq_layer* const* layers, int n, const void* act, cons
                    int64_t ldr = 0, const BcastDst* bc = nullptr, const float* row_scale = nullptr);
 // Whether the layer's codebook fits the kernel's shared memory (else it is gathered from L2).
 bool split_k_codebook_in_smem(const sacq_layer* L);
+// Whether the quantizer in front of a call of M tokens should be the one that shares SMs with this kernel (act_quant.cu).
+// Not where the codebook is gathered through L1, which the quantizer's carve-out would take from the SM (65,536 entries,
+// 2048 -> 6144 at 16 tokens 11.3 / 14.4 us), and not
+// for wide layers of several waves (2048 -> 6144 at 700 27.5 / 27.6; 2048 -> 2048 13.7 / 12.2).
+bool split_k_beside(const sacq_layer* L, int64_t M);
 void split_k_release(sacq_layer* L);
 
 }  // namespace sacq

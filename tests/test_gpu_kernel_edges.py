@@ -239,6 +239,25 @@ def test_quantizer_inside_the_call_changes_no_byte(N, K, d, C, G):
     assert mod.device_status() == 0 and other.device_status() == 0
 
 
+@pytest.mark.parametrize("N,K,d,C,G", [(256, 1152, 8, 256, None), (256, 2048, 4, 512, None), (128, 2176, 8, 256, None),
+                                       (128, 8192, 8, 256, None), (128, 8320, 8, 256, None), (4800, 512, 4, 128, 64)])
+def test_quantizer_beside_the_split_k_kernel(N, K, d, C, G):
+    """A forward whose quantizer shares SMs with the GEMM has the bytes of the separate calls: around the numbers of tokens
+    and the row lengths where its rows change hands, for rows with a pitch, of zeros, infinities and NaN, FP8 and INT8."""
+    from sacq_b200 import quantize_rows
+    mod = _layer(N, K, d, C, G)
+    wide = _x(1028, K + 24)
+    wide[3] = 0
+    wide[5, 7] = float("inf")
+    wide[40, K - 1] = float("nan")
+    for x in (wide[:, :K].contiguous(), wide[:, 8:K + 8]):
+        for M in (49, 97, 369, 370, 371, 1023, 1024, 1025):
+            for forward, gemm, mode in ((mod, mod.linear_a8, "fp8_e4m3fn"), (mod.forward_int8, mod.linear_a8i, "int8_symmetric")):
+                y, ref = forward(x[:M]), gemm(*quantize_rows(x[:M], mode))
+                assert torch.equal(y.view(torch.int16), ref.view(torch.int16)), (M, mode)
+    assert mod.device_status() == 0
+
+
 @pytest.mark.parametrize("N", [1024, 1000])
 def test_host_result_stored_by_the_gemm(N):
     """Pinned results: stored by the GEMM where the rows are whole cache lines, copied otherwise."""
