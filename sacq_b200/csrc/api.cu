@@ -66,13 +66,19 @@ int64_t small_m_slab_rows(const sacq_layer* L) {
 // Rows from which the grouped split-K kernel takes over from the index-unpacking warp-MMA kernel, which walks the
 // weights once per 48 tokens and multiplies exact weights (quantizer + GEMM, d = 4, 10-bit, group 64: 2048x6144 19.0 / 10.1 us
 // at 32 rows; 2048x2048 9.2 / 7.8 and 6144x2048 20.5 / 12.8 at 47, there with weights of 11 bits, which up to 47 rows would be
-// less than before; the smallest lose a tenth, 1024x1024 5.4 / 6.0).  Whether wide layers gain below 17 rows in calls with the
-// quantizer is not measured; the GEMM alone does (2048x6144 at 16 12.1 / 9.4).
+// less than before; the smallest lose a tenth, 1024x1024 5.4 / 6.0).  With exact weights and the quantizer beside it the
+// split-K kernel is the faster one on the widest layers from the ninth row on (2048x6144, 10-bit: 12.7 / 11.4 us at 16, 11.9 / 11.3
+// at two, but with 64 entries even at eight; 1536x6144 eager 9.8 / 9.7 at 16, 9.5 / 9.7 at eight), on 4,096 rows from the second
+// chunk on (1024x4096 at 17 to 32 10.3 / 6.6; at 16 eager 6.2 / 7.6, the other one being a single launch) and on deep layers
+// around its end (6144x2048 15.6 / 13.8 at 32, 19.4 / 14.0 at 40; 64 entries, eager, at 24 13.8 / 14.3; codebooks of
+// up to 32 entries, whose gathers meet fewer bank conflicts, are not measured and stay), not on smaller ones (2048x2048 at 41
+// 9.2 / 10.0, 4096x1024 9.2 / 10.5).
 int64_t grouped_min_m(const sacq_layer* L) {
   // ... or from the CUDA-core kernel, at any number (2048x2048, 65,536 entries, group 128: 127 / 11 us at 17 rows)
   if (!L->small_m_warp_mma) return 1;
-  if (L->d.out_features >= 32 * (int64_t)L->num_sms) return 17;
-  return 48;
+  if (L->d.out_features >= 32 * (int64_t)L->num_sms) return L->d.in_features * L->d.out_features / L->d.vector_dim >= (3 << 20) ? 9 : 17;
+  if (L->d.out_features >= 4096) return 17;
+  return L->d.in_features >= 4096 && L->d.in_features * L->d.out_features >= (8 << 20) && L->d.index_bits > 5 ? 29 : 48;
 }
 // From how many tokens the persistent kernel with the weights in tensor memory takes over; its 128-row tiles need that many
 // to fill the device.  The split-K kernel expands a wide layer again for every second 384-token tile, from about 700 tokens
@@ -90,10 +96,14 @@ int64_t tmem_min_m(const sacq_layer* L) {
 // A codebook in L2 leaves the small-M kernel 2 warps' gathers in flight per scheduler: the split-K kernel wins from one
 // token on (65,536 entries, 2048x6144: 17.4 / 11.3 us at 16 tokens; 6144x2048 13.4 / 11.1 at one, 13.7 / 11.5 at 16;
 // 2048x2048 7.2 / 7.0 and 7.6 / 7.1), on the smallest layers from the second chunk on (2048x1024 6.4 / 7.2 at 16 and
-// 7.6 / 7.2 at 32, 1024x1024 5.5 / 5.8 and 6.4 / 5.8).
+// 7.6 / 7.2 at 32, 1024x1024 5.5 / 5.8 and 6.4 / 5.8).  So it does on wide layers of many vectors, which the small-M kernel
+// takes in tiles of 48 rows (2048x6144 7.4 / 6.9 at one token, 8.0 / 7.1 at 16), but not below 1.5 M vectors of eight, where the
+// small-M kernel is even and cheaper to launch (1536x6144 6.3 / 6.4 at one token, eager 7.4 / 8.0 at 16), or on deep layers
+// (6144x2048 8.0 / 8.3 at eight).  Dim-4 vectors keep the small-M kernel, whose bytes up to 16 tokens the tests pin (8.8 / 7.8).
 bool split_wins(const sacq_layer* L, int64_t M) {
   const int64_t work = L->d.in_features * L->d.out_features;
   if (!split_k_codebook_in_smem(L)) return M > 16 || work > (2 << 20) || L->d.out_features >= 4096;
+  if (L->d.out_features >= 32 * (int64_t)L->num_sms && L->d.vector_dim == 8 && work >= (12 << 20)) return true;
   return (M > 16 && (L->d.out_features >= 4096 || work >= (8 << 20))) || M > 32;
 }
 
