@@ -82,13 +82,14 @@ int64_t grouped_min_m(const sacq_layer* L) {
 }
 // From how many tokens the persistent kernel with the weights in tensor memory takes over; its 128-row tiles need that many
 // to fill the device.  The split-K kernel expands a wide layer again for every second 384-token tile, from about 700 tokens
-// on in a second wave (1024x4096 at 1,000 tokens 23.5 / 12.6 us, 2048x6144 39 / 24).  It keeps them up to 960 all the same:
-// the two sum in different orders, and up to there the tokens of a request get the same bytes alone and in a batch of
-// three (the price: 2048x6144 at 700 tokens 30.6 / 19.4).  A codebook that is gathered from L2 makes an expansion twice as
+// on in a second wave.  Where both sum in the same order, it is measured time alone (eager, split-K / persistent: 2048x6144 at
+// 450 tokens 16.8 / 17.3 us, 512 17.5 / 17.6, 600 20.6 / 18.9, 700 21.3 / 19.5, 900 24.4 / 22.1; 1024x4096 at 512 10.1 / 10.7,
+// 600 11.7 / 11.2, 900 14.6 / 12.6).  Elsewhere the split-K kernel keeps them up to 960: up to there the tokens of a request
+// get the same bytes alone and in a batch of three.  A codebook that is gathered from L2 makes an expansion twice as
 // dear (2048x6144 at 400 30.4 / 28.7).  Narrower layers lose nothing (2048x2048 at 1,000 17.6 / 16.3, 6144x1536 30 / 37).
 int64_t tmem_min_m(const sacq_layer* L) {
   if (L->d.out_features < 4096) return 1024;
-  return split_k_codebook_in_smem(L) ? 960 : 384;
+  return !split_k_codebook_in_smem(L) ? 384 : split_k_sums_whole(L) ? 560 : 960;
 }
 
 // From how many tokens a split-K kernel, which walks the weights once, beats a small-M kernel, which walks them
@@ -217,6 +218,7 @@ SACQ_API int sacq_layer_create(const sacq_layer_desc* desc, sacq_layer_t** out_l
   }
   L->num_sms = prop.multiProcessorCount;
   L->cb_entries = (d.codebook_size + 1) & ~1;
+  L->order_rows = d.out_features;
   split_k_init(L);
   L->small_m_warp_mma = small_m_staged_warps(L, 1) > 0;
   const int64_t count = (int64_t)L->cb_entries * d.vector_dim;
@@ -346,6 +348,14 @@ SACQ_API int sacq_layer_set_kernel(sacq_layer_t* L, int which) {
   if (int rc = check_layer(L)) return rc;
   if (which < 0 || which > 15) return set_error(SACQ_ERR_INVALID_ARGUMENT, "kernel selector %d not in 0..15", which);
   L->force_kernel = which;
+  return SACQ_OK;
+}
+
+SACQ_API int sacq_layer_set_shard_of(sacq_layer_t* L, int64_t rows) {
+  if (int rc = check_layer(L)) return rc;
+  if (rows < L->d.out_features)
+    return set_error(SACQ_ERR_INVALID_ARGUMENT, "a shard of %lld rows of a layer of %lld", (long long)L->d.out_features, (long long)rows);
+  L->order_rows = rows;
   return SACQ_OK;
 }
 

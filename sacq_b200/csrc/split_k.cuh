@@ -44,6 +44,8 @@ bool split_k_choose_multi(const sacq_layer* const* layers, int n, int64_t M, Spl
 int launch_split_k(const sacq_layer* const* layers, int n, const void* act, const float* scale, int64_t M, void* const* ys,
                    const int64_t* ldys, SplitMode mode, const SplitChoice& c, cudaStream_t s, const void* residual = nullptr,
                    int64_t ldr = 0, const BcastDst* bc = nullptr, const float* row_scale = nullptr);
+// Whether batches of the layer are summed in one piece of K, the persistent kernel's order.
+bool split_k_sums_whole(const sacq_layer* L);
 // Whether the layer's codebook fits the kernel's shared memory (else it is gathered from L2).
 bool split_k_codebook_in_smem(const sacq_layer* L);
 // Whether the quantizer in front of a call of M tokens should be the one that shares SMs with this kernel (act_quant.cu).

@@ -366,3 +366,30 @@ def test_split_k_deep_layers(kernel, N, K, d, C, G):
     for M in (1, 16, 32):
         assert torch.equal(mod.linear_w8a8_int8(qi[:M], si[:M], sw), want[:M]), M
     assert mod.device_status() == 0
+
+
+@pytest.mark.parametrize("N,K,d,C,first", [(4096, 1024, 8, 256, 256), (6144, 2048, 8, 4096, 256), (4104, 3840, 8, 256, 256),
+                                           (4096, 2048, 4, 4096, 320)])
+def test_wide_batches_sum_in_one_order(N, K, d, C, first):
+    """From `first` tokens on a wide layer has one order of sums, whichever kernel and tile: rows repeat the bytes of a larger
+    call, a shard those of the whole layer, sibling layers of another width those of their own calls."""
+    from sacq_b200 import linear_a8_multi, quantize_rows, PrecomputedPackedVectorCodebookLinear
+    from sacq_b200.column_parallel import shard_payload
+    from sacq_b200.synthetic import make_payload
+    p = make_payload(N, K, vector_dim=d, codebook_size=C, seed=N + K, device="cuda", iters=1, fit=False)
+    mod = PrecomputedPackedVectorCodebookLinear(p, None, "cuda")
+    q, s = quantize_rows(_x(1200, K))
+    whole = mod.linear_a8(q, s)
+    assert mod.kernel_for(1200) == "large_tmem" and _err(mod, whole, q, s) <= TOL
+    half = PrecomputedPackedVectorCodebookLinear(shard_payload(p, 1, 2), None, "cuda")
+    half.set_shard_of(N)
+    for M in (first, first + 1, 383, 385, 513, 559, 560, 561, 959, 1023):
+        y = mod.linear_a8(q[:M], s[:M])
+        assert torch.equal(y, whole[:M]), M
+        assert torch.equal(half.linear_a8(q[:M], s[:M]), whole[:M, N // 2:]), M
+    small = PrecomputedPackedVectorCodebookLinear(shard_payload(p, 0, 4), None, "cuda")     # a layer of its own: another order
+    for M in (first - 1, first, 300, 700):
+        for pair in ([mod, mod], [mod, small], [small, mod]):
+            for layer, y in zip(pair, linear_a8_multi(pair, q[:M], s[:M])):
+                assert torch.equal(y, layer.linear_a8(q[:M], s[:M])), M
+    assert mod.device_status() == 0 and half.device_status() == 0
