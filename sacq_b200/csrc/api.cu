@@ -75,7 +75,7 @@ int64_t small_m_slab_rows(const sacq_layer* L) {
 // 9.2 / 10.0, 4096x1024 9.2 / 10.5).
 int64_t grouped_min_m(const sacq_layer* L) {
   // ... or from the CUDA-core kernel, at any number (2048x2048, 65,536 entries, group 128: 127 / 11 us at 17 rows)
-  if (!L->small_m_warp_mma) return 1;
+  if (L->small_m_warps == 0) return 1;
   if (L->d.out_features >= 32 * (int64_t)L->num_sms) return L->d.in_features * L->d.out_features / L->d.vector_dim >= (3 << 20) ? 9 : 17;
   if (L->d.out_features >= 4096) return 17;
   return L->d.in_features >= 4096 && L->d.in_features * L->d.out_features >= (8 << 20) && L->d.index_bits > 5 ? 29 : 48;
@@ -98,13 +98,14 @@ int64_t tmem_min_m(const sacq_layer* L) {
 // token on (65,536 entries, 2048x6144: 17.4 / 11.3 us at 16 tokens; 6144x2048 13.4 / 11.1 at one, 13.7 / 11.5 at 16;
 // 2048x2048 7.2 / 7.0 and 7.6 / 7.1), on the smallest layers from the second chunk on (2048x1024 6.4 / 7.2 at 16 and
 // 7.6 / 7.2 at 32, 1024x1024 5.5 / 5.8 and 6.4 / 5.8).  So it does on wide layers of many vectors, which the small-M kernel
-// takes in tiles of 48 rows (2048x6144 7.4 / 6.9 at one token, 8.0 / 7.1 at 16), but not below 1.5 M vectors of eight, where the
-// small-M kernel is even and cheaper to launch (1536x6144 6.3 / 6.4 at one token, eager 7.4 / 8.0 at 16), or on deep layers
-// (6144x2048 8.0 / 8.3 at eight).  Dim-4 vectors keep the small-M kernel, whose bytes up to 16 tokens the tests pin (8.8 / 7.8).
+// takes in tiles of 48 rows (2048x6144 7.4 / 6.9 at one token, 8.0 / 7.1 at 16), and where they are shallow, from where it alone
+// quantizes in the same launch (1024x4096, eager, 7.5 / 5.5 at eight; at one token 5.6 / 5.4, but 6.5 / 7.1 on a slower host), but
+// not between, where the small-M kernel is even (1536x6144 6.3 / 6.4 at one token, 6.7 / 6.5 at 16), or on deep layers (6144x2048 8.0 / 8.3 at eight).  Dim-4 vectors keep the small-M kernel, whose bytes up to 16 tokens the tests pin (8.8 / 7.8).
 bool split_wins(const sacq_layer* L, int64_t M) {
   const int64_t work = L->d.in_features * L->d.out_features;
   if (!split_k_codebook_in_smem(L)) return M > 16 || work > (2 << 20) || L->d.out_features >= 4096;
-  if (L->d.out_features >= 32 * (int64_t)L->num_sms && L->d.vector_dim == 8 && work >= (12 << 20)) return true;
+  if (L->d.out_features >= 4096 && L->d.vector_dim == 8 && (work >= (12 << 20) || (L->d.in_features <= 1024 && M > L->small_m_warps)))
+    return true;
   return (M > 16 && (L->d.out_features >= 4096 || work >= (8 << 20))) || M > 32;
 }
 
@@ -220,7 +221,7 @@ SACQ_API int sacq_layer_create(const sacq_layer_desc* desc, sacq_layer_t** out_l
   L->cb_entries = (d.codebook_size + 1) & ~1;
   L->order_rows = d.out_features;
   split_k_init(L);
-  L->small_m_warp_mma = small_m_staged_warps(L, 1) > 0;
+  L->small_m_warps = small_m_staged_warps(L, 1);
   const int64_t count = (int64_t)L->cb_entries * d.vector_dim;
   // one allocation for all that is derived from the layer (each of its own costs a layer's making milliseconds)
   auto up = [](int64_t v) { return (v + 255) & ~(int64_t)255; };
@@ -745,15 +746,29 @@ namespace {
 // pass over the tokens (2048x2048, d = 4, 16 tokens 6.5 us against 5.4; 2048x1024 at one 4.5 / 4.2).  A captured call
 // pays for the GPU's time only and keeps the quantizer as a launch of its own; the bytes are the same.  On layers that
 // keep the GPU busy anyway it is a loss in eager calls too (2048x6144 8.9 against 8.4 at one token, 6144x2048 10.7 / 8.4 at 8).
-bool quantizes_in_gemm(const sacq_layer* L, int64_t M, cudaStream_t s) {
-  if (L->d.in_features * L->d.out_features > (4 << 20) || M * L->d.in_features > (32 << 10) || M > small_m_staged_warps(L, M))
-    return false;
+bool eager(cudaStream_t s) {
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &status) != cudaSuccess) {   // the default stream beside another thread's capture
     cudaGetLastError();
     return false;
   }
   return status == cudaStreamCaptureStatusNone;
+}
+bool quantizes_in_gemm(const sacq_layer* L, int64_t M, cudaStream_t s) {
+  return L->d.in_features * L->d.out_features <= (4 << 20) && M * L->d.in_features <= (32 << 10) && M <= small_m_staged_warps(L, M) && eager(s);
+}
+// The same for the split-K kernel, whose expander warps quantize the tokens, a warp each, once their rows have landed in shared
+// memory.  Its CTAs enter long before the wait for the kernel in front ends, if the last call's leave them SMs: then the GPU loses
+// little or nothing (graph / eager, quantizer by itself against this: 1024 -> 4096 5.2 / 8.3 against 5.0 / 5.5 us at 8 tokens,
+// 5.5 / 8.1 against 6.1 / 6.6 at 24; codebook in L2, 2048 -> 2048 at 4 6.5 / 8.3 against 5.9 / 6.2).  CTAs that wait for SMs have
+// it ahead of them on top of their expansions: up to 16 tokens as long as a launch takes the host (2048 -> 6144 at 4
+// 7.0 / 8.2 against 7.5 / 7.8, 16 7.1 / 8.2 against 7.9 / 8.3; in L2 11.3 / 11.5 against 10.8 / 10.8), not beyond (24, 256 codewords,
+// 7.1 / 8.2 against 8.8 / 9.1).  Every CTA reads the whole rows of its tokens: not 32 of 2,048 (256 codewords, 2048 -> 1024 at 64
+// 6.5 / 7.7 against 8.0 / 8.3; 16 to a tile at 40 6.5 / 7.7 against 6.5 / 6.9).
+bool quantizes_in_split(const sacq_layer* L, int64_t M, cudaStream_t s, const SplitChoice& c) {
+  if (M > 64 || c.tok * L->d.in_features > (48 << 10) || !split_k_quantizes(L, c)) return false;
+  const bool early = 2 * split_k_ctas(L, c) <= L->num_sms, few = M <= 16;
+  return (few && (early || !split_k_codebook_in_smem(L))) || ((few || early) && eager(s));
 }
 
 // Quantizer + GEMM of one call, in one launch where the GEMM can quantize for itself (own_quantizer = false allows it).
@@ -779,8 +794,20 @@ int forward_impl(const sacq_layer_t* L, const void* x_bf16, int64_t x_pitch, int
       return launch_small_m(L, q_scratch, scale_scratch, M, y_out, ldy, workspace, workspace_bytes,
                             static_cast<cudaStream_t>(stream), residual, ldr, 0, nullptr, x_bf16, x_pitch);
     }
-    // a projection with a residual follows attention, not a GEMM: nothing to share an SM with (prefill block at 300 tokens 90.7 / 91.2 us)
-    beside = (r == kInt8Grouped || k == 2 || k == 3) && residual == nullptr && split_k_beside(L, M);
+    if (k == 2 || k == 3 || r == kInt8Grouped) {
+      const SplitMode mode = k == 2 ? kSplitHiLo : large_m_grouped_exact(L, M, int8 != 0) ? kSplitHalf2 : kSplitHalf;
+      SplitChoice c;
+      if (M <= 1024 && split_k_choose(L, M, mode, &c)) {
+        if (k == 2 && !own_quantizer && (residual == nullptr || ldr >= L->d.out_features) &&
+            quantizes_in_split(L, M, static_cast<cudaStream_t>(stream), c)) {
+          DeviceGuard guard(L->d.device);
+          return launch_split_k(&L, 1, nullptr, nullptr, M, &y_out, &ldy, kSplitHiLo, c, static_cast<cudaStream_t>(stream), residual, ldr,
+                                nullptr, nullptr, x_bf16, x_pitch);
+        }
+        // a projection with a residual follows attention, not a GEMM: nothing to share an SM with (prefill block at 300 tokens 90.7 / 91.2 us)
+        beside = residual == nullptr && split_k_beside(L, M, c);
+      }
+    }
     if (r == kInt8TmemGrouped || k == 5) {
       slab = large_m_tmem_grouped_slab();
       need = large_m_tmem_grouped_workspace_bytes(L, M);

@@ -78,10 +78,10 @@ struct SplitLayer {
 
 // mbarriers of a CTA
 constexpr int ACT_FULL = 0, ACT_EMPTY = kMaxAct, W_FULL = 2 * kMaxAct, W_EMPTY = W_FULL + kMaxW, IDX_FULL = W_EMPTY + kMaxW,
-              CB_FULL = IDX_FULL + 2, ACC_FULL = CB_FULL + 1, RECV = ACC_FULL + 1, kBarriers = RECV + 1;
+              CB_FULL = IDX_FULL + 2, ACC_FULL = CB_FULL + 1, RECV = ACC_FULL + 1, X_FULL = RECV + 1, kBarriers = X_FULL + 1;
 
 struct SplitLayout {
-  uint32_t idx_off, cb_off, sc_off, recv_off, fixed_off, sa_off, sw_off, bias_off, bar_off, misc_off, total;
+  uint32_t idx_off, cb_off, sc_off, recv_off, fixed_off, sa_off, sw_off, bias_off, bar_off, misc_off, x_off, total;
 };
 
 // What a CTA's start depends on comes first: kernel parameters are read through a cache that is cold in every launch, a miss
@@ -106,6 +106,8 @@ struct alignas(64) SplitParams {
   int64_t ldr;
   int n_bc;                     // further copies of the output (peer GPUs' buffers), same pitch as y
   uint16_t* ybc[kMaxBcast];
+  const uint16_t* x;            // QUANT: bf16 [M, x_pitch], instead of q and act_scale
+  int64_t x_pitch;
 };
 
 // tokens of the tile a rank reduces and writes
@@ -114,7 +116,7 @@ __host__ __device__ constexpr int owned_tokens(int tok, int split) { return ((to
 __host__ __device__ constexpr int index_boxes(int slices, int box_shift) { return (slices + (1 << box_shift) - 1) >> box_shift; }
 
 __host__ __device__ inline SplitLayout split_layout(int tok, int split, int act_stages, int slices, int box_shift, int groups,
-                                                    int cb_bytes, bool own_recv) {
+                                                    int cb_bytes, bool own_recv, int x_bytes = 0) {
   SplitLayout L;
   L.idx_off = (uint32_t)((act_stages * tok * 128 + 1023) & ~1023);
   L.cb_off = L.idx_off + (uint32_t)(index_boxes(slices, box_shift) * (kSliceBytes << box_shift));
@@ -129,7 +131,8 @@ __host__ __device__ inline SplitLayout split_layout(int tok, int split, int act_
   L.bias_off = L.sw_off + kRows * 4;
   L.bar_off = L.bias_off + kRows * 4;
   L.misc_off = L.bar_off + kBarriers * 8;
-  L.total = L.misc_off + 64;
+  L.x_off = (L.misc_off + 64 + 127) & ~127u;
+  L.total = x_bytes > 0 ? L.x_off + (uint32_t)x_bytes : L.misc_off + 64;
   return L;
 }
 
@@ -176,6 +179,18 @@ __device__ __forceinline__ bool mbar_wait_two(uint32_t b0, uint32_t p0, uint32_t
   const bool r0 = mbar_try_wait(b0, p0), r1 = mbar_try_wait(b1, p1);
   if (__all_sync(0xffffffffu, r0 && r1)) return true;
   return mbar_wait_warp(b0, p0, abort_flag, status) && mbar_wait_warp(b1, p1, abort_flag, status);
+}
+// Whether the phase is complete, without waiting; one answer for the warp.
+__device__ __forceinline__ bool mbar_test_warp(uint32_t bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return __all_sync(0xffffffffu, done != 0);
 }
 // 16 accumulator columns of the warp's lane quarter.
 __device__ __forceinline__ void tmem_ld_16(uint32_t taddr, uint32_t (&r)[16]) {
@@ -320,10 +335,35 @@ __device__ __forceinline__ void reduce_tokens(const SplitParams& p, const SplitL
   }
 }
 
+// One token's row x (bf16, K values in shared memory), quantized as quant_act_kernel does it: the scale to *scale, the bytes of
+// 128-byte stages [first, first + stages) to their rows of the SWIZZLE_128B tiles, `tile` bytes apart, as the TMA would put
+// them.  A warp per token; row = null: zeros.
+__device__ __forceinline__ void quantize_row(const uint4* row, int chunks, int first, int stages, uint8_t* act_row, int tile, int xor_row,
+                                             int lane, float* scale) {
+  uint32_t mx = 0u;
+  if (row != nullptr)
+    for (int c = lane; c < chunks; c += 32) {
+      const uint4 v = row[c];
+      mx = __vmaxu2(__vmaxu2(__vmaxu2(__vmaxu2(mx, v.x & 0x7fff7fffu), v.y & 0x7fff7fffu), v.z & 0x7fff7fffu), v.w & 0x7fff7fffu);
+    }
+  const RowDivisor d = scale_of<false>(__uint_as_float(warp_max_bits(max(mx << 16, mx & 0xffff0000u))));
+  if (lane == 0) *scale = d.s;
+  for (int c = lane; c < stages * 16; c += 32) {      // eight values, half of a 16-byte unit
+    uint32_t o[2] = {0u, 0u};
+    if (row != nullptr) {
+      const uint4 v = row[first * 16 + c];
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+      encode_pairs<false, 4>(w, d, o);
+    }
+    *reinterpret_cast<uint2*>(act_row + (c >> 4) * tile + ((((c >> 1) & 7) ^ xor_row) << 4) + (c & 1) * 8) = make_uint2(o[0], o[1]);
+  }
+}
+
 // grid = (row tiles x split, token tiles, layers), clusters of `split` CTAs along x.
-template <int D, int MODE, bool CB_SMEM, int BOX_SHIFT>
+template <int D, int MODE, bool CB_SMEM, int BOX_SHIFT, bool QUANT>
 __global__ void __launch_bounds__(kCtaThreads, 1)
 split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ SplitParams p) {
+  static_assert(!QUANT || MODE == kSplitHiLo, "the kernel quantizes for itself where its activations are e4m3 bytes");
   constexpr uint32_t kTmemCols = 512;
   constexpr int CW_BYTES = 2 * D;
   constexpr bool PAIR = MODE == kSplitHalf2, F16 = MODE == kSplitHalf || PAIR, RECIPE = MODE >= kSplitInt8, INT = MODE == kSplitInt8;
@@ -382,7 +422,7 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     }
   } else if (warp == 2) {
     for (int i = lane; i < kBarriers; i += 32)
-      if (i < IDX_FULL || i > CB_FULL) mbar_init(bar(i), i >= W_FULL && i < W_EMPTY ? kXWarps : i == RECV ? kXWarps * S + 1 : 1);
+      if (i < IDX_FULL || i > CB_FULL) mbar_init(bar(i), (i >= W_FULL && i < W_EMPTY) || (QUANT && i == ACT_FULL) ? kXWarps : i == RECV ? kXWarps * S + 1 : 1);
     if (lane == 0) *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_proxy_async();
@@ -406,15 +446,22 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     __syncwarp();
     if (S > 1 && p.own_recv) cluster_wait();
     asm volatile("griddepcontrol.wait;" ::: "memory");   // q and the scales come from the kernel in front
+    if constexpr (QUANT) {                            // ... or x
+      const int rows = min(tok, p.M - m0), row_bytes = p.K * 2;
+      if (elect_one()) mbar_arrive_expect_tx(bar(X_FULL), (uint32_t)(rows * row_bytes));
+      __syncwarp();
+      if (lane < rows) bulk_load(base + L.x_off + (uint32_t)(lane * row_bytes), p.x + (int64_t)(m0 + lane) * p.x_pitch, (uint32_t)row_bytes, bar(X_FULL));
+      mbar_wait_warp(bar(X_FULL), 0, abort_flag, lay.status);
+    }
     float sa[kMaxTok / 32];                           // the token scales: fetched now, put down behind the last copy
 #pragma unroll
     for (int i = 0; i < kMaxTok / 32; ++i) {
       const int t = i * 32 + lane;
-      sa[i] = t < tok && m0 + t < p.M ? __ldg(p.act_scale + m0 + t) : 0.f;
+      sa[i] = !QUANT && t < tok && m0 + t < p.M ? __ldg(p.act_scale + m0 + t) : 0.f;
     }
     int st = 0;
     uint32_t free_parity = 1;
-    for (int i = 0; i < kbs * TILES; ++i) {
+    for (int i = 0; i < (QUANT ? 0 : kbs * TILES); ++i) {
       if (i >= act_stages && !mbar_wait_warp(bar(ACT_EMPTY + st), free_parity, abort_flag, lay.status)) break;
       const uint32_t dst = base + (uint32_t)(st * tok * 128);
       const int x = (kb0 * TILES + i) * 128;
@@ -427,7 +474,7 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     }
 #pragma unroll
     for (int i = 0; i < kMaxTok / 32; ++i)
-      if (i * 32 + lane < tok) reinterpret_cast<float*>(sm + L.sa_off)[i * 32 + lane] = sa[i];
+      if (!QUANT && i * 32 + lane < tok) reinterpret_cast<float*>(sm + L.sa_off)[i * 32 + lane] = sa[i];
     // every copy has landed before the CTA ends (the expanders see to it that none lands on partial sums)
     mbar_wait_warp(bar(IDX_FULL), 0, abort_flag, lay.status);
     if (boxes > first_boxes) mbar_wait_warp(bar(IDX_FULL + 1), 0, abort_flag, lay.status);
@@ -451,7 +498,8 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       const uint32_t d_col = tmem_base + (uint32_t)(part * tok);
 #pragma unroll
       for (int sub = 0; sub < TILES; ++sub) {
-        ok = sub == 0 ? mbar_wait_two(bar(W_FULL + ws), w_parity, bar(ACT_FULL + st), act_parity, abort_flag, lay.status)
+        // QUANT: one barrier for all activation tiles, none of which is filled again
+        ok = sub == 0 ? mbar_wait_two(bar(W_FULL + ws), w_parity, bar(QUANT ? ACT_FULL : ACT_FULL + st), QUANT ? 0u : act_parity, abort_flag, lay.status)
                       : mbar_wait_warp(bar(ACT_FULL + st), act_parity, abort_flag, lay.status);
         if (!ok) break;
         tc_fence_after();
@@ -629,7 +677,24 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     if (ok) expand(0, cur, cur_s);
     __syncwarp();
     if (S > 1 && p.own_recv) cluster_wait();
-    for (int wi = 0; wi < kbs && ok; ++wi) {
+    bool quantized = !QUANT;
+    for (int wi = 0; wi < kbs + (QUANT ? 1 : 0) && ok; ++wi) {
+      if constexpr (QUANT) {
+        // The warp's tokens: as soon as their rows have landed, at the latest when nothing is left to expand ahead of the MMAs.
+        const bool now = wi >= w_stages || wi == kbs;
+        if (!quantized && (now || mbar_test_warp(bar(X_FULL), 0))) {
+          if (now) ok = mbar_wait_warp(bar(X_FULL), 0, abort_flag, lay.status);
+          if (!ok) break;
+          for (int t = warp - 2; t < tok; t += kXWarps)
+            quantize_row(m0 + t < p.M ? reinterpret_cast<const uint4*>(sm + L.x_off + t * p.K * 2) : nullptr, p.K >> 3, kb0, kbs,
+                         sm + t * 128, tok * 128, t & 7, lane, reinterpret_cast<float*>(sm + L.sa_off) + t);
+          fence_proxy_async();                        // the tensor cores read them
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(ACT_FULL));
+          quantized = true;
+        }
+        if (wi == kbs) break;
+      }
       if (wi >= w_stages) {
         ok = mbar_wait_warp(bar(W_EMPTY + ws), w_parity, abort_flag, lay.status);
         if (!ok) break;
@@ -809,13 +874,13 @@ int active_clusters(int split, int num_sms) {
   return split == 8 ? num_sms * 15 / 148 : split == 4 ? num_sms * 33 / 148 : num_sms / split;
 }
 
-template <int D, int MODE, bool CB_SMEM, int BOX_SHIFT>
+template <int D, int MODE, bool CB_SMEM, int BOX_SHIFT, bool QUANT = false>
 cudaError_t launch_kernel(const CUtensorMap& ta, const SplitParams& p, dim3 grid, size_t smem, cudaStream_t s) {
   static bool configured[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || !configured[dev]) {
-    const cudaError_t e = cudaFuncSetAttribute(split_k_kernel<D, MODE, CB_SMEM, BOX_SHIFT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    const cudaError_t e = cudaFuncSetAttribute(split_k_kernel<D, MODE, CB_SMEM, BOX_SHIFT, QUANT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
@@ -833,13 +898,16 @@ cudaError_t launch_kernel(const CUtensorMap& ta, const SplitParams& p, dim3 grid
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = p.split > 1 ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, split_k_kernel<D, MODE, CB_SMEM, BOX_SHIFT>, ta, p);
+  return cudaLaunchKernelEx(&cfg, split_k_kernel<D, MODE, CB_SMEM, BOX_SHIFT, QUANT>, ta, p);
 }
 
 template <int D, bool CB_SMEM, int BOX_SHIFT>
 cudaError_t launch_mode(SplitMode mode, const CUtensorMap& ta, const SplitParams& p, dim3 grid, size_t smem, cudaStream_t s) {
   switch (mode) {
-    case kSplitHiLo: return launch_kernel<D, kSplitHiLo, CB_SMEM, BOX_SHIFT>(ta, p, grid, smem, s);
+    case kSplitHiLo:
+      if constexpr (BOX_SHIFT == 2)
+        if (p.x != nullptr) return launch_kernel<D, kSplitHiLo, CB_SMEM, BOX_SHIFT, true>(ta, p, grid, smem, s);
+      return launch_kernel<D, kSplitHiLo, CB_SMEM, BOX_SHIFT>(ta, p, grid, smem, s);
     case kSplitHalf: return launch_kernel<D, kSplitHalf, CB_SMEM, BOX_SHIFT>(ta, p, grid, smem, s);
     case kSplitHalf2: return launch_kernel<D, kSplitHalf2, CB_SMEM, BOX_SHIFT>(ta, p, grid, smem, s);
     case kSplitInt8: return launch_kernel<D, kSplitInt8, CB_SMEM, BOX_SHIFT>(ta, p, grid, smem, s);
@@ -893,7 +961,9 @@ int slices_of(const sacq_layer* L, int64_t M, SplitMode mode) {
 // codewords: 2048 -> 6144 at 300 tokens 26.4 us with 227 KB taken, 20.6 now; 6144 -> 2048 at 400 38.8 / 27.4).
 bool split_fits(const sacq_layer* L, SplitMode mode, SplitChoice* c) {
   const int cb_bytes = codebook_smem(L), groups = mode == kSplitHiLo ? 0 : 1;
-  slice_extent(L, c->split, &c->max_slices, &c->max_groups);
+  const int cut = c->split == 1 ? 0 : c->split == 2 ? 1 : c->split == 4 ? 2 : 3;
+  c->max_slices = L->slice_idx[cut];
+  c->max_groups = L->slice_groups[cut];
   const int tiles = (stages_of(L->d.in_features) + c->split - 1) / c->split * (is_f16(mode) ? 2 : 1);
   const size_t most = (cb_bytes > 0 ? 224 : 164) * 1024;
   auto bytes = [&](int stages) {
@@ -974,6 +1044,7 @@ bool complete(const sacq_layer* L, SplitMode mode, SplitChoice* c) {
 }  // namespace
 
 void split_k_init(sacq_layer* L) {
+  for (int i = 0; i < 4; ++i) slice_extent(L, 1 << i, &L->slice_idx[i], &L->slice_groups[i]);
   for (int mode = kSplitHiLo; mode <= kSplitFp8; ++mode) {
     const SplitMode m = (SplitMode)mode;
     int tok = takes_layer(L, m) ? most_columns(m) : 0;
@@ -1010,11 +1081,24 @@ bool split_k_choose(const sacq_layer* L, int64_t M, SplitMode mode, SplitChoice*
   return complete(L, mode, out);
 }
 
-bool split_k_beside(const sacq_layer* L, int64_t M) {
-  return codebook_smem(L) > 0 && M <= (L->d.out_features < 4096 ? 1024 : 512);
+int64_t split_k_ctas(const sacq_layer* L, const SplitChoice& c) {
+  return (L->d.out_features + kRows - 1) / kRows * c.tiles * c.split;
+}
+
+bool split_k_beside(const sacq_layer* L, int64_t M, const SplitChoice& c) {
+  return codebook_smem(L) > 0 && M <= (L->d.out_features < 4096 ? 1024 : 512) && 2 * split_k_ctas(L, c) + M > L->num_sms;
 }
 
 bool split_k_codebook_in_smem(const sacq_layer* L) { return codebook_smem(L) > 0; }
+
+bool split_k_quantizes(const sacq_layer* L, const SplitChoice& c) {
+  const int64_t K = L->d.in_features;
+  if (c.tok > 32 || K > 8192 || c.parts > 1 || c.box_shift != 2 || (c.split > 1 && !c.own_recv)) return false;
+  const int stages = (stages_of(K) + c.split - 1) / c.split;
+  if (stages > c.act_stages) return false;            // every activation tile has a place of its own
+  const SplitLayout l = split_layout(c.tok, c.split, c.act_stages, c.max_slices, c.box_shift, 0, codebook_smem(L), c.own_recv, (int)(c.tok * K * 2));
+  return split_smem(l) <= (codebook_smem(L) > 0 ? 224 : 164) * 1024;
+}
 
 bool split_k_choose_multi(const sacq_layer* const* layers, int n, int64_t M, SplitMode mode, SplitChoice* out) {
   const sacq_layer_desc& d0 = layers[0]->d;
@@ -1039,17 +1123,21 @@ void split_k_release(sacq_layer* L) {
 
 int launch_split_k(const sacq_layer* const* layers, int n, const void* act, const float* scale, int64_t M, void* const* ys,
                    const int64_t* ldys, SplitMode mode, const SplitChoice& c, cudaStream_t s, const void* residual,
-                   int64_t ldr, const BcastDst* bc, const float* row_scale) {
+                   int64_t ldr, const BcastDst* bc, const float* row_scale, const void* x, int64_t x_pitch) {
   const sacq_layer_desc& d0 = layers[0]->d;
   if (reinterpret_cast<uintptr_t>(act) % 16 != 0)
     return set_error(SACQ_ERR_ALIGNMENT, "quantized activations must be 16-byte aligned");
   SplitParams p;
   memset(&p, 0, sizeof(p));
+  int rc = SACQ_OK;
   CUtensorMap ta;
   const uint64_t act_row = (uint64_t)d0.in_features * (is_f16(mode) ? 2 : 1);
-  int rc = encode_bytes_2d(&ta, act, act_row, (uint64_t)M, act_row, 128u, (uint32_t)(c.tok <= 256 ? c.tok : c.tok / 2),
-                           CU_TENSOR_MAP_SWIZZLE_128B);
+  if (x == nullptr)
+    rc = encode_bytes_2d(&ta, act, act_row, (uint64_t)M, act_row, 128u, (uint32_t)(c.tok <= 256 ? c.tok : c.tok / 2),
+                         CU_TENSOR_MAP_SWIZZLE_128B);
   if (rc != SACQ_OK) return rc;
+  p.x = static_cast<const uint16_t*>(x);
+  p.x_pitch = x_pitch;
   int64_t widest = 0;
   for (int l = 0; l < n; ++l) {
     const sacq_layer* L = layers[l];
@@ -1071,6 +1159,7 @@ int launch_split_k(const sacq_layer* const* layers, int n, const void* act, cons
                                       : ldexpf(1.f, -L->cb8_exp_shift);
     if (L->d.out_features > widest) widest = L->d.out_features;
   }
+  if (x != nullptr) ta = p.idx[0];                    // a valid map is passed either way
   p.act_scale = scale;
   p.row_scale = row_scale;
   p.shift = d0.shift_bf16;
@@ -1088,7 +1177,8 @@ int launch_split_k(const sacq_layer* const* layers, int n, const void* act, cons
   p.split_shift = log2_of(c.split);
   p.slice_shift = log2_of(c.split * c.parts);
   p.own = owned_tokens(c.tok, c.split);
-  p.lay = split_layout(c.tok, c.split, c.act_stages, c.max_slices, c.box_shift, mode == kSplitHiLo ? 0 : c.max_groups, codebook_smem(layers[0]), c.own_recv);
+  p.lay = split_layout(c.tok, c.split, c.act_stages, c.max_slices, c.box_shift, mode == kSplitHiLo ? 0 : c.max_groups, codebook_smem(layers[0]), c.own_recv,
+                       x != nullptr ? c.tok * p.K * 2 : 0);
   const dim3 grid((unsigned)((widest + kRows - 1) / kRows * c.split), (unsigned)c.tiles, (unsigned)n);
   const size_t smem = split_smem(p.lay);
   const bool cb = codebook_smem(layers[0]) > 0;

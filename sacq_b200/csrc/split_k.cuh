@@ -43,16 +43,22 @@ bool split_k_choose_multi(const sacq_layer* const* layers, int n, int64_t M, Spl
 // and kSplitHalf2 the activations already widened to fp16 [M, K].  row_scale: the recipes' per-row weight scales [N] (n = 1).
 int launch_split_k(const sacq_layer* const* layers, int n, const void* act, const float* scale, int64_t M, void* const* ys,
                    const int64_t* ldys, SplitMode mode, const SplitChoice& c, cudaStream_t s, const void* residual = nullptr,
-                   int64_t ldr = 0, const BcastDst* bc = nullptr, const float* row_scale = nullptr);
+                   int64_t ldr = 0, const BcastDst* bc = nullptr, const float* row_scale = nullptr, const void* x = nullptr,
+                   int64_t x_pitch = 0);
+// Whether the CTAs of a kSplitHiLo call cut up like that can quantize the tokens themselves (launch_split_k with x: bf16 rows
+// that are 16-byte aligned, instead of act and scale): their rows fit shared memory.
+bool split_k_quantizes(const sacq_layer* L, const SplitChoice& c);
+int64_t split_k_ctas(const sacq_layer* L, const SplitChoice& c);
 // Whether batches of the layer are summed in one piece of K, the persistent kernel's order.
 bool split_k_sums_whole(const sacq_layer* L);
 // Whether the layer's codebook fits the kernel's shared memory (else it is gathered from L2).
 bool split_k_codebook_in_smem(const sacq_layer* L);
 // Whether the quantizer in front of a call of M tokens should be the one that shares SMs with this kernel (act_quant.cu).
 // Not where the codebook is gathered through L1, which the quantizer's carve-out would take from the SM (65,536 entries,
-// 2048 -> 6144 at 16 tokens 11.3 / 14.4 us), and not
-// for wide layers of several waves (2048 -> 6144 at 700 27.5 / 27.6; 2048 -> 2048 13.7 / 12.2).
-bool split_k_beside(const sacq_layer* L, int64_t M);
+// 2048 -> 6144 at 16 tokens 11.3 / 14.4 us), not for wide layers of several waves (2048 -> 6144 at 700 27.5 / 27.6; 2048 -> 2048
+// 13.7 / 12.2), and not where the chip has room for the CTAs of two GEMMs and the quantizer's beside each other (INT8, 2048 -> 1024,
+// d = 4, at 40 tokens 9.6 / 9.9).
+bool split_k_beside(const sacq_layer* L, int64_t M, const SplitChoice& c);
 void split_k_release(sacq_layer* L);
 
 }  // namespace sacq

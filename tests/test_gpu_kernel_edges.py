@@ -258,6 +258,34 @@ def test_quantizer_beside_the_split_k_kernel(N, K, d, C, G):
     assert mod.device_status() == 0
 
 
+@pytest.mark.parametrize("N,K,d,C", [(6144, 2048, 8, 4096), (4100, 1024, 8, 256), (6200, 512, 8, 256), (1000, 1024, 4, 4096),
+                                     (2048, 2048, 8, 65536), (4096, 1536, 8, 65536)])
+def test_quantizer_inside_the_split_k_kernel(N, K, d, C):
+    """Expander warps that quantize their tokens themselves give the bytes of the separate calls: one or two tokens a warp, tiles
+    that end early, rows with a pitch, of zeros, infinities and NaN, a residual, a capture."""
+    from sacq_b200 import quantize_rows
+    mod = _layer(N, K, d, C)
+    mod.set_kernel("large")
+    wide = _x(66, K + 16)
+    wide[3] = 0
+    wide[5, 7] = float("inf")
+    wide[9, K - 1] = float("nan")
+    res = _x(66, N, seed=4)
+    for x in (wide[:, :K].contiguous(), wide[:, 8:K + 8]):
+        for M in (1, 2, 8, 15, 16, 17, 31, 32, 33, 48, 64, 65):
+            q, s = quantize_rows(x[:M])
+            for y, ref in ((mod(x[:M]), mod.linear_a8(q, s)), (mod.forward_residual(x[:M], res[:M]), mod.linear_a8(q, s, residual=res[:M]))):
+                assert torch.equal(y.view(torch.int16), ref.view(torch.int16)), M
+    x, stream = wide[:16, :K].contiguous(), torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        y = mod(x)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y.view(torch.int16), mod(x).view(torch.int16)) and mod.device_status() == 0
+
+
 @pytest.mark.parametrize("N", [1024, 1000])
 def test_host_result_stored_by_the_gemm(N):
     """Pinned results: stored by the GEMM where the rows are whole cache lines, copied otherwise."""
