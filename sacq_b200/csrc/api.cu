@@ -124,9 +124,10 @@ int pick_kernel(const sacq_layer* L, int64_t M) {
   if (L->force_kernel == 1 || L->force_kernel >= 3)
     return small_m_supported(L) ? 1 : SACQ_ERR_UNSUPPORTED;
   if (L->force_kernel == 2) return large_m_supported(L) ? 2 : SACQ_ERR_UNSUPPORTED;
-  // A shape rule, not a backend switch.  The split-K kernel sums in an order that depends on K alone, so the row shards of
-  // a split per-channel layer reproduce the whole layer bit for bit where both run it, or both the persistent kernel:
-  // where a threshold depends on the width (17 to 32 tokens, 960 to 1,023, a codebook in L2) they may differ in the last bit.
+  // A shape rule, not a backend switch.  The split-K kernel sums in an order that depends on K and, from 256 tokens on, on the
+  // width of the whole layer, so the row shards of a split per-channel layer reproduce it bit for bit where both run that kernel
+  // or, above, the persistent one: where a threshold depends on the shard's own width (up to 32 tokens, 960 to 1,023 of layers
+  // deeper than 4,095, a codebook in L2) they may differ in the last bit.
   if (large_m_tmem_supported(L) && M >= tmem_min_m(L)) return 4;
   // Below, quantizer + GEMM of the small-M and the split-K kernel at 17 tokens: 1024x4096 10.9 / 6.8 us,
   // 6144x2048 15.4 / 11.5, 2048x6144 15.5 / 8.9; at 33: 1024x1024 7.3 / 5.7, 2048x2048 9.2 / 8.8, 4096x1024

@@ -29,6 +29,8 @@
 //                   quantizer 9.1 us fetched, 8.4 sent; 128 tokens, 2048 -> 6144 10.9 / 11.7.)
 // A CTA may take several slices, each with accumulator columns of its own: the order in which an output is
 // summed stays the same when many tokens leave no use for a cluster.
+// A call of few tokens may be this launch alone (QUANT): the tokens' bf16 rows come to shared memory by bulk copies and the
+// expander warps quantize them on the way, a warp per token.
 // In a row of calls a CTA starts when one of the call before ends, its activations come 4 us later; what it can do until then
 // is done ahead: copies, and the weights of up to seven stages.
 // Every mbarrier wait is bounded (status word + CTA-wide abort flag); an aborted CTA still reaches every
@@ -81,7 +83,7 @@ constexpr int ACT_FULL = 0, ACT_EMPTY = kMaxAct, W_FULL = 2 * kMaxAct, W_EMPTY =
               CB_FULL = IDX_FULL + 2, ACC_FULL = CB_FULL + 1, RECV = ACC_FULL + 1, X_FULL = RECV + 1, kBarriers = X_FULL + 1;
 
 struct SplitLayout {
-  uint32_t idx_off, cb_off, sc_off, recv_off, fixed_off, sa_off, sw_off, bias_off, bar_off, misc_off, x_off, total;
+  uint32_t idx_off, cb_off, sc_off, recv_off, fixed_off, sa_off, sw_off, bias_off, bar_off, misc_off, total;
 };
 
 // What a CTA's start depends on comes first: kernel parameters are read through a cache that is cold in every launch, a miss
@@ -131,8 +133,8 @@ __host__ __device__ inline SplitLayout split_layout(int tok, int split, int act_
   L.bias_off = L.sw_off + kRows * 4;
   L.bar_off = L.bias_off + kRows * 4;
   L.misc_off = L.bar_off + kBarriers * 8;
-  L.x_off = (L.misc_off + 64 + 127) & ~127u;
-  L.total = x_bytes > 0 ? L.x_off + (uint32_t)x_bytes : L.misc_off + 64;
+  L.total = L.misc_off + 64;
+  if (x_bytes > 0) L.total = ((L.total + 127) & ~127u) + (uint32_t)x_bytes;      // the rows of x come last
   return L;
 }
 
@@ -450,7 +452,7 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       const int rows = min(tok, p.M - m0), row_bytes = p.K * 2;
       if (elect_one()) mbar_arrive_expect_tx(bar(X_FULL), (uint32_t)(rows * row_bytes));
       __syncwarp();
-      if (lane < rows) bulk_load(base + L.x_off + (uint32_t)(lane * row_bytes), p.x + (int64_t)(m0 + lane) * p.x_pitch, (uint32_t)row_bytes, bar(X_FULL));
+      if (lane < rows) bulk_load(base + L.total - (uint32_t)((tok - lane) * row_bytes), p.x + (int64_t)(m0 + lane) * p.x_pitch, (uint32_t)row_bytes, bar(X_FULL));
       mbar_wait_warp(bar(X_FULL), 0, abort_flag, lay.status);
     }
     float sa[kMaxTok / 32];                           // the token scales: fetched now, put down behind the last copy
@@ -686,7 +688,7 @@ split_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
           if (now) ok = mbar_wait_warp(bar(X_FULL), 0, abort_flag, lay.status);
           if (!ok) break;
           for (int t = warp - 2; t < tok; t += kXWarps)
-            quantize_row(m0 + t < p.M ? reinterpret_cast<const uint4*>(sm + L.x_off + t * p.K * 2) : nullptr, p.K >> 3, kb0, kbs,
+            quantize_row(m0 + t < p.M ? reinterpret_cast<const uint4*>(sm + L.total - (tok - t) * p.K * 2) : nullptr, p.K >> 3, kb0, kbs,
                          sm + t * 128, tok * 128, t & 7, lane, reinterpret_cast<float*>(sm + L.sa_off) + t);
           fence_proxy_async();                        // the tensor cores read them
           __syncwarp();
