@@ -160,7 +160,6 @@ class ColumnParallelCodebookLinear(torch.nn.Module):
         local_bias = None if bias is None else bias[begin:end]
         self.local = PrecomputedPackedVectorCodebookLinear(shard_payload(payload, self.rank, self.world), local_bias,
                                                            device)
-        self.local.set_shard_of(self.out_features)     # the whole layer's order of sums
         self.chunks = max(1, int(chunks))
         self._comm_stream = None
         self.fused_exchange = bool(fused_exchange) and self.world > 1

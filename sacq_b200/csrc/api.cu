@@ -82,14 +82,14 @@ int64_t grouped_min_m(const sacq_layer* L) {
 }
 // From how many tokens the persistent kernel with the weights in tensor memory takes over; its 128-row tiles need that many
 // to fill the device.  The split-K kernel expands a wide layer again for every second 384-token tile, from about 700 tokens
-// on in a second wave.  Where both sum in the same order, it is measured time alone (eager, split-K / persistent: 2048x6144 at
-// 450 tokens 16.8 / 17.3 us, 512 17.5 / 17.6, 600 20.6 / 18.9, 700 21.3 / 19.5, 900 24.4 / 22.1; 1024x4096 at 512 10.1 / 10.7,
-// 600 11.7 / 11.2, 900 14.6 / 12.6).  Elsewhere the split-K kernel keeps them up to 960: up to there the tokens of a request
-// get the same bytes alone and in a batch of three.  A codebook that is gathered from L2 makes an expansion twice as
-// dear (2048x6144 at 400 30.4 / 28.7).  Narrower layers lose nothing (2048x2048 at 1,000 17.6 / 16.3, 6144x1536 30 / 37).
+// on in a second wave (1024x4096 at 1,000 tokens 23.5 / 12.6 us, 2048x6144 39 / 24).  It keeps them up to 960 all the same:
+// the two sum in different orders, and up to there the tokens of a request get the same bytes alone and in a batch of
+// three (the price: 2048x6144 at 700 tokens 30.6 / 19.4).  Below 1,024 of K they do sum alike, but there sibling layers gain by the
+// split-K kernel's shared launch what one layer loses (768x4096 at 560 9.7 / 9.1, two of them 11.2 / 16.2).  A codebook that is
+// gathered from L2 makes an expansion twice as dear (2048x6144 at 400 30.4 / 28.7).  Narrower layers lose nothing (2048x2048 at 1,000 17.6 / 16.3, 6144x1536 30 / 37).
 int64_t tmem_min_m(const sacq_layer* L) {
   if (L->d.out_features < 4096) return 1024;
-  return !split_k_codebook_in_smem(L) ? 384 : split_k_sums_whole(L) ? 560 : 960;
+  return split_k_codebook_in_smem(L) ? 960 : 384;
 }
 
 // From how many tokens a split-K kernel, which walks the weights once, beats a small-M kernel, which walks them
@@ -124,10 +124,9 @@ int pick_kernel(const sacq_layer* L, int64_t M) {
   if (L->force_kernel == 1 || L->force_kernel >= 3)
     return small_m_supported(L) ? 1 : SACQ_ERR_UNSUPPORTED;
   if (L->force_kernel == 2) return large_m_supported(L) ? 2 : SACQ_ERR_UNSUPPORTED;
-  // A shape rule, not a backend switch.  The split-K kernel sums in an order that depends on K and, from 256 tokens on, on the
-  // width of the whole layer, so the row shards of a split per-channel layer reproduce it bit for bit where both run that kernel
-  // or, above, the persistent one: where a threshold depends on the shard's own width (up to 32 tokens, 960 to 1,023 of layers
-  // deeper than 4,095, a codebook in L2) they may differ in the last bit.
+  // A shape rule, not a backend switch.  The split-K kernel sums in an order that depends on K alone, so the row shards of
+  // a split per-channel layer reproduce the whole layer bit for bit where both run it, or both the persistent kernel:
+  // where a threshold depends on the width (up to 32 tokens, 960 to 1,023, a codebook in L2) they may differ in the last bit.
   if (large_m_tmem_supported(L) && M >= tmem_min_m(L)) return 4;
   // Below, quantizer + GEMM of the small-M and the split-K kernel at 17 tokens: 1024x4096 10.9 / 6.8 us,
   // 6144x2048 15.4 / 11.5, 2048x6144 15.5 / 8.9; at 33: 1024x1024 7.3 / 5.7, 2048x2048 9.2 / 8.8, 4096x1024
@@ -220,7 +219,6 @@ SACQ_API int sacq_layer_create(const sacq_layer_desc* desc, sacq_layer_t** out_l
   }
   L->num_sms = prop.multiProcessorCount;
   L->cb_entries = (d.codebook_size + 1) & ~1;
-  L->order_rows = d.out_features;
   split_k_init(L);
   L->small_m_warps = small_m_staged_warps(L, 1);
   const int64_t count = (int64_t)L->cb_entries * d.vector_dim;
@@ -350,14 +348,6 @@ SACQ_API int sacq_layer_set_kernel(sacq_layer_t* L, int which) {
   if (int rc = check_layer(L)) return rc;
   if (which < 0 || which > 15) return set_error(SACQ_ERR_INVALID_ARGUMENT, "kernel selector %d not in 0..15", which);
   L->force_kernel = which;
-  return SACQ_OK;
-}
-
-SACQ_API int sacq_layer_set_shard_of(sacq_layer_t* L, int64_t rows) {
-  if (int rc = check_layer(L)) return rc;
-  if (rows < L->d.out_features)
-    return set_error(SACQ_ERR_INVALID_ARGUMENT, "a shard of %lld rows of a layer of %lld", (long long)L->d.out_features, (long long)rows);
-  L->order_rows = rows;
   return SACQ_OK;
 }
 

@@ -41,9 +41,7 @@ struct sacq_layer {
   float* row_mul;            // [N] power of two: 1 / what brings the row's largest scale into [2^11, 2^12)
   int* d_status;             // device status word, 0 = ok
   int small_m_warps;         // warps of the small-M path's staged warp-MMA kernel at one token, 0 if it has none for the layer
-  int64_t order_rows;        // rows of the whole layer that this one is a shard of (its own unless told): decides the order of sums
   int slice_idx[4], slice_groups[4];   // split-K kernel: index slices and scale groups of the largest slice of K cut into 1, 2, 4, 8
-  bool one_slice;            // split-K kernel: K fits a CTA in one piece (linear_split_k.cu)
   int split_tok[5];          // per form of the split-K kernel (SplitMode): its widest token tile, 0 if it cannot run the layer
   int64_t resident_bytes;
   sacq::LargeMPlan* large_plan;

@@ -201,7 +201,7 @@ int launch_large_m(const sacq_layer* L, const void* q, const float* scale, int64
 
 // Several layers of one geometry on the same quantized activations as ONE launch.  Returns
 // SACQ_ERR_UNSUPPORTED (nothing launched) when they cannot share one: the caller falls back
-// to one launch per layer.  Layers that sum in different orders do not share one, so the results are
+// to one launch per layer.  An output's summation order depends on K alone, so the results are
 // byte-identical to separate launches.
 int launch_large_m_multi(const sacq_layer* const* layers, int n, const void* q, const float* scale, int64_t M,
                          void* const* ys, const int64_t* ldys, cudaStream_t s) {

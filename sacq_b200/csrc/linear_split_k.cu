@@ -938,25 +938,13 @@ void slice_extent(const sacq_layer* L, int split, int* slices, int* groups) {
   }
 }
 
-// How many slices K is cut into: a function of K, so the order in which an output is summed does not depend on the
-// number of tokens -- a batch gives each of its rows the bytes of a smaller call, sibling layers share a launch,
-// and the row shards of a split layer reproduce it.  About 1,024 of K per CTA: measured at 64 and 300 tokens, two
-// slices are the best or within 10 % of it for K = 1,024 and 2,048 on 1,024- to 6,144-row layers, four for K = 4,096
-// and 6,144 (larger clusters leave SMs idle: 33 clusters of 4, 22 of 6, 15 of 8 run at once); eight above, where a
-// slice's indices would no longer fit shared memory.
+// How many slices K is cut into: a function of K alone, so the order in which an output is summed depends
+// neither on the number of tokens nor on the layer's width -- a batch gives each of its rows the bytes of a
+// smaller call, sibling layers share a launch, and the row shards of a split layer reproduce it.  About 1,024
+// of K per CTA: measured at 64 and 300 tokens, two slices are the best or within 10 % of it for K = 1,024 and
+// 2,048 on 1,024- to 6,144-row layers, four for K = 4,096 and 6,144 (larger clusters leave SMs idle: 33 clusters
+// of 4, 22 of 6, 15 of 8 run at once); eight above, where a slice's indices would no longer fit shared memory.
 int slices_for(int64_t K) { return K < 1024 ? 1 : K < 4096 ? 2 : K < 8192 ? 4 : 8; }
-
-// But from 256 tokens on a wide layer of two slices is summed in one piece: its row tiles alone fill most of the chip, the
-// columns that a second slice's accumulators would take hold twice the tokens, so two sibling layers are one wave instead
-// of two (2048 -> 6144, with the quantizer, eager: 300 tokens 15.4 / 14.4 us, 512 19.6 / 17.6; at 200 12.3 / 13.4; 1024 -> 4096
-// at 300 9.2 / 9.0); with dim-4 vectors, whose gathers take longer and whose indices twice the room, from 320 (4,096 entries,
-// 2048 -> 6144 at 256 14.1 / 15.4, 300 16.1 / 15.8, 400 18.7 / 17.4).  It is the order of the persistent kernel (linear_large_m_tmem.cu), which can therefore take over where
-// it is faster, at 560 tokens, and a request keeps its bytes in a batch.  Shards follow the width of the whole layer.
-constexpr int64_t kWholeMinRows = 4096;
-bool sums_whole(const sacq_layer* L) { return L->one_slice && L->order_rows >= kWholeMinRows; }
-int slices_of(const sacq_layer* L, int64_t M, SplitMode mode) {
-  return mode == kSplitHiLo && M >= (L->d.vector_dim == 8 ? 256 : 320) && sums_whole(L) ? 1 : slices_for(L->d.in_features);
-}
 
 // Completes a choice of tokens and slices; false if it does not fit shared memory.  Gathers from global memory need the
 // rest of the SM's memory as L1, a line for every miss in flight: beyond 164 KB only what is needed at all (65,536
@@ -1056,12 +1044,7 @@ void split_k_init(sacq_layer* L) {
     }
     L->split_tok[mode] = tok > 0 ? tok : 0;
   }
-  SplitChoice whole = cut_of(256, 256, 1, 1);
-  L->one_slice = slices_for(L->d.in_features) == 2 && codebook_smem(L) > 0 && takes_layer(L, kSplitHiLo) &&
-                 split_fits(L, kSplitHiLo, &whole);
 }
-
-bool split_k_sums_whole(const sacq_layer* L) { return slices_for(L->d.in_features) == 1 || sums_whole(L); }
 
 bool split_k_tiles_fit(const sacq_layer* L, int64_t M, SplitMode mode) {
   return L->split_tok[mode] == most_columns(mode) || M <= L->split_tok[mode];
@@ -1070,7 +1053,7 @@ bool split_k_tiles_fit(const sacq_layer* L, int64_t M, SplitMode mode) {
 bool split_k_choose(const sacq_layer* L, int64_t M, SplitMode mode, SplitChoice* out) {
   *out = SplitChoice();
   if (L->split_tok[mode] == 0 || M <= 0 || M > kSplitMaxM) return false;
-  const int slices = slices_of(L, M, mode);
+  const int slices = slices_for(L->d.in_features);
   for (int split = 1; split <= slices; split *= 2) {
     const int parts = slices / split;
     for (int tiles = least_tiles(M); parts <= 4 && tiles <= most_tiles(M); ++tiles) {
@@ -1108,8 +1091,7 @@ bool split_k_choose_multi(const sacq_layer* const* layers, int n, int64_t M, Spl
   for (int l = 0; l < n; ++l) {
     const sacq_layer_desc& d = layers[l]->d;
     if (d.in_features != d0.in_features || d.vector_dim != d0.vector_dim || d.index_bits != d0.index_bits ||
-        d.codebook_size != d0.codebook_size || d.group_size != d0.group_size || d.device != d0.device || d.out_features <= 0 ||
-        slices_of(layers[l], M, mode) != slices_of(layers[0], M, mode))
+        d.codebook_size != d0.codebook_size || d.group_size != d0.group_size || d.device != d0.device || d.out_features <= 0)
       return false;
     rows += (d.out_features + kRows - 1) / kRows * kRows;
   }

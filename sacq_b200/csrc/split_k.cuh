@@ -49,8 +49,6 @@ int launch_split_k(const sacq_layer* const* layers, int n, const void* act, cons
 // that are 16-byte aligned, instead of act and scale): their rows fit shared memory.
 bool split_k_quantizes(const sacq_layer* L, const SplitChoice& c);
 int64_t split_k_ctas(const sacq_layer* L, const SplitChoice& c);
-// Whether batches of the layer are summed in one piece of K, the persistent kernel's order.
-bool split_k_sums_whole(const sacq_layer* L);
 // Whether the layer's codebook fits the kernel's shared memory (else it is gathered from L2).
 bool split_k_codebook_in_smem(const sacq_layer* L);
 // Whether the quantizer in front of a call of M tokens should be the one that shares SMs with this kernel (act_quant.cu).

@@ -447,11 +447,6 @@ class PrecomputedPackedVectorCodebookLinear(torch.nn.Module):
         _lib.check(self._lib.sacq_layer_set_kernel(self._handle, int(code)))
         self._native.forget_sizes()
 
-    def set_shard_of(self, out_features: int) -> None:
-        """This layer holds some of the rows of a layer of ``out_features``: its outputs are summed in that layer's order."""
-        _lib.check(self._lib.sacq_layer_set_shard_of(self._handle, int(out_features)))
-        self._native.forget_sizes()
-
     def kernel_for(self, m: int) -> str:
         k = self._lib.sacq_layer_kernel_for(self._handle, m)
         if k < 0:

@@ -396,28 +396,27 @@ def test_split_k_deep_layers(kernel, N, K, d, C, G):
     assert mod.device_status() == 0
 
 
-@pytest.mark.parametrize("N,K,d,C,first", [(4096, 1024, 8, 256, 256), (6144, 2048, 8, 4096, 256), (4104, 3840, 8, 256, 256),
-                                           (4096, 2048, 4, 4096, 320)])
-def test_wide_batches_sum_in_one_order(N, K, d, C, first):
-    """From `first` tokens on a wide layer has one order of sums, whichever kernel and tile: rows repeat the bytes of a larger
-    call, a shard those of the whole layer, sibling layers of another width those of their own calls."""
+@pytest.mark.parametrize("N,K,d,C", [(4096, 1024, 8, 256), (6144, 2048, 8, 4096), (4104, 3840, 8, 256), (4096, 2048, 4, 4096),
+                                     (4160, 512, 8, 256)])
+def test_wide_layers_have_one_order_of_sums(N, K, d, C):
+    """A token's outputs are the same bytes in every call of 33 to 959 tokens: alone, in a batch, in the pieces of a chunked call, on
+    the rows of a shard; and layers of any widths share a launch."""
     from sacq_b200 import linear_a8_multi, quantize_rows, PrecomputedPackedVectorCodebookLinear
     from sacq_b200.column_parallel import shard_payload
     from sacq_b200.synthetic import make_payload
     p = make_payload(N, K, vector_dim=d, codebook_size=C, seed=N + K, device="cuda", iters=1, fit=False)
     mod = PrecomputedPackedVectorCodebookLinear(p, None, "cuda")
-    q, s = quantize_rows(_x(1200, K))
-    whole = mod.linear_a8(q, s)
-    assert mod.kernel_for(1200) == "large_tmem" and _err(mod, whole, q, s) <= TOL
     half = PrecomputedPackedVectorCodebookLinear(shard_payload(p, 1, 2), None, "cuda")
-    half.set_shard_of(N)
-    for M in (first, first + 1, 383, 385, 513, 559, 560, 561, 959, 1023):
-        y = mod.linear_a8(q[:M], s[:M])
-        assert torch.equal(y, whole[:M]), M
+    q, s = quantize_rows(_x(959, K))
+    whole = mod.linear_a8(q, s)
+    assert _err(mod, whole, q, s) <= TOL
+    for M in (33, 100, 255, 256, 257, 300, 319, 320, 385, 513, 559, 560, 561, 700, 958):
+        assert torch.equal(mod.linear_a8(q[:M], s[:M]), whole[:M]), M
         assert torch.equal(half.linear_a8(q[:M], s[:M]), whole[:M, N // 2:]), M
-    small = PrecomputedPackedVectorCodebookLinear(shard_payload(p, 0, 4), None, "cuda")     # a layer of its own: another order
-    for M in (first - 1, first, 300, 700):
-        for pair in ([mod, mod], [mod, small], [small, mod]):
-            for layer, y in zip(pair, linear_a8_multi(pair, q[:M], s[:M])):
-                assert torch.equal(y, layer.linear_a8(q[:M], s[:M])), M
+    for lo, hi in ((100, 200), (200, 300), (300, 959)):
+        assert torch.equal(mod.linear_a8(q[lo:hi], s[lo:hi]), whole[lo:hi]), (lo, hi)
+    before = mod._lib.sacq_launch_count()
+    both = linear_a8_multi([mod, half], q[:300], s[:300])
+    assert mod._lib.sacq_launch_count() - before == 1
+    assert torch.equal(both[0], whole[:300]) and torch.equal(both[1], whole[:300, N // 2:])
     assert mod.device_status() == 0 and half.device_status() == 0
