@@ -310,6 +310,12 @@ SACQ_API int64_t sacq_static_scratch_bytes(void);
  * tiles of 128, 256, 384 tokens), 12 = that design for grouped scales (13, 14, 15: likewise).
  * Returns SACQ_ERR_UNSUPPORTED from the next forward if the forced kernel cannot run the layer. */
 SACQ_API int sacq_layer_set_kernel(sacq_layer_t* layer, int which);
+/* Tells a layer that its rows are a shard of a layer of `rows` output features.  Which kernel a call runs on, and with it the
+ * order in which an output is summed, depends on the width of the layer; it is then the whole layer's, so that shards reproduce
+ * its bytes.  (Not on the CUDA-core kernel, which spreads a row's sum over as many CTAs as the rows leave: layers with a
+ * shift or a geometry that no tensor-core kernel takes.)  A narrow shard pays for it with kernels that are not the fastest for
+ * its own width; not told, it is equal to the whole layer up to the last bf16 bit. */
+SACQ_API int sacq_layer_set_shard_of(sacq_layer_t* layer, int64_t rows);
 /* Which kernel a forward with M rows would use (1 = small-M, 2 = split-K tensor-core kernel,
  * 3 = the same for grouped scales, 4 = tensor-core kernel for batches, 5 = the same for grouped scales), or a negative error. */
 SACQ_API int sacq_layer_kernel_for(const sacq_layer_t* layer, int64_t M);

@@ -90,6 +90,7 @@ SIGNATURES = {
     "sacq_linear_a8_static_scratch": (_int, [_vp, _vp, _fp, _i64, _vp, _i64, _vp]),
     "sacq_static_scratch_bytes": (_i64, []),
     "sacq_layer_set_kernel": (_int, [_vp, _int]),
+    "sacq_layer_set_shard_of": (_int, [_vp, _i64]),
     "sacq_layer_kernel_for": (_int, [_vp, _i64]),
     "sacq_layer_status": (_int, [_vp, ctypes.POINTER(_int)]),
     "sacq_launch_count": (_i64, []),

@@ -7,9 +7,16 @@ a row's bits end on a byte boundary -- computes ``y[:, rows]`` with the single-G
 and the ranks exchange their column blocks with ONE all-gather over NVLink (NCCL through
 ``torch.distributed``).  Activations and their per-token scales are replicated, so each
 output element is produced by exactly one GPU.  The gathered result is bit-identical to the
-one-GPU result whenever the shard and the whole layer sum an output in the same order (always
-on the tensor-core kernel, whose order does not depend on the tile shape; on the small-M
-kernel when both pick the same tile class), and otherwise equal up to the last bf16 bit.
+one-GPU result whenever shard and whole layer run on the same kernel: none of the tensor-core
+kernels sums an output in an order that depends on the tile shape.  Per-channel layers do so in calls
+of 49 to 383 tokens (unless they are so deep that shared memory narrows the split-K kernel's tiles).
+Elsewhere rules that look at a layer's width may pick different kernels, or two tile classes of the
+small-M kernel, and the results are equal up to the last bf16 bit.  ``same_bytes=True``
+makes the shard follow the whole layer's rules, at the price of kernels that are not the fastest
+for its own width (4-way shards of 2048 x 6144 at 16 tokens: 4.9 -> 6.3 us, dim 4 with grouped
+scales 6.2 -> 9.3).  Not then either: on the CUDA-core kernel (layers that no tensor-core kernel
+takes), which spreads a sum over as many CTAs as the rows leave, and with ``chunks > 1`` where a
+piece has fewer tokens than the whole call's kernel takes.
 
 The reference has no multi-GPU inference path (its only collective is the calibration
 trainer's gradient all-reduce); this module is new work on top of the same payload format.
@@ -145,10 +152,11 @@ class ColumnParallelCodebookLinear(torch.nn.Module):
 
     ``forward(x)`` takes the replicated ``[..., K]`` activations and returns the full
     ``[..., N]`` output on every rank.  ``chunks > 1`` splits the token dimension so the
-    gather of one chunk overlaps the GEMM of the next."""
+    gather of one chunk overlaps the GEMM of the next.  ``same_bytes=True`` runs the shard on the
+    kernel that one GPU would run the whole layer on."""
 
     def __init__(self, payload: dict, bias: torch.Tensor | None, device: str, group=None, chunks: int = 1,
-                 fused_exchange: bool = False, max_tokens: int = 8192):
+                 fused_exchange: bool = False, max_tokens: int = 8192, same_bytes: bool = False):
         super().__init__()
         from .linear import PrecomputedPackedVectorCodebookLinear
         self.group = group
@@ -160,6 +168,8 @@ class ColumnParallelCodebookLinear(torch.nn.Module):
         local_bias = None if bias is None else bias[begin:end]
         self.local = PrecomputedPackedVectorCodebookLinear(shard_payload(payload, self.rank, self.world), local_bias,
                                                            device)
+        if same_bytes:
+            self.local.set_shard_of(self.out_features)
         self.chunks = max(1, int(chunks))
         self._comm_stream = None
         self.fused_exchange = bool(fused_exchange) and self.world > 1

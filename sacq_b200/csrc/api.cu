@@ -118,15 +118,19 @@ bool large_m_cedes(const sacq_layer* L, int64_t M) {
 }
 
 int pick_kernel(const sacq_layer* L, int64_t M) {
+  if (is_shard(L)) {                                   // whether a kernel can run a layer does not depend on its width
+    const sacq_layer whole = whole_layer(L);
+    return pick_kernel(&whole, M);
+  }
   if (L->force_kernel == 7) return large_m_grouped_supported(L) ? 3 : SACQ_ERR_UNSUPPORTED;
   if (L->force_kernel >= 12) return large_m_tmem_grouped_supported(L) ? 5 : SACQ_ERR_UNSUPPORTED;
   if (L->force_kernel >= 8) return large_m_tmem_supported(L) ? 4 : SACQ_ERR_UNSUPPORTED;
   if (L->force_kernel == 1 || L->force_kernel >= 3)
     return small_m_supported(L) ? 1 : SACQ_ERR_UNSUPPORTED;
   if (L->force_kernel == 2) return large_m_supported(L) ? 2 : SACQ_ERR_UNSUPPORTED;
-  // A shape rule, not a backend switch.  The split-K kernel sums in an order that depends on K alone, so the row shards of
-  // a split per-channel layer reproduce the whole layer bit for bit where both run it, or both the persistent kernel:
-  // where a threshold depends on the width (up to 32 tokens, 960 to 1,023, a codebook in L2) they may differ in the last bit.
+  // A shape rule, not a backend switch.  The tensor-core kernels sum in an order that depends on K alone (the staged warp-MMA
+  // kernel on its tile class too, see make_plan), so the row shards of a split layer reproduce the whole layer bit for bit
+  // where they run the same kernel.  Thresholds depend on the width, hence the whole layer's.
   if (large_m_tmem_supported(L) && M >= tmem_min_m(L)) return 4;
   // Below, quantizer + GEMM of the small-M and the split-K kernel at 17 tokens: 1024x4096 10.9 / 6.8 us,
   // 6144x2048 15.4 / 11.5, 2048x6144 15.5 / 8.9; at 33: 1024x1024 7.3 / 5.7, 2048x2048 9.2 / 8.8, 4096x1024
@@ -219,6 +223,7 @@ SACQ_API int sacq_layer_create(const sacq_layer_desc* desc, sacq_layer_t** out_l
   }
   L->num_sms = prop.multiProcessorCount;
   L->cb_entries = (d.codebook_size + 1) & ~1;
+  L->order_rows = d.out_features;
   split_k_init(L);
   L->small_m_warps = small_m_staged_warps(L, 1);
   const int64_t count = (int64_t)L->cb_entries * d.vector_dim;
@@ -351,6 +356,15 @@ SACQ_API int sacq_layer_set_kernel(sacq_layer_t* L, int which) {
   return SACQ_OK;
 }
 
+SACQ_API int sacq_layer_set_shard_of(sacq_layer_t* L, int64_t rows) {
+  if (int rc = check_layer(L)) return rc;
+  if (rows < L->d.out_features || rows > (1 << 24))
+    return set_error(SACQ_ERR_INVALID_ARGUMENT, "a shard of %lld rows of a layer of %lld", (long long)L->d.out_features, (long long)rows);
+  L->order_rows = rows;
+  L->small_m_warps = small_m_staged_warps(L, 1);
+  return SACQ_OK;
+}
+
 SACQ_API int sacq_layer_kernel_for(const sacq_layer_t* L, int64_t M) {
   if (int rc = check_layer(L)) return rc;
   const int k = pick_kernel(L, M);
@@ -428,6 +442,10 @@ namespace {
 // 13.9 / 12.7 at 40, 1536x1536 8.9 / 10.6 at 40), else the CUDA-core kernel.
 enum Int8Route { kInt8Small, kInt8Grouped, kInt8TmemGrouped };
 Int8Route int8_route(const sacq_layer* L, int64_t M) {
+  if (is_shard(L)) {
+    const sacq_layer whole = whole_layer(L);
+    return int8_route(&whole, M);
+  }
   if (large_m_tmem_grouped_supported(L) && M >= large_m_tmem_grouped_min_m(L)) return kInt8TmemGrouped;
   if (large_m_grouped_cedes(L, M, true)) return kInt8TmemGrouped;
   if (!large_m_grouped_supported(L)) return kInt8Small;
@@ -534,7 +552,7 @@ namespace {
 bool recipe_in_one(const sacq_layer* L, const void* q, const float* act_scale, const float* w_scale, int64_t M, void* y,
                    int64_t ldy, SplitMode mode, cudaStream_t s, int* rc) {
   SplitChoice c;
-  const bool wide = L->d.out_features >= 4096 && L->d.in_features >= 2048;
+  const bool wide = L->order_rows >= 4096 && L->d.in_features >= 2048;
   if (M > (!wide ? 32 : split_k_codebook_in_smem(L) ? 320 : 200) || reinterpret_cast<uintptr_t>(q) % 16 != 0 ||
       reinterpret_cast<uintptr_t>(L->d.codebook) % 16 != 0 ||
       (mode == kSplitInt8 && L->d.in_features * 127 * 127 > 2147483647LL) || !split_k_tiles_fit(L, M, mode) ||

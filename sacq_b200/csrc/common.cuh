@@ -41,6 +41,7 @@ struct sacq_layer {
   float* row_mul;            // [N] power of two: 1 / what brings the row's largest scale into [2^11, 2^12)
   int* d_status;             // device status word, 0 = ok
   int small_m_warps;         // warps of the small-M path's staged warp-MMA kernel at one token, 0 if it has none for the layer
+  int64_t order_rows;        // rows of the whole layer that this one is a shard of (its own unless told): they choose the kernel
   int slice_idx[4], slice_groups[4];   // split-K kernel: index slices and scale groups of the largest slice of K cut into 1, 2, 4, 8
   int split_tok[5];          // per form of the split-K kernel (SplitMode): its widest token tile, 0 if it cannot run the layer
   int64_t resident_bytes;
@@ -55,6 +56,14 @@ namespace sacq {
 // reconstruction, which a shift larger than the weights makes visible.  Shifted layers therefore
 // run on kernels that rebuild bf16(bf16(c * s) + shift) per weight.
 inline bool has_shift(const sacq_layer* L) { return (L->d.shift_bf16 & 0x7fffu) != 0; }
+
+inline bool is_shard(const sacq_layer* L) { return L->order_rows != L->d.out_features; }
+// The whole layer of a shard, for rules that ask for its width: no kernel may be launched with it.
+inline sacq_layer whole_layer(const sacq_layer* L) {
+  sacq_layer whole = *L;
+  whole.d.out_features = L->order_rows;
+  return whole;
+}
 
 int set_error(int code, const char* fmt, ...);
 int cuda_fail(cudaError_t e, const char* what);

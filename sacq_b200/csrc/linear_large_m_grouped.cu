@@ -38,7 +38,7 @@ bool large_m_grouped_exact(const sacq_layer* L, int64_t M, bool int8) {
   if (!split_k_codebook_in_smem(L)) return true;
   if (int8) return M < 48;
   if (L->force_kernel == 7) return false;
-  return M < (L->d.out_features >= 32 * (int64_t)L->num_sms ? 33 : L->d.out_features >= 2048 ? 48 : 96);
+  return M < (L->order_rows >= 32 * (int64_t)L->num_sms ? 33 : L->order_rows >= 2048 ? 48 : 96);
 }
 
 bool large_m_grouped_supported(const sacq_layer* L) { return L->d.index_bits >= 1 && L->split_tok[kSplitHalf] > 0; }

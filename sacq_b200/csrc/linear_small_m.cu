@@ -402,10 +402,15 @@ bool plan_unpacked(const sacq_layer* L, Plan& pl) {
 // M from which the warp-MMA variant is preferred over the CUDA-core one.
 constexpr int64_t kMmaMinM = 1;
 
-// halves_req: 0 = free choice of the tile height; 2 / 1 = only tile heights whose staged kernel
-// runs two / one warp per span (the summation order of an output depends on that, not on N).
+// halves_req: 0 = free choice of the tile height, on a shard among those of the whole layer's class; 2 / 1 = only tile heights
+// whose staged kernel runs two / one warp per span (the summation order of an output depends on that, not on N).
 Plan make_plan(const sacq_layer* L, int64_t M, int halves_req = 0) {
   const sacq_layer_desc& d = L->d;
+  if (halves_req == 0 && is_shard(L)) {
+    const sacq_layer whole = whole_layer(L);
+    const Plan pl = make_plan(&whole, M);
+    if (pl.mma && pl.staged && !pl.unpacked) halves_req = staged_halves(pl.r8);
+  }
   Plan pl{};
   pl.fast = fast_eligible(L);
   pl.mma = pl.fast && (L->force_kernel == 4 || L->force_kernel == 5 || (L->force_kernel != 3 && M >= kMmaMinM));
@@ -718,7 +723,7 @@ int launch_small_m_multi(const sacq_layer* const* layers, int n, const void* q, 
   }
   // plan for the concatenation of the layers' rows: tile height and CTA count
   sacq_layer virt = *L0;
-  virt.d.out_features = n_total;
+  virt.d.out_features = virt.order_rows = n_total;
   Plan pl = make_plan(&virt, M, halves);
   if (!pl.mma || !pl.staged || pl.unpacked || pl.smem > kSmemBudget || staged_halves(pl.r8) != halves)
     return SACQ_ERR_UNSUPPORTED;

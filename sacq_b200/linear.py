@@ -447,6 +447,12 @@ class PrecomputedPackedVectorCodebookLinear(torch.nn.Module):
         _lib.check(self._lib.sacq_layer_set_kernel(self._handle, int(code)))
         self._native.forget_sizes()
 
+    def set_shard_of(self, out_features: int) -> None:
+        """This layer holds some of the rows of a layer of ``out_features``: it runs the kernels that layer would, and so gives
+        its bytes."""
+        _lib.check(self._lib.sacq_layer_set_shard_of(self._handle, int(out_features)))
+        self._native.forget_sizes()
+
     def kernel_for(self, m: int) -> str:
         k = self._lib.sacq_layer_kernel_for(self._handle, m)
         if k < 0:

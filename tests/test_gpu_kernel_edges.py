@@ -420,3 +420,32 @@ def test_wide_layers_have_one_order_of_sums(N, K, d, C):
     assert mod._lib.sacq_launch_count() - before == 1
     assert torch.equal(both[0], whole[:300]) and torch.equal(both[1], whole[:300, N // 2:])
     assert mod.device_status() == 0 and half.device_status() == 0
+
+
+@pytest.mark.parametrize("N,K,d,C,G", [(6144, 2048, 8, 4096, None), (4096, 1024, 8, 256, None), (2048, 1024, 8, 65536, None),
+                                       (6144, 1536, 4, 4096, None), (6144, 2048, 4, 1024, 64), (4096, 1024, 4, 64, 64),
+                                       (2048, 6144, 4, 1024, 64)])
+def test_a_shard_gives_the_bytes_of_the_whole_layer(N, K, d, C, G):
+    """Told of the whole layer, its rows run the kernel that the layer would, at every number of tokens where a rule looks at the
+    width: FP8 and INT8 activations, quantized before or inside the call."""
+    from sacq_b200 import quantize_rows, PrecomputedPackedVectorCodebookLinear
+    from sacq_b200._lib import SacqError
+    from sacq_b200.column_parallel import shard_payload
+    from sacq_b200.synthetic import make_payload
+    p = make_payload(N, K, vector_dim=d, codebook_size=C, group_size=G, seed=N + K, device="cuda", iters=1, fit=False)
+    mod = PrecomputedPackedVectorCodebookLinear(p, None, "cuda")
+    x = _x(1030, K)
+    sizes = (1, 8, 9, 16, 17, 28, 29, 32, 33, 40, 47, 48, 50, 95, 96, 384, 448, 600, 959, 960, 1023, 1025)
+    want = {M: (mod(x[:M]), mod.forward_int8(x[:M])) for M in sizes}
+    for rank, world in ((1, 2), (2, 4), (7, 8)):
+        part = PrecomputedPackedVectorCodebookLinear(shard_payload(p, rank, world), None, "cuda")
+        part.set_shard_of(N)
+        cols = slice(rank * N // world, (rank + 1) * N // world)
+        for M in sizes:
+            assert part.kernel_for(M) == mod.kernel_for(M)
+            assert torch.equal(part(x[:M]), want[M][0][:, cols]), (world, M)
+            assert torch.equal(part.linear_a8(*quantize_rows(x[:M])), want[M][0][:, cols]), (world, M)
+            assert torch.equal(part.forward_int8(x[:M]), want[M][1][:, cols]), (world, M)
+        with pytest.raises(SacqError):
+            part.set_shard_of(N // world - 1)
+        assert part.device_status() == 0
