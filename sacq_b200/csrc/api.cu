@@ -386,7 +386,7 @@ namespace {
 // form: what q holds (fp16 only where the chosen kernel takes it, see sacq_forward_call).
 int linear_a8_impl(const sacq_layer_t* L, const void* q, const float* scale, int64_t M, const void* residual,
                    int64_t ldr, void* y_out, int64_t ldy, void* workspace, int64_t workspace_bytes, void* stream,
-                   const BcastDst* bc = nullptr, ActForm form = kActE4M3) {
+                   const BcastDst* bc = nullptr, ActForm form = kActE4M3, const SplitChoice* cut = nullptr) {
   if (int rc = check_layer(L)) return rc;
   if (M < 0) return set_error(SACQ_ERR_INVALID_ARGUMENT, "M=%lld is negative", (long long)M);
   if (M == 0 || L->d.out_features == 0) return SACQ_OK;
@@ -402,7 +402,7 @@ int linear_a8_impl(const sacq_layer_t* L, const void* q, const float* scale, int
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int k = pick_kernel(L, M);
   if (k < 0) return set_error(k, "no kernel can run this layer geometry");
-  if (k == 2) return launch_large_m(L, q, scale, M, y_out, ldy, s, residual, ldr, bc);
+  if (k == 2) return launch_large_m(L, q, scale, M, y_out, ldy, s, residual, ldr, bc, cut);
   if (k == 4)
     return launch_large_m_tmem(L, q, scale, M, y_out, ldy, s, residual, ldr, bc,
                                L->force_kernel >= 9 ? L->force_kernel - 8 : 0);
@@ -415,7 +415,7 @@ int linear_a8_impl(const sacq_layer_t* L, const void* q, const float* scale, int
                                          workspace_bytes - kCounterBytes, s, residual, ldr, form, bc,
                                          L->force_kernel >= 13 ? L->force_kernel - 12 : 0);
     return launch_large_m_grouped(L, q, scale, M, y_out, ldy, static_cast<uint8_t*>(workspace) + kCounterBytes,
-                                  workspace_bytes - kCounterBytes, s, residual, ldr, form, large_m_grouped_exact(L, M, false), bc);
+                                  workspace_bytes - kCounterBytes, s, residual, ldr, form, large_m_grouped_exact(L, M, false), bc, cut);
   }
   const int64_t slab = small_m_slab_rows(L);
   for (int64_t m0 = 0; m0 < M; m0 += slab) {
@@ -481,7 +481,7 @@ SACQ_API int64_t sacq_workspace_bytes_int8(const sacq_layer_t* L, int64_t M) {
 
 namespace {
 int linear_a8i_impl(const sacq_layer_t* L, const void* q, const float* scale, int64_t M, void* y_out, int64_t ldy,
-                    void* workspace, int64_t workspace_bytes, void* stream, ActForm form) {
+                    void* workspace, int64_t workspace_bytes, void* stream, ActForm form, const SplitChoice* cut = nullptr) {
   DeviceGuard guard(L->d.device);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const Int8Route r = int8_route(L, M);
@@ -493,7 +493,7 @@ int linear_a8i_impl(const sacq_layer_t* L, const void* q, const float* scale, in
                ? launch_large_m_tmem_grouped(L, q, scale, M, y_out, ldy, static_cast<uint8_t*>(workspace) + kCounterBytes,
                                              workspace_bytes - kCounterBytes, s, nullptr, 0, form)
                : launch_large_m_grouped(L, q, scale, M, y_out, ldy, static_cast<uint8_t*>(workspace) + kCounterBytes,
-                                        workspace_bytes - kCounterBytes, s, nullptr, 0, form, large_m_grouped_exact(L, M, true));
+                                        workspace_bytes - kCounterBytes, s, nullptr, 0, form, large_m_grouped_exact(L, M, true), nullptr, cut);
   }
   if (!small_m_supported(L)) return set_error(SACQ_ERR_UNSUPPORTED, "no kernel can run this layer geometry");
   sacq_layer view = *L;
@@ -790,6 +790,8 @@ int forward_impl(const sacq_layer_t* L, const void* x_bf16, int64_t x_pitch, int
   if (M == 0) return SACQ_OK;
   const int64_t K = L->d.in_features;
   bool beside = false;                                // the quantizer runs beside the split-K kernel
+  SplitChoice c;                                      // how that kernel's call is cut up: searched once (0.2 to 0.4 us)
+  const SplitChoice* cut = nullptr;
   int64_t slab = 0;                                   // tokens up to which the GEMM takes fp16 activations in one piece
   int64_t need = 0;
   const bool rows_ok = M > 0 && L->d.out_features > 0 && K % 8 == 0 && x_bf16 != nullptr &&
@@ -805,8 +807,8 @@ int forward_impl(const sacq_layer_t* L, const void* x_bf16, int64_t x_pitch, int
     }
     if (k == 2 || k == 3 || r == kInt8Grouped) {
       const SplitMode mode = k == 2 ? kSplitHiLo : large_m_grouped_exact(L, M, int8 != 0) ? kSplitHalf2 : kSplitHalf;
-      SplitChoice c;
       if (M <= 1024 && split_k_choose(L, M, mode, &c)) {
+        cut = &c;
         if (k == 2 && !own_quantizer && (residual == nullptr || ldr >= L->d.out_features) &&
             quantizes_in_split(L, M, static_cast<cudaStream_t>(stream), c)) {
           DeviceGuard guard(L->d.device);
@@ -832,9 +834,9 @@ int forward_impl(const sacq_layer_t* L, const void* x_bf16, int64_t x_pitch, int
     void* a16 = static_cast<uint8_t*>(workspace) + kCounterBytes;
     if (int rc = launch_quant_act(x_bf16, x_pitch, M, K, int8 != 0, true, a16, scale_scratch, static_cast<cudaStream_t>(stream), beside))
       return rc;
-    if (int8) return linear_a8i_impl(L, a16, scale_scratch, M, y_out, ldy, workspace, workspace_bytes, stream, kActHalf);
+    if (int8) return linear_a8i_impl(L, a16, scale_scratch, M, y_out, ldy, workspace, workspace_bytes, stream, kActHalf, cut);
     return linear_a8_impl(L, a16, scale_scratch, M, residual, ldr, y_out, ldy, workspace, workspace_bytes, stream, nullptr,
-                          kActHalf);
+                          kActHalf, cut);
   }
   const int rc = beside && q_scratch != nullptr && scale_scratch != nullptr
                      ? launch_quant_act(x_bf16, x_pitch, M, K, int8 != 0, false, q_scratch, scale_scratch, static_cast<cudaStream_t>(stream), true)
@@ -842,7 +844,8 @@ int forward_impl(const sacq_layer_t* L, const void* x_bf16, int64_t x_pitch, int
                         : sacq_quant_act_fp8(x_bf16, x_pitch, M, K, q_scratch, scale_scratch, stream);
   if (rc != SACQ_OK) return rc;
   if (int8) return sacq_linear_a8i(L, q_scratch, scale_scratch, M, y_out, ldy, workspace, workspace_bytes, stream);
-  return linear_a8_impl(L, q_scratch, scale_scratch, M, residual, ldr, y_out, ldy, workspace, workspace_bytes, stream);
+  return linear_a8_impl(L, q_scratch, scale_scratch, M, residual, ldr, y_out, ldy, workspace, workspace_bytes, stream, nullptr,
+                        kActE4M3, cut);
 }
 
 // Whether the kernel of a call with M tokens may store its result straight into pinned host memory: one whose stores

@@ -19,6 +19,7 @@ constexpr float kE4M3Max = 448.0f;
 
 struct LargeMPlan;  // built lazily by the large-M kernel's host code
 struct SplitPlan;   // ... and by the split-K kernel's
+struct SplitChoice; // how one of its calls is cut up (split_k.cuh)
 
 }  // namespace sacq
 
@@ -117,8 +118,10 @@ int launch_small_m_multi(const sacq_layer* const* layers, int n, const void* q, 
                          void* const* ys, const int64_t* ldys, cudaStream_t s);
 
 bool large_m_supported(const sacq_layer* L);
+// cut: how the call is cut up, if its caller has searched that already (M at most one slab; launch_large_m_grouped likewise)
 int launch_large_m(const sacq_layer* L, const void* q, const float* scale, int64_t M, void* y, int64_t ldy,
-                   cudaStream_t s, const void* residual = nullptr, int64_t ldr = 0, const BcastDst* bc = nullptr);
+                   cudaStream_t s, const void* residual = nullptr, int64_t ldr = 0, const BcastDst* bc = nullptr,
+                   const SplitChoice* cut = nullptr);
 int launch_large_m_multi(const sacq_layer* const* layers, int n, const void* q, const float* scale, int64_t M,
                          void* const* ys, const int64_t* ldys, cudaStream_t s);
 void large_m_release(sacq_layer* L);
@@ -146,7 +149,7 @@ bool large_m_grouped_exact(const sacq_layer* L, int64_t M, bool int8);
 bool large_m_grouped_cedes(const sacq_layer* L, int64_t M, bool int8);
 int launch_large_m_grouped(const sacq_layer* L, const void* q, const float* scale, int64_t M, void* y, int64_t ldy,
                            void* ws, int64_t ws_bytes, cudaStream_t s, const void* residual, int64_t ldr, ActForm form,
-                           bool exact, const BcastDst* bc = nullptr);
+                           bool exact, const BcastDst* bc = nullptr, const SplitChoice* cut = nullptr);
 int64_t large_m_grouped_slab(void);
 
 int launch_large_m_grouped_multi(const sacq_layer* const* layers, int n, const void* q, const float* scale, int64_t M,

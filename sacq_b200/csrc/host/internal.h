@@ -15,6 +15,9 @@ SACQ_API int sacq_forward_call(const sacq_layer_t* layer, const void* x_bf16, in
                                const void* residual, int64_t ldr, void* q_scratch, float* scale_scratch, void* y_out,
                                int64_t ldy, void* workspace, int64_t workspace_bytes, void* stream);
 
+/* How often the cut of a split-K call has been searched so far (host time that a call should pay once). */
+SACQ_API int64_t sacq_split_search_count(void);
+
 #ifdef __cplusplus
 }
 #endif

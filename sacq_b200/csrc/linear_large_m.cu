@@ -180,14 +180,15 @@ int tile_output(const sacq_layer* L, int64_t M, void* y, int64_t ldy, const void
 }
 
 int launch_large_m(const sacq_layer* L, const void* q, const float* scale, int64_t M, void* y, int64_t ldy,
-                   cudaStream_t s, const void* residual, int64_t ldr, const BcastDst* bc) {
+                   cudaStream_t s, const void* residual, int64_t ldr, const BcastDst* bc, const SplitChoice* cut) {
   if (!large_m_supported(L)) return set_error(SACQ_ERR_UNSUPPORTED, "large-M kernel cannot run this layer geometry");
   if (M <= 0 || L->d.out_features == 0) return SACQ_OK;
   if (M > (1 << 30)) return set_error(SACQ_ERR_UNSUPPORTED, "M=%lld too large", (long long)M);
   for (int64_t m0 = 0; m0 < M; m0 += kSplitMaxM) {
     const int64_t rows = M - m0 < kSplitMaxM ? M - m0 : kSplitMaxM;
     SplitChoice c;
-    if (!split_k_choose(L, rows, kSplitHiLo, &c)) return set_error(SACQ_ERR_UNSUPPORTED, "split-K kernel: no tile fits");
+    if (cut != nullptr) c = *cut;
+    else if (!split_k_choose(L, rows, kSplitHiLo, &c)) return set_error(SACQ_ERR_UNSUPPORTED, "split-K kernel: no tile fits");
     BcastDst slab{};
     for (int i = 0; bc != nullptr && i < bc->n; ++i) slab.ptr[slab.n++] = static_cast<uint16_t*>(bc->ptr[i]) + m0 * ldy;
     void* y_slab = static_cast<uint16_t*>(y) + m0 * ldy;

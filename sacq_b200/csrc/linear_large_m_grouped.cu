@@ -63,7 +63,7 @@ int64_t large_m_grouped_workspace_bytes(const sacq_layer* L, int64_t M) {
 
 int launch_large_m_grouped(const sacq_layer* L, const void* q, const float* scale, int64_t M, void* y, int64_t ldy,
                            void* ws, int64_t ws_bytes, cudaStream_t s, const void* residual, int64_t ldr,
-                           ActForm form, bool exact, const BcastDst* bc) {
+                           ActForm form, bool exact, const BcastDst* bc, const SplitChoice* cut) {
   if (!large_m_grouped_supported(L))
     return set_error(SACQ_ERR_UNSUPPORTED, "grouped tensor-core kernel cannot run this layer geometry");
   if (M <= 0 || L->d.out_features == 0) return SACQ_OK;
@@ -72,8 +72,9 @@ int launch_large_m_grouped(const sacq_layer* L, const void* q, const float* scal
   if (form == kActHalf) {
     SplitChoice c;
     const SplitMode mode = form_of(exact);
-    if (M > kSlabTokens || !split_k_choose(L, M, mode, &c)) return set_error(SACQ_ERR_UNSUPPORTED, "M=%lld exceeds a slab", (long long)M);
-    return launch_split_k(&L, 1, q, scale, M, &y, &ldy, mode, c, s, residual, ldr, bc);
+    if (M > kSlabTokens || (cut == nullptr && !split_k_choose(L, M, mode, &c)))
+      return set_error(SACQ_ERR_UNSUPPORTED, "M=%lld exceeds a slab", (long long)M);
+    return launch_split_k(&L, 1, q, scale, M, &y, &ldy, mode, cut != nullptr ? *cut : c, s, residual, ldr, bc);
   }
   const int64_t need = large_m_grouped_workspace_bytes(L, M);
   if (ws == nullptr || ws_bytes < need)
@@ -87,7 +88,8 @@ int launch_large_m_grouped(const sacq_layer* L, const void* q, const float* scal
     const int64_t rows = (M - m0) < kSlabTokens ? (M - m0) : kSlabTokens;
     if (int rc = launch_widen(static_cast<const uint8_t*>(q) + m0 * K, rows, K, form == kActInt8, ws, s)) return rc;
     SplitChoice c;
-    if (!split_k_choose(L, rows, mode, &c)) return set_error(SACQ_ERR_UNSUPPORTED, "grouped tensor-core kernel: no tile fits");
+    if (cut != nullptr && M <= kSlabTokens) c = *cut;
+    else if (!split_k_choose(L, rows, mode, &c)) return set_error(SACQ_ERR_UNSUPPORTED, "grouped tensor-core kernel: no tile fits");
     BcastDst slab{};
     for (int i = 0; bc != nullptr && i < bc->n; ++i) slab.ptr[slab.n++] = static_cast<uint16_t*>(bc->ptr[i]) + m0 * ldy;
     void* y_slab = static_cast<uint16_t*>(y) + m0 * ldy;

@@ -39,11 +39,13 @@
 #include <math.h>
 #include <string.h>
 
+#include <atomic>
 #include <mutex>
 #include <type_traits>
 
 #include "common.cuh"
 #include "encode.cuh"
+#include "host/internal.h"
 #include "split_k.cuh"
 #include "tmem_weights.cuh"
 #include "umma.cuh"
@@ -843,6 +845,7 @@ struct SplitPlan {
 
 namespace {
 
+std::atomic<int64_t> g_searches{0};
 std::mutex g_split_mutex;       // layers build their index maps on first use, possibly from several host threads
 
 // Boxes of 64 bytes of 128 rows over the packed rows.  (Boxes of 16 bytes, in the order the expanders read them, cost the
@@ -1052,6 +1055,7 @@ bool split_k_tiles_fit(const sacq_layer* L, int64_t M, SplitMode mode) {
 
 bool split_k_choose(const sacq_layer* L, int64_t M, SplitMode mode, SplitChoice* out) {
   *out = SplitChoice();
+  g_searches.fetch_add(1, std::memory_order_relaxed);
   if (L->split_tok[mode] == 0 || M <= 0 || M > kSplitMaxM) return false;
   const int slices = slices_for(L->d.in_features);
   for (int split = 1; split <= slices; split *= 2) {
@@ -1178,3 +1182,5 @@ int launch_split_k(const sacq_layer* const* layers, int n, const void* act, cons
 }
 
 }  // namespace sacq
+
+extern "C" SACQ_API int64_t sacq_split_search_count(void) { return sacq::g_searches.load(std::memory_order_relaxed); }

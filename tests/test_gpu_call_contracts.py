@@ -1,5 +1,7 @@
 """What a call has to keep whichever kernel it runs on: the kernel that was asked for, the precision of its operands, the
 order of the stream, the errors it raises.  Oracle: float64 sums of the payload's own codewords and scales."""
+import ctypes
+
 import pytest
 import torch
 
@@ -356,3 +358,21 @@ def test_recipe_takes_more_tokens_than_the_small_tiles_can():
     q, s = quantize_rows(_x(1 << 12, 16).repeat(M // (1 << 12) + 1, 1)[:M], "int8_symmetric")
     y = mod.linear_w8a8_int8(q, s, sw)
     assert torch.equal(y[-500:], mod.linear_w8a8_int8(q[-500:].contiguous(), s[-500:].contiguous(), sw))
+
+
+@pytest.mark.parametrize("N,K,d,C,G,M", [(2048, 6144, 8, 4096, None, 64), (6144, 2048, 8, 4096, None, 16), (6144, 2048, 8, 4096, None, 700),
+                                         (2048, 2048, 4, 1024, 64, 64), (6144, 2048, 4, 1024, 64, 16), (1536, 1536, 4, 1024, 64, 16)])
+def test_a_call_is_cut_up_once(N, K, d, C, G, M):
+    """The search for the cut of a split-K call is host time that each call pays, no more than once."""
+    from sacq_b200 import _lib, quantize_rows
+    mod = _layer(N, K, d, C, G)
+    x, res = _x(M, K), _x(M, N, seed=4)
+    q, s = quantize_rows(x)
+    lib = ctypes.CDLL(_lib.LIB_PATH)
+    lib.sacq_split_search_count.restype = ctypes.c_int64
+    for call, most in ((lambda: mod(x), 1), (lambda: mod.forward_int8(x), 1), (lambda: mod.forward_residual(x, res), 1),
+                       (lambda: mod.linear_a8(q, s), 1)):
+        call()
+        before = lib.sacq_split_search_count()
+        call()
+        assert lib.sacq_split_search_count() - before <= most
