@@ -132,6 +132,7 @@ quant_act_kernel(const uint16_t* __restrict__ x, int64_t pitch, int64_t K, uint8
 constexpr int kRowsPerCta = 8;
 constexpr int kKeepChunks = 8;
 constexpr int64_t kRowsKernelMaxK = 256 * kKeepChunks;   // rows the lanes hold entirely in registers
+constexpr int64_t kRowsKernelMinM = 256;   // from here on the per-row CTAs outnumber what the device holds at once
 
 template <bool I8, bool WIDE>
 __global__ void __launch_bounds__(kRowsPerCta * 32)
@@ -169,7 +170,7 @@ quant_act_rows_kernel(const uint16_t* __restrict__ x, int64_t pitch, int64_t M, 
 // The same quantizer in front of a split-K GEMM (linear_split_k.cu), made to share an SM with that kernel's CTAs.  In a row of
 // calls this grid waits for the GEMM before it while the GEMM behind it already fetches and expands weights, so whatever
 // keeps the three apart is paid on every call.  Two things did.  An SM whose memory is divided for a kernel of little
-// shared memory takes no CTA of the GEMM before it is idle again, hence the launch's carve-out.  And a GEMM CTA (18 warps of
+// shared memory takes no CTA of the GEMM before it is idle again, hence the carve-out.  And a GEMM CTA (18 warps of
 // 88 registers) leaves 2,304 registers of an SM quarter: a warp of up to 72, where the row kernels have two or six.  GEMM CTAs
 // entered only when the one before had left, 1 to 2 us late.  Quantizer + GEMM in a graph, without / with this kernel:
 // 2048 -> 2048 at 64 tokens 7.5 / 6.5 us, 128 9.2 / 7.6, 6144 -> 2048 at 64 11.0 / 9.6, 128 13.2 / 11.5, 2048 -> 6144 at 64
@@ -219,12 +220,32 @@ quant_act_beside_kernel(const uint16_t* __restrict__ x, int64_t pitch, int64_t M
   }
 }
 
-// Threads per row of the kernel above; 0: one of the others.  A row per CTA while about two per SM hold the rows (370:
-// 6144 -> 2048 at 290 tokens 16.1 / 15.1 us, at 450 18.9 / 19.5), beyond that a warp per row, where its registers hold one
-// (2048 -> 2048 at 700: row CTAs 13.6, warps 12.2 us).
-inline int beside_threads(int64_t M, int64_t K) {
-  if (M <= 370 && K <= kBesideThreads * 8 * kKeepChunks) return kBesideThreads;
-  return K <= kRowsKernelMaxK ? 32 : 0;
+// Threads per row of the kernel above; 0: one of the others.  Quantizer + GEMM in a graph, without / row CTAs / warps:
+// up to 255 tokens a row per CTA (2048 -> 2048 at 100 9.0 / 7.5 / 7.7 us); from there a warp per row, which is four times fewer
+// CTAs to start (2048 -> 1024 at 300 8.8 / 9.4 / 8.4, grouped scales 10.2 / 11.3 / 9.4; 2048 -> 2048 at 700 13.6 / 12.2), but up to
+// 340 row CTAs where GEMM CTAs on most SMs leave few warps a place (2048 -> 6144 at 300 16.0 / 14.3 / 14.9, 370 16.8 / 15.9 / 15.7).
+// Rows that a warp's registers do not hold keep to row CTAs while about two per SM hold them, 370 (4096 -> 1024 at 300
+// 12.1 / 10.2, 6144 -> 1536 INT8 at 340 a twentieth), and 3.5 MB of them next to GEMM CTAs on most SMs (6144 -> 2048 at 290
+// 15.8 / 15.2, 300 15.7 / 16.2, 370 16.8 / 17.6).
+inline int beside_threads(Beside beside, int64_t M, int64_t K) {
+  if (K > kRowsKernelMaxK)
+    return K <= kBesideThreads * 8 * kKeepChunks && M <= 370 && (beside == kBesideSome || M * K <= (7 << 18)) ? kBesideThreads : 0;
+  return M < kRowsKernelMinM || (beside == kBesideMost && M <= 340) ? kBesideThreads : 32;
+}
+
+// The carve-out as an attribute of the function: as one of each launch it costs the host 0.25 us a call (1536 x 1536 at 80 tokens,
+// eager 8.3 against 8.0).
+template <auto Kern, typename... Args>
+cudaError_t launch_carved(const cudaLaunchConfig_t& cfg, Args... args) {
+  static bool configured[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64 || !configured[dev]) {
+    const cudaError_t e = cudaFuncSetAttribute(Kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) return e;
+    if (dev >= 0 && dev < 64) configured[dev] = true;
+  }
+  return cudaLaunchKernelEx(&cfg, Kern, args...);
 }
 
 template <int T, bool I8, bool WIDE>
@@ -233,22 +254,18 @@ cudaError_t launch_beside(cudaLaunchConfig_t& cfg, const uint16_t* x, int64_t pi
   cfg.gridDim = dim3((unsigned)((M + R - 1) / R));
   cfg.blockDim = dim3(kBesideThreads);
   const int64_t per_thread = (K / 8 + T - 1) / T;
-  if (per_thread <= 2) return cudaLaunchKernelEx(&cfg, quant_act_beside_kernel<T, 2, I8, WIDE>, x, pitch, M, K, q, scale);
-  if (per_thread <= 4) return cudaLaunchKernelEx(&cfg, quant_act_beside_kernel<T, 4, I8, WIDE>, x, pitch, M, K, q, scale);
-  return cudaLaunchKernelEx(&cfg, quant_act_beside_kernel<T, kKeepChunks, I8, WIDE>, x, pitch, M, K, q, scale);
+  if (per_thread <= 2) return launch_carved<quant_act_beside_kernel<T, 2, I8, WIDE>>(cfg, x, pitch, M, K, q, scale);
+  if (per_thread <= 4) return launch_carved<quant_act_beside_kernel<T, 4, I8, WIDE>>(cfg, x, pitch, M, K, q, scale);
+  return launch_carved<quant_act_beside_kernel<T, kKeepChunks, I8, WIDE>>(cfg, x, pitch, M, K, q, scale);
 }
 
-constexpr int64_t kRowsKernelMinM = 256;   // from here on the per-row CTAs outnumber what the device holds at once
-
 template <bool I8, bool WIDE>
-cudaError_t launch_quant(cudaLaunchConfig_t& cfg, bool vec, bool beside, const uint16_t* x, int64_t pitch, int64_t M, int64_t K,
+cudaError_t launch_quant(cudaLaunchConfig_t& cfg, bool vec, Beside beside, const uint16_t* x, int64_t pitch, int64_t M, int64_t K,
                          uint8_t* q, float* scale) {
-  const int t = vec && beside ? beside_threads(M, K) : 0;
-  if (t > 0) {
-    cfg.numAttrs = 2;
+  const int t = vec && beside != kBesideNone ? beside_threads(beside, M, K) : 0;
+  if (t > 0)
     return t == 32 ? launch_beside<32, I8, WIDE>(cfg, x, pitch, M, K, q, scale)
                    : launch_beside<kBesideThreads, I8, WIDE>(cfg, x, pitch, M, K, q, scale);
-  }
   if (vec && M >= kRowsKernelMinM && K <= kRowsKernelMaxK) {
     cfg.gridDim = dim3((unsigned)((M + kRowsPerCta - 1) / kRowsPerCta));
     cfg.blockDim = dim3(kRowsPerCta * 32);
@@ -277,7 +294,7 @@ SACQ_TL_DEFINE_DUMP(sacq_debug_timeline_quant)
 #endif
 
 int launch_quant_act(const void* x, int64_t pitch, int64_t M, int64_t K, bool int8, bool wide, void* q, float* scale,
-                     cudaStream_t s, bool beside) {
+                     cudaStream_t s, Beside beside) {
   if (M == 0 || K == 0) return SACQ_OK;
   const bool vec = (K % 8 == 0) && (pitch % 8 == 0) && (reinterpret_cast<uintptr_t>(x) % 16 == 0) &&
                    (reinterpret_cast<uintptr_t>(q) % (wide ? 16 : 8) == 0);
@@ -287,11 +304,9 @@ int launch_quant_act(const void* x, int64_t pitch, int64_t M, int64_t K, bool in
   cfg.gridDim = dim3((unsigned)M);
   cfg.blockDim = dim3(kThreads);
   cfg.stream = s;
-  cudaLaunchAttribute attr[2];
+  cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;      // used by quant_act_beside_kernel
-  attr[1].val.sharedMemCarveout = cudaSharedmemCarveoutMaxShared;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   const uint16_t* xp = static_cast<const uint16_t*>(x);

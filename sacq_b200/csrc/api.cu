@@ -789,7 +789,7 @@ int forward_impl(const sacq_layer_t* L, const void* x_bf16, int64_t x_pitch, int
   if (int rc = check_layer(L)) return rc;
   if (M == 0) return SACQ_OK;
   const int64_t K = L->d.in_features;
-  bool beside = false;                                // the quantizer runs beside the split-K kernel
+  Beside beside = kBesideNone;                        // the quantizer runs beside the split-K kernel
   SplitChoice c;                                      // how that kernel's call is cut up: searched once (0.2 to 0.4 us)
   const SplitChoice* cut = nullptr;
   int64_t slab = 0;                                   // tokens up to which the GEMM takes fp16 activations in one piece
@@ -816,7 +816,7 @@ int forward_impl(const sacq_layer_t* L, const void* x_bf16, int64_t x_pitch, int
                                 nullptr, nullptr, x_bf16, x_pitch);
         }
         // a projection with a residual follows attention, not a GEMM: nothing to share an SM with (prefill block at 300 tokens 90.7 / 91.2 us)
-        beside = residual == nullptr && split_k_beside(L, M, c);
+        if (residual == nullptr) beside = split_k_beside(L, M, c);
       }
     }
     if (r == kInt8TmemGrouped || k == 5) {
@@ -838,8 +838,8 @@ int forward_impl(const sacq_layer_t* L, const void* x_bf16, int64_t x_pitch, int
     return linear_a8_impl(L, a16, scale_scratch, M, residual, ldr, y_out, ldy, workspace, workspace_bytes, stream, nullptr,
                           kActHalf, cut);
   }
-  const int rc = beside && q_scratch != nullptr && scale_scratch != nullptr
-                     ? launch_quant_act(x_bf16, x_pitch, M, K, int8 != 0, false, q_scratch, scale_scratch, static_cast<cudaStream_t>(stream), true)
+  const int rc = beside != kBesideNone && q_scratch != nullptr && scale_scratch != nullptr
+                     ? launch_quant_act(x_bf16, x_pitch, M, K, int8 != 0, false, q_scratch, scale_scratch, static_cast<cudaStream_t>(stream), beside)
                  : int8 ? sacq_quant_act_int8(x_bf16, x_pitch, M, K, q_scratch, scale_scratch, stream)
                         : sacq_quant_act_fp8(x_bf16, x_pitch, M, K, q_scratch, scale_scratch, stream);
   if (rc != SACQ_OK) return rc;

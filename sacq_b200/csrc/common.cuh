@@ -82,9 +82,11 @@ int launch_weight_row_scale(const sacq_layer* L, float* sw, cudaStream_t s, floa
 int launch_decode_weight_fp8(const sacq_layer* L, const float* sw, void* wq, cudaStream_t s);
 int launch_decode_weight_int8(const sacq_layer* L, const float* sw, void* wq, cudaStream_t s);
 // Per-token quantizer, e4m3 or int8.  wide: the encoded values go out as fp16 [M, K] (the operand of the fp16
-// tensor-core kernels) instead of bytes.  beside: the kernel behind it is a split-K GEMM whose CTAs it should share SMs with.
+// tensor-core kernels) instead of bytes.  beside: whether the kernel behind it is a split-K GEMM whose CTAs it should share SMs
+// with, and whether those are on nearly all SMs.
+enum Beside { kBesideNone = 0, kBesideSome = 1, kBesideMost = 2 };
 int launch_quant_act(const void* x, int64_t pitch, int64_t M, int64_t K, bool int8, bool wide, void* q, float* scale,
-                     cudaStream_t s, bool beside = false);
+                     cudaStream_t s, Beside beside = kBesideNone);
 int launch_act_quant_fp8(int kind, const void* a, int64_t a_pitch, const void* b, int64_t b_pitch, const void* c,
                          int64_t M, int64_t K, void* q, float* scale, cudaStream_t s);
 int launch_layernorm_quant_fp8(const void* x, int64_t pitch, const void* gamma, const void* beta, float eps,

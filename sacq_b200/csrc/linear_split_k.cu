@@ -1074,8 +1074,11 @@ int64_t split_k_ctas(const sacq_layer* L, const SplitChoice& c) {
   return (L->d.out_features + kRows - 1) / kRows * c.tiles * c.split;
 }
 
-bool split_k_beside(const sacq_layer* L, int64_t M, const SplitChoice& c) {
-  return codebook_smem(L) > 0 && M <= (L->d.out_features < 4096 ? 1024 : 512) && 2 * split_k_ctas(L, c) + M > L->num_sms;
+Beside split_k_beside(const sacq_layer* L, int64_t M, const SplitChoice& c) {
+  const bool wide = L->d.out_features >= 4096;
+  const int64_t ctas = split_k_ctas(L, c), room = L->num_sms + (L->d.in_features <= 2048 ? 12 : 0);
+  if (codebook_smem(L) == 0 || M > (wide ? 512 : 1024) || 2 * ctas + M <= room) return kBesideNone;
+  return wide || 6 * ctas > 5 * L->num_sms ? kBesideMost : kBesideSome;
 }
 
 bool split_k_codebook_in_smem(const sacq_layer* L) { return codebook_smem(L) > 0; }

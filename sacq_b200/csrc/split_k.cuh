@@ -55,8 +55,9 @@ bool split_k_codebook_in_smem(const sacq_layer* L);
 // Not where the codebook is gathered through L1, which the quantizer's carve-out would take from the SM (65,536 entries,
 // 2048 -> 6144 at 16 tokens 11.3 / 14.4 us), not for wide layers of several waves (2048 -> 6144 at 700 27.5 / 27.6; 2048 -> 2048
 // 13.7 / 12.2), and not where the chip has room for the CTAs of two GEMMs and the quantizer's beside each other (INT8, 2048 -> 1024,
-// d = 4, at 40 tokens 9.6 / 9.9).
-bool split_k_beside(const sacq_layer* L, int64_t M, const SplitChoice& c);
+// d = 4, at 40 tokens 9.6 / 9.9; at the edge, 2048 -> 1536 INT8 at 64 with 2 x 48 + 64 CTAs, 7.8 / 7.6 in a graph, but 7.7 / 8.2
+// eager), which deep layers with their longer rows need not wait for (6144 -> 1536 at 64, as many CTAs, 10.4 / 9.5).
+Beside split_k_beside(const sacq_layer* L, int64_t M, const SplitChoice& c);
 void split_k_release(sacq_layer* L);
 
 }  // namespace sacq

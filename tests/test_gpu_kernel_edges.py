@@ -258,6 +258,19 @@ def test_quantizer_beside_the_split_k_kernel(N, K, d, C, G):
     assert mod.device_status() == 0
 
 
+@pytest.mark.parametrize("N,K,d,C,G", [(2048, 2048, 8, 4096, None), (4224, 1024, 8, 256, None), (1536, 1536, 4, 64, 64),
+                                       (1024, 2176, 8, 256, None), (2048, 6144, 8, 256, None)])
+def test_rows_per_cta_of_the_quantizer_beside_the_split_k_kernel(N, K, d, C, G):
+    """The numbers of tokens at which that quantizer takes a row per CTA or per warp, or leaves the rows to another one."""
+    from sacq_b200 import quantize_rows
+    mod = _layer(N, K, d, C, G)
+    x = _x(372, K)
+    for M in (52, 64, 65, 100, 255, 256, 257, 298, 299, 340, 341, 372):
+        for forward, gemm, mode in ((mod, mod.linear_a8, "fp8_e4m3fn"), (mod.forward_int8, mod.linear_a8i, "int8_symmetric")):
+            assert torch.equal(forward(x[:M]), gemm(*quantize_rows(x[:M], mode))), (M, mode)
+    assert mod.device_status() == 0
+
+
 @pytest.mark.parametrize("N,K,d,C", [(6144, 2048, 8, 4096), (4100, 1024, 8, 256), (6200, 512, 8, 256), (1000, 1024, 4, 4096),
                                      (2048, 2048, 8, 65536), (4096, 1536, 8, 65536)])
 def test_quantizer_inside_the_split_k_kernel(N, K, d, C):
