@@ -63,22 +63,29 @@ int64_t small_m_slab_rows(const sacq_layer* L) {
   return chunks * 16;
 }
 
+// Rows of a layer in whole row tiles of the split-K kernel.
+int64_t tiled_rows(const sacq_layer* L) { return (L->d.out_features + 127) / 128 * 128; }
+
 // Rows from which the grouped split-K kernel takes over from the index-unpacking warp-MMA kernel, which walks the
 // weights once per 48 tokens and multiplies exact weights (quantizer + GEMM, d = 4, 10-bit, group 64: 2048x6144 19.0 / 10.1 us
 // at 32 rows; 2048x2048 9.2 / 7.8 and 6144x2048 20.5 / 12.8 at 47, there with weights of 11 bits, which up to 47 rows would be
-// less than before; the smallest lose a tenth, 1024x1024 5.4 / 6.0).  With exact weights and the quantizer beside it the
-// split-K kernel is the faster one on the widest layers from the ninth row on (2048x6144, 10-bit: 12.7 / 11.4 us at 16, 11.9 / 11.3
-// at two, but with 64 entries even at eight; 1536x6144 eager 9.8 / 9.7 at 16, 9.5 / 9.7 at eight), on 4,096 rows from the second
-// chunk on (1024x4096 at 17 to 32 10.3 / 6.6; at 16 eager 6.2 / 7.6, the other one being a single launch) and on deep layers
-// around its end (6144x2048 15.6 / 13.8 at 32, 19.4 / 14.0 at 40; 64 entries, eager, at 24 13.8 / 14.3; codebooks of
-// up to 32 entries, whose gathers meet fewer bank conflicts, are not measured and stay), not on smaller ones (2048x2048 at 41
-// 9.2 / 10.0, 4096x1024 9.2 / 10.5).
+// less than before; the smallest lose a tenth, 1024x1024 5.4 / 6.0).  With exact weights, a forward and a call on quantized
+// activations, which this kernel has to widen, in a graph as shares of the other kernel's time:
+//  * on the widest layers from the ninth row on, if they have many vectors (d = 4, at 9 / 16 rows: 2048x6144 0.91 / 0.89 and
+//    0.96 / 0.94, 3072x5632 0.73 / 0.72 and 0.77 / 0.78; 2048x5000 0.95 / 0.91 and 0.99 / 0.98, but eager 0.99 / 0.96 and 1.03 / 1.02;
+//    3072x4736, fewer row tiles, 0.97 / 0.96 and 1.20 / 1.20; below nine rows gains and losses are even);
+//  * on 4,096 rows from the second chunk on (at 17 / 32: 1024x4096 0.66 / 0.73 and 0.77 / 0.75, 3072x4096 0.81 / 0.78 and 0.95 / 0.91,
+//    d = 8 0.84 / 0.81 and 0.99 / 0.96; at 16 eager 1024x4096 6.2 / 7.6 us, the other one being a single launch);
+//  * on deep layers from the third on (at 32 / 33: 6144x2048 0.93 / 0.76 and 1.14 / 0.91, 4096x2048 0.93 / 0.77 and 1.11 / 0.91).
+//    Codebooks of up to 32 entries gain as much, but the tests hold the other kernel's bytes on them;
+//  * not on smaller ones (2048x2048 at 41 9.2 / 10.0 us, 4096x1024 9.2 / 10.5).
 int64_t grouped_min_m(const sacq_layer* L) {
   // ... or from the CUDA-core kernel, at any number (2048x2048, 65,536 entries, group 128: 127 / 11 us at 17 rows)
   if (L->small_m_warps == 0) return 1;
-  if (L->d.out_features >= 32 * (int64_t)L->num_sms) return L->d.in_features * L->d.out_features / L->d.vector_dim >= (3 << 20) ? 9 : 17;
+  const int64_t rows = tiled_rows(L);
+  if (rows >= 44 * 128) return L->d.in_features * rows / L->d.vector_dim >= (3 << 20) ? 9 : 17;
   if (L->d.out_features >= 4096) return 17;
-  return L->d.in_features >= 4096 && L->d.in_features * L->d.out_features >= (8 << 20) && L->d.index_bits > 5 ? 29 : 48;
+  return L->d.in_features >= 4096 && L->d.in_features * L->d.out_features >= (8 << 20) && L->d.index_bits > 5 ? 33 : 48;
 }
 // From how many tokens the persistent kernel with the weights in tensor memory takes over; its 128-row tiles need that many
 // to fill the device.  The split-K kernel expands a wide layer again for every second 384-token tile, from about 700 tokens

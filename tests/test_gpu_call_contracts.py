@@ -376,3 +376,17 @@ def test_a_call_is_cut_up_once(N, K, d, C, G, M):
         before = lib.sacq_split_search_count()
         call()
         assert lib.sacq_split_search_count() - before <= most
+
+
+@pytest.mark.parametrize("N,K,first", [(2048, 6144, 33), (2048, 4096, 33), (4736, 3072, 17), (4096, 1024, 17), (5632, 3072, 9),
+                                       (6144, 2048, 9), (6020, 2048, 9), (5000, 2048, 17), (2048, 2048, 48)])
+def test_where_the_grouped_split_k_kernel_takes_over(N, K, first):
+    """From the first number of tokens at which it is the faster one both for a forward and for a call on quantized activations;
+    below, the bytes are the index-unpacking kernel's."""
+    from sacq_b200 import quantize_rows
+    mod = _layer(N, K, 4, 1024, 64)
+    q, s = quantize_rows(_x(first, K))
+    assert mod.kernel_for(first - 1) == "small" and mod.kernel_for(first) == "large_grouped"
+    below = mod.linear_a8(q[:first - 1], s[:first - 1])
+    mod.set_kernel("small_mma_unpacked")
+    assert torch.equal(mod.linear_a8(q[:first - 1], s[:first - 1]), below)
