@@ -93,7 +93,8 @@ int64_t grouped_min_m(const sacq_layer* L) {
 // the two sum in different orders, and up to there the tokens of a request get the same bytes alone and in a batch of
 // three (the price: 2048x6144 at 700 tokens 30.6 / 19.4).  Below 1,024 of K they do sum alike, but there sibling layers gain by the
 // split-K kernel's shared launch what one layer loses (768x4096 at 560 9.7 / 9.1, two of them 11.2 / 16.2).  A codebook that is
-// gathered from L2 makes an expansion twice as dear (2048x6144 at 400 30.4 / 28.7).  Narrower layers lose nothing (2048x2048 at 1,000 17.6 / 16.3, 6144x1536 30 / 37).
+// gathered from L2 makes an expansion twice as dear (2048x6144 at 400 30.4 / 28.7).  Narrower layers lose nothing (2048x2048
+// at 1,000 17.6 / 16.3, 6144x1536 30 / 37).
 int64_t tmem_min_m(const sacq_layer* L) {
   if (L->d.out_features < 4096) return 1024;
   return split_k_codebook_in_smem(L) ? 960 : 384;
@@ -104,14 +105,20 @@ int64_t tmem_min_m(const sacq_layer* L) {
 // A codebook in L2 leaves the small-M kernel 2 warps' gathers in flight per scheduler: the split-K kernel wins from one
 // token on (65,536 entries, 2048x6144: 17.4 / 11.3 us at 16 tokens; 6144x2048 13.4 / 11.1 at one, 13.7 / 11.5 at 16;
 // 2048x2048 7.2 / 7.0 and 7.6 / 7.1), on the smallest layers from the second chunk on (2048x1024 6.4 / 7.2 at 16 and
-// 7.6 / 7.2 at 32, 1024x1024 5.5 / 5.8 and 6.4 / 5.8).  So it does on wide layers of many vectors, which the small-M kernel
-// takes in tiles of 48 rows (2048x6144 7.4 / 6.9 at one token, 8.0 / 7.1 at 16), and where they are shallow, from where it alone
-// quantizes in the same launch (1024x4096, eager, 7.5 / 5.5 at eight; at one token 5.6 / 5.4, but 6.5 / 7.1 on a slower host), but
-// not between, where the small-M kernel is even (1536x6144 6.3 / 6.4 at one token, 6.7 / 6.5 at 16), or on deep layers (6144x2048 8.0 / 8.3 at eight).  Dim-4 vectors keep the small-M kernel, whose bytes up to 16 tokens the tests pin (8.8 / 7.8).
+// 7.6 / 7.2 at 32, 1024x1024 5.5 / 5.8 and 6.4 / 5.8).
+// Dim-8 layers of 4,096 rows and more, shares of the small-M kernel's time in a graph / eager:
+//  * 12 M weights: from one token on (2048x6144 0.93 / 0.93 at one, 0.90 / 0.94 at 16; 3072x4096 0.95 / 0.96 and 0.94 / 0.90; 4096x4096
+//    0.93 / 0.89 and 0.89 / 0.85; 2048x8192 0.80 / 0.82 and 0.70 / 0.75).  2048x5120 gains as much (0.92 / 0.93), but the tests hold the
+//    small-M kernel's bytes on 5,992 rows of 2,048, a row tile below the line; 1536x6144 is even (1.00 / 0.99 and 0.95 / 0.98);
+//  * at most 1,024 of K: from where the split-K kernel alone quantizes in the same launch (1024x4096 eager 7.5 / 5.5 us at eight; at one
+//    token 5.6 / 5.4 on one host, 6.5 / 7.1 on another).
+// Narrower deep layers keep the small-M kernel (6144x2048 8.0 / 8.3 at eight), and so do dim-4 vectors, whose bytes up to 16
+// tokens the tests hold (2048x6144 8.8 / 7.8).
 bool split_wins(const sacq_layer* L, int64_t M) {
   const int64_t work = L->d.in_features * L->d.out_features;
   if (!split_k_codebook_in_smem(L)) return M > 16 || work > (2 << 20) || L->d.out_features >= 4096;
-  if (L->d.out_features >= 4096 && L->d.vector_dim == 8 && (work >= (12 << 20) || (L->d.in_features <= 1024 && M > L->small_m_warps)))
+  if (L->d.out_features >= 4096 && L->d.vector_dim == 8 &&
+      (L->d.in_features * tiled_rows(L) >= (12 << 20) || (L->d.in_features <= 1024 && M > L->small_m_warps)))
     return true;
   return (M > 16 && (L->d.out_features >= 4096 || work >= (8 << 20))) || M > 32;
 }

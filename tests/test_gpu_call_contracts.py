@@ -390,3 +390,18 @@ def test_where_the_grouped_split_k_kernel_takes_over(N, K, first):
     below = mod.linear_a8(q[:first - 1], s[:first - 1])
     mod.set_kernel("small_mma_unpacked")
     assert torch.equal(mod.linear_a8(q[:first - 1], s[:first - 1]), below)
+
+
+@pytest.mark.parametrize("N,K,kernel", [(6144, 2048, "large"), (6020, 2048, "large"), (4090, 3072, "small"), (4096, 3072, "large"),
+                                        (5992, 2048, "small"), (6144, 1536, "small"), (2048, 6144, "small")])
+def test_which_layers_leave_the_small_m_kernel_at_one_token(N, K, kernel):
+    """Rows count in whole row tiles, so a layer that lacks a few rows of a wider one runs on its kernel."""
+    from sacq_b200 import quantize_rows
+    mod = _layer(N, K)
+    q, s = quantize_rows(_x(16, K))
+    for M in (1, 16):
+        assert mod.kernel_for(M) == kernel
+        y = mod.linear_a8(q[:M], s[:M])
+        mod.set_kernel(kernel)
+        assert torch.equal(mod.linear_a8(q[:M], s[:M]), y)
+        mod.set_kernel("auto")
