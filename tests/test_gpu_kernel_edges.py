@@ -275,10 +275,12 @@ def test_rows_per_cta_of_the_quantizer_beside_the_split_k_kernel(N, K, d, C, G):
                                      (2048, 2048, 8, 65536), (4096, 1536, 8, 65536)])
 def test_quantizer_inside_the_split_k_kernel(N, K, d, C):
     """Expander warps that quantize their tokens themselves give the bytes of the separate calls: one or two tokens a warp, tiles
-    that end early, rows with a pitch, of zeros, infinities and NaN, a residual, a capture."""
+    that end early, rows with a pitch, of zeros, infinities and NaN, a residual, a capture.  It is one launch up to 16 tokens, two
+    from 65 on; captured, two where the layer's CTAs wait for SMs."""
     from sacq_b200 import quantize_rows
     mod = _layer(N, K, d, C)
     mod.set_kernel("large")
+    count = mod._lib.sacq_launch_count
     wide = _x(66, K + 16)
     wide[3] = 0
     wide[5, 7] = float("inf")
@@ -287,13 +289,19 @@ def test_quantizer_inside_the_split_k_kernel(N, K, d, C):
     for x in (wide[:, :K].contiguous(), wide[:, 8:K + 8]):
         for M in (1, 2, 8, 15, 16, 17, 31, 32, 33, 48, 64, 65):
             q, s = quantize_rows(x[:M])
-            for y, ref in ((mod(x[:M]), mod.linear_a8(q, s)), (mod.forward_residual(x[:M], res[:M]), mod.linear_a8(q, s, residual=res[:M]))):
+            before = count()
+            got = mod(x[:M]), mod.forward_residual(x[:M], res[:M])
+            launches = count() - before
+            assert launches == (2 if M <= 16 else 4 if M == 65 else launches), M
+            for y, ref in zip(got, (mod.linear_a8(q, s), mod.linear_a8(q, s, residual=res[:M]))):
                 assert torch.equal(y.view(torch.int16), ref.view(torch.int16)), M
     x, stream = wide[:16, :K].contiguous(), torch.cuda.Stream()
     graph = torch.cuda.CUDAGraph()
     torch.cuda.synchronize()
+    before = count()
     with torch.cuda.graph(graph, stream=stream):
         y = mod(x)
+    assert count() - before == (2 if (N, C) == (6144, 4096) else 1)
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(y.view(torch.int16), mod(x).view(torch.int16)) and mod.device_status() == 0
