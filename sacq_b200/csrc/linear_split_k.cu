@@ -1085,7 +1085,7 @@ bool split_k_codebook_in_smem(const sacq_layer* L) { return codebook_smem(L) > 0
 
 bool split_k_quantizes(const sacq_layer* L, const SplitChoice& c) {
   const int64_t K = L->d.in_features;
-  if (c.tok > 32 || K > 8192 || c.parts > 1 || c.box_shift != 2 || (c.split > 1 && !c.own_recv)) return false;
+  if (c.tok > 32 || c.parts > 1 || c.box_shift != 2 || (c.split > 1 && !c.own_recv)) return false;
   const int stages = (stages_of(K) + c.split - 1) / c.split;
   if (stages > c.act_stages) return false;            // every activation tile has a place of its own
   const SplitLayout l = split_layout(c.tok, c.split, c.act_stages, c.max_slices, c.box_shift, 0, codebook_smem(L), c.own_recv, (int)(c.tok * K * 2));
